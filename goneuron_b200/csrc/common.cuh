@@ -67,6 +67,12 @@ inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 #define GN_LAUNCH(ctx, kernel, grid, block, smem, ...)                         \
   do { kernel<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__); (ctx)->launches++; } while (0)
 
+// The same with `cx` neighbouring blocks of the grid's x dimension as one thread-block cluster.
+#define GN_CLUSTER_LAUNCH(ctx, kernel, grid, block, cx, ...)                   \
+  do { cudaLaunchConfig_t cfg_{}; cfg_.gridDim = (grid); cfg_.blockDim = dim3(block); cfg_.stream = (ctx)->stream;                                   \
+       cudaLaunchAttribute at_[1]; at_[0].id = cudaLaunchAttributeClusterDimension; at_[0].val.clusterDim.x = (cx); at_[0].val.clusterDim.y = at_[0].val.clusterDim.z = 1; \
+       cfg_.attrs = at_; cfg_.numAttrs = 1; GN_CUDA(cudaLaunchKernelEx(&cfg_, kernel, __VA_ARGS__)); (ctx)->launches++; } while (0)
+
 inline int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(GN_ERR_CUDA, "kernel launch failed (%s): %s", what, cudaGetErrorString(e));

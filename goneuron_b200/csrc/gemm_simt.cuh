@@ -7,6 +7,7 @@
 // kernel.  It is the exact-fp32 engine: small and oddly shaped contractions use it,
 // and the tensor-core engine is checked against it.
 #pragma once
+#include <cooperative_groups.h>
 #include "common.cuh"
 
 namespace gn {
@@ -29,6 +30,7 @@ struct GemmDesc {
   const void* b_planes = nullptr;                       // tensor-core engine: prepared operand planes of B (a BfPlanes), e.g. of a weight matrix
   const void* a_planes = nullptr;                       // ... and of A (written by the epilogue of the contraction that produced A)
   const void* plane_out = nullptr;                      // tensor-core engine: a TcPlaneOut; the result is written as operand planes instead of fp32
+  float* a_sum = nullptr;                               // CUDA-core engine: receives sum_k A(m,k), [M] (the bias gradient next to a weight gradient)
   float* a_rownorm = nullptr;                           // tensor-core engine: receives the L2 norm of every row of A (from the split pass)
   int batch1 = 1, batch2 = 1;                           // batch index b -> (b / batch2, b % batch2)
   long a_b1 = 0, a_b2 = 0, b_b1 = 0, b_b2 = 0, c_b1 = 0, c_b2 = 0, r_b1 = 0, r_b2 = 0;
@@ -39,112 +41,212 @@ struct GemmDesc {
   int flags = 0;
 };
 
-constexpr int SG_BM = 128, SG_BN = 128, SG_BK = 16, SG_PAD = 4, SG_THREADS = 256;
+// ------------------------------------------------------------------ tiled kernel
+// One BM x BN output tile per cluster of `splits` blocks (1, 2, 4 or 8).  The contraction is cut into `splits` equal runs, one
+// per block of the cluster; the blocks leave their sums in shared memory, and after a cluster barrier each of them adds up and
+// stores its share of the tile's elements, always in rank order, so a result does not depend on scheduling.  This is what
+// these products need: they come from small batches and narrow layers (a [64, 784] x [784, 128] forward product, a
+// [96, 96] weight gradient over 5000 rows), where a single 128 x 128 tile per block left all but a few SMs idle and one block
+// walking the whole contraction -- 72 us for the former and 430 us for the latter, against 7 and 12 us now.
+// Global loads of a k-step go to registers while the previous one is multiplied, then to the other shared-memory buffer.
+// 16-byte loads along the operand's fast index where base, stride and range allow it.
+constexpr int SG_PAD = 4, SG_MAX_SPLITS = 8, SG_RUN = 32;      // runs start at multiples of SG_RUN, whatever the tile
+template <int BM, int BN, int BK, int TM, int TN> struct SgCfg {
+  static constexpr int THREADS = (BM / TM) * (BN / TN);
+  static constexpr int LDA = BM + SG_PAD, LDB = BN + SG_PAD;
+  static constexpr int STAGE = BK * (LDA + LDB);
+  static constexpr int SMEM_FLOATS = 2 * STAGE > BM * BN ? 2 * STAGE : BM * BN;
+};
 
-template <bool A_KFAST, bool B_NFAST>
-__global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(GemmDesc g) {
-  __shared__ __align__(16) float As[SG_BK][SG_BM + SG_PAD];
-  __shared__ __align__(16) float Bs[SG_BK][SG_BN + SG_PAD];
-  const int b = blockIdx.z, b1 = b / g.batch2, b2 = b % g.batch2;
+// A rows x BK slab of an operand: element (r, k) at p[r * s_r + k * s_k], r < nr, k < nk (both relative), zero outside.
+// Thread t owns vectors of four: along k (KFAST) or along r.
+template <int ROWS, int BK, int THREADS, bool KFAST>
+struct SgSlab {
+  static constexpr int NV = (ROWS * BK / 4 + THREADS - 1) / THREADS;
+  float4 v[NV];
+  static constexpr bool EXACT = (ROWS * BK / 4) % THREADS == 0;
+  __device__ __forceinline__ static void place(int i, int& r, int& k) {
+    if (KFAST) { k = (i % (BK / 4)) * 4; r = i / (BK / 4); } else { r = (i % (ROWS / 4)) * 4; k = i / (ROWS / 4); }
+  }
+  __device__ __forceinline__ void fetch(const float* __restrict__ p, long s_r, long s_k, int nr, int nk, bool vec) {
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+      const int i = threadIdx.x + q * THREADS; int r, k; place(i, r, k);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (EXACT || i < ROWS * BK / 4) {
+        if (KFAST) {
+          const float* s = p + r * s_r + k;
+          if (r < nr) {
+            if (vec && k + 3 < nk) x = *reinterpret_cast<const float4*>(s);
+            else { if (k < nk) x.x = s[0]; if (k + 1 < nk) x.y = s[1]; if (k + 2 < nk) x.z = s[2]; if (k + 3 < nk) x.w = s[3]; }
+          }
+        } else {
+          const float* s = p + r + k * s_k;
+          if (k < nk) {
+            if (vec && r + 3 < nr) x = *reinterpret_cast<const float4*>(s);
+            else { if (r < nr) x.x = s[0]; if (r + 1 < nr) x.y = s[1]; if (r + 2 < nr) x.z = s[2]; if (r + 3 < nr) x.w = s[3]; }
+          }
+        }
+      }
+      v[q] = x;
+    }
+  }
+  __device__ __forceinline__ void put(float* __restrict__ sm, int ld) const {      // sm[k][r]
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+      const int i = threadIdx.x + q * THREADS; int r, k; place(i, r, k);
+      if (!EXACT && i >= ROWS * BK / 4) continue;
+      if (KFAST) { sm[k * ld + r] = v[q].x; sm[(k + 1) * ld + r] = v[q].y; sm[(k + 2) * ld + r] = v[q].z; sm[(k + 3) * ld + r] = v[q].w; }
+      else *reinterpret_cast<float4*>(sm + k * ld + r) = v[q];
+    }
+  }
+};
+
+__device__ __forceinline__ float sg_finish(const GemmDesc& g, const float* R, int m, int n, float acc) {
+  float v = g.alpha * acc;
+  if (g.bias) v += g.bias[n];
+  if (R) v += R[m * g.ldr + n];
+  if (g.act == GN_ACT_RELU) v = v > 0.f ? v : 0.f;
+  if (g.mask && !(g.mask[(long)(m / g.mask_group) * g.mask_ld + n] > 0.f)) v = 0.f;
+  return v;
+}
+
+template <int BM, int BN, int BK, int TM, int TN, bool A_KFAST, bool B_NFAST>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmDesc g, int splits, int vec_a, int vec_b) {
+  using Cfg = SgCfg<BM, BN, BK, TM, TN>;
+  constexpr int THREADS = Cfg::THREADS, LDA = Cfg::LDA, LDB = Cfg::LDB, CX = BN / TN;
+  __shared__ __align__(16) float sm[Cfg::SMEM_FLOATS];
+  __shared__ float asum_sh[BM];
+  const int b = blockIdx.z, b1 = b / g.batch2, b2 = b % g.batch2, rank = blockIdx.x % splits, nt = blockIdx.x / splits;
   const float* A = g.A + b1 * g.a_b1 + b2 * g.a_b2;
   const float* B = g.B + b1 * g.b_b1 + b2 * g.b_b2;
   float* C = g.C + b1 * g.c_b1 + b2 * g.c_b2;
-  const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
-  if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + SG_BM - 1) return;
-  int kbeg = 0, kend = g.K;
-  if (g.flags & GEMM_KBEG_AT_M0) kbeg = (m0 / SG_BK) * SG_BK;
-  if (g.flags & GEMM_KEND_AT_M0) kend = min(g.K, m0 + SG_BM);
-  const int t = threadIdx.x, ty = t / 16, tx = t % 16;
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; i++)
-#pragma unroll
-    for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-
-  for (int k0 = kbeg; k0 < kend; k0 += SG_BK) {
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      int idx = t + SG_THREADS * e;
-      int m, k;
-      if (A_KFAST) { k = idx % SG_BK; m = idx / SG_BK; } else { m = idx % SG_BM; k = idx / SG_BM; }
-      int gm = m0 + m, gk = k0 + k;
-      As[k][m] = (gm < g.M && gk < kend) ? A[gm * g.sa_m + gk * g.sa_k] : 0.f;
-    }
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      int idx = t + SG_THREADS * e;
-      int n, k;
-      if (B_NFAST) { n = idx % SG_BN; k = idx / SG_BN; } else { k = idx % SG_BK; n = idx / SG_BK; }
-      int gn_ = n0 + n, gk = k0 + k;
-      Bs[k][n] = (gn_ < g.N && gk < kend) ? B[gk * g.sb_k + gn_ * g.sb_n] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < SG_BK; k++) {
-      float4 a0 = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      float4 a1 = *reinterpret_cast<const float4*>(&As[k][64 + ty * 4]);
-      float4 c0 = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
-      float4 c1 = *reinterpret_cast<const float4*>(&Bs[k][64 + tx * 4]);
-      float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      float bv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
   const float* R = g.R ? g.R + b1 * g.r_b1 + b2 * g.r_b2 : nullptr;
+  const int m0 = blockIdx.y * BM, n0 = nt * BN;
+  if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + BM - 1) return;             // (the whole cluster returns)
+  int kbeg = 0, kend = g.K;
+  if (g.flags & GEMM_KBEG_AT_M0) kbeg = (m0 / BK) * BK;
+  if (g.flags & GEMM_KEND_AT_M0) kend = min(g.K, m0 + BM);
+  if (splits > 1) {
+    const int per = (((kend - kbeg + splits - 1) / splits + SG_RUN - 1) / SG_RUN) * SG_RUN;
+    kbeg = min(kend, kbeg + rank * per); kend = min(kend, kbeg + per);
+  }
+  const int t = threadIdx.x, ty = t / CX, tx = t % CX;
+  float acc[TM][TN];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-    if (m >= g.M) continue;
+  for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-      if (n >= g.N) continue;
-      float v = g.alpha * acc[i][j];
-      if (g.bias) v += g.bias[n];
-      if (R) v += R[m * g.ldr + n];
-      if (g.act == GN_ACT_RELU) v = v > 0.f ? v : 0.f;
-      if (g.mask && !(g.mask[(long)(m / g.mask_group) * g.mask_ld + n] > 0.f)) v = 0.f;
-      C[m * g.ldc + n] = v;
+    for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
+  const bool want_asum = g.a_sum != nullptr && nt == 0;
+  float asum = 0.f;
+
+  SgSlab<BM, BK, THREADS, A_KFAST> fa; SgSlab<BN, BK, THREADS, !B_NFAST> fb;
+  auto fetch = [&](int k0) {
+    const int nk = kend - k0;
+    fa.fetch(A + (long)m0 * g.sa_m + (long)k0 * g.sa_k, g.sa_m, g.sa_k, g.M - m0, nk, vec_a);
+    fb.fetch(B + (long)n0 * g.sb_n + (long)k0 * g.sb_k, g.sb_n, g.sb_k, g.N - n0, nk, vec_b);
+  };
+  if (kbeg < kend) {
+    fetch(kbeg);
+    fa.put(sm, LDA); fb.put(sm + BK * LDA, LDB);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = kbeg; k0 < kend; k0 += BK, buf ^= 1) {
+      const bool more = k0 + BK < kend;
+      if (more) fetch(k0 + BK);
+      const float* As = sm + buf * Cfg::STAGE; const float* Bs = As + BK * LDA;
+#pragma unroll
+      for (int k = 0; k < BK; k++) {
+        float av[TM], bv[TN];
+#pragma unroll
+        for (int i = 0; i < TM; i++) av[i] = As[k * LDA + ty * TM + i];
+#pragma unroll
+        for (int j = 0; j < TN; j++) bv[j] = Bs[k * LDB + tx * TN + j];
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+          for (int j = 0; j < TN; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      }
+      if (want_asum && t < BM) {
+#pragma unroll
+        for (int k = 0; k < BK; k++) asum += As[k * LDA + t];
+      }
+      if (more) { float* nx = sm + (buf ^ 1) * Cfg::STAGE; fa.put(nx, LDA); fb.put(nx + BK * LDA, LDB); }
+      __syncthreads();
     }
   }
+  if (splits == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; i++) {
+      const int m = m0 + ty * TM + i;
+      if (m >= g.M) continue;
+#pragma unroll
+      for (int j = 0; j < TN; j++) { const int n = n0 + tx * TN + j; if (n < g.N) C[m * g.ldc + n] = sg_finish(g, R, m, n, acc[i][j]); }
+    }
+    if (want_asum && t < BM && m0 + t < g.M) g.a_sum[m0 + t] = asum;
+    return;
+  }
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < TN; j++) sm[(ty * TM + i) * BN + tx * TN + j] = acc[i][j];
+  if (want_asum && t < BM) asum_sh[t] = asum;
+  cluster.sync();
+  const int share = BM * BN / splits;
+  for (int e = rank * share + t; e < (rank + 1) * share; e += THREADS) {
+    const int m = m0 + e / BN, n = n0 + e % BN;
+    if (m >= g.M || n >= g.N) continue;
+    float v = 0.f;
+    for (int q = 0; q < splits; q++) v += cluster.map_shared_rank(sm, q)[e];
+    C[m * g.ldc + n] = sg_finish(g, R, m, n, v);
+  }
+  if (want_asum && rank == 0 && t < BM && m0 + t < g.M) {
+    float v = 0.f;
+    for (int q = 0; q < splits; q++) v += cluster.map_shared_rank(asum_sh, q)[t];
+    g.a_sum[m0 + t] = v;
+  }
+  cluster.sync();                                             // nobody leaves while its sums are being read
 }
 
-// Skinny outputs (N <= 16, both operands K-major, one problem): the tiled kernel would run a handful of CTAs over a
-// long K loop.  Here one block owns one output row: its threads stride over K with all N sums in registers, then
-// combine through shared memory.  C(m,n) = act(sum_k A(m,k) B(n,k) + bias[n] + R(m,n)).
+// Skinny outputs (N <= 16, both operands K-major, one problem): a tile would be mostly padding.  A cluster of `splits`
+// blocks owns one output row: their threads stride over K with all N sums in registers, combine through shared memory, and
+// rank 0 adds the blocks' sums in rank order.  C(m,n) = act(sum_k A(m,k) B(n,k) + bias[n] + R(m,n)).  One block per row (K = 4704,
+// N = 10: 18 loads deep) took 18 us for 50 rows; eight take 4.
 constexpr int SKINNY_N = 16;
-__global__ void __launch_bounds__(256) gemm_skinny_kernel(GemmDesc g) {
+__global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmDesc g, int splits) {
   __shared__ float red[8][SKINNY_N];
-  const int m = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __shared__ float tot[SKINNY_N];
+  const int m = blockIdx.x / splits, rank = blockIdx.x % splits, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float* a = g.A + (long)m * g.sa_m;
   float acc[SKINNY_N];
 #pragma unroll
   for (int n = 0; n < SKINNY_N; n++) acc[n] = 0.f;
-  for (int k = threadIdx.x; k < g.K; k += 256) {
+  for (int k = rank * 256 + threadIdx.x; k < g.K; k += 256 * splits) {
     const float av = a[k];
 #pragma unroll
     for (int n = 0; n < SKINNY_N; n++) if (n < g.N) acc[n] = fmaf(av, g.B[(long)n * g.sb_n + k], acc[n]);
   }
 #pragma unroll
-  for (int n = 0; n < SKINNY_N; n++) { const float v = warp_sum(acc[n]); if (lane == 0) red[w][n] = v; }
+  for (int n = 0; n < SKINNY_N; n++) { if (n < g.N) { const float v = warp_sum(acc[n]); if (lane == 0) red[w][n] = v; } }
   __syncthreads();
   if (threadIdx.x < g.N) {
+    float v = 0.f;
+    for (int q = 0; q < 8; q++) v += red[q][threadIdx.x];
+    tot[threadIdx.x] = v;
+  }
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  if (splits > 1) cluster.sync(); else __syncthreads();
+  if (rank == 0 && threadIdx.x < g.N) {
     const int n = threadIdx.x;
     float v = 0.f;
-    for (int q = 0; q < 8; q++) v += red[q][n];
-    if (g.bias) v += g.bias[n];
-    if (g.R) v += g.R[(long)m * g.ldr + n];
-    if (g.act == GN_ACT_RELU) v = v > 0.f ? v : 0.f;
-    g.C[(long)m * g.ldc + n] = v;
+    for (int q = 0; q < splits; q++) v += splits > 1 ? cluster.map_shared_rank(tot, q)[n] : tot[n];
+    g.C[(long)m * g.ldc + n] = sg_finish(g, g.R, m, n, v);
   }
+  if (splits > 1) cluster.sync();
 }
 inline bool gemm_skinny_ok(const GemmDesc& g) {
-  return g.batch1 * g.batch2 == 1 && g.N <= SKINNY_N && g.K >= 256 && g.sa_k == 1 && g.sb_k == 1 && !g.mask && g.alpha == 1.f && g.flags == 0 &&
-         (g.act == GN_ACT_LINEAR || g.act == GN_ACT_RELU);
+  return g.batch1 * g.batch2 == 1 && g.N <= SKINNY_N && g.K >= 128 && g.sa_k == 1 && g.sb_k == 1 && g.alpha == 1.f && g.flags == 0 && !g.a_sum;
 }
 
 // Sum of at most 64 outer products: C[M,N] = sum_k A(m,k) B(k,n) with both operands stored contraction-major (A(m,k) at
@@ -154,7 +256,7 @@ inline bool gemm_skinny_ok(const GemmDesc& g) {
 // product on 64 blocks of 128 x 128 with a contraction of two 16-steps; this one fills the SMs and is bound by writing C.
 constexpr int OS_KMAX = 64;
 __global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict__ A, long sa_k, const float* __restrict__ B, long sb_k, float* __restrict__ C, long ldc,
-                                                        int M, int N, int K, float alpha) {
+                                                        int M, int N, int K, float alpha, float* __restrict__ a_sum) {
   __shared__ __align__(16) float As[OS_KMAX][64];
   __shared__ __align__(16) float Bs[OS_KMAX][64];
   const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -164,6 +266,7 @@ __global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict_
     Bs[k][c] = n0 + c < N ? B[(long)k * sb_k + n0 + c] : 0.f;
   }
   __syncthreads();
+  if (a_sum && blockIdx.x == 0 && tid < 64 && m0 + tid < M) { float v = 0.f; for (int k = 0; k < K; k++) v += As[k][tid]; a_sum[m0 + tid] = v; }
   float acc[4][4] = {};
   for (int k = 0; k < K; k++) {
     const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]), b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
@@ -188,20 +291,43 @@ inline bool gemm_outer_small_ok(const GemmDesc& g) {
          !g.a_planes && !g.b_planes && !g.plane_out && !g.a_rownorm && (long)g.M * g.N >= 64 * 64;
 }
 
+template <int BM, int BN, int BK, int TM, int TN>
+inline int gemm_simt_tile(Ctx* ctx, const GemmDesc& g, int splits) {
+  auto vec = [](const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; };
+  const bool ak = g.sa_k == 1, bn = g.sb_n == 1;
+  const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
+  const dim3 grid(cdiv(g.N, BN) * splits, cdiv(g.M, BM), g.batch1 * g.batch2); constexpr int THREADS = SgCfg<BM, BN, BK, TM, TN>::THREADS;
+  if (ak && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, splits, g, splits, va, vb);
+  else if (ak && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, splits, g, splits, va, vb);
+  else if (g.sa_m == 1 && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, splits, g, splits, va, vb);
+  else if (g.sa_m == 1 && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, splits, g, splits, va, vb);
+  else return fail(GN_ERR_UNSUPPORTED, "gemm_simt: neither stride of an operand is 1");
+  return check_launch("gemm_simt");
+}
+// Blocks per output tile.  A run shorter than 64 is not worth a block.  Where the rows of A are samples (or tokens), the
+// number does not depend on how many there are: a sample's result is the same in every batch.
+inline int gemm_simt_splits(const GemmDesc& g, int sm_count, long tiles_all, long tiles_n) {
+  const long have = g.sa_k == 1 ? tiles_n : tiles_all;
+  int s = 1;
+  while (s < SG_MAX_SPLITS && g.K >= 128 * s && have * s < sm_count) s *= 2;
+  return s;
+}
 inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
   if (g.M <= 0 || g.N <= 0) return GN_OK;
   if (gemm_outer_small_ok(g)) {
-    GN_LAUNCH(ctx, outer_sum_kernel, dim3(cdiv(g.N, 64), cdiv(g.M, 64)), 256, 0, g.A, g.sa_k, g.B, g.sb_k, g.C, g.ldc, g.M, g.N, g.K, g.alpha);
+    GN_LAUNCH(ctx, outer_sum_kernel, dim3(cdiv(g.N, 64), cdiv(g.M, 64)), 256, 0, g.A, g.sa_k, g.B, g.sb_k, g.C, g.ldc, g.M, g.N, g.K, g.alpha, g.a_sum);
     return check_launch("outer_sum");
   }
-  if (gemm_skinny_ok(g)) { GN_LAUNCH(ctx, gemm_skinny_kernel, g.M, 256, 0, g); return check_launch("gemm_skinny"); }
-  dim3 grid(cdiv(g.N, SG_BN), cdiv(g.M, SG_BM), g.batch1 * g.batch2);
-  bool ak = (g.sa_k == 1), bn = (g.sb_n == 1);
-  if (ak && bn) GN_LAUNCH(ctx, (gemm_simt_kernel<true, true>), grid, SG_THREADS, 0, g);
-  else if (ak && !bn) GN_LAUNCH(ctx, (gemm_simt_kernel<true, false>), grid, SG_THREADS, 0, g);
-  else if (!ak && bn) GN_LAUNCH(ctx, (gemm_simt_kernel<false, true>), grid, SG_THREADS, 0, g);
-  else GN_LAUNCH(ctx, (gemm_simt_kernel<false, false>), grid, SG_THREADS, 0, g);
-  return check_launch("gemm_simt");
+  if (gemm_skinny_ok(g)) {
+    int s = 1; while (s < SG_MAX_SPLITS && g.K >= 512 * s) s *= 2;
+    GN_CLUSTER_LAUNCH(ctx, gemm_skinny_kernel, dim3(g.M * s), 256, s, g, s); return check_launch("gemm_skinny");
+  }
+  const long nb = (long)g.batch1 * g.batch2, t64 = (long)cdiv(g.M, 64) * cdiv(g.N, 64) * nb;
+  const int s = gemm_simt_splits(g, ctx->sm_count, t64, (long)cdiv(g.N, 64));
+  // 16-row tiles for a handful of rows; 32 x 32 tiles (a quarter of the work per block) when 64 x 64 would not give every SM one
+  if (g.M <= 16) return gemm_simt_tile<16, 64, 32, 2, 4>(ctx, g, s);
+  if (t64 * s < ctx->sm_count) return gemm_simt_tile<32, 32, 32, 4, 2>(ctx, g, s);
+  return gemm_simt_tile<64, 64, 16, 4, 4>(ctx, g, s);
 }
 
 }  // namespace gn

@@ -33,9 +33,10 @@ namespace gn {
 // ------------------------------------------------------------------ contraction dispatch
 static bool force_simt_engine() { static const bool f = [] { const char* e = getenv("GONEURON_CUDA_ENGINE"); return e && strcmp(e, "simt") == 0; }(); return f; }
 // Chooses the tensor-core engine for large K-major x K-major products and the SIMT engine for the rest.
+static bool gemm_on_tc(Ctx* ctx, const GemmDesc& g) { return !force_simt_engine() && gemm_tc_eligible(ctx, g) && !gemm_outer_small_ok(g); }
 static int gemm(Ctx* ctx, const GemmDesc& g) {
   int rc;
-  if (!force_simt_engine() && gemm_tc_eligible(ctx, g) && !gemm_outer_small_ok(g)) {     // brackets its kernel launches itself
+  if (gemm_on_tc(ctx, g)) {     // brackets its kernel launches itself
     GemmDesc h = g; if (!h.b_planes) h.b_planes = wplanes_lookup(ctx, g);                 // weight matrices come with prepared planes
     rc = gemm_tc(ctx, h);
   }
@@ -61,6 +62,14 @@ static int gemm_nn(Ctx* ctx, int M, int N, int K, const float* dZ, long ldz, con
 static int gemm_tn(Ctx* ctx, int R, int N, int K, const float* dZ, long ldz, const float* X, long ldx, float* gW) {
   GemmDesc g; g.M = N; g.N = K; g.K = R; g.A = dZ; g.sa_m = 1; g.sa_k = ldz; g.B = X; g.sb_k = ldx; g.sb_n = 1;
   g.C = gW; g.ldc = K; return gemm(ctx, g);
+}
+
+// The same with the bias gradient gb[N] = sum of dZ over its rows, inside the product where the CUDA-core engine runs it.
+static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate);
+static int weight_bias_grads(gn_model* m, Ctx* ctx, int R, int N, int K, const float* dZ, long ldz, const float* X, long ldx, float* gW, float* gb) {
+  GemmDesc g; g.M = N; g.N = K; g.K = R; g.A = dZ; g.sa_m = 1; g.sa_k = ldz; g.B = X; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = K;
+  if (gemm_on_tc(ctx, g)) GN_TRY(colsum(m, dZ, ldz, R, N, gb, false)); else g.a_sum = gb;
+  return gemm(ctx, g);
 }
 
 struct LayerRT;
@@ -669,9 +678,8 @@ static int inner_dense_param_grads(gn_model* m, const float* dz, int B, int T, i
   else if (out % 4 == 0 && ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(delta)) & 15) == 0)
     GN_LAUNCH(ctx, token_sum_vec_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, dz, T, out, delta);
   else GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(out, 128), B), dim3(128, 4), 0, dz, T, out, delta);
-  GN_TRY(colsum(m, delta, out, B, out, gb, false));
-  if (x_last) return gemm_tn(ctx, B, out, in, delta, out, x_last, (long)in, gW);
-  return gemm_tn(ctx, B, out, in, delta, out, x + (long)(T - 1) * in, (long)T * in, gW);
+  if (x_last) return weight_bias_grads(m, ctx, B, out, in, delta, out, x_last, (long)in, gW, gb);
+  return weight_bias_grads(m, ctx, B, out, in, delta, out, x + (long)(T - 1) * in, (long)T * in, gW, gb);
 }
 // Can the FFN's hidden activation (and its gradient) of this block live as operand planes only?  The two contractions on
 // either side must both run on the tensor-core engine with prepared weight planes, and the plane-writing epilogue's shape
@@ -915,8 +923,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
           else GN_LAUNCH(ctx, act_backward_kernel, ew_grid(ctx, n), 256, 0, g, d.activation == GN_ACT_RELU ? l.out.p : l.z.p, dzb, n, d.activation, act_alpha_of(d.activation, d.reserved));
           dz = dzb;
         }
-        GN_TRY(colsum(m, dz, d.out_size, B, d.out_size, gr + wn, false));
-        GN_TRY(gemm_tn(ctx, B, d.out_size, d.in_size, dz, d.out_size, xin, d.in_size, gr));
+        GN_TRY(weight_bias_grads(m, ctx, B, d.out_size, d.in_size, dz, d.out_size, xin, d.in_size, gr, gr + wn));
         if (need_dx) { GN_TRY(gemm_nn(ctx, B, d.out_size, d.in_size, dz, d.out_size, W, dx, d.in_size)); g = dx; flip ^= 1; }
         break; }
       case GN_LAYER_CONV2D: {
