@@ -313,6 +313,113 @@ __global__ void __launch_bounds__(AT_THREADS) attn_bwd_dkv_kernel(const float* _
   }
 }
 
+// ---------------------------------------------------------------- a few query rows
+// Attention of TE = 1 or 2 query rows per sequence (token 0, and the last token) against all T keys, any head size: what the
+// top block below a CLSPooling needs (plan_token_rows in model.cu).  Q and O are [B * TE, D], K and V [B * T, D].  One block per
+// (head, sequence); a thread forms the scores of its keys (16-byte loads along a key's row where they are aligned: `vec`), then
+// the threads split into groups of hd columns for the weighted sum.  Bound by reading K and V once.
+constexpr int AR_THREADS = 256;
+__device__ __forceinline__ float ar_dot(const float* __restrict__ q, const float* __restrict__ k, int hd, bool vec) {
+  float s = 0.f;
+  if (vec) {
+#pragma unroll 4
+    for (int d = 0; d < hd; d += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(k + d);
+      s = fmaf(q[d], x.x, s); s = fmaf(q[d + 1], x.y, s); s = fmaf(q[d + 2], x.z, s); s = fmaf(q[d + 3], x.w, s);
+    }
+  } else for (int d = 0; d < hd; d++) s = fmaf(q[d], k[d], s);
+  return s;
+}
+// out[d] = sum_j w[j] X[j * D + d], d < hd, in a fixed order; `part`: AR_THREADS floats
+__device__ __forceinline__ void ar_weighted(const float* __restrict__ w, const float* __restrict__ X, int n, int D, int hd, float* part, float* out) {
+  for (int d0 = 0; d0 < hd; d0 += AR_THREADS) {
+    const int cols = min(hd - d0, AR_THREADS), groups = AR_THREADS / cols, g = threadIdx.x / cols, d = threadIdx.x - g * cols;
+    float s = 0.f;
+    if (g < groups) {
+      const float* x = X + d0 + d;
+#pragma unroll 8
+      for (int j = g; j < n; j += groups) s = fmaf(w[j], x[(long)j * D], s);
+    }
+    __syncthreads();
+    part[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < cols) { float a = 0.f; for (int q = 0; q < groups; q++) a += part[q * cols + threadIdx.x]; out[d0 + threadIdx.x] = a; }
+  }
+}
+__global__ void __launch_bounds__(AR_THREADS) attn_rows_fwd_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V, float* __restrict__ O,
+                                                                   int T, int TE, int D, int hd, int causal, float inv_scale, int vec) {
+  extern __shared__ float sm[];
+  __shared__ float red[33], part[AR_THREADS];
+  float* q = sm; float* p = sm + hd;                        // one query at a time: its row, its T scores
+  const int h = blockIdx.x; const long b = blockIdx.y; const float* Kh = K + b * T * D + (long)h * hd; const float* Vh = V + b * T * D + (long)h * hd;
+  for (int e = 0; e < TE; e++) {
+    const int n = causal && e == 0 ? 1 : T;                 // keys that token 0 / the last token sees
+    const long row = (b * TE + e) * D + (long)h * hd;
+    __syncthreads();
+    for (int d = threadIdx.x; d < hd; d += AR_THREADS) q[d] = Q[row + d];
+    __syncthreads();
+    float mx = -INFINITY;
+    for (int j = threadIdx.x; j < n; j += AR_THREADS) { const float s = ar_dot(q, Kh + (long)j * D, hd, vec) * inv_scale; p[j] = s; mx = fmaxf(mx, s); }
+    mx = block_max(mx, red);
+    float l = 0.f;
+    for (int j = threadIdx.x; j < n; j += AR_THREADS) { const float v = expf(p[j] - mx); p[j] = v; l += v; }
+    l = block_sum(l, red);
+    const float il = 1.f / l;
+    for (int j = threadIdx.x; j < n; j += AR_THREADS) p[j] *= il;
+    __syncthreads();
+    ar_weighted(p, Vh, n, D, hd, part, O + row);
+  }
+}
+// Backward of query token 0 without a mask (transformer.go:589-657 for one query): dq [B, D]; dk, dv [B * T, D]; and the sums of
+// dk and dv over the tokens, [B, D].  q rows are `ldq` floats apart per sequence; probabilities are recomputed.
+__global__ void __launch_bounds__(AR_THREADS) attn_rows_bwd_kernel(const float* __restrict__ Q, long ldq, const float* __restrict__ K, const float* __restrict__ V,
+                                                                   const float* __restrict__ dO, float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV,
+                                                                   float* __restrict__ dKsum, float* __restrict__ dVsum, int T, int D, int hd, float inv_scale, int vec) {
+  extern __shared__ float sm[];
+  __shared__ float red[33], part[AR_THREADS];
+  float* q = sm; float* g = q + hd; float* p = g + hd; float* ds = p + T;
+  const int h = blockIdx.x; const long b = blockIdx.y, base = b * T * D + (long)h * hd, row = b * D + (long)h * hd;
+  for (int d = threadIdx.x; d < hd; d += AR_THREADS) { q[d] = Q[b * ldq + (long)h * hd + d]; g[d] = dO[row + d]; }
+  __syncthreads();
+  float mx = -INFINITY;
+  for (int j = threadIdx.x; j < T; j += AR_THREADS) {
+    const float s = ar_dot(q, K + base + (long)j * D, hd, vec) * inv_scale;
+    p[j] = s; mx = fmaxf(mx, s); ds[j] = ar_dot(g, V + base + (long)j * D, hd, vec);
+  }
+  mx = block_max(mx, red);
+  float l = 0.f;
+  for (int j = threadIdx.x; j < T; j += AR_THREADS) { const float v = expf(p[j] - mx); p[j] = v; l += v; }
+  l = block_sum(l, red);
+  const float il = 1.f / l;
+  float dd = 0.f, ps = 0.f;
+  for (int j = threadIdx.x; j < T; j += AR_THREADS) { const float v = p[j] * il; p[j] = v; ps += v; dd = fmaf(v, ds[j], dd); }
+  dd = block_sum(dd, red); ps = block_sum(ps, red);
+  float ss = 0.f;
+  for (int j = threadIdx.x; j < T; j += AR_THREADS) { const float v = p[j] * (ds[j] - dd) * inv_scale; ds[j] = v; ss += v; }
+  ss = block_sum(ss, red);
+  for (int d = threadIdx.x; d < hd; d += AR_THREADS) { dKsum[row + d] = ss * q[d]; dVsum[row + d] = ps * g[d]; }
+  for (int e = threadIdx.x; e < T * hd; e += AR_THREADS) {
+    const int j = e / hd, d = e - j * hd; const long o = base + (long)j * D + d;
+    dK[o] = ds[j] * q[d]; dV[o] = p[j] * g[d];
+  }
+  ar_weighted(ds, K + base, T, D, hd, part, dQ + row);
+}
+constexpr int AR_MAX_T = 16384;                             // scores of a row (twice, in the backward kernel) live in shared memory
+inline bool ar_vec(const float* a, const float* b, int D, int hd) { return D % 4 == 0 && hd % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0; }
+inline int attn_rows_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, int B, int T, int TE, int D, int H, int causal) {
+  const int hd = D / H; const size_t smem = ((size_t)hd + T) * sizeof(float);
+  if (smem > 40 * 1024) GN_CUDA(cudaFuncSetAttribute(attn_rows_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GN_LAUNCH(ctx, attn_rows_fwd_kernel, dim3(H, B), AR_THREADS, smem, Q, K, V, O, T, TE, D, hd, causal, 1.f / sqrtf((float)hd), ar_vec(K, K, D, hd) ? 1 : 0);
+  return check_launch("attn_rows_fwd");
+}
+inline int attn_rows_bwd(Ctx* ctx, const float* Q, long ldq, const float* K, const float* V, const float* dO, float* dQ, float* dK, float* dV, float* dKsum, float* dVsum,
+                         int B, int T, int D, int H) {
+  const int hd = D / H; const size_t smem = ((size_t)2 * hd + 2 * T) * sizeof(float);
+  if (smem > 40 * 1024) GN_CUDA(cudaFuncSetAttribute(attn_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GN_LAUNCH(ctx, attn_rows_bwd_kernel, dim3(H, B), AR_THREADS, smem, Q, ldq, K, V, dO, dQ, dK, dV, dKsum, dVsum, T, D, hd, 1.f / sqrtf((float)hd), ar_vec(K, V, D, hd) ? 1 : 0);
+  return check_launch("attn_rows_bwd");
+}
+
 // ---------------------------------------------------------------- launchers
 inline bool attn_fused_supported(int hd, int D) { return (hd == 16 || hd == 32 || hd == 64) && D % 4 == 0; }
 

@@ -93,6 +93,10 @@ struct LayerRT {
   DevBuf idx;                          // int32 payload: MaxPool argmax / embedding token ids
   const float* fin = nullptr;          // input of the last forward call (device pointer, not owned)
   int64_t s_off = 0, s_cnt = 0;        // BatchNorm2D: slice of the model's state buffer (running mean | running variance)
+  // Tokens that the layers above read (TransformerBlock, Embedding; see plan_token_rows): 0 = all of a sequence's tokens, 1 = token 0,
+  // 2 = token 0 and the last one.  `out` (and everything behind a block's attention) then holds that many rows per sequence.
+  int out_rows = 0;
+  bool in_row0 = false, row0_grad = false;   // block input is token 0 only; the gradient of the output is nonzero at token 0 only
   bool grad_replicated = false;        // multi-GPU: every rank already holds the gradient of the whole global batch (no all-reduce)
   float bn_eps = 1e-5f, bn_mom = 0.1f;
 };
@@ -128,7 +132,7 @@ struct gn_model {
 
 namespace gn {
 
-enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_COUNT };
+enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_COUNT };
 
 static int ensure(gn_model* m, int slot, size_t n, float** out) {
   if ((int)m->scratch.size() < S_COUNT) m->scratch.resize(S_COUNT);
@@ -446,11 +450,132 @@ static BlockParams block_params(const float* p, int D, int F, bool rms = false, 
   b.w2 = p; b.b2 = p + (long)F * D; return b;
 }
 
+// Which tokens of a TransformerBlock's output are read at all.  CLSPooling passes on token 0 and nothing else
+// (transformer.go:1684), and the gradient it returns is zero at every other token (:1715-1724).  So, of the block below it:
+//   * inference needs token 0 only; training also the last token, whose activations are the input side of the inner Dense
+//     layers' weight gradients (layer.go:496-497) -- the queries, the output projection, the norms and the feed-forward
+//     part run on those one or two rows per sequence, keys and values on all tokens;
+//   * with a causal mask token 0 sees key 0 alone: its attention output is its own value row.  In inference the blocks
+//     further down are then only needed at token 0 as well, and in training the gradient stays at token 0 through all of
+//     them (the softmax over one score is the constant 1: no gradient reaches the queries and keys).
+// The values of the rows that are computed, and every gradient, are those of the computation over all tokens: what is left
+// out there are rows that nothing reads and products with rows of zeros.
+static void plan_token_rows(gn_model* m, bool training) {
+  for (auto& l : m->L) { l.out_rows = 0; l.in_row0 = l.row0_grad = false; }
+  for (int li = (int)m->L.size() - 1; li > 0; li--) {
+    if (m->L[li].d.kind != GN_LAYER_CLS_POOLING) continue;
+    const int T = m->L[li].d.seq_len, D = m->L[li].d.dim; bool top = T <= AR_MAX_T;
+    if (!top) continue;
+    for (int k = li - 1; k >= 0 && m->L[k].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[k].d.dim == D && m->L[k].d.seq_len == T; k--) {
+      LayerRT& b = m->L[k];
+      b.row0_grad = training;
+      if (top || !training) b.out_rows = training && T > 1 ? 2 : 1;
+      top = false;
+      if (!b.d.causal) break;
+      b.in_row0 = !training && T > 1;
+    }
+  }
+}
+// Rows per sequence that the layer after `li` wants of an embedding's output: 1 (token 0) or 0 (all).
+static int next_rows(const gn_model* m, size_t li, int T, int D) {
+  if (li + 1 >= m->L.size()) return 0;
+  const LayerRT& n = m->L[li + 1];
+  return n.d.kind == GN_LAYER_TRANSFORMER_BLOCK && n.in_row0 && n.d.seq_len == T && n.d.dim == D ? 1 : 0;
+}
+
+// One TransformerBlock forward.  `TE` rows per sequence go through everything behind the keys and values: all T, or the one
+// or two that the layers above read (plan_token_rows).  The backward pass finds the same number in l.out_rows.
+static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool training, const float** out) {
+  Ctx* ctx = &m->ctx->c; LayerRT& l = m->L[li]; const gn_layer_desc& d = l.d; const float* p = m->params.p + l.p_off;
+  const int T = d.seq_len, D = d.dim, F = d.ff_dim, hd = D / d.heads, N = B * T; const BlockParams bp = block_params(p, D, F, l.rms, l.ff_act);
+  const int TE = l.out_rows ? l.out_rows : T, NE = B * TE; const bool rows_only = l.out_rows != 0;
+  // the block's input rows of the TE tokens: in place, strided (token 0 of every sequence) or gathered (tokens 0 and T - 1)
+  const float* xe = cur; long ldx = D;
+  const bool in_compact = li > 0 && m->L[li - 1].out_rows == 1;
+  if (rows_only && !in_compact && T > 1) {
+    if (TE == 1) ldx = (long)T * D;
+    else { GN_TRY(ensure(m, S_XROWS, (size_t)NE * D, const_cast<float**>(&xe))); GN_LAUNCH(ctx, gather_ends_kernel, NE, 128, 0, cur, const_cast<float*>(xe), T, D); }
+  }
+  if (l.in_row0) {
+    // causal, token 0 only: it attends to itself alone, so its attention output is its value row
+    GN_TRY(gemm_nt(ctx, B, D, D, xe, ldx, bp.wv, bp.bv, l.att.p, D));
+  } else {
+    // the Q, K and V projections read the same input: its operand planes come from the LayerNorm that produced it
+    // (the previous block's), or are still in the engine's scratch after the first of the three
+    GemmDesc g; g.M = N; g.N = D; g.K = D; g.A = cur; g.sa_m = D; g.sa_k = 1; g.sb_k = 1; g.sb_n = D; g.ldc = D;
+    if (m->fwd_planes_src == cur && m->fwd_planes.rows == N && m->fwd_planes.K == D) g.a_planes = &m->fwd_planes;
+    if (!rows_only) { g.B = bp.wq; g.bias = bp.bq; g.C = l.q.p; GN_TRY(gemm(ctx, g)); g.reuse_a_planes = true; }
+    g.B = bp.wk; g.bias = bp.bk; g.C = l.k.p; GN_TRY(gemm(ctx, g));
+    g.reuse_a_planes = true;
+    g.B = bp.wv; g.bias = bp.bv; g.C = l.v.p; GN_TRY(gemm(ctx, g));
+    if (rows_only) GN_TRY(gemm_nt(ctx, NE, D, D, xe, ldx, bp.wq, bp.bq, l.q.p, D));
+    if (l.use_rope) {   // rotary embeddings on q and k, in place: attention and its backward pass see the rotated tensors (transformer.go:457-461)
+      GN_TRY(rope_table(ctx, l));
+      const long tot = (long)N * (D / 2), tq = (long)NE * (D / 2);
+      GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tq), 256, 0, l.q.p, (const float*)l.rope.p, (long)NE, TE, D, hd, 1.f, rows_only ? T - 1 : 1);
+      GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, l.k.p, (const float*)l.rope.p, (long)N, T, D, hd, 1.f, 1);
+    }
+    if (rows_only) GN_TRY(attn_rows_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, B, T, TE, D, d.heads, d.causal));
+    else if (use_fused_attention(d)) {
+      // planes of Q, K and V are kept for a backward pass that walks all queries
+      if (attn_tc_supported(ctx, hd, T, B, d.heads, D)) GN_TRY(attn_tc_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal, training && !l.row0_grad ? &l.attn_saved : nullptr));
+      else GN_TRY(attn_fwd(ctx, hd, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal));
+    } else {
+      float* P; GN_TRY(ensure(m, S_ATT0, (size_t)B * d.heads * T * T, &P));
+      GN_TRY(attention_forward(m, l, B, P));
+    }
+  }
+  m->fwd_planes_src = nullptr;
+  GN_TRY(gemm_nt(ctx, NE, D, D, l.att.p, D, bp.wo, bp.bo, l.r1.p, D, GN_ACT_LINEAR, xe, ldx));          // res1 = x + att
+  float* st = l.stat.p;
+  // norm 1 hands its output to ff1 as operand planes (and the row norms ff1's plane-writing epilogue needs)
+  RowPlaneOut po1{}; BfPlanes n1p{}; bool n1_planes = false; float* rn1 = nullptr;
+  if (norm_planes_wanted(ctx, l.rms, NE, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)NE, &rn1)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, NE, D, &po1, &n1p, rn1)); }
+  GN_TRY(block_norm_forward(ctx, l.rms, l.r1.p, bp.g1, bp.be1, l.n1.p, st, (long)NE, D, po1.p0 ? &po1 : nullptr, &n1_planes));
+  {   // feed-forward: ff1 -> ff2, res2 = norm1 + ff
+    GemmDesc g1; g1.M = NE; g1.N = F; g1.K = D; g1.A = l.n1.p; g1.sa_m = D; g1.sa_k = 1; g1.B = bp.w1; g1.sb_k = 1; g1.sb_n = D; g1.C = l.mid.p; g1.ldc = F; g1.bias = bp.b1;
+    if (n1_planes) g1.a_planes = &n1p;
+    const long nf = (long)NE * F;
+    BfPlanes midp{reinterpret_cast<__half*>(l.mid.p), l.mid_inv.p, NE, F, F, 1};
+    l.mid_is_planes = ffn_planes_possible(ctx, l, NE, bp.w1, bp.w2);
+    if (l.mid_is_planes) {
+      // the hidden activation is only ever the A operand of ff2 (and, for its last-token rows, a gate and a weight-gradient
+      // input): the epilogue writes it as operand planes into the same buffer, no fp32 copy and no split pass
+      const WeightPlaneEntry* we = nullptr; wplanes_lookup(ctx, g1, &we);
+      float* rn; GN_TRY(ensure(m, S_RN, (size_t)NE, &rn));
+      TcPlaneOut po{midp, we->maxabs, l.mid_last.p, TE};
+      g1.act = GN_ACT_RELU; g1.C = nullptr; g1.plane_out = &po; g1.a_rownorm = rn; GN_TRY(gemm(ctx, g1));
+    } else if (l.ff_act == GN_ACT_RELU) { g1.act = GN_ACT_RELU; GN_TRY(gemm(ctx, g1)); }
+    else if (l.ff_act == GN_ACT_GELU) {
+      // the pre-activation of every sequence's last token is what the backward pass differentiates at (layer.go:563-567)
+      GN_TRY(gemm(ctx, g1));
+      if (training) GN_LAUNCH(ctx, last_token_rows_kernel, ew_grid(ctx, (long)B * F), 256, 0, (const float*)l.mid.p, l.zlast.p, TE, F, (long)B * F);
+      GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.mid.p, l.mid.p, nf, (int)GN_ACT_GELU, 0.f);
+    } else {              // SwiGLU: gate and up projections (no biases) share the input's operand planes
+      g1.C = l.gate.p; g1.bias = nullptr; GN_TRY(gemm(ctx, g1));
+      g1.B = bp.v1; g1.C = l.up.p; g1.reuse_a_planes = true; GN_TRY(gemm(ctx, g1));
+      GN_LAUNCH(ctx, swiglu_fwd_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.gate.p, (const float*)l.up.p, l.mid.p, nf);
+    }
+    GemmDesc g2; g2.M = NE; g2.N = D; g2.K = F; g2.A = l.mid.p; g2.sa_m = F; g2.sa_k = 1; g2.B = bp.w2; g2.sb_k = 1; g2.sb_n = F; g2.C = l.r2.p; g2.ldc = D; g2.bias = bp.b2; g2.R = l.n1.p; g2.ldr = D;
+    if (l.mid_is_planes) g2.a_planes = &midp;
+    GN_TRY(gemm(ctx, g2));
+  }
+  {   // norm 2 hands its output to the next block's projections as operand planes
+    RowPlaneOut po2{}; BfPlanes outp{}; bool emitted = false;
+    const bool next_is_block = !rows_only && li + 1 < m->L.size() && m->L[li + 1].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[li + 1].d.dim == D && m->L[li + 1].d.seq_len == T;
+    if (next_is_block && norm_planes_wanted(ctx, l.rms, NE, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP1, S_LNI1, NE, D, &po2, &outp, nullptr));
+    GN_TRY(block_norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * NE, (long)NE, D, po2.p0 ? &po2 : nullptr, &emitted));
+    if (emitted) { m->fwd_planes = outp; m->fwd_planes_src = l.out.p; }
+  }
+  *out = l.out.p; return GN_OK;
+}
+
 static int forward(gn_model* m, const float* x, int B, const float** y_out, bool training) {
   Ctx* ctx = &m->ctx->c;
   GN_TRY(wplanes_refresh(ctx, m->wplanes));          // no-op unless the parameters changed since the last pass
   ctx->weight_planes = &m->wplanes;
   m->fwd_planes_src = nullptr;
+  plan_token_rows(m, training);
   const float* cur = x;
   for (size_t li = 0; li < m->L.size(); li++) {
     LayerRT& l = m->L[li]; const gn_layer_desc& d = l.d; const float* p = m->params.p + l.p_off;
@@ -529,82 +654,17 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
         bool fuse = li + 1 < m->L.size() && m->L[li + 1].d.kind == GN_LAYER_POSENC && m->L[li + 1].d.dim == d.out_size;
         if (fuse) P = m->params.p + m->L[li + 1].p_off;
         float* dst = fuse ? m->L[li + 1].out.p : l.out.p;
-        GN_LAUNCH(ctx, embedding_fwd_kernel, (unsigned)tokens, 128, 0, cur, p, P, dst, tokens, d.seq_len, d.out_size, d.in_size, (int*)l.idx.p, ctx->d_status);
-        cur = dst; if (fuse) li++; break; }
+        l.out_rows = next_rows(m, fuse ? li + 1 : li, d.seq_len, d.out_size);
+        GN_LAUNCH(ctx, embedding_fwd_kernel, (unsigned)tokens, 128, 0, cur, p, P, dst, tokens, d.seq_len, d.out_size, d.in_size, (int*)l.idx.p, ctx->d_status, l.out_rows);
+        cur = dst; if (fuse) { m->L[li + 1].out_rows = l.out_rows; li++; } break; }
       case GN_LAYER_POSENC: {
-        long n = (long)B * l.out_size;
+        long n = (long)B * l.out_size; l.out_rows = 0;
         GN_LAUNCH(ctx, posenc_fwd_kernel, ew_grid(ctx, n), 256, 0, cur, p, l.out.p, n, (long)l.out_size);
         cur = l.out.p; break; }
-      case GN_LAYER_TRANSFORMER_BLOCK: {
-        const int T = d.seq_len, D = d.dim, F = d.ff_dim; const int N = B * T; BlockParams bp = block_params(p, D, F, l.rms, l.ff_act);
-        {   // the Q, K and V projections read the same input: its operand planes come from the LayerNorm that produced it
-            // (the previous block's), or are still in the engine's scratch after the first of the three
-          GemmDesc g; g.M = N; g.N = D; g.K = D; g.A = cur; g.sa_m = D; g.sa_k = 1; g.sb_k = 1; g.sb_n = D; g.ldc = D;
-          const bool have = m->fwd_planes_src == cur && m->fwd_planes.rows == N && m->fwd_planes.K == D;
-          if (have) g.a_planes = &m->fwd_planes;
-          g.B = bp.wq; g.bias = bp.bq; g.C = l.q.p; GN_TRY(gemm(ctx, g));
-          g.reuse_a_planes = true;
-          g.B = bp.wk; g.bias = bp.bk; g.C = l.k.p; GN_TRY(gemm(ctx, g));
-          g.B = bp.wv; g.bias = bp.bv; g.C = l.v.p; GN_TRY(gemm(ctx, g));
-          m->fwd_planes_src = nullptr;
-        }
-        if (l.use_rope) {   // rotary embeddings on q and k, in place: attention and its backward pass see the rotated tensors (transformer.go:457-461)
-          GN_TRY(rope_table(ctx, l));
-          const long tot = (long)N * (D / 2);
-          GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, l.q.p, (const float*)l.rope.p, (long)N, T, D, D / d.heads, 1.f);
-          GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, l.k.p, (const float*)l.rope.p, (long)N, T, D, D / d.heads, 1.f);
-        }
-        if (use_fused_attention(d)) {
-          if (attn_tc_supported(ctx, D / d.heads, T, B, d.heads, D)) GN_TRY(attn_tc_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal, training ? &l.attn_saved : nullptr));
-          else GN_TRY(attn_fwd(ctx, D / d.heads, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal));
-        } else {
-          float* P; GN_TRY(ensure(m, S_ATT0, (size_t)B * d.heads * T * T, &P));
-          GN_TRY(attention_forward(m, l, B, P));
-        }
-        GN_TRY(gemm_nt(ctx, N, D, D, l.att.p, D, bp.wo, bp.bo, l.r1.p, D, GN_ACT_LINEAR, cur, D));          // res1 = x + att
-        float* st = l.stat.p;
-        // norm 1 hands its output to ff1 as operand planes (and the row norms ff1's plane-writing epilogue needs)
-        RowPlaneOut po1{}; BfPlanes n1p{}; bool n1_planes = false; float* rn1 = nullptr;
-        if (norm_planes_wanted(ctx, l.rms, N, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)N, &rn1)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &po1, &n1p, rn1)); }
-        GN_TRY(block_norm_forward(ctx, l.rms, l.r1.p, bp.g1, bp.be1, l.n1.p, st, (long)N, D, po1.p0 ? &po1 : nullptr, &n1_planes));
-        {   // feed-forward: ff1 -> ff2, res2 = norm1 + ff
-          GemmDesc g1; g1.M = N; g1.N = F; g1.K = D; g1.A = l.n1.p; g1.sa_m = D; g1.sa_k = 1; g1.B = bp.w1; g1.sb_k = 1; g1.sb_n = D; g1.C = l.mid.p; g1.ldc = F; g1.bias = bp.b1;
-          if (n1_planes) g1.a_planes = &n1p;
-          const long nf = (long)N * F;
-          BfPlanes midp{reinterpret_cast<__half*>(l.mid.p), l.mid_inv.p, N, F, F, 1};
-          l.mid_is_planes = ffn_planes_possible(ctx, l, N, bp.w1, bp.w2);
-          if (l.mid_is_planes) {
-            // the hidden activation is only ever the A operand of ff2 (and, for its last-token rows, a gate and a weight-gradient
-            // input): the epilogue writes it as operand planes into the same buffer, no fp32 copy and no split pass
-            const WeightPlaneEntry* we = nullptr; wplanes_lookup(ctx, g1, &we);
-            float* rn; GN_TRY(ensure(m, S_RN, (size_t)N, &rn));
-            TcPlaneOut po{midp, we->maxabs, l.mid_last.p, T};
-            g1.act = GN_ACT_RELU; g1.C = nullptr; g1.plane_out = &po; g1.a_rownorm = rn; GN_TRY(gemm(ctx, g1));
-          } else if (l.ff_act == GN_ACT_RELU) { g1.act = GN_ACT_RELU; GN_TRY(gemm(ctx, g1)); }
-          else if (l.ff_act == GN_ACT_GELU) {
-            // the pre-activation of every sequence's last token is what the backward pass differentiates at (layer.go:563-567)
-            GN_TRY(gemm(ctx, g1));
-            GN_LAUNCH(ctx, last_token_rows_kernel, ew_grid(ctx, (long)B * F), 256, 0, (const float*)l.mid.p, l.zlast.p, T, F, (long)B * F);
-            GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.mid.p, l.mid.p, nf, (int)GN_ACT_GELU, 0.f);
-          } else {              // SwiGLU: gate and up projections (no biases) share the input's operand planes
-            g1.C = l.gate.p; g1.bias = nullptr; GN_TRY(gemm(ctx, g1));
-            g1.B = bp.v1; g1.C = l.up.p; g1.reuse_a_planes = true; GN_TRY(gemm(ctx, g1));
-            GN_LAUNCH(ctx, swiglu_fwd_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.gate.p, (const float*)l.up.p, l.mid.p, nf);
-          }
-          GemmDesc g2; g2.M = N; g2.N = D; g2.K = F; g2.A = l.mid.p; g2.sa_m = F; g2.sa_k = 1; g2.B = bp.w2; g2.sb_k = 1; g2.sb_n = F; g2.C = l.r2.p; g2.ldc = D; g2.bias = bp.b2; g2.R = l.n1.p; g2.ldr = D;
-          if (l.mid_is_planes) g2.a_planes = &midp;
-          GN_TRY(gemm(ctx, g2));
-        }
-        {   // norm 2 hands its output to the next block's projections as operand planes
-          RowPlaneOut po2{}; BfPlanes outp{}; bool emitted = false;
-          const bool next_is_block = li + 1 < m->L.size() && m->L[li + 1].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[li + 1].d.dim == D && m->L[li + 1].d.seq_len == T;
-          if (next_is_block && norm_planes_wanted(ctx, l.rms, N, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP1, S_LNI1, N, D, &po2, &outp, nullptr));
-          GN_TRY(block_norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * N, (long)N, D, po2.p0 ? &po2 : nullptr, &emitted));
-          if (emitted) { m->fwd_planes = outp; m->fwd_planes_src = l.out.p; }
-        }
-        cur = l.out.p; break; }
-      case GN_LAYER_CLS_POOLING:
-        GN_LAUNCH(ctx, cls_fwd_kernel, B, 128, 0, cur, l.out.p, d.seq_len, d.dim); cur = l.out.p; break;
+      case GN_LAYER_TRANSFORMER_BLOCK: GN_TRY(block_forward(m, li, B, cur, training, &cur)); break;
+      case GN_LAYER_CLS_POOLING: {
+        const int rows = li > 0 && m->L[li - 1].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[li - 1].out_rows ? m->L[li - 1].out_rows : d.seq_len;
+        GN_LAUNCH(ctx, cls_fwd_kernel, B, 128, 0, cur, l.out.p, rows, d.dim); cur = l.out.p; break; }
       case GN_LAYER_BATCHNORM2D: {
         const int C = d.in_size, S = d.in_h * d.in_w; const long BC = (long)B * C; float* run = m->state.p + l.s_off;
         if (training) {
@@ -787,8 +847,8 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   }
   if (l.use_rope) {   // the conjugate rotation on the gradients of q and k (transformer.go:659-663)
     const long tot = (long)N * (D / 2);
-    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, dQ, (const float*)l.rope.p, (long)N, T, D, hd, -1.f);
-    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, dK, (const float*)l.rope.p, (long)N, T, D, hd, -1.f);
+    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, dQ, (const float*)l.rope.p, (long)N, T, D, hd, -1.f, 1);
+    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, dK, (const float*)l.rope.p, (long)N, T, D, hd, -1.f, 1);
   }
   // q, k, v projections; gradIn = dq + dk + dv, block input gradient = gradRes1 + gradIn
   GN_TRY(inner_dense_param_grads(m, dQ, B, T, D, xin, D, (float*)gp.wq, (float*)gp.bq));
@@ -798,6 +858,66 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   GN_TRY(gemm_nn(ctx, N, D, D, dK, D, bp.wk, dx, D, dx, D));
   GN_TRY(gemm_nn(ctx, N, D, D, dV, D, bp.wv, dx, D, dx, D));
   return check_launch("block_backward");
+}
+
+// Backward pass of a block whose output gradient is zero except at token 0 (plan_token_rows): gout is [B, D], and so is everything
+// up to the attention.  The inner layers' other factor is the last token's activation, as always.  dx: [B, D] for a causal
+// block (*dx_row0 = true), else [B * T, D].
+static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin, const float* gout, float* dx, bool* dx_row0) {
+  Ctx* ctx = &m->ctx->c; const gn_layer_desc& d = l.d;
+  const int T = d.seq_len, D = d.dim, F = d.ff_dim, TE = l.out_rows ? l.out_rows : T; const long ND = (long)B * T * D, BD = (long)B * D, BF = (long)B * F;
+  const BlockParams bp = block_params(m->params.p + l.p_off, D, F, l.rms, l.ff_act); const BlockParams gp = block_params(m->grads.p + l.p_off, D, F, l.rms, l.ff_act);
+  const long ldD = (long)TE * D, ldF = (long)TE * F, NE = (long)B * TE; const float* st = l.stat.p;
+  const float* n1_last = l.n1.p + (long)(TE - 1) * D; const float* att_last = l.att.p + (long)(TE - 1) * D; const float* x_last = xin + (long)(T - 1) * D;
+  const float* mid_last = l.mid_is_planes ? l.mid_last.p : l.mid.p + (long)(TE - 1) * F; const long ld_mid = l.mid_is_planes ? F : ldF;
+  float *dR2, *dR1, *comb, *dA, *dM;
+  GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, d.causal ? BD : ND, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
+  auto norm = [&](const float* g, const float* x, const float* gamma, const float* stat, float* out, float* gG, float* gB) -> int {
+    GN_LAUNCH(ctx, norm_bwd_rows_kernel, cdiv(B, 4), 128, 0, g, x, ldD, gamma, stat, l.rms ? nullptr : stat + NE, (long)TE, out, B, D);
+    GN_LAUNCH(ctx, norm_pgrad_rows_kernel, cdiv(D, 32), 256, 0, g, x, ldD, stat, l.rms ? nullptr : stat + NE, (long)TE, B, D, gG, gB);
+    return check_launch("norm_rows");
+  };
+  GN_TRY(norm(gout, l.r2.p, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, F, dR2, D, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
+  GemmDesc g; g.M = B; g.N = F; g.K = D; g.A = dR2; g.sa_m = D; g.sa_k = 1; g.B = bp.w2; g.sb_k = F; g.sb_n = 1; g.C = dM; g.ldc = F;
+  if (l.ff_act == GN_ACT_RELU) { g.mask = mid_last; g.mask_ld = ld_mid; }
+  GN_TRY(gemm(ctx, g));
+  if (l.ff_act == GN_ACT_SILU) {
+    float *dG, *dU; GN_TRY(ensure(m, S_NFF2, BF, &dG)); GN_TRY(ensure(m, S_NFF3, BF, &dU));
+    GN_LAUNCH(ctx, swiglu_bwd_rows_kernel, ew_grid(ctx, BF), 256, 0, (const float*)dM, (const float*)(l.gate.p + (long)(TE - 1) * F), (const float*)(l.up.p + (long)(TE - 1) * F), ldF, dG, dU, F, BF);
+    GN_TRY(gemm_tn(ctx, B, F, D, dG, F, n1_last, ldD, (float*)gp.w1));
+    GN_TRY(gemm_tn(ctx, B, F, D, dU, F, n1_last, ldD, (float*)gp.v1));
+    GN_TRY(gemm_nn(ctx, B, F, D, dG, F, bp.w1, comb, D, dR2, D));
+    GN_TRY(gemm_nn(ctx, B, F, D, dU, F, bp.v1, comb, D, comb, D));
+  } else {
+    if (l.ff_act == GN_ACT_GELU) GN_LAUNCH(ctx, scale_by_last_deriv_kernel, ew_grid(ctx, BF), 256, 0, dM, (const float*)l.zlast.p, 1, F, BF, (int)GN_ACT_GELU);
+    GN_TRY(weight_bias_grads(m, ctx, B, F, D, dM, F, n1_last, ldD, (float*)gp.w1, (float*)gp.b1));
+    GN_TRY(gemm_nn(ctx, B, F, D, dM, F, bp.w1, comb, D, dR2, D));
+  }
+  GN_TRY(norm(comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, dR1, D, att_last, ldD, (float*)gp.wo, (float*)gp.bo));
+  GN_TRY(gemm_nn(ctx, B, D, D, dR1, D, bp.wo, dA, D));
+  if (d.causal) {
+    // the one probability of token 0 is 1: dV = dA at token 0, dQ = dK = 0 (the gradient buffer was cleared)
+    GN_TRY(weight_bias_grads(m, ctx, B, D, D, dA, D, x_last, (long)T * D, (float*)gp.wv, (float*)gp.bv));
+    GN_TRY(gemm_nn(ctx, B, D, D, dA, D, bp.wv, dx, D, dR1, D));
+    *dx_row0 = true; return check_launch("block_backward_row0");
+  }
+  float *dQ, *dK, *dV, *ks, *vs;
+  GN_TRY(ensure(m, S_XROWS, 3 * BD, &dQ)); ks = dQ + BD; vs = ks + BD; GN_TRY(ensure(m, S_ND1, ND, &dK)); GN_TRY(ensure(m, S_ND4, ND, &dV));
+  GN_TRY(attn_rows_bwd(ctx, l.q.p, ldD, l.k.p, l.v.p, dA, dQ, dK, dV, ks, vs, B, T, D, d.heads));
+  if (l.use_rope) {   // the conjugate rotation (transformer.go:659-663); token 0's angle is zero
+    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, ND / 2), 256, 0, dK, (const float*)l.rope.p, (long)B * T, T, D, D / d.heads, -1.f, 1);
+    GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(D, 128), B), dim3(128, 4), 0, (const float*)dK, T, D, ks);
+  }
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, dQ, D, x_last, (long)T * D, (float*)gp.wq, (float*)gp.bq));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, ks, D, x_last, (long)T * D, (float*)gp.wk, (float*)gp.bk));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, vs, D, x_last, (long)T * D, (float*)gp.wv, (float*)gp.bv));
+  GN_TRY(gemm_nn(ctx, B, D, D, dQ, D, bp.wq, dR1, D, dR1, D));
+  GN_TRY(gemm_nn(ctx, B * T, D, D, dK, D, bp.wk, dx, D));
+  GN_TRY(gemm_nn(ctx, B * T, D, D, dV, D, bp.wv, dx, D, dx, D));
+  GN_LAUNCH(ctx, add_row0_kernel, B, 128, 0, (const float*)dR1, dx, T, D);
+  *dx_row0 = false; return check_launch("block_backward_row0");
 }
 
 static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float* xin, const float* gout, int global_batch, int first_sample, float* dx) {
@@ -890,6 +1010,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
   // for all layers after the backward pass instead (no overlap; for measurements).
   static const bool comm_at_end = [] { const char* e = getenv("GONEURON_CUDA_COMM"); return e && !strcmp(e, "end"); }();
   std::vector<int> deferred;
+  bool row0 = false; int row0_T = 0, row0_D = 0;            // g holds the gradient of token 0 of every sequence, [B, row0_D]; the other tokens' is zero
   auto layer_comm = [&](int li) -> int {
     LayerRT& l = m->L[li]; float* gr = m->grads.p + l.p_off;
     GN_CUDA(cudaEventRecord(m->layer_ev[li], ctx->stream));
@@ -911,6 +1032,10 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
   for (int li = (int)m->L.size() - 1; li >= 0; li--) {
     LayerRT& l = m->L[li]; const gn_layer_desc& d = l.d;
     const float* xin = l.fin;
+    if (row0 && d.kind != GN_LAYER_TRANSFORMER_BLOCK && d.kind != GN_LAYER_POSENC && d.kind != GN_LAYER_EMBEDDING) {
+      const long n = (long)B * row0_T * row0_D;             // a layer that wants the gradient of every token: zeros except token 0
+      GN_LAUNCH(ctx, cls_bwd_kernel, ew_grid(ctx, n), 256, 0, g, pp[flip], row0_T, row0_D, n); g = pp[flip]; flip ^= 1; row0 = false;
+    }
     const float* p = m->params.p + l.p_off; float* gr = m->grads.p + l.p_off;
     float* dx = pp[flip]; bool need_dx = li > 0;
     switch (d.kind) {
@@ -973,7 +1098,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
       case GN_LAYER_EMBEDDING: {
         // Only the last sample of every worker chunk reaches the table (embedding.go:151-154): global samples
         // c*chunk + chunk - 1 and the very last one.
-        const int chunk = (global_batch + m->W - 1) / m->W, T = d.seq_len, dim = d.out_size;
+        const int chunk = (global_batch + m->W - 1) / m->W, T = row0 ? 1 : d.seq_len, Tid = d.seq_len, dim = d.out_size;     // T: tokens of a sample with a gradient
         const int nq = (global_batch + chunk - 1) / chunk;                       // qualifying samples of the global batch
         auto q_sample = [&](int q) { return std::min(global_batch - 1, q * chunk + chunk - 1); };
         const size_t smem = (size_t)T * sizeof(int);
@@ -987,7 +1112,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
           GN_CUDA(cudaMemsetAsync(buf, 0, (size_t)nq * T * (dim + 1) * sizeof(float), ctx->stream));
           for (int q = 0; q < nq; q++) {
             const int sl = q_sample(q) - first_sample; if (sl < 0 || sl >= B) continue;
-            GN_LAUNCH(ctx, embedding_pack_kernel, T, 128, 0, g + (size_t)sl * T * dim, (const int*)l.idx.p + (size_t)sl * T, rows + (size_t)q * T * dim, idsf + (size_t)q * T, T, dim);
+            GN_LAUNCH(ctx, embedding_pack_kernel, T, 128, 0, g + (size_t)sl * T * dim, (const int*)l.idx.p + (size_t)sl * Tid, rows + (size_t)q * T * dim, idsf + (size_t)q * T, T, dim);
           }
           GN_CUDA(cudaEventRecord(m->gather_ev, ctx->stream));
           GN_CUDA(cudaStreamWaitEvent(ctx->comm_stream, m->gather_ev, 0));
@@ -1002,17 +1127,19 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
         } else {
           for (int q = 0; q < nq; q++) {
             const int sl = q_sample(q) - first_sample; if (sl < 0 || sl >= B) continue;
-            GN_LAUNCH(ctx, embedding_bwd_sample_kernel, T, 128, smem, g + (size_t)sl * T * dim, (const int*)l.idx.p + (size_t)sl * T, gr, T, dim);
+            GN_LAUNCH(ctx, embedding_bwd_sample_kernel, T, 128, smem, g + (size_t)sl * T * dim, (const int*)l.idx.p + (size_t)sl * Tid, gr, T, dim);
           }
           l.grad_replicated = false;
         }
         break; }
       case GN_LAYER_POSENC:
-        GN_TRY(colsum(m, g, l.out_size, B, l.out_size, gr, false)); break;     // gP = sum over samples; dx = g
+        { const int n = row0 ? d.dim : l.out_size; GN_TRY(colsum(m, g, n, B, n, gr, false)); } break;     // gP = sum over samples; dx = g
       case GN_LAYER_TRANSFORMER_BLOCK:
-        GN_TRY(block_backward(m, l, B, xin, g, dx)); g = dx; flip ^= 1; break;
+        if (row0) GN_TRY(block_backward_row0(m, l, B, xin, g, dx, &row0)); else GN_TRY(block_backward(m, l, B, xin, g, dx));
+        g = dx; flip ^= 1; break;
       case GN_LAYER_CLS_POOLING: {
         long n = (long)B * l.in_size;
+        if (li > 0 && m->L[li - 1].row0_grad) { row0 = true; row0_T = d.seq_len; row0_D = d.dim; break; }
         GN_LAUNCH(ctx, cls_bwd_kernel, ew_grid(ctx, n), 256, 0, g, dx, d.seq_len, d.dim, n); g = dx; flip ^= 1; break; }
       case GN_LAYER_BATCHNORM2D: {
         const int C = d.in_size, S = d.in_h * d.in_w; const long BC = (long)B * C;

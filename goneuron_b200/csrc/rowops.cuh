@@ -409,6 +409,47 @@ __global__ void rmsnorm_pgrad_final_kernel(const float* __restrict__ part, int c
   gGamma[c] += a;
 }
 
+// Norm backward on a few rows: rows s of g and dx are dense [rows, n], row s of the norm's input lies at x + s * ldx and its
+// statistics at mean[s * lds], sd[s * lds] (LayerNorm) or mean[s * lds] = rms (sd = null: RMSNorm).  One warp per row; the
+// formulas of the kernels above.
+__global__ void __launch_bounds__(128) norm_bwd_rows_kernel(const float* __restrict__ g, const float* __restrict__ x, long ldx, const float* __restrict__ gamma,
+                                                            const float* __restrict__ mean_in, const float* __restrict__ sd_in, long lds, float* __restrict__ dx, int rows, int n) {
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31; if (row >= rows) return;
+  const float* xr = x + row * ldx; const float* gr = g + (long)row * n; float* dr = dx + (long)row * n;
+  const float c = mean_in[row * lds], fn = (float)n; float sg = 0.f, sgx = 0.f;
+  if (sd_in) {
+    const float sd = sd_in[row * lds], isd = 1.f / sd;
+    for (int i = lane; i < n; i += 32) { const float q = gr[i] * gamma[i]; sg += q; sgx += q * (xr[i] - c); }
+    sg = warp_sum(sg) / fn; const float w = warp_sum(sgx) / (fn * sd * sd);
+    for (int i = lane; i < n; i += 32) dr[i] = (gr[i] * gamma[i] - sg) * isd - (xr[i] - c) * w;
+  } else {
+    const float inv = 1.f / c;
+    for (int i = lane; i < n; i += 32) sgx += gr[i] * gamma[i] * xr[i];
+    const float f = warp_sum(sgx) / (fn * c * c);
+    for (int i = lane; i < n; i += 32) dr[i] = (gamma[i] * inv) * (gr[i] - xr[i] * f);
+  }
+}
+// ... and its parameter gradients, written (not added); block = 32 columns x 8 groups of rows, combined in a fixed order
+__global__ void __launch_bounds__(256) norm_pgrad_rows_kernel(const float* __restrict__ g, const float* __restrict__ x, long ldx, const float* __restrict__ mean_in,
+                                                              const float* __restrict__ sd_in, long lds, int rows, int n, float* __restrict__ gGamma, float* __restrict__ gBeta) {
+  __shared__ float sa[8][33], sb[8][33];
+  const int tx = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  float a = 0.f, b = 0.f;
+  if (c < n) {
+#pragma unroll 4
+    for (int r = grp; r < rows; r += 8) {
+      const float gg = g[(long)r * n + c], st = mean_in[r * lds];
+      a += sd_in ? gg * ((x[r * ldx + c] - st) / sd_in[r * lds]) : gg * (x[r * ldx + c] * (1.f / st)); b += gg;
+    }
+  }
+  sa[grp][tx] = a; sb[grp][tx] = b;
+  __syncthreads();
+  if (grp == 0 && c < n) {
+    for (int k = 1; k < 8; k++) { a += sa[k][tx]; b += sb[k][tx]; }
+    gGamma[c] = a; if (gBeta) gBeta[c] = b;
+  }
+}
+
 // ---------------------------------------------------------------- Dropout
 // The reference's generator (layer.go:61-75): s <- s * 6364136223846793005 + 1, value = float32(s >> 33) / 2^31, one
 // stream per layer seeded with 42 and consumed element by element, sample by sample (dropout.go:139-152).  Draw k of the
@@ -454,12 +495,13 @@ __global__ void dropout_advance_kernel(float* __restrict__ cnt, unsigned long lo
 // with a clamped id, so that nothing is read out of bounds.
 constexpr int GN_STATUS_BAD_TOKEN = 100;
 __global__ void embedding_fwd_kernel(const float* __restrict__ ids, const float* __restrict__ E, const float* __restrict__ P,
-                                     float* __restrict__ out, long tokens, int T, int d, int V, int* __restrict__ idx_out, int* __restrict__ status) {
+                                     float* __restrict__ out, long tokens, int T, int d, int V, int* __restrict__ idx_out, int* __restrict__ status, int row0_only) {
   long tok = blockIdx.x; if (tok >= tokens) return;
   int id = (int)floorf(ids[tok]);
   if (id < 0 || id >= V || !(ids[tok] == ids[tok])) { if (threadIdx.x == 0) atomicCAS(status, 0, GN_STATUS_BAD_TOKEN); id = id < 0 ? 0 : V - 1; }
   if (threadIdx.x == 0 && idx_out) idx_out[tok] = id;
-  const float* e = E + (long)id * d; float* o = out + tok * d;
+  if (row0_only && tok % T) return;                        // the layers above read token 0 of every sequence: out is [sequences, d]
+  const float* e = E + (long)id * d; float* o = out + (row0_only ? tok / T : tok) * d;
   if (P) { const float* p = P + (long)(tok % T) * d; for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = e[i] + p[i]; }
   else for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = e[i];
 }
@@ -501,6 +543,11 @@ __global__ void embedding_pack_kernel(const float* __restrict__ g, const int* __
 }
 __global__ void ids_to_int_kernel(const float* __restrict__ f, int* __restrict__ out, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x; if (i < n) out[i] = (int)f[i];
+}
+// out [2 B, d] <- tokens 0 and T - 1 of every sequence of x [B, T, d]; one block per row
+__global__ void gather_ends_kernel(const float* __restrict__ x, float* __restrict__ out, int T, int d) {
+  const long r = blockIdx.x; const float* src = x + ((r >> 1) * T + (r & 1) * (T - 1)) * (long)d; float* dst = out + r * d;
+  for (int i = threadIdx.x; i < d; i += blockDim.x) dst[i] = src[i];
 }
 // CLSPooling: y[s,:] = x[s,0,:]; backward: zeros except token 0   transformer.go:1684, :1715-1724
 __global__ void cls_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int T, int d) {
@@ -556,10 +603,11 @@ __global__ void relu_mask_last_token_kernel(float* __restrict__ dM, const float*
 // Rotary embeddings on a [tokens, D] tensor in place (transformer.go:212-236): within every head, element i of the first
 // half and element i + hd/2 are rotated by the angle of (position, i); `tab` holds cos | sin per (position, i), computed on
 // the host with the reference's float32 / float64 conversions.  sign = -1 applies the conjugate (backward pass).
-__global__ void rope_kernel(float* __restrict__ x, const float* __restrict__ tab, long tokens, int T, int D, int hd, float sign) {
+// Row r of a sequence's T rows is its token r * tstep.
+__global__ void rope_kernel(float* __restrict__ x, const float* __restrict__ tab, long tokens, int T, int D, int hd, float sign, int tstep) {
   const int half = hd >> 1; const long per = (long)(D >> 1), total = tokens * per;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-    const long tok = e / per; const int r = (int)(e - tok * per), h = r / half, i = r - h * half, t = (int)(tok % T);
+    const long tok = e / per; const int r = (int)(e - tok * per), h = r / half, i = r - h * half, t = (int)(tok % T) * tstep;
     const float c = tab[((long)t * half + i) * 2], s = sign * tab[((long)t * half + i) * 2 + 1];
     float* p = x + tok * D + (long)h * hd + i;
     const float v1 = p[0], v2 = p[half];
@@ -589,6 +637,19 @@ __global__ void swiglu_bwd_paired_kernel(const float* __restrict__ dOut, const f
     const float g = gate[pe], u = up[pe], sig = act_fwd(GN_ACT_SIGMOID, g), sw = g * sig, go = dOut[e];
     dUpP[pe] = go * sw; dGateP[pe] = go * (sw + sig * (1.f - sw)) * u;
   }
+}
+// The same for the gradient of token 0 alone: rows s of dOut, dGate, dUp are dense, the last token's projections lie `ld` apart
+__global__ void swiglu_bwd_rows_kernel(const float* __restrict__ dOut, const float* __restrict__ gate, const float* __restrict__ up, long ld,
+                                       float* __restrict__ dGate, float* __restrict__ dUp, int C, long total) {
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
+    const long s = e / C, o = s * ld + (e - s * C);
+    const float g = gate[o], u = up[o], sig = act_fwd(GN_ACT_SIGMOID, g), sw = g * sig, go = dOut[e];
+    dUp[e] = go * sw; dGate[e] = go * (sw + sig * (1.f - sw)) * u;
+  }
+}
+// dx[s, 0, :] += r[s, :]; one block per sequence
+__global__ void add_row0_kernel(const float* __restrict__ r, float* __restrict__ dx, int T, int d) {
+  for (int i = threadIdx.x; i < d; i += blockDim.x) dx[(long)blockIdx.x * T * d + i] += r[(long)blockIdx.x * d + i];
 }
 // out[s,t,:] = a[s,t,:] + b[s,T-1-t,:]
 __global__ void add_token_reversed_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, int T, int C, long total) {

@@ -1,0 +1,63 @@
+"""Which tokens of a TransformerBlock are computed depends on the layers above it (CLSPooling reads token 0 only): parity with
+the CPU checker where that rule changes the path -- one and two blocks, one token, causal and not, mixed, every feed-forward
+variant, and models without CLSPooling, whose blocks run all tokens in both directions."""
+import numpy as np
+import pytest
+
+from goneuron_b200 import configs, descriptors as D
+from tests.parity import TOL, assert_grads_close, norm_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    from goneuron_b200.sequential import Device
+    d = Device(0)
+    yield d
+    d.close()
+
+
+def _model(T, dim, heads, ff, masks, pool, vocab=60, classes=11, **kw):
+    layers = [D.Embedding(vocab, dim, T), D.PositionalEncoding(T, dim)]
+    layers += [D.TransformerBlock(dim, heads, T, ff, c, **kw) for c in masks]
+    layers += [D.CLSPooling(T, dim), D.Dense(dim, classes, D.LOGSOFTMAX)] if pool else [D.Flatten(), D.Dense(T * dim, classes, D.LOGSOFTMAX)]
+    return layers
+
+
+CASES = [
+    (1, 32, 2, 48, [True, True], True, {}), (1, 32, 2, 48, [False], True, {}),                       # a single token
+    (2, 32, 2, 48, [False, False], True, {}),                                                        # token 0 and the last one are all
+    (37, 48, 3, 100, [True, True, True], True, {}), (37, 48, 3, 100, [False, False], True, {}),
+    (37, 48, 3, 100, [True, False, True], True, {}), (37, 48, 3, 100, [False, True], True, {}),       # mixed masks
+    (300, 40, 5, 64, [False, False], True, {}),                                                      # head size 8, more keys than threads
+    (20, 600, 1, 64, [False], True, {}),                                                             # head size above the block width
+    (21, 66, 6, 36, [False, False], True, {}),                                                       # head size 11: no 16-byte loads
+    (24, 64, 2, 96, [True, True], True, dict(ff_act=D.SILU, rms_norm=True, rope=True)),
+    (24, 64, 2, 96, [False, False], True, dict(ff_act=D.SILU, rms_norm=True, rope=True)),
+    (24, 64, 2, 96, [True, True], True, dict(ff_act=D.GELU, rope=True)), (24, 64, 2, 96, [False], True, dict(ff_act=D.GELU)),
+    (128, 128, 2, 256, [True, True], False, {}), (128, 128, 2, 256, [False], False, {}), (40, 64, 2, 96, [True, True], False, dict(rope=True)),
+]
+
+
+@pytest.mark.parametrize("T,dim,heads,ff,masks,pool,kw", CASES)
+def test_token_rows_parity(device, oracle, T, dim, heads, ff, masks, pool, kw):
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = _model(T, dim, heads, ff, masks, pool, **kw)
+    rng = np.random.Generator(np.random.PCG64(99))
+    params = configs.init_params(layers, rng)
+    x, y = configs.make_inputs("transformer", layers, 3, rng)
+    ref = oracle.OracleState(layers, D.CROSS_ENTROPY, params, lr=1e-4)
+    out = oracle.OracleState(layers, D.CROSS_ENTROPY, params).forward_batch(x, threads=3, precision=64)
+    lit = oracle.OracleState(layers, D.CROSS_ENTROPY, params, lr=1e-4)
+    loss_ref = ref.train_batch(x, y, W=2, threads=4, precision=64)
+    lit.train_batch(x, y, W=2, threads=2, precision=32)
+    model = Sequential(layers, device, virtual_workers=2).Compile(Adam(1e-4), D.CROSS_ENTROPY)
+    model.SetParams(params)
+    assert norm_err(model.PredictBatch(x), out) <= TOL
+    loss = model.TrainBatch(x, y)
+    assert abs(loss - loss_ref) <= TOL * max(1.0, abs(loss_ref))
+    assert_grads_close(layers, model.Gradients(), ref.grads, floor=lit.grads)
+    model.SetParams(params)
+    assert norm_err(model.PredictBatch(x), out) <= TOL          # and inference after a training step
+    model.Close()
