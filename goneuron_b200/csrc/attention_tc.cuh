@@ -714,12 +714,12 @@ inline int attn_tc_prepare(Ctx* ctx, int n, const float* const* X, const bool* w
 }
 // the two tensor maps (hi, lo) of row planes [Z][T][64] with `box_rows` rows per copy, or of transposed planes [Z][64][T]
 inline int attn_tc_maps_rows(Ctx* ctx, CUtensorMap* m, const AttnPlanes& p, int T, int Z, int box_rows) {
-  GN_TRY(tc_make_map_bf16_raw(ctx, &m[0], p.rh, ATC_HD, T, ATC_HD, Z, 0, box_rows, 64, CU_TENSOR_MAP_DATA_TYPE_FLOAT16));
-  return tc_make_map_bf16_raw(ctx, &m[1], p.rl, ATC_HD, T, ATC_HD, Z, 0, box_rows, 64, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+  GN_TRY(tc_make_map_f16(ctx, &m[0], p.rh, ATC_HD, T, ATC_HD, Z, box_rows));
+  return tc_make_map_f16(ctx, &m[1], p.rl, ATC_HD, T, ATC_HD, Z, box_rows);
 }
 inline int attn_tc_maps_cols(Ctx* ctx, CUtensorMap* m, const AttnPlanes& p, int T, int Z) {
-  GN_TRY(tc_make_map_bf16_raw(ctx, &m[0], p.ch, T, ATC_HD, T, Z, 0, ATC_HD, 64, CU_TENSOR_MAP_DATA_TYPE_FLOAT16));
-  return tc_make_map_bf16_raw(ctx, &m[1], p.cl, T, ATC_HD, T, Z, 0, ATC_HD, 64, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+  GN_TRY(tc_make_map_f16(ctx, &m[0], p.ch, T, ATC_HD, T, Z, ATC_HD));
+  return tc_make_map_f16(ctx, &m[1], p.cl, T, ATC_HD, T, Z, ATC_HD);
 }
 inline int attn_tc_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal,
                        AttnSaved* save = nullptr) {

@@ -32,7 +32,7 @@ __device__ __forceinline__ float patch_elem(const float* __restrict__ sb, const 
   return sb[((long)ch * g.sH + iy) * g.sW + ix];
 }
 // One warp per plane row (one output position), lanes over the contraction index.  rows = B*oH*oW, K = C*k*k.
-__global__ void __launch_bounds__(256) conv_patch_rows_split_kernel(const float* __restrict__ src, PatchGeom g, long rows, int K, __half* __restrict__ p0, __half* __restrict__ p1,
+__global__ void __launch_bounds__(256) conv_patch_rows_split_kernel(const float* __restrict__ src, PatchGeom g, long rows, int K, __half* __restrict__ pl,
                                                                     float* __restrict__ inv_scale, int ldp) {
   const int lane = threadIdx.x & 31;
   const long r = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -44,16 +44,16 @@ __global__ void __launch_bounds__(256) conv_patch_rows_split_kernel(const float*
   mx = warp_max(mx);
   float inv; const float sc = row_scale(mx, &inv);
   if (lane == 0) inv_scale[r] = inv;
-  __half* q0 = p0 + r * ldp; __half* q1 = p1 + r * ldp;
+  __half* o = pl + r * 2 * ldp;
   for (int kidx = lane; kidx < ldp; kidx += 32) {
     const float v = kidx < K ? patch_elem(sb, g, oy, ox, kidx) * sc : 0.f;
     const __half h = __float2half_rn(v);
-    q0[kidx] = h; q1[kidx] = __float2half_rn(v - __half2float(h));
+    o[pl_off(kidx)] = h; o[pl_off(kidx) + PL_LO] = __float2half_rn(v - __half2float(h));
   }
 }
 // Transposed patches of one sample for the weight gradient: plane row = (b, kidx), kidx in [0, K] with row K = ones;
 // contraction index = output position.  One warp per plane row, lanes over the positions.
-__global__ void __launch_bounds__(256) conv_patch_cols_split_kernel(const float* __restrict__ src, PatchGeom g, int B, int K, __half* __restrict__ p0, __half* __restrict__ p1,
+__global__ void __launch_bounds__(256) conv_patch_cols_split_kernel(const float* __restrict__ src, PatchGeom g, int B, int K, __half* __restrict__ pl,
                                                                     float* __restrict__ inv_scale, int ldp) {
   const int lane = threadIdx.x & 31, P = g.oH * g.oW, rows = K + 1;
   const long r = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -66,11 +66,11 @@ __global__ void __launch_bounds__(256) conv_patch_cols_split_kernel(const float*
   mx = warp_max(mx);
   float inv; const float sc = row_scale(mx, &inv);
   if (lane == 0) inv_scale[r] = inv;
-  __half* q0 = p0 + r * ldp; __half* q1 = p1 + r * ldp;
+  __half* o = pl + r * 2 * ldp;
   for (int pix = lane; pix < ldp; pix += 32) {
     const float v = pix < P ? elem(pix) * sc : 0.f;
     const __half h = __float2half_rn(v);
-    q0[pix] = h; q1[pix] = __float2half_rn(v - __half2float(h));
+    o[pl_off(pix)] = h; o[pl_off(pix) + PL_LO] = __float2half_rn(v - __half2float(h));
   }
 }
 // Wd[ic, (oc,kh,kw)] = W[oc, ic, kh, kw]: the weight matrix of the input-gradient product
@@ -103,7 +103,7 @@ inline int conv_tc_forward(Ctx* ctx, const ConvShape& c, const float* x, const f
   const int K = c.inC * c.k * c.k, P = c.oH * c.oW; const long M = (long)c.B * P;
   BfPlanes A, Bp; GN_TRY(tc_planes(ctx, 0, 1, M, K, &A)); GN_TRY(tc_planes(ctx, 1, 1, c.outC, K, &Bp));
   PatchGeom g{c.inC, c.k, c.s, 1, -c.p, c.H, c.W, c.oH, c.oW};
-  GN_LAUNCH(ctx, conv_patch_rows_split_kernel, cdiv(M, 8), 256, 0, x, g, M, K, A.p0(), A.p1(), A.inv_scale, A.ldp);
+  GN_LAUNCH(ctx, conv_patch_rows_split_kernel, cdiv(M, 8), 256, 0, x, g, M, K, A.base, A.inv_scale, A.ldp);
   ctx->split_bytes += 8.0 * (double)M * K;
   GN_TRY(tc_split(ctx, TcSrc{W, (long)K, 1, 0, 0, 1}, Bp, nullptr));
   TcParams ep{dst, (long)c.outC, 0, 0, bias, nullptr, 0, 0, 0, epilogue_act, (int)M, c.outC, K, 1, 0, ctx->d_status, nullptr, 0, 1};
@@ -116,7 +116,7 @@ inline int conv_tc_dgrad(Ctx* ctx, const ConvShape& c, const float* dz, const fl
   const int kk = c.k * c.k, Kd = c.outC * kk, P = c.H * c.W; const long M = (long)c.B * P;
   BfPlanes A, Bp; GN_TRY(tc_planes(ctx, 0, 1, M, Kd, &A)); GN_TRY(tc_planes(ctx, 1, 1, c.inC, Kd, &Bp));
   PatchGeom g{c.outC, c.k, 1, -1, c.p, c.oH, c.oW, c.H, c.W};
-  GN_LAUNCH(ctx, conv_patch_rows_split_kernel, cdiv(M, 8), 256, 0, dz, g, M, Kd, A.p0(), A.p1(), A.inv_scale, A.ldp);
+  GN_LAUNCH(ctx, conv_patch_rows_split_kernel, cdiv(M, 8), 256, 0, dz, g, M, Kd, A.base, A.inv_scale, A.ldp);
   ctx->split_bytes += 8.0 * (double)M * Kd;
   GN_LAUNCH(ctx, conv_w_dgrad_layout_kernel, cdiv((long)Kd * c.inC, 256), 256, 0, W, wtmp, c.outC, c.inC, kk);
   GN_TRY(tc_split(ctx, TcSrc{wtmp, (long)Kd, 1, 0, 0, 1}, Bp, nullptr));
@@ -131,7 +131,7 @@ inline int conv_tc_wgrad(Ctx* ctx, const ConvShape& c, const float* dz, const fl
   BfPlanes A, Bp; GN_TRY(tc_planes(ctx, 0, c.B, c.outC, P, &A)); GN_TRY(tc_planes(ctx, 1, c.B, N, P, &Bp));
   GN_TRY(tc_split(ctx, TcSrc{dz, (long)P, 1, (long)c.outC * P, 0, 1}, A, nullptr));          // g[b] is [outC][P] as stored
   PatchGeom g{c.inC, c.k, c.s, 1, -c.p, c.H, c.W, c.oH, c.oW};
-  GN_LAUNCH(ctx, conv_patch_cols_split_kernel, cdiv((long)c.B * N, 8), 256, 0, x, g, c.B, K, Bp.p0(), Bp.p1(), Bp.inv_scale, Bp.ldp);
+  GN_LAUNCH(ctx, conv_patch_cols_split_kernel, cdiv((long)c.B * N, 8), 256, 0, x, g, c.B, K, Bp.base, Bp.inv_scale, Bp.ldp);
   ctx->split_bytes += 8.0 * (double)c.B * N * P;
   TcParams ep{part, (long)N, (long)c.outC * N, 0, nullptr, nullptr, 0, 0, 0, GN_ACT_LINEAR, c.outC, N, P, 1, 0, ctx->d_status, nullptr, 0, 1};
   conv_tc_count(ctx, (double)c.B * c.outC, N, P);

@@ -54,22 +54,27 @@ extern "C" int gn_op_gemm_nt_static(gn_ctx* ctx, int M, int N, int K, const floa
   if (!ctx || !ctx->alive || !A_dev || !B_dev || !C_dev || M <= 0 || N <= 0 || K <= 0) return fail(GN_ERR_INVALID_ARG, "op_gemm_nt_static: bad argument");
   Ctx* c = &ctx->c;
   if (!c->tc_ok) return fail(GN_ERR_UNSUPPORTED, "the tensor-core engine is not available on this context");
-  const long ldp = tc_ldp(K);
-  const long need = ((long)M + N) * (ldp + 1);
+  const long ldp8 = (K + 7) / 8 * 8L, need = ((long)M + N) * (ldp8 + 1);      // the documented limit
   if (need > GN_STATIC_SCRATCH_FLOATS)
     return fail(GN_ERR_INVALID_ARG, "op_gemm_nt_static: M=%d N=%d K=%d needs %ld scratch floats, the fixed array holds %ld ((M+N)*(roundup8(K)+1) must not exceed it)",
                 M, N, K, need, GN_STATIC_SCRATCH_FLOATS);
   std::lock_guard<std::mutex> lk(c->run_mu);
   GN_CUDA(cudaSetDevice(c->device));
   float* base = nullptr; GN_TRY(static_scratch_ptr(c->device, &base));
-  float* scales = base + ((long)M + N) * ldp;          // [M] for A, then [N] for B; (M + N) * ldp is a multiple of 8 floats, so B's start is 16-byte aligned when M % 4 == 0
-  float* sb = scales + (((long)M + 3) & ~3L);
-  if (sb + N > base + GN_STATIC_SCRATCH_FLOATS) return fail(GN_ERR_INVALID_ARG, "op_gemm_nt_static: M=%d N=%d K=%d does not fit the fixed array", M, N, K);
-  BfPlanes PA{reinterpret_cast<__half*>(base), scales, M, K, (int)ldp, 1}, PB{reinterpret_cast<__half*>(base + (long)M * ldp), sb, N, K, (int)ldp, 1};
-  GN_TRY(tc_split(c, TcSrc{A_dev, (long)K, 1, 0, 0, 1}, PA, nullptr));
-  GN_TRY(tc_split(c, TcSrc{B_dev, (long)K, 1, 0, 0, 1}, PB, nullptr));
-  TcParams ep{C_dev, (long)N, 0, 0, bias_dev, nullptr, 0, 0, 0, GN_ACT_LINEAR, M, N, K, 1, 0, c->d_status, nullptr, 0, 1};
-  GN_TRY(tc_run(c, PA, PB, ep));
+  // Plane rows are padded to whole blocks of 32, so a product near the limit may not fit at once: then the larger of its two
+  // sides is walked in pieces (every output element is formed in the same way).
+  const long ldp = tc_ldp(K); long mc = M, nc = N;
+  auto floats = [&](long m, long n) { return (m + n) * ldp + ((m + 3) & ~3L) + n; };
+  while (floats(mc, nc) > GN_STATIC_SCRATCH_FLOATS) { long& x = mc >= nc ? mc : nc; x = ((x + 1) / 2 + 3) & ~3L; }
+  for (long n0 = 0; n0 < N; n0 += nc) for (long m0 = 0; m0 < M; m0 += mc) {
+    const int m = (int)std::min(mc, M - m0), n = (int)std::min(nc, N - n0);
+    float* sa = base + ((long)m + n) * ldp; float* sb = sa + ((m + 3) & ~3);        // row scales: A's, then B's on a 16-byte boundary
+    BfPlanes PA{reinterpret_cast<__half*>(base), sa, m, K, (int)ldp, 1}, PB{reinterpret_cast<__half*>(base + (long)m * ldp), sb, n, K, (int)ldp, 1};
+    GN_TRY(tc_split(c, TcSrc{A_dev + m0 * K, (long)K, 1, 0, 0, 1}, PA, nullptr));
+    GN_TRY(tc_split(c, TcSrc{B_dev + n0 * K, (long)K, 1, 0, 0, 1}, PB, nullptr));
+    TcParams ep{C_dev + m0 * N + n0, (long)N, 0, 0, bias_dev ? bias_dev + n0 : nullptr, nullptr, 0, 0, 0, GN_ACT_LINEAR, m, n, K, 1, 0, c->d_status, nullptr, 0, 1};
+    GN_TRY(tc_run(c, PA, PB, ep));
+  }
   GN_CUDA(cudaStreamSynchronize(c->stream));
   return check_status_word(c);
 }

@@ -19,15 +19,14 @@
 // memory (8 KB per 64 tensor cycles = the full 128 B/clk) while TMA writes the next stage into the same memory.  The
 // large-problem variant therefore uses 128 x 256 tiles (12 KB per 128 tensor cycles).
 //
-// The operand planes (K-major fp16, row stride a multiple of 8 elements) and the per-row inverse scales are written
+// The operand planes (K-major fp16, interleaved in blocks of 32 indices) and the per-row inverse scales are written
 // by a memory-bound pass (split2_rows_kernel / split2_cols_kernel); the contraction kernel itself is a pure
 // TMA -> shared memory -> tcgen05.mma pipeline:
 //
-//   warp 0   TMA producer: 4 tiled bulk copies per stage (64-byte rows, 64-byte swizzle; 3-D maps, third
+//   warp 0   TMA producer: 3 tiled bulk copies per stage (128-byte rows, 128-byte swizzle; 3-D maps, third
 //            coordinate = problem index of a batch)
 //   warp 1   allocates TMEM, issues the MMAs (one elected lane), commits to mbarriers
-//   warps 2-5  epilogue: tcgen05.ld of the accumulators, scales / bias / residual / ReLU / gate, one output row
-//              per thread with 16-byte stores
+//   warps 2-9  epilogue: tcgen05.ld of the accumulators, scales / bias / residual / ReLU / gate, whole 128-byte lines
 //
 // Persistent: one CTA per SM walks 128 x BN output tiles.  TMEM holds two accumulator slots, so the epilogue
 // of tile i runs under the mainloop of tile i+1.  The tensor core truncates when it adds a group of products
@@ -55,14 +54,20 @@ constexpr unsigned TC_SPIN_LIMIT = 1u << 24;    // default number of polls of on
 constexpr unsigned TC_DRAIN_LIMIT = 1u << 20;   // polls spent waiting for own work in flight after a wait gave up
 constexpr int TC_QUEUE_POOL = 2048;   // tile-queue counters per context before the pool is cleared again
 constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by the host when every pointer and stride allows it)
-// One stage = 32 contraction indices of both operands: two fp16 planes each, 64-byte rows.
-constexpr int TC_BK = 32;
+// One stage = 32 contraction indices of both operands.  The two fp16 planes of an operand are interleaved in blocks of 32:
+// element (r, k) of a plane row has its high part at pl_off(k) and its low part PL_LO halves further, so a block of a row is 128
+// contiguous bytes, one TMA copy brings both planes of a stage, and the tile has 128-byte rows (128-byte swizzle).  With separate
+// planes and 64-byte rows (64-byte swizzle) every MMA took 141 cycles, whatever its width (128 x 128 x 16 needs 64 of arithmetic).
+// With this, the issue loops in uniform registers and the epilogue below, [8192, 256] x [256, 256] went from 16.5 to 10.4 us,
+// [8192, 1024] x [1024, 256] from 26.8 to 18.6, [32768, 1024] x [1024, 1024] from 136 to 119 (zeros as data: no power limit).
+constexpr int TC_BK = 32, PL_LO = 32;
+__host__ __device__ __forceinline__ int pl_off(int k) { return ((k >> 5) << 6) | (k & 31); }
 template <int BN> struct TcCfg {
-  static constexpr int A_PL = TC_BM * TC_BK * 2, B_PL = BN * TC_BK * 2;           // one plane of a stage: 8 KB, BN * 64 B
-  static constexpr int STAGE_BYTES = 2 * A_PL + 2 * B_PL;
+  static constexpr int A_BYTES = TC_BM * 128, B_BYTES = BN * 128;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (192 * 1024) / STAGE_BYTES > 8 ? 8 : (192 * 1024) / STAGE_BYTES;
   static constexpr int COLV_FLOATS = TC_EPI_WARPS * BN;                           // per epilogue warp: scale and bias of its BN / 2 columns
-  static constexpr int STG_FLOATS = TC_EPI_WARPS * 32 * 20;                       // per epilogue warp: 32 rows x 16 (+4) accumulators in transit
+  static constexpr int STG_FLOATS = TC_EPI_WARPS * 16 * 36;                       // per epilogue warp: 16 rows x 32 (+4) accumulators in transit
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/ + (COLV_FLOATS + STG_FLOATS) * 4;
   static constexpr bool MERGED = BN > 128;                                        // one accumulator per slot
   static constexpr int SLOT_COLS = MERGED ? BN : 2 * BN;
@@ -103,6 +108,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
 }
+// One lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -112,10 +123,16 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint
   asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Two consecutive products with the same A operand: the first leaves it in the tensor core's collector, the second takes it
+// from there instead of reading shared memory again (128 x 128 tiles over 1024 indices: 20.4 -> 18.6 us).
+__device__ __forceinline__ void tc_mma_f16_same_a(uint32_t d1, uint32_t d2, uint64_t adesc, uint64_t b1, uint64_t b2, uint32_t idesc, uint32_t acc1, uint32_t acc2) {
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %6, 0;\nsetp.ne.b32 q, %7, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %2, %3, %5, p;\n"
+               "tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%1], %2, %4, %5, q;\n}"
+               ::"r"(d1), "r"(d2), "l"(adesc), "l"(b1), "l"(b2), "r"(idesc), "r"(acc1), "r"(acc2) : "memory");
+}
 // Shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows are 128 bytes apart, groups of 8
 // rows 1024 bytes apart (stride byte offset), descriptor version 1 (sm_100), layout type 2 = SWIZZLE_128B.
-// With 64-byte rows (make_desc<16>: 16 fp32 or 32 bf16 per row): groups of 8 rows are 512 bytes apart and the layout
-// type is 4 = SWIZZLE_64B.
 template <int BK>
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
   constexpr uint64_t sbo = (8 * BK * 4) >> 4, layout = BK == 32 ? 2 : 4;
@@ -164,9 +181,9 @@ struct TcParams {
   const float* isa = nullptr; const float* isb = nullptr;   // inverse row scales of the operand planes: [nbatch][M], [nbatch][N]
   unsigned spin_limit = TC_SPIN_LIMIT;                // polls per wait before the kernel gives up
   int nchw_P = 0;      // > 0: output row r = (sample r / P, position r % P) is stored as C[sample][col][position] (N channels of P positions)
-  // Plane output (out_p0 != null): the result is not stored as fp32 but directly as the operand planes of the next
-  // contraction (two fp16 planes [M][out_ldp] and an inverse scale per row), see TcPlaneOut.  C may then be null.
-  __half* out_p0 = nullptr; __half* out_p1 = nullptr; float* out_inv = nullptr; long out_ldp = 0;
+  // Plane output (out_p != null): the result is not stored as fp32 but directly as the operand planes of the next
+  // contraction (two interleaved fp16 planes [M][2 out_ldp] and an inverse scale per row), see TcPlaneOut.  C may then be null.
+  __half* out_p = nullptr; float* out_inv = nullptr; long out_ldp = 0;
   const float* a_rownorm = nullptr; const int* b_maxabs = nullptr;     // the bound's factors: |row of A|_2 and max |entry of B (and bias)| as float bits
   float* c_last = nullptr; int last_T = 0;                             // fp32 copy of the rows r with r % last_T == last_T - 1: c_last[(r / last_T) * N + col]
   float* rowsum32 = nullptr;                                           // plane output: sums of the result over every 32 consecutive rows, [ceil(M / 32)][N]
@@ -193,149 +210,170 @@ __device__ __forceinline__ void tc_epilogue_stage(const TcParams& ep, int n0, in
     }
     __syncwarp();
 }
-// `stg`: this warp's staging buffer of 32 rows x TC_STG_LD floats.  The TMEM load gives every thread ITS row (lane =
-// row), and a store of that shape touches 32 different 128-byte lines per instruction -- measured: 19 000 cycles of
-// epilogue per 128 x 256 tile, twice that for the two planes of a plane output, which then set the pace instead of the
-// MMAs.  So the accumulators of 16 columns go through shared memory and come back with four neighbouring lanes on one
-// row (8 rows per instruction); scale, bias, residual, activation and gate are applied on that side, where the residual
-// and gate reads are coalesced too.
-constexpr int TC_STG_LD = 20;
+// `stg`: this warp's staging buffer of 16 rows x TC_STG_LD floats.  The TMEM load gives every thread ITS row (lane = row), and a
+// store of that shape touches 32 different 128-byte lines per instruction.  So the accumulators of 32 columns go through
+// shared memory, 16 rows at a time, and come back with eight neighbouring lanes on one row: every store, residual and gate
+// access is four whole 128-byte lines.  The loops over chunks and row halves are not unrolled: a launch with one tile per CTA runs
+// this code once, from a cold instruction cache, and there the previous, fully unrolled version (with all variants in one body)
+// took 12 000 cycles for a 128 x 128 tile against 6 000 for the tiles after it -- as much as the MMAs of a contraction over 512.
+constexpr int TC_STG_LD = 36;
+// acc[j] of column c * 32 + j for this lane's row, times the row's inverse scale
+template <bool MERGED>
+__device__ __forceinline__ void tc_acc_chunk(uint32_t taddr, uint32_t acc_main, uint32_t acc_cross, bool any, float isa, float (&v)[32]) {
+  if (any) {
+    uint32_t r[32];
+    tmem_ld32(taddr + acc_main, r);
+    if constexpr (!MERGED) {
+      uint32_t q[32];
+      tmem_ld32(taddr + acc_cross, q);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] = (__uint_as_float(r[j]) + __uint_as_float(q[j])) * isa;
+    } else {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]) * isa;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; j++) v[j] = 0.f;
+  }
+}
+__device__ __forceinline__ void tc_stage_rows(float* stg, const float (&v)[32], int lane, int hh) {
+  __syncwarp();                                               // the previous half has been read back
+  if ((lane >> 4) == hh) {
+    float* s = stg + (lane & 15) * TC_STG_LD;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(s + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  }
+  __syncwarp();
+}
 template <int BN, bool MERGED>
 __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tmem_base, uint32_t acc_main, uint32_t acc_cross,
                                                  int m0, int n0, int z, int quad, int chalf, int lane, int nkb, int bw, const float* colv, float* stg) {
-    const int z1 = z / ep.batch2, z2 = z % ep.batch2;
-    float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
-    const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
-    const bool vec = (ep.flags & TC_FLAG_VEC) != 0;
-    const float* isb = ep.isb + (long)z * ep.N;
-    const int nch = bw / 64;                                               // chunks of 32 columns per warp
-    if (vec) {
-      // after the transposition: lane -> row 8 t + lane / 4 of the warp's 32 (t = 0..3), columns 4 (lane % 4) .. + 3 of 16
-      const int rl = lane >> 2, c4 = (lane & 3) * 4, rbase = m0 + quad * 32;
-      float isa4[4], osc4[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int row = rbase + 8 * t + rl; const bool row_ok = row < ep.M;
-        isa4[t] = row_ok ? ep.isa[(long)z * ep.M + row] : 1.f;              // 1 / (scale of this output row's A vector), a power of two
-        osc4[t] = 1.f;                                                       // plane output: this row's scale
-        if (ep.out_p0 && row_ok) {
-          const float an = ep.a_rownorm[row], bound = sqrtf(fmaf(an, an, 1.f)) * sqrtf((float)ep.K + 1.f) * __int_as_float(*ep.b_maxabs);
-          float oinv; osc4[t] = row_scale(bound, &oinv);
-          if (n0 == 0 && chalf == 0 && c4 == 0) ep.out_inv[row] = oinv;
-        }
-      }
-      for (int cc = 0; cc < nch; cc++) {
-        const int c = chalf * nch + cc, col0 = n0 + c * 32;
-        if (col0 >= ep.N) break;
-        uint32_t r[32], q[MERGED ? 1 : 32];
-        if (nkb > 0) {
-          const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32);
-          tmem_ld32(taddr + acc_main, r);
-          if constexpr (!MERGED) tmem_ld32(taddr + acc_cross, q);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if constexpr (!MERGED) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(q[j]));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; j++) r[j] = 0u;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int col = col0 + 16 * h + c4; const bool col_ok = col < ep.N;
-          // residual and gate of this half, fetched before the exchange so that their latency overlaps it
-          float4 rv[4], mv[4];
-#pragma unroll
-          for (int t = 0; t < 4; t++) {
-            const int row = rbase + 8 * t + rl; const bool in = col_ok && row < ep.M;
-            rv[t] = (R && in) ? *reinterpret_cast<const float4*>(R + (long)row * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-            mv[t] = (ep.mask && in) ? *reinterpret_cast<const float4*>(ep.mask + (long)(row / ep.mask_group) * ep.mask_ld + col) : make_float4(1.f, 1.f, 1.f, 1.f);
-          }
-          __syncwarp();                                       // the previous half has been read back
-#pragma unroll
-          for (int j = 0; j < 16; j += 4) {
-            const float4 a = make_float4(__uint_as_float(r[16 * h + j]), __uint_as_float(r[16 * h + j + 1]), __uint_as_float(r[16 * h + j + 2]), __uint_as_float(r[16 * h + j + 3]));
-            *reinterpret_cast<float4*>(stg + lane * TC_STG_LD + j) = a;
-          }
-          __syncwarp();
-          const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + 16 * h + c4), bv = *reinterpret_cast<const float4*>(colv + BN / 2 + cc * 32 + 16 * h + c4);
-          float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);      // plane output: this lane's part of the warp's 32-row column sums
-#pragma unroll
-          for (int t = 0; t < 4; t++) {
-            const int row = rbase + 8 * t + rl;
-            if (!col_ok || row >= ep.M) continue;
-            const float4 a = *reinterpret_cast<const float4*>(stg + (8 * t + rl) * TC_STG_LD + c4);
-            const float isa = isa4[t];
-            float4 v;
-            v.x = a.x * isa * sv.x + bv.x + rv[t].x; v.y = a.y * isa * sv.y + bv.y + rv[t].y;
-            v.z = a.z * isa * sv.z + bv.z + rv[t].z; v.w = a.w * isa * sv.w + bv.w + rv[t].w;
-            if (ep.act == GN_ACT_RELU) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
-            if (!(mv[t].x > 0.f)) v.x = 0.f; if (!(mv[t].y > 0.f)) v.y = 0.f; if (!(mv[t].z > 0.f)) v.z = 0.f; if (!(mv[t].w > 0.f)) v.w = 0.f;
-            if (ep.out_p0) {
-              uint2 p0, p1; split2_pair(v.x, v.y, osc4[t], p0.x, p1.x); split2_pair(v.z, v.w, osc4[t], p0.y, p1.y);
-              const long o = (long)row * ep.out_ldp + col;
-              *reinterpret_cast<uint2*>(ep.out_p0 + o) = p0; *reinterpret_cast<uint2*>(ep.out_p1 + o) = p1;
-              if (ep.c_last && row % ep.last_T == ep.last_T - 1) *reinterpret_cast<float4*>(ep.c_last + (long)(row / ep.last_T) * ep.N + col) = v;
-              csum.x += v.x; csum.y += v.y; csum.z += v.z; csum.w += v.w;
-            } else *reinterpret_cast<float4*>(C + (long)row * ep.ldc + col) = v;
-          }
-          if (ep.rowsum32) {
-            // the consumer of a plane output's token sums (the weight gradient of the layer below) gets them from here instead
-            // of re-reading the planes: rows 8 t + rl of this lane, then the eight lanes that share its columns, in a fixed order
-#pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-              csum.x += __shfl_xor_sync(0xffffffffu, csum.x, o); csum.y += __shfl_xor_sync(0xffffffffu, csum.y, o);
-              csum.z += __shfl_xor_sync(0xffffffffu, csum.z, o); csum.w += __shfl_xor_sync(0xffffffffu, csum.w, o);
-            }
-            if (rl == 0 && col_ok && rbase < ep.M) *reinterpret_cast<float4*>(ep.rowsum32 + (long)(rbase >> 5) * ep.N + col) = csum;
-          }
-        }
-      }
-      __syncwarp();
-      return;
+  const int z1 = z / ep.batch2, z2 = z - z1 * ep.batch2, nch = bw / 64;      // chunks of 32 columns per warp
+  const int rbase = m0 + quad * 32, row = rbase + lane;
+  const uint32_t tquad = tmem_base + ((uint32_t)(quad * 32) << 16);
+  const float isa = row < ep.M ? ep.isa[(long)z * ep.M + row] : 1.f;         // 1 / (scale of this row's A vector), a power of two
+  const int rl = lane >> 3, c4 = (lane & 7) * 4;                             // after the exchange: rows 4 t + rl, columns c4 .. c4 + 3
+  if (ep.out_p) {
+    // plane output: the result becomes the next contraction's A operand
+    float osc = 1.f;                                                         // this lane's row's scale
+    if (row < ep.M) {
+      const float an = ep.a_rownorm[row], bound = sqrtf(fmaf(an, an, 1.f)) * sqrtf((float)ep.K + 1.f) * __int_as_float(*ep.b_maxabs);
+      float oinv; osc = row_scale(bound, &oinv);
+      if (n0 == 0 && chalf == 0) ep.out_inv[row] = oinv;
     }
-    // scalar path (unaligned operands, NCHW store): one output row per thread
-    const int row = m0 + quad * 32 + lane;
-    const bool row_ok = row < ep.M;
-    const float* Rrow = (R && row_ok) ? R + (long)row * ep.ldr : nullptr;
-    const float* Mrow = (ep.mask && row_ok) ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
-    float* Crow = C + (long)row * ep.ldc;
-    const float isa = row_ok ? ep.isa[(long)z * ep.M + row] : 1.f;
+#pragma unroll 1
     for (int cc = 0; cc < nch; cc++) {
-      const int c = chalf * nch + cc, col0 = n0 + c * 32;
-      if (col0 >= ep.N) break;
-      uint32_t r[32], q[MERGED ? 1 : 32];
-      if (nkb > 0) {
-        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32);
-        tmem_ld32(taddr + acc_main, r);
-        if constexpr (!MERGED) tmem_ld32(taddr + acc_cross, q);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      }
+      const int c = chalf * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
+      if (n0 + c * 32 >= ep.N) break;
+      float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
+      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + BN / 2 + cc * 32 + c4);
+      float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);                         // this lane's part of the warp's 32-row column sums
+#pragma unroll 1
+      for (int hh = 0; hh < 2; hh++) {
+        float4 mv[4];
 #pragma unroll
-      for (int j = 0; j < 32; j++) {
-        const int col = col0 + j;
-        if (!row_ok || col >= ep.N) continue;
-        float a = 0.f;
-        if (nkb > 0) { if constexpr (MERGED) a = __uint_as_float(r[j]); else a = __uint_as_float(r[j]) + __uint_as_float(q[j]); }
-        float v = a * isa * isb[col];
-        if (ep.bias) v += ep.bias[col];
-        if (Rrow) v += Rrow[col];
-        if (ep.act == GN_ACT_RELU) v = fmaxf(v, 0.f);
-        if (Mrow && !(Mrow[col] > 0.f)) v = 0.f;
-        if (ep.nchw_P > 0) C[((long)(row / ep.nchw_P) * ep.N + col) * ep.nchw_P + row % ep.nchw_P] = v;
-        else Crow[col] = v;
+        for (int t = 0; t < 4; t++) {
+          const int r = rbase + 16 * hh + 4 * t + rl;
+          mv[t] = (ep.mask && col_ok && r < ep.M) ? *reinterpret_cast<const float4*>(ep.mask + (long)(r / ep.mask_group) * ep.mask_ld + col) : make_float4(1.f, 1.f, 1.f, 1.f);
+        }
+        tc_stage_rows(stg, v, lane, hh);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const int rr = 16 * hh + 4 * t + rl, r = rbase + rr; const float os = __shfl_sync(0xffffffffu, osc, rr);
+          if (!col_ok || r >= ep.M) continue;
+          const float4 a = *reinterpret_cast<const float4*>(stg + (4 * t + rl) * TC_STG_LD + c4);
+          float4 x = make_float4(a.x * sv.x + bv.x, a.y * sv.y + bv.y, a.z * sv.z + bv.z, a.w * sv.w + bv.w);
+          if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
+          if (!(mv[t].x > 0.f)) x.x = 0.f; if (!(mv[t].y > 0.f)) x.y = 0.f; if (!(mv[t].z > 0.f)) x.z = 0.f; if (!(mv[t].w > 0.f)) x.w = 0.f;
+          uint2 p0, p1; split2_pair(x.x, x.y, os, p0.x, p1.x); split2_pair(x.z, x.w, os, p0.y, p1.y);
+          __half* o = ep.out_p + (long)r * 2 * ep.out_ldp + pl_off(col);
+          *reinterpret_cast<uint2*>(o) = p0; *reinterpret_cast<uint2*>(o + PL_LO) = p1;
+          if (ep.c_last && r % ep.last_T == ep.last_T - 1) *reinterpret_cast<float4*>(ep.c_last + (long)(r / ep.last_T) * ep.N + col) = x;
+          csum.x += x.x; csum.y += x.y; csum.z += x.z; csum.w += x.w;
+        }
       }
+      if (ep.rowsum32) {
+        // the consumer of a plane output's token sums (the weight gradient of the layer below) gets them from here instead of
+        // re-reading the planes: this lane's rows, then the four lanes that share its columns, in a fixed order
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+          csum.x += __shfl_xor_sync(0xffffffffu, csum.x, o); csum.y += __shfl_xor_sync(0xffffffffu, csum.y, o);
+          csum.z += __shfl_xor_sync(0xffffffffu, csum.z, o); csum.w += __shfl_xor_sync(0xffffffffu, csum.w, o);
+        }
+        if (rl == 0 && col_ok && rbase < ep.M) *reinterpret_cast<float4*>(ep.rowsum32 + (long)(rbase >> 5) * ep.N + col) = csum;
+      }
+    }
+    __syncwarp();
+    return;
+  }
+  float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
+  const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
+  if (ep.flags & TC_FLAG_VEC) {
+#pragma unroll 1
+    for (int cc = 0; cc < nch; cc++) {
+      const int c = chalf * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
+      if (n0 + c * 32 >= ep.N) break;
+      float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
+      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + BN / 2 + cc * 32 + c4);
+#pragma unroll 1
+      for (int hh = 0; hh < 2; hh++) {
+        const int r0 = rbase + 16 * hh + rl;
+        float4 rv[4];                                                        // residual, fetched before the exchange so that its latency overlaps it
+#pragma unroll
+        for (int t = 0; t < 4; t++) rv[t] = (R && col_ok && r0 + 4 * t < ep.M) ? *reinterpret_cast<const float4*>(R + (long)(r0 + 4 * t) * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        tc_stage_rows(stg, v, lane, hh);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const int r = r0 + 4 * t;
+          const float4 a = *reinterpret_cast<const float4*>(stg + (4 * t + rl) * TC_STG_LD + c4);
+          float4 x = make_float4(a.x * sv.x + bv.x + rv[t].x, a.y * sv.y + bv.y + rv[t].y, a.z * sv.z + bv.z + rv[t].z, a.w * sv.w + bv.w + rv[t].w);
+          if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
+          if (!col_ok || r >= ep.M) continue;
+          if (ep.mask) {
+            const float4 mv = *reinterpret_cast<const float4*>(ep.mask + (long)(r / ep.mask_group) * ep.mask_ld + col);
+            if (!(mv.x > 0.f)) x.x = 0.f; if (!(mv.y > 0.f)) x.y = 0.f; if (!(mv.z > 0.f)) x.z = 0.f; if (!(mv.w > 0.f)) x.w = 0.f;
+          }
+          *reinterpret_cast<float4*>(C + (long)r * ep.ldc + col) = x;
+        }
+      }
+    }
+    __syncwarp();
+    return;
+  }
+  // scalar path (unaligned operands, NCHW store): one output row per thread
+  const bool row_ok = row < ep.M;
+  const float* isb = ep.isb + (long)z * ep.N;
+  const float* Rrow = (R && row_ok) ? R + (long)row * ep.ldr : nullptr;
+  const float* Mrow = (ep.mask && row_ok) ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
+  float* Crow = ep.nchw_P > 0 ? C + (long)(row / ep.nchw_P) * ep.N * ep.nchw_P + row % ep.nchw_P : C + (long)row * ep.ldc;
+  const long cstep = ep.nchw_P > 0 ? ep.nchw_P : 1;
+#pragma unroll 1
+  for (int cc = 0; cc < nch; cc++) {
+    const int col0 = n0 + (chalf * nch + cc) * 32;
+    if (col0 >= ep.N) break;
+    float v[32]; tc_acc_chunk<MERGED>(tquad + (chalf * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
+#pragma unroll
+    for (int j = 0; j < 32; j++) {
+      const int col = col0 + j;
+      if (!row_ok || col >= ep.N) continue;
+      float x = v[j] * isb[col];
+      if (ep.bias) x += ep.bias[col];
+      if (Rrow) x += Rrow[col];
+      if (ep.act == GN_ACT_RELU) x = fmaxf(x, 0.f);
+      if (Mrow && !(Mrow[col] > 0.f)) x = 0.f;
+      Crow[col * cstep] = x;
     }
   }
+}
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
-                       const __grid_constant__ CUtensorMap mapB0, const __grid_constant__ CUtensorMap mapB1,
-                       TcParams ep, int tiles_m, int tiles_n, int total_tiles, int full_end, int n_half, int* tile_queue) {
+gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ TcParams ep, int tiles_m, int tiles_n, int total_tiles, int full_end, int n_half, int* tile_queue) {
   using Cfg = TcCfg<BN>;
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES, BK = TC_BK;
   constexpr bool MERGED = Cfg::MERGED;
@@ -351,12 +389,14 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_c
   float* colv_all = (float*)(smem + STAGES * STAGE_BYTES + 256);   // epilogue warps' column factors
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
   const uint32_t drain = smem_u32(bars + 2 * STAGES + 4);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // stage layout: A plane 0 | A plane 1 | B plane 0 | B plane 1
-  constexpr uint32_t OFF_A1 = Cfg::A_PL, OFF_B0 = 2 * Cfg::A_PL, OFF_B1 = OFF_B0 + Cfg::B_PL;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp-uniform for the compiler, too)
+  const uint32_t smem0 = smem_u32(smem);
+  constexpr uint32_t OFF_B = Cfg::A_BYTES;                         // stage layout: A | B, rows of hi 32 | lo 32
   const unsigned limit = ep.spin_limit;
 
   if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
     for (int s = 0; s < STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
     for (int b = 0; b < 2; b++) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, TC_EPI_WARPS); }
     mbar_init(drain, 1);
@@ -392,19 +432,19 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_c
   auto work = [&](int k, int& tile, int& half) -> bool {
     if (!queued) return item((long)blockIdx.x + (long)k * gridDim.x, tile, half);
     const uint32_t qs = (uint32_t)k & 3, qu = (uint32_t)k >> 2; int t = -1;
-    if (warp == 0) {                                      // producer thread: draw and publish
-      if (qu > 0 && !mbar_wait(qempty0 + 8 * qs, (qu - 1) & 1, limit, abort_flag)) { if (!*abort_flag) give_up(4); return false; }
-      t = atomicAdd(tile_queue, 1);
-      if ((long)t >= (long)full_end + n_half) t = -1;
-      qitem[qs] = t;
-      mbar_arrive(qfull0 + 8 * qs);
-    } else {                                              // consumers: one thread per warp reads
-      if (lane == 0) {
-        if (mbar_wait(qfull0 + 8 * qs, qu & 1, limit, abort_flag)) { t = qitem[qs]; mbar_arrive(qempty0 + 8 * qs); }
-        else if (!*abort_flag) give_up(5);
-      }
-      if (warp >= 2) t = __shfl_sync(0xffffffffu, t, 0);
+    if (lane == 0) {
+      if (warp == 0) {                                    // producer: draw and publish
+        if (qu > 0 && !mbar_wait(qempty0 + 8 * qs, (qu - 1) & 1, limit, abort_flag)) { if (!*abort_flag) give_up(4); t = -2; }
+        else {
+          t = atomicAdd(tile_queue, 1);
+          if ((long)t >= (long)full_end + n_half) t = -1;
+          qitem[qs] = t;
+          mbar_arrive(qfull0 + 8 * qs);
+        }
+      } else if (mbar_wait(qfull0 + 8 * qs, qu & 1, limit, abort_flag)) { t = qitem[qs]; mbar_arrive(qempty0 + 8 * qs); }      // consumers: one thread per warp reads
+      else if (!*abort_flag) give_up(5);
     }
+    t = __shfl_sync(0xffffffffu, t, 0);
     return t >= 0 && item(t, tile, half);
   };
   // tile -> coordinates and contraction range
@@ -419,77 +459,77 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_c
     return true;
   };
 
-  uint32_t issued = 0;          // producer thread: stages whose copies it has started
+  // The producer and the MMA warp run their loops with all lanes and issue from one elected lane: the loop state then lives in
+  // uniform registers.  With `if (lane == 0)` around the loops every MMA took its issuing thread 70 cycles (descriptors moved to
+  // uniform registers one word at a time) and every stage 400 more, 820 cycles per stage whatever the tile's width.
+  uint32_t issued = 0;          // producer: stages whose copies it has started
+  const bool elected = elect_one();
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true; uint32_t it = 0;
-      int tile, half;
-      for (int w = 0; ok && work(w, tile, half); w++) {
-        int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
-        for (int i = 0; i < nkb; i++, it++) {
-          const uint32_t s = it % STAGES, use = it / STAGES; const int kc = (kb0 + i) * BK;
-          if (use > 0 && !mbar_wait(empty0 + 8 * s, (use - 1) & 1, limit, abort_flag)) { ok = false; break; }
-          const uint32_t base = smem_u32(smem + s * STAGE_BYTES), bar = full0 + 8 * s;
-          mbar_expect_tx(bar, half < 0 ? STAGE_BYTES : STAGE_BYTES - Cfg::B_PL);
-          tma_load_3d(base, &mapA0, kc, m0, z, bar);
-          tma_load_3d(base + OFF_A1, &mapA1, kc, m0, z, bar);
-          tma_load_3d(base + OFF_B0, &mapB0, kc, n0, z, bar);          // the B copies are BN / 2 rows each
-          tma_load_3d(base + OFF_B1, &mapB1, kc, n0, z, bar);
-          if (half < 0) {
-            tma_load_3d(base + OFF_B0 + Cfg::B_PL / 2, &mapB0, kc, n0 + BN / 2, z, bar);
-            tma_load_3d(base + OFF_B1 + Cfg::B_PL / 2, &mapB1, kc, n0 + BN / 2, z, bar);
-          }
+    bool ok = true; uint32_t s = 0, ph = 0;                   // next stage and the parity of its previous use
+    int tile, half;
+    for (int w = 0; ok && work(w, tile, half); w++) {
+      int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
+      for (int i = 0; i < nkb; i++) {
+        const int kc = 2 * (kb0 + i) * BK;
+        if (issued >= (uint32_t)STAGES && !mbar_wait(empty0 + 8 * s, ph ^ 1, limit, abort_flag)) { ok = false; break; }
+        if (elected) {
+          const uint32_t base = smem0 + s * STAGE_BYTES, bar = full0 + 8 * s;
+          mbar_expect_tx(bar, half < 0 ? STAGE_BYTES : STAGE_BYTES - Cfg::B_BYTES / 2);
+          tma_load_3d(base, &mapA, kc, m0, z, bar);
+          tma_load_3d(base + OFF_B, &mapB, kc, n0, z, bar);        // the B copies are BN / 2 rows each
+          if (half < 0) tma_load_3d(base + OFF_B + Cfg::B_BYTES / 2, &mapB, kc, n0 + BN / 2, z, bar);
         }
+        issued++;
+        if (++s == STAGES) { s = 0; ph ^= 1; }
       }
-      if (!ok && !*abort_flag) give_up(1);
-      issued = it;
     }
+    if (!ok && !*abort_flag) give_up(1);
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = true; uint32_t it = 0, lt = 0;
-      constexpr uint32_t idesc_full = make_idesc_f16(TC_BM, BN), idesc_half = make_idesc_f16(TC_BM, BN / 2);
-      int tile, half;
-      for (int w = 0; ok && work(w, tile, half); w++) {
-        int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
-        const uint32_t idesc = half < 0 ? idesc_full : idesc_half;
-        const uint32_t slot = lt & 1, u = lt >> 1; lt++;
-        if (!mbar_wait(tempty0 + 8 * slot, (u & 1) ^ 1, limit, abort_flag)) { ok = false; break; }     // slot drained by the epilogue (passes at once the first time)
+    bool ok = true; uint32_t s = 0, ph = 0, lt = 0;
+    constexpr uint32_t idesc_full = make_idesc_f16(TC_BM, BN), idesc_half = make_idesc_f16(TC_BM, BN / 2);
+    const uint64_t desc0 = make_desc<32>(smem0);
+    int tile, half;
+    for (int w = 0; ok && work(w, tile, half); w++) {
+      int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
+      const uint32_t idesc = half < 0 ? idesc_full : idesc_half;
+      const uint32_t slot = lt & 1, u = lt >> 1; lt++;
+      if (!mbar_wait(tempty0 + 8 * slot, (u & 1) ^ 1, limit, abort_flag)) { ok = false; break; }     // slot drained by the epilogue (passes at once the first time)
+      tc_fence_after();
+      const uint32_t acc_main = tmem_base + slot * SLOT_COLS, acc_cross = MERGED ? acc_main : acc_main + BN;
+      for (int i = 0; i < nkb; i++) {
+        if (!mbar_wait(full0 + 8 * s, ph, limit, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t acc_main = tmem_base + slot * SLOT_COLS, acc_cross = MERGED ? acc_main : acc_main + BN;
-        for (int i = 0; i < nkb; i++, it++) {
-          const uint32_t s = it % STAGES, use = it / STAGES;
-          if (!mbar_wait(full0 + 8 * s, use & 1, limit, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t base = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t a0 = make_desc<16>(base), a1 = make_desc<16>(base + OFF_A1), b0 = make_desc<16>(base + OFF_B0), b1 = make_desc<16>(base + OFF_B1);
+        if (elected) {
+          const uint64_t a0 = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), b0 = a0 + (OFF_B >> 4), a1 = a0 + 4, b1 = b0 + 4;      // the low parts lie 64 bytes along the row
 #pragma unroll
           for (int k = 0; k < 2; k++) {                      // 16 contraction indices = 32 bytes per instruction
             const uint64_t adv = (uint64_t)(2 * k);
             if constexpr (MERGED) {
               // small terms first, so that they meet the accumulator before the large term of this group is added
               tc_mma_f16(acc_main, a1 + adv, b0 + adv, idesc, (i > 0 || k > 0) ? 1u : 0u);
-              tc_mma_f16(acc_main, a0 + adv, b1 + adv, idesc, 1u);
-              tc_mma_f16(acc_main, a0 + adv, b0 + adv, idesc, 1u);
+              tc_mma_f16_same_a(acc_main, acc_main, a0 + adv, b1 + adv, b0 + adv, idesc, 1u, 1u);
             } else {
               tc_mma_f16(acc_cross, a1 + adv, b0 + adv, idesc, (i > 0 || k > 0) ? 1u : 0u);
-              tc_mma_f16(acc_cross, a0 + adv, b1 + adv, idesc, 1u);
-              tc_mma_f16(acc_main, a0 + adv, b0 + adv, idesc, (i > 0 || k > 0) ? 1u : 0u);
+              tc_mma_f16_same_a(acc_cross, acc_main, a0 + adv, b1 + adv, b0 + adv, idesc, 1u, (i > 0 || k > 0) ? 1u : 0u);
             }
           }
           tc_commit(empty0 + 8 * s);
+          if (i == nkb - 1) tc_commit(tfull0 + 8 * slot);
         }
-        if (ok) tc_commit(tfull0 + 8 * slot);
+        if (++s == STAGES) { s = 0; ph ^= 1; }
       }
-      if (!ok) {
-        if (!*abort_flag) give_up(2);
-        tc_commit(drain);                                   // own instructions in flight must finish before TMEM is released
-        mbar_wait(drain, 0, TC_DRAIN_LIMIT);
-      }
+      if (ok && nkb == 0 && elected) tc_commit(tfull0 + 8 * slot);
     }
+    if (!ok) {
+      if (!*abort_flag) give_up(2);
+      if (elected) { tc_commit(drain); mbar_wait(drain, 0, TC_DRAIN_LIMIT); }      // own instructions in flight must finish before TMEM is released
+    }
+    __syncwarp();
   } else {
     const int quad = warp & 3, chalf = (warp - 2) >> 2; uint32_t lt = 0;
     float* colv = colv_all + (warp - 2) * BN;
-    float* stg = colv_all + Cfg::COLV_FLOATS + (warp - 2) * 32 * TC_STG_LD;
+    float* stg = colv_all + Cfg::COLV_FLOATS + (warp - 2) * 16 * TC_STG_LD;
     int tile, half;
     for (int w = 0; work(w, tile, half); w++) {
       int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
@@ -510,7 +550,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (threadIdx.x == 0 && *abort_flag) {
+  if (warp == 0 && elected && *abort_flag) {
     // a wait gave up somewhere in this CTA: the producer's last copies may still be in flight and nobody consumes
     // them any more; the CTA must not exit (and hand its shared memory on) before they have landed
     const uint32_t n_back = issued < (uint32_t)STAGES ? issued : (uint32_t)STAGES;
@@ -523,12 +563,12 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_c
 // Batched, strided split: planes[z][r][c] (row stride ldp, c < ldp, zero beyond cols) of the source element
 // (z, r, c) at p + (z / batch2) * b1 + (z % batch2) * b2 + r * s_r + c * s_c.  One of s_r, s_c is 1:
 // s_c == 1 reads rows directly; s_r == 1 (the operand is the transpose of what is stored) goes through a shared tile.
-// Two fp16 planes per operand, p0 = fp16(x s), p1 = fp16(x s - p0), and the inverse 1/s of every plane row's scale.
+// Two fp16 planes per operand, fp16(x s) and fp16(x s - fp16(x s)), interleaved (pl_off), and the inverse 1/s of every plane row's scale.
 struct TcSrc { const float* p; long s_r, s_c, b1, b2; int batch2; };
 // One warp per plane row: first the row's largest magnitude (the row is read a second time from L1 / L2 afterwards),
 // then eight elements per lane and step (two 16-byte loads, one 16-byte store per plane).  blockIdx.y = problem index.
 // `rownorm` (may be null): receives the L2 norm of every row (a factor of the bound of a plane-output contraction).
-__global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int cols, __half* __restrict__ p0, __half* __restrict__ p1, float* __restrict__ inv_scale, int ldp,
+__global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int cols, __half* __restrict__ pl, float* __restrict__ inv_scale, int ldp,
                                                           float* __restrict__ rownorm) {
   const int z = blockIdx.y, lane = threadIdx.x & 31;
   const long r = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -547,7 +587,7 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int
   if (rownorm) { sq = warp_sum(sq); if (lane == 0) rownorm[(long)z * rows + r] = sqrtf(sq) * 1.0001f; }
   float inv; const float sc = row_scale(mx, &inv);
   if (lane == 0) inv_scale[(long)z * rows + r] = inv;
-  const long o = ((long)z * rows + r) * ldp;
+  __half* o = pl + ((long)z * rows + r) * 2 * ldp;
   for (int c = lane * 8; c < ldp; c += 256) {
     float t[8];
     if (c + 7 < cols8) {
@@ -560,8 +600,8 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int
     uint4 a, b;
     split2_pair(t[0], t[1], sc, a.x, b.x); split2_pair(t[2], t[3], sc, a.y, b.y);
     split2_pair(t[4], t[5], sc, a.z, b.z); split2_pair(t[6], t[7], sc, a.w, b.w);
-    *reinterpret_cast<uint4*>(p0 + o + c) = a;
-    *reinterpret_cast<uint4*>(p1 + o + c) = b;
+    *reinterpret_cast<uint4*>(o + pl_off(c)) = a;
+    *reinterpret_cast<uint4*>(o + pl_off(c) + PL_LO) = b;
   }
 }
 // Largest magnitude of every plane row of a transposed operand (= of every column of the stored matrix): a block covers
@@ -583,7 +623,7 @@ __global__ void __launch_bounds__(256) colmax_kernel(TcSrc s, int rows, int cols
 }
 // Transposing split: 64 x 64 source tile through shared memory; reads run along the source's fast index (r), each
 // thread then writes two neighbouring contraction indices of one plane row as one 4-byte word.  `mx` = colmax_kernel's result.
-__global__ void __launch_bounds__(256) split2_cols_kernel(TcSrc s, int rows, int cols, __half* __restrict__ p0, __half* __restrict__ p1, const int* __restrict__ mx,
+__global__ void __launch_bounds__(256) split2_cols_kernel(TcSrc s, int rows, int cols, __half* __restrict__ pl, const int* __restrict__ mx,
                                                           float* __restrict__ inv_scale, int ldp) {
   __shared__ float t[64][65];
   const int z = blockIdx.z, c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
@@ -591,7 +631,7 @@ __global__ void __launch_bounds__(256) split2_cols_kernel(TcSrc s, int rows, int
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
   for (int j = ty; j < 64; j += 4) { const int c = c0 + j, r = r0 + tx; t[j][tx] = (r < rows && c < cols) ? src[r + (long)c * s.s_c] : 0.f; }
   __syncthreads();
-  const long zo = (long)z * rows * ldp;
+  const long zo = (long)z * rows * 2 * ldp;
   const int cx = (threadIdx.x & 31) * 2, ry = threadIdx.x >> 5;
   for (int j = ry; j < 64; j += 8) {
     const int r = r0 + j, c = c0 + cx;
@@ -599,8 +639,8 @@ __global__ void __launch_bounds__(256) split2_cols_kernel(TcSrc s, int rows, int
       float inv; const float sc = row_scale(__int_as_float(mx[(long)z * rows + r]), &inv);
       if (c == 0) inv_scale[(long)z * rows + r] = inv;
       uint32_t a, b; split2_pair(t[cx][j], t[cx + 1][j], sc, a, b);
-      const long o = zo + (long)r * ldp + c;
-      *reinterpret_cast<uint32_t*>(p0 + o) = a; *reinterpret_cast<uint32_t*>(p1 + o) = b;
+      __half* o = pl + zo + (long)r * 2 * ldp + pl_off(c);
+      *reinterpret_cast<uint32_t*>(o) = a; *reinterpret_cast<uint32_t*>(o + PL_LO) = b;
     }
   }
 }
@@ -609,14 +649,9 @@ __global__ void __launch_bounds__(256) split2_cols_kernel(TcSrc s, int rows, int
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                     CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// Operand planes of the contraction engine: two fp16 planes [nbatch][rows][ldp] in one buffer, plane 1 after plane 0, and
-// the inverse scale of every plane row [nbatch][rows].
-struct BfPlanes {
-  __half* base; float* inv_scale; int rows, K, ldp, nbatch; int koff = 0;
-  size_t plane_elems() const { return (size_t)nbatch * rows * ldp; }
-  __half* p0() const { return base; }
-  __half* p1() const { return base + plane_elems(); }
-};
+// Operand planes of the contraction engine: two interleaved fp16 planes [nbatch][rows][2 ldp] (pl_off; ldp a multiple of 32, zero
+// beyond K), and the inverse scale of every plane row [nbatch][rows].  koff (a multiple of 32): first contraction index used.
+struct BfPlanes { __half* base; float* inv_scale; int rows, K, ldp, nbatch; int koff = 0; };
 // Where a contraction's result goes when it is only ever used as the A operand of another contraction (the FFN's hidden
 // activation and its gradient: half of all operand elements of a TransformerBlock).  A row's scale must be known before
 // its first element is written, and a tile sees only 256 of the row's columns, so the scale comes from a bound instead of
@@ -625,7 +660,7 @@ struct BfPlanes {
 // be exceeded, so the fp16 planes cannot overflow.  `last`: fp32 copy of every sequence's last row (the only rows of
 // these tensors that are read as numbers: ReLU gate and weight-gradient input of the reference's last-token rule).
 struct TcPlaneOut { BfPlanes planes; const int* b_maxabs; float* last; int last_T; float* rowsum32 = nullptr; };
-inline int tc_ldp(int K) { return ((K + 7) / 8) * 8; }              // plane row stride: a multiple of 16 bytes for TMA
+inline int tc_ldp(int K) { return ((K + 31) / 32) * 32; }           // plane row length: whole blocks of 32
 inline size_t bf_plane_floats(long nbatch, long rows, long ldp) { return (size_t)nbatch * rows * ldp; }   // two fp16 planes = one float per element
 
 // Per-context operand-plane scratch of the contraction engine (calls on a context are serialised by Ctx::run_mu).
@@ -666,20 +701,20 @@ inline void tc_init(Ctx* ctx) {
   }
 }
 
-// 16-bit plane [nbatch][rows][ldp], K valid columns from column koff, box_cols columns x box_rows per copy: 32 columns = 64
-// bytes with the 64-byte swizzle (contraction engine), 64 columns = 128 bytes with the 128-byte swizzle (attention tiles)
-inline int tc_make_map_bf16_raw(Ctx* ctx, CUtensorMap* map, const void* base_v, int K, int rows, int ldp, int nbatch, int koff, int box_rows, int box_cols,
-                                CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
-  const uint16_t* base = static_cast<const uint16_t*>(base_v);
-  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)nbatch};
-  cuuint64_t strides[2] = {(cuuint64_t)ldp * 2, (cuuint64_t)rows * ldp * 2};
-  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+// 16-bit plane [nbatch][rows][ld], `cols` valid columns, 64 columns (128 bytes, 128-byte swizzle) x box_rows per copy
+inline int tc_make_map_f16(Ctx* ctx, CUtensorMap* map, const __half* base, int cols, int rows, long ld, int nbatch, int box_rows) {
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)nbatch};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * ld * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = ((PFN_encodeTiled)ctx->encode_tiled)(map, dtype, 3, (void*)(base + koff), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                                    box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(GN_ERR_CUDA, "cuTensorMapEncodeTiled (16-bit) failed with %d (rows %d K %d ld %d batch %d)", (int)r, rows, K, ldp, nbatch);
+  CUresult r = ((PFN_encodeTiled)ctx->encode_tiled)(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(GN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (rows %d columns %d ld %ld batch %d)", (int)r, rows, cols, ld, nbatch);
   return GN_OK;
+}
+// ... of a contraction operand: the interleaved blocks of K contraction indices from koff on
+inline int tc_operand_map(Ctx* ctx, CUtensorMap* map, const BfPlanes& p, int box_rows) {
+  return tc_make_map_f16(ctx, map, p.base + 2 * (long)p.koff, 2 * tc_ldp(p.K), p.rows, 2L * p.ldp, p.nbatch, box_rows);
 }
 
 // Writes the planes and inverse row scales of an operand.  `mx` (only used by the transposing variant): nbatch * rows ints.
@@ -687,13 +722,13 @@ inline int tc_split(Ctx* ctx, const TcSrc& src, const BfPlanes& p, int* mx, floa
   if (rownorm && src.s_c != 1) return fail(GN_ERR_UNSUPPORTED, "tc_split: row norms are only formed by the row-wise split");
   if (src.s_c == 1) {
     if (p.nbatch > 65535) return fail(GN_ERR_UNSUPPORTED, "tc_split: more than 65535 problems in a batch");
-    GN_LAUNCH(ctx, split2_rows_kernel, dim3(cdiv(p.rows, 8), p.nbatch), 256, 0, src, p.rows, p.K, p.p0(), p.p1(), p.inv_scale, p.ldp, rownorm);
+    GN_LAUNCH(ctx, split2_rows_kernel, dim3(cdiv(p.rows, 8), p.nbatch), 256, 0, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, rownorm);
   } else if (src.s_r == 1) {
     if (p.nbatch > 65535 || cdiv(p.rows, 64) > 65535 || cdiv(p.K, 256) > 65535) return fail(GN_ERR_UNSUPPORTED, "tc_split: operand too large for the transposing split");
     if (!mx) return fail(GN_ERR_INVALID_ARG, "tc_split: the transposing split needs a row-maximum buffer");
     GN_CUDA(cudaMemsetAsync(mx, 0, (size_t)p.nbatch * p.rows * sizeof(int), ctx->stream));
     GN_LAUNCH(ctx, colmax_kernel, dim3(cdiv(p.rows, 64), cdiv(p.K, 256), p.nbatch), 256, 0, src, p.rows, p.K, mx);
-    GN_LAUNCH(ctx, split2_cols_kernel, dim3(cdiv(p.ldp, 64), cdiv(p.rows, 64), p.nbatch), 256, 0, src, p.rows, p.K, p.p0(), p.p1(), (const int*)mx, p.inv_scale, p.ldp);
+    GN_LAUNCH(ctx, split2_cols_kernel, dim3(cdiv(p.ldp, 64), cdiv(p.rows, 64), p.nbatch), 256, 0, src, p.rows, p.K, p.base, (const int*)mx, p.inv_scale, p.ldp);
   } else return fail(GN_ERR_UNSUPPORTED, "tc_split: neither stride of the operand is 1");
   ctx->split_bytes += 8.0 * (double)p.nbatch * p.rows * p.K;
   return check_launch("tc_split");
@@ -718,11 +753,9 @@ inline int tc_next_queue(Ctx* ctx, int** out) {
 }
 template <int BN>
 inline int tc_launch_persist(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams& ep) {
-  CUtensorMap mA0, mA1, mB0, mB1;
-  constexpr CUtensorMapDataType F16 = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  GN_TRY(tc_make_map_bf16_raw(ctx, &mA0, A.p0(), A.K, A.rows, A.ldp, A.nbatch, A.koff, TC_BM, TC_BK, F16)); GN_TRY(tc_make_map_bf16_raw(ctx, &mA1, A.p1(), A.K, A.rows, A.ldp, A.nbatch, A.koff, TC_BM, TC_BK, F16));
+  CUtensorMap mA, mB;
   // the B tile of a stage arrives as two copies of BN / 2 rows, so that a half tile (see the kernel's work list) is one of them
-  GN_TRY(tc_make_map_bf16_raw(ctx, &mB0, B.p0(), B.K, B.rows, B.ldp, B.nbatch, B.koff, BN / 2, TC_BK, F16)); GN_TRY(tc_make_map_bf16_raw(ctx, &mB1, B.p1(), B.K, B.rows, B.ldp, B.nbatch, B.koff, BN / 2, TC_BK, F16));
+  GN_TRY(tc_operand_map(ctx, &mA, A, TC_BM)); GN_TRY(tc_operand_map(ctx, &mB, B, BN / 2));
   const int tiles_m = cdiv(ep.M, TC_BM), tiles_n = cdiv(ep.N, BN); const long total = (long)tiles_m * tiles_n * A.nbatch;
   if (total > 0x7fffffffL) return fail(GN_ERR_UNSUPPORTED, "too many output tiles");
   const unsigned grid = (unsigned)std::min<long>(total, persist_sms(ctx));
@@ -731,7 +764,7 @@ inline int tc_launch_persist(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, con
   int* queue = nullptr;
   if (ctx->tc_tile_queue && total > grid) GN_TRY(tc_next_queue(ctx, &queue));
   ProfScope prof(ctx);
-  GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN>), grid, TC_THREADS, (TcCfg<BN>::SMEM_BYTES), mA0, mA1, mB0, mB1, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN>), grid, TC_THREADS, (TcCfg<BN>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
   return check_launch("gemm_tc_persist");
 }
 // Output tile width for a problem: 64 for narrow outputs; 256 (three quarters of the shared-memory traffic per MMA
@@ -758,7 +791,7 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
   if (ep.R) vec = vec && ep.ldr % 4 == 0 && ep.r_b1 % 4 == 0 && ep.r_b2 % 4 == 0 && a16(ep.R);
   if (ep.mask) vec = vec && ep.mask_ld % 4 == 0 && a16(ep.mask);
   if (ep.nchw_P > 0) { if (ep.R || A.nbatch != 1) return fail(GN_ERR_UNSUPPORTED, "tc_launch: NCHW store with a residual or a batch"); vec = false; }
-  if (ep.out_p0) {
+  if (ep.out_p) {
     if (!(ep.N % 4 == 0 && (!ep.bias || a16(ep.bias)) && a16(ep.isb) && (!ep.mask || (ep.mask_ld % 4 == 0 && a16(ep.mask))) && ep.out_ldp % 4 == 0 && (!ep.c_last || a16(ep.c_last))))
       return fail(GN_ERR_INVALID_ARG, "tc_launch: plane output needs 16-byte aligned operands");
     vec = true;
@@ -781,7 +814,7 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
 inline int tc_run_rows(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams& ep, int bn) {
   const int kslice = ctx->tc_kslice > 0 ? ctx->tc_kslice : (bn == 256 ? 2048 : 4096);
   if (ep.K <= kslice || (ep.flags & (GEMM_KBEG_AT_M0 | GEMM_KEND_AT_M0))) return tc_launch(ctx, A, B, ep, bn);
-  if (ep.out_p0) return fail(GN_ERR_UNSUPPORTED, "a contraction that writes operand planes must fit one accumulator run (K = %d)", ep.K);
+  if (ep.out_p) return fail(GN_ERR_UNSUPPORTED, "a contraction that writes operand planes must fit one accumulator run (K = %d)", ep.K);
   for (int k0 = 0; k0 < ep.K; k0 += kslice) {
     const int kl = std::min(kslice, ep.K - k0); const bool first = k0 == 0, last = k0 + kl >= ep.K;
     BfPlanes As = A, Bs = B; As.koff = A.koff + k0; As.K = kl; Bs.koff = B.koff + k0; Bs.K = kl;
@@ -805,7 +838,7 @@ inline int tc_run(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams
 // GPUs.  Instead all registered matrices are split once per parameter update, both orientations from one read, by two
 // launches in all: the matrices get ONE power-of-two scale each (their entries are of similar size, unlike activation
 // rows), found by wplanes_max_kernel, and wplanes_split_kernel writes every 64 x 64 tile as stored and transposed.
-struct WPlaneJob { const float* src; const float* bias; int out, in, ldp_r, ldp_c; __half *r0, *r1, *c0, *c1; float *inv_r, *inv_c; int tile0, tiles_in; };
+struct WPlaneJob { const float* src; const float* bias; int out, in, ldp_r, ldp_c; __half *r, *c; float *inv_r, *inv_c; int tile0, tiles_in; };
 __device__ __forceinline__ int wplane_find(const WPlaneJob* jobs, int njobs, int tile) {
   int lo = 0, hi = njobs - 1;
   while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (jobs[mid].tile0 <= tile) lo = mid; else hi = mid - 1; }
@@ -835,8 +868,8 @@ __global__ void __launch_bounds__(256) wplanes_split_kernel(const WPlaneJob* __r
     const int r = r0 + rr, c = c0 + x2;
     if (r < jb.out && c < jb.in) {                            // (in is even-padded by ldp_r; an odd last column writes its zero neighbour)
       uint32_t a, b; split2_pair(tl[rr][x2], tl[rr][x2 + 1], sc, a, b);
-      const long o = (long)r * jb.ldp_r + c;
-      *reinterpret_cast<uint32_t*>(jb.r0 + o) = a; *reinterpret_cast<uint32_t*>(jb.r1 + o) = b;
+      __half* o = jb.r + (long)r * 2 * jb.ldp_r + pl_off(c);
+      *reinterpret_cast<uint32_t*>(o) = a; *reinterpret_cast<uint32_t*>(o + PL_LO) = b;
     }
     if (c0 == 0 && x2 == 0 && r < jb.out) jb.inv_r[r] = inv;
   }
@@ -844,8 +877,8 @@ __global__ void __launch_bounds__(256) wplanes_split_kernel(const WPlaneJob* __r
     const int c = c0 + cc, r = r0 + x2;
     if (c < jb.in && r < jb.out) {
       uint32_t a, b; split2_pair(tl[x2][cc], tl[x2 + 1][cc], sc, a, b);
-      const long o = (long)c * jb.ldp_c + r;
-      *reinterpret_cast<uint32_t*>(jb.c0 + o) = a; *reinterpret_cast<uint32_t*>(jb.c1 + o) = b;
+      __half* o = jb.c + (long)c * 2 * jb.ldp_c + pl_off(r);
+      *reinterpret_cast<uint32_t*>(o) = a; *reinterpret_cast<uint32_t*>(o + PL_LO) = b;
     }
     if (r0 == 0 && x2 == 0 && c < jb.in) jb.inv_c[c] = inv;
   }
@@ -878,7 +911,7 @@ inline int wplanes_build(Ctx* ctx, WeightPlaneTable& t, const std::vector<Weight
     x.rows = BfPlanes{hp, sp, x.out, x.in, lr, 1}; hp += 2 * (size_t)x.out * lr; sp += (x.out + 3) & ~3;
     x.cols = BfPlanes{hp, sp, x.in, x.out, lc, 1}; hp += 2 * (size_t)x.in * lc; sp += (x.in + 3) & ~3;
     x.maxabs = reinterpret_cast<const int*>(t.mx.p) + jobs.size();
-    WPlaneJob jb{x.src, x.bias, x.out, x.in, lr, lc, x.rows.p0(), x.rows.p1(), x.cols.p0(), x.cols.p1(), x.rows.inv_scale, x.cols.inv_scale, tiles, (int)cdiv(x.in, 64)};
+    WPlaneJob jb{x.src, x.bias, x.out, x.in, lr, lc, x.rows.base, x.cols.base, x.rows.inv_scale, x.cols.inv_scale, tiles, (int)cdiv(x.in, 64)};
     x.tile0 = tiles; x.tiles = (int)cdiv(x.out, 64) * (int)cdiv(x.in, 64);
     tiles += x.tiles; jobs.push_back(jb);
   }
@@ -925,10 +958,12 @@ inline bool gemm_tc_supported(Ctx* ctx, const GemmDesc& g) {
   if (g.act != GN_ACT_LINEAR && g.act != GN_ACT_RELU) return false;
   return g.M > 0 && g.N > 0 && g.K > 0;
 }
-// Is it worth it?  Small or skinny problems stay on the SIMT engine.
+// Is it worth it?  Small or skinny problems stay on the CUDA-core engine, which needs no operand planes: 1e8 multiply-adds take it
+// about 8 us.  Products over many rows come here somewhat earlier: several of them share the planes of one input (Q, K and V).
 inline bool gemm_tc_eligible(Ctx* ctx, const GemmDesc& g) {
   if (!gemm_tc_supported(ctx, g)) return false;
-  return g.M >= 16 && g.N >= 32 && g.K >= 32 && (double)g.M * g.N * g.K * g.batch1 * g.batch2 >= 1.0e8;
+  const double work = (double)g.M * g.N * g.K * g.batch1 * g.batch2;
+  return g.M >= 16 && g.N >= 32 && g.K >= 32 && work >= (g.M >= 512 ? 6.0e7 : 1.0e8);
 }
 
 // General entry: splits both operands into the context's scratch planes, then runs the contraction.
@@ -958,7 +993,7 @@ inline int gemm_tc(Ctx* ctx, const GemmDesc& g) {
     const TcPlaneOut& po = *static_cast<const TcPlaneOut*>(g.plane_out);
     if (nb != 1 || g.R || !g.a_rownorm || !po.b_maxabs || g.N % 32 || po.planes.rows != g.M || po.planes.K != g.N || (g.flags & (GEMM_SKIP_UPPER | GEMM_KBEG_AT_M0 | GEMM_KEND_AT_M0)))
       return fail(GN_ERR_INVALID_ARG, "gemm_tc: this contraction cannot write its result as operand planes");
-    ep.out_p0 = po.planes.p0(); ep.out_p1 = po.planes.p1(); ep.out_inv = po.planes.inv_scale; ep.out_ldp = po.planes.ldp;
+    ep.out_p = po.planes.base; ep.out_inv = po.planes.inv_scale; ep.out_ldp = po.planes.ldp;
     ep.a_rownorm = g.a_rownorm; ep.b_maxabs = po.b_maxabs; ep.c_last = po.last; ep.last_T = po.last_T > 0 ? po.last_T : 1; ep.rowsum32 = po.rowsum32;
   }
   return tc_run(ctx, A, B, ep);

@@ -304,7 +304,7 @@ static int layernorm_forward(Ctx* ctx, const float* x, const float* gamma, const
                              const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
   const bool vec = n % 128 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15) == 0;
   const RowPlaneOut out = (po && vec && layernorm_vec_width(n)) ? *po : RowPlaneOut{};
-  if (emitted) *emitted = out.p0 != nullptr;
+  if (emitted) *emitted = out.p != nullptr;
   switch (vec ? n / 128 : 0) {
     case 1: GN_LAUNCH(ctx, layernorm_fwd_vec_kernel<1>, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, 1e-5f, out); break;
     case 2: GN_LAUNCH(ctx, layernorm_fwd_vec_kernel<2>, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, 1e-5f, out); break;
@@ -365,7 +365,7 @@ static bool norm_planes_wanted(Ctx* ctx, bool rms, int rows, int n, int consumer
 static int norm_planes_alloc(gn_model* m, int slotp, int sloti, int rows, int n, RowPlaneOut* po, BfPlanes* planes, float* rownorm) {
   float *pp, *pi; GN_TRY(ensure(m, slotp, (size_t)rows * n, &pp)); GN_TRY(ensure(m, sloti, (size_t)rows, &pi));
   *planes = BfPlanes{reinterpret_cast<__half*>(pp), pi, rows, n, n, 1};
-  *po = RowPlaneOut{planes->p0(), planes->p1(), pi, rownorm};
+  *po = RowPlaneOut{planes->base, pi, rownorm};
   return GN_OK;
 }
 
@@ -531,7 +531,7 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
   // norm 1 hands its output to ff1 as operand planes (and the row norms ff1's plane-writing epilogue needs)
   RowPlaneOut po1{}; BfPlanes n1p{}; bool n1_planes = false; float* rn1 = nullptr;
   if (norm_planes_wanted(ctx, l.rms, NE, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)NE, &rn1)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, NE, D, &po1, &n1p, rn1)); }
-  GN_TRY(block_norm_forward(ctx, l.rms, l.r1.p, bp.g1, bp.be1, l.n1.p, st, (long)NE, D, po1.p0 ? &po1 : nullptr, &n1_planes));
+  GN_TRY(block_norm_forward(ctx, l.rms, l.r1.p, bp.g1, bp.be1, l.n1.p, st, (long)NE, D, po1.p ? &po1 : nullptr, &n1_planes));
   {   // feed-forward: ff1 -> ff2, res2 = norm1 + ff
     GemmDesc g1; g1.M = NE; g1.N = F; g1.K = D; g1.A = l.n1.p; g1.sa_m = D; g1.sa_k = 1; g1.B = bp.w1; g1.sb_k = 1; g1.sb_n = D; g1.C = l.mid.p; g1.ldc = F; g1.bias = bp.b1;
     if (n1_planes) g1.a_planes = &n1p;
@@ -564,7 +564,7 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
     RowPlaneOut po2{}; BfPlanes outp{}; bool emitted = false;
     const bool next_is_block = !rows_only && li + 1 < m->L.size() && m->L[li + 1].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[li + 1].d.dim == D && m->L[li + 1].d.seq_len == T;
     if (next_is_block && norm_planes_wanted(ctx, l.rms, NE, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP1, S_LNI1, NE, D, &po2, &outp, nullptr));
-    GN_TRY(block_norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * NE, (long)NE, D, po2.p0 ? &po2 : nullptr, &emitted));
+    GN_TRY(block_norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * NE, (long)NE, D, po2.p ? &po2 : nullptr, &emitted));
     if (emitted) { m->fwd_planes = outp; m->fwd_planes_src = l.out.p; }
   }
   *out = l.out.p; return GN_OK;
@@ -703,7 +703,7 @@ static int layernorm_backward(gn_model* m, const float* g, const float* x, const
   Ctx* ctx = &m->ctx->c;
   const bool vec = n % 128 == 0 && ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
   const RowPlaneOut out = (po && vec && layernorm_vec_width(n)) ? *po : RowPlaneOut{};
-  if (emitted) *emitted = out.p0 != nullptr;
+  if (emitted) *emitted = out.p != nullptr;
   if (vec) {
     const int chunks = (int)std::max<long>(1, std::min<long>(rows / 32, 4L * ctx->sm_count));
     float* part; GN_TRY(ensure(m, S_PART2, (size_t)chunks * 2 * n, &part));
@@ -734,7 +734,7 @@ static int inner_dense_param_grads(gn_model* m, const float* dz, int B, int T, i
                                    const float* x_last = nullptr, const BfPlanes* dz_planes = nullptr, const float* dz_rowsum32 = nullptr) {
   Ctx* ctx = &m->ctx->c; float* delta; GN_TRY(ensure(m, S_DELTA, (size_t)B * out, &delta));
   if (dz_rowsum32) GN_LAUNCH(ctx, token_sum_part32_kernel, dim3(cdiv(out, 512), B), 128, 0, dz_rowsum32, T / 32, out, delta);
-  else if (dz_planes) GN_LAUNCH(ctx, token_sum_planes_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, (const __half*)dz_planes->p0(), (const __half*)dz_planes->p1(), (const float*)dz_planes->inv_scale, (long)dz_planes->ldp, T, out, delta);
+  else if (dz_planes) GN_LAUNCH(ctx, token_sum_planes_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, (const __half*)dz_planes->base, (const float*)dz_planes->inv_scale, (long)dz_planes->ldp, T, out, delta);
   else if (out % 4 == 0 && ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(delta)) & 15) == 0)
     GN_LAUNCH(ctx, token_sum_vec_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, dz, T, out, delta);
   else GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(out, 128), B), dim3(128, 4), 0, dz, T, out, delta);
@@ -769,7 +769,7 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   // its result goes to the contraction with W2 as operand planes, with the row norms that contraction's plane-writing epilogue needs
   RowPlaneOut pob{}; BfPlanes dR2p{}; bool dR2_planes = false; float* rnb = nullptr;
   if (norm_planes_wanted(ctx, l.rms, N, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)N, &rnb)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &pob, &dR2p, rnb)); }
-  GN_TRY(block_norm_backward(m, l.rms, gout, l.r2.p, bp.g2, st + 2 * N, dR2, (float*)gp.g2, (float*)gp.be2, (long)N, D, pob.p0 ? &pob : nullptr, &dR2_planes));
+  GN_TRY(block_norm_backward(m, l.rms, gout, l.r2.p, bp.g2, st + 2 * N, dR2, (float*)gp.g2, (float*)gp.be2, (long)N, D, pob.p ? &pob : nullptr, &dR2_planes));
   // ff2 then ff1, token by token in the reference (transformer.go:1238-1250)
   GN_TRY(inner_dense_param_grads(m, dR2, B, T, D, l.mid.p, F, (float*)gp.w2, (float*)gp.b2, l.mid_is_planes ? l.mid_last.p : nullptr));
   {
@@ -816,7 +816,7 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   // norm 1
   RowPlaneOut poa{}; BfPlanes dR1p{}; bool dR1_planes = false;
   if (norm_planes_wanted(ctx, l.rms, N, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &poa, &dR1p, nullptr));      // the planes of dR2 are dead by now
-  GN_TRY(block_norm_backward(m, l.rms, comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, (long)N, D, poa.p0 ? &poa : nullptr, &dR1_planes));
+  GN_TRY(block_norm_backward(m, l.rms, comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, (long)N, D, poa.p ? &poa : nullptr, &dR1_planes));
   // output projection
   GN_TRY(inner_dense_param_grads(m, dR1, B, T, D, l.att.p, D, (float*)gp.wo, (float*)gp.bo));
   {

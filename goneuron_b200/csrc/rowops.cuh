@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128) token_sum_part32_kernel(const float* __re
 }
 // The same sum over a tensor that exists only as operand planes (two fp16 planes and an inverse scale per row, written by a
 // contraction's epilogue): element = (p0 + p1) * inv_scale[row].  Same block shape as above: 4 columns per thread.
-__global__ void __launch_bounds__(256) token_sum_planes_kernel(const __half* __restrict__ p0, const __half* __restrict__ p1, const float* __restrict__ inv, long ldp,
+__global__ void __launch_bounds__(256) token_sum_planes_kernel(const __half* __restrict__ pl, const float* __restrict__ inv, long ldp,
                                                                int T, int C, float* __restrict__ out) {
   __shared__ float4 part[8][32];
   const int c = (blockIdx.x * 32 + threadIdx.x) * 4, grp = threadIdx.y;
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(256) token_sum_planes_kernel(const __half* __r
   if (c < C) {
     const long row0 = (long)blockIdx.y * T;
     for (int t = grp; t < T; t += 8) {
-      const long o = (row0 + t) * ldp + c; const float is = inv[row0 + t];
-      const uint2 a = *reinterpret_cast<const uint2*>(p0 + o), b = *reinterpret_cast<const uint2*>(p1 + o);
+      const __half* o = pl + (row0 + t) * 2 * ldp + pl_off(c); const float is = inv[row0 + t];
+      const uint2 a = *reinterpret_cast<const uint2*>(o), b = *reinterpret_cast<const uint2*>(o + PL_LO);
       const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&a.x)), a1 = __half22float2(*reinterpret_cast<const __half2*>(&a.y));
       const float2 b0 = __half22float2(*reinterpret_cast<const __half2*>(&b.x)), b1 = __half22float2(*reinterpret_cast<const __half2*>(&b.y));
       s.x += (a0.x + b0.x) * is; s.y += (a0.y + b0.y) * is; s.z += (a1.x + b1.x) * is; s.w += (a1.y + b1.y) * is;
@@ -267,10 +267,10 @@ __global__ void __launch_bounds__(1024) layernorm_pgrad_final_kernel(const float
 // Row-in-registers variants for n = 128 * NV (NV <= 16): one warp per row, the row is read once with 16-byte loads
 // and kept in registers between the reduction and the output pass.  Same arithmetic as the kernels above.
 // Optional second output of the row-in-registers kernels: the row as operand planes of the contraction engine (two fp16
-// planes with row stride n, the row's inverse scale, its 2-norm) -- the kernel holds the whole row, so the row maximum
+// planes interleaved in blocks of 32 columns, row length 2 n, the row's inverse scale, its 2-norm) -- the kernel holds the whole row, so the row maximum
 // and norm cost two warp reductions, and the separate split pass (a second read of the tensor) is not needed for the contraction that
 // consumes this output.
-struct RowPlaneOut { __half* p0 = nullptr; __half* p1 = nullptr; float* inv = nullptr; float* rownorm = nullptr; };
+struct RowPlaneOut { __half* p = nullptr; float* inv = nullptr; float* rownorm = nullptr; };
 template <int NV>
 __device__ __forceinline__ void row_planes_emit(const float4 (&o)[NV], long row, int lane, const RowPlaneOut& po) {
   constexpr int n = 128 * NV;
@@ -283,11 +283,11 @@ __device__ __forceinline__ void row_planes_emit(const float4 (&o)[NV], long row,
   mx = warp_max(mx); sq = warp_sum(sq);
   float inv; const float sc = row_scale(mx, &inv);
   if (lane == 0) { po.inv[row] = inv; if (po.rownorm) po.rownorm[row] = sqrtf(sq) * 1.0001f; }
-  uint2* h = reinterpret_cast<uint2*>(po.p0 + row * n) + lane; uint2* l = reinterpret_cast<uint2*>(po.p1 + row * n) + lane;
+  __half* h = po.p + row * 2 * n + pl_off(4 * lane);          // columns 4 lane + 128 k
 #pragma unroll
   for (int k = 0; k < NV; k++) {
     uint2 a, b; split2_pair(o[k].x, o[k].y, sc, a.x, b.x); split2_pair(o[k].z, o[k].w, sc, a.y, b.y);
-    h[32 * k] = a; l[32 * k] = b;
+    *reinterpret_cast<uint2*>(h + 256 * k) = a; *reinterpret_cast<uint2*>(h + 256 * k + PL_LO) = b;
   }
 }
 template <int NV>
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256) layernorm_fwd_vec_kernel(const float* __r
     yr[32 * k] = v[k];
   }
   if (lane == 0) { mean_out[row] = mean; std_out[row] = sd; }
-  if (po.p0) row_planes_emit<NV>(v, row, lane, po);
+  if (po.p) row_planes_emit<NV>(v, row, lane, po);
 }
 template <int NV>
 __global__ void __launch_bounds__(256) layernorm_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ gamma,
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_vec_kernel(const float* __r
                        (q[k].z - sgn) * isd - d[k].z * w, (q[k].w - sgn) * isd - d[k].w * w);
     dr[32 * k] = q[k];
   }
-  if (po.p0) row_planes_emit<NV>(q, row, lane, po);
+  if (po.p) row_planes_emit<NV>(q, row, lane, po);
 }
 // Partial column sums for gGamma / gBeta with 16-byte loads: block = 256 threads = up to 1024 columns, grid.x covers the
 // columns, grid.y the row chunks; part layout as in layernorm_pgrad_partial_kernel.

@@ -59,3 +59,25 @@ def test_static_scratch_gemm_matches_regular_entry_point_twice():
                 dev.free(p)
     finally:
         dev.close()
+
+
+def test_static_scratch_takes_every_size_of_the_documented_limit():
+    """(M + N) (roundup8(K) + 1) <= 4 Mi floats: plane rows are padded to blocks of 32, so with a short contraction one side of
+    such a product is walked in pieces."""
+    from goneuron_b200 import _lib
+    from goneuron_b200.sequential import Device
+    L = _lib.load()
+    dev = Device(0)
+    try:
+        for M, N, K in [(200_000, 12, 5), (24, 150_001, 9), (60_000, 7, 60)]:
+            rng = np.random.default_rng(M)
+            A, B = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+            dA, dB, dC = dev.alloc(A), dev.alloc(B), dev.alloc(np.zeros((M, N), np.float32))
+            _lib.check(L.gn_op_gemm_nt_static(dev.handle, M, N, K, dA, dB, None, dC))
+            out = np.empty((M, N), np.float32)
+            _lib.check(L.gn_device_download(dev.handle, _f(out), dC, out.size))
+            assert norm_err(out, A.astype(np.float64) @ B.astype(np.float64).T) <= 1e-5, (M, N, K)
+            for p in (dA, dB, dC):
+                dev.free(p)
+    finally:
+        dev.close()
