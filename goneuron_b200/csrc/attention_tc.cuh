@@ -668,7 +668,7 @@ inline AttnTcScratch& attn_tc_scratch(Ctx* ctx) {
 }
 inline int attn_tc_buf(Ctx* ctx, int i, size_t n, float** out) {
   DevBuf& b = attn_tc_scratch(ctx).buf[i];
-  if (b.n < n) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); GN_TRY(b.alloc(n)); }
+  if (b.n < n) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++; GN_TRY(b.alloc(n)); }
   *out = b.p; return GN_OK;
 }
 inline bool attn_tc_supported(Ctx* ctx, int hd, int T, int B, int H, int D) {
@@ -730,7 +730,7 @@ inline int attn_tc_fwd(Ctx* ctx, const float* Q, const float* K, const float* V,
   if (save && attn_keep_planes()) {
     const size_t need = attn_store_floats(3, Z, T);
     if (save->store.n < need) {
-      GN_CUDA(cudaStreamSynchronize(ctx->stream));
+      GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++;
       if (save->store.alloc(need) != GN_OK) { cudaGetLastError(); save = nullptr; }      // no room: the backward pass prepares its own operands
     }
   } else save = nullptr;

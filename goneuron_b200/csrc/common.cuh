@@ -30,6 +30,7 @@ struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t comm_stream = nullptr;   // gradient all-reduces run here, overlapped with the rest of the backward pass
+  cudaStream_t copy_stream = nullptr; cudaEvent_t copy_ev = nullptr;      // targets of a large host batch, copied under the forward pass
   int rank = 0, world = 1;
   void* comm = nullptr;            // ncclComm_t
   NcclApi* nccl = nullptr;
@@ -42,6 +43,10 @@ struct Ctx {
   double gemm_bytes = 0, split_bytes = 0;   // algorithmic bytes of the step's contraction launches (operand planes + output + residual) / of its operand split passes
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_pool; size_t ev_used = 0;
   int* d_status = nullptr;         // device word set by kernels whose bounded waits gave up
+  // pinned host memory of the context's calls (they run one at a time): results (loss sum | status word bits), a block for small
+  // inputs, one for small outputs; d_ret / d_out: the device's addresses
+  float *h_block = nullptr, *h_ret = nullptr, *h_stage = nullptr, *h_out = nullptr, *d_ret = nullptr, *d_out = nullptr;
+  uint64_t epoch = 0;              // counts replacements of the context's scratch buffers
   bool tc_ok = false;              // tcgen05 engine usable (driver entry point for tensor maps found)
   void* encode_tiled = nullptr;    // cuTensorMapEncodeTiled
   unsigned spin_limit = 1u << 24;  // polls per bounded device-side wait (gn_ctx_set_spin_limit)
@@ -51,7 +56,7 @@ struct Ctx {
   int tc_force_bn = 0, tc_kslice = 0;   // experiment switches of the contraction engine (GONEURON_CUDA_TC_BN / _KSLICE); 0 = automatic
   void* tc_scratch = nullptr;      // operand planes of the contraction engine (TcScratch, owned)
   void* attn_scratch = nullptr;    // operand planes of the tcgen05 attention kernels (AttnTcScratch, owned)
-  const void* weight_planes = nullptr;   // the running model's table of prepared weight planes (WeightPlaneTable), or null
+  void* weight_planes = nullptr;         // the running model's table of prepared weight planes (WeightPlaneTable), or null
   std::mutex run_mu;               // serialises every entry point that launches work on this context (they share the scratch above)
   cudaEvent_t t0 = nullptr, t1 = nullptr;   // gn_timer_start / gn_timer_stop
   // Scratch objects created on demand for this context (operand planes of the contraction and attention engines),
@@ -101,19 +106,59 @@ struct ProfScope {
   ~ProfScope() { if (e1) cudaEventRecord(e1, c->stream); }
 };
 
-// Owning device buffer.
+// Device memory of the library's buffers comes from one CUDA memory pool per GPU, which keeps up to POOL_KEEP_BYTES of what models
+// and scratch buffers have released (a model of the same size created later gets it back without going to the driver: mapping a
+// few GB takes it 0.1 to 1 s) and gives the rest back at once; shutting down the last context on a GPU empties it.  The pool is
+// the driver's and thread-safe.  An allocation is usable on every stream when alloc() returns; release() waits for the
+// device, as cudaFree does, so no stream can still be using what it hands back.
+constexpr unsigned long long POOL_KEEP_BYTES = 8ull << 30;
+struct DevicePools {
+  static constexpr int MAX = 64;
+  std::mutex mu; cudaMemPool_t pool[MAX] = {}; int contexts[MAX] = {};
+  static DevicePools& get() { static DevicePools* p = new DevicePools(); return *p; }      // (lives until the process ends)
+  cudaMemPool_t of(int dev) {
+    if (dev < 0 || dev >= MAX) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pool[dev]) {
+      cudaMemPoolProps pr{}; pr.allocType = cudaMemAllocationTypePinned; pr.location.type = cudaMemLocationTypeDevice; pr.location.id = dev;
+      if (cudaMemPoolCreate(&pool[dev], &pr) != cudaSuccess) { cudaGetLastError(); pool[dev] = nullptr; return nullptr; }
+      unsigned long long keep = POOL_KEEP_BYTES; cudaMemPoolSetAttribute(pool[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    return pool[dev];
+  }
+  void opened(int dev) { if (dev >= 0 && dev < MAX) { std::lock_guard<std::mutex> lk(mu); contexts[dev]++; } }
+  void closed(int dev) {
+    if (dev < 0 || dev >= MAX) return;
+    std::lock_guard<std::mutex> lk(mu);
+    if (--contexts[dev] <= 0 && pool[dev]) { cudaDeviceSynchronize(); cudaMemPoolTrimTo(pool[dev], 0); }
+  }
+};
+
+// Owning device buffer, or a view of part of another one.
 struct DevBuf {
-  float* p = nullptr; size_t n = 0;
+  float* p = nullptr; size_t n = 0; bool owner = true; int dev = 0;
   DevBuf() {}
   DevBuf(const DevBuf&) = delete; DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
-  DevBuf& operator=(DevBuf&& o) noexcept { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; return *this; }
+  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), owner(o.owner), dev(o.dev) { o.p = nullptr; o.n = 0; }
+  DevBuf& operator=(DevBuf&& o) noexcept { release(); p = o.p; n = o.n; owner = o.owner; dev = o.dev; o.p = nullptr; o.n = 0; return *this; }
   ~DevBuf() { release(); }
-  void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
+  void release() {
+    if (p && owner) {
+      int cur = dev; cudaGetDevice(&cur);
+      if (cur != dev) cudaSetDevice(dev);
+      cudaDeviceSynchronize(); cudaFreeAsync(p, cudaStreamLegacy);
+      if (cur != dev) cudaSetDevice(cur);
+    }
+    p = nullptr; n = 0; owner = true;
+  }
+  void view(float* q, size_t count) { release(); p = q; n = count; owner = false; }
   int alloc(size_t count) {
     release(); if (count == 0) return GN_OK;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(float));
-    if (e != cudaSuccess) { p = nullptr; return fail(GN_ERR_OOM, "cudaMalloc of %zu bytes failed: %s", count * sizeof(float), cudaGetErrorString(e)); }
+    cudaGetDevice(&dev);
+    cudaMemPool_t pool = DevicePools::get().of(dev);
+    cudaError_t e = pool ? cudaMallocFromPoolAsync((void**)&p, count * sizeof(float), pool, cudaStreamLegacy) : cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) { cudaGetLastError(); p = nullptr; return fail(GN_ERR_OOM, "device allocation of %zu bytes failed: %s", count * sizeof(float), cudaGetErrorString(e)); }
     n = count; return GN_OK;
   }
 };

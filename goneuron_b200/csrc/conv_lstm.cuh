@@ -49,7 +49,7 @@ __global__ void conv2d_dgrad_kernel(const float* __restrict__ g, const float* __
     dx[i] = acc;
   }
 }
-// One block per weight: dW[oc,ic,kh,kw] += sum_{b,oh,ow} g * x ; blocks >= nW reduce one bias each.
+// One block per weight: dW[oc,ic,kh,kw] = sum_{b,oh,ow} g * x ; blocks >= nW reduce one bias each.
 __global__ void conv2d_wgrad_kernel(const float* __restrict__ g, const float* __restrict__ x, float* __restrict__ dW, float* __restrict__ db, ConvShape c) {
   __shared__ float red[33];
   int nW = c.outC * c.inC * c.k * c.k;
@@ -65,7 +65,7 @@ __global__ void conv2d_wgrad_kernel(const float* __restrict__ g, const float* __
       s = fmaf(g[(((long)b * c.outC + oc) * c.oH + oh) * c.oW + ow], x[(((long)b * c.inC + ic) * c.H + ih) * c.W + iw], s);
     }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) dW[wi] += s;
+    if (threadIdx.x == 0) dW[wi] = s;
   } else {
     int oc = wi - nW;
     for (long i = threadIdx.x; i < span; i += blockDim.x) {
@@ -73,7 +73,7 @@ __global__ void conv2d_wgrad_kernel(const float* __restrict__ g, const float* __
       s += g[((long)q * c.outC + oc) * c.oH * c.oW + rem];
     }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) db[oc] += s;
+    if (threadIdx.x == 0) db[oc] = s;
   }
 }
 
@@ -122,7 +122,7 @@ __global__ void conv2d_wgrad_final_kernel(const float* __restrict__ part, int sl
   const int i = blockIdx.x * blockDim.x + threadIdx.x; if (i >= n) return;
   float s = 0.f;
   for (int k = 0; k < slices; k++) s += part[(long)k * n + i];
-  dW[i] += s;                                             // weights, then biases: the gradient slice is laid out W | b
+  dW[i] = s;                                              // weights, then biases: the gradient slice is laid out W | b
 }
 // Input gradient for stride 1 (no division in the tap loops); same sum as conv2d_dgrad_kernel.
 template <int K>
@@ -179,7 +179,7 @@ __global__ void conv1d_dgrad_kernel(const float* __restrict__ g, const float* __
     dx[i] = acc;
   }
 }
-// One block per weight: dW[oc,ic,k] += sum_{b,ol} g x ; blocks >= nW reduce one bias each.
+// One block per weight: dW[oc,ic,k] = sum_{b,ol} g x ; blocks >= nW reduce one bias each.
 __global__ void conv1d_wgrad_kernel(const float* __restrict__ g, const float* __restrict__ x, float* __restrict__ dW, float* __restrict__ db, Conv1Shape c) {
   __shared__ float red[33];
   const int nW = c.outC * c.inC * c.k, wi = blockIdx.x; const long span = (long)c.B * c.oL;
@@ -192,12 +192,12 @@ __global__ void conv1d_wgrad_kernel(const float* __restrict__ g, const float* __
       s = fmaf(g[((long)b * c.outC + oc) * c.oL + ol], x[((long)b * c.inC + ic) * c.L + pos], s);
     }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) dW[wi] += s;
+    if (threadIdx.x == 0) dW[wi] = s;
   } else {
     const int oc = wi - nW;
     for (long i = threadIdx.x; i < span; i += blockDim.x) s += g[((long)(i / c.oL) * c.outC + oc) * c.oL + i % c.oL];
     s = block_sum(s, red);
-    if (threadIdx.x == 0) db[oc] += s;
+    if (threadIdx.x == 0) db[oc] = s;
   }
 }
 

@@ -81,13 +81,13 @@ __global__ void conv_w_dgrad_layout_kernel(const float* __restrict__ W, float* _
     Wd[((long)ic * outC + oc) * kk + t] = W[i];
   }
 }
-// dW[oc, kidx] += sum_b part[b][oc][kidx] (kidx < K), db[oc] += sum_b part[b][oc][K]; samples added in batch order
+// dW[oc, kidx] = sum_b part[b][oc][kidx] (kidx < K), db[oc] = sum_b part[b][oc][K]; samples added in batch order
 __global__ void conv_wgrad_reduce_kernel(const float* __restrict__ part, int B, int outC, int K, float* __restrict__ dW, float* __restrict__ db) {
   const int n = outC * (K + 1), i = blockIdx.x * blockDim.x + threadIdx.x; if (i >= n) return;
   float s = 0.f;
   for (int b = 0; b < B; b++) s += part[(long)b * n + i];
   const int oc = i / (K + 1), kidx = i - oc * (K + 1);
-  if (kidx < K) dW[(long)oc * K + kidx] += s; else db[oc] += s;
+  if (kidx < K) dW[(long)oc * K + kidx] = s; else db[oc] = s;
 }
 
 inline bool conv_tc_supported(Ctx* ctx, const ConvShape& c) {
@@ -125,7 +125,7 @@ inline int conv_tc_dgrad(Ctx* ctx, const ConvShape& c, const float* dz, const fl
   conv_tc_count(ctx, (double)M, c.inC, Kd);
   return tc_run(ctx, A, Bp, ep);
 }
-// gW[outC, inC*k*k] += ..., gb[outC] += ...; `part`: B * outC * (inC*k*k + 1) floats.
+// gW[outC, inC*k*k], gb[outC] are written; `part`: B * outC * (inC*k*k + 1) floats.
 inline int conv_tc_wgrad(Ctx* ctx, const ConvShape& c, const float* dz, const float* x, float* part, float* gW, float* gb) {
   const int K = c.inC * c.k * c.k, P = c.oH * c.oW, N = K + 1;
   BfPlanes A, Bp; GN_TRY(tc_planes(ctx, 0, c.B, c.outC, P, &A)); GN_TRY(tc_planes(ctx, 1, c.B, N, P, &Bp));

@@ -667,15 +667,17 @@ inline size_t bf_plane_floats(long nbatch, long rows, long ldp) { return (size_t
 struct TcScratch { DevBuf a, b, sa, sb, mx; const float* last_a = nullptr; int last_m = 0, last_k = 0; long last_ld = 0; };
 inline TcScratch& tc_scratch(Ctx* ctx) { if (!ctx->tc_scratch) ctx->tc_scratch = ctx->own(new TcScratch()); return *static_cast<TcScratch*>(ctx->tc_scratch); }
 
+// After a replayed graph the scratch no longer holds what the last directly issued call left there.
+inline void forget_planes(Ctx* ctx) { if (ctx->tc_scratch) tc_scratch(ctx).last_a = nullptr; }
 // Operand planes for `nbatch` problems of rows x K in the context's scratch (which = 0: A side, 1: B side).
 inline int tc_planes(Ctx* ctx, int which, long nbatch, long rows, int K, BfPlanes* out) {
   TcScratch& sc = tc_scratch(ctx);
   const int ldp = tc_ldp(K); const size_t n = bf_plane_floats(nbatch, rows, ldp), ns = (size_t)nbatch * rows;
   if (rows > 0x7fffffffL || nbatch > 65535) return fail(GN_ERR_UNSUPPORTED, "tc_planes: operand too large");
   DevBuf& pl = which == 0 ? sc.a : sc.b; DevBuf& scl = which == 0 ? sc.sa : sc.sb;
-  if (pl.n < n) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); GN_TRY(pl.alloc(n)); }
-  if (scl.n < ns) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); GN_TRY(scl.alloc(ns + 1024)); }
-  if (sc.mx.n < ns) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); GN_TRY(sc.mx.alloc(ns + 1024)); }
+  if (pl.n < n) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++; GN_TRY(pl.alloc(n)); }
+  if (scl.n < ns) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++; GN_TRY(scl.alloc(ns + 1024)); }
+  if (sc.mx.n < ns) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++; GN_TRY(sc.mx.alloc(ns + 1024)); }
   if (which == 0) sc.last_a = nullptr;
   *out = BfPlanes{reinterpret_cast<__half*>(pl.p), scl.p, (int)rows, K, ldp, (int)nbatch}; return GN_OK;
 }
@@ -886,7 +888,7 @@ __global__ void __launch_bounds__(256) wplanes_split_kernel(const WPlaneJob* __r
 // Host side of the table: one entry per registered matrix, looked up by the matrix's device address.
 struct WeightPlaneEntry { const float* src; int out, in; BfPlanes rows, cols; const float* bias = nullptr; const int* maxabs = nullptr; int layer = -1; int tile0 = 0, tiles = 0; };
 struct WeightPlaneTable {
-  std::vector<WeightPlaneEntry> e; DevBuf planes, scales, mx, jobs; int total_tiles = 0; bool dirty = true;
+  std::vector<WeightPlaneEntry> e; DevBuf planes, scales, mx, jobs; int total_tiles = 0; bool dirty = true, used = false;      // used: some product has looked a matrix up
   // entries [j0, j1) that belong to model layer `layer` (they are registered layer by layer, so the range is contiguous)
   void layer_range(int layer, int* j0, int* j1) const {
     *j0 = *j1 = 0; bool in = false;
@@ -940,9 +942,11 @@ inline int wplanes_refresh(Ctx* ctx, WeightPlaneTable& t) {
 }
 // Prepared planes for B of this contraction, if B is a registered matrix used in one of its two orientations.
 inline const BfPlanes* wplanes_lookup(Ctx* ctx, const GemmDesc& g, const WeightPlaneEntry** entry = nullptr) {
-  const WeightPlaneTable* t = static_cast<const WeightPlaneTable*>(ctx->weight_planes);
-  if (!t || t->dirty || g.batch1 * g.batch2 != 1) return nullptr;
+  WeightPlaneTable* t = static_cast<WeightPlaneTable*>(ctx->weight_planes);
+  if (!t || g.batch1 * g.batch2 != 1) return nullptr;
   const WeightPlaneEntry* x = t->find(g.B); if (!x) return nullptr;
+  if (t->dirty && wplanes_refresh(ctx, *t) != GN_OK) return nullptr;       // once per parameter update, when the first product asks
+  t->used = true;
   if (entry) *entry = x;
   if (g.sb_k == 1 && g.sb_n == x->in && g.N == x->out && g.K == x->in) return &x->rows;     // B(k, n) = W[n, k]
   if (g.sb_n == 1 && g.sb_k == x->in && g.N == x->in && g.K == x->out) return &x->cols;     // B(k, n) = W[k, n]

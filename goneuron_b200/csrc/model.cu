@@ -13,6 +13,7 @@
 //    which at batch level is  gW = Delta^T * X_last  (a contraction over the batch) with Delta[s] = sum_t dz[s,t];
 //  * Embedding gradient: only the last sample of each worker chunk (embedding.go:151-154);
 //  * LSTM: see conv_lstm.cuh.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -96,6 +97,9 @@ struct LayerRT {
   // Tokens that the layers above read (TransformerBlock, Embedding; see plan_token_rows): 0 = all of a sequence's tokens, 1 = token 0,
   // 2 = token 0 and the last one.  `out` (and everything behind a block's attention) then holds that many rows per sequence.
   int out_rows = 0;
+  // A block whose backward pass needs a few rows only (token 0, last token) copies them to `keep` (keep_rows) and shares its
+  // activation buffers with the other blocks
+  DevBuf keep; bool kept = false;
   bool in_row0 = false, row0_grad = false;   // block input is token 0 only; the gradient of the output is nonzero at token 0 only
   bool grad_replicated = false;        // multi-GPU: every rank already holds the gradient of the whole global batch (no all-reduce)
   float bn_eps = 1e-5f, bn_mom = 0.1f;
@@ -105,7 +109,10 @@ struct LayerRT {
 
 struct gn_ctx { gn::Ctx c; bool alive = true; };
 
+namespace gn { struct StepGraph; }
 struct gn_model {
+  ~gn_model();
+  void drop_graphs();
   gn_ctx* ctx = nullptr;
   std::mutex mu;
   std::vector<gn::LayerRT> L;
@@ -114,14 +121,19 @@ struct gn_model {
   gn::DevBuf params, grads, m1, v2, state; int64_t NS = 0;
   int cur_first_sample = 0;             // global index of the first sample of the batch being processed (Dropout's stream position)
   int cur_global_batch = 0;             // size of the global batch being processed (all ranks)
+  uint64_t epoch = 0;                   // counts (re)allocations of the model's buffers
   bool wplanes_layerwise = false;       // this step renewed the weight planes layer by layer behind the parameter update
   const float* fwd_planes_src = nullptr; gn::BfPlanes fwd_planes{};     // operand planes of the tensor at fwd_planes_src, written by the LayerNorm that produced it
   float lr = 1e-3f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f; int timestep = 0;
-  int cap = 0;                          // batch capacity of the activation buffers
-  gn::DevBuf xin, yin, lossg, loss_s, loss_sum;
+  int cap = 0; bool cap_training = false;   // batch capacity of the activation buffers, and whether they can hold a training pass
+  gn::DevBuf shared[19];                // activation buffers that TransformerBlocks share
+  gn::DevBuf lossg, loss_s, loss_sum;
   std::vector<gn::DevBuf> scratch;      // growable shared scratch, by slot
   float last_inv_batch = 1.f;
-  float* h_ret = nullptr;               // pinned host block: [0] loss sum, [1] status word (bits), read back once per step
+  bool head_fused = false;              // the last forward pass left the head's softmax to head_loss_kernel
+  bool stats_timed = false;             // the last step's event times have been read
+  gn::DevBuf io;                        // Adam coefficients | host batch: x, y
+  std::vector<std::unique_ptr<gn::StepGraph>> graphs; uint64_t graph_clock = 0;
   gn_step_stats stats{};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ar0 = nullptr, ar1 = nullptr, comm_done = nullptr, gather_ev = nullptr;
   std::vector<cudaEvent_t> layer_ev;    // gradient of layer i complete (multi-GPU: releases its all-reduce)
@@ -132,12 +144,16 @@ struct gn_model {
 
 namespace gn {
 
+// Head of gn_model::io (floats); size of the context's pinned blocks (1 MiB); largest batch that goes through the inbound one
+// (beyond that the driver's own pageable copy, which overlaps its two stages, is the quicker way)
+constexpr size_t IO_ARGS = 64, STAGE_FLOATS = 1 << 18, STAGE_IN = 1 << 17;
+
 enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_COUNT };
 
 static int ensure(gn_model* m, int slot, size_t n, float** out) {
   if ((int)m->scratch.size() < S_COUNT) m->scratch.resize(S_COUNT);
   DevBuf& b = m->scratch[slot];
-  if (b.n < n) { GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream)); GN_TRY(b.alloc(n)); }
+  if (b.n < n) { GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream)); m->epoch++; GN_TRY(b.alloc(n)); }
   *out = b.p; return GN_OK;
 }
 
@@ -239,11 +255,42 @@ static int plan_layers(gn_model* m, const gn_layer_desc* layers, int n) {
   m->out_size = cur; m->P = off; return GN_OK;
 }
 
+static void plan_token_rows(gn_model* m, bool training);
+// Activation buffers of a TransformerBlock, by number.
+constexpr int NBLK = 18;
+static DevBuf& block_buf(LayerRT& l, int k) {
+  DevBuf* b[NBLK] = {&l.q, &l.k, &l.v, &l.att, &l.r1, &l.n1, &l.mid, &l.r2, &l.out, &l.stat, &l.gate, &l.up, &l.mid_last, &l.zlast, &l.mid_inv, &l.att_m, &l.att_l, &l.att_d};
+  return *b[k];
+}
+static void block_sizes(const LayerRT& l, size_t c, size_t (&n)[NBLK]) {
+  const gn_layer_desc& d = l.d; const size_t nd = c * d.seq_len * d.dim, nf = c * d.seq_len * d.ff_dim, nt = c * d.seq_len, bf = c * d.ff_dim;
+  const size_t v[NBLK] = {nd, nd, nd, nd, nd, nd, nf, nd, nd, 4 * nt, l.ff_act == GN_ACT_SILU ? nf : 0, l.ff_act == GN_ACT_SILU ? nf : 0, bf, l.ff_act == GN_ACT_GELU ? bf : 0, nt, nt * d.heads, nt * d.heads, nt * d.heads};
+  for (int k = 0; k < NBLK; k++) n[k] = v[k];
+}
+// Which blocks can use one set of activation buffers: all of them in inference; in training those whose backward pass needs the
+// few rows in `keep` (gradient at token 0 only, causal), and the top one, which runs last in the forward pass and first in
+// the backward pass.  `out` alternates between two buffers (a block reads its input until its end).
+static bool block_shares(const gn_model* m, const LayerRT& l, bool training) {
+  if (!training) return true;
+  int n_cls = 0, after = 0;
+  for (auto& x : m->L) { if (x.d.kind == GN_LAYER_CLS_POOLING) n_cls++; else if (n_cls && x.d.kind == GN_LAYER_TRANSFORMER_BLOCK) after++; }
+  return n_cls == 1 && after == 0 && l.row0_grad && (l.d.causal || l.out_rows);
+}
 // (Re)allocates every per-layer activation buffer for `cap` samples.
-static int alloc_activations(gn_model* m, int cap) {
+static int alloc_activations(gn_model* m, int cap, bool training) {
   GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream));
   size_t c = (size_t)cap;
-  GN_TRY(m->xin.alloc(c * m->in_size)); GN_TRY(m->yin.alloc(c * m->out_size));
+  plan_token_rows(m, training);
+  m->epoch++;
+  size_t most[NBLK] = {}; int n_shared = 0;
+  for (auto& l : m->L) if (l.d.kind == GN_LAYER_TRANSFORMER_BLOCK) {
+    for (int k = 0; k < NBLK; k++) block_buf(l, k).release();
+    if (block_shares(m, l, training)) { size_t need[NBLK]; block_sizes(l, c, need); for (int k = 0; k < NBLK; k++) most[k] = std::max(most[k], need[k]); n_shared++; }
+  }
+  for (int k = 0; k < NBLK; k++) GN_TRY(m->shared[k].alloc(most[k]));
+  GN_TRY(m->shared[NBLK].alloc(n_shared > 1 ? most[8] : 0));
+  n_shared = 0;
+  GN_TRY(m->io.alloc(IO_ARGS + (c * m->in_size + 63) / 64 * 64 + 64 + c * m->out_size));
   GN_TRY(m->lossg.alloc(c * m->out_size)); GN_TRY(m->loss_s.alloc(c)); GN_TRY(m->loss_sum.alloc(4));
   for (auto& l : m->L) {
     const gn_layer_desc& d = l.d;
@@ -267,13 +314,15 @@ static int alloc_activations(gn_model* m, int cap) {
       case GN_LAYER_EMBEDDING: GN_TRY(l.out.alloc(c * l.out_size)); GN_TRY(l.idx.alloc(c * d.seq_len)); break;
       case GN_LAYER_POSENC: GN_TRY(l.out.alloc(c * l.out_size)); break;
       case GN_LAYER_TRANSFORMER_BLOCK: {
-        size_t nd = c * d.seq_len * d.dim, nf = c * d.seq_len * d.ff_dim, nt = c * d.seq_len;
-        GN_TRY(l.q.alloc(nd)); GN_TRY(l.k.alloc(nd)); GN_TRY(l.v.alloc(nd)); GN_TRY(l.att.alloc(nd)); GN_TRY(l.r1.alloc(nd)); GN_TRY(l.n1.alloc(nd));
-        GN_TRY(l.mid.alloc(nf)); GN_TRY(l.r2.alloc(nd)); GN_TRY(l.out.alloc(nd)); GN_TRY(l.stat.alloc(4 * nt));
-        GN_TRY(l.att_m.alloc(nt * d.heads)); GN_TRY(l.att_l.alloc(nt * d.heads)); GN_TRY(l.att_d.alloc(nt * d.heads));
-        GN_TRY(l.mid_inv.alloc(nt)); GN_TRY(l.mid_last.alloc(c * d.ff_dim));
-        if (l.ff_act == GN_ACT_SILU) { GN_TRY(l.gate.alloc(nf)); GN_TRY(l.up.alloc(nf)); }
-        if (l.ff_act == GN_ACT_GELU) GN_TRY(l.zlast.alloc(c * d.ff_dim));
+        size_t need[NBLK]; block_sizes(l, c, need);
+        const bool share = block_shares(m, l, training), kept = share && training && !l.out_rows;
+        for (int k = 0; k < NBLK; k++) {
+          DevBuf& b = block_buf(l, k);
+          const bool own = !share || (training && (k == 12 || k == 13));      // the last token's feed-forward rows are read by the backward pass
+          if (own) GN_TRY(b.alloc(need[k])); else b.view(need[k] ? m->shared[k == 8 && n_shared % 2 ? NBLK : k].p : nullptr, need[k]);
+        }
+        if (share) n_shared++;
+        if (kept) GN_TRY(l.keep.alloc(c * (5 * (size_t)d.dim + 3 * (size_t)d.ff_dim + 4))); else l.keep.release();
         break; }
       case GN_LAYER_CLS_POOLING: GN_TRY(l.out.alloc(c * l.out_size)); break;
       case GN_LAYER_LAYERNORM: GN_TRY(l.out.alloc(c * l.out_size)); GN_TRY(l.stat.alloc(2 * c * (l.in_size / d.dim))); break;
@@ -281,7 +330,11 @@ static int alloc_activations(gn_model* m, int cap) {
       case GN_LAYER_BATCHNORM2D: GN_TRY(l.out.alloc(c * l.out_size)); GN_TRY(l.stat.alloc(3 * c * d.in_size)); break;
     }
   }
-  m->cap = cap; return GN_OK;
+  m->cap = cap; m->cap_training = training; return GN_OK;
+}
+static int ensure_capacity(gn_model* m, int B, bool training) {
+  if (B <= m->cap && (!training || m->cap_training)) return GN_OK;
+  return alloc_activations(m, std::max(B, m->cap), training || m->cap_training);
 }
 
 static inline unsigned ew_grid(Ctx* ctx, long n, int block = 256) { long g = (n + block - 1) / block; long mx = (long)ctx->sm_count * 16; return (unsigned)std::max<long>(1, std::min(g, mx)); }
@@ -483,6 +536,10 @@ static int next_rows(const gn_model* m, size_t li, int T, int D) {
   return n.d.kind == GN_LAYER_TRANSFORMER_BLOCK && n.in_row0 && n.d.seq_len == T && n.d.dim == D ? 1 : 0;
 }
 
+static KeepRows keep_layout(const LayerRT& l, int B) {
+  const long BD = (long)B * l.d.dim, BF = (long)B * l.d.ff_dim; float* p = l.keep.p;
+  return KeepRows{p, p + BD, p + 2 * BD, p + 3 * BD, p + 4 * BD, p + 5 * BD, p + 5 * BD + BF, p + 5 * BD + 2 * BF, p + 5 * BD + 3 * BF};
+}
 // One TransformerBlock forward.  `TE` rows per sequence go through everything behind the keys and values: all T, or the one
 // or two that the layers above read (plan_token_rows).  The backward pass finds the same number in l.out_rows.
 static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool training, const float** out) {
@@ -567,13 +624,24 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
     GN_TRY(block_norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * NE, (long)NE, D, po2.p ? &po2 : nullptr, &emitted));
     if (emitted) { m->fwd_planes = outp; m->fwd_planes_src = l.out.p; }
   }
+  l.kept = training && l.keep.n != 0;
+  if (l.kept) {
+    const KeepRows k = keep_layout(l, B);
+    GN_LAUNCH(ctx, keep_rows_kernel, B, 256, 0, (const float*)l.r2.p, (const float*)l.r1.p, (const float*)l.n1.p, (const float*)l.att.p, cur, l.mid_is_planes ? (const float*)nullptr : (const float*)l.mid.p,
+              (const float*)l.gate.p, (const float*)l.up.p, (const float*)st, k, T, D, F, B);
+  }
   *out = l.out.p; return GN_OK;
 }
 
+// A softmax or log-softmax head at the end of the model whose rows fit head_loss_kernel's registers.
+static bool head_can_fuse(const gn_model* m) {
+  const gn_layer_desc& d = m->L.back().d;
+  return d.kind == GN_LAYER_DENSE && (d.activation == GN_ACT_SOFTMAX || d.activation == GN_ACT_LOGSOFTMAX) && d.out_size <= HEAD_MAX_CS * HEAD_THREADS * HEAD_MAX_E;
+}
 static int forward(gn_model* m, const float* x, int B, const float** y_out, bool training) {
   Ctx* ctx = &m->ctx->c;
-  GN_TRY(wplanes_refresh(ctx, m->wplanes));          // no-op unless the parameters changed since the last pass
-  ctx->weight_planes = &m->wplanes;
+  ctx->weight_planes = &m->wplanes;                  // (renewed by the first product of the pass that looks one up)
+  m->head_fused = training && head_can_fuse(m);
   m->fwd_planes_src = nullptr;
   plan_token_rows(m, training);
   const float* cur = x;
@@ -587,7 +655,8 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
           GN_TRY(gemm_nt(ctx, B, d.out_size, d.in_size, cur, d.in_size, W, bias, l.out.p, d.out_size, d.activation));
         } else {
           GN_TRY(gemm_nt(ctx, B, d.out_size, d.in_size, cur, d.in_size, W, bias, l.z.p, d.out_size));
-          if (d.activation == GN_ACT_SOFTMAX || d.activation == GN_ACT_LOGSOFTMAX)
+          if (m->head_fused && li + 1 == m->L.size()) {}     // head_loss_kernel takes z
+          else if (d.activation == GN_ACT_SOFTMAX || d.activation == GN_ACT_LOGSOFTMAX)
             GN_LAUNCH(ctx, softmax_rows_kernel, B, 256, 0, l.z.p, l.out.p, d.out_size, d.activation == GN_ACT_LOGSOFTMAX ? 1 : 0);
           else { long n = (long)B * d.out_size; GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, n), 256, 0, l.z.p, l.out.p, n, d.activation, act_alpha_of(d.activation, d.reserved)); }
         }
@@ -867,24 +936,29 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
   Ctx* ctx = &m->ctx->c; const gn_layer_desc& d = l.d;
   const int T = d.seq_len, D = d.dim, F = d.ff_dim, TE = l.out_rows ? l.out_rows : T; const long ND = (long)B * T * D, BD = (long)B * D, BF = (long)B * F;
   const BlockParams bp = block_params(m->params.p + l.p_off, D, F, l.rms, l.ff_act); const BlockParams gp = block_params(m->grads.p + l.p_off, D, F, l.rms, l.ff_act);
-  const long ldD = (long)TE * D, ldF = (long)TE * F, NE = (long)B * TE; const float* st = l.stat.p;
-  const float* n1_last = l.n1.p + (long)(TE - 1) * D; const float* att_last = l.att.p + (long)(TE - 1) * D; const float* x_last = xin + (long)(T - 1) * D;
-  const float* mid_last = l.mid_is_planes ? l.mid_last.p : l.mid.p + (long)(TE - 1) * F; const long ld_mid = l.mid_is_planes ? F : ldF;
+  // token 0's row of the norms' inputs (and statistics), the last token's rows of the rest; rows of consecutive sequences are ldD (ldF, ldX) apart
+  const KeepRows kr = keep_layout(l, B); const int TR = l.kept ? 1 : TE;
+  const long ldD = (long)TR * D, ldF = (long)TR * F, NE = (long)B * TR, ldX = l.kept ? D : (long)T * D; const float* st = l.kept ? kr.st : l.stat.p;
+  auto last = [&](const DevBuf& b, const float* k, long w) -> const float* { return l.kept ? k : b.p + (long)(TE - 1) * w; };
+  const float* r2_0 = l.kept ? kr.r2 : l.r2.p; const float* r1_0 = l.kept ? kr.r1 : l.r1.p;
+  const float* n1_last = last(l.n1, kr.n1, D); const float* att_last = last(l.att, kr.att, D); const float* x_last = l.kept ? kr.x : xin + (long)(T - 1) * D;
+  const float* gate_last = last(l.gate, kr.gate, F); const float* up_last = last(l.up, kr.up, F);
+  const float* mid_last = l.mid_is_planes ? l.mid_last.p : last(l.mid, kr.mid, F); const long ld_mid = l.mid_is_planes ? F : ldF;
   float *dR2, *dR1, *comb, *dA, *dM;
   GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, d.causal ? BD : ND, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
   auto norm = [&](const float* g, const float* x, const float* gamma, const float* stat, float* out, float* gG, float* gB) -> int {
-    GN_LAUNCH(ctx, norm_bwd_rows_kernel, cdiv(B, 4), 128, 0, g, x, ldD, gamma, stat, l.rms ? nullptr : stat + NE, (long)TE, out, B, D);
-    GN_LAUNCH(ctx, norm_pgrad_rows_kernel, cdiv(D, 32), 256, 0, g, x, ldD, stat, l.rms ? nullptr : stat + NE, (long)TE, B, D, gG, gB);
+    GN_LAUNCH(ctx, norm_bwd_rows_kernel, cdiv(B, 4), 128, 0, g, x, ldD, gamma, stat, l.rms ? nullptr : stat + NE, (long)TR, out, B, D);
+    GN_LAUNCH(ctx, norm_pgrad_rows_kernel, cdiv(D, 32), 256, 0, g, x, ldD, stat, l.rms ? nullptr : stat + NE, (long)TR, B, D, gG, gB);
     return check_launch("norm_rows");
   };
-  GN_TRY(norm(gout, l.r2.p, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2));
+  GN_TRY(norm(gout, r2_0, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2));
   GN_TRY(weight_bias_grads(m, ctx, B, D, F, dR2, D, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
   GemmDesc g; g.M = B; g.N = F; g.K = D; g.A = dR2; g.sa_m = D; g.sa_k = 1; g.B = bp.w2; g.sb_k = F; g.sb_n = 1; g.C = dM; g.ldc = F;
   if (l.ff_act == GN_ACT_RELU) { g.mask = mid_last; g.mask_ld = ld_mid; }
   GN_TRY(gemm(ctx, g));
   if (l.ff_act == GN_ACT_SILU) {
     float *dG, *dU; GN_TRY(ensure(m, S_NFF2, BF, &dG)); GN_TRY(ensure(m, S_NFF3, BF, &dU));
-    GN_LAUNCH(ctx, swiglu_bwd_rows_kernel, ew_grid(ctx, BF), 256, 0, (const float*)dM, (const float*)(l.gate.p + (long)(TE - 1) * F), (const float*)(l.up.p + (long)(TE - 1) * F), ldF, dG, dU, F, BF);
+    GN_LAUNCH(ctx, swiglu_bwd_rows_kernel, ew_grid(ctx, BF), 256, 0, (const float*)dM, gate_last, up_last, ldF, dG, dU, F, BF);
     GN_TRY(gemm_tn(ctx, B, F, D, dG, F, n1_last, ldD, (float*)gp.w1));
     GN_TRY(gemm_tn(ctx, B, F, D, dU, F, n1_last, ldD, (float*)gp.v1));
     GN_TRY(gemm_nn(ctx, B, F, D, dG, F, bp.w1, comb, D, dR2, D));
@@ -894,25 +968,26 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
     GN_TRY(weight_bias_grads(m, ctx, B, F, D, dM, F, n1_last, ldD, (float*)gp.w1, (float*)gp.b1));
     GN_TRY(gemm_nn(ctx, B, F, D, dM, F, bp.w1, comb, D, dR2, D));
   }
-  GN_TRY(norm(comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1));
+  GN_TRY(norm(comb, r1_0, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1));
   GN_TRY(weight_bias_grads(m, ctx, B, D, D, dR1, D, att_last, ldD, (float*)gp.wo, (float*)gp.bo));
   GN_TRY(gemm_nn(ctx, B, D, D, dR1, D, bp.wo, dA, D));
   if (d.causal) {
-    // the one probability of token 0 is 1: dV = dA at token 0, dQ = dK = 0 (the gradient buffer was cleared)
-    GN_TRY(weight_bias_grads(m, ctx, B, D, D, dA, D, x_last, (long)T * D, (float*)gp.wv, (float*)gp.bv));
+    // the one probability of token 0 is 1: dV = dA at token 0, dQ = dK = 0
+    GN_CUDA(cudaMemsetAsync((void*)gp.wq, 0, (size_t)(gp.wv - gp.wq) * sizeof(float), ctx->stream));
+    GN_TRY(weight_bias_grads(m, ctx, B, D, D, dA, D, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
     GN_TRY(gemm_nn(ctx, B, D, D, dA, D, bp.wv, dx, D, dR1, D));
     *dx_row0 = true; return check_launch("block_backward_row0");
   }
   float *dQ, *dK, *dV, *ks, *vs;
   GN_TRY(ensure(m, S_XROWS, 3 * BD, &dQ)); ks = dQ + BD; vs = ks + BD; GN_TRY(ensure(m, S_ND1, ND, &dK)); GN_TRY(ensure(m, S_ND4, ND, &dV));
-  GN_TRY(attn_rows_bwd(ctx, l.q.p, ldD, l.k.p, l.v.p, dA, dQ, dK, dV, ks, vs, B, T, D, d.heads));
+  GN_TRY(attn_rows_bwd(ctx, l.q.p, (long)TE * D, l.k.p, l.v.p, dA, dQ, dK, dV, ks, vs, B, T, D, d.heads));
   if (l.use_rope) {   // the conjugate rotation (transformer.go:659-663); token 0's angle is zero
     GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, ND / 2), 256, 0, dK, (const float*)l.rope.p, (long)B * T, T, D, D / d.heads, -1.f, 1);
     GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(D, 128), B), dim3(128, 4), 0, (const float*)dK, T, D, ks);
   }
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, dQ, D, x_last, (long)T * D, (float*)gp.wq, (float*)gp.bq));
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, ks, D, x_last, (long)T * D, (float*)gp.wk, (float*)gp.bk));
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, vs, D, x_last, (long)T * D, (float*)gp.wv, (float*)gp.bv));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, dQ, D, x_last, ldX, (float*)gp.wq, (float*)gp.bq));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, ks, D, x_last, ldX, (float*)gp.wk, (float*)gp.bk));
+  GN_TRY(weight_bias_grads(m, ctx, B, D, D, vs, D, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
   GN_TRY(gemm_nn(ctx, B, D, D, dQ, D, bp.wq, dR1, D, dR1, D));
   GN_TRY(gemm_nn(ctx, B * T, D, D, dK, D, bp.wk, dx, D));
   GN_TRY(gemm_nn(ctx, B * T, D, D, dV, D, bp.wv, dx, D, dx, D));
@@ -994,10 +1069,11 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
   return check_launch("lstm_backward");
 }
 
-static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, int64_t n, float lr, float b1, float b2, float eps, int t, float grad_scale,
-                       const int* status, cudaStream_t stream);
+static AdamArgs adam_args(float lr, float b1, float b2, float eps, int t, float grad_scale);
+static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, int64_t n, const AdamArgs& a, const AdamArgs* dargs, const int* status, cudaStream_t stream,
+                       const float* loss_sum, float* ret);
 
-static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, int global_batch, int first_sample) {
+static int backward(gn_model* m, int B, const float* gloss, int global_batch, int first_sample) {
   Ctx* ctx = &m->ctx->c;
   const float* g = gloss;
   float* pp[2] = {nullptr, nullptr}; int flip = 0;
@@ -1010,6 +1086,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
   // for all layers after the backward pass instead (no overlap; for measurements).
   static const bool comm_at_end = [] { const char* e = getenv("GONEURON_CUDA_COMM"); return e && !strcmp(e, "end"); }();
   std::vector<int> deferred;
+  bool gated = false;                                       // g already carries the derivative of the ReLU below it
   bool row0 = false; int row0_T = 0, row0_D = 0;            // g holds the gradient of token 0 of every sequence, [B, row0_D]; the other tokens' is zero
   auto layer_comm = [&](int li) -> int {
     LayerRT& l = m->L[li]; float* gr = m->grads.p + l.p_off;
@@ -1019,10 +1096,10 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
       int rc = ctx->nccl->AllReduce(gr, gr, (size_t)l.p_cnt, NCCL_FLOAT32, NCCL_SUM, ctx->comm, ctx->comm_stream);
       if (rc) return fail(GN_ERR_NCCL, "ncclAllReduce(grads of layer %d): %s", li, ctx->nccl->GetErrorString(rc));
     }
-    GN_TRY(adam_launch(ctx, m->params.p + l.p_off, gr, m->m1.p + l.p_off, m->v2.p + l.p_off, l.p_cnt, m->lr, m->b1, m->b2, m->eps, m->timestep + 2,
-                       (float)(1.0 / (double)global_batch), ctx->d_status, ctx->comm_stream));
+    GN_TRY(adam_launch(ctx, m->params.p + l.p_off, gr, m->m1.p + l.p_off, m->v2.p + l.p_off, l.p_cnt,
+                       adam_args(m->lr, m->b1, m->b2, m->eps, m->timestep + 2, (float)(1.0 / (double)global_batch)), nullptr, ctx->d_status, ctx->comm_stream, nullptr, nullptr));
     // ... and the layer's prepared operand planes right behind the update, still hidden behind the earlier layers' backward pass
-    if (!m->wplanes.e.empty()) {
+    if (!m->wplanes.e.empty() && m->wplanes.used) {
       int j0, j1; m->wplanes.layer_range(li, &j0, &j1);
       GN_TRY(wplanes_refresh_range(ctx, m->wplanes, j0, j1, ctx->comm_stream));
       m->wplanes_layerwise = true;
@@ -1041,7 +1118,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
     switch (d.kind) {
       case GN_LAYER_DENSE: {
         const float* W = p; long wn = (long)d.in_size * d.out_size; const float* dz = g;
-        if (d.activation != GN_ACT_LINEAR) {
+        if (d.activation != GN_ACT_LINEAR && !(m->head_fused && li + 1 == (int)m->L.size()) && !gated) {
           float* dzb; GN_TRY(ensure(m, S_DZ, (size_t)B * d.out_size, &dzb)); long n = (long)B * d.out_size;
           if (d.activation == GN_ACT_SOFTMAX || d.activation == GN_ACT_LOGSOFTMAX)
             GN_LAUNCH(ctx, head_jacobian_kernel, B, 256, 0, g, l.out.p, dzb, d.out_size, d.activation == GN_ACT_LOGSOFTMAX ? 1 : 0);
@@ -1049,7 +1126,14 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
           dz = dzb;
         }
         GN_TRY(weight_bias_grads(m, ctx, B, d.out_size, d.in_size, dz, d.out_size, xin, d.in_size, gr, gr + wn));
-        if (need_dx) { GN_TRY(gemm_nn(ctx, B, d.out_size, d.in_size, dz, d.out_size, W, dx, d.in_size)); g = dx; flip ^= 1; }
+        gated = false;
+        if (need_dx) {
+          // a Dense(ReLU) below: its derivative, [activation > 0], gates this product's epilogue
+          const LayerRT& b = m->L[li - 1]; gated = b.d.kind == GN_LAYER_DENSE && b.d.activation == GN_ACT_RELU;
+          GemmDesc gd; gd.M = B; gd.N = d.in_size; gd.K = d.out_size; gd.A = dz; gd.sa_m = d.out_size; gd.sa_k = 1; gd.B = W; gd.sb_k = d.in_size; gd.sb_n = 1; gd.C = dx; gd.ldc = d.in_size;
+          if (gated) { gd.mask = b.out.p; gd.mask_ld = d.in_size; }
+          GN_TRY(gemm(ctx, gd)); g = dx; flip ^= 1;
+        }
         break; }
       case GN_LAYER_CONV2D: {
         ConvShape c{B, d.in_size, d.out_size, d.kernel, d.stride, d.padding, d.in_h, d.in_w,
@@ -1101,6 +1185,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
         const int chunk = (global_batch + m->W - 1) / m->W, T = row0 ? 1 : d.seq_len, Tid = d.seq_len, dim = d.out_size;     // T: tokens of a sample with a gradient
         const int nq = (global_batch + chunk - 1) / chunk;                       // qualifying samples of the global batch
         auto q_sample = [&](int q) { return std::min(global_batch - 1, q * chunk + chunk - 1); };
+        GN_CUDA(cudaMemsetAsync(gr, 0, (size_t)l.p_cnt * sizeof(float), ctx->stream));     // most rows of the table have no gradient
         const size_t smem = (size_t)T * sizeof(int);
         if (smem > 48 * 1024) GN_CUDA(cudaFuncSetAttribute(embedding_bwd_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const bool sparse = ctx->world > 1 && (double)nq * T * (dim + 1) < 0.5 * (double)l.p_cnt;
@@ -1133,6 +1218,7 @@ static int backward(gn_model* m, const float* /*x*/, int B, const float* gloss, 
         }
         break; }
       case GN_LAYER_POSENC:
+        if (row0) GN_CUDA(cudaMemsetAsync(gr, 0, (size_t)l.p_cnt * sizeof(float), ctx->stream));
         { const int n = row0 ? d.dim : l.out_size; GN_TRY(colsum(m, g, n, B, n, gr, false)); } break;     // gP = sum over samples; dx = g
       case GN_LAYER_TRANSFORMER_BLOCK:
         if (row0) GN_TRY(block_backward_row0(m, l, B, xin, g, dx, &row0)); else GN_TRY(block_backward(m, l, B, xin, g, dx));
@@ -1176,10 +1262,13 @@ static void adam_coeffs(float lr, float b1, float b2, int t, float* effLR) {
   float bias2 = (float)(1.0 - std::pow((double)b2, (double)t));
   *effLR = lr * (float)std::sqrt((double)bias2) / bias1;
 }
-static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, int64_t n, float lr, float b1, float b2, float eps, int t, float grad_scale,
-                       const int* status = nullptr, cudaStream_t stream = nullptr) {
+static AdamArgs adam_args(float lr, float b1, float b2, float eps, int t, float grad_scale) {
   float effLR; adam_coeffs(lr, b1, b2, t, &effLR);
-  adam_kernel<<<ew_grid(ctx, (n + 3) / 4), 256, 0, stream ? stream : ctx->stream>>>(p, g, m1, v, (long)n, effLR, b1, b2, 1.f - b1, 1.f - b2, eps, grad_scale, status);
+  return AdamArgs{effLR, b1, b2, 1.f - b1, 1.f - b2, eps, grad_scale};
+}
+static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, int64_t n, const AdamArgs& a, const AdamArgs* dargs, const int* status,
+                       cudaStream_t stream, const float* loss_sum, float* ret) {
+  adam_kernel<<<ew_grid(ctx, (n + 3) / 4), 256, 0, stream ? stream : ctx->stream>>>(p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret);
   ctx->launches++;
   return check_launch("adam");
 }
@@ -1188,27 +1277,33 @@ static int status_error(int st) {
   if (st == GN_STATUS_BAD_TOKEN) return fail(GN_ERR_INVALID_ARG, "a token id outside [0, vocabulary) was given to an Embedding layer (embedding.go:124-129); parameters and optimiser state are unchanged");
   return fail(GN_ERR_TIMEOUT, "a device-side bounded wait gave up (status word %d); parameters and optimiser state are unchanged", st);
 }
+static int clear_status(Ctx* c, int st) { cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream); cudaStreamSynchronize(c->stream); return status_error(st); }
 // Reads the status word; non-zero clears it and becomes an error (GN_ERR_TIMEOUT: a bounded device-side wait gave up).
 static int check_status_word(Ctx* c) {
   int st = 0; GN_CUDA(copy_d2h(c, &st, c->d_status, sizeof(int)));
-  if (st != 0) { cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream); cudaStreamSynchronize(c->stream); return status_error(st); }
-  return GN_OK;
+  return st != 0 ? clear_status(c, st) : GN_OK;
 }
 
-// The step proper.  Anything that fails after work has been queued must not leave that work running behind the caller's
-// back: train_step() below drains both streams before it reports the error.
-static int train_step_issue(gn_model* m, const float* x_dev, const float* y_dev, int B, int global_batch, int first_sample) {
+// The step in two halves: everything that needs x only, then what needs y.  A host y is copied while the first half runs.
+static int issue_forward(gn_model* m, const float* x_dev, int B, int global_batch, int first_sample, const float** yp) {
   Ctx* ctx = &m->ctx->c;
-  GN_CUDA(cudaEventRecord(m->ev0, ctx->stream));
-  GN_CUDA(cudaMemsetAsync(m->grads.p, 0, (size_t)m->P * sizeof(float), ctx->stream));     // Network.ClearGradients, net.go:813-823
-  const float* yp;
   m->cur_first_sample = first_sample; m->cur_global_batch = global_batch;
-  GN_TRY(forward(m, x_dev, B, &yp, true));
+  GN_TRY(forward(m, x_dev, B, yp, true));
   for (auto& l : m->L) if (l.d.kind == GN_LAYER_DROPOUT)          // every rank moves the stream on by the whole global batch
     GN_LAUNCH(ctx, dropout_advance_kernel, 1, 1, 0, m->state.p + l.s_off, (unsigned long long)global_batch * (unsigned long long)l.in_size);
-  GN_LAUNCH(ctx, loss_rows_kernel, B, 256, 0, yp, y_dev, m->lossg.p, m->loss_s.p, m->out_size, m->loss_kind);
-  GN_LAUNCH(ctx, loss_total_kernel, 1, 32, 0, m->loss_s.p, B, m->loss_sum.p);
-  GN_TRY(backward(m, x_dev, B, m->lossg.p, global_batch, first_sample));
+  return GN_OK;
+}
+static int issue_backward(gn_model* m, const float* yp, const float* y_dev, int B, int global_batch, int first_sample, const AdamArgs& a) {
+  Ctx* ctx = &m->ctx->c; unsigned* ticket = reinterpret_cast<unsigned*>(ctx->d_status + 1);
+  if (m->head_fused) {
+    // z -> loss and dz in one kernel; the smallest cluster whose registers hold a row
+    const LayerRT& h = m->L.back(); const int n = m->out_size, lg = h.d.activation == GN_ACT_LOGSOFTMAX;
+    int cs = 1; while (cs < HEAD_MAX_CS && n > cs * HEAD_THREADS * 4) cs *= 2;
+    const int per = cdiv(n, cs * HEAD_THREADS); const dim3 grid(B * cs);
+    auto* K = per <= 1 ? head_loss_kernel<1> : per <= 4 ? head_loss_kernel<4> : head_loss_kernel<HEAD_MAX_E>;
+    GN_CLUSTER_LAUNCH(ctx, K, grid, HEAD_THREADS, cs, (const float*)h.z.p, y_dev, m->lossg.p, m->loss_s.p, n, B, cs, lg, m->loss_kind, ticket, m->loss_sum.p);
+  } else GN_LAUNCH(ctx, loss_rows_kernel, B, m->out_size <= 64 ? 32 : 256, 0, yp, y_dev, m->lossg.p, m->loss_s.p, m->out_size, m->loss_kind, ticket, m->loss_sum.p);
+  GN_TRY(backward(m, B, m->lossg.p, global_batch, first_sample));
   if (ctx->world > 1) {
     // loss sum over the ranks, then the main stream waits for the communication stream (per-layer gradient
     // all-reduces were issued during the backward pass); ar0..ar1 brackets the exposed wait
@@ -1220,51 +1315,177 @@ static int train_step_issue(gn_model* m, const float* x_dev, const float* y_dev,
     GN_CUDA(cudaEventRecord(m->ar0, ctx->stream));
     GN_CUDA(cudaStreamWaitEvent(ctx->stream, m->comm_done, 0));
     GN_CUDA(cudaEventRecord(m->ar1, ctx->stream));
+    // (the update was applied slice by slice behind each layer's all-reduce, see backward())
+    GN_LAUNCH(ctx, finish_kernel, 1, 32, 0, (const float*)m->loss_sum.p, ctx->d_ret, 1, (const int*)ctx->d_status, ctx->d_ret);
+    return check_launch("finish");
   }
   // Network.Step (net.go:260-284): NewStep() then StepInPlace with t = timestep + 1.  The pass reads the status word
   // first: after a bounded wait gave up it changes nothing.
-  float inv = (float)(1.0 / (double)global_batch);                                        // net.go:703
+  return adam_launch(ctx, m->params.p, m->grads.p, m->m1.p, m->v2.p, m->P, a, reinterpret_cast<const AdamArgs*>(m->io.p), ctx->d_status, nullptr, m->loss_sum.p, ctx->d_ret);
+}
+
+// Captured launches of a step (or of an inference pass).  A call whose sizes and buffers have been seen before is replayed as one or
+// two CUDA graphs: a step is 10 to 300 launches of a few microseconds each, which the host would otherwise issue one by one.  The
+// first call with a set of sizes runs launch by launch (it may allocate), the second is captured.  A graph refers to
+// buffers by address, so it is dropped when the model or the context has replaced one (epoch).  What differs from call to
+// call lies in memory: inputs, the Adam coefficients (head of the model's `io` buffer), the results.
+struct StepGraph {
+  int B, global_batch, first_sample; const float *x, *y; bool staged, training; unsigned spin; uint64_t epoch_m, epoch_c;
+  bool same(const StepGraph& o) const {
+    return B == o.B && global_batch == o.global_batch && first_sample == o.first_sample && x == o.x && y == o.y && staged == o.staged && training == o.training && spin == o.spin &&
+           epoch_m == o.epoch_m && epoch_c == o.epoch_c;
+  }
+  cudaGraphExec_t exec[2] = {nullptr, nullptr}; bool captured = false, refused = false; uint64_t last_use = 0;
+  int64_t launches = 0, gemm_launches = 0; double gemm_flops = 0, gemm_bytes = 0, split_bytes = 0; const float* out = nullptr;
+  void drop() { for (auto& e : exec) if (e) { cudaGraphExecDestroy(e); e = nullptr; } captured = false; }
+};
+constexpr size_t MAX_GRAPHS = 8;                             // per model: batch sizes and device-resident batches in turn
+static StepGraph* find_graph(gn_model* m, StepGraph key) {
+  Ctx* ctx = &m->ctx->c;
+  static const bool off = getenv("GONEURON_CUDA_NO_GRAPHS") != nullptr;
+  if (off || ctx->world > 1 || ctx->profile || ctx->tc_tile_queue) return nullptr;
+  key.epoch_m = m->epoch; key.epoch_c = ctx->epoch; key.spin = ctx->spin_limit; key.last_use = ++m->graph_clock;
+  for (auto& g : m->graphs) if (g->same(key)) { g->last_use = key.last_use; return g.get(); }
+  return nullptr;
+}
+// Remembers a set of sizes that has just run launch by launch (the epochs are those after the run).
+static void note_graph(gn_model* m, StepGraph key) {
+  Ctx* ctx = &m->ctx->c;
+  key.epoch_m = m->epoch; key.epoch_c = ctx->epoch; key.spin = ctx->spin_limit; key.last_use = ++m->graph_clock;
+  for (auto it = m->graphs.begin(); it != m->graphs.end();) {      // stale ones can never match again
+    if ((*it)->epoch_m != key.epoch_m || (*it)->epoch_c != key.epoch_c) { (*it)->drop(); it = m->graphs.erase(it); } else ++it;
+  }
+  for (auto& g : m->graphs) if (g->same(key)) return;
+  if (m->graphs.size() >= MAX_GRAPHS) {
+    auto old = std::min_element(m->graphs.begin(), m->graphs.end(), [](auto& a, auto& b) { return a->last_use < b->last_use; });
+    (*old)->drop(); m->graphs.erase(old);
+  }
+  m->graphs.emplace_back(new StepGraph(key));
+}
+// Runs `issue` under stream capture; *out stays null when the work cannot be captured (the caller then runs it directly).
+template <class F> static int capture(Ctx* ctx, F&& issue, cudaGraphExec_t* out) {
+  *out = nullptr; cudaGraph_t g = nullptr;
+  GN_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+  const int rc = issue();
+  const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+  if (rc == GN_OK && e == cudaSuccess && g && cudaGraphInstantiate(out, g, 0) != cudaSuccess) *out = nullptr;
+  if (g) cudaGraphDestroy(g);
+  cudaGetLastError(); return GN_OK;
+}
+static void reset_counters(Ctx* ctx) { ctx->gemm_flops = 0; ctx->gemm_launches = 0; ctx->gemm_ms = 0; ctx->ev_used = 0; ctx->gemm_bytes = 0; ctx->split_bytes = 0; }
+
+// x and y: device memory, or (host = true) host memory.
+static int train_step_issue(gn_model* m, const float* x, const float* y, bool host, int B, int global_batch, int first_sample) {
+  Ctx* ctx = &m->ctx->c; const size_t nx = (size_t)B * m->in_size, ny = (size_t)B * m->out_size, y_at = IO_ARGS + (nx + 63) / 64 * 64;
+  const float inv = (float)(1.0 / (double)global_batch);                                        // net.go:703
   m->last_inv_batch = inv;
-  if (ctx->world == 1) GN_TRY(adam_launch(ctx, m->params.p, m->grads.p, m->m1.p, m->v2.p, m->P, m->lr, m->b1, m->b2, m->eps, m->timestep + 2, inv, ctx->d_status));
-  // (with more than one rank the update was applied slice by slice behind each layer's all-reduce, see backward())
+  const AdamArgs a = adam_args(m->lr, m->b1, m->b2, m->eps, m->timestep + 2, inv);
+  // small host batches go through one pinned block together with the coefficients: one copy instead of three
+  const bool staged = host && y_at + ny <= STAGE_IN;
+  memcpy(ctx->h_stage, &a, sizeof a);
+  const float* xd = host ? m->io.p + IO_ARGS : x; const float* yd = host ? m->io.p + y_at : y;
+  if (staged) { memcpy(ctx->h_stage + IO_ARGS, x, nx * 4); memcpy(ctx->h_stage + y_at, y, ny * 4); }
+  StepGraph key{B, global_batch, first_sample, xd, yd, staged, true};
+  StepGraph* g = find_graph(m, key);
+  const float* yp = nullptr;
+  auto copy_in = [&]() -> int { GN_CUDA(cudaMemcpyAsync(m->io.p, ctx->h_stage, (staged ? y_at + ny : IO_ARGS) * 4, cudaMemcpyHostToDevice, ctx->stream)); return GN_OK; };
+  auto first = [&]() -> int { return issue_forward(m, xd, B, global_batch, first_sample, &yp); };
+  auto second = [&]() -> int { return issue_backward(m, yp, yd, B, global_batch, first_sample, a); };
+  const bool split = host && !staged;                          // y is copied between the halves
+  if (g && !g->captured && !g->refused) {
+    const int64_t l0 = ctx->launches; reset_counters(ctx);
+    m->wplanes.dirty = true;                                   // as in every step: the parameters have moved since the planes were written
+    if (split) {
+      GN_TRY(capture(ctx, [&]() -> int { GN_TRY(copy_in()); return first(); }, &g->exec[0]));
+      if (g->exec[0]) GN_TRY(capture(ctx, second, &g->exec[1]));
+    } else GN_TRY(capture(ctx, [&]() -> int { GN_TRY(copy_in()); GN_TRY(first()); return second(); }, &g->exec[0]));
+    g->captured = g->exec[0] && (!split || g->exec[1]); g->refused = !g->captured;
+    g->launches = ctx->launches - l0; ctx->launches = l0; g->gemm_launches = ctx->gemm_launches; g->gemm_flops = ctx->gemm_flops; g->gemm_bytes = ctx->gemm_bytes; g->split_bytes = ctx->split_bytes;
+    if (g->refused) { g->drop(); m->wplanes.dirty = true; }
+  }
+  reset_counters(ctx);
+  if (split) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, x, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
+  GN_CUDA(cudaEventRecord(m->ev0, ctx->stream));
+  const bool replay = g && g->captured;
+  if (replay) { GN_CUDA(cudaGraphLaunch(g->exec[0], ctx->stream)); }
+  else { GN_TRY(copy_in()); GN_TRY(first()); }
+  if (split) {                                               // on a stream of its own: it must not wait for the first half
+    GN_CUDA(cudaMemcpyAsync(m->io.p + y_at, y, ny * 4, cudaMemcpyHostToDevice, ctx->copy_stream));
+    GN_CUDA(cudaEventRecord(ctx->copy_ev, ctx->copy_stream)); GN_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->copy_ev, 0));
+  }
+  if (replay) { if (split) GN_CUDA(cudaGraphLaunch(g->exec[1], ctx->stream)); }
+  else GN_TRY(second());
   GN_CUDA(cudaEventRecord(m->ev1, ctx->stream));
-  // one read-back for the caller: the loss sum and the status word land in the same pinned block, one wait
-  GN_CUDA(cudaMemcpyAsync(&m->h_ret[0], m->loss_sum.p, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-  GN_CUDA(cudaMemcpyAsync(&m->h_ret[1], ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  GN_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (replay) {
+    ctx->launches += g->launches; ctx->gemm_launches = g->gemm_launches; ctx->gemm_flops = g->gemm_flops; ctx->gemm_bytes = g->gemm_bytes; ctx->split_bytes = g->split_bytes;
+    forget_planes(ctx);
+  }
+  GN_CUDA(cudaStreamSynchronize(ctx->stream));                // the loss sum and the status word are in host memory now
+  if (!g) note_graph(m, key);
   return GN_OK;
 }
 
-static int train_step(gn_model* m, const float* x_dev, const float* y_dev, int B, int global_batch, int first_sample, float* mean_loss) {
+static int train_step(gn_model* m, const float* x, const float* y, bool host, int B, int global_batch, int first_sample, float* mean_loss) {
   Ctx* ctx = &m->ctx->c;
   if (global_batch <= 0) { global_batch = B; first_sample = 0; }
-  if (B > m->cap) GN_TRY(alloc_activations(m, B));
-  int64_t launches0 = ctx->launches; ctx->gemm_flops = 0; ctx->gemm_launches = 0; ctx->gemm_ms = 0; ctx->ev_used = 0; ctx->gemm_bytes = 0; ctx->split_bytes = 0;
+  GN_TRY(ensure_capacity(m, B, true));
+  int64_t launches0 = ctx->launches;
   m->wplanes_layerwise = false;
-  int rc = train_step_issue(m, x_dev, y_dev, B, global_batch, first_sample);
+  // Anything that fails after work has been queued must not leave that work running behind the caller's back.
+  int rc = train_step_issue(m, x, y, host, B, global_batch, first_sample);
   if (rc != GN_OK) {
     // drain what was queued before the failure (both streams) so that nothing of this step runs after the call returned
     const std::string msg = last_error();
     if (ctx->comm_stream) cudaStreamSynchronize(ctx->comm_stream);
-    cudaStreamSynchronize(ctx->stream); cudaGetLastError();
+    cudaStreamSynchronize(ctx->copy_stream); cudaStreamSynchronize(ctx->stream); cudaGetLastError();
     last_error() = msg; return rc;
   }
-  int st; memcpy(&st, &m->h_ret[1], sizeof(int));
-  if (st != 0) {    // the Adam pass saw the same word and left parameters, moments and the step counter alone
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream); cudaStreamSynchronize(ctx->stream);
-    return status_error(st);
-  }
+  int st; memcpy(&st, &ctx->h_ret[1], sizeof(int));
+  if (st != 0) return clear_status(ctx, st);         // the Adam pass saw the same word and left parameters, moments and the step counter alone
   m->timestep += 1;
   m->wplanes.dirty = !m->wplanes_layerwise;          // the parameters moved: their operand planes are stale, unless they were renewed layer by layer behind the update
   m->wplanes_layerwise = false;
-  if (mean_loss) *mean_loss = m->h_ret[0] / (float)global_batch;
+  if (mean_loss) *mean_loss = ctx->h_ret[0] / (float)global_batch;
   m->stats.kernel_launches = ctx->launches - launches0;
-  cudaEventElapsedTime(&m->stats.step_ms, m->ev0, m->ev1);
-  m->stats.allreduce_ms = 0.f; if (ctx->world > 1) cudaEventElapsedTime(&m->stats.allreduce_ms, m->ar0, m->ar1);
   m->stats.gemm_flops = ctx->gemm_flops; m->stats.gemm_launches = ctx->gemm_launches; m->stats.gemm_ms = 0.f;
-  m->stats.gemm_bytes = ctx->gemm_bytes; m->stats.split_bytes = ctx->split_bytes;
+  m->stats.gemm_bytes = ctx->gemm_bytes; m->stats.split_bytes = ctx->split_bytes; m->stats_timed = false;
   if (ctx->profile) { float tot = 0.f; for (size_t i = 0; i < ctx->ev_used; i++) { float ms = 0.f; cudaEventElapsedTime(&ms, ctx->ev_pool[i].first, ctx->ev_pool[i].second); tot += ms; } m->stats.gemm_ms = tot; }
   return GN_OK;
+}
+
+// Batched inference, host to host.
+static int forward_batch(gn_model* m, const float* x, int B, float* out) {
+  Ctx* ctx = &m->ctx->c; const size_t nx = (size_t)B * m->in_size, ny = (size_t)B * m->out_size;
+  GN_TRY(ensure_capacity(m, B, false));
+  const bool staged = nx <= STAGE_IN, small = ny <= STAGE_FLOATS;      // through the pinned blocks, in and out
+  const float* xd = m->io.p + IO_ARGS; const float* yp = nullptr;
+  if (staged) memcpy(ctx->h_stage, x, nx * 4);
+  if (m->wplanes.used) GN_TRY(wplanes_refresh(ctx, m->wplanes));           // no-op unless the parameters changed since the last pass
+  auto body = [&]() -> int {
+    if (staged) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, ctx->h_stage, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
+    GN_TRY(forward(m, xd, B, &yp, false));
+    // a few KB are written to host memory by a kernel, more by the copy engine
+    const bool by_kernel = ny <= 4096;
+    if (small && !by_kernel) GN_CUDA(cudaMemcpyAsync(ctx->h_out, yp, ny * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    GN_LAUNCH(ctx, finish_kernel, by_kernel ? cdiv(ny, 256) : 1, by_kernel ? 256 : 32, 0, yp, ctx->d_out, by_kernel ? (int)ny : 0, (const int*)ctx->d_status, ctx->d_ret);
+    return check_launch("finish");
+  };
+  StepGraph key{B, 0, 0, xd, nullptr, staged, false};
+  StepGraph* g = find_graph(m, key);
+  if (g && !g->captured && !g->refused) {
+    const int64_t l0 = ctx->launches;
+    GN_TRY(capture(ctx, body, &g->exec[0]));
+    ctx->launches = l0; g->captured = g->exec[0] != nullptr; g->refused = !g->captured; g->out = yp;
+  }
+  if (!staged) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, x, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
+  if (g && g->captured) { GN_CUDA(cudaGraphLaunch(g->exec[0], ctx->stream)); yp = g->out; forget_planes(ctx); }
+  else GN_TRY(body());
+  if (!small) GN_CUDA(cudaMemcpyAsync(out, yp, ny * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  GN_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (!g) note_graph(m, key);
+  if (small) memcpy(out, ctx->h_out, ny * 4);
+  int st; memcpy(&st, &ctx->h_ret[1], sizeof(int));
+  return st != 0 ? clear_status(ctx, st) : GN_OK;
 }
 
 static int make_ctx(int device, int rank, int world, const unsigned char* id, gn_ctx** out) {
@@ -1280,15 +1501,22 @@ static int make_ctx(int device, int rank, int world, const unsigned char* id, gn
       if (c->c.comm && c->c.nccl) c->c.nccl->CommDestroy(c->c.comm);
       if (c->c.comm_stream) cudaStreamDestroy(c->c.comm_stream);
       if (c->c.d_status) cudaFree(c->c.d_status);
+      if (c->c.h_block) cudaFreeHost(c->c.h_block);
       if (c->c.tc_queue_pool) cudaFree(c->c.tc_queue_pool);
+      if (c->c.copy_ev) cudaEventDestroy(c->c.copy_ev);
+      if (c->c.copy_stream) cudaStreamDestroy(c->c.copy_stream);
       if (c->c.stream) cudaStreamDestroy(c->c.stream);
       delete c; } } guard{new gn_ctx()};
   gn_ctx* c = guard.c;
   c->c.device = device; c->c.rank = rank; c->c.world = world; c->c.sm_count = prop.multiProcessorCount;
   if (const char* e = getenv("GONEURON_CUDA_SM_RESERVE")) c->c.sm_reserve = std::max(0, std::min(atoi(e), prop.multiProcessorCount / 2));
   GN_CUDA(cudaStreamCreateWithFlags(&c->c.stream, cudaStreamNonBlocking));
-  GN_CUDA(cudaMalloc(&c->c.d_status, sizeof(int)));
-  GN_CUDA(cudaMemsetAsync(c->c.d_status, 0, sizeof(int), c->c.stream)); GN_CUDA(cudaStreamSynchronize(c->c.stream));
+  GN_CUDA(cudaStreamCreateWithFlags(&c->c.copy_stream, cudaStreamNonBlocking)); GN_CUDA(cudaEventCreateWithFlags(&c->c.copy_ev, cudaEventDisableTiming));
+  GN_CUDA(cudaMalloc(&c->c.d_status, 4 * sizeof(int)));      // status word | ticket of the loss kernels | a scratch word
+  GN_CUDA(cudaMemsetAsync(c->c.d_status, 0, 4 * sizeof(int), c->c.stream)); GN_CUDA(cudaStreamSynchronize(c->c.stream));
+  GN_CUDA(cudaHostAlloc((void**)&c->c.h_block, (2 * STAGE_FLOATS + 64) * sizeof(float), cudaHostAllocMapped));
+  c->c.h_ret = c->c.h_block; c->c.h_stage = c->c.h_block + 64; c->c.h_out = c->c.h_stage + STAGE_FLOATS;
+  GN_CUDA(cudaHostGetDevicePointer((void**)&c->c.d_ret, c->c.h_ret, 0)); c->c.d_out = c->c.d_ret + (c->c.h_out - c->c.h_ret);
   tc_init(&c->c);
   if (world > 1) {
     NcclApi* api = nccl_api(); if (!api) return fail(GN_ERR_NCCL, "libnccl.so.2 could not be loaded");
@@ -1299,12 +1527,16 @@ static int make_ctx(int device, int rank, int world, const unsigned char* id, gn
     GN_CUDA(cudaStreamCreateWithFlags(&c->c.comm_stream, cudaStreamNonBlocking));
   }
   guard.c = nullptr;
+  DevicePools::get().opened(device);
   *out = c; return GN_OK;
 }
 
 }  // namespace gn
 
 using namespace gn;
+
+void gn_model::drop_graphs() { for (auto& g : graphs) g->drop(); graphs.clear(); }
+gn_model::~gn_model() { drop_graphs(); }
 
 #define CHECK_MODEL(m) do { if (!(m) || !(m)->alive) return fail(GN_ERR_INVALID_ARG, "model handle is null or destroyed"); } while (0)
 #define USE_DEVICE(m) GN_CUDA(cudaSetDevice((m)->ctx->c.device))
@@ -1338,12 +1570,16 @@ int gn_shutdown(gn_ctx* ctx) {
   ctx->c.ev_pool.clear();
   ctx->c.release_owned();                               // operand-plane scratch of the contraction and attention engines
   if (ctx->c.d_status) cudaFree(ctx->c.d_status);
+  if (ctx->c.h_block) { cudaFreeHost(ctx->c.h_block); ctx->c.h_block = nullptr; }
   if (ctx->c.tc_queue_pool) { cudaFree(ctx->c.tc_queue_pool); ctx->c.tc_queue_pool = nullptr; }
   if (ctx->c.t0) { cudaEventDestroy(ctx->c.t0); cudaEventDestroy(ctx->c.t1); ctx->c.t0 = ctx->c.t1 = nullptr; }
+  if (ctx->c.copy_ev) { cudaEventDestroy(ctx->c.copy_ev); ctx->c.copy_ev = nullptr; }
+  if (ctx->c.copy_stream) { cudaStreamDestroy(ctx->c.copy_stream); ctx->c.copy_stream = nullptr; }
   if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
   if (ctx->c.comm_stream) cudaStreamDestroy(ctx->c.comm_stream);
   ctx->c.comm_stream = nullptr;
   ctx->c.comm = nullptr; ctx->c.d_status = nullptr; ctx->c.stream = nullptr; ctx->alive = false;
+  DevicePools::get().closed(ctx->c.device);
   return GN_OK;   // the handle itself stays allocated so that a second call is harmless
 }
 
@@ -1426,7 +1662,6 @@ int gn_model_create(gn_ctx* ctx, const gn_layer_desc* layers, int n_layers, int 
   m->layer_ev.resize(m->L.size() + 1);
   for (auto& e : m->layer_ev) GN_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   m->scratch.resize(S_COUNT);
-  GN_CUDA(cudaHostAlloc((void**)&m->h_ret, 4 * sizeof(float), cudaHostAllocDefault));
   *out = m.release(); return GN_OK;
 }
 
@@ -1437,11 +1672,11 @@ int gn_model_destroy(gn_model* m) {
   if (m->ctx->alive && m->ctx->c.stream) cudaStreamSynchronize(m->ctx->c.stream);
   if (m->ctx->c.weight_planes == &m->wplanes) m->ctx->c.weight_planes = nullptr;
   m->wplanes = gn::WeightPlaneTable();
-  m->L.clear(); m->scratch.clear(); m->state.release(); m->params.release(); m->grads.release(); m->m1.release(); m->v2.release();
-  m->xin.release(); m->yin.release(); m->lossg.release(); m->loss_s.release(); m->loss_sum.release();
+  m->drop_graphs();
+  m->L.clear(); m->scratch.clear(); for (auto& b : m->shared) b.release(); m->state.release(); m->params.release(); m->grads.release(); m->m1.release(); m->v2.release();
+  m->io.release(); m->lossg.release(); m->loss_s.release(); m->loss_sum.release();
   if (m->ev0) cudaEventDestroy(m->ev0); if (m->ev1) cudaEventDestroy(m->ev1); if (m->ar0) cudaEventDestroy(m->ar0); if (m->ar1) cudaEventDestroy(m->ar1);
   if (m->comm_done) cudaEventDestroy(m->comm_done); if (m->gather_ev) cudaEventDestroy(m->gather_ev); m->gather_ev = nullptr; for (auto e : m->layer_ev) cudaEventDestroy(e); m->layer_ev.clear();
-  if (m->h_ret) cudaFreeHost(m->h_ret); m->h_ret = nullptr;
   m->ev0 = m->ev1 = m->ar0 = m->ar1 = m->comm_done = nullptr; m->alive = false; return GN_OK;
 }
 
@@ -1511,28 +1746,19 @@ int gn_adam_set_state(gn_model* m, const float* m1, const float* v, int64_t n, i
 int gn_train_batch_device(gn_model* m, const float* x_dev, const float* y_dev, int batch, int global_batch, int first_sample, float* mean_loss) {
   CHECK_MODEL(m); if (!x_dev || !y_dev || batch <= 0) return fail(GN_ERR_INVALID_ARG, "train_batch: null input or batch <= 0");
   std::lock_guard<std::mutex> lk(m->mu); std::lock_guard<std::mutex> run_lk(m->ctx->c.run_mu); USE_DEVICE(m);
-  return train_step(m, x_dev, y_dev, batch, global_batch, first_sample, mean_loss);
+  return train_step(m, x_dev, y_dev, false, batch, global_batch, first_sample, mean_loss);
 }
 
 int gn_train_batch(gn_model* m, const float* x, const float* y, int batch, int global_batch, int first_sample, float* mean_loss) {
   CHECK_MODEL(m); if (!x || !y || batch <= 0) return fail(GN_ERR_INVALID_ARG, "train_batch: null input or batch <= 0");
   std::lock_guard<std::mutex> lk(m->mu); std::lock_guard<std::mutex> run_lk(m->ctx->c.run_mu); USE_DEVICE(m);
-  if (batch > m->cap) GN_TRY(alloc_activations(m, batch));
-  cudaStream_t s = m->ctx->c.stream;
-  GN_CUDA(cudaMemcpyAsync(m->xin.p, x, (size_t)batch * m->in_size * 4, cudaMemcpyHostToDevice, s));
-  GN_CUDA(cudaMemcpyAsync(m->yin.p, y, (size_t)batch * m->out_size * 4, cudaMemcpyHostToDevice, s));
-  return train_step(m, m->xin.p, m->yin.p, batch, global_batch, first_sample, mean_loss);
+  return train_step(m, x, y, true, batch, global_batch, first_sample, mean_loss);
 }
 
 int gn_forward_batch(gn_model* m, const float* x, int batch, float* out) {
   CHECK_MODEL(m); if (!x || !out || batch <= 0) return fail(GN_ERR_INVALID_ARG, "forward_batch: null pointer or batch <= 0");
   std::lock_guard<std::mutex> lk(m->mu); std::lock_guard<std::mutex> run_lk(m->ctx->c.run_mu); USE_DEVICE(m);
-  if (batch > m->cap) GN_TRY(alloc_activations(m, batch));
-  cudaStream_t s = m->ctx->c.stream;
-  GN_CUDA(cudaMemcpyAsync(m->xin.p, x, (size_t)batch * m->in_size * 4, cudaMemcpyHostToDevice, s));
-  const float* yp; GN_TRY(forward(m, m->xin.p, batch, &yp, false));
-  GN_CUDA(cudaMemcpyAsync(out, yp, (size_t)batch * m->out_size * 4, cudaMemcpyDeviceToHost, s));
-  GN_CUDA(cudaStreamSynchronize(s)); return check_status_word(&m->ctx->c);
+  return forward_batch(m, x, batch, out);
 }
 
 int gn_device_alloc(gn_ctx* ctx, int64_t n, float** dev) {
@@ -1550,7 +1776,14 @@ int gn_device_download(gn_ctx* ctx, float* host, const float* dev, int64_t n) {
   GN_CUDA(cudaSetDevice(ctx->c.device)); GN_CUDA(cudaMemcpyAsync(host, dev, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->c.stream)); GN_CUDA(cudaStreamSynchronize(ctx->c.stream)); return GN_OK;
 }
 
-int gn_model_last_stats(gn_model* m, gn_step_stats* out) { CHECK_MODEL(m); if (!out) return fail(GN_ERR_INVALID_ARG, "out is null"); *out = m->stats; return GN_OK; }
+int gn_model_last_stats(gn_model* m, gn_step_stats* out) { CHECK_MODEL(m); if (!out) return fail(GN_ERR_INVALID_ARG, "out is null");
+  std::lock_guard<std::mutex> lk(m->mu);
+  if (!m->stats_timed && m->stats.kernel_launches > 0) {      // event times are read when somebody asks for them
+    cudaEventElapsedTime(&m->stats.step_ms, m->ev0, m->ev1);
+    m->stats.allreduce_ms = 0.f; if (m->ctx->c.world > 1) cudaEventElapsedTime(&m->stats.allreduce_ms, m->ar0, m->ar1);
+    m->stats_timed = true;
+  }
+  *out = m->stats; return GN_OK; }
 int gn_model_set_profiling(gn_model* m, int level) { CHECK_MODEL(m); m->ctx->c.profile = level; return GN_OK; }
 
 int gn_op_gemm_nt(gn_ctx* ctx, int engine, int M, int N, int K, const float* A, const float* B, const float* bias, float* C) {
@@ -1572,7 +1805,7 @@ int gn_op_adam(gn_ctx* ctx, float* params, const float* grads, float* m1, float*
   DevBuf dp, dg, dm, dv; size_t nn = (size_t)n; GN_TRY(dp.alloc(nn + 4)); GN_TRY(dg.alloc(nn + 4)); GN_TRY(dm.alloc(nn + 4)); GN_TRY(dv.alloc(nn + 4));
   GN_CUDA(copy_h2d(c, dp.p, params, nn * 4)); GN_CUDA(copy_h2d(c, dg.p, grads, nn * 4));
   GN_CUDA(copy_h2d(c, dm.p, m1, nn * 4)); GN_CUDA(copy_h2d(c, dv.p, v, nn * 4));
-  GN_TRY(adam_launch(c, dp.p, dg.p, dm.p, dv.p, n, lr, beta1, beta2, eps, t, grad_scale));
+  GN_TRY(adam_launch(c, dp.p, dg.p, dm.p, dv.p, n, adam_args(lr, beta1, beta2, eps, t, grad_scale), nullptr, nullptr, nullptr, nullptr, nullptr));
   GN_CUDA(cudaStreamSynchronize(c->stream));
   GN_CUDA(copy_d2h(c, params, dp.p, nn * 4)); GN_CUDA(copy_d2h(c, m1, dm.p, nn * 4)); GN_CUDA(copy_d2h(c, v, dv.p, nn * 4));
   return GN_OK;

@@ -76,7 +76,7 @@ int gn_op_softmax_ce(gn_ctx* ctx, int B, int V, int log_softmax, const float* z,
   float *Z = io.in(z, tot), *Y = io.in(y, tot), *A = io.out(tot), *G = io.out(tot), *Ls = io.out(B), *DZ = io.out(tot);
   GN_TRY(io.rc);
   GN_LAUNCH(c, softmax_rows_kernel, B, 256, 0, Z, A, V, log_softmax ? 1 : 0);
-  GN_LAUNCH(c, loss_rows_kernel, B, 256, 0, (const float*)A, (const float*)Y, G, Ls, V, (int)GN_LOSS_CROSS_ENTROPY);
+  GN_LAUNCH(c, loss_rows_kernel, B, 256, 0, (const float*)A, (const float*)Y, G, Ls, V, (int)GN_LOSS_CROSS_ENTROPY, reinterpret_cast<unsigned*>(c->d_status + 1), reinterpret_cast<float*>(c->d_status + 2));
   GN_LAUNCH(c, head_jacobian_kernel, B, 256, 0, (const float*)G, (const float*)A, DZ, V, log_softmax ? 1 : 0);
   GN_TRY(check_launch("op_softmax_ce"));
   GN_TRY(io.back(out, A, tot)); GN_TRY(io.back(loss, Ls, B)); GN_TRY(io.back(dz, DZ, tot));

@@ -4,6 +4,7 @@
 // samples and tokens, and the fused Adam update.  All are coalesced, 128-bit where the
 // shape allows, and reduce with warp shuffles.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include "common.cuh"
 
@@ -67,18 +68,29 @@ __global__ void softmax_rows_kernel(const float* __restrict__ z, float* __restri
   else for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = expf(zr[i] - mx) / s;
 }
 
+// The batch's loss sum (net.go:711-716), formed by the block that finishes last: `ticket` counts finished rows and is left at zero.
+// Strided sums per thread, then the block's tree: a fixed order.
+__device__ __forceinline__ void loss_row_done(float value, float* __restrict__ loss, int row, int rows, unsigned* __restrict__ ticket, float* __restrict__ total, float* red) {
+  __shared__ int is_last;
+  if (threadIdx.x == 0) { loss[row] = value; __threadfence(); is_last = atomicAdd(ticket, 1u) == (unsigned)rows - 1u; }
+  __syncthreads();
+  if (!is_last) return;
+  float s = 0.f;
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) s += __ldcg(loss + i);
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) { total[0] = s; *ticket = 0u; }
+}
 // Per-sample loss value and dL/dy.  reference: loss.go:53-68,91-105 (MSE), :120-140,165-178 (CrossEntropy:
 // value = -sum y*log(max(p,1e-10)); gradient returned as p - y).
 __global__ void loss_rows_kernel(const float* __restrict__ p, const float* __restrict__ y, float* __restrict__ grad,
-                                 float* __restrict__ loss, int n, int kind) {
+                                 float* __restrict__ loss, int n, int kind, unsigned* __restrict__ ticket, float* __restrict__ total) {
   __shared__ float red[33];
   const long off = (long)blockIdx.x * n;
   float s = 0.f;
   if (kind == GN_LOSS_MSE) {
     float f = 2.f / (float)n;
     for (int i = threadIdx.x; i < n; i += blockDim.x) { float d = p[off + i] - y[off + i]; s += d * d; grad[off + i] = f * d; }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) loss[blockIdx.x] = s / (float)n;
+    s = block_sum(s, red) / (float)n;
   } else {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       float pr = p[off + i], yy = y[off + i];
@@ -86,8 +98,61 @@ __global__ void loss_rows_kernel(const float* __restrict__ p, const float* __res
       if (yy != 0.f) s -= yy * logf(fmaxf(pr, 1e-10f));
     }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) loss[blockIdx.x] = s;
   }
+  loss_row_done(s, loss, blockIdx.x, gridDim.x, ticket, total, red);
+}
+// The whole head of a training step in one pass over the logits: softmax or log-softmax of z, the sample's loss against y, and
+// the gradient that reaches z (the loss gradient through the head's Jacobian, see head_jacobian_kernel).  A cluster of `cs`
+// blocks holds one row in registers, E values per thread; the four reductions (maximum, exponential sum, and loss and Jacobian
+// sum together) meet in distributed shared memory.  Three kernels of one block per row (softmax, loss, Jacobian) read
+// the row nine times: 180 us for 64 rows of 32000, against 21 now.
+constexpr int HEAD_THREADS = 256, HEAD_MAX_CS = 8, HEAD_MAX_E = 16;
+template <int E>
+__global__ void __launch_bounds__(HEAD_THREADS) head_loss_kernel(const float* __restrict__ z, const float* __restrict__ y, float* __restrict__ dz, float* __restrict__ loss,
+                                                                 int n, int rows, int cs, int log_mode, int kind, unsigned* __restrict__ ticket, float* __restrict__ total) {
+  __shared__ float red[33], slot[4];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int row = blockIdx.x / cs, rank = blockIdx.x % cs, i0 = rank * HEAD_THREADS * E + threadIdx.x; const long off = (long)row * n;
+  float v[E], t[E];
+  float mx = -INFINITY;
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int i = i0 + e * HEAD_THREADS; const bool in = i < n;
+    v[e] = in ? z[off + i] : -INFINITY; t[e] = in ? y[off + i] : 0.f; mx = fmaxf(mx, v[e]);
+  }
+  auto gather = [&](int k, float x, bool is_max) -> float {      // over the cluster's blocks, in rank order
+    if (cs == 1) return x;
+    if (threadIdx.x == 0) slot[k] = x;
+    cluster.sync();
+    float a = *cluster.map_shared_rank(&slot[k], 0);
+    for (int q = 1; q < cs; q++) { const float b = *cluster.map_shared_rank(&slot[k], q); a = is_max ? fmaxf(a, b) : a + b; }
+    return a;
+  };
+  mx = gather(0, block_max(mx, red), true);
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; e++) s += i0 + e * HEAD_THREADS < n ? expf(v[e] - mx) : 0.f;
+  s = gather(1, block_sum(s, red), false);
+  const float ls = logf(s), f = kind == GN_LOSS_MSE ? 2.f / (float)n : 1.f;
+  float lv = 0.f, js = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    if (i0 + e * HEAD_THREADS < n) {
+      const float p = log_mode ? v[e] - mx - ls : expf(v[e] - mx) / s, d = p - t[e], g = f * d;
+      if (kind == GN_LOSS_MSE) lv += d * d; else if (t[e] != 0.f) lv -= t[e] * logf(fmaxf(p, 1e-10f));
+      js += log_mode ? g : g * p;
+      v[e] = p; t[e] = g;
+    }
+  }
+  lv = gather(2, block_sum(lv, red), false);
+  js = gather(3, block_sum(js, red), false);
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int i = i0 + e * HEAD_THREADS;
+    if (i < n) dz[off + i] = log_mode ? t[e] - expf(v[e]) * js : v[e] * (t[e] - js);
+  }
+  if (cs > 1) cluster.sync();                                 // nobody leaves while its slots are being read
+  if (rank == 0) loss_row_done(kind == GN_LOSS_MSE ? lv / (float)n : lv, loss, row, rows, ticket, total, red);
 }
 
 // Dense.Backward for a Softmax head (layer.go:516-528):  dz_k = sum_i g_i p_i (delta_ik - p_k) = p_k (g_k - sum_i g_i p_i)
@@ -101,11 +166,6 @@ __global__ void head_jacobian_kernel(const float* __restrict__ g, const float* _
   s = block_sum(s, red);
   if (log_mode) for (int i = threadIdx.x; i < n; i += blockDim.x) dz[off + i] = g[off + i] - expf(out[off + i]) * s;
   else for (int i = threadIdx.x; i < n; i += blockDim.x) dz[off + i] = out[off + i] * (g[off + i] - s);
-}
-
-// mean loss = sum_s loss_s / global_batch; sequential like net.go:711-716 (one thread: B is small)
-__global__ void loss_total_kernel(const float* __restrict__ loss, int n, float* __restrict__ out_sum) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) { float s = 0.f; for (int i = 0; i < n; i++) s += loss[i]; out_sum[0] = s; }
 }
 
 // ---------------------------------------------------------------- reductions
@@ -240,7 +300,7 @@ __global__ void layernorm_bwd_kernel(const float* __restrict__ g, const float* _
     dr[i] = v;
   }
 }
-// gGamma[c] += sum_r g*(x-mean)/std ; gBeta[c] += sum_r g     (layernorm.go:421-433)
+// gGamma[c] = sum_r g*(x-mean)/std ; gBeta[c] = sum_r g     (layernorm.go:421-433)
 __global__ void layernorm_pgrad_partial_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ mean_in,
                                                const float* __restrict__ std_in, long rows, int n, float* __restrict__ part) {
   int c = blockIdx.x * blockDim.x + threadIdx.x; if (c >= n) return;
@@ -260,7 +320,7 @@ __global__ void __launch_bounds__(1024) layernorm_pgrad_final_kernel(const float
   if (grp == 0 && c < n) {
     float ta = 0.f, tb = 0.f;
     for (int k = 0; k < 32; k++) { ta += sa[k][tx]; tb += sb[k][tx]; }
-    gGamma[c] += ta; gBeta[c] += tb;
+    gGamma[c] = ta; gBeta[c] = tb;
   }
 }
 
@@ -406,7 +466,7 @@ __global__ void rmsnorm_pgrad_final_kernel(const float* __restrict__ part, int c
   int c = blockIdx.x * blockDim.x + threadIdx.x; if (c >= n) return;
   float a = 0.f;
   for (int k = 0; k < chunks; k++) a += part[(long)k * n + c];
-  gGamma[c] += a;
+  gGamma[c] = a;
 }
 
 // Norm backward on a few rows: rows s of g and dx are dense [rows, n], row s of the norm's input lies at x + s * ldx and its
@@ -515,23 +575,36 @@ __global__ void posenc_fwd_kernel(const float* __restrict__ x, const float* __re
 // the result to the row.  No two blocks touch the same row, so there are no atomics and the result does not depend on
 // scheduling; the samples of a batch are processed by consecutive launches in sample order (the order in which the
 // reference adds its workers' gradients, net.go:694-700).
-__global__ void embedding_bwd_sample_kernel(const float* __restrict__ g, const int* __restrict__ ids, float* __restrict__ gE, int T, int d) {
-  extern __shared__ int same[];                 // positions after t that hold the same id
-  __shared__ int n_same, first;
-  const int t = blockIdx.x, id = ids[t];
-  if (threadIdx.x == 0) {
-    first = 1; n_same = 0;
-    for (int u = 0; u < t; u++) if (ids[u] == id) { first = 0; break; }
-    if (first) for (int u = t + 1; u < T; u++) if (ids[u] == id) same[n_same++] = u;
+__global__ void __launch_bounds__(128) embedding_bwd_sample_kernel(const float* __restrict__ g, const int* __restrict__ ids, float* __restrict__ gE, int T, int d) {
+  extern __shared__ int same[];                 // positions after t that hold the same id, ascending
+  __shared__ int count[5];
+  const int t = blockIdx.x, id = ids[t], lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int mine = 0;
+  for (int u = threadIdx.x; u < t; u += 128) mine |= ids[u] == id;
+  if (__syncthreads_or(mine)) return;           // an earlier position of this id adds the row
+  int n_same = 0;
+  for (int u0 = t + 1; u0 < T; u0 += 128) {     // 128 positions at a time, kept in order (one thread walking the ids took 12 us)
+    const int u = u0 + threadIdx.x; const bool hit = u < T && ids[u] == id;
+    const unsigned b = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) count[w] = __popc(b);
+    __syncthreads();
+    int before = n_same;
+    for (int q = 0; q < w; q++) before += count[q];
+    if (hit) same[before + __popc(b & ((1u << lane) - 1u))] = u;
+    n_same += count[0] + count[1] + count[2] + count[3];
+    __syncthreads();
   }
-  __syncthreads();
-  if (!first) return;
   float* dst = gE + (long)id * d;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) {
+  for (int i = threadIdx.x; i < d; i += 128) {
     float s = g[(long)t * d + i];
     for (int k = 0; k < n_same; k++) s += g[(long)same[k] * d + i];
     dst[i] += s;
   }
+}
+// Results of a small inference call and the status word, straight to host memory.
+__global__ void finish_kernel(const float* __restrict__ src, float* __restrict__ dst, int n, const int* __restrict__ status, float* __restrict__ ret) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) ret[1] = __int_as_float(*status);
 }
 // Multi-GPU exchange of the few samples that reach the table: slot q of the buffers belongs to the q-th qualifying
 // sample of the global batch; the rank that owns it copies its gradient rows [T, d] and token ids (as floats) there,
@@ -647,6 +720,23 @@ __global__ void swiglu_bwd_rows_kernel(const float* __restrict__ dOut, const flo
     dUp[e] = go * sw; dGate[e] = go * (sw + sig * (1.f - sw)) * u;
   }
 }
+// What a block's backward pass needs when only token 0 has a gradient: token 0's rows of the two norms' inputs and their statistics
+// (st: mean 1 | deviation 1 | mean 2 | deviation 2, [B] each), the last token's rows of everything that meets a weight gradient.
+struct KeepRows { float *r2, *r1, *n1, *att, *x, *mid, *gate, *up, *st; };
+__global__ void __launch_bounds__(256) keep_rows_kernel(const float* __restrict__ r2, const float* __restrict__ r1, const float* __restrict__ n1, const float* __restrict__ att,
+                                                        const float* __restrict__ x, const float* __restrict__ mid, const float* __restrict__ gate, const float* __restrict__ up,
+                                                        const float* __restrict__ st, const KeepRows k, int T, int D, int F, int B) {
+  const long s = blockIdx.x, N = (long)B * T, first = s * T, last = first + T - 1;
+  for (int i = threadIdx.x; i < D; i += 256) {
+    k.r2[s * D + i] = r2[first * D + i]; k.r1[s * D + i] = r1[first * D + i];
+    k.n1[s * D + i] = n1[last * D + i]; k.att[s * D + i] = att[last * D + i]; k.x[s * D + i] = x[last * D + i];
+  }
+  for (int i = threadIdx.x; i < F; i += 256) {
+    if (mid) k.mid[s * F + i] = mid[last * F + i];
+    if (gate) { k.gate[s * F + i] = gate[last * F + i]; k.up[s * F + i] = up[last * F + i]; }
+  }
+  if (threadIdx.x < 4) k.st[threadIdx.x * (long)B + s] = st[threadIdx.x * N + first];
+}
 // dx[s, 0, :] += r[s, :]; one block per sequence
 __global__ void add_row0_kernel(const float* __restrict__ r, float* __restrict__ dx, int T, int d) {
   for (int i = threadIdx.x; i < d; i += blockDim.x) dx[(long)blockIdx.x * T * d + i] += r[(long)blockIdx.x * d + i];
@@ -673,9 +763,15 @@ __global__ void scale_kernel(float* __restrict__ x, long n, float s) {
 //   m = b1*m + (1-b1)*g' ; v = b2*v + (1-b2)*g'*g' ; p -= effLR * m / (sqrt(v) + eps)
 // `status` (may be null): the context's status word; when a bounded wait of an earlier kernel of this step gave up, the
 // gradients are not trustworthy and the pass leaves the parameters and moments untouched.
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, long n,
-                            float effLR, float b1, float b2, float omb1, float omb2, float eps, float grad_scale, const int* __restrict__ status) {
+// `dargs` (may be null): the coefficients are read from there instead of `a`, so that a captured launch follows the schedule.
+// `ret` (may be null; host memory): receives the step's loss sum and the status word, the caller's one read-back.
+struct AdamArgs { float effLR, b1, b2, omb1, omb2, eps, grad_scale; };
+__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, long n, const AdamArgs a, const AdamArgs* __restrict__ dargs,
+                            const int* __restrict__ status, const float* __restrict__ loss_sum, float* __restrict__ ret) {
+  if (ret && blockIdx.x == 0 && threadIdx.x == 0) { ret[0] = *loss_sum; ret[1] = __int_as_float(*status); }
   if (status && *status != 0) return;
+  const AdamArgs c = dargs ? *dargs : a;
+  const float effLR = c.effLR, b1 = c.b1, b2 = c.b2, omb1 = c.omb1, omb2 = c.omb2, eps = c.eps, grad_scale = c.grad_scale;
   // The four arrays are slices of the flat buffers at the same offset, so they share their position relative to a
   // 16-byte boundary: `head` leading elements are handled one by one, then float4s, then the tail.
   const long head = min(n, (long)((4 - ((reinterpret_cast<uintptr_t>(p) >> 2) & 3)) & 3));
@@ -722,6 +818,7 @@ __global__ void bn_fwd_kernel(const float* __restrict__ x, const float* __restri
 __global__ void bn_running_kernel(const float* __restrict__ stat, float* __restrict__ run, int B, int C, long BC, float mom) {
   int c = blockIdx.x * blockDim.x + threadIdx.x; if (c >= C) return;
   float rm = run[c], rv = run[C + c];
+#pragma unroll 8                                            // the loads of eight samples in flight; the updates stay in order (one sample at a time: 30 us for 50)
   for (int b = 0; b < B; b++) { rm = (1.f - mom) * rm + mom * stat[(long)b * C + c]; rv = (1.f - mom) * rv + mom * stat[2 * BC + (long)b * C + c]; }
   run[c] = rm; run[C + c] = rv;
 }
@@ -730,6 +827,7 @@ __global__ void bn_running_kernel(const float* __restrict__ stat, float* __restr
 __global__ void bn_running_gathered_kernel(const float* __restrict__ mean, const float* __restrict__ var, float* __restrict__ run, int B, int C, float mom) {
   int c = blockIdx.x * blockDim.x + threadIdx.x; if (c >= C) return;
   float rm = run[c], rv = run[C + c];
+#pragma unroll 8                                            // the loads of eight samples in flight; the updates stay in order (one sample at a time: 30 us for 50)
   for (int b = 0; b < B; b++) { rm = (1.f - mom) * rm + mom * mean[(long)b * C + c]; rv = (1.f - mom) * rv + mom * var[(long)b * C + c]; }
   run[c] = rm; run[C + c] = rv;
 }
