@@ -68,15 +68,29 @@ struct Ctx {
 
 inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 
-// Every kernel launch of the library goes through this macro so that the launch count is exact.
+// Every kernel launch of the library goes through these macros, so that the launch count is exact.
+// launch_kernel(): `cluster` > 0: that many neighbouring blocks of the grid's x dimension form a thread-block cluster; `early`: the
+// blocks may be placed while the preceding kernel still runs (programmatic stream serialisation), which wants a kernel that calls
+// pdl_wait() in every block before it touches anything its predecessors write, and pdl_launch() to let its own successor in.
+// (Launching every kernel of a step that way, waiting at its first instruction, was measured: within a replayed graph it is
+// slower than the ordinary edge, 78 -> 85 us for a step of 15 launches.  It pays where a kernel has something to fetch first.)
+template <class... P, class... A>
+inline cudaError_t launch_kernel(cudaStream_t stream, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster, bool early, A&&... args) {
+  cudaLaunchConfig_t cfg{}; cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute at[2]; int n = 0;
+  if (early) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n++].val.programmaticStreamSerializationAllowed = 1; }
+  if (cluster > 0) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1; n++; }
+  cfg.attrs = at; cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 #define GN_LAUNCH(ctx, kernel, grid, block, smem, ...)                         \
   do { kernel<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__); (ctx)->launches++; } while (0)
-
-// The same with `cx` neighbouring blocks of the grid's x dimension as one thread-block cluster.
 #define GN_CLUSTER_LAUNCH(ctx, kernel, grid, block, cx, ...)                   \
-  do { cudaLaunchConfig_t cfg_{}; cfg_.gridDim = (grid); cfg_.blockDim = dim3(block); cfg_.stream = (ctx)->stream;                                   \
-       cudaLaunchAttribute at_[1]; at_[0].id = cudaLaunchAttributeClusterDimension; at_[0].val.clusterDim.x = (cx); at_[0].val.clusterDim.y = at_[0].val.clusterDim.z = 1; \
-       cfg_.attrs = at_; cfg_.numAttrs = 1; GN_CUDA(cudaLaunchKernelEx(&cfg_, kernel, __VA_ARGS__)); (ctx)->launches++; } while (0)
+  do { GN_CUDA(gn::launch_kernel((ctx)->stream, kernel, dim3(grid), dim3(block), (size_t)0, cx, false, __VA_ARGS__)); (ctx)->launches++; } while (0)
+#define GN_EARLY_LAUNCH(ctx, kernel, grid, block, smem, ...)                   \
+  do { GN_CUDA(gn::launch_kernel((ctx)->stream, kernel, dim3(grid), dim3(block), (size_t)(smem), 0, true, __VA_ARGS__)); (ctx)->launches++; } while (0)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();

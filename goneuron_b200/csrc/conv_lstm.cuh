@@ -1,4 +1,4 @@
-// conv_lstm.cuh -- Conv2D / MaxPool2D kernels (NCHW) and the LSTM recurrence kernels.
+// conv_lstm.cuh -- Conv2D / MaxPool2D kernels (NCHW), wide GRUs, and the LSTM clipping recurrence on the gradient matrix itself.
 #pragma once
 #include <cooperative_groups.h>
 #include "common.cuh"
@@ -263,52 +263,7 @@ __global__ void avgpool_bwd_kernel(const float* __restrict__ g, float* __restric
   }
 }
 
-// ---------------------------------------------------------------- LSTM
-// Forward recurrence of one sample per block, thread i = hidden unit i.
-// reference: lstm.go:276-407.  The reference's gate helpers (lstm.go:1065-1101) run over the first H of the
-// 4H pre-activation rows, so only the input gate receives Wx*x + Wh*h; forget, cell and output gates see
-// their biases alone and are constant over time.
-// Saves per (sample, t): input-gate pre-activation, cell state, hidden state.
-// `xproj` != 0: pre_i already holds the input projection Wx[0:H] x_t of every (sample, t) (one tensor-core contraction
-// over all B*T rows, issued before this kernel); the kernel then only runs the recurrent part.
-__global__ void lstm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ Wx, const float* __restrict__ Wh, const float* __restrict__ bias,
-                                float* __restrict__ pre_i, float* __restrict__ c_all, float* __restrict__ h_all, float* __restrict__ out,
-                                int T, int in, int H, int return_seq, int xproj) {
-  extern __shared__ float sm[];
-  float* WhT = sm;                 // [H][H]  WhT[j*H+i] = Wh[i,j], rows 0..H-1 of the 4H
-  float* WxT = WhT + (long)H * H;  // [in][H]
-  float* hbuf = WxT + (long)in * H;  // [2][H]
-  float* xbuf = hbuf + 2 * H;        // [in]
-  const int s = blockIdx.x, i = threadIdx.x;
-  for (int e = threadIdx.x; e < H * H; e += blockDim.x) { int r = e / H, j = e % H; WhT[j * H + r] = Wh[e]; }
-  if (!xproj) for (int e = threadIdx.x; e < H * in; e += blockDim.x) { int r = e / in, j = e % in; WxT[j * H + r] = Wx[e]; }
-  if (i < H) { hbuf[i] = 0.f; hbuf[H + i] = 0.f; }
-  float bi = 0.f, fg = 0.f, cg = 0.f, og = 0.f, c = 0.f;
-  if (i < H) { bi = bias[i]; fg = act_fwd(GN_ACT_SIGMOID, bias[H + i]); cg = act_fwd(GN_ACT_TANH, bias[2 * H + i]); og = act_fwd(GN_ACT_SIGMOID, bias[3 * H + i]); }
-  __syncthreads();
-  const float* xs = x + (long)s * T * in;
-  for (int t = 0; t < T; t++) {
-    if (!xproj) { for (int e = threadIdx.x; e < in; e += blockDim.x) xbuf[e] = xs[(long)t * in + e]; }
-    __syncthreads();
-    const float* hp = hbuf + (t & 1) * H; float* hn = hbuf + ((t + 1) & 1) * H;
-    if (i < H) {
-      float sx = 0.f;
-      if (xproj) sx = pre_i[((long)s * T + t) * H + i];
-      else for (int j = 0; j < in; j++) sx = fmaf(WxT[j * H + i], xbuf[j], sx);
-      float pre = bi + sx;
-      for (int j = 0; j < H; j++) pre = fmaf(WhT[j * H + i], hp[j], pre);
-      float ig = act_fwd(GN_ACT_SIGMOID, pre);
-      c = fg * c + ig * cg;
-      float h = og * act_fwd(GN_ACT_TANH, c);
-      long o = ((long)s * T + t) * H + i;
-      pre_i[o] = pre; c_all[o] = c; h_all[o] = h; hn[i] = h;
-      if (return_seq) out[o] = h; else if (t == T - 1) out[(long)s * H + i] = h;
-    }
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------- GRU
+// ---------------------------------------------------------------- GRU with more than 128 units (smaller ones: recurrent.cuh)
 // Forward recurrence of one sample per block, thread i = hidden unit i.  reference: gru.go:192-288.
 // `pre` [B, T, 3H] holds b + Wx x_t of every step on entry (one contraction over all B*T rows, issued before) and the
 // complete pre-activations (update | reset | candidate) on exit.  The layer has 2H recurrent rows: the candidate's
@@ -385,44 +340,6 @@ __global__ void gru_bwd_kernel(const float* __restrict__ gout, const float* __re
     __syncthreads();
   }
 }
-// Back-propagation through time of one sample per block; writes the gate deltas D[s,t,4H].
-// reference: lstm.go:476-698 + unroller.go:190-209: the hidden-state gradient handed to step t-1 is the
-// gradient of step t PLUS Wh^T d (a running sum), because LSTM.Backward adds dhPrev into its argument.
-__global__ void lstm_bwd_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ bias,
-                                const float* __restrict__ pre_i, const float* __restrict__ c_all, float* __restrict__ D,
-                                int T, int H, int return_seq) {
-  extern __shared__ float sm[];
-  float* d = sm;   // [4H]
-  const int s = blockIdx.x, i = threadIdx.x;
-  float cur = 0.f, dcNext = 0.f, bf = 0.f, bg = 0.f, bo = 0.f;
-  if (i < H) { bf = bias[H + i]; bg = bias[2 * H + i]; bo = bias[3 * H + i]; }
-  for (int t = T - 1; t >= 0; t--) {
-    if (i < H) {
-      if (return_seq) cur += gout[((long)s * T + t) * H + i]; else if (t == T - 1) cur += gout[(long)s * H + i];
-      long o = ((long)s * T + t) * H + i;
-      float pre = pre_i[o], c = c_all[o], cprev = t > 0 ? c_all[o - H] : 0.f;
-      float ig = act_fwd(GN_ACT_SIGMOID, pre), fg = act_fwd(GN_ACT_SIGMOID, bf), cgt = act_fwd(GN_ACT_TANH, bg), og = act_fwd(GN_ACT_SIGMOID, bo);
-      float tanhC = act_fwd(GN_ACT_TANH, c);
-      float dc = cur * og * (1.f - tanhC * tanhC) + dcNext;
-      float di = dc * cgt * act_der(GN_ACT_SIGMOID, pre);
-      float df = dc * cprev * act_der(GN_ACT_SIGMOID, bf);
-      float dg = dc * ig * act_der(GN_ACT_TANH, bg);
-      float dout = cur * tanhC * act_der(GN_ACT_SIGMOID, bo);
-      dcNext = dc * fg;
-      d[i] = di; d[H + i] = df; d[2 * H + i] = dg; d[3 * H + i] = dout;
-      float* Dr = D + ((long)s * T + t) * 4 * H;
-      Dr[i] = di; Dr[H + i] = df; Dr[2 * H + i] = dg; Dr[3 * H + i] = dout;
-    }
-    __syncthreads();
-    if (i < H) {
-      float sum = 0.f;
-      for (int r = 0; r < 4 * H; r++) sum = fmaf(Wh[(long)r * H + i], d[r], sum);
-      cur += sum;
-    }
-    __syncthreads();
-  }
-}
-
 // The reference clips the WHOLE accumulated LSTM gradient to L2 norm <= 1 after every time-step of every
 // sample (lstm.go:694, :725-751), so the gradient of a worker chunk is a sequential recurrence over its
 // (sample, t) updates  g <- clip(g + d_k (x) [x_last ; h_{t-1} ; 1]).  One thread-block cluster runs one
@@ -492,155 +409,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) lstm_grad_scan_kernel(
     else o[(long)R4 * in + (long)R4 * H + gr] = v;
   }
   cluster.sync();
-}
-
-
-// ---------------------------------------------------------------- the same recurrence through Gram matrices
-// Every update is rank one, u_k = d_k (x) z_k, so the gradient after any number of clipped updates is a weighted sum
-// g = sum_j w_j u_j, and the only thing the clipping needs is the norm:
-//     |g + u_k|^2 = |g|^2 + 2 <g, u_k> + |u_k|^2,   <u_j, u_k> = <d_j, d_k> <z_j, z_k> =: G[j,k].
-// With f_k the clip factor of update k and S_k = f_0 ... f_k, the coefficient of u_j after update k is S_k / S_{j-1},
-// hence <g_{k-1}, u_k> = S_{k-1} sum_{j<k} G[j,k] / S_{j-1}.  The two Gram products and the final g = (diag(w) D)^T Z
-// are contractions (tensor cores); what stays sequential is one dot product of length k per update.
-//
-// Rows of Dm [n, 4H] and Zm [n, in+H+1] in update order: chunk by chunk, samples ascending, time descending.
-__global__ void lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all,
-                                           float* __restrict__ Dm, float* __restrict__ Zm, int T, int in, int H, long n_updates) {
-  const int R4 = 4 * H, ZW = in + H + 1;
-  const long k = blockIdx.x; if (k >= n_updates) return;
-  const int s = (int)(k / T), t = T - 1 - (int)(k % T);
-  for (int e = threadIdx.x; e < R4 + ZW; e += blockDim.x) {
-    if (e < R4) Dm[k * R4 + e] = D[((long)s * T + t) * R4 + e];
-    else {
-      const int c = e - R4; float v;
-      if (c < in) v = x[(long)s * T * in + (long)(T - 1) * in + c];                 // input of the LAST forward call (lstm.go:592-621)
-      else if (c < in + H) v = t > 0 ? h_all[((long)s * T + (t - 1)) * H + (c - in)] : 0.f;
-      else v = 1.f;
-      Zm[k * ZW + c] = v;
-    }
-  }
-}
-// G <- G (.) G2 on the lower triangles (row k, columns j <= k) of `nb` matrices of size Kc x Kc
-__global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restrict__ G2, int Kc, long total) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int j = (int)(i % Kc), k = (int)((i / Kc) % Kc);
-    if (j <= k) G[i] *= G2[i];
-  }
-}
-// The updates of a worker chunk are walked in groups of GRAM_BS.  cw[j] holds the CURRENT coefficient of update j (the
-// product of all clip factors applied since it was added: at most 1, and free to underflow to 0, which is then also
-// what the literal recurrence has made of that update).  For the group starting at k0,
-//     v[r] = sum_{j<k0} cw[j] G[k0+r, j] = <g_{k0-1}, u_{k0+r}>
-// is a matrix-vector product over all SMs (lstm_gram_prefix_kernel, one block per row and chunk); inside the group the
-// earlier updates only get scaled by s = product of the group's clip factors so far, and the group's own GRAM_BS
-// coefficients live in shared memory and are walked sequentially by one warp (lstm_gram_group_kernel), which finally
-// scales cw[0..k0) by s and appends its own.  The two kernels are launched once per group; the stream orders them.
-// The norm recurrence and the coefficients are kept in double.  n2[chunk] = |g|^2.
-constexpr int GRAM_BS = 128, GRAM_MAX_K = 1 << 20;
-constexpr size_t GRAM_GROUP_SMEM = (size_t)GRAM_BS * (GRAM_BS + 1) * sizeof(float);
-__global__ void lstm_gram_prefix_kernel(const float* __restrict__ G, const double* __restrict__ cw, double* __restrict__ v, int Kc, long n_total, int k0) {
-  __shared__ double red[8];
-  const int chunk = blockIdx.y, r = blockIdx.x, tid = threadIdx.x;
-  const long first = (long)chunk * Kc; const int n = (int)max(0L, min((long)Kc, n_total - first));
-  if (k0 + r >= n) return;
-  const float* row = G + (long)chunk * Kc * Kc + (long)(k0 + r) * Kc; const double* c = cw + first;
-  double acc = 0.0;
-  int j = tid;
-  for (; j + 3 * 256 < k0; j += 4 * 256)
-    acc += (c[j] * (double)row[j] + c[j + 256] * (double)row[j + 256]) + (c[j + 512] * (double)row[j + 512] + c[j + 768] * (double)row[j + 768]);
-  for (; j < k0; j += 256) acc += c[j] * (double)row[j];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((tid & 31) == 0) red[tid >> 5] = acc;
-  __syncthreads();
-  if (tid == 0) { double a = 0.0; for (int q = 0; q < 8; q++) a += red[q]; v[(long)chunk * GRAM_BS + r] = a; }
-}
-// One warp walks the group.  Lane l owns rows l, l+32, ... of the diagonal block and keeps for each of them
-//     q[r'] = <g, u_{k0+r'}>  under the gradient g as it stands after the steps done so far,
-// which starts at v[r'] and follows q <- f (q + G[r'][r]) when step r adds u_r and scales by the clip factor f.  Step r
-// therefore needs one broadcast of q[r] and no reduction.  The factors are kept, and the group's coefficients are
-// their suffix products.
-__global__ void __launch_bounds__(256) lstm_gram_group_kernel(const float* __restrict__ G, double* __restrict__ cw, const double* __restrict__ v,
-                                                              double* __restrict__ n2buf, int Kc, long n_total, int k0) {
-  constexpr int QN = GRAM_BS / 32;
-  extern __shared__ __align__(16) float gram_smem[];
-  float (*Gd)[GRAM_BS + 1] = reinterpret_cast<float (*)[GRAM_BS + 1]>(gram_smem);
-  __shared__ double fr[GRAM_BS], om[GRAM_BS];
-  const int chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long first = (long)chunk * Kc; const int n = (int)max(0L, min((long)Kc, n_total - first));
-  if (k0 >= n) return;
-  const int nb = min(GRAM_BS, n - k0);
-  const float* Gc = G + (long)chunk * Kc * Kc; double* c = cw + first;
-  for (int e = tid; e < GRAM_BS * GRAM_BS; e += 256) {
-    const int r = e / GRAM_BS, q = e % GRAM_BS;
-    Gd[r][q] = (r < nb && q < nb) ? Gc[(long)(k0 + r) * Kc + k0 + q] : 0.f;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    double n2 = k0 == 0 ? 0.0 : n2buf[chunk];
-    double q[QN];
-#pragma unroll
-    for (int i = 0; i < QN; i++) { const int r = lane + 32 * i; q[i] = (k0 > 0 && r < nb) ? v[(long)chunk * GRAM_BS + r] : 0.0; }
-    // the block's column r and its diagonal entry are fetched one step ahead, so that the step itself is only the
-    // broadcast, the norm update and the clip factor (single-precision reciprocal square root + one Newton step)
-    float gcol[QN], gdiag = Gd[0][0];
-#pragma unroll
-    for (int i2 = 0; i2 < QN; i2++) gcol[i2] = Gd[lane + 32 * i2][0];
-#pragma unroll
-    for (int i = 0; i < QN; i++) {
-      for (int rl = 0; rl < 32; rl++) {
-        const int r = 32 * i + rl;
-        if (r >= nb) break;
-        const double qr = __shfl_sync(0xffffffffu, q[i], rl);
-        float ncol[QN]; const int rn = min(r + 1, GRAM_BS - 1);
-#pragma unroll
-        for (int i2 = 0; i2 < QN; i2++) ncol[i2] = Gd[lane + 32 * i2][rn];
-        const float ndiag = Gd[rn][rn];
-        double qg[QN];
-#pragma unroll
-        for (int i2 = 0; i2 < QN; i2++) qg[i2] = q[i2] + (double)gcol[i2];
-        const double np = n2 + 2.0 * qr + (double)gdiag;
-        double f0 = (double)rsqrtf((float)np);
-        f0 = f0 * (1.5 - 0.5 * np * f0 * f0);
-        const bool clip = np > 1.0;                                               // clip to norm 1 (lstm.go:738-750)
-        const double f = clip ? f0 : 1.0;
-        n2 = clip ? 1.0 : np;
-#pragma unroll
-        for (int i2 = 0; i2 < QN; i2++) { q[i2] = f * qg[i2]; gcol[i2] = ncol[i2]; }
-        gdiag = ndiag;
-        if (lane == 0) fr[r] = f;
-      }
-    }
-    __syncwarp();
-    if (lane == 0) {
-      double a = 1.0;
-      for (int r = nb - 1; r >= 0; r--) { a *= fr[r]; om[r] = a; }
-      n2buf[chunk] = n2;
-    }
-  }
-  __syncthreads();
-  const double sg = om[0];
-  for (int j = tid; j < k0; j += 256) c[j] *= sg;
-  if (tid < nb) c[k0 + tid] = om[tid];
-}
-// w[j] = (float) cw[j], zero beyond the chunk's last update
-__global__ void lstm_gram_weights_kernel(const double* __restrict__ cw, float* __restrict__ w, int Kc, long n_total, long total) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long chunk = i / Kc; const long n = max(0L, min((long)Kc, n_total - chunk * Kc));
-    w[i] = (i - chunk * Kc) < n ? (float)cw[i] : 0.f;
-  }
-}
-__global__ void lstm_scale_rows_kernel(float* __restrict__ Dm, const float* __restrict__ w, int R4, long total) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) Dm[i] *= w[i / R4];
-}
-// chunk results [nchunks][4H][in+H+1] -> flat layout gWx[4H,in] | gWh[4H,H] | gb[4H], chunks added in worker order
-__global__ void lstm_scatter_grad_kernel(const float* __restrict__ Gc, int nchunks, int in, int H, float* __restrict__ out) {
-  const int R4 = 4 * H, ZW = in + H + 1; const long total = (long)R4 * ZW;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int r = (int)(i / ZW), c = (int)(i % ZW);
-    float v = 0.f; for (int q = 0; q < nchunks; q++) v += Gc[(long)q * total + i];
-    if (c < in) out[(long)r * in + c] = v; else if (c < in + H) out[(long)R4 * in + (long)r * H + (c - in)] = v; else out[(long)R4 * in + (long)R4 * H + r] = v;
-  }
 }
 
 }  // namespace gn

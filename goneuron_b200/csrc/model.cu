@@ -24,6 +24,7 @@
 #include "gemm_tc.cuh"
 #include "rowops.cuh"
 #include "conv_lstm.cuh"
+#include "recurrent.cuh"
 #include "attention.cuh"
 #include "attention_tc.cuh"
 #include "conv_tc.cuh"
@@ -307,7 +308,7 @@ static int alloc_activations(gn_model* m, int cap, bool training) {
       case GN_LAYER_FLATTEN: break;
       case GN_LAYER_LSTM_UNROLLED: {
         size_t th = c * d.seq_len * d.out_size;
-        GN_TRY(l.out.alloc(c * l.out_size)); GN_TRY(l.pre_i.alloc(th)); GN_TRY(l.c_all.alloc(th)); GN_TRY(l.h_all.alloc(th)); GN_TRY(l.dgate.alloc(4 * th)); break; }
+        GN_TRY(l.out.alloc(c * l.out_size)); GN_TRY(l.pre_i.alloc(th)); GN_TRY(l.c_all.alloc(th)); GN_TRY(l.h_all.alloc(th)); GN_TRY(l.z.alloc(th)); GN_TRY(l.dgate.alloc(4 * th)); break; }      // pre_i: input gates, z: tanh of the cell states
       case GN_LAYER_GRU_UNROLLED: {
         size_t th = c * d.seq_len * d.out_size;     // pre_i: pre-activations [.,T,3H]; c_all: h_{t-1}; z: r (.) h_{t-1}; dgate: deltas [.,T,3H]
         GN_TRY(l.out.alloc(c * l.out_size)); GN_TRY(l.pre_i.alloc(3 * th)); GN_TRY(l.c_all.alloc(th)); GN_TRY(l.h_all.alloc(th)); GN_TRY(l.z.alloc(th)); GN_TRY(l.dgate.alloc(3 * th)); break; }
@@ -693,26 +694,20 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
         cur = l.out.p; break; }
       case GN_LAYER_FLATTEN: break;
       case GN_LAYER_LSTM_UNROLLED: {
-        int H = d.out_size, in = d.in_size; int threads = ((H + 31) / 32) * 32;
-        size_t smem = ((size_t)H * H + (size_t)in * H + 2 * H + in) * sizeof(float);
+        const int H = d.out_size, in = d.in_size, T = d.seq_len;
+        const size_t smem = ((size_t)H * H + (size_t)in * H + 2 * H + in) * sizeof(float);
         if (smem > 200 * 1024) return fail(GN_ERR_UNSUPPORTED, "LSTM of hidden size %d needs %zu bytes of shared memory", H, smem);
-        GN_CUDA(cudaFuncSetAttribute(lstm_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        // The input projection has no recurrence in it: Wx[0:H] x_t for all B*T rows is one contraction on the tensor cores
-        // (only the first H of the 4H gate rows receive it, lstm.go:319-326, :1065-1101); the kernel then adds the bias and
-        // the recurrent product step by step.
-        int xproj = 0;
-        {
-          GemmDesc g; g.M = B * d.seq_len; g.N = H; g.K = in; g.A = cur; g.sa_m = in; g.sa_k = 1; g.B = p; g.sb_k = 1; g.sb_n = in; g.C = l.pre_i.p; g.ldc = H;
-          if (!force_simt_engine() && gemm_tc_supported(ctx, g)) { GN_TRY(gemm_tc(ctx, g)); ctx->gemm_flops += 2.0 * g.M * (double)g.N * g.K; ctx->gemm_launches++; xproj = 1; }
-        }
-        GN_LAUNCH(ctx, lstm_fwd_kernel, B, threads, smem, cur, p, p + (long)4 * H * in, p + (long)4 * H * in + (long)4 * H * H,
-                  l.pre_i.p, l.c_all.p, l.h_all.p, l.out.p, d.seq_len, in, H, d.return_seq, xproj);
+        // The input projection has no recurrence in it: Wx[0:H] x_t for all B*T rows is one contraction (only the first H of the
+        // 4H gate rows receive it, lstm.go:319-326, :1065-1101); the kernel adds the bias and the recurrent product step by step.
+        GN_TRY(gemm_nt(ctx, B * T, H, in, cur, in, p, nullptr, l.pre_i.p, H));
+        GN_TRY(lstm_fwd(ctx, p + (long)4 * H * in, p + (long)4 * H * in + (long)4 * H * H, l.pre_i.p, l.c_all.p, l.z.p, l.h_all.p, l.out.p, RecShape{T, in, H, d.return_seq, B}));
         cur = l.out.p; break; }
       case GN_LAYER_GRU_UNROLLED: {
         const int H = d.out_size, in = d.in_size, T = d.seq_len, threads = ((H + 31) / 32) * 32;
         const float* Wx = p; const float* Wh = p + (long)3 * H * in; const float* bias = Wh + (long)2 * H * H;
         // input projection of all three gates and all B*T rows as one contraction (bias in its epilogue), then the recurrence
         GN_TRY(gemm_nt(ctx, B * T, 3 * H, in, cur, in, Wx, bias, l.pre_i.p, 3 * H));
+        if (gru_reg_ok(H)) { GN_TRY(gru_fwd_reg(ctx, Wh, l.pre_i.p, l.h_all.p, l.out.p, RecShape{T, in, H, d.return_seq, B})); cur = l.out.p; break; }
         const size_t smem = ((size_t)2 * H * H + 3 * (size_t)H) * sizeof(float);
         GN_CUDA(cudaFuncSetAttribute(gru_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         GN_LAUNCH(ctx, gru_fwd_kernel, B, threads, smem, Wh, l.pre_i.p, l.h_all.p, l.out.p, T, H, d.return_seq);
@@ -998,8 +993,7 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
 static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float* xin, const float* gout, int global_batch, int first_sample, float* dx) {
   Ctx* ctx = &m->ctx->c; const gn_layer_desc& d = l.d; const int H = d.out_size, in = d.in_size, T = d.seq_len;
   const float* p = m->params.p + l.p_off; const float* Wx = p; const float* Wh = p + (long)4 * H * in; const float* bias = Wh + (long)4 * H * H;
-  int threads = ((H + 31) / 32) * 32;
-  GN_LAUNCH(ctx, lstm_bwd_kernel, B, threads, (size_t)4 * H * sizeof(float), gout, Wh, bias, l.pre_i.p, l.c_all.p, l.dgate.p, T, H, d.return_seq);
+  GN_TRY(lstm_bwd(ctx, gout, Wh, bias, l.pre_i.p, l.c_all.p, l.z.p, l.dgate.p, RecShape{T, in, H, d.return_seq, B}));
   if (li > 0) GN_TRY(gemm_nn(ctx, B * T, 4 * H, in, l.dgate.p, 4 * H, Wx, dx, in));   // dx_t = Wx^T d_t
   // The clipping recurrence (lstm.go:694, :725-751) walks the rank-1 updates d_k z_k^T of a whole worker chunk in sample
   // order, and a chunk may span ranks.  With more than one rank every rank therefore gathers the update factors of the
@@ -1010,48 +1004,48 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
   l.grad_replicated = world > 1;
   int chunk = (global_batch + m->W - 1) / m->W, nchunks = (GB + chunk - 1) / chunk;
   {
-    // Gram-matrix form of the clipping recurrence (conv_lstm.cuh): the default whenever its matrices fit.  The
-    // cluster kernel below runs only for chunks too long for it, or when GONEURON_CUDA_LSTM_SCAN=cluster asks for it.
+    // The walk over scalars (recurrent.cuh) is the default; GONEURON_CUDA_LSTM_SCAN=cluster asks for the kernel below, which
+    // applies the updates one by one to the matrix and otherwise runs only for chunks that are too long.
     static const int mode = [] { const char* e = getenv("GONEURON_CUDA_LSTM_SCAN"); return !e ? 0 : (strcmp(e, "cluster") == 0 ? 1 : (strcmp(e, "gram") == 0 ? 2 : 0)); }();
-    const long Kc = (long)chunk * T, n_updates = (long)GB * T, n_local = (long)B * T; const int R4g = 4 * H, ZWg = in + H + 1;
-    const bool fits = Kc <= GRAM_MAX_K && (double)nchunks * Kc * Kc * 8 <= 8.0e9;
-    if (world > 1 && !(mode != 1 && fits)) return fail(GN_ERR_UNSUPPORTED, "LSTM on more than one GPU needs the Gram form of the clipping recurrence (worker chunk of %ld updates)", Kc);
+    const int R4g = 4 * H, ZWg = in + H + 1, zs = clip_zs(ZWg), slabs = cdiv(R4g, 8);
+    const long Kc = (long)chunk * T, n_updates = (long)GB * T, n_local = (long)B * T, groups = (Kc + CG - 1) / CG, stride = CG_PAD + groups * CG, ng = (long)nchunks * groups, rows = nchunks * stride;
+    const bool fits = Kc <= CG_MAX_K && ng <= 65535;
+    if (world > 1 && !(mode != 1 && fits)) return fail(GN_ERR_UNSUPPORTED, "LSTM on more than one GPU needs the scalar form of the clipping recurrence (worker chunk of %ld updates)", Kc);
     if (mode != 1 && fits) {
-      float *G0, *G1, *Dm, *Zm, *wv, *res;
-      GN_TRY(ensure(m, S_GRAM0, (size_t)nchunks * Kc * Kc, &G0)); GN_TRY(ensure(m, S_GRAM1, (size_t)nchunks * Kc * Kc, &G1));
-      GN_TRY(ensure(m, S_DM, (size_t)nchunks * Kc * R4g, &Dm)); GN_TRY(ensure(m, S_ZM, (size_t)nchunks * Kc * ZWg, &Zm));
-      GN_TRY(ensure(m, S_W, (size_t)nchunks * Kc, &wv)); GN_TRY(ensure(m, S_SCAN, (size_t)nchunks * R4g * ZWg, &res));
-      if ((long)nchunks * Kc > n_updates) {     // the last chunk is short: its unused rows must be zero for the final contraction
-        GN_CUDA(cudaMemsetAsync(Dm, 0, (size_t)nchunks * Kc * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm, 0, (size_t)nchunks * Kc * ZWg * 4, ctx->stream));
-        GN_CUDA(cudaMemsetAsync(wv, 0, (size_t)nchunks * Kc * 4, ctx->stream));
+      float *G0, *G1, *Dm, *Zm, *dbl, *gmat;
+      const size_t n_om = (size_t)ng * CG, n_p = (size_t)nchunks * 2 * CG * slabs;
+      GN_TRY(ensure(m, S_GRAM0, (size_t)ng * CG * 2 * CG, &G0)); GN_TRY(ensure(m, S_GRAM1, (size_t)ng * CG * 2 * CG, &G1));
+      GN_TRY(ensure(m, S_DM, (size_t)rows * R4g, &Dm)); GN_TRY(ensure(m, S_ZM, (size_t)rows * zs, &Zm));
+      GN_TRY(ensure(m, S_TV, 2 * (n_om + n_p + (size_t)ng * 2), &dbl)); GN_TRY(ensure(m, S_SCAN, (size_t)nchunks * 2 * R4g * ZWg, &gmat));
+      // rows of zeros: the group before every chunk's first, and what its last group lacks
+      if (nchunks > 8) { GN_CUDA(cudaMemsetAsync(Dm, 0, (size_t)rows * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm, 0, (size_t)rows * zs * 4, ctx->stream)); }
+      else for (int c = 0; c < nchunks; c++) {
+        const long n = std::min(Kc, n_updates - c * Kc), r0 = c * stride, r1 = r0 + CG_PAD + n, left = stride - CG_PAD - n;
+        GN_CUDA(cudaMemsetAsync(Dm + r0 * R4g, 0, (size_t)CG_PAD * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm + r0 * zs, 0, (size_t)CG_PAD * zs * 4, ctx->stream));
+        if (left > 0) { GN_CUDA(cudaMemsetAsync(Dm + r1 * R4g, 0, (size_t)left * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm + r1 * zs, 0, (size_t)left * zs * 4, ctx->stream)); }
       }
-      float* Dloc = Dm + (size_t)row0 * T * R4g; float* Zloc = Zm + (size_t)row0 * T * ZWg;      // this rank's rows inside the global arrays
-      GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)n_local, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dloc, Zloc, T, in, H, n_local);
       if (world > 1) {
-        GN_TRY(all_gather_on_comm(m, Dloc, Dm, (size_t)n_local * R4g, "LSTM update factors D"));
-        GN_TRY(all_gather_on_comm(m, Zloc, Zm, (size_t)n_local * ZWg, "LSTM update factors Z"));
-      }
-      GemmDesc g; g.M = (int)Kc; g.N = (int)Kc; g.batch1 = nchunks; g.c_b1 = Kc * Kc; g.ldc = Kc; g.flags = GEMM_SKIP_UPPER;
-      g.K = R4g; g.A = Dm; g.sa_m = R4g; g.sa_k = 1; g.B = Dm; g.sb_k = 1; g.sb_n = R4g; g.a_b1 = g.b_b1 = Kc * R4g; g.C = G0; GN_TRY(gemm(ctx, g));
-      g.K = ZWg; g.A = Zm; g.sa_m = ZWg; g.B = Zm; g.sb_n = ZWg; g.a_b1 = g.b_b1 = Kc * ZWg; g.C = G1; GN_TRY(gemm(ctx, g));
-      const long tot = (long)nchunks * Kc * Kc;
-      GN_LAUNCH(ctx, lstm_gram_mul_kernel, ew_grid(ctx, tot), 256, 0, G0, (const float*)G1, (int)Kc, tot);
-      // cw (double) | v (double, one group) | |g|^2 per chunk (double) live in one scratch slot
-      float* tv; GN_TRY(ensure(m, S_TV, (size_t)2 * ((size_t)nchunks * Kc + (size_t)nchunks * GRAM_BS + 2 * nchunks + 2), &tv));
-      double* tco = reinterpret_cast<double*>(tv); double* vbuf = tco + (size_t)nchunks * Kc; double* state = vbuf + (size_t)nchunks * GRAM_BS;
-      GN_CUDA(cudaFuncSetAttribute(lstm_gram_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GRAM_GROUP_SMEM));
-      for (int k0 = 0; k0 < Kc; k0 += GRAM_BS) {
-        if (k0 > 0) GN_LAUNCH(ctx, lstm_gram_prefix_kernel, dim3(GRAM_BS, nchunks), 256, 0, (const float*)G0, (const double*)tco, vbuf, (int)Kc, n_updates, k0);
-        GN_LAUNCH(ctx, lstm_gram_group_kernel, nchunks, 256, GRAM_GROUP_SMEM, (const float*)G0, tco, (const double*)vbuf, state, (int)Kc, n_updates, k0);
-      }
-      const long wtot = (long)nchunks * Kc;
-      GN_LAUNCH(ctx, lstm_gram_weights_kernel, ew_grid(ctx, wtot), 256, 0, (const double*)tco, wv, (int)Kc, n_updates, wtot);
-      const long dtot = (long)nchunks * Kc * R4g;
-      GN_LAUNCH(ctx, lstm_scale_rows_kernel, ew_grid(ctx, dtot), 256, 0, Dm, (const float*)wv, R4g, dtot);
-      GemmDesc f; f.M = R4g; f.N = ZWg; f.K = (int)Kc; f.batch1 = nchunks; f.A = Dm; f.sa_m = 1; f.sa_k = R4g; f.a_b1 = Kc * R4g;
-      f.B = Zm; f.sb_k = ZWg; f.sb_n = 1; f.b_b1 = Kc * ZWg; f.C = res; f.ldc = ZWg; f.c_b1 = (long)R4g * ZWg; GN_TRY(gemm(ctx, f));
-      GN_LAUNCH(ctx, lstm_scatter_grad_kernel, cdiv((long)R4g * ZWg, 256), 256, 0, (const float*)res, nchunks, in, H, m->grads.p + l.p_off);
-      return check_launch("lstm_backward(gram)");
+        float* all; GN_TRY(ensure(m, S_W, (size_t)n_updates * (R4g + zs), &all));
+        float* Da = all; float* Za = all + (size_t)n_updates * R4g; float* Dl = Da + (size_t)row0 * T * R4g; float* Zl = Za + (size_t)row0 * T * zs;      // this rank's rows
+        GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)n_local, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, n_local, n_local, 0L, 0L);
+        GN_TRY(all_gather_on_comm(m, Dl, Da, (size_t)n_local * R4g, "LSTM update factors D"));
+        GN_TRY(all_gather_on_comm(m, Zl, Za, (size_t)n_local * zs, "LSTM update factors Z"));
+        GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Da, Dm, R4g, Kc, stride, (long)CG_PAD);
+        GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Za, Zm, zs, Kc, stride, (long)CG_PAD);
+      } else GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)n_local, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dm, Zm, T, in, H, zs, n_local, Kc, stride, (long)CG_PAD);
+      // Gram blocks of every group against the group before it and itself
+      GemmDesc g; g.M = CG; g.N = 2 * CG; g.batch1 = nchunks; g.batch2 = (int)groups; g.ldc = 2 * CG; g.c_b1 = groups * CG * 2 * CG; g.c_b2 = CG * 2 * CG; g.sa_k = g.sb_k = 1;
+      g.K = R4g; g.A = Dm + (long)CG_PAD * R4g; g.sa_m = R4g; g.B = Dm; g.sb_n = R4g; g.a_b1 = g.b_b1 = stride * R4g; g.a_b2 = g.b_b2 = (long)CG * R4g; g.C = G0; GN_TRY(gemm(ctx, g));
+      g.K = ZWg; g.A = Zm + (long)CG_PAD * zs; g.sa_m = zs; g.B = Zm; g.sb_n = zs; g.a_b1 = g.b_b1 = stride * zs; g.a_b2 = g.b_b2 = (long)CG * zs; g.C = G1; GN_TRY(gemm(ctx, g));
+      const long q4 = ng * CG * 2 * CG / 4;
+      GN_LAUNCH(ctx, lstm_gram_mul_kernel, ew_grid(ctx, q4), 256, 0, G0, (const float*)G1, q4);
+      double* db = reinterpret_cast<double*>(dbl);
+      const ClipArgs a{Dm, Zm, G0, db, db + n_om, db + n_om + n_p, gmat, R4g, ZWg, (int)groups, slabs, stride};
+      const size_t smem = clip_smem(ZWg);
+      GN_CUDA(cudaFuncSetAttribute(lstm_clip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      for (int j = 0; j <= groups; j++) GN_EARLY_LAUNCH(ctx, lstm_clip_kernel, dim3(1 + slabs, nchunks), CG_THREADS, smem, a, j);
+      GN_LAUNCH(ctx, lstm_scatter_grad_kernel, cdiv((long)R4g * ZWg, 256), 256, 0, (const float*)gmat, (int)(groups & 1), nchunks, in, H, m->grads.p + l.p_off);
+      return check_launch("lstm_backward");
     }
   }
   const int R4 = 4 * H, ZW = in + H + 1, rpc = (R4 + SCAN_CLUSTER - 1) / SCAN_CLUSTER;
@@ -1170,7 +1164,8 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         const int H = d.out_size, in = d.in_size, T = d.seq_len, threads = ((H + 31) / 32) * 32;
         const float* Wx = p; const float* Wh = p + (long)3 * H * in;
         float* gWx = gr; float* gWh = gr + (long)3 * H * in; float* gb = gWh + (long)2 * H * H;
-        GN_LAUNCH(ctx, gru_bwd_kernel, B, threads, (size_t)2 * H * sizeof(float), g, Wh, (const float*)l.pre_i.p, (const float*)l.h_all.p, l.dgate.p, l.c_all.p, l.z.p, T, H, d.return_seq);
+        if (gru_reg_ok(H)) GN_TRY(gru_bwd_reg(ctx, g, Wh, l.pre_i.p, l.h_all.p, l.dgate.p, l.c_all.p, l.z.p, RecShape{T, in, H, d.return_seq, B}));
+        else GN_LAUNCH(ctx, gru_bwd_kernel, B, threads, (size_t)2 * H * sizeof(float), g, Wh, (const float*)l.pre_i.p, (const float*)l.h_all.p, l.dgate.p, l.c_all.p, l.z.p, T, H, d.return_seq);
         // input weights and biases: every step's delta meets the input of the LAST forward call (gru.go:429-447), so per sample
         // gWx = (sum_t d_t) (x) x_{T-1}: the same batch-level contraction as the inner Dense layers of a TransformerBlock
         GN_TRY(inner_dense_param_grads(m, l.dgate.p, B, T, 3 * H, xin, in, gWx, gb));

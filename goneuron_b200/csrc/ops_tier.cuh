@@ -91,26 +91,22 @@ int gn_op_lstm(gn_ctx* ctx, int engine, int B, int T, int in_size, int H, const 
   Ctx* c = &ctx->c; std::lock_guard<std::mutex> run_lk(c->run_mu); GN_CUDA(cudaSetDevice(c->device));
   HostIO io(c); const size_t th = (size_t)B * T * H;
   float *X = io.in(x, (size_t)B * T * in_size), *Wx = io.in(wx, (size_t)4 * H * in_size), *Wh = io.in(wh, (size_t)4 * H * H), *Bi = io.in(bias, (size_t)4 * H);
-  float *pre = io.out(th), *C_ = io.out(th), *Hh = io.out(th), *out = io.out((size_t)B * H);
+  float *ig = io.out(th), *tc = io.out(th), *C_ = io.out(th), *Hh = io.out(th), *out = io.out((size_t)B * H);
   GN_TRY(io.rc);
-  const int threads = ((H + 31) / 32) * 32;
   const size_t smem = ((size_t)H * H + (size_t)in_size * H + 2 * H + in_size) * sizeof(float);
   if (smem > 200 * 1024) return fail(GN_ERR_UNSUPPORTED, "op_lstm: hidden size %d needs %zu bytes of shared memory", H, smem);
-  GN_CUDA(cudaFuncSetAttribute(lstm_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int xproj = 0;
+  GemmDesc g; g.M = B * T; g.N = H; g.K = in_size; g.A = X; g.sa_m = in_size; g.sa_k = 1; g.B = Wx; g.sb_k = 1; g.sb_n = in_size; g.C = ig; g.ldc = H;
   if (engine == 1) {
-    GemmDesc g; g.M = B * T; g.N = H; g.K = in_size; g.A = X; g.sa_m = in_size; g.sa_k = 1; g.B = Wx; g.sb_k = 1; g.sb_n = in_size; g.C = pre; g.ldc = H;
     if (!gemm_tc_supported(c, g)) return fail(GN_ERR_UNSUPPORTED, "op_lstm: the tensor-core engine is not available");
-    GN_TRY(gemm_tc(c, g)); xproj = 1;
-  }
-  GN_LAUNCH(c, lstm_fwd_kernel, B, threads, smem, (const float*)X, (const float*)Wx, (const float*)Wh, (const float*)Bi, pre, C_, Hh, out, T, in_size, H, 0, xproj);
-  GN_TRY(check_launch("op_lstm forward"));
+    GN_TRY(gemm_tc(c, g));
+  } else GN_TRY(gemm_simt(c, g));
+  const RecShape q{T, in_size, H, 0, B};
+  GN_TRY(lstm_fwd(c, Wh, Bi, ig, C_, tc, Hh, out, q));
   GN_TRY(io.back(h_all, Hh, th)); GN_TRY(io.back(c_all, C_, th));
   if (dh_last) {
     float *G = io.in(dh_last, (size_t)B * H), *D = io.out(4 * th);
     GN_TRY(io.rc);
-    GN_LAUNCH(c, lstm_bwd_kernel, B, threads, (size_t)4 * H * sizeof(float), (const float*)G, (const float*)Wh, (const float*)Bi, (const float*)pre, (const float*)C_, D, T, H, 0);
-    GN_TRY(check_launch("op_lstm backward"));
+    GN_TRY(lstm_bwd(c, G, Wh, Bi, ig, C_, tc, D, q));
     GN_TRY(io.back(dgate, D, 4 * th));
   }
   return check_status_word(c);

@@ -1,0 +1,563 @@
+// recurrent.cuh -- LSTM and GRU recurrences, forward and back-propagation through time, and the LSTM gradient-clipping recurrence.
+#pragma once
+#include <cooperative_groups.h>
+#include "common.cuh"
+#include "rowops.cuh"
+
+namespace gn {
+
+// ------------------------------------------------------------------ recurrence kernels
+// A recurrence is a chain of T small matrix-vector products, bound by the latency of one step.  A block owns NS samples (two when
+// there are more samples than SMs) and has four threads per hidden unit, each with a quarter of the unit's dot product: a step
+// is a quarter of the multiply-adds in a row, one exchange through shared memory, and the activations.  For up to 128
+// hidden units a thread keeps its weights in registers for the whole sequence (RU_Q per matrix).  One thread per unit with the
+// weights in shared memory (forward) or L2 (backward) took 147 / 888 us for the LSTM of 128 units, 64 steps, 256 samples.
+constexpr int RU_Q = 32;
+struct RecShape { int T, in, H, return_seq, B; };
+__host__ __device__ __forceinline__ int rec_hp(int H) { return (H + 31) & ~31; }
+__host__ __device__ __forceinline__ int rec_jq(int H) { return (((H + 3) / 4) + 3) & ~3; }        // length of a quarter, a multiple of 4
+
+// dot product of a quarter: w . v over jq values; w in registers (REGS) or at ws[jj * ld]
+template <bool REGS>
+__device__ __forceinline__ float rec_dot(const float (&w)[RU_Q], const float* __restrict__ ws, int ld, const float* __restrict__ v, int jq) {
+  float a = 0.f, b = 0.f;
+  if (REGS) {
+#pragma unroll
+    for (int j = 0; j < RU_Q; j += 8) {
+      if (j < jq) { const float4 x = *reinterpret_cast<const float4*>(v + j); a = fmaf(w[j], x.x, a); b = fmaf(w[j + 1], x.y, b); a = fmaf(w[j + 2], x.z, a); b = fmaf(w[j + 3], x.w, b); }
+      if (j + 4 < jq) { const float4 x = *reinterpret_cast<const float4*>(v + j + 4); a = fmaf(w[j + 4], x.x, a); b = fmaf(w[j + 5], x.y, b); a = fmaf(w[j + 6], x.z, a); b = fmaf(w[j + 7], x.w, b); }
+    }
+  } else {
+#pragma unroll 4
+    for (int j = 0; j < jq; j += 2) { a = fmaf(ws[j * ld], v[j], a); b = fmaf(ws[(j + 1) * ld], v[j + 1], b); }
+  }
+  return a + b;
+}
+
+// LSTM forward.  reference: lstm.go:276-407.  The reference's gate helpers (lstm.go:1065-1101) run over the first H of the 4H
+// pre-activation rows, so only the input gate receives Wx x + Wh h; forget, cell and output gates see their biases alone and
+// are constant over time.  `ig` holds the input projections Wx[0:H] x_t of every (sample, step) on entry (one contraction, issued
+// before) and the input gate on exit; cell, tanh(cell) and hidden states are kept too.
+template <int NS, bool REGS>
+__global__ void __launch_bounds__(REGS ? 512 : 1024) lstm_fwd_kernel(const float* __restrict__ Wh, const float* __restrict__ bias, float* __restrict__ ig_all, float* __restrict__ c_all,
+                                                                     float* __restrict__ tc_all, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
+  extern __shared__ __align__(16) float sm[];
+  const int H = q_.H, T = q_.T, Hp = rec_hp(H), jq = rec_jq(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
+  float* hb = sm;                              // [2][NS][4 jq]
+  float* part = hb + 2 * NS * 4 * jq;          // [4][NS][Hp]
+  float* ws = part + 4 * NS * Hp;              // !REGS: [4 jq][Hp]
+  float w[RU_Q];
+  if (REGS) {
+#pragma unroll
+    for (int j = 0; j < RU_Q; j++) { const int k = q * jq + j; w[j] = (i < H && j < jq && k < H) ? Wh[(long)i * H + k] : 0.f; }
+  } else for (int e = threadIdx.x; e < 4 * jq * Hp; e += blockDim.x) { const int k = e / Hp, r = e - k * Hp; ws[e] = (r < H && k < H) ? Wh[(long)r * H + k] : 0.f; }
+  for (int e = threadIdx.x; e < 2 * NS * 4 * jq; e += blockDim.x) hb[e] = 0.f;
+  // the elementwise part of (sample, unit): the first NS * Hp threads
+  const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
+  float bi = 0.f, fg = 0.f, cg = 0.f, og = 0.f, c = 0.f, x = 0.f;
+  const long base = ((long)s * T) * H + i;
+  if (el) {
+    bi = bias[i]; fg = act_fwd(GN_ACT_SIGMOID, bias[H + i]); cg = act_fwd(GN_ACT_TANH, bias[2 * H + i]); og = act_fwd(GN_ACT_SIGMOID, bias[3 * H + i]);
+    x = ig_all[base];
+  }
+  __syncthreads();
+  for (int t = 0; t < T; t++) {
+    const float* hp = hb + (t & 1) * NS * 4 * jq; float* hn = hb + ((t + 1) & 1) * NS * 4 * jq;
+#pragma unroll
+    for (int k = 0; k < NS; k++) part[(q * NS + k) * Hp + i] = rec_dot<REGS>(w, ws + (q * jq) * Hp + i, Hp, hp + k * 4 * jq + q * jq, jq);
+    __syncthreads();
+    if (el) {
+      const long o = base + (long)t * H;
+      float pre = bi + x;
+      if (t + 1 < T) x = ig_all[o + H];
+#pragma unroll
+      for (int k = 0; k < 4; k++) pre += part[(k * NS + es) * Hp + i];
+      const float ig = act_fwd(GN_ACT_SIGMOID, pre);
+      c = fg * c + ig * cg;
+      const float tc = act_fwd(GN_ACT_TANH, c), h = og * tc;
+      hn[es * 4 * jq + i] = h;
+      ig_all[o] = ig; c_all[o] = c; tc_all[o] = tc; h_all[o] = h;
+      if (q_.return_seq) out[o] = h; else if (t == T - 1) out[(long)s * H + i] = h;
+    }
+    __syncthreads();
+  }
+}
+
+// LSTM back-propagation through time; writes the gate deltas D[s, t, 4H].  reference: lstm.go:476-698 + unroller.go:190-209: the
+// hidden-state gradient handed to step t-1 is the gradient of step t PLUS Wh^T d (a running sum), because LSTM.Backward adds
+// dhPrev into its argument.  Thread (gate q, unit i) sums over gate q's H rows of column i: the first `rs` rows (a multiple of
+// four) from shared memory, the next RR from registers, the rest (none up to 128 units) from global memory.
+template <int NS, int RR, int MAXT>
+__global__ void __launch_bounds__(MAXT) lstm_bwd_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ bias, const float* __restrict__ ig_all,
+                                                        const float* __restrict__ c_all, const float* __restrict__ tc_all, float* __restrict__ D, const RecShape q_, int rs) {
+  extern __shared__ __align__(16) float sm[];
+  const int H = q_.H, T = q_.T, Hp = rec_hp(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
+  float* db = sm;                              // [NS][4][Hp]
+  float* part = db + NS * 4 * Hp;              // [4][NS][Hp]
+  float* ws = part + 4 * NS * Hp;              // [rs][4][Hp]
+  for (int e = threadIdx.x; e < rs * 4 * Hp; e += blockDim.x) { const int r = e / (4 * Hp), gq = (e / Hp) & 3, c = e % Hp; ws[e] = c < H ? Wh[((long)gq * H + r) * H + c] : 0.f; }
+  float w[RR];
+#pragma unroll
+  for (int j = 0; j < RR; j++) w[j] = (i < H && rs + j < H) ? Wh[((long)q * H + rs + j) * H + i] : 0.f;
+  for (int e = threadIdx.x; e < NS * 4 * Hp; e += blockDim.x) db[e] = 0.f;
+  const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
+  float cur = 0.f, dcn = 0.f, fg = 0.f, cg = 0.f, og = 0.f, kf = 0.f, kg = 0.f, ko = 0.f, ig = 0.f, tc = 0.f, cp = 0.f;
+  const long base = ((long)s * T) * H + i;
+  if (el) {
+    const float bf = bias[H + i], bg = bias[2 * H + i], bo = bias[3 * H + i];
+    fg = act_fwd(GN_ACT_SIGMOID, bf); cg = act_fwd(GN_ACT_TANH, bg); og = act_fwd(GN_ACT_SIGMOID, bo);
+    kf = act_der(GN_ACT_SIGMOID, bf); kg = act_der(GN_ACT_TANH, bg); ko = act_der(GN_ACT_SIGMOID, bo);
+    const long o = base + (long)(T - 1) * H;
+    ig = ig_all[o]; tc = tc_all[o]; cp = T > 1 ? c_all[o - H] : 0.f;
+    if (!q_.return_seq) cur = gout[(long)s * H + i];
+  }
+  __syncthreads();
+  for (int t = T - 1; t >= 0; t--) {
+    if (el) {
+      const long o = base + (long)t * H;
+      if (q_.return_seq) cur += gout[o];
+      const float dc = cur * og * (1.f - tc * tc) + dcn;
+      const float di = dc * cg * (ig * (1.f - ig)), df = dc * cp * kf, dg = dc * ig * kg, dq = cur * tc * ko;
+      dcn = dc * fg;
+      float* d = db + es * 4 * Hp + i; d[0] = di; d[Hp] = df; d[2 * Hp] = dg; d[3 * Hp] = dq;
+      float* Dr = D + ((long)s * T + t) * 4 * H + i; Dr[0] = di; Dr[H] = df; Dr[2 * H] = dg; Dr[3 * H] = dq;
+      if (t > 0) { ig = ig_all[o - H]; tc = tc_all[o - H]; cp = t > 1 ? c_all[o - 2 * H] : 0.f; }
+    }
+    if (t == 0) break;
+    __syncthreads();
+    float acc[NS];
+#pragma unroll
+    for (int k = 0; k < NS; k++) acc[k] = 0.f;
+    const float* d0 = db + q * Hp; const float* wq = ws + q * Hp + i;
+#pragma unroll 4
+    for (int r = 0; r < rs; r += 4) {
+      const float w0 = wq[r * 4 * Hp], w1 = wq[(r + 1) * 4 * Hp], w2 = wq[(r + 2) * 4 * Hp], w3 = wq[(r + 3) * 4 * Hp];
+#pragma unroll
+      for (int k = 0; k < NS; k++) { const float4 x = *reinterpret_cast<const float4*>(d0 + k * 4 * Hp + r); acc[k] = fmaf(w0, x.x, fmaf(w1, x.y, fmaf(w2, x.z, fmaf(w3, x.w, acc[k])))); }
+    }
+#pragma unroll
+    for (int j = 0; j < RR; j += 4) {
+      if (rs + j < Hp) {                       // (rows H .. Hp - 1 of d are zero; Hp and rs are multiples of four)
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+          const float4 x = *reinterpret_cast<const float4*>(d0 + k * 4 * Hp + rs + j);
+          acc[k] = fmaf(w[j], x.x, fmaf(w[j + 1], x.y, fmaf(w[j + 2], x.z, fmaf(w[j + 3], x.w, acc[k]))));
+        }
+      }
+    }
+    if (i < H) for (int r = rs + RR; r < H; r++) {
+      const float wv = __ldg(Wh + ((long)q * H + r) * H + i);
+#pragma unroll
+      for (int k = 0; k < NS; k++) acc[k] = fmaf(wv, d0[k * 4 * Hp + r], acc[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < NS; k++) part[(q * NS + k) * Hp + i] = acc[k];
+    __syncthreads();
+    if (el) cur += (part[es * Hp + i] + part[(NS + es) * Hp + i]) + (part[(2 * NS + es) * Hp + i] + part[(3 * NS + es) * Hp + i]);
+  }
+}
+
+// GRU forward for up to 128 units.  reference: gru.go:192-288.  `gates` [B, T, 3H] holds b + Wx x_t of every step on entry (one
+// contraction over all rows, issued before) and the gate values z | r | candidate on exit.  The layer has 2H recurrent rows: the
+// candidate's recurrent product uses the reset gate's rows on r (.) h_prev (gru.go:247-258).
+template <int NS>
+__global__ void __launch_bounds__(512) gru_fwd_reg_kernel(const float* __restrict__ Wh, float* __restrict__ gates, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
+  extern __shared__ __align__(16) float sm[];
+  const int H = q_.H, T = q_.T, Hp = rec_hp(H), jq = rec_jq(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
+  float* hb = sm;                              // [NS][4 jq]  h_prev
+  float* rb = hb + NS * 4 * jq;                // [NS][4 jq]  r (.) h_prev
+  float* part = rb + NS * 4 * jq;              // [2][4][NS][Hp]
+  float wz[RU_Q], wr[RU_Q];
+#pragma unroll
+  for (int j = 0; j < RU_Q; j++) {
+    const int k = q * jq + j; const bool in = i < H && j < jq && k < H;
+    wz[j] = in ? Wh[(long)i * H + k] : 0.f; wr[j] = in ? Wh[(long)(H + i) * H + k] : 0.f;
+  }
+  for (int e = threadIdx.x; e < 2 * NS * 4 * jq; e += blockDim.x) hb[e] = 0.f;
+  const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
+  float* gp = gates + (long)s * T * 3 * H + i; float h = 0.f, az = 0.f, ar = 0.f, ac = 0.f;
+  if (el) { az = gp[0]; ar = gp[H]; ac = gp[2 * H]; }
+  __syncthreads();
+  for (int t = 0; t < T; t++) {
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+      const float* v = hb + k * 4 * jq + q * jq;
+      part[(q * NS + k) * Hp + i] = rec_dot<true>(wz, nullptr, 0, v, jq);
+      part[((4 + q) * NS + k) * Hp + i] = rec_dot<true>(wr, nullptr, 0, v, jq);
+    }
+    __syncthreads();
+    float z = 0.f, r = 0.f;
+    if (el) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) { az += part[(k * NS + es) * Hp + i]; ar += part[((4 + k) * NS + es) * Hp + i]; }
+      r = act_fwd(GN_ACT_SIGMOID, ar);
+      rb[es * 4 * jq + i] = r * h;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NS; k++) part[(q * NS + k) * Hp + i] = rec_dot<true>(wr, nullptr, 0, rb + k * 4 * jq + q * jq, jq);
+    if (el) z = act_fwd(GN_ACT_SIGMOID, az);
+    __syncthreads();
+    if (el) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) ac += part[(k * NS + es) * Hp + i];
+      const float c = act_fwd(GN_ACT_TANH, ac);
+      h = h + z * (c - h);
+      hb[es * 4 * jq + i] = h;
+      float* g = gp + (long)t * 3 * H; g[0] = z; g[H] = r; g[2 * H] = c;
+      const long o = ((long)s * T + t) * H + i;
+      h_all[o] = h;
+      if (q_.return_seq) out[o] = h; else if (t == T - 1) out[(long)s * H + i] = h;
+      if (t + 1 < T) { g += 3 * H; az = g[0]; ar = g[H]; ac = g[2 * H]; }
+    }
+    __syncthreads();
+  }
+}
+// GRU back-propagation through time for up to 128 units.  reference: gru.go:360-534 with unroller.go:190-209, literal: the reset
+// gate's delta is never formed (stays zero), the candidate's gradient is scaled by (1 - z) and the hidden-state pass-through by
+// z, the candidate's contribution to dh_prev is indexed by the output unit's reset gate, and dh_prev is ADDED to the incoming
+// gradient before it is handed to the previous step.  Writes the gate deltas D [B,T,3H] (update | zero | candidate), h_{t-1} [B,T,H]
+// and r (.) h_{t-1} [B,T,H] for the weight-gradient contractions.
+template <int NS>
+__global__ void __launch_bounds__(512) gru_bwd_reg_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ gates, const float* __restrict__ h_all,
+                                                          float* __restrict__ D, float* __restrict__ hprev_all, float* __restrict__ rh_all, const RecShape q_) {
+  extern __shared__ __align__(16) float sm[];
+  const int H = q_.H, T = q_.T, Hp = rec_hp(H), jq = rec_jq(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
+  float* ub = sm;                              // [NS][4 jq]  update deltas
+  float* cb = ub + NS * 4 * jq;                // [NS][4 jq]  candidate deltas times r
+  float* part = cb + NS * 4 * jq;              // [4][NS][Hp]
+  float wz[RU_Q], wr[RU_Q];
+#pragma unroll
+  for (int j = 0; j < RU_Q; j++) {
+    const int k = q * jq + j; const bool in = i < H && j < jq && k < H;
+    wz[j] = in ? Wh[(long)k * H + i] : 0.f; wr[j] = in ? Wh[((long)H + k) * H + i] : 0.f;
+  }
+  for (int e = threadIdx.x; e < 2 * NS * 4 * jq; e += blockDim.x) ub[e] = 0.f;
+  const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
+  const float* gp = gates + (long)s * T * 3 * H + i; const long base = ((long)s * T) * H + i;
+  float cur = 0.f, z = 0.f, r = 0.f, c = 0.f, hp = 0.f;
+  if (el) {
+    const float* g = gp + (long)(T - 1) * 3 * H; z = g[0]; r = g[H]; c = g[2 * H]; hp = T > 1 ? h_all[base + (long)(T - 2) * H] : 0.f;
+    if (!q_.return_seq) cur = gout[(long)s * H + i];
+  }
+  __syncthreads();
+  for (int t = T - 1; t >= 0; t--) {
+    const float zt = z;
+    if (el) {
+      const long o = base + (long)t * H;
+      if (q_.return_seq) cur += gout[o];
+      const float du = cur * (c - hp) * z * (1.f - z), dc = cur * (1.f - z) * (1.f - c * c);
+      float* Dr = D + ((long)s * T + t) * 3 * H + i; Dr[0] = du; Dr[H] = 0.f; Dr[2 * H] = dc;
+      hprev_all[o] = hp; rh_all[o] = r * hp;
+      ub[es * 4 * jq + i] = du; cb[es * 4 * jq + i] = dc * r;
+      if (t > 0) { const float* g = gp + (long)(t - 1) * 3 * H; z = g[0]; r = g[H]; c = g[2 * H]; hp = t > 1 ? h_all[o - 2 * H] : 0.f; }
+    }
+    if (t == 0) break;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NS; k++)
+      part[(q * NS + k) * Hp + i] = rec_dot<true>(wz, nullptr, 0, ub + k * 4 * jq + q * jq, jq) + rec_dot<true>(wr, nullptr, 0, cb + k * 4 * jq + q * jq, jq);
+    __syncthreads();
+    if (el) { const float sum = (part[es * Hp + i] + part[(NS + es) * Hp + i]) + (part[(2 * NS + es) * Hp + i] + part[(3 * NS + es) * Hp + i]); cur = cur + (sum + cur * zt); }
+  }
+}
+
+// ------------------------------------------------------------------ launchers
+inline int lstm_fwd(Ctx* ctx, const float* Wh, const float* bias, float* ig, float* c, float* tc, float* h, float* out, const RecShape& q) {
+  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const bool regs = q.H <= 4 * RU_Q;
+  const size_t smem = ((size_t)2 * ns * 4 * jq + 4 * ns * Hp + (regs ? 0 : (size_t)4 * jq * Hp)) * sizeof(float);
+  auto* K = regs ? (ns == 2 ? lstm_fwd_kernel<2, true> : lstm_fwd_kernel<1, true>) : (ns == 2 ? lstm_fwd_kernel<2, false> : lstm_fwd_kernel<1, false>);
+  if (4 * Hp > 1024 || smem > 220 * 1024) return fail(GN_ERR_UNSUPPORTED, "LSTM of hidden size %d needs %zu bytes of shared memory", q.H, smem);
+  GN_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GN_LAUNCH(ctx, K, cdiv(q.B, ns), 4 * Hp, smem, Wh, bias, ig, c, tc, h, out, q);
+  return check_launch("lstm_fwd");
+}
+inline int lstm_bwd(Ctx* ctx, const float* gout, const float* Wh, const float* bias, const float* ig, const float* c, const float* tc, float* D, const RecShape& q) {
+  const int Hp = rec_hp(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const bool small = Hp <= 128;
+  const size_t fixed = (size_t)8 * ns * Hp * sizeof(float), row = (size_t)4 * Hp * sizeof(float);
+  // registers hold 64 (24) rows of each gate's column, shared memory as many of the others as fit, in fours
+  const int rs = (int)std::min<size_t>((std::max(0, q.H - (small ? 64 : 24)) + 3) & ~3, ((200 * 1024 - fixed) / row) & ~(size_t)3); const size_t smem = fixed + rs * row;
+  auto* K = small ? (ns == 2 ? lstm_bwd_kernel<2, 64, 512> : lstm_bwd_kernel<1, 64, 512>) : (ns == 2 ? lstm_bwd_kernel<2, 24, 1024> : lstm_bwd_kernel<1, 24, 1024>);
+  GN_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GN_LAUNCH(ctx, K, cdiv(q.B, ns), 4 * Hp, smem, gout, Wh, bias, ig, c, tc, D, q, rs);
+  return check_launch("lstm_bwd");
+}
+inline bool gru_reg_ok(int H) { return H <= 4 * RU_Q; }
+inline int gru_fwd_reg(Ctx* ctx, const float* Wh, float* gates, float* h, float* out, const RecShape& q) {
+  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const size_t smem = ((size_t)8 * ns * jq + 8 * ns * Hp) * sizeof(float);
+  GN_LAUNCH(ctx, (ns == 2 ? gru_fwd_reg_kernel<2> : gru_fwd_reg_kernel<1>), cdiv(q.B, ns), 4 * Hp, smem, Wh, gates, h, out, q);
+  return check_launch("gru_fwd");
+}
+inline int gru_bwd_reg(Ctx* ctx, const float* gout, const float* Wh, const float* gates, const float* h, float* D, float* hprev, float* rh, const RecShape& q) {
+  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const size_t smem = ((size_t)8 * ns * jq + 4 * ns * Hp) * sizeof(float);
+  GN_LAUNCH(ctx, (ns == 2 ? gru_bwd_reg_kernel<2> : gru_bwd_reg_kernel<1>), cdiv(q.B, ns), 4 * Hp, smem, gout, Wh, gates, h, D, hprev, rh, q);
+  return check_launch("gru_bwd");
+}
+
+// ------------------------------------------------------------------ LSTM gradient clipping
+// The reference clips the WHOLE accumulated LSTM gradient to L2 norm <= 1 after every time-step of every sample (lstm.go:694,
+// :725-751): g <- clip(g + u_k) over the rank-one updates u_k = d_k z_k^T of a worker chunk, z_k = [x_last ; h_{t-1} ; 1], samples
+// ascending, time descending.  The clipping needs only the norm, |g + u_k|^2 = |g|^2 + 2 <g, u_k> + |u_k|^2, so the walk is over
+// scalars; it goes in groups of CG updates.  Within a group the inner products come from the group's own Gram block, <u_q, u_r>
+// = <d_q, d_r> <z_q, z_r>; across groups <g, u_r> = d_r^T g z_r comes from the gradient matrix itself, formed one group ahead, and
+// the Gram block against the group before.  One launch per group (all inputs come from earlier launches: nothing waits inside
+// one; g_j is the gradient before group j):
+//   block 0     walks group j: v = s_{j-1} p_j + X_j om_{j-1}, then CG dependent steps; leaves om_j[r], the weight of u_r in the
+//               gradient after the group, and s_j, the weight of what was there before
+//   the others  eight rows of the matrix each: g_j = s_{j-1} g_{j-1} + sum_r om_{j-1}[r] d_r z_r^T, and that slab's part of
+//               p_{j+1}[r] = d_r^T g_j z_r for the updates of group j+1
+// (The full Gram matrix of all updates, 16384^2 for 256 samples of 64 steps, took two products of 137 GFLOP, 1 GB, and a pass over
+// all earlier updates per group: 7.1 ms.  This takes 1.3.)
+// Norms, factors and the sums over updates are kept in double.
+constexpr int CG = 128, CG_THREADS = 512, CG_PAD = CG, CG_TILE = 160;        // CG_PAD: rows of zeros before a chunk: group -1
+constexpr int CG_GD = CG + 1;
+constexpr long CG_MAX_K = 1L << 20;                         // updates per worker chunk
+__host__ __device__ __forceinline__ int clip_zs(int ZW) { return (ZW + 3) & ~3; }                 // row stride of Zm
+__host__ __device__ __forceinline__ int clip_tile(int ZW) { const int n = (ZW + CG_TILE - 1) / CG_TILE; return (ZW + n - 1) / n; }
+inline size_t clip_smem(int ZW) {
+  const int wp = clip_tile(ZW) | 1; const size_t slab = ((size_t)2 * CG * wp + CG * 8 + (size_t)wp * 8 + 8) * sizeof(float), walk = (size_t)CG * CG_GD * sizeof(double);
+  return slab > walk ? slab : walk;
+}
+// Rows of Dm [., 4H] and Zm [., zs]: chunk c's updates from row c * stride + lead on.  k: update in global order.
+__global__ void lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
+                                           int T, int in, int H, int zs, long n_updates, long Kc, long stride, long lead) {
+  const int R4 = 4 * H, ZW = in + H + 1;
+  const long k = blockIdx.x; if (k >= n_updates) return;
+  const int s = (int)(k / T), t = T - 1 - (int)(k % T); const long row = (k / Kc) * stride + lead + k % Kc;
+  for (int e = threadIdx.x; e < R4 + zs; e += blockDim.x) {
+    if (e < R4) Dm[row * R4 + e] = D[((long)s * T + t) * R4 + e];
+    else {
+      const int c = e - R4; float v;
+      if (c < in) v = x[(long)s * T * in + (long)(T - 1) * in + c];                 // input of the LAST forward call (lstm.go:592-621)
+      else if (c < in + H) v = t > 0 ? h_all[((long)s * T + (t - 1)) * H + (c - in)] : 0.f;
+      else v = c < ZW ? 1.f : 0.f;
+      Zm[row * zs + c] = v;
+    }
+  }
+}
+// rows of `w` floats from contiguous order into the chunks' layout (after a gather over the ranks)
+__global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int w, long Kc, long stride, long lead) {
+  const long k = blockIdx.x, row = (k / Kc) * stride + lead + k % Kc;
+  for (int e = threadIdx.x; e < w; e += blockDim.x) dst[row * w + e] = src[k * w + e];
+}
+__global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restrict__ G2, long total4) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total4; i += (long)gridDim.x * blockDim.x) {
+    float4 a = reinterpret_cast<float4*>(G)[i]; const float4 b = reinterpret_cast<const float4*>(G2)[i];
+    a.x *= b.x; a.y *= b.y; a.z *= b.z; a.w *= b.w; reinterpret_cast<float4*>(G)[i] = a;
+  }
+}
+struct ClipArgs {
+  const float *D, *Z, *G;        // rows of a chunk start at chunk * stride (CG_PAD rows of zeros first); G [chunk][group][CG][2 CG]: against groups j-1, j
+  double *om, *p, *st;           // [chunk][groups][CG] weights of a group's updates; [chunk][2][CG][slabs] parts of p by parity of the group; [chunk][groups][2]: s_j, |g|^2
+  float* g;                      // [chunk][2][4H][ZW]
+  int R4, ZW, groups, slabs; long stride;
+};
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__global__ void __launch_bounds__(CG_THREADS) lstm_clip_kernel(const ClipArgs a, int j) {
+  extern __shared__ __align__(16) float sm[];
+  const int chunk = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R4 = a.R4, ZW = a.ZW, zs = clip_zs(ZW);
+  double* om = a.om + (long)chunk * a.groups * CG; double* st = a.st + (long)chunk * a.groups * 2; double* pp = a.p + (long)chunk * 2 * CG * a.slabs;
+  // Z and the Gram blocks are written before the loop over the groups: launch 0 waits for them, and the next launch is only let
+  // in (pdl_launch) behind a wait, so every later launch can fetch them before it waits for its predecessor.
+  if (j == 0) pdl_wait();
+  if (blockIdx.x == 0) {
+    if (j >= a.groups) { pdl_wait(); return; }
+    double* Gd = reinterpret_cast<double*>(sm);                   // [CG][CG_GD]
+    __shared__ double vs[CG], fs[CG], cs[2][33];
+    const float* Gj = a.G + ((long)chunk * a.groups + j) * CG * 2 * CG;
+    const double* pj = pp + (long)(j & 1) * CG * a.slabs;
+    double x[CG / 16][4];                                         // the Gram blocks come from before the loop over the groups
+#pragma unroll
+    for (int k = 0; k < CG / 16; k++) {
+      const int r = warp + 16 * k; const float* gr = Gj + (long)r * 2 * CG + lane; double* gd = Gd + r * CG_GD + lane;
+#pragma unroll
+      for (int q = 0; q < 4; q++) { x[k][q] = gr[32 * q]; gd[32 * q] = gr[CG + 32 * q]; }
+    }
+    pdl_wait(); pdl_launch();
+    const double s1 = j >= 1 ? st[2 * (j - 1)] : 0.0;            // s_{j-1}
+    {   // v_r: a warp per eight rows, a row's terms over the lanes
+      double v[CG / 16];
+#pragma unroll
+      for (int k = 0; k < CG / 16; k++) v[k] = 0.0;
+      if (j >= 1) {
+        const double* o = om + (long)(j - 1) * CG + lane; double ov[4], ps[CG / 16][4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) ov[q] = o[32 * q];
+#pragma unroll
+        for (int k = 0; k < CG / 16; k++) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) ps[k][q] = lane + 32 * q < a.slabs ? pj[(long)(warp + 16 * k) * a.slabs + lane + 32 * q] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < CG / 16; k++)
+          v[k] = fma(s1, (ps[k][0] + ps[k][1]) + (ps[k][2] + ps[k][3]), fma(ov[0], x[k][0], ov[1] * x[k][1]) + fma(ov[2], x[k][2], ov[3] * x[k][3]));
+      }
+      // sums over the lanes of all eight rows at once: at every exchange a lane keeps half of the rows it still holds
+#pragma unroll
+      for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; k++) { const double give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k]; v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o); }
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2); v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      if ((lane & 3) == 0) vs[warp + 16 * (lane >> 2)] = v[0];    // lane bits 4, 3, 2 select row 4, 2, 1
+    }
+    __syncthreads();
+    // Warp 0 walks 32 updates at a time, a row per lane.  With S the product of the clip factors so far and a_r = <g, u_r> / S,
+    // adding u_k (whose weight relative to S is c_k = 1 / S) is a_r += c_k G[r][k], off the dependent chain, which is the norm, its
+    // reciprocal root (the hardware's approximation and one step of third order) and nothing else.  S is folded into a (and the
+    // weights) every eight updates.  The other warps bring the rows after the next 32 up to date meanwhile.
+    double n2 = j >= 1 ? st[2 * (j - 1) + 1] : 0.0, f = 1.0, Sm = 1.0, c = 1.0, npp = 1.0;
+#pragma unroll 1                                                 // (run once per launch: straight-line code would come from a cold instruction cache)
+    for (int b = 0; b < 4; b++) {
+      if (warp == 0) {
+        const int row = 32 * b + lane; const double* gr = Gd + row * CG_GD;
+        double av = vs[row];
+        if (b > 0) {                                              // what the 32 updates just walked add to this lane's row
+          const double* cb = cs[(b - 1) & 1]; double v1 = 0.0, v2 = 0.0;
+          av *= cb[32];
+#pragma unroll 8
+          for (int q = 0; q < 32; q += 2) { v1 = fma(cb[q], gr[32 * (b - 1) + q], v1); v2 = fma(cb[q + 1], gr[32 * (b - 1) + q + 1], v2); }
+          av += v1 + v2;
+        }
+        // at the head of a step f is the last update's factor and Sm the product before it; a and c are relative to that product
+        double ck = 0.0, R = 1.0, fk = 1.0, X = 2.0 * Sm * __shfl_sync(0xffffffffu, av, 0), gc = gr[32 * b], dg = Gd[(32 * b) * CG_GD + 32 * b];
+        const double* gd = Gd + (32 * b) * CG_GD + 32 * b;        // the diagonal
+#pragma unroll 1
+        for (int r8 = 0; r8 < 32; r8 += 8) {
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int r = r8 + i, rn = min(r + 1, 31);
+            const double np = fma(f, X, n2 + dg);
+            double f0; asm volatile("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(f0) : "d"(np));
+            c = c * (npp * f); Sm *= f;                           // this update's weight, and the product before its own factor
+            av = fma(c, gc, av);
+            const double an = __shfl_sync(0xffffffffu, av, (r + 1) & 31);
+            const double h = fma(-np * f0, f0, 1.0), fc = fma(f0 * h, fma(h, 0.375, 0.5), f0);
+            const bool clip = np > 1.0;                           // clip to norm 1 (lstm.go:738-750)
+            gc = gr[32 * b + rn]; dg = gd[rn * (CG_GD + 1)];
+            if (lane == r) ck = c;
+            f = clip ? fc : 1.0; n2 = clip ? 1.0 : np; npp = clip ? np : 1.0;
+            X = 2.0 * Sm * an;
+            if (lane == r) fk = f;
+          }
+          av *= Sm; ck *= Sm; R *= Sm; c = 1.0; Sm = 1.0;
+        }
+        fs[32 * b + lane] = fk;
+        cs[b & 1][lane] = ck; if (lane == 0) cs[b & 1][32] = R;
+      }
+      __syncthreads();
+      if (b < 2 && warp > 0) {
+        const int row = 32 * (b + 2) + tid - 32;
+        if (row < CG) {
+          const double* gr = Gd + row * CG_GD + 32 * b; const double* cb = cs[b & 1]; double v1 = 0.0, v2 = 0.0;
+#pragma unroll 8
+          for (int q = 0; q < 32; q += 2) { v1 = fma(cb[q], gr[q], v1); v2 = fma(cb[q + 1], gr[q + 1], v2); }
+          vs[row] = fma(cb[32], vs[row], v1 + v2);
+        }
+      }
+    }
+    if (warp != 0) return;
+    // suffix products of the factors, 32 rows at a time
+    double p[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[i] = fs[32 * i + lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) { const double y = __shfl_down_sync(0xffffffffu, p[i], o); if (lane + o < 32) p[i] *= y; }
+    }
+    double tail = 1.0;
+#pragma unroll
+    for (int i = 3; i >= 0; i--) { p[i] *= tail; om[(long)j * CG + lane + 32 * i] = p[i]; tail = __shfl_sync(0xffffffffu, p[i], 0); }
+    if (lane == 0) { st[2 * j] = tail; st[2 * j + 1] = n2; }
+    return;
+  }
+  // eight rows of the gradient matrix
+  const int slab = blockIdx.x - 1, i0 = slab * 8, nr = min(8, R4 - i0), tile = clip_tile(ZW), wp = tile | 1;
+  float* zp = sm; float* zn = zp + CG * wp; float* od = zn + CG * wp; float* gt = od + CG * 8;      // Z of group j-1, of group j+1 [CG][wp]; om d [CG][8]; the new rows [tile][8]
+  __shared__ double red[4][CG];
+  const float* D = a.D + chunk * a.stride * R4; const float* Z = a.Z + chunk * a.stride * zs;
+  const float* go = a.g + ((long)chunk * 2 + ((j - 1) & 1)) * R4 * ZW; float* gw = a.g + ((long)chunk * 2 + (j & 1)) * R4 * ZW;
+  const bool old = j >= 1, next = j + 1 < a.groups;
+  auto stage = [&](float* dst, int group, int c0, int w) {         // rows of a group, columns c0 .. c0 + w - 1, all copies in flight at once
+    const float* src = Z + ((long)CG_PAD + (long)group * CG) * zs + c0;
+    for (int r = warp; r < CG; r += CG_THREADS / 32) for (int c = lane; c < w; c += 32) cp_async4(dst + r * wp + c, src + (long)r * zs + c);
+  };
+  if (old) stage(zp, j - 1, 0, min(tile, ZW));
+  if (next) stage(zn, j + 1, 0, min(tile, ZW));
+  pdl_wait(); pdl_launch();                                        // what follows reads the launch before
+  const double s1 = j >= 1 ? st[2 * (j - 1)] : 0.0;              // s_{j-1}
+  if (old) for (int e = tid; e < CG * 8; e += CG_THREADS) {
+    const int r = e >> 3, i = e & 7;
+    od[e] = i < nr ? (float)(om[(long)(j - 1) * CG + r] * (double)D[((long)CG_PAD + (long)(j - 1) * CG + r) * R4 + i0 + i]) : 0.f;
+  }
+  float t[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) t[i] = 0.f;
+  const int pr = tid & (CG - 1), pq = tid >> 7;                    // second half of the work: row r of group j+1, a quarter of the columns
+  for (int c0 = 0; c0 < ZW; c0 += tile) {
+    const int w = min(tile, ZW - c0);
+    float gv[4] = {0.f, 0.f, 0.f, 0.f};                            // the old rows' values
+    if (old && tid < 2 * w) {
+      const int rg = tid >= w ? 4 : 0, c = tid - (rg ? w : 0);
+#pragma unroll
+      for (int i = 0; i < 4; i++) if (rg + i < nr) gv[i] = go[(long)(i0 + rg + i) * ZW + c0 + c];
+    }
+    if (c0 > 0) __syncthreads();
+    if (c0 > 0 && old) stage(zp, j - 1, c0, w);                   // (the first tile is under way)
+    if (c0 > 0 && next) stage(zn, j + 1, c0, w);
+    cp_async_wait();
+    __syncthreads();
+    if (tid < 2 * w) {                                             // four rows of a column (2 CG_TILE <= CG_THREADS)
+      const int rg = tid >= w ? 4 : 0, c = tid - (rg ? w : 0);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      if (old) {
+        const float* zc = zp + c; const float* oc = od + rg;
+#pragma unroll 16
+        for (int r = 0; r < CG; r++) {
+          const float z = zc[r * wp]; const float4 q = *reinterpret_cast<const float4*>(oc + 8 * r);
+          acc[0] = fmaf(q.x, z, acc[0]); acc[1] = fmaf(q.y, z, acc[1]); acc[2] = fmaf(q.z, z, acc[2]); acc[3] = fmaf(q.w, z, acc[3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) if (rg + i < nr) {
+        if (old) acc[i] = (float)fma(s1, (double)gv[i], (double)acc[i]);
+        gw[(long)(i0 + rg + i) * ZW + c0 + c] = acc[i];
+      }
+      *reinterpret_cast<float4*>(gt + 8 * c + rg) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+    __syncthreads();
+    if (next && old) {
+      const int per = (w + 3) >> 2, ce = min(w, (pq + 1) * per);
+#pragma unroll 4
+      for (int c = pq * per; c < ce; c++) {
+        const float z = zn[pr * wp + c]; const float4 q0 = *reinterpret_cast<const float4*>(gt + 8 * c), q1 = *reinterpret_cast<const float4*>(gt + 8 * c + 4);
+        t[0] = fmaf(q0.x, z, t[0]); t[1] = fmaf(q0.y, z, t[1]); t[2] = fmaf(q0.z, z, t[2]); t[3] = fmaf(q0.w, z, t[3]);
+        t[4] = fmaf(q1.x, z, t[4]); t[5] = fmaf(q1.y, z, t[5]); t[6] = fmaf(q1.z, z, t[6]); t[7] = fmaf(q1.w, z, t[7]);
+      }
+    }
+  }
+  if (!next) return;
+  double acc = 0.0;
+  if (old) {
+    const float* d = D + ((long)CG_PAD + (long)(j + 1) * CG + pr) * R4 + i0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) if (i < nr) acc = fma((double)d[i], (double)t[i], acc);
+  }
+  red[pq][pr] = acc;
+  __syncthreads();
+  if (tid < CG) pp[((long)((j + 1) & 1) * CG + tid) * a.slabs + slab] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
+}
+// chunk results [nchunks][2][4H][in+H+1], buffer `par` -> flat layout gWx[4H,in] | gWh[4H,H] | gb[4H], chunks added in worker order
+__global__ void lstm_scatter_grad_kernel(const float* __restrict__ Gc, int par, int nchunks, int in, int H, float* __restrict__ out) {
+  const int R4 = 4 * H, ZW = in + H + 1; const long total = (long)R4 * ZW;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const int r = (int)(i / ZW), c = (int)(i % ZW);
+    float v = 0.f; for (int q = 0; q < nchunks; q++) v += Gc[(2L * q + par) * total + i];
+    if (c < in) out[(long)r * in + c] = v; else if (c < in + H) out[(long)R4 * in + (long)r * H + (c - in)] = v; else out[(long)R4 * in + (long)R4 * H + r] = v;
+  }
+}
+
+}  // namespace gn

@@ -7,6 +7,7 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include "common.cuh"
+#include "fmath.cuh"
 
 namespace gn {
 
@@ -21,27 +22,27 @@ __host__ __device__ inline float act_alpha_of(int act, int bits) {
 __device__ __forceinline__ float act_fwd(int act, float x, float alpha = 0.f) {
   switch (act) {
     case GN_ACT_RELU: return x > 0.f ? x : 0.f;
-    case GN_ACT_SIGMOID: return 1.f / (1.f + (float)exp((double)-x));
-    case GN_ACT_TANH: return (float)tanh((double)x);
+    case GN_ACT_SIGMOID: return 1.f / (1.f + exp_rn(-x));
+    case GN_ACT_TANH: return tanh_rn(x);
     case GN_ACT_LEAKY_RELU: return x > 0.f ? x : alpha * x;
-    case GN_ACT_ELU: return x > 0.f ? x : alpha * ((float)exp((double)x) - 1.f);
-    case GN_ACT_GELU: { float x3 = x * x * x; float arg = 0.7978845608028654f * (x + 0.044715f * x3); return 0.5f * x * (1.f + (float)tanh((double)arg)); }
-    case GN_ACT_SILU: { if (x >= 0.f) return x * (1.f / (1.f + (float)exp((double)-x))); float e = (float)exp((double)x); return x * e / (1.f + e); }
+    case GN_ACT_ELU: return x > 0.f ? x : alpha * (exp_rn(x) - 1.f);
+    case GN_ACT_GELU: { float x3 = x * x * x; float arg = 0.7978845608028654f * (x + 0.044715f * x3); return 0.5f * x * (1.f + tanh_rn(arg)); }
+    case GN_ACT_SILU: { if (x >= 0.f) return x * (1.f / (1.f + exp_rn(-x))); float e = exp_rn(x); return x * e / (1.f + e); }
     default: return x;
   }
 }
 __device__ __forceinline__ float act_der(int act, float x, float alpha = 0.f) {
   switch (act) {
     case GN_ACT_RELU: return x > 0.f ? 1.f : 0.f;
-    case GN_ACT_SIGMOID: { float s = 1.f / (1.f + (float)exp((double)-x)); return s * (1.f - s); }
-    case GN_ACT_TANH: { float t = (float)tanh((double)x); return 1.f - t * t; }
+    case GN_ACT_SIGMOID: { float s = 1.f / (1.f + exp_rn(-x)); return s * (1.f - s); }
+    case GN_ACT_TANH: { float t = tanh_rn(x); return 1.f - t * t; }
     case GN_ACT_LEAKY_RELU: return x > 0.f ? 1.f : alpha;
-    case GN_ACT_ELU: return x > 0.f ? 1.f : alpha * (float)exp((double)x);
+    case GN_ACT_ELU: return x > 0.f ? 1.f : alpha * exp_rn(x);
     case GN_ACT_GELU: {
       const double c = 0.044715, k = 0.7978845608028654, xd = (double)x, x2 = xd * xd, t = tanh(k * (xd + c * xd * x2));
       return (float)(0.5 * (1.0 + t) + 0.5 * xd * (1.0 - t * t) * k * (1.0 + 3.0 * c * x2));
     }
-    case GN_ACT_SILU: { float sg; if (x >= 0.f) sg = 1.f / (1.f + (float)exp((double)-x)); else { float e = (float)exp((double)x); sg = e / (1.f + e); } return sg + x * sg * (1.f - sg); }
+    case GN_ACT_SILU: { const float e = exp_rn(x >= 0.f ? -x : x), sg = (x >= 0.f ? 1.f : e) / (1.f + e); return sg + x * sg * (1.f - sg); }
     default: return 1.f;
   }
 }

@@ -258,7 +258,7 @@ int gn_op_softmax_ce(gn_ctx* ctx, int B, int V, int log_softmax, const float* z,
  * wh [4H, H], bias [4H] (gate order i, f, g, o); h_all, c_all [B, T, H] receive every step's hidden and cell state
  * (lstm.go:276-407: only the input-gate rows receive wx x + wh h).  With dh_last != NULL ([B, H], gradient of the last
  * hidden state) also the gate deltas of back-propagation through time, dgate [B, T, 4H] (lstm.go:476-691).
- * engine: 0 = input projection inside the recurrence kernel, 1 = as one tensor-core contraction over all B*T rows. */
+ * engine: 0 = input projection of all B*T rows as one CUDA-core contraction, 1 = as one tensor-core contraction. */
 int gn_op_lstm(gn_ctx* ctx, int engine, int B, int T, int in_size, int H, const float* x, const float* wx, const float* wh, const float* bias,
                const float* dh_last, float* h_all, float* c_all, float* dgate);
 
