@@ -79,7 +79,7 @@ __global__ void conv2d_wgrad_kernel(const float* __restrict__ g, const float* __
 
 // Weight gradient, tiled: one block per (oc, ic) pair and batch slice, so the K*K taps of the pair share every load of
 // g and the input plane is read from L1; partial sums go to part[slice][nW + outC] (bias partials from the ic == 0
-// blocks) and conv2d_wgrad_final_kernel adds the slices in order.  Same sums as conv2d_wgrad_kernel.
+// blocks) and conv_wgrad_final_kernel adds the slices in order.  Same sums as conv2d_wgrad_kernel.
 template <int K>
 __global__ void __launch_bounds__(256) conv2d_wgrad_tile_kernel(const float* __restrict__ g, const float* __restrict__ x, float* __restrict__ part, ConvShape c, int slices) {
   __shared__ float red[8][K * K + 1];
@@ -118,36 +118,6 @@ __global__ void __launch_bounds__(256) conv2d_wgrad_tile_kernel(const float* __r
     else if (ic == 0) prow[nW + oc] = v;
   }
 }
-__global__ void conv2d_wgrad_final_kernel(const float* __restrict__ part, int slices, int n, float* __restrict__ dW) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x; if (i >= n) return;
-  float s = 0.f;
-  for (int k = 0; k < slices; k++) s += part[(long)k * n + i];
-  dW[i] = s;                                              // weights, then biases: the gradient slice is laid out W | b
-}
-// Input gradient for stride 1 (no division in the tap loops); same sum as conv2d_dgrad_kernel.
-template <int K>
-__global__ void __launch_bounds__(256) conv2d_dgrad_s1_kernel(const float* __restrict__ g, const float* __restrict__ Wt, float* __restrict__ dx, ConvShape c) {
-  const long total = (long)c.B * c.inC * c.H * c.W;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int iw = (int)(i % c.W); long r = i / c.W; const int ih = (int)(r % c.H); r /= c.H; const int ic = (int)(r % c.inC), b = (int)(r / c.inC);
-    const float* gb = g + (long)b * c.outC * c.oH * c.oW;
-    float acc = 0.f;
-    for (int oc = 0; oc < c.outC; oc++) {
-      const float* gp = gb + (long)oc * c.oH * c.oW; const float* wp = Wt + ((long)oc * c.inC + ic) * K * K;
-#pragma unroll
-      for (int kh = 0; kh < K; kh++) {
-        const int oh = ih + c.p - kh; if (oh < 0 || oh >= c.oH) continue;
-#pragma unroll
-        for (int kw = 0; kw < K; kw++) {
-          const int ow = iw + c.p - kw; if (ow < 0 || ow >= c.oW) continue;
-          acc = fmaf(gp[oh * c.oW + ow], __ldg(wp + kh * K + kw), acc);
-        }
-      }
-    }
-    dx[i] = acc;
-  }
-}
-
 // ---------------------------------------------------------------- Conv1D
 // Input [B, inC, L], output [B, outC, oL], weights [outC, inC, k].  reference: conv1d.go:178-216 (the sum starts from the
 // bias), :254-288 (the backward pass uses the incoming gradient as it is: no activation derivative).
@@ -202,19 +172,38 @@ __global__ void conv1d_wgrad_kernel(const float* __restrict__ g, const float* __
 }
 
 struct PoolShape { int B, C, k, s, p, H, W, oH, oW; };
-// reference: maxpool2d.go:192-221 (init -inf, strict '>', first maximum wins, argmax = flat CHW index)
-__global__ void maxpool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int* __restrict__ arg, PoolShape c) {
-  long total = (long)c.B * c.C * c.oH * c.oW;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    int ow = (int)(i % c.oW); long r = i / c.oW; int oh = (int)(r % c.oH); r /= c.oH; int ch = (int)(r % c.C); int b = (int)(r / c.C);
-    const float* xb = x + (long)b * c.C * c.H * c.W;
-    float mv = -INFINITY; int mi = -1;
-    for (int kh = 0; kh < c.k; kh++) for (int kw = 0; kw < c.k; kw++) {
-      int ih = oh * c.s + kh - c.p, iw = ow * c.s + kw - c.p;
-      if (ih >= 0 && ih < c.H && iw >= 0 && iw < c.W) { int idx = (ch * c.H + ih) * c.W + iw; float v = xb[idx]; if (v > mv) { mv = v; mi = idx; } }
-    }
-    y[i] = mv; arg[i] = mi;
+// reference: maxpool2d.go:192-221 (init -inf, strict '>', first maximum wins, argmax = flat CHW index).  A block takes a piece of one
+// (sample, channel) plane: the index arithmetic is 32-bit and per pixel of the plane.
+__global__ void __launch_bounds__(256) maxpool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int* __restrict__ arg, PoolShape c) {
+  const long pl = blockIdx.x; const int ch = (int)(pl % c.C), i = blockIdx.y * 256 + threadIdx.x; if (i >= c.oH * c.oW) return;
+  const int oh = i / c.oW, ow = i - oh * c.oW, h0 = oh * c.s - c.p, w0 = ow * c.s - c.p;
+  const float* xp = x + pl * c.H * c.W;
+  float mv = -INFINITY; int mi = -1;
+  if (c.k == 2 && c.p == 0) {                              // whole windows: both rows in flight
+    const float* q = xp + h0 * c.W + w0; const float a = q[0], b = q[1], d = q[c.W], e = q[c.W + 1]; const int at = (ch * c.H + h0) * c.W + w0;
+    if (a > mv) { mv = a; mi = at; } if (b > mv) { mv = b; mi = at + 1; } if (d > mv) { mv = d; mi = at + c.W; } if (e > mv) { mv = e; mi = at + c.W + 1; }
+  } else for (int kh = 0; kh < c.k; kh++) for (int kw = 0; kw < c.k; kw++) {
+    const int ih = h0 + kh, iw = w0 + kw;
+    if (ih >= 0 && ih < c.H && iw >= 0 && iw < c.W) { const float v = xp[ih * c.W + iw]; if (v > mv) { mv = v; mi = (ch * c.H + ih) * c.W + iw; } }
   }
+  y[pl * c.oH * c.oW + i] = mv; arg[pl * c.oH * c.oW + i] = mi;
+}
+// Windows that do not overlap: every input element looks its one window up (no zero fill, no atomics).  `relu`: the derivative of a
+// ReLU right below is applied as well -- the element that won its window passes the gradient on only if it is positive (y > 0).
+__global__ void __launch_bounds__(256) maxpool_bwd_gather_kernel(const float* __restrict__ g, const int* __restrict__ arg, const float* __restrict__ y, float* __restrict__ dx, PoolShape c, int relu) {
+  const long pl = blockIdx.x; const int ch = (int)(pl % c.C), i = blockIdx.y * 256 + threadIdx.x; if (i >= c.H * c.W) return;
+  const int ih = i / c.W, iw = i - ih * c.W, oh = (ih + c.p) / c.s, ow = (iw + c.p) / c.s; float v = 0.f;
+  if (oh < c.oH && ow < c.oW) { const long o = pl * c.oH * c.oW + oh * c.oW + ow; if (arg[o] == ch * c.H * c.W + i && (!relu || y[o] > 0.f)) v = g[o]; }
+  dx[pl * c.H * c.W + i] = v;
+}
+// 2 x 2 windows that tile the plane (W even, 8-byte aligned rows): a thread per window
+__global__ void __launch_bounds__(256) maxpool_bwd_2x2_kernel(const float* __restrict__ g, const int* __restrict__ arg, const float* __restrict__ y, float* __restrict__ dx, PoolShape c, int relu) {
+  const long pl = blockIdx.x; const int i = blockIdx.y * 256 + threadIdx.x; if (i >= c.oH * c.oW) return;
+  const int oh = i / c.oW, ow = i - oh * c.oW; const long o = pl * c.oH * c.oW + i;
+  const float v = relu && !(y[o] > 0.f) ? 0.f : g[o]; const int at = ((int)(pl % c.C) * c.H + 2 * oh) * c.W + 2 * ow, d = arg[o] - at;
+  float* q = dx + (pl * c.H + 2 * oh) * c.W + 2 * ow;
+  *reinterpret_cast<float2*>(q) = make_float2(d == 0 ? v : 0.f, d == 1 ? v : 0.f);
+  *reinterpret_cast<float2*>(q + c.W) = make_float2(d == c.W ? v : 0.f, d == c.W + 1 ? v : 0.f);
 }
 // dx zero-filled beforehand; windows may overlap when stride < kernel, hence the atomic add (maxpool2d.go:395-406)
 __global__ void maxpool_bwd_kernel(const float* __restrict__ g, const int* __restrict__ arg, float* __restrict__ dx, PoolShape c) {

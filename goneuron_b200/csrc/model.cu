@@ -27,6 +27,7 @@
 #include "recurrent.cuh"
 #include "attention.cuh"
 #include "attention_tc.cuh"
+#include "conv_direct.cuh"
 #include "conv_tc.cuh"
 #include "nccl_dl.cuh"
 
@@ -430,45 +431,58 @@ static bool use_fused_attention(const gn_layer_desc& d) {
   return !unfused && attn_fused_supported(d.dim / d.heads, d.dim);
 }
 
-// ---------------------------------------------------------------- Conv2D (both paths)
-// z / out: [B, outC, oH, oW].  Implicit GEMM on the tensor cores when `allow_tc` and the engine takes the shape (bias
-// and ReLU in the epilogue, other activations from the kept pre-activation z); else the direct kernel (writes z and out).
-static int conv_forward(Ctx* ctx, const ConvShape& c, int act, float alpha, const float* x, const float* p, float* z, float* out, bool allow_tc) {
+// ---------------------------------------------------------------- Conv2D
+// Register-tiled CUDA-core kernels (conv_direct.cuh) or implicit GEMM on the tensor cores (conv_tc.cuh); what neither takes (a stride
+// above one on the CUDA cores, other windows) runs on the plain direct kernels of conv_lstm.cuh.
+enum ConvEngine { CONV_AUTO, CONV_CUDA, CONV_TC };
+static ConvEngine conv_engine(Ctx* ctx, const ConvShape& c, ConvEngine want) {
+  if (want == CONV_AUTO) want = conv_direct_preferred(c) ? CONV_CUDA : CONV_TC;
+  return want == CONV_TC && conv_tc_supported(ctx, c) ? CONV_TC : CONV_CUDA;
+}
+// z / out: [B, outC, oH, oW].  Bias and the activation are applied by the kernel that makes the sums (on the tensor cores LINEAR and
+// RELU; the others from the kept pre-activation z, which only they need).
+static int conv_forward(Ctx* ctx, const ConvShape& c, int act, float alpha, const float* x, const float* p, float* z, float* out, ConvEngine want) {
   const long n = (long)c.B * c.outC * c.oH * c.oW; const float* bias = p + (long)c.outC * c.inC * c.k * c.k;
-  if (allow_tc && conv_tc_supported(ctx, c)) {
-    const bool in_epilogue = act == GN_ACT_LINEAR || act == GN_ACT_RELU;
-    GN_TRY(conv_tc_forward(ctx, c, x, p, bias, in_epilogue ? out : z, in_epilogue ? act : GN_ACT_LINEAR));
-    if (!in_epilogue) GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, n), 256, 0, z, out, n, act, alpha);
-  } else GN_LAUNCH(ctx, conv2d_fwd_kernel, ew_grid(ctx, n), 256, 0, x, p, bias, z, out, c, act, alpha);
+  const bool simple = act == GN_ACT_LINEAR || act == GN_ACT_RELU;
+  if (conv_engine(ctx, c, want) == CONV_TC) {
+    GN_TRY(conv_tc_forward(ctx, c, x, p, bias, simple ? out : z, simple ? act : GN_ACT_LINEAR));
+    if (!simple) GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, n), 256, 0, z, out, n, act, alpha);
+  } else if (conv_direct_supported(c)) return conv_direct_forward(ctx, c, x, p, bias, simple ? nullptr : z, out, act, alpha);
+  else GN_LAUNCH(ctx, conv2d_fwd_kernel, ew_grid(ctx, n), 256, 0, x, p, bias, z, out, c, act, alpha);
   return check_launch("conv_forward");
 }
-// g: gradient with respect to the activation; gW / gb are added to; dx (may be null) is written.
+// g: gradient with respect to the activation; gW / gb and dx (may be null) are written.
 static int conv_backward(gn_model* m, const ConvShape& c, int act, float alpha, const float* g, const float* x, const float* p, const float* z, const float* out,
-                         float* gW, float* gb, float* dx, bool allow_tc) {
+                         float* gW, float* gb, float* dx, ConvEngine want) {
   Ctx* ctx = &m->ctx->c;
-  const long n = (long)c.B * c.outC * c.oH * c.oW; float* dzb; GN_TRY(ensure(m, S_DZ, (size_t)n, &dzb));
-  // ReLU'(z) = [z > 0] = [a > 0], so ReLU (and the identity) work from the activation; the others need the pre-activation
-  const float* zsrc = (act == GN_ACT_RELU || act == GN_ACT_LINEAR) ? out : z;
-  GN_LAUNCH(ctx, act_backward_kernel, ew_grid(ctx, n), 256, 0, g, zsrc, dzb, n, act, alpha);
-  const int nW = c.outC * c.inC * c.k * c.k;
-  const bool conv_tc = allow_tc && conv_tc_supported(ctx, c);
-  if (conv_tc) {
+  const long n = (long)c.B * c.outC * c.oH * c.oW; const int nW = c.outC * c.inC * c.k * c.k;
+  const ConvEngine eng = conv_engine(ctx, c, want); const bool direct = eng == CONV_CUDA && conv_direct_supported(c);
+  // ReLU'(z) = [z > 0] = [a > 0], so ReLU works from the activation (the caller passes LINEAR if g already carries it)
+  const float* dz = g;
+  if (act != GN_ACT_LINEAR) {
+    float* dzb; GN_TRY(ensure(m, S_DZ, (size_t)n, &dzb));
+    GN_LAUNCH(ctx, act_backward_kernel, ew_grid(ctx, n), 256, 0, g, act == GN_ACT_RELU ? out : z, dzb, n, act, alpha); dz = dzb;
+  }
+  if (direct) {
+    float* part; GN_TRY(ensure(m, S_PART, conv_wgrad_part_floats(ctx, c), &part));
+    GN_TRY(conv_direct_wgrad(ctx, c, dz, x, part, gW));
+    return dx ? conv_direct_dgrad(ctx, c, dz, p, dx) : GN_OK;
+  }
+  if (eng == CONV_TC) {
     float* part; GN_TRY(ensure(m, S_PART, (size_t)c.B * (nW + c.outC), &part));
-    GN_TRY(conv_tc_wgrad(ctx, c, dzb, x, part, gW, gb));
+    GN_TRY(conv_tc_wgrad(ctx, c, dz, x, part, gW, gb));
   } else if (c.k == 3 || c.k == 5 || c.k == 1) {
     const int pairs = c.outC * c.inC, slices = std::max(1, std::min(c.B, (4 * ctx->sm_count + pairs - 1) / pairs)), ng = nW + c.outC;
     float* part; GN_TRY(ensure(m, S_PART, (size_t)slices * ng, &part));
-    if (c.k == 3) GN_LAUNCH(ctx, conv2d_wgrad_tile_kernel<3>, dim3(pairs, slices), 256, 0, dzb, x, part, c, slices);
-    else if (c.k == 5) GN_LAUNCH(ctx, conv2d_wgrad_tile_kernel<5>, dim3(pairs, slices), 256, 0, dzb, x, part, c, slices);
-    else GN_LAUNCH(ctx, conv2d_wgrad_tile_kernel<1>, dim3(pairs, slices), 256, 0, dzb, x, part, c, slices);
-    GN_LAUNCH(ctx, conv2d_wgrad_final_kernel, cdiv(ng, 256), 256, 0, part, slices, ng, gW);          // weights, then biases: gb follows gW
-  } else GN_LAUNCH(ctx, conv2d_wgrad_kernel, nW + c.outC, 256, 0, dzb, x, gW, gb, c);
+    if (c.k == 3) GN_LAUNCH(ctx, conv2d_wgrad_tile_kernel<3>, dim3(pairs, slices), 256, 0, dz, x, part, c, slices);
+    else if (c.k == 5) GN_LAUNCH(ctx, conv2d_wgrad_tile_kernel<5>, dim3(pairs, slices), 256, 0, dz, x, part, c, slices);
+    else GN_LAUNCH(ctx, conv2d_wgrad_tile_kernel<1>, dim3(pairs, slices), 256, 0, dz, x, part, c, slices);
+    GN_LAUNCH(ctx, conv_wgrad_final_kernel, cdiv(ng, 32), 256, 0, (const float*)part, slices, ng, gW);          // weights, then biases: gb follows gW
+  } else GN_LAUNCH(ctx, conv2d_wgrad_kernel, nW + c.outC, 256, 0, dz, x, gW, gb, c);
   if (dx) {
     const long ni = (long)c.B * c.inC * c.H * c.W;
-    if (conv_tc && c.s == 1) { float* wtmp; GN_TRY(ensure(m, S_DELTA, (size_t)nW, &wtmp)); GN_TRY(conv_tc_dgrad(ctx, c, dzb, p, wtmp, dx)); }
-    else if (c.s == 1 && c.k == 3) GN_LAUNCH(ctx, conv2d_dgrad_s1_kernel<3>, ew_grid(ctx, ni), 256, 0, dzb, p, dx, c);
-    else if (c.s == 1 && c.k == 5) GN_LAUNCH(ctx, conv2d_dgrad_s1_kernel<5>, ew_grid(ctx, ni), 256, 0, dzb, p, dx, c);
-    else GN_LAUNCH(ctx, conv2d_dgrad_kernel, ew_grid(ctx, ni), 256, 0, dzb, p, dx, c);
+    if (eng == CONV_TC && c.s == 1) { float* wtmp; GN_TRY(ensure(m, S_DELTA, (size_t)nW, &wtmp)); GN_TRY(conv_tc_dgrad(ctx, c, dz, p, wtmp, dx)); }
+    else GN_LAUNCH(ctx, conv2d_dgrad_kernel, ew_grid(ctx, ni), 256, 0, dz, p, dx, c);
   }
   return check_launch("conv_backward");
 }
@@ -665,13 +679,12 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
       case GN_LAYER_CONV2D: {
         ConvShape c{B, d.in_size, d.out_size, d.kernel, d.stride, d.padding, d.in_h, d.in_w,
                     (d.in_h + 2 * d.padding - d.kernel) / d.stride + 1, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
-        GN_TRY(conv_forward(ctx, c, d.activation, act_alpha_of(d.activation, d.reserved), cur, p, l.z.p, l.out.p, !force_simt_engine()));
+        GN_TRY(conv_forward(ctx, c, d.activation, act_alpha_of(d.activation, d.reserved), cur, p, l.z.p, l.out.p, force_simt_engine() ? CONV_CUDA : CONV_AUTO));
         cur = l.out.p; break; }
       case GN_LAYER_MAXPOOL2D: {
         PoolShape c{B, d.in_size, d.kernel, d.stride, d.padding, d.in_h, d.in_w,
                     (d.in_h + 2 * d.padding - d.kernel) / d.stride + 1, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
-        long n = (long)B * l.out_size;
-        GN_LAUNCH(ctx, maxpool_fwd_kernel, ew_grid(ctx, n), 256, 0, cur, l.out.p, (int*)l.idx.p, c);
+        GN_LAUNCH(ctx, maxpool_fwd_kernel, dim3(B * c.C, cdiv((long)c.oH * c.oW, 256)), 256, 0, cur, l.out.p, (int*)l.idx.p, c);
         cur = l.out.p; break; }
       case GN_LAYER_CONV1D: {
         Conv1Shape c{B, d.in_size, d.out_size, d.kernel, d.stride, d.padding, d.in_w, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
@@ -741,8 +754,8 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
             float* g; GN_TRY(ensure(m, S_BNG, (size_t)2 * GB * C, &g));
             GN_TRY(all_gather_on_comm(m, l.stat.p, g, (size_t)BC, "BatchNorm2D means"));
             GN_TRY(all_gather_on_comm(m, l.stat.p + 2 * BC, g + (size_t)GB * C, (size_t)BC, "BatchNorm2D variances"));
-            GN_LAUNCH(ctx, bn_running_gathered_kernel, cdiv(C, 128), 128, 0, (const float*)g, (const float*)(g + (size_t)GB * C), run, GB, C, l.bn_mom);
-          } else GN_LAUNCH(ctx, bn_running_kernel, cdiv(C, 128), 128, 0, l.stat.p, run, B, C, BC, l.bn_mom);
+            GN_LAUNCH(ctx, bn_running_kernel, cdiv(C, 32), 256, 0, (const float*)g, (const float*)(g + (size_t)GB * C), run, GB, C, l.bn_mom);
+          } else GN_LAUNCH(ctx, bn_running_kernel, cdiv(C, 32), 256, 0, (const float*)l.stat.p, (const float*)(l.stat.p + 2 * BC), run, B, C, l.bn_mom);
         } else {
           long n = BC * S; GN_LAUNCH(ctx, bn_eval_kernel, ew_grid(ctx, n), 256, 0, cur, p, p + C, run, l.out.p, C, S, n, l.bn_eps);
         }
@@ -1081,6 +1094,7 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
   static const bool comm_at_end = [] { const char* e = getenv("GONEURON_CUDA_COMM"); return e && !strcmp(e, "end"); }();
   std::vector<int> deferred;
   bool gated = false;                                       // g already carries the derivative of the ReLU below it
+  auto relu_conv_below = [&](int li) { return li > 0 && m->L[li - 1].d.kind == GN_LAYER_CONV2D && m->L[li - 1].d.activation == GN_ACT_RELU; };
   bool row0 = false; int row0_T = 0, row0_D = 0;            // g holds the gradient of token 0 of every sequence, [B, row0_D]; the other tokens' is zero
   auto layer_comm = [&](int li) -> int {
     LayerRT& l = m->L[li]; float* gr = m->grads.p + l.p_off;
@@ -1133,12 +1147,20 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         ConvShape c{B, d.in_size, d.out_size, d.kernel, d.stride, d.padding, d.in_h, d.in_w,
                     (d.in_h + 2 * d.padding - d.kernel) / d.stride + 1, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
         const int nW = d.out_size * d.in_size * d.kernel * d.kernel;
-        GN_TRY(conv_backward(m, c, d.activation, act_alpha_of(d.activation, d.reserved), g, xin, p, l.z.p, l.out.p, gr, gr + nW, need_dx ? dx : nullptr, !force_simt_engine()));
+        GN_TRY(conv_backward(m, c, gated ? (int)GN_ACT_LINEAR : d.activation, act_alpha_of(d.activation, d.reserved), g, xin, p, l.z.p, l.out.p, gr, gr + nW, need_dx ? dx : nullptr, force_simt_engine() ? CONV_CUDA : CONV_AUTO));
+        gated = false;
         if (need_dx) { g = dx; flip ^= 1; }
         break; }
       case GN_LAYER_MAXPOOL2D: {
         PoolShape c{B, d.in_size, d.kernel, d.stride, d.padding, d.in_h, d.in_w,
                     (d.in_h + 2 * d.padding - d.kernel) / d.stride + 1, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
+        if (c.k <= c.s) {
+          gated = relu_conv_below(li);
+          if (c.k == 2 && c.s == 2 && c.p == 0 && c.H == 2 * c.oH && c.W == 2 * c.oW)
+            GN_LAUNCH(ctx, maxpool_bwd_2x2_kernel, dim3(B * c.C, cdiv((long)c.oH * c.oW, 256)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
+          else GN_LAUNCH(ctx, maxpool_bwd_gather_kernel, dim3(B * c.C, cdiv((long)c.H * c.W, 256)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
+          g = dx; flip ^= 1; break;
+        }
         GN_CUDA(cudaMemsetAsync(dx, 0, (size_t)B * l.in_size * sizeof(float), ctx->stream));
         long n = (long)B * l.out_size;
         GN_LAUNCH(ctx, maxpool_bwd_kernel, ew_grid(ctx, n), 256, 0, g, (const int*)l.idx.p, dx, c);
@@ -1225,7 +1247,8 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
       case GN_LAYER_BATCHNORM2D: {
         const int C = d.in_size, S = d.in_h * d.in_w; const long BC = (long)B * C;
         float* pg; GN_TRY(ensure(m, S_DELTA, (size_t)B * 2 * C, &pg));
-        GN_LAUNCH(ctx, bn_bwd_kernel, (unsigned)BC, 256, 0, g, xin, p, l.stat.p, dx, pg, C, S, BC);
+        gated = relu_conv_below(li);
+        GN_LAUNCH(ctx, bn_bwd_kernel, (unsigned)BC, 256, 0, g, xin, p, l.stat.p, dx, pg, C, S, BC, gated ? 1 : 0);
         GN_TRY(colsum(m, pg, 2 * C, B, 2 * C, gr, false));
         g = dx; flip ^= 1; break; }
       case GN_LAYER_LAYERNORM: {

@@ -55,13 +55,13 @@ int gn_op_conv2d(gn_ctx* ctx, int engine, int B, int in_c, int out_c, int kernel
   GN_CUDA(copy_h2d(c, P, w, nW * 4)); GN_CUDA(copy_h2d(c, P + nW, bias, (size_t)out_c * 4));
   float *dX = io.in(x, nx), *Z = io.out(ny), *A = io.out(ny);
   GN_TRY(io.rc);
-  GN_TRY(conv_forward(c, cs, activation, act_alpha_of(activation, 0), dX, P, Z, A, engine == 1));
+  GN_TRY(conv_forward(c, cs, activation, act_alpha_of(activation, 0), dX, P, Z, A, engine == 1 ? CONV_TC : CONV_CUDA));
   GN_TRY(io.back(y, A, ny));
   if (dy) {
     gn_model tmp; tmp.ctx = ctx;
     float *G = io.in(dy, ny), *gP = io.zeros(nW + out_c), *dDx = io.out(nx);
     GN_TRY(io.rc);
-    GN_TRY(conv_backward(&tmp, cs, activation, act_alpha_of(activation, 0), G, dX, P, Z, A, gP, gP + nW, dDx, engine == 1));
+    GN_TRY(conv_backward(&tmp, cs, activation, act_alpha_of(activation, 0), G, dX, P, Z, A, gP, gP + nW, dDx, engine == 1 ? CONV_TC : CONV_CUDA));
     GN_TRY(io.back(dx, dDx, nx)); GN_TRY(io.back(dw, gP, nW)); GN_TRY(io.back(db, gP + nW, out_c));
     GN_CUDA(cudaStreamSynchronize(c->stream));
   }

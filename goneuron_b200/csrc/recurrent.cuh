@@ -352,8 +352,6 @@ struct ClipArgs {
   float* g;                      // [chunk][2][4H][ZW]
   int R4, ZW, groups, slabs; long stride;
 };
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory"); }
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __global__ void __launch_bounds__(CG_THREADS) lstm_clip_kernel(const ClipArgs a, int j) {
   extern __shared__ __align__(16) float sm[];
   const int chunk = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R4 = a.R4, ZW = a.ZW, zs = clip_zs(ZW);

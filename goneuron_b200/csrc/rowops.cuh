@@ -815,22 +815,25 @@ __global__ void bn_fwd_kernel(const float* __restrict__ x, const float* __restri
   for (int i = threadIdx.x; i < S; i += blockDim.x) yp[i] = g * ((xp[i] - mean) * istd) + b;
   if (threadIdx.x == 0) { stat[bc] = mean; stat[BC + bc] = sd; stat[2 * BC + bc] = var; }
 }
-// running = (1 - momentum) * running + momentum * statistic, once per sample in batch order (batchnorm2d.go:352, :376)
-__global__ void bn_running_kernel(const float* __restrict__ stat, float* __restrict__ run, int B, int C, long BC, float mom) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x; if (c >= C) return;
-  float rm = run[c], rv = run[C + c];
-#pragma unroll 8                                            // the loads of eight samples in flight; the updates stay in order (one sample at a time: 30 us for 50)
-  for (int b = 0; b < B; b++) { rm = (1.f - mom) * rm + mom * stat[(long)b * C + c]; rv = (1.f - mom) * rv + mom * stat[2 * BC + (long)b * C + c]; }
-  run[c] = rm; run[C + c] = rv;
-}
-// The same walk over per-sample statistics gathered from every rank (mean and variance as separate [B, C] arrays in
-// global sample order), so that every replica applies the updates of the whole global batch in the reference's order.
-__global__ void bn_running_gathered_kernel(const float* __restrict__ mean, const float* __restrict__ var, float* __restrict__ run, int B, int C, float mom) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x; if (c >= C) return;
-  float rm = run[c], rv = run[C + c];
-#pragma unroll 8                                            // the loads of eight samples in flight; the updates stay in order (one sample at a time: 30 us for 50)
-  for (int b = 0; b < B; b++) { rm = (1.f - mom) * rm + mom * mean[(long)b * C + c]; rv = (1.f - mom) * rv + mom * var[(long)b * C + c]; }
-  run[c] = rm; run[C + c] = rv;
+// running = (1 - momentum) * running + momentum * statistic, once per sample in batch order (batchnorm2d.go:352, :376); `mean`, `var`:
+// [B, C] per-sample statistics of the whole global batch (with several ranks every replica walks all of them).  A block stages 128
+// samples of 32 channels at a time; one warp then walks the means, one the variances (from global memory: 30 us for 50 samples).
+__global__ void __launch_bounds__(256) bn_running_kernel(const float* __restrict__ mean, const float* __restrict__ var, float* __restrict__ run, int B, int C, float mom) {
+  __shared__ float st[2][128][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane; const bool in = c < C;
+  float r = in && w < 2 ? run[(long)w * C + c] : 0.f;
+  for (int b0 = 0; b0 < B; b0 += 128) {
+    const int n = min(128, B - b0);
+    __syncthreads();
+#pragma unroll 4
+    for (int b = w; b < n; b += 8) if (in) { st[0][b][lane] = mean[(long)(b0 + b) * C + c]; st[1][b][lane] = var[(long)(b0 + b) * C + c]; }
+    __syncthreads();
+    if (w < 2) {
+#pragma unroll 8
+      for (int b = 0; b < n; b++) r = (1.f - mom) * r + mom * st[w][b][lane];
+    }
+  }
+  if (in && w < 2) run[(long)w * C + c] = r;
 }
 // inference mode: running statistics (batchnorm2d.go:492-509)
 __global__ void bn_eval_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ run,
@@ -842,7 +845,7 @@ __global__ void bn_eval_kernel(const float* __restrict__ x, const float* __restr
 }
 // reference: batchnorm2d.go:626-660, m = S.  pg: per (sample, channel) contributions [B, 2C] = gGamma | gBeta, summed over samples afterwards.
 __global__ void bn_bwd_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ stat,
-                              float* __restrict__ dx, float* __restrict__ pg, int C, int S, long BC) {
+                              float* __restrict__ dx, float* __restrict__ pg, int C, int S, long BC, int relu) {
   __shared__ float red[33];
   const long bc = blockIdx.x; const int c = (int)(bc % C); const long b = bc / C;
   const float* xp = x + bc * S; const float* gp = g + bc * S; float* dp = dx + bc * S;
@@ -852,7 +855,8 @@ __global__ void bn_bwd_kernel(const float* __restrict__ g, const float* __restri
   sg = block_sum(sg, red); sgx = block_sum(sgx, red);
   for (int i = threadIdx.x; i < S; i += blockDim.x) {
     float d = xp[i] - mean, gi = gp[i] * gm;
-    dp[i] = gi / sd - (sg * gm) / m / sd - d * (sgx * gm) / m / (sd * sd * sd);
+    const float v = gi / sd - (sg * gm) / m / sd - d * (sgx * gm) / m / (sd * sd * sd);
+    dp[i] = relu && !(xp[i] > 0.f) ? 0.f : v;               // (the derivative of a ReLU right below: its output is this layer's input)
   }
   if (threadIdx.x == 0) { pg[b * 2 * C + c] = sgx / sd; pg[b * 2 * C + C + c] = sg; }     // sum g*(x-mean)/std ; sum g
 }

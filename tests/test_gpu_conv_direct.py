@@ -1,0 +1,87 @@
+"""The register-tiled convolution kernels (engine 0 of gn_op_conv2d) where their tiling can go wrong: widths that are no multiple of four,
+channel counts around the groups of eight, images taller than a band, several source-channel chunks, one image and many, and
+the pooling gradient's two forms -- against float64 numpy."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from goneuron_b200 import configs, descriptors as D
+from tests.parity import TOL, assert_grads_close, norm_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    from goneuron_b200.sequential import Device
+    d = Device(0)
+    yield d
+    d.close()
+
+
+def _f(a):
+    return a.ctypes.data_as(C.POINTER(C.c_float))
+
+
+@pytest.mark.parametrize("B,inC,outC,k,p,H,W,act", [
+    (1, 1, 1, 1, 0, 1, 1, D.LINEAR), (2, 3, 8, 1, 0, 5, 7, D.RELU), (3, 9, 17, 3, 1, 7, 6, D.RELU), (2, 5, 7, 3, 0, 9, 10, D.TANH), (1, 33, 40, 3, 2, 12, 13, D.RELU),
+    (200, 1, 24, 3, 1, 28, 28, D.RELU), (2, 70, 65, 3, 1, 8, 8, D.LINEAR), (3, 4, 6, 5, 2, 31, 33, D.SIGMOID), (2, 40, 9, 5, 4, 6, 5, D.RELU), (1, 2, 3, 3, 1, 300, 301, D.RELU),
+    (2, 3, 100, 3, 1, 40, 40, D.RELU), (4, 16, 4, 3, 1, 2, 3, D.LINEAR)])
+def test_conv_direct(device, B, inC, outC, k, p, H, W, act):
+    from goneuron_b200 import _lib
+    oH, oW = H + 2 * p - k + 1, W + 2 * p - k + 1
+    rng = np.random.default_rng(B * 1000 + inC * 100 + outC * 10 + k)
+    x, w = rng.standard_normal((B, inC, H, W)).astype(np.float32), (rng.standard_normal((outC, inC, k, k)) / np.sqrt(inC * k * k)).astype(np.float32)
+    bias, dy = rng.standard_normal(outC).astype(np.float32), rng.standard_normal((B, outC, oH, oW)).astype(np.float32)
+    y, dx, dw, db = np.empty((B, outC, oH, oW), np.float32), np.empty_like(x), np.empty_like(w), np.empty_like(bias)
+    _lib.check(_lib.load().gn_op_conv2d(device.handle, 0, B, inC, outC, k, 1, p, H, W, act, _f(x), _f(w), _f(bias), _f(dy), _f(y), _f(dx), _f(dw), _f(db)))
+    xp = np.pad(x.astype(np.float64), ((0, 0), (0, 0), (p, p), (p, p)))
+    z = np.zeros((B, outC, oH, oW)) + bias.astype(np.float64)[None, :, None, None]
+    for i in range(k):
+        for j in range(k):
+            z += np.einsum("bchw,oc->bohw", xp[:, :, i:i + oH, j:j + oW], w[:, :, i, j].astype(np.float64), optimize=True)
+    a = {D.LINEAR: z, D.RELU: np.maximum(z, 0), D.TANH: np.tanh(z), D.SIGMOID: 1 / (1 + np.exp(-z))}[act]
+    der = {D.LINEAR: np.ones_like(z), D.RELU: y > 0, D.TANH: 1 - a * a, D.SIGMOID: a * (1 - a)}[act]      # (ReLU: the pattern of the result itself)
+    assert norm_err(y, a) <= 1e-5
+    dz = dy * der
+    dxp, dwr = np.zeros_like(xp), np.zeros(w.shape)
+    for i in range(k):
+        for j in range(k):
+            dxp[:, :, i:i + oH, j:j + oW] += np.einsum("bohw,oc->bchw", dz, w[:, :, i, j].astype(np.float64), optimize=True)
+            dwr[:, :, i, j] = np.einsum("bohw,bchw->oc", dz, xp[:, :, i:i + oH, j:j + oW], optimize=True)
+    dxr = dxp[:, :, p:p + H, p:p + W]
+    assert norm_err(dx, dxr) <= 1e-5 and norm_err(dw, dwr) <= 1e-5 and norm_err(db, dz.sum((0, 2, 3))) <= 1e-5
+
+
+@pytest.mark.parametrize("k,s,p,hw", [(2, 2, 0, 9), (2, 3, 1, 10), (3, 3, 1, 11), (3, 2, 1, 9), (1, 2, 0, 7)])
+def test_maxpool_gradient(device, oracle, k, s, p, hw):
+    from goneuron_b200.sequential import Adam, Sequential
+    o = (hw + 2 * p - k) // s + 1
+    layers = [D.Conv2D(2, 3, 3, 1, 1, D.TANH, hw, hw), D.MaxPool2D(3, k, s, p, hw, hw), D.Flatten(), D.Dense(3 * o * o, 4, D.SOFTMAX)]
+    rng = np.random.Generator(np.random.PCG64(k * 10 + s))
+    params = configs.init_params(layers, rng)
+    x, y = configs.make_inputs("cnn", layers, 5, rng)
+    ref = oracle.OracleState(layers, D.CROSS_ENTROPY, params, lr=1e-3)
+    ref.train_batch(x, y, precision=64)
+    model = Sequential(layers, device).Compile(Adam(1e-3), D.CROSS_ENTROPY)
+    model.SetParams(params)
+    model.TrainBatch(x, y)
+    assert_grads_close(layers, model.Gradients(), ref.grads)
+    model.Close()
+
+
+def test_batchnorm_running_statistics_of_a_long_batch(device, oracle):
+    """More samples than a block stages at a time, more channels than a block has lanes."""
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = [D.Conv2D(1, 40, 1, 1, 0, D.LINEAR, 4, 4), D.BatchNorm2D(40, 4, 4), D.Flatten(), D.Dense(640, 3, D.SOFTMAX)]
+    rng = np.random.Generator(np.random.PCG64(8))
+    params = configs.init_params(layers, rng)
+    x, y = configs.make_inputs("cnn_bn", layers, 300, rng)
+    ref = oracle.OracleState(layers, D.CROSS_ENTROPY, params, lr=1e-3)
+    ref.train_batch(x, y, precision=64)
+    model = Sequential(layers, device).Compile(Adam(1e-3), D.CROSS_ENTROPY)
+    model.SetParams(params)
+    model.TrainBatch(x, y)
+    assert norm_err(model.State(), ref.state) <= TOL
+    model.Close()
