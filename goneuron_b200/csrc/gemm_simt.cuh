@@ -32,6 +32,10 @@ struct GemmDesc {
   const void* plane_out = nullptr;                      // tensor-core engine: a TcPlaneOut; the result is written as operand planes instead of fp32
   float* a_sum = nullptr;                               // CUDA-core engine: receives sum_k A(m,k), [M] (the bias gradient next to a weight gradient)
   float* a_rownorm = nullptr;                           // tensor-core engine: receives the L2 norm of every row of A (from the split pass)
+  // tensor-core engine, several products in one launch: the columns of the result come in segments of n_seg, segment j at C + j c_seg
+  // (bias + j bias_seg): X [Wq; Wk; Wv]^T; the contraction runs over segments of k_seg of A's rows, segment j at A + j a_seg:
+  // dQ Wq + dK Wk + dV Wv; the rows of a transposed A come in segments of m_seg at A + j a_seg.
+  int n_seg = 0, k_seg = 0, m_seg = 0; long c_seg = 0, bias_seg = 0, a_seg = 0;
   int batch1 = 1, batch2 = 1;                           // batch index b -> (b / batch2, b % batch2)
   long a_b1 = 0, a_b2 = 0, b_b1 = 0, b_b2 = 0, c_b1 = 0, c_b2 = 0, r_b1 = 0, r_b2 = 0;
   // Causal structure of attention: tiles that are entirely masked are never touched.
@@ -252,34 +256,47 @@ inline bool gemm_skinny_ok(const GemmDesc& g) {
 // Sum of at most 64 outer products: C[M,N] = sum_k A(m,k) B(k,n) with both operands stored contraction-major (A(m,k) at
 // A[k * sa_k + m], B(k,n) at B[k * sb_k + n]) -- the weight gradient of an inner Dense layer, which only sees one input
 // row per sample (layer.go:591-625), when the batch (or a rank's shard of it) is small.  Every block stages both operand
-// panels of its 64 x 64 output tile in shared memory once; each thread owns a 4 x 4 patch.  The general kernel runs such a
-// product on 64 blocks of 128 x 128 with a contraction of two 16-steps; this one fills the SMs and is bound by writing C.
+// panels of its 16 TM x 64 output tile in shared memory once (16 bytes per asynchronous copy where the alignment allows it); each
+// thread owns a TM x 4 patch.  The general kernel runs such a product on few blocks with a contraction of four 16-steps; this one
+// fills the SMs.  TM = 8 halves the shared-memory reads per multiply-add and the panel traffic: for outputs with enough tiles of that
+// size.  blockIdx.z: several products of one shape, their C (and a_sum) c_b apart (the Q, K and V projections' gradients).
 constexpr int OS_KMAX = 64;
-__global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict__ A, long sa_k, const float* __restrict__ B, long sb_k, float* __restrict__ C, long ldc,
-                                                        int M, int N, int K, float alpha, float* __restrict__ a_sum) {
-  __shared__ __align__(16) float As[OS_KMAX][64];
+template <int TM>
+__global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict__ A, long sa_k, long a_b, const float* __restrict__ B, long sb_k, long b_b, float* __restrict__ C, long ldc, long c_b,
+                                                        int M, int N, int K, float alpha, float* __restrict__ a_sum, int va, int vb) {
+  constexpr int BM = 16 * TM;
+  __shared__ __align__(16) float As[OS_KMAX][BM];
   __shared__ __align__(16) float Bs[OS_KMAX][64];
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int i = tid; i < K * 64; i += 256) {
-    const int k = i >> 6, c = i & 63;
-    As[k][c] = m0 + c < M ? A[(long)k * sa_k + m0 + c] : 0.f;
-    Bs[k][c] = n0 + c < N ? B[(long)k * sb_k + n0 + c] : 0.f;
-  }
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  A += blockIdx.z * a_b; B += blockIdx.z * b_b; C += blockIdx.z * c_b;
+  if (va && m0 + BM <= M) for (int i = tid; i < K * (BM / 4); i += 256) { const int k = i / (BM / 4), c = i % (BM / 4) * 4; cp_async16(&As[k][c], A + (long)k * sa_k + m0 + c); }
+  else
+#pragma unroll 4
+    for (int i = tid; i < K * BM; i += 256) { const int k = i / BM, c = i % BM; As[k][c] = m0 + c < M ? A[(long)k * sa_k + m0 + c] : 0.f; }
+  if (vb && n0 + 64 <= N) for (int i = tid; i < K * 16; i += 256) { const int k = i >> 4, c = (i & 15) * 4; cp_async16(&Bs[k][c], B + (long)k * sb_k + n0 + c); }
+  else
+#pragma unroll 4
+    for (int i = tid; i < K * 64; i += 256) { const int k = i >> 6, c = i & 63; Bs[k][c] = n0 + c < N ? B[(long)k * sb_k + n0 + c] : 0.f; }
+  cp_async_wait();
   __syncthreads();
-  if (a_sum && blockIdx.x == 0 && tid < 64 && m0 + tid < M) { float v = 0.f; for (int k = 0; k < K; k++) v += As[k][tid]; a_sum[m0 + tid] = v; }
-  float acc[4][4] = {};
+  if (a_sum && blockIdx.x == 0 && tid < BM && m0 + tid < M) { float v = 0.f; for (int k = 0; k < K; k++) v += As[k][tid]; a_sum[blockIdx.z * c_b + m0 + tid] = v; }
+  float acc[TM][4] = {};
+#pragma unroll 4
   for (int k = 0; k < K; k++) {
-    const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]), b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
-    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    const float4 b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]); const float bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int h = 0; h < TM / 4; h++) {
+      const float4 a = *reinterpret_cast<const float4*>(&As[k][h * 64 + ty * 4]); const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[4 * h + i][j] = fmaf(av[i], bv[j], acc[4 * h + i][j]);
+    }
   }
   const bool vec = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && n0 + tx * 4 + 3 < N;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int m = m0 + ty * 4 + i; if (m >= M) break;
+  for (int i = 0; i < TM; i++) {
+    const int m = m0 + (i >> 2) * 64 + ty * 4 + (i & 3); if (m >= M) continue;
     float* crow = C + (long)m * ldc + n0 + tx * 4;
     if (vec) *reinterpret_cast<float4*>(crow) = make_float4(alpha * acc[i][0], alpha * acc[i][1], alpha * acc[i][2], alpha * acc[i][3]);
     else
@@ -287,8 +304,8 @@ __global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict_
   }
 }
 inline bool gemm_outer_small_ok(const GemmDesc& g) {
-  return g.sa_m == 1 && g.sb_n == 1 && g.K >= 1 && g.K <= OS_KMAX && g.batch1 * g.batch2 == 1 && !g.bias && !g.R && !g.mask && g.act == GN_ACT_LINEAR && g.flags == 0 &&
-         !g.a_planes && !g.b_planes && !g.plane_out && !g.a_rownorm && (long)g.M * g.N >= 64 * 64;
+  return g.sa_m == 1 && g.sb_n == 1 && g.K >= 1 && g.K <= OS_KMAX && g.batch2 == 1 && g.batch1 <= 65535 && !g.bias && !g.R && !g.mask && g.act == GN_ACT_LINEAR && g.flags == 0 &&
+         !g.a_planes && !g.b_planes && !g.plane_out && !g.a_rownorm && !g.m_seg && (long)g.M * g.N >= 64 * 64;
 }
 
 template <int BM, int BN, int BK, int TM, int TN>
@@ -315,7 +332,12 @@ inline int gemm_simt_splits(const GemmDesc& g, int sm_count, long tiles_all, lon
 inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
   if (g.M <= 0 || g.N <= 0) return GN_OK;
   if (gemm_outer_small_ok(g)) {
-    GN_LAUNCH(ctx, outer_sum_kernel, dim3(cdiv(g.N, 64), cdiv(g.M, 64)), 256, 0, g.A, g.sa_k, g.B, g.sb_k, g.C, g.ldc, g.M, g.N, g.K, g.alpha, g.a_sum);
+    auto vec = [](const float* p, long ld, long bs) { return (int)((reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && bs % 4 == 0); };
+    const int va = vec(g.A, g.sa_k, g.a_b1), vb = vec(g.B, g.sb_k, g.b_b1);
+    // 128-row tiles once they give every SM two blocks
+    if ((long)cdiv(g.N, 64) * cdiv(g.M, 128) * g.batch1 >= 2 * ctx->sm_count)
+      GN_LAUNCH(ctx, outer_sum_kernel<8>, dim3(cdiv(g.N, 64), cdiv(g.M, 128), g.batch1), 256, 0, g.A, g.sa_k, g.a_b1, g.B, g.sb_k, g.b_b1, g.C, g.ldc, g.c_b1, g.M, g.N, g.K, g.alpha, g.a_sum, va, vb);
+    else GN_LAUNCH(ctx, outer_sum_kernel<4>, dim3(cdiv(g.N, 64), cdiv(g.M, 64), g.batch1), 256, 0, g.A, g.sa_k, g.a_b1, g.B, g.sb_k, g.b_b1, g.C, g.ldc, g.c_b1, g.M, g.N, g.K, g.alpha, g.a_sum, va, vb);
     return check_launch("outer_sum");
   }
   if (gemm_skinny_ok(g)) {

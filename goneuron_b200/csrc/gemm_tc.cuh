@@ -43,6 +43,7 @@
 #include <cuda_fp16.h>
 #include <cstdlib>
 #include "common.cuh"
+#include "fmath.cuh"
 #include "gemm_simt.cuh"
 
 namespace gn {
@@ -53,6 +54,7 @@ constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;   // TMA warp, MMA warp, epil
 constexpr unsigned TC_SPIN_LIMIT = 1u << 24;    // default number of polls of one wait (Ctx::spin_limit overrides it)
 constexpr unsigned TC_DRAIN_LIMIT = 1u << 20;   // polls spent waiting for own work in flight after a wait gave up
 constexpr int TC_QUEUE_POOL = 2048;   // tile-queue counters per context before the pool is cleared again
+constexpr int TC_FLAG_SCALE = 8192; // plane output: `mask` holds factors (a GELU layer's derivatives, all below 1.25), not a gate
 constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by the host when every pointer and stride allows it)
 // One stage = 32 contraction indices of both operands.  The two fp16 planes of an operand are interleaved in blocks of 32:
 // element (r, k) of a plane row has its high part at pl_off(k) and its low part PL_LO halves further, so a block of a row is 128
@@ -186,6 +188,8 @@ struct TcParams {
   __half* out_p = nullptr; float* out_inv = nullptr; long out_ldp = 0;
   const float* a_rownorm = nullptr; const int* b_maxabs = nullptr;     // the bound's factors: |row of A|_2 and max |entry of B (and bias)| as float bits
   float* c_last = nullptr; int last_T = 0;                             // fp32 copy of the rows r with r % last_T == last_T - 1: c_last[(r / last_T) * N + col]
+  float* z_last = nullptr;                                             // ... and of their values before the activation
+  int n_seg = 0; long c_seg = 0, bias_seg = 0;                         // > 0 (a multiple of 32): columns j n_seg .. lie c_seg (biases: bias_seg) floats after those of segment j - 1, see GemmDesc::n_seg
   float* rowsum32 = nullptr;                                           // plane output: sums of the result over every 32 consecutive rows, [ceil(M / 32)][N]
 };
 
@@ -205,8 +209,9 @@ __device__ __forceinline__ void tc_epilogue_stage(const TcParams& ep, int n0, in
     __syncwarp();
     for (int i = lane * 4; i < ncw; i += 128) {
       const int col = cbase + i; const bool in = col < ep.N;
+      const long bo = ep.n_seg ? col + (col / ep.n_seg) * (ep.bias_seg - ep.n_seg) : col;
       *reinterpret_cast<float4*>(colv + i) = in ? __ldg(reinterpret_cast<const float4*>(isb + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(colv + BN / 2 + i) = (in && ep.bias) ? __ldg(reinterpret_cast<const float4*>(ep.bias + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(colv + BN / 2 + i) = (in && ep.bias) ? __ldg(reinterpret_cast<const float4*>(ep.bias + bo)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncwarp();
 }
@@ -261,7 +266,7 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
     float osc = 1.f;                                                         // this lane's row's scale
     if (row < ep.M) {
       const float an = ep.a_rownorm[row], bound = sqrtf(fmaf(an, an, 1.f)) * sqrtf((float)ep.K + 1.f) * __int_as_float(*ep.b_maxabs);
-      float oinv; osc = row_scale(bound, &oinv);
+      float oinv; osc = row_scale(ep.flags & TC_FLAG_SCALE ? 1.25f * bound : bound, &oinv);
       if (n0 == 0 && chalf == 0) ep.out_inv[row] = oinv;
     }
 #pragma unroll 1
@@ -286,12 +291,18 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
           if (!col_ok || r >= ep.M) continue;
           const float4 a = *reinterpret_cast<const float4*>(stg + (4 * t + rl) * TC_STG_LD + c4);
           float4 x = make_float4(a.x * sv.x + bv.x, a.y * sv.y + bv.y, a.z * sv.z + bv.z, a.w * sv.w + bv.w);
+          const bool is_last = ep.c_last && r % ep.last_T == ep.last_T - 1; const long lo = (long)(r / ep.last_T) * ep.N + col;
           if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
-          if (!(mv[t].x > 0.f)) x.x = 0.f; if (!(mv[t].y > 0.f)) x.y = 0.f; if (!(mv[t].z > 0.f)) x.z = 0.f; if (!(mv[t].w > 0.f)) x.w = 0.f;
+          else if (ep.act == GN_ACT_GELU) {
+            if (is_last && ep.z_last) *reinterpret_cast<float4*>(ep.z_last + lo) = x;
+            x.x = gelu_f(x.x); x.y = gelu_f(x.y); x.z = gelu_f(x.z); x.w = gelu_f(x.w);
+          }
+          if (ep.flags & TC_FLAG_SCALE) { x.x *= mv[t].x; x.y *= mv[t].y; x.z *= mv[t].z; x.w *= mv[t].w; }
+          else { if (!(mv[t].x > 0.f)) x.x = 0.f; if (!(mv[t].y > 0.f)) x.y = 0.f; if (!(mv[t].z > 0.f)) x.z = 0.f; if (!(mv[t].w > 0.f)) x.w = 0.f; }
           uint2 p0, p1; split2_pair(x.x, x.y, os, p0.x, p1.x); split2_pair(x.z, x.w, os, p0.y, p1.y);
           __half* o = ep.out_p + (long)r * 2 * ep.out_ldp + pl_off(col);
           *reinterpret_cast<uint2*>(o) = p0; *reinterpret_cast<uint2*>(o + PL_LO) = p1;
-          if (ep.c_last && r % ep.last_T == ep.last_T - 1) *reinterpret_cast<float4*>(ep.c_last + (long)(r / ep.last_T) * ep.N + col) = x;
+          if (is_last) *reinterpret_cast<float4*>(ep.c_last + lo) = x;
           csum.x += x.x; csum.y += x.y; csum.z += x.z; csum.w += x.w;
         }
       }
@@ -318,12 +329,14 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
       if (n0 + c * 32 >= ep.N) break;
       float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
       const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + BN / 2 + cc * 32 + c4);
+      const long so = ep.n_seg ? ((n0 + c * 32) / ep.n_seg) * (ep.c_seg - ep.n_seg) : 0;      // (32 columns lie in one segment; with segments R is C)
+      float* Cs = C + so; const float* Rs = R + so;
 #pragma unroll 1
       for (int hh = 0; hh < 2; hh++) {
         const int r0 = rbase + 16 * hh + rl;
         float4 rv[4];                                                        // residual, fetched before the exchange so that its latency overlaps it
 #pragma unroll
-        for (int t = 0; t < 4; t++) rv[t] = (R && col_ok && r0 + 4 * t < ep.M) ? *reinterpret_cast<const float4*>(R + (long)(r0 + 4 * t) * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t = 0; t < 4; t++) rv[t] = (R && col_ok && r0 + 4 * t < ep.M) ? *reinterpret_cast<const float4*>(Rs + (long)(r0 + 4 * t) * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
         tc_stage_rows(stg, v, lane, hh);
 #pragma unroll
         for (int t = 0; t < 4; t++) {
@@ -336,7 +349,7 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
             const float4 mv = *reinterpret_cast<const float4*>(ep.mask + (long)(r / ep.mask_group) * ep.mask_ld + col);
             if (!(mv.x > 0.f)) x.x = 0.f; if (!(mv.y > 0.f)) x.y = 0.f; if (!(mv.z > 0.f)) x.z = 0.f; if (!(mv.w > 0.f)) x.w = 0.f;
           }
-          *reinterpret_cast<float4*>(C + (long)r * ep.ldc + col) = x;
+          *reinterpret_cast<float4*>(Cs + (long)r * ep.ldc + col) = x;
         }
       }
     }
@@ -354,17 +367,18 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
   for (int cc = 0; cc < nch; cc++) {
     const int col0 = n0 + (chalf * nch + cc) * 32;
     if (col0 >= ep.N) break;
+    const int seg = ep.n_seg ? col0 / ep.n_seg : 0; const long c_off = ep.n_seg ? seg * (ep.c_seg - ep.n_seg) : 0, b_off = ep.n_seg ? seg * (ep.bias_seg - ep.n_seg) : 0;
     float v[32]; tc_acc_chunk<MERGED>(tquad + (chalf * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
 #pragma unroll
     for (int j = 0; j < 32; j++) {
       const int col = col0 + j;
       if (!row_ok || col >= ep.N) continue;
       float x = v[j] * isb[col];
-      if (ep.bias) x += ep.bias[col];
-      if (Rrow) x += Rrow[col];
+      if (ep.bias) x += ep.bias[b_off + col];
+      if (Rrow) x += Rrow[c_off + col];
       if (ep.act == GN_ACT_RELU) x = fmaxf(x, 0.f);
       if (Mrow && !(Mrow[col] > 0.f)) x = 0.f;
-      Crow[col * cstep] = x;
+      Crow[c_off + col * cstep] = x;
     }
   }
 }
@@ -564,7 +578,9 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
 // (z, r, c) at p + (z / batch2) * b1 + (z % batch2) * b2 + r * s_r + c * s_c.  One of s_r, s_c is 1:
 // s_c == 1 reads rows directly; s_r == 1 (the operand is the transpose of what is stored) goes through a shared tile.
 // Two fp16 planes per operand, fp16(x s) and fp16(x s - fp16(x s)), interleaved (pl_off), and the inverse 1/s of every plane row's scale.
-struct TcSrc { const float* p; long s_r, s_c, b1, b2; int batch2; };
+// Rows may consist of segments of `seg` elements (> 0, a multiple of 32), each `seg_stride` floats after the one before: column c at
+// p + r * s_r + c % seg + (c / seg) * seg_stride.
+struct TcSrc { const float* p; long s_r, s_c, b1, b2; int batch2; int seg = 0; long seg_stride = 0; };
 // One warp per plane row: first the row's largest magnitude (the row is read a second time from L1 / L2 afterwards),
 // then eight elements per lane and step (two 16-byte loads, one 16-byte store per plane).  blockIdx.y = problem index.
 // `rownorm` (may be null): receives the L2 norm of every row (a factor of the bound of a plane-output contraction).
@@ -574,28 +590,32 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int
   const long r = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= rows) return;
   const float* src = s.p + (z / s.batch2) * s.b1 + (z % s.batch2) * s.b2 + r * s.s_r;
-  const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  const int seg = s.seg ? s.seg : cols; const long over = s.seg ? s.seg_stride - s.seg : 0;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(over * 4)) & 15) == 0;
   const int cols8 = vec ? (cols & ~7) : 0;                  // columns handled with 16-byte loads
   float mx = 0.f, sq = 0.f;
+#pragma unroll 2
   for (int c = lane * 8; c < cols8; c += 256) {
-    const float4 a = *reinterpret_cast<const float4*>(src + c), b = *reinterpret_cast<const float4*>(src + c + 4);
+    const float* q = src + c + (over ? c / seg * over : 0);
+    const float4 a = *reinterpret_cast<const float4*>(q), b = *reinterpret_cast<const float4*>(q + 4);
     mx = fmaxf(mx, fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))), fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w)))));
     sq += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w + b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
   }
-  for (int c = cols8 + lane; c < cols; c += 32) { const float v = src[c]; mx = fmaxf(mx, fabsf(v)); sq += v * v; }
+  for (int c = cols8 + lane; c < cols; c += 32) { const float v = src[c + (over ? c / seg * over : 0)]; mx = fmaxf(mx, fabsf(v)); sq += v * v; }
   mx = warp_max(mx);
   if (rownorm) { sq = warp_sum(sq); if (lane == 0) rownorm[(long)z * rows + r] = sqrtf(sq) * 1.0001f; }
   float inv; const float sc = row_scale(mx, &inv);
   if (lane == 0) inv_scale[(long)z * rows + r] = inv;
   __half* o = pl + ((long)z * rows + r) * 2 * ldp;
+#pragma unroll 2
   for (int c = lane * 8; c < ldp; c += 256) {
-    float t[8];
+    float t[8]; const float* q = src + c + (over ? c / seg * over : 0);
     if (c + 7 < cols8) {
-      const float4 a = *reinterpret_cast<const float4*>(src + c), b = *reinterpret_cast<const float4*>(src + c + 4);
+      const float4 a = *reinterpret_cast<const float4*>(q), b = *reinterpret_cast<const float4*>(q + 4);
       t[0] = a.x; t[1] = a.y; t[2] = a.z; t[3] = a.w; t[4] = b.x; t[5] = b.y; t[6] = b.z; t[7] = b.w;
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; j++) t[j] = c + j < cols ? src[c + j] : 0.f;
+      for (int j = 0; j < 8; j++) t[j] = c + j < cols ? q[j] : 0.f;
     }
     uint4 a, b;
     split2_pair(t[0], t[1], sc, a.x, b.x); split2_pair(t[2], t[3], sc, a.y, b.y);
@@ -659,7 +679,7 @@ struct BfPlanes { __half* base; float* inv_scale; int rows, K, ldp, nbatch; int 
 // random-sign data the bound is about 8-16 times the row's actual maximum, i.e. 3-4 of the planes' 22 bits; it can never
 // be exceeded, so the fp16 planes cannot overflow.  `last`: fp32 copy of every sequence's last row (the only rows of
 // these tensors that are read as numbers: ReLU gate and weight-gradient input of the reference's last-token rule).
-struct TcPlaneOut { BfPlanes planes; const int* b_maxabs; float* last; int last_T; float* rowsum32 = nullptr; };
+struct TcPlaneOut { BfPlanes planes; const int* b_maxabs; float* last; int last_T; float* rowsum32 = nullptr; float* z_last = nullptr; bool scale = false; };
 inline int tc_ldp(int K) { return ((K + 31) / 32) * 32; }           // plane row length: whole blocks of 32
 inline size_t bf_plane_floats(long nbatch, long rows, long ldp) { return (size_t)nbatch * rows * ldp; }   // two fp16 planes = one float per element
 
@@ -791,10 +811,11 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
   auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   bool vec = ep.N % 4 == 0 && ep.ldc % 4 == 0 && ep.c_b1 % 4 == 0 && ep.c_b2 % 4 == 0 && a16(ep.C) && (!ep.bias || a16(ep.bias)) && a16(ep.isb);
   if (ep.R) vec = vec && ep.ldr % 4 == 0 && ep.r_b1 % 4 == 0 && ep.r_b2 % 4 == 0 && a16(ep.R);
+  if (ep.n_seg) vec = vec && ep.c_seg % 4 == 0 && ep.bias_seg % 4 == 0;
   if (ep.mask) vec = vec && ep.mask_ld % 4 == 0 && a16(ep.mask);
   if (ep.nchw_P > 0) { if (ep.R || A.nbatch != 1) return fail(GN_ERR_UNSUPPORTED, "tc_launch: NCHW store with a residual or a batch"); vec = false; }
   if (ep.out_p) {
-    if (!(ep.N % 4 == 0 && (!ep.bias || a16(ep.bias)) && a16(ep.isb) && (!ep.mask || (ep.mask_ld % 4 == 0 && a16(ep.mask))) && ep.out_ldp % 4 == 0 && (!ep.c_last || a16(ep.c_last))))
+    if (!(ep.N % 4 == 0 && (!ep.bias || a16(ep.bias)) && a16(ep.isb) && (!ep.mask || (ep.mask_ld % 4 == 0 && a16(ep.mask))) && ep.out_ldp % 4 == 0 && (!ep.c_last || a16(ep.c_last)) && (!ep.z_last || a16(ep.z_last))))
       return fail(GN_ERR_INVALID_ARG, "tc_launch: plane output needs 16-byte aligned operands");
     vec = true;
   }
@@ -840,7 +861,10 @@ inline int tc_run(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams
 // GPUs.  Instead all registered matrices are split once per parameter update, both orientations from one read, by two
 // launches in all: the matrices get ONE power-of-two scale each (their entries are of similar size, unlike activation
 // rows), found by wplanes_max_kernel, and wplanes_split_kernel writes every 64 x 64 tile as stored and transposed.
-struct WPlaneJob { const float* src; const float* bias; int out, in, ldp_r, ldp_c; __half *r, *c; float *inv_r, *inv_c; int tile0, tiles_in; };
+// A registered matrix may be a stack of several (Q, K and V projections; SwiGLU gate and up): rows [j part, (j + 1) part) come from
+// src + j * stride.  Products may then use the whole stack or a run of its parts.
+struct WPlaneJob { const float* src; const float* bias; int part; long stride; int out, in, ldp_r, ldp_c; __half *r, *c; float *inv_r, *inv_c; int tile0, tiles_in; };
+__device__ __forceinline__ const float* wplane_row(const WPlaneJob& jb, int r) { const int j = r / jb.part; return jb.src + j * jb.stride + (long)(r - j * jb.part) * jb.in; }
 __device__ __forceinline__ int wplane_find(const WPlaneJob* jobs, int njobs, int tile) {
   int lo = 0, hi = njobs - 1;
   while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (jobs[mid].tile0 <= tile) lo = mid; else hi = mid - 1; }
@@ -852,8 +876,8 @@ __global__ void __launch_bounds__(256) wplanes_max_kernel(const WPlaneJob* __res
   const int j = wplane_find(jobs, njobs, tile); const WPlaneJob jb = jobs[j];
   const int t = tile - jb.tile0, r0 = (t / jb.tiles_in) * 64, c0 = (t % jb.tiles_in) * 64;
   float m = 0.f;
-  for (int e = threadIdx.x; e < 4096; e += 256) { const int r = r0 + (e >> 6), c = c0 + (e & 63); if (r < jb.out && c < jb.in) m = fmaxf(m, fabsf(jb.src[(long)r * jb.in + c])); }
-  if (jb.bias && c0 == 0 && threadIdx.x < 64 && r0 + (int)threadIdx.x < jb.out) m = fmaxf(m, fabsf(jb.bias[r0 + threadIdx.x]));      // the layer's biases count towards the maximum (bounds of plane-output contractions)
+  for (int e = threadIdx.x; e < 4096; e += 256) { const int r = r0 + (e >> 6), c = c0 + (e & 63); if (r < jb.out && c < jb.in) m = fmaxf(m, fabsf(wplane_row(jb, r)[c])); }
+  if (jb.bias && c0 == 0 && threadIdx.x < 64 && r0 + (int)threadIdx.x < jb.out) m = fmaxf(m, fabsf(jb.bias[(r0 + (int)threadIdx.x) / jb.part * jb.stride + (r0 + (int)threadIdx.x) % jb.part]));      // the layer's biases count towards the maximum (bounds of plane-output contractions)
   m = block_max(m, red);
   if (threadIdx.x == 0) { if (!(m <= 3.0e38f)) m = 3.4e38f; atomicMax(mx + j, __float_as_int(m)); }
 }
@@ -863,7 +887,7 @@ __global__ void __launch_bounds__(256) wplanes_split_kernel(const WPlaneJob* __r
   const int j = wplane_find(jobs, njobs, tile); const WPlaneJob jb = jobs[j];
   const int t = tile - jb.tile0, r0 = (t / jb.tiles_in) * 64, c0 = (t % jb.tiles_in) * 64;
   float inv; const float sc = row_scale(__int_as_float(mx[j]), &inv);
-  for (int e = threadIdx.x; e < 4096; e += 256) { const int rr = e >> 6, cc = e & 63; const int r = r0 + rr, c = c0 + cc; tl[rr][cc] = (r < jb.out && c < jb.in) ? jb.src[(long)r * jb.in + c] : 0.f; }
+  for (int e = threadIdx.x; e < 4096; e += 256) { const int rr = e >> 6, cc = e & 63; const int r = r0 + rr, c = c0 + cc; tl[rr][cc] = (r < jb.out && c < jb.in) ? wplane_row(jb, r)[c] : 0.f; }
   __syncthreads();
   const int x2 = (threadIdx.x & 31) * 2, y = threadIdx.x >> 5;
   for (int rr = y; rr < 64; rr += 8) {                        // as stored: plane row = out index, two neighbouring in indices per thread
@@ -886,7 +910,8 @@ __global__ void __launch_bounds__(256) wplanes_split_kernel(const WPlaneJob* __r
   }
 }
 // Host side of the table: one entry per registered matrix, looked up by the matrix's device address.
-struct WeightPlaneEntry { const float* src; int out, in; BfPlanes rows, cols; const float* bias = nullptr; const int* maxabs = nullptr; int layer = -1; int tile0 = 0, tiles = 0; };
+struct WeightPlaneEntry { const float* src; int out, in; BfPlanes rows, cols; int part = 0; long stride = 0;      // (part = out: a single matrix)
+  const float* bias = nullptr; const int* maxabs = nullptr; int layer = -1; int tile0 = 0, tiles = 0; };
 struct WeightPlaneTable {
   std::vector<WeightPlaneEntry> e; DevBuf planes, scales, mx, jobs; int total_tiles = 0; bool dirty = true, used = false;      // used: some product has looked a matrix up
   // entries [j0, j1) that belong to model layer `layer` (they are registered layer by layer, so the range is contiguous)
@@ -894,13 +919,17 @@ struct WeightPlaneTable {
     *j0 = *j1 = 0; bool in = false;
     for (int j = 0; j < (int)e.size(); j++) if (e[j].layer == layer) { if (!in) { *j0 = j; in = true; } *j1 = j + 1; }
   }
-  const WeightPlaneEntry* find(const float* p) const { for (auto& x : e) if (x.src == p) return &x; return nullptr; }
+  const WeightPlaneEntry* find(const float* p, int* part) const {
+    for (auto& x : e) for (int j = 0; j < x.out / x.part; j++) if (x.src + j * x.stride == p) { *part = j; return &x; }
+    return nullptr;
+  }
 };
 // Lays the table out for the matrices (src, out, in) and allocates its buffers (planes zeroed once: the padding columns
 // of a plane row are never written afterwards and must read as zero).
 inline int wplanes_build(Ctx* ctx, WeightPlaneTable& t, const std::vector<WeightPlaneEntry>& mats) {
   t.e = mats; size_t halves = 0, nscale = 0; int tiles = 0; std::vector<WPlaneJob> jobs;
   for (auto& x : t.e) {
+    if (x.part == 0) { x.part = x.out; x.stride = 0; }
     const int lr = tc_ldp(x.in), lc = tc_ldp(x.out);
     halves += 2 * ((size_t)x.out * lr + (size_t)x.in * lc); nscale += (size_t)x.out + x.in + 8;
   }
@@ -913,7 +942,7 @@ inline int wplanes_build(Ctx* ctx, WeightPlaneTable& t, const std::vector<Weight
     x.rows = BfPlanes{hp, sp, x.out, x.in, lr, 1}; hp += 2 * (size_t)x.out * lr; sp += (x.out + 3) & ~3;
     x.cols = BfPlanes{hp, sp, x.in, x.out, lc, 1}; hp += 2 * (size_t)x.in * lc; sp += (x.in + 3) & ~3;
     x.maxabs = reinterpret_cast<const int*>(t.mx.p) + jobs.size();
-    WPlaneJob jb{x.src, x.bias, x.out, x.in, lr, lc, x.rows.base, x.cols.base, x.rows.inv_scale, x.cols.inv_scale, tiles, (int)cdiv(x.in, 64)};
+    WPlaneJob jb{x.src, x.bias, x.part, x.stride, x.out, x.in, lr, lc, x.rows.base, x.cols.base, x.rows.inv_scale, x.cols.inv_scale, tiles, (int)cdiv(x.in, 64)};
     x.tile0 = tiles; x.tiles = (int)cdiv(x.out, 64) * (int)cdiv(x.in, 64);
     tiles += x.tiles; jobs.push_back(jb);
   }
@@ -941,16 +970,20 @@ inline int wplanes_refresh(Ctx* ctx, WeightPlaneTable& t) {
   t.dirty = false; return GN_OK;
 }
 // Prepared planes for B of this contraction, if B is a registered matrix used in one of its two orientations.
-inline const BfPlanes* wplanes_lookup(Ctx* ctx, const GemmDesc& g, const WeightPlaneEntry** entry = nullptr) {
+inline bool wplanes_lookup(Ctx* ctx, const GemmDesc& g, BfPlanes* p, const WeightPlaneEntry** entry = nullptr) {
   WeightPlaneTable* t = static_cast<WeightPlaneTable*>(ctx->weight_planes);
-  if (!t || g.batch1 * g.batch2 != 1) return nullptr;
-  const WeightPlaneEntry* x = t->find(g.B); if (!x) return nullptr;
-  if (t->dirty && wplanes_refresh(ctx, *t) != GN_OK) return nullptr;       // once per parameter update, when the first product asks
+  if (!t || g.batch1 * g.batch2 != 1) return false;
+  int part = 0; const WeightPlaneEntry* x = t->find(g.B, &part); if (!x) return false;
+  const int r0 = part * x->part;
+  const bool stored = g.sb_k == 1 && g.sb_n == x->in && g.K == x->in && g.N % x->part == 0 && r0 + g.N <= x->out;          // B(k, n) = W[r0 + n, k]
+  const bool transposed = !stored && g.sb_n == 1 && g.sb_k == x->in && g.N == x->in && g.K % x->part == 0 && r0 + g.K <= x->out;      // B(k, n) = W[r0 + k, n]
+  if (!stored && !transposed) return false;
+  if (t->dirty && wplanes_refresh(ctx, *t) != GN_OK) return false;         // once per parameter update, when the first product asks
   t->used = true;
   if (entry) *entry = x;
-  if (g.sb_k == 1 && g.sb_n == x->in && g.N == x->out && g.K == x->in) return &x->rows;     // B(k, n) = W[n, k]
-  if (g.sb_n == 1 && g.sb_k == x->in && g.N == x->in && g.K == x->out) return &x->cols;     // B(k, n) = W[k, n]
-  return nullptr;
+  if (stored) { *p = x->rows; p->base += 2 * (long)r0 * p->ldp; p->inv_scale += r0; p->rows = g.N; }
+  else { *p = x->cols; p->koff = r0; p->K = g.K; }
+  return true;
 }
 
 // Can the engine run this contraction at all?  One of each operand's strides must be 1; LINEAR/RELU epilogue; alpha 1.
@@ -959,7 +992,7 @@ inline bool gemm_tc_supported(Ctx* ctx, const GemmDesc& g) {
   if (g.alpha != 1.f) return false;
   if (!(g.sa_k == 1 || g.sa_m == 1)) return false;
   if (!(g.sb_k == 1 || g.sb_n == 1)) return false;
-  if (g.act != GN_ACT_LINEAR && g.act != GN_ACT_RELU) return false;
+  if (g.act != GN_ACT_LINEAR && g.act != GN_ACT_RELU && !(g.act == GN_ACT_GELU && g.plane_out)) return false;
   return g.M > 0 && g.N > 0 && g.K > 0;
 }
 // Is it worth it?  Small or skinny problems stay on the CUDA-core engine, which needs no operand planes: 1e8 multiply-adds take it
@@ -982,6 +1015,14 @@ inline int gemm_tc(Ctx* ctx, const GemmDesc& g) {
   if (g.a_planes) {
     A = *static_cast<const BfPlanes*>(g.a_planes);
     if (A.rows != g.M || A.K != g.K || A.nbatch != nb) return fail(GN_ERR_INVALID_ARG, "gemm_tc: prepared planes of A do not match the contraction");
+  } else if (g.m_seg) {
+    // the rows of A (a transposed operand) come from M / m_seg arrays: as a batch, whose planes lie one after the other
+    if (g.sa_m != 1 || nb != 1 || g.M % g.m_seg) return fail(GN_ERR_INVALID_ARG, "gemm_tc: row segments need a transposed A");
+    BfPlanes S = A; S.rows = g.m_seg; S.nbatch = g.M / g.m_seg;
+    GN_TRY(tc_split(ctx, TcSrc{g.A, g.sa_m, g.sa_k, g.a_seg, 0, 1}, S, mx)); sc.last_a = nullptr;
+  } else if (g.k_seg) {
+    if (g.sa_k != 1 || nb != 1 || g.k_seg % 32) return fail(GN_ERR_INVALID_ARG, "gemm_tc: contraction segments need a row-major A and a multiple of 32");
+    GN_TRY(tc_split(ctx, TcSrc{g.A, g.sa_m, g.sa_k, g.a_b1, g.a_b2, g.batch2, g.k_seg, g.a_seg}, A, mx, g.a_rownorm)); sc.last_a = nullptr;
   } else if (!g.a_rownorm && g.reuse_a_planes && nb == 1 && sc.last_a == g.A && sc.last_m == g.M && sc.last_k == g.K && sc.last_ld == g.sa_m && g.sa_k == 1) {
     // same tensor as the previous call (the Q, K and V projections share their input): planes still valid
   } else {
@@ -993,12 +1034,17 @@ inline int gemm_tc(Ctx* ctx, const GemmDesc& g) {
     if (B.rows != g.N || B.K != g.K || B.nbatch != nb) return fail(GN_ERR_INVALID_ARG, "gemm_tc: prepared planes of B do not match the contraction");
   } else GN_TRY(tc_split(ctx, TcSrc{g.B, g.sb_n, g.sb_k, g.b_b1, g.b_b2, g.batch2}, B, mx));
   TcParams ep{g.C, g.ldc, g.c_b1, g.c_b2, g.bias, g.R, g.ldr, g.r_b1, g.r_b2, g.act, g.M, g.N, g.K, g.batch2, g.flags, ctx->d_status, g.mask, g.mask_ld, g.mask_group};
+  if (g.n_seg) {
+    if (g.n_seg % 32 || nb != 1 || g.R || g.plane_out) return fail(GN_ERR_INVALID_ARG, "gemm_tc: this contraction cannot write its columns in segments");
+    ep.n_seg = g.n_seg; ep.c_seg = g.c_seg; ep.bias_seg = g.bias_seg;
+  }
   if (g.plane_out) {
     const TcPlaneOut& po = *static_cast<const TcPlaneOut*>(g.plane_out);
     if (nb != 1 || g.R || !g.a_rownorm || !po.b_maxabs || g.N % 32 || po.planes.rows != g.M || po.planes.K != g.N || (g.flags & (GEMM_SKIP_UPPER | GEMM_KBEG_AT_M0 | GEMM_KEND_AT_M0)))
       return fail(GN_ERR_INVALID_ARG, "gemm_tc: this contraction cannot write its result as operand planes");
     ep.out_p = po.planes.base; ep.out_inv = po.planes.inv_scale; ep.out_ldp = po.planes.ldp;
-    ep.a_rownorm = g.a_rownorm; ep.b_maxabs = po.b_maxabs; ep.c_last = po.last; ep.last_T = po.last_T > 0 ? po.last_T : 1; ep.rowsum32 = po.rowsum32;
+    ep.a_rownorm = g.a_rownorm; ep.b_maxabs = po.b_maxabs; ep.c_last = po.last; ep.last_T = po.last_T > 0 ? po.last_T : 1; ep.rowsum32 = po.rowsum32; ep.z_last = po.z_last;
+    if (po.scale) ep.flags |= TC_FLAG_SCALE;
   }
   return tc_run(ctx, A, B, ep);
 }

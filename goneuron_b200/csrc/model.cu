@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 
 #include "common.cuh"
@@ -40,7 +41,7 @@ static bool gemm_on_tc(Ctx* ctx, const GemmDesc& g) { return !force_simt_engine(
 static int gemm(Ctx* ctx, const GemmDesc& g) {
   int rc;
   if (gemm_on_tc(ctx, g)) {     // brackets its kernel launches itself
-    GemmDesc h = g; if (!h.b_planes) h.b_planes = wplanes_lookup(ctx, g);                 // weight matrices come with prepared planes
+    GemmDesc h = g; BfPlanes w; if (!h.b_planes && wplanes_lookup(ctx, g, &w)) h.b_planes = &w;                 // weight matrices come with prepared planes
     rc = gemm_tc(ctx, h);
   }
   else { ProfScope prof(ctx); rc = gemm_simt(ctx, g); }
@@ -67,7 +68,36 @@ static int gemm_tn(Ctx* ctx, int R, int N, int K, const float* dZ, long ldz, con
   g.C = gW; g.ldc = K; return gemm(ctx, g);
 }
 
-// The same with the bias gradient gb[N] = sum of dZ over its rows, inside the product where the CUDA-core engine runs it.
+// Products with several weight matrices W_j [n, d], `ws` floats apart, in one launch where the tensor-core engine runs them and holds
+// their planes as a stack, else one by one.  At 3600 rows of 384 the three projections are 87 tiles each: 1.8 rounds of the SMs
+// together, three alone.
+// Y_j[M, n] = X W_j^T + b_j; Y_j and b_j are cs and ws floats apart
+static int gemm_nt_stack(Ctx* ctx, int parts, int M, int n, int d, const float* X, long ldx, const float* W, long ws, const float* bias, float* Y, long cs, const BfPlanes* x_planes = nullptr) {
+  GemmDesc g; g.M = M; g.N = parts * n; g.K = d; g.A = X; g.sa_m = ldx; g.sa_k = 1; g.B = W; g.sb_k = 1; g.sb_n = d; g.C = Y; g.ldc = n; g.bias = bias;
+  g.n_seg = n; g.c_seg = cs; g.bias_seg = ws; g.a_planes = x_planes; BfPlanes w;
+  if (parts > 1 && n % 32 == 0 && gemm_on_tc(ctx, g) && wplanes_lookup(ctx, g, &w)) { g.b_planes = &w; return gemm(ctx, g); }
+  g.N = n; g.n_seg = 0;
+  for (int j = 0; j < parts; j++) { g.B = W + j * ws; g.C = Y + j * cs; g.bias = bias ? bias + j * ws : nullptr; GN_TRY(gemm(ctx, g)); g.reuse_a_planes = true; }
+  return GN_OK;
+}
+// dX[M, d] = sum_j dZ_j W_j + R; dZ_j [M, n] are zs floats apart
+static int gemm_nn_stack(Ctx* ctx, int parts, int M, int n, int d, const float* dZ, long zs, const float* W, long ws, float* dX, const float* R, const BfPlanes* z_planes = nullptr) {
+  GemmDesc g; g.M = M; g.N = d; g.K = parts * n; g.A = dZ; g.sa_m = n; g.sa_k = 1; g.B = W; g.sb_k = d; g.sb_n = 1; g.C = dX; g.ldc = d; g.R = R; g.ldr = d;
+  g.k_seg = n; g.a_seg = zs; g.a_planes = z_planes; BfPlanes w;
+  if (parts > 1 && n % 32 == 0 && gemm_on_tc(ctx, g) && wplanes_lookup(ctx, g, &w)) { g.b_planes = &w; return gemm(ctx, g); }
+  g.K = n; g.k_seg = 0; g.a_planes = nullptr;
+  for (int j = 0; j < parts; j++) { g.A = dZ + j * zs; g.B = W + j * ws; GN_TRY(gemm(ctx, g)); g.R = dX; }
+  return GN_OK;
+}
+// gW_j[n, d] = dZ_j^T X, one after the other in memory
+static int gemm_tn_stack(Ctx* ctx, int parts, int R, int n, int d, const float* dZ, long zs, const float* X, long ldx, float* gW) {
+  GemmDesc g; g.M = parts * n; g.N = d; g.K = R; g.A = dZ; g.sa_m = 1; g.sa_k = n; g.B = X; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = d; g.m_seg = n; g.a_seg = zs;
+  if (parts > 1 && gemm_on_tc(ctx, g)) return gemm(ctx, g);
+  g.M = n; g.m_seg = 0;
+  for (int j = 0; j < parts; j++) { g.A = dZ + j * zs; g.C = gW + (long)j * n * d; GN_TRY(gemm(ctx, g)); }
+  return GN_OK;
+}
+// gemm_tn with the bias gradient gb[N] = sum of dZ over its rows, inside the product where the CUDA-core engine runs it.
 static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate);
 static int weight_bias_grads(gn_model* m, Ctx* ctx, int R, int N, int K, const float* dZ, long ldz, const float* X, long ldx, float* gW, float* gb) {
   GemmDesc g; g.M = N; g.N = K; g.K = R; g.A = dZ; g.sa_m = 1; g.sa_k = ldz; g.B = X; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = K;
@@ -258,7 +288,7 @@ static int plan_layers(gn_model* m, const gn_layer_desc* layers, int n) {
 }
 
 static void plan_token_rows(gn_model* m, bool training);
-// Activation buffers of a TransformerBlock, by number.
+// Activation buffers of a TransformerBlock, by number (k, v and up are views: q | k | v and gate | up lie in one buffer each).
 constexpr int NBLK = 18;
 static DevBuf& block_buf(LayerRT& l, int k) {
   DevBuf* b[NBLK] = {&l.q, &l.k, &l.v, &l.att, &l.r1, &l.n1, &l.mid, &l.r2, &l.out, &l.stat, &l.gate, &l.up, &l.mid_last, &l.zlast, &l.mid_inv, &l.att_m, &l.att_l, &l.att_d};
@@ -266,7 +296,7 @@ static DevBuf& block_buf(LayerRT& l, int k) {
 }
 static void block_sizes(const LayerRT& l, size_t c, size_t (&n)[NBLK]) {
   const gn_layer_desc& d = l.d; const size_t nd = c * d.seq_len * d.dim, nf = c * d.seq_len * d.ff_dim, nt = c * d.seq_len, bf = c * d.ff_dim;
-  const size_t v[NBLK] = {nd, nd, nd, nd, nd, nd, nf, nd, nd, 4 * nt, l.ff_act == GN_ACT_SILU ? nf : 0, l.ff_act == GN_ACT_SILU ? nf : 0, bf, l.ff_act == GN_ACT_GELU ? bf : 0, nt, nt * d.heads, nt * d.heads, nt * d.heads};
+  const size_t v[NBLK] = {3 * nd, 0, 0, nd, nd, nd, nf, nd, nd, 4 * nt, l.ff_act == GN_ACT_SILU ? 2 * nf : 0, 0, bf, l.ff_act == GN_ACT_GELU ? bf : 0, nt, nt * d.heads, nt * d.heads, nt * d.heads};
   for (int k = 0; k < NBLK; k++) n[k] = v[k];
 }
 // Which blocks can use one set of activation buffers: all of them in inference; in training those whose backward pass needs the
@@ -324,6 +354,8 @@ static int alloc_activations(gn_model* m, int cap, bool training) {
           if (own) GN_TRY(b.alloc(need[k])); else b.view(need[k] ? m->shared[k == 8 && n_shared % 2 ? NBLK : k].p : nullptr, need[k]);
         }
         if (share) n_shared++;
+        const size_t nd = need[3], nf = need[6]; l.k.view(l.q.p + nd, nd); l.v.view(l.q.p + 2 * nd, nd);
+        if (need[10]) l.up.view(l.gate.p + nf, nf);
         if (kept) GN_TRY(l.keep.alloc(c * (5 * (size_t)d.dim + 3 * (size_t)d.ff_dim + 4))); else l.keep.release();
         break; }
       case GN_LAYER_CLS_POOLING: GN_TRY(l.out.alloc(c * l.out_size)); break;
@@ -351,48 +383,63 @@ static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* ou
   return check_launch("colsum");
 }
 
-// LayerNorm forward: the row-in-registers kernel when the row length allows it.
-// `po` (optional): the output also as operand planes; *emitted tells the caller whether the kernel that ran could do it
-// (the row-in-registers kernels for widths 128, 256, 512, 1024).
-static bool layernorm_vec_width(int n) { return n == 128 || n == 256 || n == 512 || n == 1024; }
-static int layernorm_forward(Ctx* ctx, const float* x, const float* gamma, const float* beta, float* y, float* mean, float* sd, long rows, int n,
-                             const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
-  const bool vec = n % 128 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15) == 0;
-  const RowPlaneOut out = (po && vec && layernorm_vec_width(n)) ? *po : RowPlaneOut{};
-  if (emitted) *emitted = out.p != nullptr;
-  switch (vec ? n / 128 : 0) {
-    case 1: GN_LAUNCH(ctx, layernorm_fwd_vec_kernel<1>, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, 1e-5f, out); break;
-    case 2: GN_LAUNCH(ctx, layernorm_fwd_vec_kernel<2>, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, 1e-5f, out); break;
-    case 4: GN_LAUNCH(ctx, layernorm_fwd_vec_kernel<4>, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, 1e-5f, out); break;
-    case 8: GN_LAUNCH(ctx, layernorm_fwd_vec_kernel<8>, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, 1e-5f, out); break;
-    default: GN_LAUNCH(ctx, layernorm_fwd_kernel, cdiv(rows, 8), 256, 0, x, gamma, beta, y, mean, sd, rows, n, 1e-5f);
+// LayerNorm / RMSNorm: the row-in-registers kernels where the row length and the alignment allow it.  stat: [2][rows] mean | deviation, or [rows] rms.
+// `po` (optional): the output also as operand planes; *emitted tells the caller whether the kernel that ran could do it.
+static bool norm_vec_ok(int n, std::initializer_list<const void*> ptrs) {
+  uintptr_t a = 0; for (auto p : ptrs) a |= reinterpret_cast<uintptr_t>(p);
+  return n % 4 == 0 && n <= 1024 && (a & 15) == 0;
+}
+template <bool RMS, int NV> struct NormRun {
+  static void fwd(Ctx* ctx, const float* x, const float* ga, const float* be, float* y, float* sa, float* sb, long rows, int n, float eps, const RowPlaneOut& po) {
+    if ((n + 127) / 128 == NV) { GN_LAUNCH(ctx, (norm_fwd_vec_kernel<NV, RMS>), cdiv(rows, 8), 256, 0, x, ga, be, y, sa, sb, rows, n, eps, po); }
+    else if constexpr (NV > 1) NormRun<RMS, NV - 1>::fwd(ctx, x, ga, be, y, sa, sb, rows, n, eps, po);
   }
-  return check_launch("layernorm_forward");
+  static void bwd(Ctx* ctx, int blocks, const float* g, const float* x, const float* ga, const float* sa, const float* sb, float* dx, float* part, long rows, int n, const RowPlaneOut& po) {
+    if ((n + 127) / 128 == NV) { GN_LAUNCH(ctx, (norm_bwd_vec_kernel<NV, RMS>), blocks, 256, 0, g, x, ga, sa, sb, dx, part, rows, n, po); }
+    else if constexpr (NV > 1) NormRun<RMS, NV - 1>::bwd(ctx, blocks, g, x, ga, sa, sb, dx, part, rows, n, po);
+  }
+};
+static int norm_forward(Ctx* ctx, bool rms, const float* x, const float* gamma, const float* beta, float* y, float* stat, long rows, int n, float eps,
+                        const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
+  if (norm_vec_ok(n, {x, y, gamma, beta})) {
+    const RowPlaneOut out = po ? *po : RowPlaneOut{};
+    if (emitted) *emitted = out.p != nullptr;
+    if (rms) NormRun<true, 8>::fwd(ctx, x, gamma, beta, y, stat, stat, rows, n, eps, out);
+    else NormRun<false, 8>::fwd(ctx, x, gamma, beta, y, stat, stat + rows, rows, n, eps, out);
+  } else {
+    if (emitted) *emitted = false;
+    if (rms) GN_LAUNCH(ctx, rmsnorm_fwd_kernel, cdiv(rows, 8), 256, 0, x, gamma, y, stat, rows, n, eps);
+    else GN_LAUNCH(ctx, layernorm_fwd_kernel, cdiv(rows, 8), 256, 0, x, gamma, beta, y, stat, stat + rows, rows, n, eps);
+  }
+  return check_launch("norm_forward");
 }
-
-
-// The two norms of a TransformerBlock: LayerNorm (row mean and deviation in stat[0:rows], stat[rows:2 rows]) or RMSNorm
-// (row RMS in stat[0:rows]); rmsnorm.go:157-240, :246-336.
-static int block_norm_forward(Ctx* ctx, bool rms, const float* x, const float* gamma, const float* beta, float* y, float* stat, long rows, int n,
-                              const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
+// dx (may alias g), gGamma and gBeta (null for RMSNorm) are written.
+static int norm_backward(gn_model* m, bool rms, const float* g, const float* x, const float* gamma, const float* stat, float* dx, float* gGamma, float* gBeta, long rows, int n,
+                         const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
+  Ctx* ctx = &m->ctx->c; float* part;
+  if (norm_vec_ok(n, {g, x, dx, gamma})) {
+    const RowPlaneOut out = po ? *po : RowPlaneOut{};
+    if (emitted) *emitted = out.p != nullptr;
+    const int blocks = (int)std::max<long>(1, std::min<long>((rows + 7) / 8, (n <= 512 ? 2L : 1L) * ctx->sm_count));      // as many as are resident
+    GN_TRY(ensure(m, S_PART2, (size_t)blocks * 2 * n, &part));
+    if (rms) NormRun<true, 8>::bwd(ctx, blocks, g, x, gamma, stat, stat, dx, part, rows, n, out);
+    else NormRun<false, 8>::bwd(ctx, blocks, g, x, gamma, stat, stat + rows, dx, part, rows, n, out);
+    GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, blocks, n, gGamma, rms ? nullptr : gBeta);
+    return check_launch("norm_backward");
+  }
   if (emitted) *emitted = false;
-  if (!rms) return layernorm_forward(ctx, x, gamma, beta, y, stat, stat + rows, rows, n, po, emitted);
-  GN_LAUNCH(ctx, rmsnorm_fwd_kernel, cdiv(rows, 8), 256, 0, x, gamma, y, stat, rows, n, 1e-5f);
-  return check_launch("rmsnorm_forward");
-}
-static int layernorm_backward(gn_model* m, const float* g, const float* x, const float* gamma, const float* mean, const float* sd, float* dx,
-                              float* gGamma, float* gBeta, long rows, int n, const RowPlaneOut* po = nullptr, bool* emitted = nullptr);
-static int block_norm_backward(gn_model* m, bool rms, const float* g, const float* x, const float* gamma, const float* stat, float* dx, float* gGamma, float* gBeta, long rows, int n,
-                               const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
-  if (emitted) *emitted = false;
-  if (!rms) return layernorm_backward(m, g, x, gamma, stat, stat + rows, dx, gGamma, gBeta, rows, n, po, emitted);
-  Ctx* ctx = &m->ctx->c;
   const int chunks = (int)std::max<long>(1, std::min<long>(rows / 64, 128));
-  float* part; GN_TRY(ensure(m, S_PART2, (size_t)chunks * n, &part));
-  GN_LAUNCH(ctx, rmsnorm_pgrad_partial_kernel, dim3(cdiv(n, 128), chunks), 128, 0, g, x, stat, rows, n, part);
-  GN_LAUNCH(ctx, rmsnorm_pgrad_final_kernel, cdiv(n, 128), 128, 0, part, chunks, n, gGamma);
-  GN_LAUNCH(ctx, rmsnorm_bwd_kernel, cdiv(rows, 8), 256, 0, g, x, gamma, stat, dx, rows, n);
-  return check_launch("rmsnorm_backward");
+  GN_TRY(ensure(m, S_PART2, (size_t)chunks * 2 * n, &part));
+  if (rms) {
+    GN_LAUNCH(ctx, rmsnorm_pgrad_partial_kernel, dim3(cdiv(n, 128), chunks), 128, 0, g, x, stat, rows, n, part);
+    GN_LAUNCH(ctx, rmsnorm_pgrad_final_kernel, cdiv(n, 128), 128, 0, part, chunks, n, gGamma);
+    GN_LAUNCH(ctx, rmsnorm_bwd_kernel, cdiv(rows, 8), 256, 0, g, x, gamma, stat, dx, rows, n);
+  } else {
+    GN_LAUNCH(ctx, layernorm_pgrad_partial_kernel, dim3(cdiv(n, 128), chunks), 128, 0, g, x, stat, stat + rows, rows, n, part);
+    GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, chunks, n, gGamma, gBeta);
+    GN_LAUNCH(ctx, layernorm_bwd_kernel, cdiv(rows, 8), 256, 0, g, x, gamma, stat, stat + rows, dx, rows, n);
+  }
+  return check_launch("norm_backward");
 }
 // cos | sin of the rotary embedding per (position, pair index), with the reference's conversions (transformer.go:217-221):
 // theta and position * theta are rounded to float32, cos and sin taken in float64 and rounded to float32.
@@ -409,17 +456,24 @@ static int rope_table(Ctx* ctx, LayerRT& l) {
   GN_CUDA(copy_h2d(ctx, l.rope.p, tab.data(), tab.size() * 4)); return GN_OK;
 }
 
+// Rotation of one or two arrays of `rows` rows, T positions per sequence, in place
+static void rope(Ctx* ctx, const LayerRT& l, float* x, float* y, int rows, int T, float sign, int tstep) {
+  const int D = l.d.dim, hd = D / l.d.heads;
+  const bool vec = hd % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  if (vec) GN_LAUNCH(ctx, rope_kernel<4>, dim3(ew_grid(ctx, (long)rows * (D / 8)), y ? 2 : 1), 256, 0, x, y, (const float*)l.rope.p, (long)rows, T, D, hd, sign, tstep);
+  else GN_LAUNCH(ctx, rope_kernel<1>, dim3(ew_grid(ctx, (long)rows * (D / 2)), y ? 2 : 1), 256, 0, x, y, (const float*)l.rope.p, (long)rows, T, D, hd, sign, tstep);
+}
 // A LayerNorm of a block can hand its output to the next contraction as operand planes (RowPlaneOut) when that
 // contraction runs on the tensor-core engine; `slotp` / `sloti` receive the planes and the inverse row scales.
-static bool norm_planes_wanted(Ctx* ctx, bool rms, int rows, int n, int consumer_n) {
+static bool norm_planes_wanted(Ctx* ctx, int rows, int n, int consumer_n) {
   static const bool off = getenv("GONEURON_CUDA_NO_NORM_PLANES") != nullptr;
-  if (off || rms || force_simt_engine() || !layernorm_vec_width(n)) return false;
+  if (off || force_simt_engine() || n % 4 || n > 1024) return false;
   GemmDesc g; g.M = rows; g.N = consumer_n; g.K = n; g.sa_m = n; g.sa_k = 1; g.sb_k = 1; g.sb_n = n;
   return gemm_tc_eligible(ctx, g) && !gemm_outer_small_ok(g);
 }
 static int norm_planes_alloc(gn_model* m, int slotp, int sloti, int rows, int n, RowPlaneOut* po, BfPlanes* planes, float* rownorm) {
-  float *pp, *pi; GN_TRY(ensure(m, slotp, (size_t)rows * n, &pp)); GN_TRY(ensure(m, sloti, (size_t)rows, &pi));
-  *planes = BfPlanes{reinterpret_cast<__half*>(pp), pi, rows, n, n, 1};
+  float *pp, *pi; const int ldp = tc_ldp(n); GN_TRY(ensure(m, slotp, (size_t)rows * ldp, &pp)); GN_TRY(ensure(m, sloti, (size_t)rows, &pi));
+  *planes = BfPlanes{reinterpret_cast<__half*>(pp), pi, rows, n, ldp, 1};
   *po = RowPlaneOut{planes->base, pi, rownorm};
   return GN_OK;
 }
@@ -551,6 +605,22 @@ static int next_rows(const gn_model* m, size_t li, int T, int D) {
   return n.d.kind == GN_LAYER_TRANSFORMER_BLOCK && n.in_row0 && n.d.seq_len == T && n.d.dim == D ? 1 : 0;
 }
 
+// Rows that the SwiGLU kernels with plane output take
+static bool swiglu_planes_ok(const LayerRT& l) {
+  const int F = l.d.ff_dim;
+  return !force_simt_engine() && F % 32 == 0 && F <= 4096 && ((reinterpret_cast<uintptr_t>(l.gate.p) | reinterpret_cast<uintptr_t>(l.up.p)) & 15) == 0;
+}
+template <int NV> struct SwigluRun {
+  static void fwd(Ctx* ctx, const float* gate, const float* up, const BfPlanes& p, float* last, int T, int rows, int F) {
+    if ((F + 511) / 512 == NV) { GN_LAUNCH(ctx, swiglu_fwd_planes_kernel<NV>, rows, SW_THREADS, 0, gate, up, p.base, p.inv_scale, last, T, F); }
+    else if constexpr (NV > 1) SwigluRun<NV - 1>::fwd(ctx, gate, up, p, last, T, rows, F);
+  }
+  static void bwd(Ctx* ctx, const float* g, const float* gate, const float* up, float* dG, float* dU, const BfPlanes& p, int T, int rows, int F) {
+    if ((F + 511) / 512 == NV) { GN_LAUNCH(ctx, swiglu_bwd_planes_kernel<NV>, rows, SW_THREADS, 0, g, gate, up, dG, dU, p.base, p.inv_scale, T, F); }
+    else if constexpr (NV > 1) SwigluRun<NV - 1>::bwd(ctx, g, gate, up, dG, dU, p, T, rows, F);
+  }
+};
+
 static KeepRows keep_layout(const LayerRT& l, int B) {
   const long BD = (long)B * l.d.dim, BF = (long)B * l.d.ff_dim; float* p = l.keep.p;
   return KeepRows{p, p + BD, p + 2 * BD, p + 3 * BD, p + 4 * BD, p + 5 * BD, p + 5 * BD + BF, p + 5 * BD + 2 * BF, p + 5 * BD + 3 * BF};
@@ -572,20 +642,18 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
     // causal, token 0 only: it attends to itself alone, so its attention output is its value row
     GN_TRY(gemm_nt(ctx, B, D, D, xe, ldx, bp.wv, bp.bv, l.att.p, D));
   } else {
-    // the Q, K and V projections read the same input: its operand planes come from the LayerNorm that produced it
-    // (the previous block's), or are still in the engine's scratch after the first of the three
-    GemmDesc g; g.M = N; g.N = D; g.K = D; g.A = cur; g.sa_m = D; g.sa_k = 1; g.sb_k = 1; g.sb_n = D; g.ldc = D;
-    if (m->fwd_planes_src == cur && m->fwd_planes.rows == N && m->fwd_planes.K == D) g.a_planes = &m->fwd_planes;
-    if (!rows_only) { g.B = bp.wq; g.bias = bp.bq; g.C = l.q.p; GN_TRY(gemm(ctx, g)); g.reuse_a_planes = true; }
-    g.B = bp.wk; g.bias = bp.bk; g.C = l.k.p; GN_TRY(gemm(ctx, g));
-    g.reuse_a_planes = true;
-    g.B = bp.wv; g.bias = bp.bv; g.C = l.v.p; GN_TRY(gemm(ctx, g));
-    if (rows_only) GN_TRY(gemm_nt(ctx, NE, D, D, xe, ldx, bp.wq, bp.bq, l.q.p, D));
+    // the operand planes of the projections' input come from the norm that produced it (the previous block's) if it made any
+    const BfPlanes* xp = m->fwd_planes_src == cur && m->fwd_planes.rows == N && m->fwd_planes.K == D ? &m->fwd_planes : nullptr;
+    const long dd = (long)D * D + D;
+    if (!rows_only) GN_TRY(gemm_nt_stack(ctx, 3, N, D, D, cur, D, bp.wq, dd, bp.bq, l.q.p, l.k.p - l.q.p, xp));
+    else {
+      GN_TRY(gemm_nt_stack(ctx, 2, N, D, D, cur, D, bp.wk, dd, bp.bk, l.k.p, l.k.p - l.q.p, xp));
+      GN_TRY(gemm_nt(ctx, NE, D, D, xe, ldx, bp.wq, bp.bq, l.q.p, D));
+    }
     if (l.use_rope) {   // rotary embeddings on q and k, in place: attention and its backward pass see the rotated tensors (transformer.go:457-461)
       GN_TRY(rope_table(ctx, l));
-      const long tot = (long)N * (D / 2), tq = (long)NE * (D / 2);
-      GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tq), 256, 0, l.q.p, (const float*)l.rope.p, (long)NE, TE, D, hd, 1.f, rows_only ? T - 1 : 1);
-      GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, l.k.p, (const float*)l.rope.p, (long)N, T, D, hd, 1.f, 1);
+      rope(ctx, l, l.q.p, rows_only ? nullptr : l.k.p, NE, TE, 1.f, rows_only ? T - 1 : 1);
+      if (rows_only) rope(ctx, l, l.k.p, nullptr, N, T, 1.f, 1);
     }
     if (rows_only) GN_TRY(attn_rows_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, B, T, TE, D, d.heads, d.causal));
     else if (use_fused_attention(d)) {
@@ -602,8 +670,8 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
   float* st = l.stat.p;
   // norm 1 hands its output to ff1 as operand planes (and the row norms ff1's plane-writing epilogue needs)
   RowPlaneOut po1{}; BfPlanes n1p{}; bool n1_planes = false; float* rn1 = nullptr;
-  if (norm_planes_wanted(ctx, l.rms, NE, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)NE, &rn1)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, NE, D, &po1, &n1p, rn1)); }
-  GN_TRY(block_norm_forward(ctx, l.rms, l.r1.p, bp.g1, bp.be1, l.n1.p, st, (long)NE, D, po1.p ? &po1 : nullptr, &n1_planes));
+  if (norm_planes_wanted(ctx, NE, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)NE, &rn1)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, NE, D, &po1, &n1p, rn1)); }
+  GN_TRY(norm_forward(ctx, l.rms, l.r1.p, bp.g1, bp.be1, l.n1.p, st, (long)NE, D, 1e-5f, po1.p ? &po1 : nullptr, &n1_planes));
   {   // feed-forward: ff1 -> ff2, res2 = norm1 + ff
     GemmDesc g1; g1.M = NE; g1.N = F; g1.K = D; g1.A = l.n1.p; g1.sa_m = D; g1.sa_k = 1; g1.B = bp.w1; g1.sb_k = 1; g1.sb_n = D; g1.C = l.mid.p; g1.ldc = F; g1.bias = bp.b1;
     if (n1_planes) g1.a_planes = &n1p;
@@ -613,20 +681,22 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
     if (l.mid_is_planes) {
       // the hidden activation is only ever the A operand of ff2 (and, for its last-token rows, a gate and a weight-gradient
       // input): the epilogue writes it as operand planes into the same buffer, no fp32 copy and no split pass
-      const WeightPlaneEntry* we = nullptr; wplanes_lookup(ctx, g1, &we);
+      const WeightPlaneEntry* we = nullptr; BfPlanes w; wplanes_lookup(ctx, g1, &w, &we);
       float* rn; GN_TRY(ensure(m, S_RN, (size_t)NE, &rn));
-      TcPlaneOut po{midp, we->maxabs, l.mid_last.p, TE};
-      g1.act = GN_ACT_RELU; g1.C = nullptr; g1.plane_out = &po; g1.a_rownorm = rn; GN_TRY(gemm(ctx, g1));
+      TcPlaneOut po{midp, we->maxabs, l.mid_last.p, TE}; po.z_last = training && l.ff_act == GN_ACT_GELU ? l.zlast.p : nullptr;
+      g1.act = l.ff_act; g1.C = nullptr; g1.plane_out = &po; g1.a_rownorm = rn; GN_TRY(gemm(ctx, g1));
     } else if (l.ff_act == GN_ACT_RELU) { g1.act = GN_ACT_RELU; GN_TRY(gemm(ctx, g1)); }
     else if (l.ff_act == GN_ACT_GELU) {
       // the pre-activation of every sequence's last token is what the backward pass differentiates at (layer.go:563-567)
       GN_TRY(gemm(ctx, g1));
       if (training) GN_LAUNCH(ctx, last_token_rows_kernel, ew_grid(ctx, (long)B * F), 256, 0, (const float*)l.mid.p, l.zlast.p, TE, F, (long)B * F);
       GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.mid.p, l.mid.p, nf, (int)GN_ACT_GELU, 0.f);
-    } else {              // SwiGLU: gate and up projections (no biases) share the input's operand planes
-      g1.C = l.gate.p; g1.bias = nullptr; GN_TRY(gemm(ctx, g1));
-      g1.B = bp.v1; g1.C = l.up.p; g1.reuse_a_planes = true; GN_TRY(gemm(ctx, g1));
-      GN_LAUNCH(ctx, swiglu_fwd_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.gate.p, (const float*)l.up.p, l.mid.p, nf);
+    } else {              // SwiGLU: gate and up projections (no biases)
+      GN_TRY(gemm_nt_stack(ctx, 2, NE, F, D, l.n1.p, D, bp.w1, (long)F * D, nullptr, l.gate.p, l.up.p - l.gate.p, n1_planes ? &n1p : nullptr));
+      GemmDesc c; c.M = NE; c.N = D; c.K = F; c.B = bp.w2; c.sb_k = 1; c.sb_n = F; c.sa_k = 1; c.sa_m = F;
+      l.mid_is_planes = swiglu_planes_ok(l) && gemm_on_tc(ctx, c);
+      if (l.mid_is_planes) SwigluRun<8>::fwd(ctx, l.gate.p, l.up.p, midp, l.mid_last.p, TE, NE, F);
+      else GN_LAUNCH(ctx, swiglu_fwd_kernel, ew_grid(ctx, nf), 256, 0, (const float*)l.gate.p, (const float*)l.up.p, l.mid.p, nf);
     }
     GemmDesc g2; g2.M = NE; g2.N = D; g2.K = F; g2.A = l.mid.p; g2.sa_m = F; g2.sa_k = 1; g2.B = bp.w2; g2.sb_k = 1; g2.sb_n = F; g2.C = l.r2.p; g2.ldc = D; g2.bias = bp.b2; g2.R = l.n1.p; g2.ldr = D;
     if (l.mid_is_planes) g2.a_planes = &midp;
@@ -635,8 +705,8 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
   {   // norm 2 hands its output to the next block's projections as operand planes
     RowPlaneOut po2{}; BfPlanes outp{}; bool emitted = false;
     const bool next_is_block = !rows_only && li + 1 < m->L.size() && m->L[li + 1].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[li + 1].d.dim == D && m->L[li + 1].d.seq_len == T;
-    if (next_is_block && norm_planes_wanted(ctx, l.rms, NE, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP1, S_LNI1, NE, D, &po2, &outp, nullptr));
-    GN_TRY(block_norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * NE, (long)NE, D, po2.p ? &po2 : nullptr, &emitted));
+    if (next_is_block && norm_planes_wanted(ctx, NE, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP1, S_LNI1, NE, D, &po2, &outp, nullptr));
+    GN_TRY(norm_forward(ctx, l.rms, l.r2.p, bp.g2, bp.be2, l.out.p, st + 2 * NE, (long)NE, D, 1e-5f, po2.p ? &po2 : nullptr, &emitted));
     if (emitted) { m->fwd_planes = outp; m->fwd_planes_src = l.out.p; }
   }
   l.kept = training && l.keep.n != 0;
@@ -762,11 +832,11 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
         cur = l.out.p; break; }
       case GN_LAYER_LAYERNORM: {
         long rows = (long)B * (l.in_size / d.dim);
-        GN_TRY(layernorm_forward(ctx, cur, p, p + d.dim, l.out.p, l.stat.p, l.stat.p + rows, rows, d.dim));
+        GN_TRY(norm_forward(ctx, false, cur, p, p + d.dim, l.out.p, l.stat.p, rows, d.dim, 1e-5f));
         cur = l.out.p; break; }
       case GN_LAYER_RMSNORM: {
         long rows = (long)B * (l.in_size / d.dim);
-        GN_LAUNCH(ctx, rmsnorm_fwd_kernel, cdiv(rows, 8), 256, 0, cur, p, l.out.p, l.stat.p, rows, d.dim, l.bn_eps);
+        GN_TRY(norm_forward(ctx, true, cur, p, nullptr, l.out.p, l.stat.p, rows, d.dim, l.bn_eps));
         cur = l.out.p; break; }
     }
     GN_TRY(check_launch("forward"));
@@ -774,49 +844,34 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
   *y_out = cur; return GN_OK;
 }
 
-// LayerNorm backward: dx, and gGamma / gBeta accumulated into the gradient slice.
-static int layernorm_backward(gn_model* m, const float* g, const float* x, const float* gamma, const float* mean, const float* sd, float* dx,
-                              float* gGamma, float* gBeta, long rows, int n, const RowPlaneOut* po, bool* emitted) {
-  Ctx* ctx = &m->ctx->c;
-  const bool vec = n % 128 == 0 && ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
-  const RowPlaneOut out = (po && vec && layernorm_vec_width(n)) ? *po : RowPlaneOut{};
-  if (emitted) *emitted = out.p != nullptr;
-  if (vec) {
-    const int chunks = (int)std::max<long>(1, std::min<long>(rows / 32, 4L * ctx->sm_count));
-    float* part; GN_TRY(ensure(m, S_PART2, (size_t)chunks * 2 * n, &part));
-    GN_LAUNCH(ctx, layernorm_pgrad_partial_vec_kernel, dim3(cdiv(n, 1024), chunks), 256, 0, g, x, mean, sd, rows, n, part);
-    GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, chunks, n, gGamma, gBeta);
-  } else {
-    const int chunks = (int)std::max<long>(1, std::min<long>(rows / 64, 128));
-    float* part; GN_TRY(ensure(m, S_PART2, (size_t)chunks * 2 * n, &part));
-    GN_LAUNCH(ctx, layernorm_pgrad_partial_kernel, dim3(cdiv(n, 128), chunks), 128, 0, g, x, mean, sd, rows, n, part);
-    GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, chunks, n, gGamma, gBeta);
-  }
-  switch (vec ? n / 128 : 0) {
-    case 1: GN_LAUNCH(ctx, layernorm_bwd_vec_kernel<1>, cdiv(rows, 8), 256, 0, g, x, gamma, mean, sd, dx, rows, out); break;
-    case 2: GN_LAUNCH(ctx, layernorm_bwd_vec_kernel<2>, cdiv(rows, 8), 256, 0, g, x, gamma, mean, sd, dx, rows, out); break;
-    case 4: GN_LAUNCH(ctx, layernorm_bwd_vec_kernel<4>, cdiv(rows, 8), 256, 0, g, x, gamma, mean, sd, dx, rows, out); break;
-    case 8: GN_LAUNCH(ctx, layernorm_bwd_vec_kernel<8>, cdiv(rows, 8), 256, 0, g, x, gamma, mean, sd, dx, rows, out); break;
-    default: GN_LAUNCH(ctx, layernorm_bwd_kernel, cdiv(rows, 8), 256, 0, g, x, gamma, mean, sd, dx, rows, n);
-  }
-  return check_launch("layernorm_backward");
-}
-
 // ---------------------------------------------------------------- backward
 // Gradient of one inner Dense of a TransformerBlock at batch level:
 //   gb = sum over all tokens of dz ; gW = Delta^T * X_last with Delta[s] = sum_t dz[s,t], X_last[s] = x[s,T-1]
 // `x_last` != null: the last-token inputs as a dense [B, in] array instead of a strided view of x; `dz_planes` != null: dz
 // exists only as operand planes.
-static int inner_dense_param_grads(gn_model* m, const float* dz, int B, int T, int out, const float* x, int in, float* gW, float* gb,
-                                   const float* x_last = nullptr, const BfPlanes* dz_planes = nullptr, const float* dz_rowsum32 = nullptr) {
-  Ctx* ctx = &m->ctx->c; float* delta; GN_TRY(ensure(m, S_DELTA, (size_t)B * out, &delta));
-  if (dz_rowsum32) GN_LAUNCH(ctx, token_sum_part32_kernel, dim3(cdiv(out, 512), B), 128, 0, dz_rowsum32, T / 32, out, delta);
-  else if (dz_planes) GN_LAUNCH(ctx, token_sum_planes_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, (const __half*)dz_planes->base, (const float*)dz_planes->inv_scale, (long)dz_planes->ldp, T, out, delta);
-  else if (out % 4 == 0 && ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(delta)) & 15) == 0)
+// `stack` > 1: several layers with the same input, whose dz (and, `ws` apart, whose weight gradients) follow one another.
+static int token_sums(Ctx* ctx, const float* dz, int B, int T, int out, float* delta) {
+  if (out % 4 == 0 && ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(delta)) & 15) == 0)
     GN_LAUNCH(ctx, token_sum_vec_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, dz, T, out, delta);
   else GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(out, 128), B), dim3(128, 4), 0, dz, T, out, delta);
-  if (x_last) return weight_bias_grads(m, ctx, B, out, in, delta, out, x_last, (long)in, gW, gb);
-  return weight_bias_grads(m, ctx, B, out, in, delta, out, x + (long)(T - 1) * in, (long)T * in, gW, gb);
+  return check_launch("token_sums");
+}
+static int weight_bias_grads_stack(gn_model* m, int stack, int B, int out, int in, const float* delta, const float* x_last, long ldx, float* gW, float* gb, long ws) {
+  Ctx* ctx = &m->ctx->c;
+  GemmDesc g; g.M = out; g.N = in; g.K = B; g.A = delta; g.sa_m = 1; g.sa_k = out; g.B = x_last; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = in;
+  g.batch1 = stack; g.a_b1 = (long)B * out; g.c_b1 = ws; g.a_sum = gb;
+  if (gemm_outer_small_ok(g)) return gemm(ctx, g);
+  for (int j = 0; j < stack; j++) GN_TRY(weight_bias_grads(m, ctx, B, out, in, delta + (long)j * B * out, out, x_last, ldx, gW + j * ws, gb + j * ws));
+  return GN_OK;
+}
+static int inner_dense_param_grads(gn_model* m, const float* dz, int B, int T, int out, const float* x, int in, float* gW, float* gb,
+                                   const float* x_last = nullptr, const BfPlanes* dz_planes = nullptr, const float* dz_rowsum32 = nullptr, int stack = 1, long ws = 0) {
+  Ctx* ctx = &m->ctx->c; float* delta; GN_TRY(ensure(m, S_DELTA, (size_t)stack * B * out, &delta));
+  if (dz_rowsum32) GN_LAUNCH(ctx, token_sum_part32_kernel, dim3(cdiv(out, 512), B), 128, 0, dz_rowsum32, T / 32, out, delta);
+  else if (dz_planes) GN_LAUNCH(ctx, token_sum_planes_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, (const __half*)dz_planes->base, (const float*)dz_planes->inv_scale, (long)dz_planes->ldp, T, out, delta);
+  else GN_TRY(token_sums(ctx, dz, stack * B, T, out, delta));
+  return x_last ? weight_bias_grads_stack(m, stack, B, out, in, delta, x_last, (long)in, gW, gb, ws)
+                : weight_bias_grads_stack(m, stack, B, out, in, delta, x + (long)(T - 1) * in, (long)T * in, gW, gb, ws);
 }
 // Can the FFN's hidden activation (and its gradient) of this block live as operand planes only?  The two contractions on
 // either side must both run on the tensor-core engine with prepared weight planes, and the plane-writing epilogue's shape
@@ -824,13 +879,13 @@ static int inner_dense_param_grads(gn_model* m, const float* dz, int B, int T, i
 static bool ffn_planes_possible(Ctx* ctx, const LayerRT& l, int N, const float* w1, const float* w2) {
   static const bool off = getenv("GONEURON_CUDA_NO_PLANE_OUTPUT") != nullptr;
   const gn_layer_desc& d = l.d; const int D = d.dim, F = d.ff_dim;
-  if (off || force_simt_engine() || l.ff_act != GN_ACT_RELU || F % 32 || D % 32 || D > 2048 || F % 4) return false;
+  if (off || force_simt_engine() || (l.ff_act != GN_ACT_RELU && l.ff_act != GN_ACT_GELU) || F % 32 || D % 32 || D > 2048 || F % 4) return false;
   if ((reinterpret_cast<uintptr_t>(w1 + (long)D * F) & 15) != 0) return false;                                 // ff1's bias is read with 16-byte loads
-  GemmDesc a; a.M = N; a.N = F; a.K = D; a.B = w1; a.sb_k = 1; a.sb_n = D; a.sa_k = 1; a.sa_m = D;            // n1 W1^T        -> planes
+  BfPlanes w; GemmDesc a; a.M = N; a.N = F; a.K = D; a.B = w1; a.sb_k = 1; a.sb_n = D; a.sa_k = 1; a.sa_m = D;            // n1 W1^T        -> planes
   GemmDesc b; b.M = N; b.N = F; b.K = D; b.B = w2; b.sb_k = F; b.sb_n = 1; b.sa_k = 1; b.sa_m = D;            // dR2 W2         -> planes
   GemmDesc c; c.M = N; c.N = D; c.K = F; c.B = w2; c.sb_k = 1; c.sb_n = F; c.sa_k = 1; c.sa_m = F;            // planes W2^T    (consumer, forward)
   GemmDesc e; e.M = N; e.N = D; e.K = F; e.B = w1; e.sb_k = D; e.sb_n = 1; e.sa_k = 1; e.sa_m = F;            // planes W1      (consumer, backward)
-  return gemm_tc_eligible(ctx, a) && gemm_tc_eligible(ctx, b) && gemm_tc_eligible(ctx, c) && gemm_tc_eligible(ctx, e) && wplanes_lookup(ctx, a) && wplanes_lookup(ctx, b);
+  return gemm_tc_eligible(ctx, a) && gemm_tc_eligible(ctx, b) && gemm_tc_eligible(ctx, c) && gemm_tc_eligible(ctx, e) && wplanes_lookup(ctx, a, &w) && wplanes_lookup(ctx, b, &w);
 }
 
 static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, const float* gout, float* dx) {
@@ -845,23 +900,30 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   // norm 2
   // its result goes to the contraction with W2 as operand planes, with the row norms that contraction's plane-writing epilogue needs
   RowPlaneOut pob{}; BfPlanes dR2p{}; bool dR2_planes = false; float* rnb = nullptr;
-  if (norm_planes_wanted(ctx, l.rms, N, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)N, &rnb)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &pob, &dR2p, rnb)); }
-  GN_TRY(block_norm_backward(m, l.rms, gout, l.r2.p, bp.g2, st + 2 * N, dR2, (float*)gp.g2, (float*)gp.be2, (long)N, D, pob.p ? &pob : nullptr, &dR2_planes));
+  if (norm_planes_wanted(ctx, N, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)N, &rnb)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &pob, &dR2p, rnb)); }
+  GN_TRY(norm_backward(m, l.rms, gout, l.r2.p, bp.g2, st + 2 * N, dR2, (float*)gp.g2, (float*)gp.be2, (long)N, D, pob.p ? &pob : nullptr, &dR2_planes));
   // ff2 then ff1, token by token in the reference (transformer.go:1238-1250)
   GN_TRY(inner_dense_param_grads(m, dR2, B, T, D, l.mid.p, F, (float*)gp.w2, (float*)gp.b2, l.mid_is_planes ? l.mid_last.p : nullptr));
   {
     // dM[s,t,:] = W2^T dR2[s,t,:]; with a ReLU first layer gated by the ReLU pattern of the LAST token of sequence s (fused into the epilogue)
     GemmDesc g; g.M = N; g.N = F; g.K = D; g.A = dR2; g.sa_m = D; g.sa_k = 1; g.B = bp.w2; g.sb_k = F; g.sb_n = 1; g.C = dM; g.ldc = F;
     if (dR2_planes) g.a_planes = &dR2p;
-    if (l.mid_is_planes) { g.mask = l.mid_last.p; g.mask_ld = F; g.mask_group = T; }
+    const bool ffn_planes = l.mid_is_planes && l.ff_act != GN_ACT_SILU;
+    if (ffn_planes) {
+      g.mask = l.mid_last.p; g.mask_ld = F; g.mask_group = T;
+      if (l.ff_act == GN_ACT_GELU) {      // GELU'(z) of the last token multiplies every token's gradient (layer.go:563-567): factors instead of a gate
+        float* der; GN_TRY(ensure(m, S_NFF2, (size_t)B * F, &der));
+        GN_LAUNCH(ctx, act_deriv_kernel, ew_grid(ctx, (long)B * F), 256, 0, (const float*)l.zlast.p, der, (long)B * F, (int)GN_ACT_GELU); g.mask = der;
+      }
+    }
     else if (l.ff_act == GN_ACT_RELU) { g.mask = l.mid.p + (long)(T - 1) * F; g.mask_ld = (long)T * F; g.mask_group = T; }
     const long nf = (long)N * F;
-    if (l.mid_is_planes) {
+    if (ffn_planes) {
       // the gradient of the hidden activation likewise only feeds a token sum and the next contraction: planes only
-      const WeightPlaneEntry* we = nullptr; wplanes_lookup(ctx, g, &we);
+      const WeightPlaneEntry* we = nullptr; BfPlanes w; wplanes_lookup(ctx, g, &w, &we);
       float *rn, *dinv; GN_TRY(ensure(m, S_RN, (size_t)N, &rn)); GN_TRY(ensure(m, S_NFFI, (size_t)N, &dinv));
       BfPlanes dMp{reinterpret_cast<__half*>(dM), dinv, N, F, F, 1};
-      TcPlaneOut po{dMp, we->maxabs, nullptr, 1};
+      TcPlaneOut po{dMp, we->maxabs, nullptr, 1}; po.scale = l.ff_act == GN_ACT_GELU;
       float* rs32 = nullptr;                               // 32-row sums of dM from the epilogue: the token sums of the ff1 weight gradient
       if (T % 32 == 0 && F % 4 == 0) { GN_TRY(ensure(m, S_RS32, (size_t)(N / 32) * F, &rs32)); po.rowsum32 = rs32; }
       g.C = nullptr; g.plane_out = &po; g.a_rownorm = rn; GN_TRY(gemm(ctx, g));
@@ -881,19 +943,26 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
       // over all tokens with the layer's inputs; the input gradient comes out in partner order and is reversed when it is
       // added to the residual path.
       float *dGP, *dUP, *Y;
-      GN_TRY(ensure(m, S_NFF2, (size_t)nf, &dGP)); GN_TRY(ensure(m, S_NFF3, (size_t)nf, &dUP)); GN_TRY(ensure(m, S_ND3, ND, &Y));
-      GN_LAUNCH(ctx, swiglu_bwd_paired_kernel, ew_grid(ctx, nf), 256, 0, (const float*)dM, (const float*)l.gate.p, (const float*)l.up.p, dGP, dUP, T, F, nf);
-      GN_TRY(gemm_tn(ctx, N, F, D, dGP, F, l.n1.p, D, (float*)gp.w1));
-      GN_TRY(gemm_tn(ctx, N, F, D, dUP, F, l.n1.p, D, (float*)gp.v1));
-      GN_TRY(gemm_nn(ctx, N, F, D, dGP, F, bp.w1, Y, D));
-      GN_TRY(gemm_nn(ctx, N, F, D, dUP, F, bp.v1, Y, D, Y, D));
+      GN_TRY(ensure(m, S_NFF2, (size_t)2 * nf, &dGP)); dUP = dGP + nf; GN_TRY(ensure(m, S_ND3, ND, &Y));
+      BfPlanes dp{}; bool planes = false;
+      if (swiglu_planes_ok(l)) {
+        GemmDesc q; q.M = N; q.N = D; q.K = 2 * F; q.B = bp.w1; q.sb_k = D; q.sb_n = 1; q.sa_k = 1; q.sa_m = F; BfPlanes w;
+        planes = gemm_on_tc(ctx, q) && wplanes_lookup(ctx, q, &w);
+      }
+      if (planes) {
+        float *pp, *pi; GN_TRY(ensure(m, S_NFF3, (size_t)2 * nf, &pp)); GN_TRY(ensure(m, S_NFFI, (size_t)N, &pi));
+        dp = BfPlanes{reinterpret_cast<__half*>(pp), pi, N, 2 * F, 2 * F, 1};
+        SwigluRun<8>::bwd(ctx, dM, l.gate.p, l.up.p, dGP, dUP, dp, T, N, F);
+      } else GN_LAUNCH(ctx, swiglu_bwd_paired_kernel, ew_grid(ctx, nf), 256, 0, (const float*)dM, (const float*)l.gate.p, (const float*)l.up.p, dGP, dUP, T, F, nf);
+      GN_TRY(gemm_tn_stack(ctx, 2, N, F, D, dGP, nf, l.n1.p, D, (float*)gp.w1));
+      GN_TRY(gemm_nn_stack(ctx, 2, N, F, D, dGP, nf, bp.w1, (long)F * D, Y, nullptr, planes ? &dp : nullptr));
       GN_LAUNCH(ctx, add_token_reversed_kernel, ew_grid(ctx, ND), 256, 0, (const float*)dR2, (const float*)Y, comb, T, D, ND);
     }
   }
   // norm 1
   RowPlaneOut poa{}; BfPlanes dR1p{}; bool dR1_planes = false;
-  if (norm_planes_wanted(ctx, l.rms, N, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &poa, &dR1p, nullptr));      // the planes of dR2 are dead by now
-  GN_TRY(block_norm_backward(m, l.rms, comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, (long)N, D, poa.p ? &poa : nullptr, &dR1_planes));
+  if (norm_planes_wanted(ctx, N, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &poa, &dR1p, nullptr));      // the planes of dR2 are dead by now
+  GN_TRY(norm_backward(m, l.rms, comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, (long)N, D, poa.p ? &poa : nullptr, &dR1_planes));
   // output projection
   GN_TRY(inner_dense_param_grads(m, dR1, B, T, D, l.att.p, D, (float*)gp.wo, (float*)gp.bo));
   {
@@ -902,8 +971,7 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
     GN_TRY(gemm(ctx, g));
   }
   // attention: recompute P (transformer.go:610-622), then dP, dS, dQ, dK, dV
-  float *dQ, *dK, *dV;
-  GN_TRY(ensure(m, S_ND0, ND, &dQ)); GN_TRY(ensure(m, S_ND1, ND, &dK)); GN_TRY(ensure(m, S_ND4, ND, &dV));   // dR2 / comb are dead by now
+  float *dQ; GN_TRY(ensure(m, S_ND4, 3 * ND, &dQ)); float *dK = dQ + ND, *dV = dK + ND;
   if (fused) {
     static const bool tc_bwd = [] { const char* e = getenv("GONEURON_CUDA_ATTENTION_BWD"); return !(e && !strcmp(e, "mma")); }();
     if (tc_bwd && attn_tc_supported(ctx, hd, T, B, Hh, D)) GN_TRY(attn_tc_bwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, dA, l.att_m.p, l.att_l.p, l.att_d.p, dQ, dK, dV, B, T, D, Hh, d.causal, &l.attn_saved));
@@ -923,17 +991,11 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
     q.A = P; q.B = dA; q.C = dV; GN_TRY(gemm(ctx, q));                                                                          // dV = P^T dA
   }
   if (l.use_rope) {   // the conjugate rotation on the gradients of q and k (transformer.go:659-663)
-    const long tot = (long)N * (D / 2);
-    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, dQ, (const float*)l.rope.p, (long)N, T, D, hd, -1.f, 1);
-    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, tot), 256, 0, dK, (const float*)l.rope.p, (long)N, T, D, hd, -1.f, 1);
+    rope(ctx, l, dQ, dK, N, T, -1.f, 1);
   }
   // q, k, v projections; gradIn = dq + dk + dv, block input gradient = gradRes1 + gradIn
-  GN_TRY(inner_dense_param_grads(m, dQ, B, T, D, xin, D, (float*)gp.wq, (float*)gp.bq));
-  GN_TRY(inner_dense_param_grads(m, dK, B, T, D, xin, D, (float*)gp.wk, (float*)gp.bk));
-  GN_TRY(inner_dense_param_grads(m, dV, B, T, D, xin, D, (float*)gp.wv, (float*)gp.bv));
-  GN_TRY(gemm_nn(ctx, N, D, D, dQ, D, bp.wq, dx, D, dR1, D));
-  GN_TRY(gemm_nn(ctx, N, D, D, dK, D, bp.wk, dx, D, dx, D));
-  GN_TRY(gemm_nn(ctx, N, D, D, dV, D, bp.wv, dx, D, dx, D));
+  GN_TRY(inner_dense_param_grads(m, dQ, B, T, D, xin, D, (float*)gp.wq, (float*)gp.bq, nullptr, nullptr, nullptr, 3, (long)D * D + D));
+  GN_TRY(gemm_nn_stack(ctx, 3, N, D, D, dQ, ND, bp.wq, (long)D * D + D, dx, dR1));
   return check_launch("block_backward");
 }
 
@@ -953,7 +1015,7 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
   const float* gate_last = last(l.gate, kr.gate, F); const float* up_last = last(l.up, kr.up, F);
   const float* mid_last = l.mid_is_planes ? l.mid_last.p : last(l.mid, kr.mid, F); const long ld_mid = l.mid_is_planes ? F : ldF;
   float *dR2, *dR1, *comb, *dA, *dM;
-  GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, d.causal ? BD : ND, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
+  GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, BD, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
   auto norm = [&](const float* g, const float* x, const float* gamma, const float* stat, float* out, float* gG, float* gB) -> int {
     GN_LAUNCH(ctx, norm_bwd_rows_kernel, cdiv(B, 4), 128, 0, g, x, ldD, gamma, stat, l.rms ? nullptr : stat + NE, (long)TR, out, B, D);
     GN_LAUNCH(ctx, norm_pgrad_rows_kernel, cdiv(D, 32), 256, 0, g, x, ldD, stat, l.rms ? nullptr : stat + NE, (long)TR, B, D, gG, gB);
@@ -987,18 +1049,15 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
     *dx_row0 = true; return check_launch("block_backward_row0");
   }
   float *dQ, *dK, *dV, *ks, *vs;
-  GN_TRY(ensure(m, S_XROWS, 3 * BD, &dQ)); ks = dQ + BD; vs = ks + BD; GN_TRY(ensure(m, S_ND1, ND, &dK)); GN_TRY(ensure(m, S_ND4, ND, &dV));
+  GN_TRY(ensure(m, S_XROWS, 3 * BD, &dQ)); ks = dQ + BD; vs = ks + BD; GN_TRY(ensure(m, S_ND4, 2 * ND, &dK)); dV = dK + ND;
   GN_TRY(attn_rows_bwd(ctx, l.q.p, (long)TE * D, l.k.p, l.v.p, dA, dQ, dK, dV, ks, vs, B, T, D, d.heads));
   if (l.use_rope) {   // the conjugate rotation (transformer.go:659-663); token 0's angle is zero
-    GN_LAUNCH(ctx, rope_kernel, ew_grid(ctx, ND / 2), 256, 0, dK, (const float*)l.rope.p, (long)B * T, T, D, D / d.heads, -1.f, 1);
+    rope(ctx, l, dK, nullptr, B * T, T, -1.f, 1);
     GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(D, 128), B), dim3(128, 4), 0, (const float*)dK, T, D, ks);
   }
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, dQ, D, x_last, ldX, (float*)gp.wq, (float*)gp.bq));
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, ks, D, x_last, ldX, (float*)gp.wk, (float*)gp.bk));
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, vs, D, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
+  GN_TRY(weight_bias_grads_stack(m, 3, B, D, D, dQ, x_last, ldX, (float*)gp.wq, (float*)gp.bq, (long)D * D + D));      // dQ | sum of dK | sum of dV
   GN_TRY(gemm_nn(ctx, B, D, D, dQ, D, bp.wq, dR1, D, dR1, D));
-  GN_TRY(gemm_nn(ctx, B * T, D, D, dK, D, bp.wk, dx, D));
-  GN_TRY(gemm_nn(ctx, B * T, D, D, dV, D, bp.wv, dx, D, dx, D));
+  GN_TRY(gemm_nn_stack(ctx, 2, B * T, D, D, dK, ND, bp.wk, (long)D * D + D, dx, nullptr));
   GN_LAUNCH(ctx, add_row0_kernel, B, 128, 0, (const float*)dR1, dx, T, D);
   *dx_row0 = false; return check_launch("block_backward_row0");
 }
@@ -1253,15 +1312,11 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         g = dx; flip ^= 1; break; }
       case GN_LAYER_LAYERNORM: {
         long rows = (long)B * (l.in_size / d.dim);
-        GN_TRY(layernorm_backward(m, g, xin, p, l.stat.p, l.stat.p + rows, dx, gr, gr + d.dim, rows, d.dim));
+        GN_TRY(norm_backward(m, false, g, xin, p, l.stat.p, dx, gr, gr + d.dim, rows, d.dim));
         g = dx; flip ^= 1; break; }
       case GN_LAYER_RMSNORM: {
         long rows = (long)B * (l.in_size / d.dim);
-        const int chunks = (int)std::max<long>(1, std::min<long>(rows / 64, 128));
-        float* part; GN_TRY(ensure(m, S_PART2, (size_t)chunks * d.dim, &part));
-        GN_LAUNCH(ctx, rmsnorm_pgrad_partial_kernel, dim3(cdiv(d.dim, 128), chunks), 128, 0, g, xin, (const float*)l.stat.p, rows, d.dim, part);
-        GN_LAUNCH(ctx, rmsnorm_pgrad_final_kernel, cdiv(d.dim, 128), 128, 0, part, chunks, d.dim, gr);
-        if (need_dx) { GN_LAUNCH(ctx, rmsnorm_bwd_kernel, cdiv(rows, 8), 256, 0, g, xin, p, (const float*)l.stat.p, dx, rows, d.dim); g = dx; flip ^= 1; }
+        GN_TRY(norm_backward(m, true, g, xin, p, l.stat.p, dx, gr, nullptr, rows, d.dim)); g = dx; flip ^= 1;
         break; }
     }
     GN_TRY(check_launch("backward"));
@@ -1651,18 +1706,23 @@ int gn_model_create(gn_ctx* ctx, const gn_layer_desc* layers, int n_layers, int 
   if (ctx->c.tc_ok && !force_simt_engine() && !getenv("GONEURON_CUDA_NO_WEIGHT_PLANES")) {
     // weight matrices large enough to run on the tensor-core engine get prepared operand planes (both orientations)
     std::vector<WeightPlaneEntry> mats; int cur_layer = 0;
-    auto add = [&](int64_t off, int out, int in, bool has_bias = true) {
+    auto add = [&](int64_t off, int out, int in, bool has_bias = true, int parts = 1, int64_t stride = 0) {      // (a stack's parts: multiples of 32 rows)
       if ((double)out * in < 64.0 * 64.0) return;
-      WeightPlaneEntry e{m->params.p + off, out, in, {}, {}}; e.bias = has_bias ? m->params.p + off + (int64_t)out * in : nullptr; e.layer = cur_layer; mats.push_back(e);
+      WeightPlaneEntry e{m->params.p + off, parts * out, in, {}, {}, out, stride}; e.bias = has_bias ? m->params.p + off + (int64_t)out * in : nullptr; e.layer = cur_layer; mats.push_back(e);
     };
     for (auto& l : m->L) {
       const gn_layer_desc& d = l.d; cur_layer = (int)(&l - m->L.data());
       if (d.kind == GN_LAYER_DENSE) add(l.p_off, d.out_size, d.in_size);
       else if (d.kind == GN_LAYER_TRANSFORMER_BLOCK) {
         const int64_t dd = (int64_t)d.dim * d.dim + d.dim; int64_t o = l.p_off;
-        for (int k = 0; k < 4; k++) { add(o, d.dim, d.dim); o += dd; }
+        if (d.dim % 32 == 0) { add(o, d.dim, d.dim, true, 3, dd); o += 3 * dd; } else for (int k = 0; k < 3; k++) { add(o, d.dim, d.dim); o += dd; }
+        add(o, d.dim, d.dim); o += dd;
         o += (l.rms ? 2 : 4) * (int64_t)d.dim;
-        if (l.ff_act == GN_ACT_SILU) { add(o, d.ff_dim, d.dim, false); add(o + (int64_t)d.dim * d.ff_dim, d.ff_dim, d.dim, false); o += 2 * (int64_t)d.dim * d.ff_dim; }
+        if (l.ff_act == GN_ACT_SILU) {
+          const int64_t df = (int64_t)d.dim * d.ff_dim;
+          if (d.ff_dim % 32 == 0) add(o, d.ff_dim, d.dim, false, 2, df); else { add(o, d.ff_dim, d.dim, false); add(o + df, d.ff_dim, d.dim, false); }
+          o += 2 * df;
+        }
         else { add(o, d.ff_dim, d.dim); o += (int64_t)d.dim * d.ff_dim + d.ff_dim; }
         add(o, d.dim, d.ff_dim);
       }

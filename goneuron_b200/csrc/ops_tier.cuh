@@ -23,15 +23,15 @@ int gn_op_layernorm(gn_ctx* ctx, int64_t rows, int n, const float* x, const floa
   if (dy && (!dx || !dgamma || !dbeta)) return fail(GN_ERR_INVALID_ARG, "op_layernorm: dy given without dx, dgamma, dbeta");
   Ctx* c = &ctx->c; std::lock_guard<std::mutex> run_lk(c->run_mu); GN_CUDA(cudaSetDevice(c->device));
   HostIO io(c); const size_t tot = (size_t)rows * n;
-  float *dX = io.in(x, tot), *dG = io.in(gamma, n), *dB = io.in(beta, n), *dY = io.out(tot), *mean = io.out(rows), *sd = io.out(rows);
+  float *dX = io.in(x, tot), *dG = io.in(gamma, n), *dB = io.in(beta, n), *dY = io.out(tot), *stat = io.out(2 * rows);
   GN_TRY(io.rc);
-  GN_TRY(layernorm_forward(c, dX, dG, dB, dY, mean, sd, rows, n));
+  GN_TRY(norm_forward(c, false, dX, dG, dB, dY, stat, rows, n, 1e-5f));
   GN_TRY(io.back(y, dY, tot));
   if (dy) {
     gn_model tmp; tmp.ctx = ctx;
     float *dDy = io.in(dy, tot), *dDx = io.out(tot), *gG = io.zeros(n), *gB = io.zeros(n);
     GN_TRY(io.rc);
-    GN_TRY(layernorm_backward(&tmp, dDy, dX, dG, mean, sd, dDx, gG, gB, rows, n));
+    GN_TRY(norm_backward(&tmp, false, dDy, dX, dG, stat, dDx, gG, gB, rows, n));
     GN_TRY(io.back(dx, dDx, tot)); GN_TRY(io.back(dgamma, gG, n)); GN_TRY(io.back(dbeta, gB, n));
     GN_CUDA(cudaStreamSynchronize(c->stream));
   }

@@ -311,126 +311,161 @@ __global__ void layernorm_pgrad_partial_kernel(const float* __restrict__ g, cons
   part[((long)blockIdx.y * 2) * n + c] = sgam; part[((long)blockIdx.y * 2 + 1) * n + c] = sbet;
 }
 // block = 32 columns x 32 groups of chunks (1024 threads); the groups are combined through shared memory in a fixed order
+// gBeta may be null (RMSNorm)
 __global__ void __launch_bounds__(1024) layernorm_pgrad_final_kernel(const float* __restrict__ part, int chunks, int n, float* __restrict__ gGamma, float* __restrict__ gBeta) {
   __shared__ float sa[32][33], sb[32][33];
   const int tx = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
   float a = 0.f, b = 0.f;
-  if (c < n) for (int k = grp; k < chunks; k += 32) { a += part[((long)k * 2) * n + c]; b += part[((long)k * 2 + 1) * n + c]; }
+  if (c < n) {
+#pragma unroll 4
+    for (int k = grp; k < chunks; k += 32) { a += part[((long)k * 2) * n + c]; if (gBeta) b += part[((long)k * 2 + 1) * n + c]; }
+  }
   sa[grp][tx] = a; sb[grp][tx] = b;
   __syncthreads();
   if (grp == 0 && c < n) {
     float ta = 0.f, tb = 0.f;
     for (int k = 0; k < 32; k++) { ta += sa[k][tx]; tb += sb[k][tx]; }
-    gGamma[c] = ta; gBeta[c] = tb;
+    gGamma[c] = ta; if (gBeta) gBeta[c] = tb;
   }
 }
 
-// Row-in-registers variants for n = 128 * NV (NV <= 16): one warp per row, the row is read once with 16-byte loads
-// and kept in registers between the reduction and the output pass.  Same arithmetic as the kernels above.
-// Optional second output of the row-in-registers kernels: the row as operand planes of the contraction engine (two fp16
-// planes interleaved in blocks of 32 columns, row length 2 n, the row's inverse scale, its 2-norm) -- the kernel holds the whole row, so the row maximum
-// and norm cost two warp reductions, and the separate split pass (a second read of the tensor) is not needed for the contraction that
-// consumes this output.
+// ---------------------------------------------------------------- rows in registers
+// LayerNorm (RMS = false) and RMSNorm for rows of up to 1024 columns, a multiple of four, 16-byte aligned: one warp per row, the row
+// is read once and kept in registers (NV float4 per lane) between the reductions and the output.  Same arithmetic as the kernels
+// above and below, except that LayerNorm takes one reciprocal of the deviation per row instead of a division per element.
+// Optional second output: the row as operand planes of the contraction engine (two fp16 planes interleaved in blocks of 32
+// columns, row length 2 ldp, zero beyond n; the row's inverse scale, its 2-norm): the row maximum and norm are two warp
+// reductions here, and the contraction that consumes the row needs no split pass.
 struct RowPlaneOut { __half* p = nullptr; float* inv = nullptr; float* rownorm = nullptr; };
 template <int NV>
-__device__ __forceinline__ void row_planes_emit(const float4 (&o)[NV], long row, int lane, const RowPlaneOut& po) {
-  constexpr int n = 128 * NV;
-  float mx = 0.f, sq = 0.f;
+__device__ __forceinline__ void row_planes_emit(const float4 (&o)[NV], long row, int n, int lane, const RowPlaneOut& po) {
+  float mx = 0.f, sq = 0.f; const int ldp = (n + 31) & ~31;
 #pragma unroll
-  for (int k = 0; k < NV; k++) {
+  for (int k = 0; k < NV; k++) {                            // (entries beyond n are zero)
     mx = fmaxf(mx, fmaxf(fmaxf(fabsf(o[k].x), fabsf(o[k].y)), fmaxf(fabsf(o[k].z), fabsf(o[k].w))));
     sq += (o[k].x * o[k].x + o[k].y * o[k].y) + (o[k].z * o[k].z + o[k].w * o[k].w);
   }
   mx = warp_max(mx); sq = warp_sum(sq);
   float inv; const float sc = row_scale(mx, &inv);
   if (lane == 0) { po.inv[row] = inv; if (po.rownorm) po.rownorm[row] = sqrtf(sq) * 1.0001f; }
-  __half* h = po.p + row * 2 * n + pl_off(4 * lane);          // columns 4 lane + 128 k
+  __half* h = po.p + row * 2 * ldp + pl_off(4 * lane);      // columns 4 lane + 128 k
 #pragma unroll
   for (int k = 0; k < NV; k++) {
+    if (4 * lane + 128 * k >= ldp) continue;
     uint2 a, b; split2_pair(o[k].x, o[k].y, sc, a.x, b.x); split2_pair(o[k].z, o[k].w, sc, a.y, b.y);
     *reinterpret_cast<uint2*>(h + 256 * k) = a; *reinterpret_cast<uint2*>(h + 256 * k + PL_LO) = b;
   }
 }
 template <int NV>
-__global__ void __launch_bounds__(256) layernorm_fwd_vec_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
-                                                                float* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ std_out, long rows, float eps,
-                                                                const RowPlaneOut po) {
-  constexpr int n = 128 * NV;
-  const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5); if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const float4* xr = reinterpret_cast<const float4*>(x + row * n) + lane;
-  float4 v[NV];
+__device__ __forceinline__ void row_load(float4 (&v)[NV], const float* __restrict__ p, int n, int lane) {
 #pragma unroll
-  for (int k = 0; k < NV; k++) v[k] = xr[32 * k];
-  float s = 0.f;
-#pragma unroll
-  for (int k = 0; k < NV; k++) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
-  const float mean = warp_sum(s) / (float)n;
-  float ss = 0.f;
-#pragma unroll
-  for (int k = 0; k < NV; k++) { float a = v[k].x - mean, b = v[k].y - mean, c = v[k].z - mean, d = v[k].w - mean; ss += (a * a + b * b) + (c * c + d * d); }
-  const float sd = sqrtf(warp_sum(ss) / (float)n + eps), isd = 1.f / sd;     // one reciprocal per row instead of a division per element
-  float4* yr = reinterpret_cast<float4*>(y + row * n) + lane;
-#pragma unroll
-  for (int k = 0; k < NV; k++) {
-    const float4 ga = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * k), be = __ldg(reinterpret_cast<const float4*>(beta) + lane + 32 * k);
-    v[k] = make_float4(ga.x * ((v[k].x - mean) * isd) + be.x, ga.y * ((v[k].y - mean) * isd) + be.y, ga.z * ((v[k].z - mean) * isd) + be.z, ga.w * ((v[k].w - mean) * isd) + be.w);
-    yr[32 * k] = v[k];
-  }
-  if (lane == 0) { mean_out[row] = mean; std_out[row] = sd; }
-  if (po.p) row_planes_emit<NV>(v, row, lane, po);
+  for (int k = 0; k < NV; k++) v[k] = 4 * lane + 128 * k < n ? *reinterpret_cast<const float4*>(p + 4 * lane + 128 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 template <int NV>
-__global__ void __launch_bounds__(256) layernorm_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ gamma,
-                                                                const float* __restrict__ mean_in, const float* __restrict__ std_in, float* dx, long rows,
-                                                                const RowPlaneOut po) {
-  constexpr int n = 128 * NV;
+__device__ __forceinline__ void row_store(const float4 (&v)[NV], float* __restrict__ p, int n, int lane) {
+#pragma unroll
+  for (int k = 0; k < NV; k++) if (4 * lane + 128 * k < n) *reinterpret_cast<float4*>(p + 4 * lane + 128 * k) = v[k];
+}
+// stat_a: row means (RMS: row rms), stat_b: row deviations
+template <int NV, bool RMS>
+__global__ void __launch_bounds__(256) norm_fwd_vec_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ y,
+                                                           float* __restrict__ stat_a, float* __restrict__ stat_b, long rows, int n, float eps, const RowPlaneOut po) {
   const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5); if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const float4* xr = reinterpret_cast<const float4*>(x + row * n) + lane;
-  const float4* gr = reinterpret_cast<const float4*>(g + row * n) + lane;
-  float4 q[NV], d[NV];
+  const int lane = threadIdx.x & 31; const float fn = (float)n;
+  float4 v[NV]; row_load(v, x + row * n, n, lane);
+  if (RMS) {
+    float ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < NV; k++) { q[k] = gr[32 * k]; d[k] = xr[32 * k]; }
-  const float mean = mean_in[row], sd = std_in[row];
-  float sg = 0.f, sgx = 0.f;
+    for (int k = 0; k < NV; k++) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+    const float r = (float)sqrt((double)(warp_sum(ss) / fn + eps));
+#pragma unroll
+    for (int k = 0; k < NV; k++) if (4 * lane + 128 * k < n) {
+      const float4 ga = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * k);
+      v[k] = make_float4((v[k].x / r) * ga.x, (v[k].y / r) * ga.y, (v[k].z / r) * ga.z, (v[k].w / r) * ga.w);
+    }
+    if (lane == 0) stat_a[row] = r;
+  } else {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; k++) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+    const float mean = warp_sum(s) / fn;
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; k++) if (4 * lane + 128 * k < n) { const float a = v[k].x - mean, b = v[k].y - mean, c = v[k].z - mean, d = v[k].w - mean; ss += (a * a + b * b) + (c * c + d * d); }
+    const float sd = sqrtf(warp_sum(ss) / fn + eps), isd = 1.f / sd;
+#pragma unroll
+    for (int k = 0; k < NV; k++) if (4 * lane + 128 * k < n) {
+      const float4 ga = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * k), be = __ldg(reinterpret_cast<const float4*>(beta) + lane + 32 * k);
+      v[k] = make_float4(ga.x * ((v[k].x - mean) * isd) + be.x, ga.y * ((v[k].y - mean) * isd) + be.y, ga.z * ((v[k].z - mean) * isd) + be.z, ga.w * ((v[k].w - mean) * isd) + be.w);
+    }
+    if (lane == 0) { stat_a[row] = mean; stat_b[row] = sd; }
+  }
+  row_store(v, y + row * n, n, lane);
+  if (po.p) row_planes_emit(v, row, n, lane, po);
+}
+// dx (may alias g), and this block's part of the parameter gradients: part[block][0] = sum g (x - mean) / sd (RMS: sum g x / rms),
+// part[block][1] = sum g.  The warps stride over the rows with the sums of their columns in registers, so g and x are read
+// once for both outputs (two passes before, the second at 1 TB/s: 18 of 25 us at 3600 rows of 384).
+template <int NV, bool RMS>
+__global__ void __launch_bounds__(256) norm_bwd_vec_kernel(const float* g, const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ stat_a,
+                                                           const float* __restrict__ stat_b, float* dx, float* __restrict__ part, long rows, int n, const RowPlaneOut po) {
+  __shared__ float4 red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5; const float fn = (float)n;
+  float4 ga[NV], sg_[NV], sb_[NV];
+#pragma unroll
+  for (int k = 0; k < NV; k++) sg_[k] = sb_[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  row_load(ga, gamma, n, lane);
+  for (long row = (long)blockIdx.x * 8 + w; row < rows; row += (long)gridDim.x * 8) {
+    float4 q[NV], d[NV]; row_load(q, g + row * n, n, lane); row_load(d, x + row * n, n, lane);
+    const float a = stat_a[row];
+    float s = 0.f, sx = 0.f;
+    if (RMS) {
+      const float inv = 1.f / a;
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        sg_[k].x += q[k].x * (d[k].x * inv); sg_[k].y += q[k].y * (d[k].y * inv); sg_[k].z += q[k].z * (d[k].z * inv); sg_[k].w += q[k].w * (d[k].w * inv);
+        sx += (q[k].x * ga[k].x * d[k].x + q[k].y * ga[k].y * d[k].y) + (q[k].z * ga[k].z * d[k].z + q[k].w * ga[k].w * d[k].w);
+      }
+      const float f = warp_sum(sx) / (fn * a * a);
+#pragma unroll
+      for (int k = 0; k < NV; k++)
+        q[k] = make_float4((ga[k].x * inv) * (q[k].x - d[k].x * f), (ga[k].y * inv) * (q[k].y - d[k].y * f), (ga[k].z * inv) * (q[k].z - d[k].z * f), (ga[k].w * inv) * (q[k].w - d[k].w * f));
+    } else {
+      const float sd = stat_b[row], isd = 1.f / sd;
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        if (4 * lane + 128 * k < n) { d[k].x -= a; d[k].y -= a; d[k].z -= a; d[k].w -= a; }
+        sg_[k].x += q[k].x * (d[k].x * isd); sg_[k].y += q[k].y * (d[k].y * isd); sg_[k].z += q[k].z * (d[k].z * isd); sg_[k].w += q[k].w * (d[k].w * isd);
+        sb_[k].x += q[k].x; sb_[k].y += q[k].y; sb_[k].z += q[k].z; sb_[k].w += q[k].w;
+        q[k].x *= ga[k].x; q[k].y *= ga[k].y; q[k].z *= ga[k].z; q[k].w *= ga[k].w;
+        s += (q[k].x + q[k].y) + (q[k].z + q[k].w);
+        sx += (q[k].x * d[k].x + q[k].y * d[k].y) + (q[k].z * d[k].z + q[k].w * d[k].w);
+      }
+      s = warp_sum(s) / fn; const float f = warp_sum(sx) / (fn * sd * sd);
+#pragma unroll
+      for (int k = 0; k < NV; k++) if (4 * lane + 128 * k < n)
+        q[k] = make_float4((q[k].x - s) * isd - d[k].x * f, (q[k].y - s) * isd - d[k].y * f, (q[k].z - s) * isd - d[k].z * f, (q[k].w - s) * isd - d[k].w * f);
+    }
+    row_store(q, dx + row * n, n, lane);
+    if (po.p) row_planes_emit(q, row, n, lane, po);
+  }
+  float* pb = part + (long)blockIdx.x * 2 * n;
 #pragma unroll
   for (int k = 0; k < NV; k++) {
-    const float4 ga = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * k);
-    q[k].x *= ga.x; q[k].y *= ga.y; q[k].z *= ga.z; q[k].w *= ga.w;
-    d[k].x -= mean; d[k].y -= mean; d[k].z -= mean; d[k].w -= mean;
-    sg += (q[k].x + q[k].y) + (q[k].z + q[k].w);
-    sgx += (q[k].x * d[k].x + q[k].y * d[k].y) + (q[k].z * d[k].z + q[k].w * d[k].w);
-  }
-  sg = warp_sum(sg); sgx = warp_sum(sgx);
-  const float fn = (float)n, sgn = sg / fn, isd = 1.f / sd, w = sgx / (fn * sd * sd);     // reciprocals per row, not per element
-  float4* dr = reinterpret_cast<float4*>(dx + row * n) + lane;
 #pragma unroll
-  for (int k = 0; k < NV; k++) {
-    q[k] = make_float4((q[k].x - sgn) * isd - d[k].x * w, (q[k].y - sgn) * isd - d[k].y * w,
-                       (q[k].z - sgn) * isd - d[k].z * w, (q[k].w - sgn) * isd - d[k].w * w);
-    dr[32 * k] = q[k];
+    for (int h = 0; h < (RMS ? 1 : 2); h++) {
+      __syncthreads();
+      red[w][lane] = h ? sb_[k] : sg_[k];
+      __syncthreads();
+      if (w == 0 && 4 * lane + 128 * k < n) {
+        float4 t = red[0][lane];
+#pragma unroll
+        for (int r = 1; r < 8; r++) { const float4 u = red[r][lane]; t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+        *reinterpret_cast<float4*>(pb + h * n + 4 * lane + 128 * k) = t;
+      }
+    }
   }
-  if (po.p) row_planes_emit<NV>(q, row, lane, po);
 }
-// Partial column sums for gGamma / gBeta with 16-byte loads: block = 256 threads = up to 1024 columns, grid.x covers the
-// columns, grid.y the row chunks; part layout as in layernorm_pgrad_partial_kernel.
-__global__ void __launch_bounds__(256) layernorm_pgrad_partial_vec_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ mean_in,
-                                                                          const float* __restrict__ std_in, long rows, int n, float* __restrict__ part) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 4; if (c >= n) return;
-  const long chunks = gridDim.y, per = (rows + chunks - 1) / chunks, r0 = blockIdx.y * per, r1 = min(rows, r0 + per);
-  float4 sgam = make_float4(0.f, 0.f, 0.f, 0.f), sbet = sgam;
-#pragma unroll 4
-  for (long r = r0; r < r1; r++) {
-    const float4 gg = *reinterpret_cast<const float4*>(g + r * n + c), xx = *reinterpret_cast<const float4*>(x + r * n + c);
-    const float mean = mean_in[r], isd = 1.f / std_in[r];
-    sgam.x += gg.x * ((xx.x - mean) * isd); sgam.y += gg.y * ((xx.y - mean) * isd); sgam.z += gg.z * ((xx.z - mean) * isd); sgam.w += gg.w * ((xx.w - mean) * isd);
-    sbet.x += gg.x; sbet.y += gg.y; sbet.z += gg.z; sbet.w += gg.w;
-  }
-  *reinterpret_cast<float4*>(part + ((long)blockIdx.y * 2) * n + c) = sgam;
-  *reinterpret_cast<float4*>(part + ((long)blockIdx.y * 2 + 1) * n + c) = sbet;
-}
-
 // ---------------------------------------------------------------- RMSNorm
 // One warp per row.  reference: rmsnorm.go:222-240 (forward), :301-330 (backward); the row's rms is kept for the backward.
 __global__ void rmsnorm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma, float* __restrict__ y, float* __restrict__ rms_out, long rows, int n, float eps) {
@@ -677,15 +712,31 @@ __global__ void relu_mask_last_token_kernel(float* __restrict__ dM, const float*
 // Rotary embeddings on a [tokens, D] tensor in place (transformer.go:212-236): within every head, element i of the first
 // half and element i + hd/2 are rotated by the angle of (position, i); `tab` holds cos | sin per (position, i), computed on
 // the host with the reference's float32 / float64 conversions.  sign = -1 applies the conjugate (backward pass).
-// Row r of a sequence's T rows is its token r * tstep.
-__global__ void rope_kernel(float* __restrict__ x, const float* __restrict__ tab, long tokens, int T, int D, int hd, float sign, int tstep) {
-  const int half = hd >> 1; const long per = (long)(D >> 1), total = tokens * per;
+// Row r of a sequence's T rows is its token r * tstep.  blockIdx.y picks one of two arrays; V neighbouring pairs per thread (4: hd a
+// multiple of 8, rows 16-byte aligned).  Memory-bound; with one pair per thread and 64-bit index divisions a pass over 4096 x 512
+// took 11 us, twice its traffic's time, and q and k took a launch each.
+template <int V>
+__global__ void __launch_bounds__(256) rope_kernel(float* __restrict__ x0, float* __restrict__ x1, const float* __restrict__ tab, long tokens, int T, int D, int hd, float sign, int tstep) {
+  float* x = blockIdx.y ? x1 : x0;
+  const int half = hd >> 1, per = (D >> 1) / V; const long total = tokens * per;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-    const long tok = e / per; const int r = (int)(e - tok * per), h = r / half, i = r - h * half, t = (int)(tok % T) * tstep;
-    const float c = tab[((long)t * half + i) * 2], s = sign * tab[((long)t * half + i) * 2 + 1];
-    float* p = x + tok * D + (long)h * hd + i;
-    const float v1 = p[0], v2 = p[half];
-    p[0] = v1 * c - v2 * s; p[half] = v1 * s + v2 * c;
+    const long tok = total < 0x7fffffffL ? (long)((unsigned)e / (unsigned)per) : e / per;
+    const int r = (int)(e - tok * per) * V, h = r / half, i = r - h * half;
+    const int t = (total < 0x7fffffffL ? (int)((unsigned)tok % (unsigned)T) : (int)(tok % T)) * tstep;
+    const float* cs = tab + ((long)t * half + i) * 2; float* p = x + tok * D + (long)h * hd + i;
+    float a[V], b[V], c[2 * V];
+    if constexpr (V == 4) {
+      const float4 u = *reinterpret_cast<const float4*>(p), w = *reinterpret_cast<const float4*>(p + half);
+      const float4 c0 = __ldg(reinterpret_cast<const float4*>(cs)), c1 = __ldg(reinterpret_cast<const float4*>(cs) + 1);
+      a[0] = u.x; a[1] = u.y; a[2] = u.z; a[3] = u.w; b[0] = w.x; b[1] = w.y; b[2] = w.z; b[3] = w.w;
+      c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
+    } else { a[0] = p[0]; b[0] = p[half]; c[0] = cs[0]; c[1] = cs[1]; }
+    float o0[V], o1[V];
+#pragma unroll
+    for (int j = 0; j < V; j++) { const float sn = sign * c[2 * j + 1]; o0[j] = a[j] * c[2 * j] - b[j] * sn; o1[j] = a[j] * sn + b[j] * c[2 * j]; }
+    if constexpr (V == 4) {
+      *reinterpret_cast<float4*>(p) = make_float4(o0[0], o0[1], o0[2], o0[3]); *reinterpret_cast<float4*>(p + half) = make_float4(o1[0], o1[1], o1[2], o1[3]);
+    } else { p[0] = o0[0]; p[half] = o1[0]; }
   }
 }
 // rows [B, C] <- the last token's row of every sequence of in [B, T, C]
@@ -695,6 +746,9 @@ __global__ void last_token_rows_kernel(const float* __restrict__ in, float* __re
 // dz[s,t,:] *= act'(z_last[s,:]): a Dense layer called token by token differentiates at its LAST call's pre-activation (layer.go:563-567)
 __global__ void scale_by_last_deriv_kernel(float* __restrict__ dz, const float* __restrict__ z_last, int T, int C, long total, int act) {
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) { const long row = e / C; dz[e] *= act_der(act, z_last[(row / T) * C + (e - row * C)]); }
+}
+__global__ void act_deriv_kernel(const float* __restrict__ z, float* __restrict__ out, long n, int act) {
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) out[e] = act_der(act, z[e]);
 }
 // SwiGLU (swiglu.go:163-170): out = swish(gate) * up
 __global__ void swiglu_fwd_kernel(const float* __restrict__ gate, const float* __restrict__ up, float* __restrict__ out, long n) {
@@ -710,6 +764,74 @@ __global__ void swiglu_bwd_paired_kernel(const float* __restrict__ dOut, const f
     const long pe = (s * T + (T - 1 - t)) * C + c;            // partner element
     const float g = gate[pe], u = up[pe], sig = act_fwd(GN_ACT_SIGMOID, g), sw = g * sig, go = dOut[e];
     dUpP[pe] = go * sw; dGateP[pe] = go * (sw + sig * (1.f - sw)) * u;
+  }
+}
+// The two passes above for rows of up to 4096 columns (a multiple of 32) whose results feed the tensor-core engine: a block keeps its
+// row in registers between the row's maximum and the operand planes, so the separate split passes (the row read once or twice
+// more) go.  Memory-bound: 12 and 28 bytes per element.  Forward: mid only as planes, and the last token's rows in fp32 (the
+// weight gradient's input).  Backward: planes of [dGate | dUp] rows (the input gradient's operand) and both in fp32 (the weight
+// gradients need them transposed).
+constexpr int SW_THREADS = 128;
+__device__ __forceinline__ float row_block_max(float mx, float* red) {
+  mx = warp_max(mx);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  return fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+}
+__device__ __forceinline__ float max4(float m, float4 v) { return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); }
+__device__ __forceinline__ void planes_store4(__half* row, int c, float4 v, float sc) {
+  uint2 a, b; split2_pair(v.x, v.y, sc, a.x, b.x); split2_pair(v.z, v.w, sc, a.y, b.y);
+  *reinterpret_cast<uint2*>(row + pl_off(c)) = a; *reinterpret_cast<uint2*>(row + pl_off(c) + PL_LO) = b;
+}
+template <int NV>
+__global__ void __launch_bounds__(SW_THREADS) swiglu_fwd_planes_kernel(const float* __restrict__ gate, const float* __restrict__ up, __half* __restrict__ pl, float* __restrict__ inv_scale,
+                                                                       float* __restrict__ last, int T, int F) {
+  __shared__ float red[4];
+  const long row = blockIdx.x; const int c0 = threadIdx.x * 4; float4 o[NV]; float mx = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int c = c0 + 512 * k;
+    if (c < F) {
+      const float4 g = *reinterpret_cast<const float4*>(gate + row * F + c), u = *reinterpret_cast<const float4*>(up + row * F + c);
+      o[k] = make_float4((g.x * act_fwd(GN_ACT_SIGMOID, g.x)) * u.x, (g.y * act_fwd(GN_ACT_SIGMOID, g.y)) * u.y, (g.z * act_fwd(GN_ACT_SIGMOID, g.z)) * u.z, (g.w * act_fwd(GN_ACT_SIGMOID, g.w)) * u.w);
+      mx = max4(mx, o[k]);
+    }
+  }
+  float inv; const float sc = row_scale(row_block_max(mx, red), &inv);
+  if (threadIdx.x == 0) inv_scale[row] = inv;
+  const bool is_last = row % T == T - 1;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int c = c0 + 512 * k; if (c >= F) break;
+    planes_store4(pl + row * 2 * F, c, o[k], sc);
+    if (is_last) *reinterpret_cast<float4*>(last + (row / T) * F + c) = o[k];
+  }
+}
+__device__ __forceinline__ void swiglu_der(float g, float u, float go, float& dg, float& du) {
+  const float sig = act_fwd(GN_ACT_SIGMOID, g), sw = g * sig;
+  du = go * sw; dg = go * (sw + sig * (1.f - sw)) * u;
+}
+template <int NV>
+__global__ void __launch_bounds__(SW_THREADS) swiglu_bwd_planes_kernel(const float* __restrict__ dOut, const float* __restrict__ gate, const float* __restrict__ up, float* __restrict__ dGateP,
+                                                                       float* __restrict__ dUpP, __half* __restrict__ pl, float* __restrict__ inv_scale, int T, int F) {
+  __shared__ float red[4];
+  const long row = blockIdx.x, s = row / T, src = s * T + (T - 1 - (row - s * T)); const int c0 = threadIdx.x * 4; float4 dg[NV], du[NV]; float mx = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int c = c0 + 512 * k;
+    if (c < F) {
+      const float4 g = *reinterpret_cast<const float4*>(gate + row * F + c), u = *reinterpret_cast<const float4*>(up + row * F + c), go = *reinterpret_cast<const float4*>(dOut + src * F + c);
+      swiglu_der(g.x, u.x, go.x, dg[k].x, du[k].x); swiglu_der(g.y, u.y, go.y, dg[k].y, du[k].y); swiglu_der(g.z, u.z, go.z, dg[k].z, du[k].z); swiglu_der(g.w, u.w, go.w, dg[k].w, du[k].w);
+      mx = max4(max4(mx, dg[k]), du[k]);
+    }
+  }
+  float inv; const float sc = row_scale(row_block_max(mx, red), &inv);
+  if (threadIdx.x == 0) inv_scale[row] = inv;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int c = c0 + 512 * k; if (c >= F) break;
+    *reinterpret_cast<float4*>(dGateP + row * F + c) = dg[k]; *reinterpret_cast<float4*>(dUpP + row * F + c) = du[k];
+    planes_store4(pl + row * 4 * F, c, dg[k], sc); planes_store4(pl + row * 4 * F, F + c, du[k], sc);
   }
 }
 // The same for the gradient of token 0 alone: rows s of dOut, dGate, dUp are dense, the last token's projections lie `ld` apart
