@@ -6,114 +6,184 @@
 // softmax Jacobian, dQ / dK / dV).  The Jacobian row term sum_k dP_k P_k equals dO . O (O = P V), which is
 // what the backward kernels use; the row maximum and the row sum of the forward softmax are kept per row.
 //
-// Arithmetic: every product runs as 3xTF32 (hi*hi + hi*lo + lo*hi with fp32 accumulation) on warp-level
-// tensor-core MMAs, the operands being split in registers, so accuracy is fp32-level.  One CTA = 64 query
-// (or key) rows of one head, 4 warps x 16 rows, key (query) blocks of 64 streamed through shared memory;
-// causal blocks above the diagonal are never visited.
+// Arithmetic: fp32-level products from two fp16 parts per operand, x s = hi + lo with a power-of-two scale s per row (22 bits below
+// the row's maximum), hi hi + hi lo + lo hi with fp32 accumulation on warp-level tensor-core MMAs (m16n8k16).  The split happens
+// once per tile, on the way into shared memory, and the fragments come out by ldmatrix: three MMAs per fragment load of 16
+// contraction indices.  (Splitting fp32 fragments into TF32 parts in registers cost two loads and four logic operations per three
+// MMAs of 8 indices, in every warp again: 36 us forward and 140 backward at 24 x 150 tokens, 12 heads of 32.)  Where rows are
+// summed over (P V, dS K, ...) their inverse scales go into the other operand, which gets a scale per row from its maximum in turn.
+// One CTA = 64 query (or key) rows of one head, 4 warps x 16 rows, key (query) blocks of 64 streamed through shared memory;
+// causal blocks above the diagonal are never visited.  These kernels take what the tcgen05 kernels do not: heads of 16 and 32, and
+// sequences that are not a multiple of 128, where a tile of 128 would be mostly padding.
 //
 // Q, K, V, O, dO and the outputs are [batch*T, D] row-major with head h in columns [h*HD, (h+1)*HD).
 #pragma once
 #include "common.cuh"
+#include "gemm_tc.cuh"
 
 namespace gn {
 
 constexpr int AT_BLK = 64, AT_THREADS = 128;
 
-struct FragA { uint32_t hi[4], lo[4]; };
-struct FragB { uint32_t hi[2], lo[2]; };
-
-// hi = x with the 13 low mantissa bits cleared (exactly a TF32 value; a logic op, full rate -- the cvt.rna
-// conversion runs on a slow pipe), lo = x - hi (exact; the MMA reads its leading 10 mantissa bits).
-__device__ __forceinline__ void split32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = __float_as_uint(x) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi));
-}
-__device__ __forceinline__ void mma8(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-__device__ __forceinline__ void mma3(float (&d)[4], const FragA& a, const FragB& b) { mma8(d, a.lo, b.hi); mma8(d, a.hi, b.lo); mma8(d, a.hi, b.hi); }
-
-// A(r, k) = s[(row0 + r) * LD + k0 + k], 16 x 8.  Fragment order: (g,t) (g+8,t) (g,t+4) (g+8,t+4).
-__device__ __forceinline__ void load_a(FragA& f, const float* s, int LD, int row0, int k0, int g, int t) {
-  const float* p = s + (row0 + g) * LD + k0 + t;
-  split32(p[0], f.hi[0], f.lo[0]); split32(p[8 * LD], f.hi[1], f.lo[1]); split32(p[4], f.hi[2], f.lo[2]); split32(p[8 * LD + 4], f.hi[3], f.lo[3]);
-}
-// B(k, n) = s[(n0 + n) * LD + k0 + k], 8 x 8: the contraction runs along the shared-memory row.
-__device__ __forceinline__ void load_b_nk(FragB& f, const float* s, int LD, int n0, int k0, int g, int t) {
-  const float* p = s + (n0 + g) * LD + k0 + t;
-  split32(p[0], f.hi[0], f.lo[0]); split32(p[4], f.hi[1], f.lo[1]);
-}
-// B(k, n) = s[(k0 + k') * LD + n0 + n] with the contraction index permuted: MMA k-index t <-> row k0 + 2t,
-// t + 4 <-> row k0 + 2t + 1.  This is the order in which an accumulator fragment holds its 8 columns
-// (thread t owns columns 2t and 2t+1), so an accumulator can be fed back as the A operand without shuffles.
-__device__ __forceinline__ void load_b_kn2(FragB& f, const float* s, int LD, int k0, int n0, int g, int t) {
-  const float* p = s + (k0 + 2 * t) * LD + n0 + g;
-  split32(p[0], f.hi[0], f.lo[0]); split32(p[LD], f.hi[1], f.lo[1]);
-}
-// accumulator fragment (rows g, g+8; columns 2t, 2t+1) as A operand in the permuted order above
-__device__ __forceinline__ void acc_to_a(FragA& f, const float (&c)[4]) {
-  split32(c[0], f.hi[0], f.lo[0]); split32(c[2], f.hi[1], f.lo[1]); split32(c[1], f.hi[2], f.lo[2]); split32(c[3], f.hi[3], f.lo[3]);
-}
-// 64 x HD tile of a [*, D] tensor into shared memory (row stride LD), rows >= T zero-filled
-template <int HD>
-__device__ __forceinline__ void load_tile(float* s, const float* src, long base, int row0, int T, int D) {
-  constexpr int LD = HD + 4, V4 = HD / 4;
-  for (int e = threadIdx.x; e < AT_BLK * V4; e += AT_THREADS) {
-    int r = e / V4, c4 = e - r * V4, row = row0 + r;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < T) v = *reinterpret_cast<const float4*>(src + base + (long)row * D + c4 * 4);
-    *reinterpret_cast<float4*>(s + r * LD + c4 * 4) = v;
-  }
-}
 __device__ __forceinline__ float quad_max(float v) { v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1)); return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2)); }
 __device__ __forceinline__ float quad_sum(float v) { v += __shfl_xor_sync(0xffffffffu, v, 1); return v + __shfl_xor_sync(0xffffffffu, v, 2); }
+template <int HD> struct AtCfg {
+  static constexpr int LDH = 2 * HD + 8;                     // halves per tile row: hi | lo | pad; an odd number of 16-byte units, so ldmatrix is free of bank conflicts
+  static constexpr int TILE = AT_BLK * LDH;
+  static constexpr int V4 = HD / 4, RP = AT_THREADS / V4, NP = AT_BLK / RP;      // threads per row, rows per pass, passes of a tile load
+};
+__device__ __forceinline__ void mma16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+// 64 rows of a [*, D] tensor into a tile (hi | lo), inverse row scales into `inv`; rows >= T read as zero.  With `other`: also the
+// dot products of the rows with those of `other`, into `dot` (dO . O).
+template <int HD, bool DOT>
+__device__ __forceinline__ void at_load(__half* s, float* inv, const float* __restrict__ src, long base, int row0, int T, int D, const float* __restrict__ other = nullptr, float* dot = nullptr) {
+  using C = AtCfg<HD>;
+  const int c4 = threadIdx.x % C::V4, rr = threadIdx.x / C::V4;
+  float4 v[C::NP], w[DOT ? C::NP : 1];
+#pragma unroll
+  for (int p = 0; p < C::NP; p++) {
+    const int row = row0 + p * C::RP + rr; const long o = base + (long)row * D + c4 * 4;
+    v[p] = row < T ? *reinterpret_cast<const float4*>(src + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (DOT) w[p] = row < T ? *reinterpret_cast<const float4*>(other + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int p = 0; p < C::NP; p++) {
+    const int r = p * C::RP + rr;
+    float mx = fmaxf(fmaxf(fabsf(v[p].x), fabsf(v[p].y)), fmaxf(fabsf(v[p].z), fabsf(v[p].w))), d = 0.f;
+    if constexpr (DOT) d = (v[p].x * w[p].x + v[p].y * w[p].y) + (v[p].z * w[p].z + v[p].w * w[p].w);
+#pragma unroll
+    for (int o = C::V4 / 2; o > 0; o >>= 1) { mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); if constexpr (DOT) d += __shfl_xor_sync(0xffffffffu, d, o); }
+    float iv; const float sc = row_scale(mx, &iv);
+    uint2 hi, lo; split2_pair(v[p].x, v[p].y, sc, hi.x, lo.x); split2_pair(v[p].z, v[p].w, sc, hi.y, lo.y);
+    *reinterpret_cast<uint2*>(s + r * C::LDH + c4 * 4) = hi; *reinterpret_cast<uint2*>(s + r * C::LDH + HD + c4 * 4) = lo;
+    if (c4 == 0) { inv[r] = iv; if constexpr (DOT) dot[r] = d; }
+  }
+}
+// acc[n] = A(rows r0 .. r0 + 15) B(rows 8 n .. 8 n + 7)^T over the HD columns of two tiles, in units of the rows' scales.  Four
+// accumulators at a time, so that the three MMAs of one are four instructions apart (a dependent MMA waits 25 cycles, an
+// independent one 9).
+template <int HD, int NN>
+__device__ __forceinline__ void at_rows_product(float (&acc)[NN][4], const __half* A, const __half* B, int r0, int lane) {
+  using C = AtCfg<HD>;
+#pragma unroll
+  for (int n = 0; n < NN; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  const __half* ap = A + (r0 + (lane & 15)) * C::LDH + (lane >> 4) * 8;
+  const __half* bp = B + (lane & 7) * C::LDH + ((lane >> 3) & 1) * 8 + (lane >> 4) * HD;
+#pragma unroll
+  for (int k = 0; k < HD; k += 16) {
+    uint32_t ah[4], al[4]; ldm4(ah, ap + k); ldm4(al, ap + HD + k);
+#pragma unroll
+    for (int n0 = 0; n0 < NN; n0 += 4) {
+      uint32_t b[4][4];
+#pragma unroll
+      for (int n = 0; n < 4; n++) ldm4(b[n], bp + (n0 + n) * 8 * C::LDH + k);
+#pragma unroll
+      for (int n = 0; n < 4; n++) mma16(acc[n0 + n], al, b[n][0], b[n][1]);
+#pragma unroll
+      for (int n = 0; n < 4; n++) mma16(acc[n0 + n], ah, b[n][2], b[n][3]);
+#pragma unroll
+      for (int n = 0; n < 4; n++) mma16(acc[n0 + n], ah, b[n][0], b[n][1]);
+    }
+  }
+}
+// out = out * keep + X B for a 16 x 8 NN accumulator fragment X and the 8 NN rows of a tile from B on, whose inverse scales `inv` are
+// taken into X here; X gets a scale per row (g, g + 8) from its maximum, so it is destroyed.
+template <int HD, int NN>
+__device__ __forceinline__ void at_sum_rows(float (&out)[HD / 8][4], float keep0, float keep1, float (&x)[NN][4], const __half* B, const float* inv, int lane) {
+  using C = AtCfg<HD>;
+  const int t = lane & 3; float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+  for (int n = 0; n < NN; n++) {
+    const float2 iv = *reinterpret_cast<const float2*>(inv + n * 8 + 2 * t);
+    x[n][0] *= iv.x; x[n][1] *= iv.y; x[n][2] *= iv.x; x[n][3] *= iv.y;
+    m0 = fmaxf(m0, fmaxf(fabsf(x[n][0]), fabsf(x[n][1]))); m1 = fmaxf(m1, fmaxf(fabsf(x[n][2]), fabsf(x[n][3])));
+  }
+  float i0, i1; const float s0 = row_scale(quad_max(m0), &i0), s1 = row_scale(quad_max(m1), &i1);
+  float acc[HD / 8][4];
+#pragma unroll
+  for (int d = 0; d < HD / 8; d++) acc[d][0] = acc[d][1] = acc[d][2] = acc[d][3] = 0.f;
+  const __half* bp = B + ((lane & 7) + ((lane >> 3) & 1) * 8) * C::LDH + (lane >> 4) * HD;
+  constexpr int DG = HD / 8 < 4 ? HD / 8 : 4;
+#pragma unroll
+  for (int k = 0; k < NN / 2; k++) {
+    uint32_t ah[4], al[4];
+    split2_pair(x[2 * k][0], x[2 * k][1], s0, ah[0], al[0]); split2_pair(x[2 * k][2], x[2 * k][3], s1, ah[1], al[1]);
+    split2_pair(x[2 * k + 1][0], x[2 * k + 1][1], s0, ah[2], al[2]); split2_pair(x[2 * k + 1][2], x[2 * k + 1][3], s1, ah[3], al[3]);
+#pragma unroll
+    for (int d0 = 0; d0 < HD / 8; d0 += DG) {
+      uint32_t b[DG][4];
+#pragma unroll
+      for (int d = 0; d < DG; d++) ldm4t(b[d], bp + k * 16 * C::LDH + (d0 + d) * 8);
+#pragma unroll
+      for (int d = 0; d < DG; d++) mma16(acc[d0 + d], al, b[d][0], b[d][1]);
+#pragma unroll
+      for (int d = 0; d < DG; d++) mma16(acc[d0 + d], ah, b[d][2], b[d][3]);
+#pragma unroll
+      for (int d = 0; d < DG; d++) mma16(acc[d0 + d], ah, b[d][0], b[d][1]);
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < HD / 8; d++) {
+    out[d][0] = fmaf(acc[d][0], i0, out[d][0] * keep0); out[d][1] = fmaf(acc[d][1], i0, out[d][1] * keep0);
+    out[d][2] = fmaf(acc[d][2], i1, out[d][2] * keep1); out[d][3] = fmaf(acc[d][3], i1, out[d][3] * keep1);
+  }
+}
+template <int HD>
+__device__ __forceinline__ void at_store(float* __restrict__ dst, const float (&v)[HD / 8][4], float f0, float f1, long base, int i0, int i1, int T, int D, int t) {
+#pragma unroll
+  for (int d = 0; d < HD / 8; d++) {
+    if (i0 < T) *reinterpret_cast<float2*>(dst + base + (long)i0 * D + d * 8 + 2 * t) = make_float2(v[d][0] * f0, v[d][1] * f0);
+    if (i1 < T) *reinterpret_cast<float2*>(dst + base + (long)i1 * D + d * 8 + 2 * t) = make_float2(v[d][2] * f1, v[d][3] * f1);
+  }
+}
 
 // ---------------------------------------------------------------- forward
 template <int HD>
 __global__ void __launch_bounds__(AT_THREADS) attn_fwd_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                                                                float* __restrict__ O, float* __restrict__ Mst, float* __restrict__ Lst,
                                                                int T, int D, int H, int causal, float inv_scale) {
-  constexpr int LD = HD + 4, NT = HD / 8;
-  extern __shared__ __align__(16) float sm[];
-  float* Qs = sm; float* Ks = Qs + AT_BLK * LD; float* Vs = Ks + AT_BLK * LD;
-  const int qb = blockIdx.x, h = blockIdx.y, b = blockIdx.z, q0 = qb * AT_BLK;
+  using C = AtCfg<HD>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  __half* Qs = reinterpret_cast<__half*>(at_sm); __half* Ks = Qs + C::TILE; __half* Vs = Ks + C::TILE;
+  float* iq = reinterpret_cast<float*>(Vs + C::TILE); float* ik = iq + AT_BLK; float* iv = ik + AT_BLK;
+  const int qb = causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x, h = blockIdx.y, b = blockIdx.z, q0 = qb * AT_BLK;      // (causal: the long rows first)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const long base = (long)b * T * D + (long)h * HD;
-  load_tile<HD>(Qs, Q, base, q0, T, D);
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-  float o[NT][4];
+  at_load<HD, false>(Qs, iq, Q, base, q0, T, D);
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[HD / 8][4];
 #pragma unroll
-  for (int i = 0; i < NT; i++) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+  for (int i = 0; i < HD / 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   const int nkb = causal ? qb + 1 : (T + AT_BLK - 1) / AT_BLK;
   const int r0 = warp * 16, i0 = q0 + r0 + g, i1 = i0 + 8;
   for (int kb = 0; kb < nkb; kb++) {
     __syncthreads();
-    load_tile<HD>(Ks, K, base, kb * AT_BLK, T, D);
-    load_tile<HD>(Vs, V, base, kb * AT_BLK, T, D);
+    at_load<HD, false>(Ks, ik, K, base, kb * AT_BLK, T, D); at_load<HD, false>(Vs, iv, V, base, kb * AT_BLK, T, D);
     __syncthreads();
-    float s[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; n++) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
-#pragma unroll
-    for (int ks = 0; ks < NT; ks++) {
-      FragA a; load_a(a, Qs, LD, r0, ks * 8, g, t);
-#pragma unroll
-      for (int n = 0; n < 8; n++) { FragB bf; load_b_nk(bf, Ks, LD, n * 8, ks * 8, g, t); mma3(s[n], a, bf); }
-    }
+    if (q0 + r0 >= T) continue;                              // (this warp's rows are all padding)
+    float s[8][4]; at_rows_product<HD, 8>(s, Qs, Ks, r0, lane);
+    const float f0 = iq[r0 + g] * inv_scale, f1 = iq[r0 + g + 8] * inv_scale;
+    const bool edge = (kb + 1) * AT_BLK > T || (causal && kb == qb);
     float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-    for (int n = 0; n < 8; n++)
+    for (int n = 0; n < 8; n++) {
+      const float2 kk = *reinterpret_cast<const float2*>(ik + n * 8 + 2 * t);
+      s[n][0] *= f0 * kk.x; s[n][1] *= f0 * kk.y; s[n][2] *= f1 * kk.x; s[n][3] *= f1 * kk.y;
+      if (edge) {
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        int j = kb * AT_BLK + n * 8 + 2 * t + (e & 1), i = (e < 2) ? i0 : i1;
-        float v = s[n][e] * inv_scale;
-        if (j >= T || (causal && j > i)) v = -INFINITY;
-        s[n][e] = v;
-        if (e < 2) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
+        for (int e = 0; e < 4; e++) { const int j = kb * AT_BLK + n * 8 + 2 * t + (e & 1); if (j >= T || (causal && j > (e < 2 ? i0 : i1))) s[n][e] = -INFINITY; }
       }
-    mx0 = quad_max(mx0); mx1 = quad_max(mx1);
-    const float mn0 = fmaxf(m[0], mx0), mn1 = fmaxf(m[1], mx1);
+      mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1])); mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
+    }
+    const float mn0 = fmaxf(m[0], quad_max(mx0)), mn1 = fmaxf(m[1], quad_max(mx1));
     const float c0 = __expf(m[0] - mn0), c1 = __expf(m[1] - mn1);
     float rs0 = 0.f, rs1 = 0.f;
 #pragma unroll
@@ -121,23 +191,11 @@ __global__ void __launch_bounds__(AT_THREADS) attn_fwd_kernel(const float* __res
       s[n][0] = __expf(s[n][0] - mn0); s[n][1] = __expf(s[n][1] - mn0); s[n][2] = __expf(s[n][2] - mn1); s[n][3] = __expf(s[n][3] - mn1);
       rs0 += s[n][0] + s[n][1]; rs1 += s[n][2] + s[n][3];
     }
-    rs0 = quad_sum(rs0); rs1 = quad_sum(rs1);
-    l[0] = l[0] * c0 + rs0; l[1] = l[1] * c1 + rs1; m[0] = mn0; m[1] = mn1;
-#pragma unroll
-    for (int d = 0; d < NT; d++) { o[d][0] *= c0; o[d][1] *= c0; o[d][2] *= c1; o[d][3] *= c1; }
-#pragma unroll
-    for (int kt = 0; kt < 8; kt++) {
-      FragA a; acc_to_a(a, s[kt]);
-#pragma unroll
-      for (int d = 0; d < NT; d++) { FragB bf; load_b_kn2(bf, Vs, LD, kt * 8, d * 8, g, t); mma3(o[d], a, bf); }
-    }
+    l[0] = l[0] * c0 + quad_sum(rs0); l[1] = l[1] * c1 + quad_sum(rs1); m[0] = mn0; m[1] = mn1;
+    at_sum_rows<HD, 8>(o, c0, c1, s, Vs, iv, lane);
   }
-  const float il0 = 1.f / l[0], il1 = 1.f / l[1];
-#pragma unroll
-  for (int d = 0; d < NT; d++) {
-    if (i0 < T) *reinterpret_cast<float2*>(O + base + (long)i0 * D + d * 8 + 2 * t) = make_float2(o[d][0] * il0, o[d][1] * il0);
-    if (i1 < T) *reinterpret_cast<float2*>(O + base + (long)i1 * D + d * 8 + 2 * t) = make_float2(o[d][2] * il1, o[d][3] * il1);
-  }
+  if (q0 + r0 >= T) return;
+  at_store<HD>(O, o, 1.f / l[0], 1.f / l[1], base, i0, i1, T, D, t);
   if (t == 0) {
     const long sb = ((long)b * H + h) * T;
     if (i0 < T) { Mst[sb + i0] = m[0]; Lst[sb + i0] = l[0]; }
@@ -145,19 +203,9 @@ __global__ void __launch_bounds__(AT_THREADS) attn_fwd_kernel(const float* __res
   }
 }
 
-// Dv[b,h,i] = sum_d dO[b,i,h*HD+d] * O[b,i,h*HD+d]   (= sum_k dP_ik P_ik, the softmax-Jacobian row term)
-__global__ void attn_rowdot_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ Dv, int T, int D, int H, int HD, long rows) {
-  long w = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); if (w >= rows) return;     // w = (b*T + i)*H + h
-  int lane = threadIdx.x & 31; int h = (int)(w % H); long tok = w / H; int i = (int)(tok % T); long b = tok / T;
-  const float* p = dO + tok * D + (long)h * HD; const float* q = O + tok * D + (long)h * HD;
-  float s = 0.f;
-  for (int d = lane; d < HD; d += 32) s = fmaf(p[d], q[d], s);
-  s = warp_sum(s);
-  if (lane == 0) Dv[(b * H + h) * T + i] = s;
-}
-
-// The same for head size 64 and D = 64 H (rows of all heads are then consecutive 64-float segments): 16 threads per row,
-// 16-byte loads, two rows in flight per thread.
+// Dv[b,h,i] = sum_d dO[b,i,h*64+d] * O[b,i,h*64+d]   (= sum_k dP_ik P_ik, the softmax-Jacobian row term), for head size 64 and
+// D = 64 H (rows of all heads are then consecutive 64-float segments): 16 threads per row, 16-byte loads, two rows in flight
+// per thread.
 __global__ void __launch_bounds__(256) attn_rowdot64_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ Dv, int T, int H, long rows) {
   const long gid = (long)blockIdx.x * 256 + threadIdx.x, half = (long)gridDim.x * 16;      // rows per pass of the grid
   const int l16 = threadIdx.x & 15;
@@ -176,141 +224,103 @@ __global__ void __launch_bounds__(256) attn_rowdot64_kernel(const float* __restr
   }
 }
 
-
-// ---------------------------------------------------------------- backward: dQ
-// One CTA = 64 query rows; for every key block at or below the diagonal: S = Q K^T, P = exp(S/sqrt(hd) - m) / l,
-// dP = dO V^T, dS = P (dP - Dv) / sqrt(hd), dQ += dS K.
+// ---------------------------------------------------------------- backward
+// The first half of the grid's blocks: dQ of 64 query rows.  For every key block at or below the diagonal: S = Q K^T,
+// P = exp(S/sqrt(hd) - m) / l, dP = dO V^T, dS = P (dP - dO . O) / sqrt(hd), dQ += dS K.
+// The second half: dK and dV of 64 key rows.  For every query block at or above the diagonal the TRANSPOSED tiles are formed
+// directly: S^T = K Q^T, P^T, dP^T = V dO^T, dS^T; dK += dS^T Q, dV += P^T dO.
+// One launch, so that a few hundred blocks of either kind fill the SMs together; dO . O is formed while dO is loaded.
 template <int HD>
-__global__ void __launch_bounds__(AT_THREADS) attn_bwd_dq_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
-                                                                  const float* __restrict__ dO, const float* __restrict__ Mst, const float* __restrict__ Lst,
-                                                                  const float* __restrict__ Dv, float* __restrict__ dQ, int T, int D, int H, int causal, float inv_scale) {
-  constexpr int LD = HD + 4, NT = HD / 8;
-  extern __shared__ __align__(16) float sm[];
-  float* Qs = sm; float* Gs = Qs + AT_BLK * LD; float* Ks = Gs + AT_BLK * LD; float* Vs = Ks + AT_BLK * LD;
-  const int qb = blockIdx.x, h = blockIdx.y, b = blockIdx.z, q0 = qb * AT_BLK;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+__global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 3 : 4) attn_bwd_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ O,
+                                                              const float* __restrict__ dO, const float* __restrict__ Mst, const float* __restrict__ Lst,
+                                                              float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV, int T, int D, int H, int causal, float inv_scale) {
+  using C = AtCfg<HD>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  __half* Qs = reinterpret_cast<__half*>(at_sm); __half* Gs = Qs + C::TILE; __half* Ks = Gs + C::TILE; __half* Vs = Ks + C::TILE;
+  float* iq = reinterpret_cast<float*>(Vs + C::TILE); float* ig = iq + AT_BLK; float* ik = ig + AT_BLK; float* iv = ik + AT_BLK;
+  float* st_m = iv + AT_BLK; float* st_il = st_m + AT_BLK; float* st_d = st_il + AT_BLK;
+  const int nb = (T + AT_BLK - 1) / AT_BLK, h = blockIdx.y, b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, r0 = warp * 16;
   const long base = (long)b * T * D + (long)h * HD, sb = ((long)b * H + h) * T;
-  load_tile<HD>(Qs, Q, base, q0, T, D);
-  load_tile<HD>(Gs, dO, base, q0, T, D);
-  const int r0 = warp * 16, i0 = q0 + r0 + g, i1 = i0 + 8;
-  const float m0 = i0 < T ? Mst[sb + i0] : 0.f, m1 = i1 < T ? Mst[sb + i1] : 0.f;
-  const float il0 = i0 < T ? 1.f / Lst[sb + i0] : 0.f, il1 = i1 < T ? 1.f / Lst[sb + i1] : 0.f;
-  const float d0 = i0 < T ? Dv[sb + i0] : 0.f, d1 = i1 < T ? Dv[sb + i1] : 0.f;
-  float acc[NT][4];
-#pragma unroll
-  for (int i = 0; i < NT; i++) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f; }
-  const int nkb = causal ? qb + 1 : (T + AT_BLK - 1) / AT_BLK;
-  for (int kb = 0; kb < nkb; kb++) {
+  if (blockIdx.x < nb) {
+    const int qb = nb - 1 - blockIdx.x, q0 = qb * AT_BLK;
+    at_load<HD, false>(Qs, iq, Q, base, q0, T, D); at_load<HD, true>(Gs, ig, dO, base, q0, T, D, O, st_d);
     __syncthreads();
-    load_tile<HD>(Ks, K, base, kb * AT_BLK, T, D);
-    load_tile<HD>(Vs, V, base, kb * AT_BLK, T, D);
-    __syncthreads();
-    float s[8][4], dp[8][4];
+    const int i0 = q0 + r0 + g, i1 = i0 + 8;
+    const float m0 = i0 < T ? Mst[sb + i0] : 0.f, m1 = i1 < T ? Mst[sb + i1] : 0.f;
+    const float il0 = i0 < T ? 1.f / Lst[sb + i0] : 0.f, il1 = i1 < T ? 1.f / Lst[sb + i1] : 0.f;
+    const float d0 = st_d[r0 + g], d1 = st_d[r0 + g + 8], f0 = iq[r0 + g] * inv_scale, f1 = iq[r0 + g + 8] * inv_scale, g0 = ig[r0 + g], g1 = ig[r0 + g + 8];
+    float acc[HD / 8][4];
 #pragma unroll
-    for (int n = 0; n < 8; n++) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; dp[n][0] = dp[n][1] = dp[n][2] = dp[n][3] = 0.f; }
+    for (int i = 0; i < HD / 8; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    const int nkb = causal ? qb + 1 : nb;
+    for (int kb = 0; kb < nkb; kb++) {
+      __syncthreads();
+      at_load<HD, false>(Ks, ik, K, base, kb * AT_BLK, T, D); at_load<HD, false>(Vs, iv, V, base, kb * AT_BLK, T, D);
+      __syncthreads();
+      if (q0 + r0 >= T) continue;
+      const bool edge = (kb + 1) * AT_BLK > T || (causal && kb == qb);
+#pragma unroll 1
+      for (int kh = 0; kh < AT_BLK; kh += 32) {              // 32 keys at a time: half the accumulators of a whole block
+        if (kb * AT_BLK + kh >= T) break;
+        float s[4][4], dp[4][4]; at_rows_product<HD, 4>(s, Qs, Ks + kh * C::LDH, r0, lane); at_rows_product<HD, 4>(dp, Gs, Vs + kh * C::LDH, r0, lane);
 #pragma unroll
-    for (int ks = 0; ks < NT; ks++) {
-      FragA a, ga; load_a(a, Qs, LD, r0, ks * 8, g, t); load_a(ga, Gs, LD, r0, ks * 8, g, t);
+        for (int n = 0; n < 4; n++) {
+          const float2 kk = *reinterpret_cast<const float2*>(ik + kh + n * 8 + 2 * t), vv = *reinterpret_cast<const float2*>(iv + kh + n * 8 + 2 * t);
 #pragma unroll
-      for (int n = 0; n < 8; n++) {
-        FragB bf; load_b_nk(bf, Ks, LD, n * 8, ks * 8, g, t); mma3(s[n], a, bf);
-        load_b_nk(bf, Vs, LD, n * 8, ks * 8, g, t); mma3(dp[n], ga, bf);
+          for (int e = 0; e < 4; e++) {
+            const float fk = e & 1 ? kk.y : kk.x, fv = e & 1 ? vv.y : vv.x;
+            const int j = kb * AT_BLK + kh + n * 8 + 2 * t + (e & 1), i = e < 2 ? i0 : i1;
+            const float p = edge && (j >= T || (causal && j > i)) ? 0.f : __expf(s[n][e] * ((e < 2 ? f0 : f1) * fk) - (e < 2 ? m0 : m1)) * (e < 2 ? il0 : il1);      // (rows beyond T: il = 0)
+            s[n][e] = p * (dp[n][e] * ((e < 2 ? g0 : g1) * fv) - (e < 2 ? d0 : d1)) * inv_scale;        // dS
+          }
+        }
+        at_sum_rows<HD, 4>(acc, 1.f, 1.f, s, Ks + kh * C::LDH, ik + kh, lane);
       }
     }
-#pragma unroll
-    for (int n = 0; n < 8; n++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int j = kb * AT_BLK + n * 8 + 2 * t + (e & 1), i = (e < 2) ? i0 : i1;
-        const bool masked = j >= T || i >= T || (causal && j > i);
-        const float p = masked ? 0.f : __expf(s[n][e] * inv_scale - (e < 2 ? m0 : m1)) * (e < 2 ? il0 : il1);
-        s[n][e] = p * (dp[n][e] - (e < 2 ? d0 : d1)) * inv_scale;        // dS
-      }
-#pragma unroll
-    for (int kt = 0; kt < 8; kt++) {
-      FragA a; acc_to_a(a, s[kt]);
-#pragma unroll
-      for (int d = 0; d < NT; d++) { FragB bf; load_b_kn2(bf, Ks, LD, kt * 8, d * 8, g, t); mma3(acc[d], a, bf); }
-    }
+    at_store<HD>(dQ, acc, 1.f, 1.f, base, i0, i1, T, D, t);
+    return;
   }
+  const int kbk = blockIdx.x - nb, k0 = kbk * AT_BLK;
+  at_load<HD, false>(Ks, ik, K, base, k0, T, D); at_load<HD, false>(Vs, iv, V, base, k0, T, D);
+  __syncthreads();
+  const int j0 = k0 + r0 + g, j1 = j0 + 8;
+  const float f0 = ik[r0 + g] * inv_scale, f1 = ik[r0 + g + 8] * inv_scale, v0 = iv[r0 + g], v1 = iv[r0 + g + 8];
+  float ak[HD / 8][4], av[HD / 8][4];
 #pragma unroll
-  for (int d = 0; d < NT; d++) {
-    if (i0 < T) *reinterpret_cast<float2*>(dQ + base + (long)i0 * D + d * 8 + 2 * t) = make_float2(acc[d][0], acc[d][1]);
-    if (i1 < T) *reinterpret_cast<float2*>(dQ + base + (long)i1 * D + d * 8 + 2 * t) = make_float2(acc[d][2], acc[d][3]);
-  }
-}
-
-// ---------------------------------------------------------------- backward: dK, dV
-// One CTA = 64 key rows; for every query block at or above the diagonal the TRANSPOSED tiles are formed directly:
-// S^T = K Q^T, P^T, dP^T = V dO^T, dS^T = P^T (dP^T - Dv[query]) / sqrt(hd); dK += dS^T Q, dV += P^T dO.
-template <int HD>
-__global__ void __launch_bounds__(AT_THREADS) attn_bwd_dkv_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
-                                                                   const float* __restrict__ dO, const float* __restrict__ Mst, const float* __restrict__ Lst,
-                                                                   const float* __restrict__ Dv, float* __restrict__ dK, float* __restrict__ dV,
-                                                                   int T, int D, int H, int causal, float inv_scale) {
-  constexpr int LD = HD + 4, NT = HD / 8;
-  extern __shared__ __align__(16) float sm[];
-  float* Ks = sm; float* Vs = Ks + AT_BLK * LD; float* Qs = Vs + AT_BLK * LD; float* Gs = Qs + AT_BLK * LD;
-  float* st_m = Gs + AT_BLK * LD; float* st_il = st_m + AT_BLK; float* st_d = st_il + AT_BLK;
-  const int kbk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, k0 = kbk * AT_BLK;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const long base = (long)b * T * D + (long)h * HD, sb = ((long)b * H + h) * T;
-  load_tile<HD>(Ks, K, base, k0, T, D);
-  load_tile<HD>(Vs, V, base, k0, T, D);
-  const int r0 = warp * 16, j0 = k0 + r0 + g, j1 = j0 + 8;
-  float ak[NT][4], av[NT][4];
-#pragma unroll
-  for (int i = 0; i < NT; i++) { ak[i][0] = ak[i][1] = ak[i][2] = ak[i][3] = 0.f; av[i][0] = av[i][1] = av[i][2] = av[i][3] = 0.f; }
-  const int nqb = (T + AT_BLK - 1) / AT_BLK;
-  for (int qb = causal ? kbk : 0; qb < nqb; qb++) {
+  for (int i = 0; i < HD / 8; i++) { ak[i][0] = ak[i][1] = ak[i][2] = ak[i][3] = 0.f; av[i][0] = av[i][1] = av[i][2] = av[i][3] = 0.f; }
+  for (int qb = causal ? kbk : 0; qb < nb; qb++) {
     __syncthreads();
-    load_tile<HD>(Qs, Q, base, qb * AT_BLK, T, D);
-    load_tile<HD>(Gs, dO, base, qb * AT_BLK, T, D);
+    at_load<HD, false>(Qs, iq, Q, base, qb * AT_BLK, T, D); at_load<HD, true>(Gs, ig, dO, base, qb * AT_BLK, T, D, O, st_d);
     if (threadIdx.x < AT_BLK) {
       const int i = qb * AT_BLK + threadIdx.x;
-      st_m[threadIdx.x] = i < T ? Mst[sb + i] : 0.f; st_il[threadIdx.x] = i < T ? 1.f / Lst[sb + i] : 0.f; st_d[threadIdx.x] = i < T ? Dv[sb + i] : 0.f;
+      st_m[threadIdx.x] = i < T ? Mst[sb + i] : 0.f; st_il[threadIdx.x] = i < T ? 1.f / Lst[sb + i] : 0.f;
     }
     __syncthreads();
-    float s[8][4], dp[8][4];
+    if (k0 + r0 >= T) continue;
+    const bool edge = k0 + AT_BLK > T || (causal && kbk == qb);
+    // rows = keys j (g, g+8), columns = queries i (2t, 2t+1 of n-tile n), 32 queries at a time
+#pragma unroll 1
+    for (int qh = 0; qh < AT_BLK; qh += 32) {
+      if (qb * AT_BLK + qh >= T) break;
+      float s[4][4], dp[4][4]; at_rows_product<HD, 4>(s, Ks, Qs + qh * C::LDH, r0, lane); at_rows_product<HD, 4>(dp, Vs, Gs + qh * C::LDH, r0, lane);
 #pragma unroll
-    for (int n = 0; n < 8; n++) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; dp[n][0] = dp[n][1] = dp[n][2] = dp[n][3] = 0.f; }
+      for (int n = 0; n < 4; n++) {
+        const int c0 = qh + n * 8 + 2 * t;
+        const float2 qq = *reinterpret_cast<const float2*>(iq + c0), gg = *reinterpret_cast<const float2*>(ig + c0), mm = *reinterpret_cast<const float2*>(st_m + c0),
+                     ll = *reinterpret_cast<const float2*>(st_il + c0), dd = *reinterpret_cast<const float2*>(st_d + c0);
 #pragma unroll
-    for (int ks = 0; ks < NT; ks++) {
-      FragA a, va; load_a(a, Ks, LD, r0, ks * 8, g, t); load_a(va, Vs, LD, r0, ks * 8, g, t);
-#pragma unroll
-      for (int n = 0; n < 8; n++) {
-        FragB bf; load_b_nk(bf, Qs, LD, n * 8, ks * 8, g, t); mma3(s[n], a, bf);
-        load_b_nk(bf, Gs, LD, n * 8, ks * 8, g, t); mma3(dp[n], va, bf);
+        for (int e = 0; e < 4; e++) {
+          const int i = qb * AT_BLK + c0 + (e & 1), j = e < 2 ? j0 : j1;
+          const float p = edge && (j >= T || (causal && j > i)) ? 0.f : __expf(s[n][e] * ((e < 2 ? f0 : f1) * (e & 1 ? qq.y : qq.x)) - (e & 1 ? mm.y : mm.x)) * (e & 1 ? ll.y : ll.x);      // (columns beyond T: il = 0)
+          dp[n][e] = p * (dp[n][e] * ((e < 2 ? v0 : v1) * (e & 1 ? gg.y : gg.x)) - (e & 1 ? dd.y : dd.x)) * inv_scale;      // dS^T
+          s[n][e] = p;                                                                                                     // P^T
+        }
       }
-    }
-    // rows = keys j (g, g+8), columns = queries i (2t, 2t+1 of n-tile n)
-#pragma unroll
-    for (int n = 0; n < 8; n++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int ci = n * 8 + 2 * t + (e & 1), i = qb * AT_BLK + ci, j = (e < 2) ? j0 : j1;
-        const bool masked = j >= T || i >= T || (causal && j > i);
-        const float p = masked ? 0.f : __expf(s[n][e] * inv_scale - st_m[ci]) * st_il[ci];
-        dp[n][e] = p * (dp[n][e] - st_d[ci]) * inv_scale;                 // dS^T
-        s[n][e] = p;                                                     // P^T
-      }
-#pragma unroll
-    for (int kt = 0; kt < 8; kt++) {
-      FragA ap, ads; acc_to_a(ap, s[kt]); acc_to_a(ads, dp[kt]);
-#pragma unroll
-      for (int d = 0; d < NT; d++) {
-        FragB bf; load_b_kn2(bf, Qs, LD, kt * 8, d * 8, g, t); mma3(ak[d], ads, bf);
-        load_b_kn2(bf, Gs, LD, kt * 8, d * 8, g, t); mma3(av[d], ap, bf);
-      }
+      at_sum_rows<HD, 4>(av, 1.f, 1.f, s, Gs + qh * C::LDH, ig + qh, lane); at_sum_rows<HD, 4>(ak, 1.f, 1.f, dp, Qs + qh * C::LDH, iq + qh, lane);
     }
   }
-#pragma unroll
-  for (int d = 0; d < NT; d++) {
-    if (j0 < T) { *reinterpret_cast<float2*>(dK + base + (long)j0 * D + d * 8 + 2 * t) = make_float2(ak[d][0], ak[d][1]);
-                  *reinterpret_cast<float2*>(dV + base + (long)j0 * D + d * 8 + 2 * t) = make_float2(av[d][0], av[d][1]); }
-    if (j1 < T) { *reinterpret_cast<float2*>(dK + base + (long)j1 * D + d * 8 + 2 * t) = make_float2(ak[d][2], ak[d][3]);
-                  *reinterpret_cast<float2*>(dV + base + (long)j1 * D + d * 8 + 2 * t) = make_float2(av[d][2], av[d][3]); }
-  }
+  at_store<HD>(dK, ak, 1.f, 1.f, base, j0, j1, T, D, t); at_store<HD>(dV, av, 1.f, 1.f, base, j0, j1, T, D, t);
 }
 
 // ---------------------------------------------------------------- a few query rows
@@ -425,23 +435,17 @@ inline bool attn_fused_supported(int hd, int D) { return (hd == 16 || hd == 32 |
 
 template <int HD>
 inline int attn_fwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
-  size_t smem = (size_t)3 * AT_BLK * (HD + 4) * sizeof(float);
-  GN_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int smem = 3 * AtCfg<HD>::TILE * (int)sizeof(__half) + 3 * AT_BLK * (int)sizeof(float);
+  GN_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, attn_fwd_kernel<HD>, dim3(cdiv(T, AT_BLK), H, B), AT_THREADS, smem, Q, K, V, O, M, L, T, D, H, causal, 1.f / sqrtf((float)HD));
   return check_launch("attn_fwd");
 }
 template <int HD>
-inline int attn_bwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L, float* Dv,
+inline int attn_bwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
                            float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
-  const float inv_scale = 1.f / sqrtf((float)HD);
-  long rows = (long)B * T * H;
-  GN_LAUNCH(ctx, attn_rowdot_kernel, cdiv(rows, 8), 256, 0, dO, O, Dv, T, D, H, HD, rows);
-  size_t smem_q = (size_t)4 * AT_BLK * (HD + 4) * sizeof(float), smem_kv = smem_q + 3 * AT_BLK * sizeof(float);
-  GN_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q));
-  GN_CUDA(cudaFuncSetAttribute(attn_bwd_dkv_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-  dim3 grid(cdiv(T, AT_BLK), H, B);
-  GN_LAUNCH(ctx, attn_bwd_dq_kernel<HD>, grid, AT_THREADS, smem_q, Q, K, V, dO, M, L, Dv, dQ, T, D, H, causal, inv_scale);
-  GN_LAUNCH(ctx, attn_bwd_dkv_kernel<HD>, grid, AT_THREADS, smem_kv, Q, K, V, dO, M, L, Dv, dK, dV, T, D, H, causal, inv_scale);
+  const int smem = 4 * AtCfg<HD>::TILE * (int)sizeof(__half) + 7 * AT_BLK * (int)sizeof(float);
+  GN_CUDA(cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  GN_LAUNCH(ctx, attn_bwd_kernel<HD>, dim3(2 * cdiv(T, AT_BLK), H, B), AT_THREADS, smem, Q, K, V, O, dO, M, L, dQ, dK, dV, T, D, H, causal, 1.f / sqrtf((float)HD));
   return check_launch("attn_bwd");
 }
 inline int attn_fwd(Ctx* ctx, int hd, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
@@ -449,11 +453,11 @@ inline int attn_fwd(Ctx* ctx, int hd, const float* Q, const float* K, const floa
   if (hd == 32) return attn_fwd_launch<32>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
   return attn_fwd_launch<16>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
 }
-inline int attn_bwd(Ctx* ctx, int hd, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L, float* Dv,
+inline int attn_bwd(Ctx* ctx, int hd, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
                     float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
-  if (hd == 64) return attn_bwd_launch<64>(ctx, Q, K, V, O, dO, M, L, Dv, dQ, dK, dV, B, T, D, H, causal);
-  if (hd == 32) return attn_bwd_launch<32>(ctx, Q, K, V, O, dO, M, L, Dv, dQ, dK, dV, B, T, D, H, causal);
-  return attn_bwd_launch<16>(ctx, Q, K, V, O, dO, M, L, Dv, dQ, dK, dV, B, T, D, H, causal);
+  if (hd == 64) return attn_bwd_launch<64>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
+  if (hd == 32) return attn_bwd_launch<32>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
+  return attn_bwd_launch<16>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
 }
 
 }  // namespace gn

@@ -975,7 +975,7 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   if (fused) {
     static const bool tc_bwd = [] { const char* e = getenv("GONEURON_CUDA_ATTENTION_BWD"); return !(e && !strcmp(e, "mma")); }();
     if (tc_bwd && attn_tc_supported(ctx, hd, T, B, Hh, D)) GN_TRY(attn_tc_bwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, dA, l.att_m.p, l.att_l.p, l.att_d.p, dQ, dK, dV, B, T, D, Hh, d.causal, &l.attn_saved));
-    else GN_TRY(attn_bwd(ctx, hd, l.q.p, l.k.p, l.v.p, l.att.p, dA, l.att_m.p, l.att_l.p, l.att_d.p, dQ, dK, dV, B, T, D, Hh, d.causal));
+    else GN_TRY(attn_bwd(ctx, hd, l.q.p, l.k.p, l.v.p, l.att.p, dA, l.att_m.p, l.att_l.p, dQ, dK, dV, B, T, D, Hh, d.causal));
   } else {
     const long TD = (long)T * D, TT = (long)T * T; const float inv_scale = 1.f / sqrtf((float)hd); const long rows = (long)B * Hh * T;
     GemmDesc g; g.M = T; g.N = T; g.K = hd; g.A = l.q.p; g.sa_m = D; g.sa_k = 1; g.B = l.k.p; g.sb_k = 1; g.sb_n = D;
@@ -1906,7 +1906,7 @@ int gn_op_attention(gn_ctx* ctx, int engine, int B, int T, int D, int H, int cau
     GN_TRY(g.alloc(n)); GN_TRY(dv_.alloc(ns)); GN_TRY(dq.alloc(n)); GN_TRY(dk.alloc(n)); GN_TRY(dvv.alloc(n));
     GN_CUDA(copy_h2d(c, g.p, dO, n * 4));
     if (engine == 1) GN_TRY(attn_tc_bwd(c, q.p, k.p, v.p, o.p, g.p, m.p, l.p, dv_.p, dq.p, dk.p, dvv.p, B, T, D, H, causal));
-    else GN_TRY(attn_bwd(c, hd, q.p, k.p, v.p, o.p, g.p, m.p, l.p, dv_.p, dq.p, dk.p, dvv.p, B, T, D, H, causal));
+    else GN_TRY(attn_bwd(c, hd, q.p, k.p, v.p, o.p, g.p, m.p, l.p, dq.p, dk.p, dvv.p, B, T, D, H, causal));
     GN_CUDA(copy_d2h(c, dQ, dq.p, n * 4)); GN_CUDA(copy_d2h(c, dK, dk.p, n * 4)); GN_CUDA(copy_d2h(c, dV, dvv.p, n * 4));
   }
   GN_CUDA(copy_d2h(c, O, o.p, n * 4));
