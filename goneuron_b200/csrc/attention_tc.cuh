@@ -597,37 +597,23 @@ __global__ void __launch_bounds__(256) attn_prep_max_kernel(const AttnPrepJobs j
   __shared__ float red[33];
   const AttnPrepJob& jb = jobs.j[blockIdx.z];
   const int z = blockIdx.y, b = z / H, h = z % H, t0 = blockIdx.x * 64, i = threadIdx.x, c4 = i & 15, r0 = i >> 4;
-  float m = 0.f, nm = 0.f;
+  float m = 0.f;
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    const int row = r0 + 16 * r;
-    const float4 x = *reinterpret_cast<const float4*>(jb.X + ((long)b * T + t0 + row) * D + (long)h * 64 + c4 * 4);
+    const float4 x = *reinterpret_cast<const float4*>(jb.X + ((long)b * T + t0 + r0 + 16 * r) * D + (long)h * 64 + c4 * 4);
     m = fmaxf(m, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-    if (jb.rnorm) {                                        // 16 consecutive lanes hold one row
-      float sq = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      const float nr = sqrtf(sq) * 1.0001f;
-      if (c4 == 0) jb.rnorm[(long)z * T + t0 + row] = nr;
-      nm = fmaxf(nm, nr);
-    }
   }
   m = block_max(m, red);
   if (i == 0) { if (!(m <= 3.0e38f)) m = 3.4e38f; atomicMax(jb.amax + z, __float_as_int(m)); }
-  if (jb.rnorm) {
-    __syncthreads();
-    nm = block_max(nm, red);
-    if (i == 0) { if (!(nm <= 3.0e38f)) nm = 3.4e38f; atomicMax(jb.nmax + z, __float_as_int(nm)); }
-  }
 }
 __global__ void __launch_bounds__(256) attn_prep_split_kernel(const AttnPrepJobs jobs, int T, int D, int H) {
-  __shared__ float tile[64][65];
+  __shared__ float tile[64][65], red[33];
   const AttnPrepJob& jb = jobs.j[blockIdx.z];
   const int z = blockIdx.y, b = z / H, h = z % H, t0 = blockIdx.x * 64, i = threadIdx.x;
   const int c4 = i & 15, r0 = i >> 4;
   float inv; const float s = row_scale(__int_as_float(jb.amax[z]), &inv);
   if (blockIdx.x == 0 && i == 0) jb.inv[z] = inv;
-  float4 x[4];
+  float4 x[4]; float nm = 0.f;
 #pragma unroll
   for (int r = 0; r < 4; r++) x[r] = *reinterpret_cast<const float4*>(jb.X + ((long)b * T + t0 + r0 + 16 * r) * D + (long)h * 64 + c4 * 4);
 #pragma unroll
@@ -637,6 +623,14 @@ __global__ void __launch_bounds__(256) attn_prep_split_kernel(const AttnPrepJobs
       uint2 hi, lo; split2_pair(x[r].x, x[r].y, s, hi.x, lo.x); split2_pair(x[r].z, x[r].w, s, hi.y, lo.y);
       const long o = ((long)z * T + t0 + row) * 64 + c4 * 4;
       *reinterpret_cast<uint2*>(jb.rh + o) = hi; *reinterpret_cast<uint2*>(jb.rl + o) = lo;
+    }
+    if (jb.rnorm) {                                          // 16 consecutive lanes hold one row
+      float sq = x[r].x * x[r].x + x[r].y * x[r].y + x[r].z * x[r].z + x[r].w * x[r].w;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      const float nr = sqrtf(sq) * 1.0001f;
+      if (c4 == 0) jb.rnorm[(long)z * T + t0 + row] = nr;
+      nm = fmaxf(nm, nr);
     }
     if (jb.ch) { tile[row][c4 * 4] = x[r].x; tile[row][c4 * 4 + 1] = x[r].y; tile[row][c4 * 4 + 2] = x[r].z; tile[row][c4 * 4 + 3] = x[r].w; }
   }
@@ -649,6 +643,10 @@ __global__ void __launch_bounds__(256) attn_prep_split_kernel(const AttnPrepJobs
       const long o = ((long)z * 64 + d) * T + t0 + c4 * 4;
       *reinterpret_cast<uint2*>(jb.ch + o) = hi; *reinterpret_cast<uint2*>(jb.cl + o) = lo;
     }
+  }
+  if (jb.rnorm) {
+    nm = block_max(nm, red);
+    if (i == 0) { if (!(nm <= 3.0e38f)) nm = 3.4e38f; atomicMax(jb.nmax + z, __float_as_int(nm)); }
   }
 }
 // per problem, max |Dv| (a factor of the key-side dS bound)
@@ -688,12 +686,12 @@ inline bool attn_keep_planes() { static const bool on = [] { const char* e = get
 // norms), or, when `store` is given, that buffer (planes of tensor i at (2 i) ne and (2 i + 1) ne, then words, then norms).
 inline size_t attn_store_floats(int n, int Z, int T) { return (size_t)2 * n * Z * T * ATC_HD + (size_t)Z * 16 + (size_t)Z * T * 2; }
 inline int attn_tc_prepare(Ctx* ctx, int n, const float* const* X, const bool* want_rows, const bool* want_cols, const bool* want_norm, AttnPlanes* out,
-                           int B, int T, int D, int H, int** zwords_extra, float* store = nullptr) {
+                           int B, int T, int D, int H, int** zwords_extra, float* store = nullptr, bool have_max = false) {
   const int Z = B * H; const size_t ne = (size_t)Z * T * ATC_HD;      // elements of a tensor; hi + lo planes = ne floats
   float *words, *norms;
   if (store) { words = store + (size_t)2 * n * ne; norms = words + (size_t)Z * 16; }
   else { GN_TRY(attn_tc_buf(ctx, 8, (size_t)Z * 16, &words)); GN_TRY(attn_tc_buf(ctx, 9, (size_t)Z * T * 2, &norms)); }   // per tensor: amax, inv, nmax; one extra row for the caller
-  GN_CUDA(cudaMemsetAsync(words, 0, (size_t)Z * 16 * sizeof(float), ctx->stream));
+  if (!have_max) GN_CUDA(cudaMemsetAsync(words, 0, (size_t)Z * 16 * sizeof(float), ctx->stream));
   AttnPrepJobs jobs{}; int nn = 0;
   for (int i = 0; i < n; i++) {
     AttnPrepJob& j = jobs.j[i]; j.X = X[i];
@@ -708,7 +706,7 @@ inline int attn_tc_prepare(Ctx* ctx, int n, const float* const* X, const bool* w
   }
   if (zwords_extra) *zwords_extra = reinterpret_cast<int*>(words) + (size_t)12 * Z;
   const dim3 grid(T / 64, Z, n);
-  GN_LAUNCH(ctx, attn_prep_max_kernel, grid, 256, 0, jobs, T, D, H);
+  if (!have_max) GN_LAUNCH(ctx, attn_prep_max_kernel, grid, 256, 0, jobs, T, D, H);
   GN_LAUNCH(ctx, attn_prep_split_kernel, grid, 256, 0, jobs, T, D, H);
   return check_launch("attn_prep");
 }
@@ -721,26 +719,41 @@ inline int attn_tc_maps_cols(Ctx* ctx, CUtensorMap* m, const AttnPlanes& p, int 
   GN_TRY(tc_make_map_f16(ctx, &m[0], p.ch, T, ATC_HD, T, Z, ATC_HD));
   return tc_make_map_f16(ctx, &m[1], p.cl, T, ATC_HD, T, Z, ATC_HD);
 }
+// Where a forward pass puts the planes of Q, K and V: the layer's own store when a backward pass will want them and there is room.
+inline int attn_tc_store(Ctx* ctx, AttnSaved* save, int Z, int T, float** store) {
+  *store = nullptr;
+  if (!save) return GN_OK;
+  save->valid = false;
+  if (!attn_keep_planes()) return GN_OK;
+  const size_t need = attn_store_floats(3, Z, T);
+  if (save->store.n < need) {
+    GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++;
+    if (save->store.alloc(need) != GN_OK) { cudaGetLastError(); return GN_OK; }      // no room: the backward pass prepares its own operands
+  }
+  *store = save->store.p; return GN_OK;
+}
+// The largest magnitude per problem of Q, K and V can come from the epilogue of the contraction that makes them (TcParams::zmax)
+// instead of a pass over all three: this returns the zeroed words it belongs in ([tensor][Z], 3 Z apart).
+inline int attn_tc_max_words(Ctx* ctx, AttnSaved* save, int Z, int T, int** words) {
+  float *store, *w; GN_TRY(attn_tc_store(ctx, save, Z, T, &store));
+  if (store) w = store + (size_t)6 * Z * T * ATC_HD; else GN_TRY(attn_tc_buf(ctx, 8, (size_t)Z * 16, &w));
+  GN_CUDA(cudaMemsetAsync(w, 0, (size_t)Z * 16 * sizeof(float), ctx->stream));
+  *words = reinterpret_cast<int*>(w); return GN_OK;
+}
 inline int attn_tc_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal,
-                       AttnSaved* save = nullptr) {
+                       AttnSaved* save = nullptr, bool have_max = false) {
   const int Z = B * H;
   const float* X[3] = {Q, K, V};
-  AttnPlanes p[3];
-  if (save) save->valid = false;
-  if (save && attn_keep_planes()) {
-    const size_t need = attn_store_floats(3, Z, T);
-    if (save->store.n < need) {
-      GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++;
-      if (save->store.alloc(need) != GN_OK) { cudaGetLastError(); save = nullptr; }      // no room: the backward pass prepares its own operands
-    }
-  } else save = nullptr;
+  AttnPlanes p[3]; float* store;
+  GN_TRY(attn_tc_store(ctx, save, Z, T, &store));
+  if (!store) save = nullptr;
   if (save) {
     const bool all[3] = {true, true, true}, norm[3] = {false, false, true};
-    GN_TRY(attn_tc_prepare(ctx, 3, X, all, all, norm, p, B, T, D, H, nullptr, save->store.p));
+    GN_TRY(attn_tc_prepare(ctx, 3, X, all, all, norm, p, B, T, D, H, nullptr, store, have_max));
     save->q = p[0]; save->k = p[1]; save->v = p[2]; save->B = B; save->valid = true;
   } else {
     const bool rows[3] = {true, true, false}, cols[3] = {false, false, true}, norm[3] = {false, false, false};
-    GN_TRY(attn_tc_prepare(ctx, 3, X, rows, cols, norm, p, B, T, D, H, nullptr));
+    GN_TRY(attn_tc_prepare(ctx, 3, X, rows, cols, norm, p, B, T, D, H, nullptr, nullptr, have_max));
   }
   AttnMaps<6> maps;
   GN_TRY(attn_tc_maps_rows(ctx, &maps.m[0], p[0], T, Z, ATC_BQ)); GN_TRY(attn_tc_maps_rows(ctx, &maps.m[2], p[1], T, Z, ATC_BK)); GN_TRY(attn_tc_maps_cols(ctx, &maps.m[4], p[2], T, Z));

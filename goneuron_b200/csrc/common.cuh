@@ -31,6 +31,7 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t comm_stream = nullptr;   // gradient all-reduces run here, overlapped with the rest of the backward pass
   cudaStream_t copy_stream = nullptr; cudaEvent_t copy_ev = nullptr;      // targets of a large host batch, copied under the forward pass
+  cudaStream_t side_stream = nullptr; cudaEvent_t fork_ev = nullptr, join_ev = nullptr; bool side_pending = false;      // see side_run()
   int rank = 0, world = 1;
   void* comm = nullptr;            // ncclComm_t
   NcclApi* nccl = nullptr;
@@ -67,6 +68,26 @@ struct Ctx {
 };
 
 inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
+
+// Runs `f` (launches on ctx->stream) on the side stream, beside what the main stream does next.  A parameter gradient is read by nothing
+// before the update, while the gradient of the layer's input is the one thing the next layer waits for: a step of small
+// kernels is a chain of those, and the parameter gradients need not be links of it.  `f` must not use the contraction
+// engine's scratch or any buffer that the main stream writes before side_join(), which the backward pass calls after every layer.
+template <class F> inline int side_run(Ctx* ctx, F&& f) {
+  if (!ctx->side_stream || ctx->profile) return f();         // (profiling times the contractions one by one)
+  if (cudaEventRecord(ctx->fork_ev, ctx->stream) != cudaSuccess || cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0) != cudaSuccess)
+    return fail(GN_ERR_CUDA, "side stream: %s", cudaGetErrorString(cudaGetLastError()));
+  cudaStream_t main = ctx->stream; ctx->stream = ctx->side_stream; ctx->side_pending = true;
+  const int rc = f();
+  ctx->stream = main; return rc;
+}
+inline int side_join(Ctx* ctx) {
+  if (!ctx->side_pending) return GN_OK;
+  ctx->side_pending = false;
+  if (cudaEventRecord(ctx->join_ev, ctx->side_stream) != cudaSuccess || cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0) != cudaSuccess)
+    return fail(GN_ERR_CUDA, "side stream: %s", cudaGetErrorString(cudaGetLastError()));
+  return GN_OK;
+}
 
 // Every kernel launch of the library goes through these macros, so that the launch count is exact.
 // launch_kernel(): `cluster` > 0: that many neighbouring blocks of the grid's x dimension form a thread-block cluster; `early`: the

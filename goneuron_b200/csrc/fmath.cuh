@@ -76,10 +76,12 @@ __host__ __device__ __forceinline__ float tanh_rn(float x) {
 }
 
 // GELU, tanh form: 0.5 x (1 + tanh(u)) = x / (1 + exp(-2 u)), u = sqrt(2 / pi) (x + 0.044715 x^3).  The right-hand form has no cancellation
-// at negative x: largest absolute error 5e-7 (near x = 7, one ulp) and relative error 1.5e-6, where 1 + tanh(u) in float loses all digits.
+// at negative x, where 1 + tanh(u) in float loses all digits.  For results that are stored as operand planes, whose resolution is
+// 2^-22 of a bound above the row's maximum: fast exponential (relative error 2^-22 + |a| 2^-24 at argument a, i.e. below 3e-8 |x| in the result, as
+// a exp(-|a|) < 0.4) and quotient (2 ulp), a tenth of that resolution.
 __device__ __forceinline__ float gelu_f(float x) {
   const float u2 = 1.5957691216057308f * fmaf(0.044715f * x * x, x, x);
-  return x / (1.f + expf(fminf(-u2, 88.f)));                         // (u2 below -88: the quotient is under 1e-36)
+  return __fdividef(x, 1.f + __expf(fminf(-u2, 87.f)));              // (beyond: the quotient is under 1e-36)
 }
 
 }  // namespace gn

@@ -35,6 +35,7 @@ struct GemmDesc {
   // tensor-core engine, several products in one launch: the columns of the result come in segments of n_seg, segment j at C + j c_seg
   // (bias + j bias_seg): X [Wq; Wk; Wv]^T; the contraction runs over segments of k_seg of A's rows, segment j at A + j a_seg:
   // dQ Wq + dK Wk + dV Wv; the rows of a transposed A come in segments of m_seg at A + j a_seg.
+  int* zmax = nullptr; int zmax_T = 0;                  // with n_seg: largest magnitudes per sequence and head of the result (TcParams::zmax)
   int n_seg = 0, k_seg = 0, m_seg = 0; long c_seg = 0, bias_seg = 0, a_seg = 0;
   int batch1 = 1, batch2 = 1;                           // batch index b -> (b / batch2, b % batch2)
   long a_b1 = 0, a_b2 = 0, b_b1 = 0, b_b2 = 0, c_b1 = 0, c_b2 = 0, r_b1 = 0, r_b2 = 0;
@@ -51,7 +52,7 @@ struct GemmDesc {
 // stores its share of the tile's elements, always in rank order, so a result does not depend on scheduling.  This is what
 // these products need: they come from small batches and narrow layers (a [64, 784] x [784, 128] forward product, a
 // [96, 96] weight gradient over 5000 rows), where a single 128 x 128 tile per block left all but a few SMs idle and one block
-// walking the whole contraction -- 72 us for the former and 430 us for the latter, against 7 and 12 us now.
+// walking the whole contraction -- 72 us for the former and 430 us for the latter, against 7 and 13 us now.
 // Global loads of a k-step go to registers while the previous one is multiplied, then to the other shared-memory buffer.
 // 16-byte loads along the operand's fast index where base, stride and range allow it.
 constexpr int SG_PAD = 4, SG_MAX_SPLITS = 8, SG_RUN = 32;      // runs start at multiples of SG_RUN, whatever the tile
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
 // Skinny outputs (N <= 16, both operands K-major, one problem): a tile would be mostly padding.  A cluster of `splits`
 // blocks owns one output row: their threads stride over K with all N sums in registers, combine through shared memory, and
 // rank 0 adds the blocks' sums in rank order.  C(m,n) = act(sum_k A(m,k) B(n,k) + bias[n] + R(m,n)).  One block per row (K = 4704,
-// N = 10: 18 loads deep) took 18 us for 50 rows; eight take 4.
+// N = 10: 18 loads deep) took 18 us for 50 rows; eight take 7.
 constexpr int SKINNY_N = 16;
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmDesc g, int splits) {
   __shared__ float red[8][SKINNY_N];

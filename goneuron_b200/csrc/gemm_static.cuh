@@ -73,7 +73,11 @@ extern "C" int gn_op_gemm_nt_static(gn_ctx* ctx, int M, int N, int K, const floa
     GN_TRY(tc_split(c, TcSrc{A_dev + m0 * K, (long)K, 1, 0, 0, 1}, PA, nullptr));
     GN_TRY(tc_split(c, TcSrc{B_dev + n0 * K, (long)K, 1, 0, 0, 1}, PB, nullptr));
     TcParams ep{C_dev + m0 * N + n0, (long)N, 0, 0, bias_dev ? bias_dev + n0 : nullptr, nullptr, 0, 0, 0, GN_ACT_LINEAR, m, n, K, 1, 0, c->d_status, nullptr, 0, 1};
-    GN_TRY(tc_run(c, PA, PB, ep));
+    // the regular entry point's slices of a long contraction: side by side where the array has room for their partial results, else one by one
+    int bn = tc_pick_bn(c, m, n, 1, 0); const int splits = tc_split_count(c, ep, 1, &bn);
+    float* part = sb + ((n + 3) & ~3);
+    if (splits > 1 && (part - base) + (long)splits * m * n <= GN_STATIC_SCRATCH_FLOATS) GN_TRY(tc_run_slices(c, PA, PB, ep, splits, bn, part));
+    else GN_TRY(tc_run_rows(c, PA, PB, ep, bn, splits > 1 ? tc_slice_length(K, splits) : 0));
   }
   GN_CUDA(cudaStreamSynchronize(c->stream));
   return check_status_word(c);

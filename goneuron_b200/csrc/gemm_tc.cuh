@@ -49,8 +49,6 @@
 namespace gn {
 
 constexpr int TC_BM = 128;
-constexpr int TC_EPI_WARPS = 8;                 // two warps per TMEM lane quadrant, each takes half of a tile's columns
-constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;   // TMA warp, MMA warp, epilogue warps
 constexpr unsigned TC_SPIN_LIMIT = 1u << 24;    // default number of polls of one wait (Ctx::spin_limit overrides it)
 constexpr unsigned TC_DRAIN_LIMIT = 1u << 20;   // polls spent waiting for own work in flight after a wait gave up
 constexpr int TC_QUEUE_POOL = 2048;   // tile-queue counters per context before the pool is cleared again
@@ -64,12 +62,18 @@ constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by
 // [8192, 1024] x [1024, 256] from 26.8 to 18.6, [32768, 1024] x [1024, 1024] from 136 to 119 (zeros as data: no power limit).
 constexpr int TC_BK = 32, PL_LO = 32;
 __host__ __device__ __forceinline__ int pl_off(int k) { return ((k >> 5) << 6) | (k & 31); }
-template <int BN> struct TcCfg {
+// PL: the variant that writes its result as operand planes.  Its epilogue has twice the work per element (activation or factors, scale,
+// two conversions) and takes 16 warps, four per TMEM lane quadrant; the fp32 epilogue is bound by its stores and runs best with
+// eight.  [18944, 256] over 128 with GELU planes: 28.8 us with eight, 22.7 with 16; as fp32 13.5 and 14.5.
+template <int BN, bool PL> struct TcCfg {
+  static constexpr int EW = PL ? 16 : 8, CG = EW / 4, RS = 128 / EW;              // epilogue warps, column groups, rows per pass through a warp's staging buffer
+  static constexpr int THREADS = 64 + 32 * EW;                                    // TMA warp, MMA warp, epilogue warps
   static constexpr int A_BYTES = TC_BM * 128, B_BYTES = BN * 128;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (192 * 1024) / STAGE_BYTES > 8 ? 8 : (192 * 1024) / STAGE_BYTES;
-  static constexpr int COLV_FLOATS = TC_EPI_WARPS * BN;                           // per epilogue warp: scale and bias of its BN / 2 columns
-  static constexpr int STG_FLOATS = TC_EPI_WARPS * 16 * 36;                       // per epilogue warp: 16 rows x 32 (+4) accumulators in transit
+  static constexpr int CW = BN / CG < 32 ? 32 : BN / CG;                    // columns of an epilogue warp
+  static constexpr int COLV_FLOATS = EW * 2 * CW;                       // per epilogue warp: scale and bias of its columns
+  static constexpr int STG_FLOATS = EW * RS * 36;                                // per epilogue warp: RS rows x 32 (+4) accumulators in transit
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/ + (COLV_FLOATS + STG_FLOATS) * 4;
   static constexpr bool MERGED = BN > 128;                                        // one accumulator per slot
   static constexpr int SLOT_COLS = MERGED ? BN : 2 * BN;
@@ -190,28 +194,32 @@ struct TcParams {
   float* c_last = nullptr; int last_T = 0;                             // fp32 copy of the rows r with r % last_T == last_T - 1: c_last[(r / last_T) * N + col]
   float* z_last = nullptr;                                             // ... and of their values before the activation
   int n_seg = 0; long c_seg = 0, bias_seg = 0;                         // > 0 (a multiple of 32): columns j n_seg .. lie c_seg (biases: bias_seg) floats after those of segment j - 1, see GemmDesc::n_seg
+  int* zmax = nullptr; int zmax_T = 0, zmax_H = 0; long zmax_seg = 0;  // receives the largest magnitude per (segment, sequence of zmax_T rows, head of 64 columns), see attn_tc_max_words
+  int k_slice = 0, splits = 1;                                         // k_slice > 0 (a multiple of 32): z is not a problem but a slice of the contraction, C + z c_b1 its partial result
   float* rowsum32 = nullptr;                                           // plane output: sums of the result over every 32 consecutive rows, [ceil(M / 32)][N]
 };
 
-// Epilogue of one output tile.  Eight warps share it: a warp may only read the TMEM lanes of its quadrant (warp % 4), so
-// two warps serve each quadrant and take half of the tile's columns each (`chalf`); one output row per thread (TMEM lane
+// Epilogue of one output tile.  8 or 16 warps share it: a warp may only read the TMEM lanes of its quadrant (warp % 4), so
+// two or four warps serve each quadrant and take a part of the tile's columns each (`cg`); one output row per thread (TMEM lane
 // = row), 32 consecutive columns per tcgen05.ld, written as 8 float4.  The per-column factors (inverse scale of B's
 // rows, bias) of the warp's columns are staged in shared memory by tc_epilogue_stage BEFORE the warp waits for the
 // accumulator, so that their latency is hidden behind the MMAs; residual and gate values of a chunk are fetched before
 // the TMEM wait for the same reason.  (With four warps and the factors fetched per chunk the epilogue of a tile took as
 // long as its MMAs at K = 1024 and held the tensor pipe back.)  `acc_main` / `acc_cross` are the TMEM column offsets of
 // the two accumulators of this tile (MERGED: there is only acc_main); `bw` is the tile's width (BN, or BN / 2 for a half tile).
-template <int BN>
-__device__ __forceinline__ void tc_epilogue_stage(const TcParams& ep, int n0, int z, int chalf, int lane, int bw, float* colv) {
+template <int BN, bool PL>
+__device__ __forceinline__ void tc_epilogue_stage(const TcParams& ep, int n0, int z, int cg, int lane, int bw, float* colv) {
     if (!(ep.flags & TC_FLAG_VEC)) return;
-    const int ncw = bw / 2, cbase = n0 + chalf * ncw;
+    using Cfg = TcCfg<BN, PL>;
+    const int ncw = max(bw / Cfg::CG, 32), cbase = n0 + cg * ncw;
+    if (cg * ncw >= bw) return;
     const float* isb = ep.isb + (long)z * ep.N;
     __syncwarp();
     for (int i = lane * 4; i < ncw; i += 128) {
       const int col = cbase + i; const bool in = col < ep.N;
       const long bo = ep.n_seg ? col + (col / ep.n_seg) * (ep.bias_seg - ep.n_seg) : col;
       *reinterpret_cast<float4*>(colv + i) = in ? __ldg(reinterpret_cast<const float4*>(isb + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(colv + BN / 2 + i) = (in && ep.bias) ? __ldg(reinterpret_cast<const float4*>(ep.bias + bo)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(colv + Cfg::CW + i) = (in && ep.bias) ? __ldg(reinterpret_cast<const float4*>(ep.bias + bo)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncwarp();
 }
@@ -244,50 +252,53 @@ __device__ __forceinline__ void tc_acc_chunk(uint32_t taddr, uint32_t acc_main, 
     for (int j = 0; j < 32; j++) v[j] = 0.f;
   }
 }
+template <int RS>
 __device__ __forceinline__ void tc_stage_rows(float* stg, const float (&v)[32], int lane, int hh) {
   __syncwarp();                                               // the previous half has been read back
-  if ((lane >> 4) == hh) {
-    float* s = stg + (lane & 15) * TC_STG_LD;
+  if (lane / RS == hh) {
+    float* s = stg + lane % RS * TC_STG_LD;
 #pragma unroll
     for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(s + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
   }
   __syncwarp();
 }
-template <int BN, bool MERGED>
+template <int BN, bool PL, bool MERGED>
 __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tmem_base, uint32_t acc_main, uint32_t acc_cross,
-                                                 int m0, int n0, int z, int quad, int chalf, int lane, int nkb, int bw, const float* colv, float* stg) {
-  const int z1 = z / ep.batch2, z2 = z - z1 * ep.batch2, nch = bw / 64;      // chunks of 32 columns per warp
+                                                 int m0, int n0, int z, int quad, int cg, int lane, int nkb, int bw, const float* colv, float* stg) {
+  using Cfg = TcCfg<BN, PL>;
+  const int z1 = z / ep.batch2, z2 = z - z1 * ep.batch2, nch = max(bw / (32 * Cfg::CG), 1);      // chunks of 32 columns per warp
+  if (cg * nch * 32 >= bw) return;                                           // a narrow tile has fewer chunks than column groups
   const int rbase = m0 + quad * 32, row = rbase + lane;
   const uint32_t tquad = tmem_base + ((uint32_t)(quad * 32) << 16);
-  const float isa = row < ep.M ? ep.isa[(long)z * ep.M + row] : 1.f;         // 1 / (scale of this row's A vector), a power of two
+  const float isa = row < ep.M ? ep.isa[(ep.k_slice ? 0L : (long)z * ep.M) + row] : 1.f;         // 1 / (scale of this row's A vector), a power of two
   const int rl = lane >> 3, c4 = (lane & 7) * 4;                             // after the exchange: rows 4 t + rl, columns c4 .. c4 + 3
-  if (ep.out_p) {
+  if constexpr (PL) {
     // plane output: the result becomes the next contraction's A operand
     float osc = 1.f;                                                         // this lane's row's scale
     if (row < ep.M) {
       const float an = ep.a_rownorm[row], bound = sqrtf(fmaf(an, an, 1.f)) * sqrtf((float)ep.K + 1.f) * __int_as_float(*ep.b_maxabs);
       float oinv; osc = row_scale(ep.flags & TC_FLAG_SCALE ? 1.25f * bound : bound, &oinv);
-      if (n0 == 0 && chalf == 0) ep.out_inv[row] = oinv;
+      if (n0 == 0 && cg == 0) ep.out_inv[row] = oinv;
     }
 #pragma unroll 1
     for (int cc = 0; cc < nch; cc++) {
-      const int c = chalf * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
+      const int c = cg * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
       if (n0 + c * 32 >= ep.N) break;
       float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
-      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + BN / 2 + cc * 32 + c4);
+      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + Cfg::CW + cc * 32 + c4);
       float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);                         // this lane's part of the warp's 32-row column sums
 #pragma unroll 1
-      for (int hh = 0; hh < 2; hh++) {
-        float4 mv[4];
+      for (int hh = 0; hh < 32 / Cfg::RS; hh++) {
+        float4 mv[Cfg::RS / 4];
 #pragma unroll
-        for (int t = 0; t < 4; t++) {
-          const int r = rbase + 16 * hh + 4 * t + rl;
+        for (int t = 0; t < Cfg::RS / 4; t++) {
+          const int r = rbase + Cfg::RS * hh + 4 * t + rl;
           mv[t] = (ep.mask && col_ok && r < ep.M) ? *reinterpret_cast<const float4*>(ep.mask + (long)(r / ep.mask_group) * ep.mask_ld + col) : make_float4(1.f, 1.f, 1.f, 1.f);
         }
-        tc_stage_rows(stg, v, lane, hh);
+        tc_stage_rows<Cfg::RS>(stg, v, lane, hh);
 #pragma unroll
-        for (int t = 0; t < 4; t++) {
-          const int rr = 16 * hh + 4 * t + rl, r = rbase + rr; const float os = __shfl_sync(0xffffffffu, osc, rr);
+        for (int t = 0; t < Cfg::RS / 4; t++) {
+          const int rr = Cfg::RS * hh + 4 * t + rl, r = rbase + rr; const float os = __shfl_sync(0xffffffffu, osc, rr);
           if (!col_ok || r >= ep.M) continue;
           const float4 a = *reinterpret_cast<const float4*>(stg + (4 * t + rl) * TC_STG_LD + c4);
           float4 x = make_float4(a.x * sv.x + bv.x, a.y * sv.y + bv.y, a.z * sv.z + bv.z, a.w * sv.w + bv.w);
@@ -318,28 +329,28 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
       }
     }
     __syncwarp();
-    return;
-  }
+  } else {
   float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
   const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
   if (ep.flags & TC_FLAG_VEC) {
 #pragma unroll 1
     for (int cc = 0; cc < nch; cc++) {
-      const int c = chalf * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
+      const int c = cg * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
       if (n0 + c * 32 >= ep.N) break;
       float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
-      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + BN / 2 + cc * 32 + c4);
+      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + Cfg::CW + cc * 32 + c4);
+      float zm = 0.f;
       const long so = ep.n_seg ? ((n0 + c * 32) / ep.n_seg) * (ep.c_seg - ep.n_seg) : 0;      // (32 columns lie in one segment; with segments R is C)
       float* Cs = C + so; const float* Rs = R + so;
 #pragma unroll 1
-      for (int hh = 0; hh < 2; hh++) {
-        const int r0 = rbase + 16 * hh + rl;
-        float4 rv[4];                                                        // residual, fetched before the exchange so that its latency overlaps it
+      for (int hh = 0; hh < 32 / Cfg::RS; hh++) {
+        const int r0 = rbase + Cfg::RS * hh + rl;
+        float4 rv[Cfg::RS / 4];                                                        // residual, fetched before the exchange so that its latency overlaps it
 #pragma unroll
-        for (int t = 0; t < 4; t++) rv[t] = (R && col_ok && r0 + 4 * t < ep.M) ? *reinterpret_cast<const float4*>(Rs + (long)(r0 + 4 * t) * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-        tc_stage_rows(stg, v, lane, hh);
+        for (int t = 0; t < Cfg::RS / 4; t++) rv[t] = (R && col_ok && r0 + 4 * t < ep.M) ? *reinterpret_cast<const float4*>(Rs + (long)(r0 + 4 * t) * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        tc_stage_rows<Cfg::RS>(stg, v, lane, hh);
 #pragma unroll
-        for (int t = 0; t < 4; t++) {
+        for (int t = 0; t < Cfg::RS / 4; t++) {
           const int r = r0 + 4 * t;
           const float4 a = *reinterpret_cast<const float4*>(stg + (4 * t + rl) * TC_STG_LD + c4);
           float4 x = make_float4(a.x * sv.x + bv.x + rv[t].x, a.y * sv.y + bv.y + rv[t].y, a.z * sv.z + bv.z + rv[t].z, a.w * sv.w + bv.w + rv[t].w);
@@ -350,7 +361,13 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
             if (!(mv.x > 0.f)) x.x = 0.f; if (!(mv.y > 0.f)) x.y = 0.f; if (!(mv.z > 0.f)) x.z = 0.f; if (!(mv.w > 0.f)) x.w = 0.f;
           }
           *reinterpret_cast<float4*>(Cs + (long)r * ep.ldc + col) = x;
+          if (ep.zmax) zm = fmaxf(zm, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
         }
+      }
+      if (ep.zmax) {                                                         // (32 rows of one sequence, 32 columns of one head)
+        zm = warp_max(zm); if (!(zm <= 3.0e38f)) zm = 3.4e38f;
+        const int c32 = n0 + c * 32, sg = c32 / ep.n_seg;
+        if (lane == 0 && rbase < ep.M) atomicMax(ep.zmax + sg * ep.zmax_seg + (long)(rbase / ep.zmax_T) * ep.zmax_H + (c32 - sg * ep.n_seg) / 64, __float_as_int(zm));
       }
     }
     __syncwarp();
@@ -358,17 +375,17 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
   }
   // scalar path (unaligned operands, NCHW store): one output row per thread
   const bool row_ok = row < ep.M;
-  const float* isb = ep.isb + (long)z * ep.N;
+  const float* isb = ep.isb + (ep.k_slice ? 0L : (long)z * ep.N);
   const float* Rrow = (R && row_ok) ? R + (long)row * ep.ldr : nullptr;
   const float* Mrow = (ep.mask && row_ok) ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
   float* Crow = ep.nchw_P > 0 ? C + (long)(row / ep.nchw_P) * ep.N * ep.nchw_P + row % ep.nchw_P : C + (long)row * ep.ldc;
   const long cstep = ep.nchw_P > 0 ? ep.nchw_P : 1;
 #pragma unroll 1
   for (int cc = 0; cc < nch; cc++) {
-    const int col0 = n0 + (chalf * nch + cc) * 32;
+    const int col0 = n0 + (cg * nch + cc) * 32;
     if (col0 >= ep.N) break;
     const int seg = ep.n_seg ? col0 / ep.n_seg : 0; const long c_off = ep.n_seg ? seg * (ep.c_seg - ep.n_seg) : 0, b_off = ep.n_seg ? seg * (ep.bias_seg - ep.n_seg) : 0;
-    float v[32]; tc_acc_chunk<MERGED>(tquad + (chalf * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
+    float v[32]; tc_acc_chunk<MERGED>(tquad + (cg * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
 #pragma unroll
     for (int j = 0; j < 32; j++) {
       const int col = col0 + j;
@@ -381,14 +398,15 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
       Crow[c_off + col * cstep] = x;
     }
   }
+  }
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
-template <int BN>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+template <int BN, bool PL>
+__global__ void __launch_bounds__(TcCfg<BN, PL>::THREADS, 1)
 gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ TcParams ep, int tiles_m, int tiles_n, int total_tiles, int full_end, int n_half, int* tile_queue) {
-  using Cfg = TcCfg<BN>;
+  using Cfg = TcCfg<BN, PL>;
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES, BK = TC_BK;
   constexpr bool MERGED = Cfg::MERGED;
   constexpr uint32_t TMEM_COLS = Cfg::TMEM_COLS, SLOT_COLS = Cfg::SLOT_COLS;
@@ -412,9 +430,9 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
     asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
     for (int s = 0; s < STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, TC_EPI_WARPS); }
+    for (int b = 0; b < 2; b++) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, Cfg::EW); }
     mbar_init(drain, 1);
-    for (int b = 0; b < 4; b++) { mbar_init(qfull0 + 8 * b, 1); mbar_init(qempty0 + 8 * b, 1 + TC_EPI_WARPS); }
+    for (int b = 0; b < 4; b++) { mbar_init(qfull0 + 8 * b, 1); mbar_init(qempty0 + 8 * b, 1 + Cfg::EW); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -467,6 +485,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
     m0 = mt * TC_BM; n0 = nt * BN + (half > 0 ? BN / 2 : 0);
     if ((ep.flags & GEMM_SKIP_UPPER) && n0 > m0 + TC_BM - 1) return false;
     int kbeg = 0, kend = ep.K;
+    if (ep.k_slice) { kbeg = z * ep.k_slice; kend = min(ep.K, kbeg + ep.k_slice); }
     if (ep.flags & GEMM_KBEG_AT_M0) kbeg = (m0 / BK) * BK;
     if (ep.flags & GEMM_KEND_AT_M0) kend = min(ep.K, m0 + TC_BM);
     kb0 = kbeg / BK; nkb = (kend - kbeg + BK - 1) / BK;
@@ -483,6 +502,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
     int tile, half;
     for (int w = 0; ok && work(w, tile, half); w++) {
       int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
+      if (ep.k_slice) z = 0;
       for (int i = 0; i < nkb; i++) {
         const int kc = 2 * (kb0 + i) * BK;
         if (issued >= (uint32_t)STAGES && !mbar_wait(empty0 + 8 * s, ph ^ 1, limit, abort_flag)) { ok = false; break; }
@@ -541,21 +561,21 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
     }
     __syncwarp();
   } else {
-    const int quad = warp & 3, chalf = (warp - 2) >> 2; uint32_t lt = 0;
-    float* colv = colv_all + (warp - 2) * BN;
-    float* stg = colv_all + Cfg::COLV_FLOATS + (warp - 2) * 16 * TC_STG_LD;
+    const int quad = warp & 3, cg = (warp - 2) >> 2; uint32_t lt = 0;
+    float* colv = colv_all + (warp - 2) * 2 * Cfg::CW;
+    float* stg = colv_all + Cfg::COLV_FLOATS + (warp - 2) * Cfg::RS * TC_STG_LD;
     int tile, half;
     for (int w = 0; work(w, tile, half); w++) {
       int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
       const uint32_t slot = lt & 1, u = lt >> 1; lt++;
       const int bw = half < 0 ? BN : BN / 2;
-      tc_epilogue_stage<BN>(ep, n0, z, chalf, lane, bw, colv);
+      tc_epilogue_stage<BN, PL>(ep, n0, ep.k_slice ? 0 : z, cg, lane, bw, colv);
       int ok = 1;
       if (lane == 0) ok = mbar_wait(tfull0 + 8 * slot, u & 1, limit, abort_flag) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) { if (lane == 0 && !*abort_flag) give_up(3); break; }
       tc_fence_after();
-      tc_epilogue_tile<BN, MERGED>(ep, tmem_base, slot * SLOT_COLS, slot * SLOT_COLS + BN, m0, n0, z, quad, chalf, lane, nkb, bw, colv, stg);
+      tc_epilogue_tile<BN, PL, MERGED>(ep, tmem_base, slot * SLOT_COLS, slot * SLOT_COLS + BN, m0, n0, z, quad, cg, lane, nkb, bw, colv, stg);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty0 + 8 * slot);
@@ -684,7 +704,7 @@ inline int tc_ldp(int K) { return ((K + 31) / 32) * 32; }           // plane row
 inline size_t bf_plane_floats(long nbatch, long rows, long ldp) { return (size_t)nbatch * rows * ldp; }   // two fp16 planes = one float per element
 
 // Per-context operand-plane scratch of the contraction engine (calls on a context are serialised by Ctx::run_mu).
-struct TcScratch { DevBuf a, b, sa, sb, mx; const float* last_a = nullptr; int last_m = 0, last_k = 0; long last_ld = 0; };
+struct TcScratch { DevBuf a, b, sa, sb, mx, part; const float* last_a = nullptr; int last_m = 0, last_k = 0; long last_ld = 0; };
 inline TcScratch& tc_scratch(Ctx* ctx) { if (!ctx->tc_scratch) ctx->tc_scratch = ctx->own(new TcScratch()); return *static_cast<TcScratch*>(ctx->tc_scratch); }
 
 // After a replayed graph the scratch no longer holds what the last directly issued call left there.
@@ -703,12 +723,12 @@ inline int tc_planes(Ctx* ctx, int which, long nbatch, long rows, int K, BfPlane
 }
 inline int* tc_rowmax_buf(Ctx* ctx) { return reinterpret_cast<int*>(tc_scratch(ctx).mx.p); }
 
-template <int BN> inline bool tc_set_smem() { return cudaFuncSetAttribute(gemm_tc_persist_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<BN>::SMEM_BYTES) == cudaSuccess; }
+template <int BN, bool PL> inline bool tc_set_smem() { return cudaFuncSetAttribute(gemm_tc_persist_kernel<BN, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<BN, PL>::SMEM_BYTES) == cudaSuccess; }
 inline void tc_init(Ctx* ctx) {
   ctx->tc_ok = false;
   void* fn = nullptr; cudaDriverEntryPointQueryResult q;
   if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn || q != cudaDriverEntryPointSuccess) { cudaGetLastError(); return; }
-  if (!(tc_set_smem<64>() && tc_set_smem<128>() && tc_set_smem<256>())) { cudaGetLastError(); return; }
+  if (!(tc_set_smem<64, false>() && tc_set_smem<128, false>() && tc_set_smem<256, false>() && tc_set_smem<64, true>() && tc_set_smem<128, true>() && tc_set_smem<256, true>())) { cudaGetLastError(); return; }
   ctx->encode_tiled = fn; ctx->tc_ok = true;
   if (const char* e = getenv("GONEURON_CUDA_TC_BN")) ctx->tc_force_bn = atoi(e);
   if (const char* e = getenv("GONEURON_CUDA_TC_KSLICE")) ctx->tc_kslice = atoi(e);
@@ -778,7 +798,7 @@ inline int tc_launch_persist(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, con
   CUtensorMap mA, mB;
   // the B tile of a stage arrives as two copies of BN / 2 rows, so that a half tile (see the kernel's work list) is one of them
   GN_TRY(tc_operand_map(ctx, &mA, A, TC_BM)); GN_TRY(tc_operand_map(ctx, &mB, B, BN / 2));
-  const int tiles_m = cdiv(ep.M, TC_BM), tiles_n = cdiv(ep.N, BN); const long total = (long)tiles_m * tiles_n * A.nbatch;
+  const int tiles_m = cdiv(ep.M, TC_BM), tiles_n = cdiv(ep.N, BN); const long total = (long)tiles_m * tiles_n * A.nbatch * ep.splits;
   if (total > 0x7fffffffL) return fail(GN_ERR_UNSUPPORTED, "too many output tiles");
   const unsigned grid = (unsigned)std::min<long>(total, persist_sms(ctx));
   const long left = tc_tail_halves(ctx, total, BN, ep.flags);
@@ -786,7 +806,8 @@ inline int tc_launch_persist(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, con
   int* queue = nullptr;
   if (ctx->tc_tile_queue && total > grid) GN_TRY(tc_next_queue(ctx, &queue));
   ProfScope prof(ctx);
-  GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN>), grid, TC_THREADS, (TcCfg<BN>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  if (ep.out_p) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, true>), grid, (TcCfg<BN, true>::THREADS), (TcCfg<BN, true>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  else GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, false>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
   return check_launch("gemm_tc_persist");
 }
 // Output tile width for a problem: 64 for narrow outputs; 256 (three quarters of the shared-memory traffic per MMA
@@ -819,6 +840,7 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
       return fail(GN_ERR_INVALID_ARG, "tc_launch: plane output needs 16-byte aligned operands");
     vec = true;
   }
+  if (ep.zmax && !vec) return fail(GN_ERR_INVALID_ARG, "tc_launch: maxima need 16-byte aligned operands");
   if (vec) ep.flags |= TC_FLAG_VEC;
   {
     double by = 4.0 * ((double)ep.M + ep.N) * ep.K + 4.0 * (double)ep.M * ep.N * (ep.R ? 2 : 1);
@@ -834,8 +856,8 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
 // gradients over all tokens of a batch) are therefore cut into slices, each slice adding its result to C through the
 // epilogue's residual path, i.e. in properly rounded fp32: 4096 indices per run with separate accumulators for the
 // large and the small terms, 2048 with the single accumulator of the 256-wide tile.
-inline int tc_run_rows(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams& ep, int bn) {
-  const int kslice = ctx->tc_kslice > 0 ? ctx->tc_kslice : (bn == 256 ? 2048 : 4096);
+inline int tc_run_rows(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams& ep, int bn, int slice = 0) {
+  const int kslice = slice > 0 ? slice : ctx->tc_kslice > 0 ? ctx->tc_kslice : (bn == 256 ? 2048 : 4096);
   if (ep.K <= kslice || (ep.flags & (GEMM_KBEG_AT_M0 | GEMM_KEND_AT_M0))) return tc_launch(ctx, A, B, ep, bn);
   if (ep.out_p) return fail(GN_ERR_UNSUPPORTED, "a contraction that writes operand planes must fit one accumulator run (K = %d)", ep.K);
   for (int k0 = 0; k0 < ep.K; k0 += kslice) {
@@ -848,7 +870,70 @@ inline int tc_run_rows(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcP
   }
   return GN_OK;
 }
+// Few output tiles and a long contraction leave SMs idle for the whole contraction (the products of a head or of a block's token
+// rows: 64 x 1024 over 4096 is eight tiles, 45 us with one tile per CTA), or make 128-wide tiles the only ones that fill them,
+// whose main loop is bound by shared memory traffic.  The contraction can then be cut into slices, each a tile of its own with a
+// partial result; a second kernel adds the partial results in slice order (fp32) and applies the epilogue.
+__global__ void __launch_bounds__(256) tc_sum_slices_kernel(const float* __restrict__ part, int splits, int M, int N, const TcParams ep) {
+  const long mn = (long)M * N, n4 = mn >> 2; const bool vec = (N & 3) == 0;
+  for (long e = blockIdx.x * 256L + threadIdx.x; e < (vec ? n4 : mn); e += gridDim.x * 256L) {
+    const long i = vec ? 4 * e : e; const int r = (int)(i / N), c = (int)(i - (long)r * N), w = vec ? 4 : 1;
+    float x[4] = {};
+    if (vec) {
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int z = 0; z < splits; z++) { const float4 u = *reinterpret_cast<const float4*>(part + z * mn + i); t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+      x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+    } else
+#pragma unroll 4
+      for (int z = 0; z < splits; z++) x[0] += part[z * mn + i];
+    for (int k = 0; k < w; k++) {
+      if (ep.bias) x[k] += ep.bias[c + k];
+      if (ep.R) x[k] += ep.R[(long)r * ep.ldr + c + k];
+      if (ep.act == GN_ACT_RELU) x[k] = fmaxf(x[k], 0.f);
+      if (ep.mask && !(ep.mask[(long)(r / ep.mask_group) * ep.mask_ld + c + k] > 0.f)) x[k] = 0.f;
+    }
+    float* o = ep.C + (long)r * ep.ldc + c;
+    if (vec && ((ep.ldc & 3) | (long)(reinterpret_cast<uintptr_t>(ep.C) & 15)) == 0) *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
+    else for (int k = 0; k < w; k++) o[k] = x[k];
+  }
+}
+// Slices and tile width by estimated time, from measured rates (us): 0.335 / 0.43 per 32 contraction indices of a 128 / 256 wide
+// tile, 3 / 5 for the last tile's epilogue, 3 for the second launch and 4 TB/s for its partial results.  Slices keep at least 256
+// indices, and have to win by a tenth.
+inline int tc_split_count(Ctx* ctx, const TcParams& ep, long nbatch, int* bn) {
+  if (nbatch != 1 || ep.out_p || ep.n_seg || ep.nchw_P || ep.flags || ep.K < 1024 || ctx->tc_kslice > 0 || ctx->tc_force_bn) return 1;
+  const long sms = persist_sms(ctx), tm = cdiv(ep.M, TC_BM); const double kb = cdiv(ep.K, TC_BK);
+  auto cost = [&](int w, int sl) {
+    const long tiles = tm * cdiv(ep.N, w); double rounds = std::ceil((double)tiles * sl / sms);
+    if (sl == 1 && tc_tail_halves(ctx, tiles, w, 0) > 0) rounds -= 0.38;
+    return rounds * (kb / sl) * (w == 256 ? 0.43 : 0.335) + (w == 256 ? 5.0 : 3.0) + (sl > 1 ? 3.0 + 1e-6 * ep.M * ep.N * (sl + 1) : 0.0);
+  };
+  double best = 0.9 * cost(tc_pick_bn(ctx, ep.M, ep.N, 1, 0) == 256 ? 256 : 128, 1); int splits = 1;
+  for (int w : {128, 256}) if (w == 128 || ep.N > 128)
+    for (int sl = std::max(2, (int)cdiv(ep.K, w == 256 ? 2048 : 4096)); sl <= 32 && sl * 256 <= ep.K; sl++) {
+      if (tm * cdiv(ep.N, w) * (sl - 1) >= sms) break;
+      const double c = cost(w, sl); if (c < best) { best = c; splits = sl; *bn = w; }
+    }
+  return splits;
+}
+inline int tc_slice_length(int K, int splits) { return cdiv(cdiv(K, splits), TC_BK) * TC_BK; }
+// `part`: room for one partial result [M, N] per slice
+inline int tc_run_slices(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams& ep, int splits, int bn, float* part) {
+  TcParams es = ep;
+  es.k_slice = tc_slice_length(ep.K, splits); es.splits = cdiv(ep.K, es.k_slice);
+  es.C = part; es.ldc = ep.N; es.c_b1 = (long)ep.M * ep.N; es.c_b2 = 0; es.batch2 = 1; es.bias = nullptr; es.R = nullptr; es.mask = nullptr; es.act = GN_ACT_LINEAR;
+  GN_TRY(tc_launch(ctx, A, B, es, ep.N <= 64 ? 64 : bn));
+  GN_LAUNCH(ctx, tc_sum_slices_kernel, (unsigned)std::min<long>(cdiv((long)ep.M * ep.N, 1024), 4L * ctx->sm_count), 256, 0, (const float*)part, es.splits, ep.M, ep.N, ep);
+  return check_launch("tc_sum_slices");
+}
 inline int tc_run(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcParams& ep) {
+  int bn = 128; const int splits = tc_split_count(ctx, ep, A.nbatch, &bn);
+  if (splits > 1) {
+    TcScratch& sc = tc_scratch(ctx); const size_t n = (size_t)splits * ep.M * ep.N;
+    if (sc.part.n < n) { GN_CUDA(cudaStreamSynchronize(ctx->stream)); ctx->epoch++; GN_TRY(sc.part.alloc(n)); }
+    return tc_run_slices(ctx, A, B, ep, splits, bn, sc.part.p);
+  }
   // (Running the rows of a short last wave as a second launch with 128-wide tiles was measured at 16 384 rows: the second
   // launch's fixed cost ate the 9 % it should have saved, so every product is one tiling.)
   return tc_run_rows(ctx, A, B, ep, tc_pick_bn(ctx, ep.M, ep.N, A.nbatch, ep.flags));
@@ -870,6 +955,7 @@ __device__ __forceinline__ int wplane_find(const WPlaneJob* jobs, int njobs, int
   while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (jobs[mid].tile0 <= tile) lo = mid; else hi = mid - 1; }
   return lo;
 }
+// (after a training step the parameter update has left the maxima behind, see adam_kernel: this pass is for other changes)
 __global__ void __launch_bounds__(256) wplanes_max_kernel(const WPlaneJob* __restrict__ jobs, int njobs, int* __restrict__ mx, int tile_off) {
   __shared__ float red[33];
   const int tile = blockIdx.x + tile_off;
@@ -881,39 +967,58 @@ __global__ void __launch_bounds__(256) wplanes_max_kernel(const WPlaneJob* __res
   m = block_max(m, red);
   if (threadIdx.x == 0) { if (!(m <= 3.0e38f)) m = 3.4e38f; atomicMax(mx + j, __float_as_int(m)); }
 }
+// Memory-bound: 4 bytes read and 8 written per weight.  16-byte loads of a 64 x 64 tile, then four neighbouring contraction
+// indices per thread and store in either orientation: whole 64-byte runs of each plane (two indices and 4-byte stores ran at 1.8 TB/s).
 __global__ void __launch_bounds__(256) wplanes_split_kernel(const WPlaneJob* __restrict__ jobs, int njobs, const int* __restrict__ mx, int tile_off) {
   __shared__ float tl[64][65];
   const int tile = blockIdx.x + tile_off;
   const int j = wplane_find(jobs, njobs, tile); const WPlaneJob jb = jobs[j];
   const int t = tile - jb.tile0, r0 = (t / jb.tiles_in) * 64, c0 = (t % jb.tiles_in) * 64;
-  float inv; const float sc = row_scale(__int_as_float(mx[j]), &inv);
-  for (int e = threadIdx.x; e < 4096; e += 256) { const int rr = e >> 6, cc = e & 63; const int r = r0 + rr, c = c0 + cc; tl[rr][cc] = (r < jb.out && c < jb.in) ? wplane_row(jb, r)[c] : 0.f; }
-  __syncthreads();
-  const int x2 = (threadIdx.x & 31) * 2, y = threadIdx.x >> 5;
-  for (int rr = y; rr < 64; rr += 8) {                        // as stored: plane row = out index, two neighbouring in indices per thread
-    const int r = r0 + rr, c = c0 + x2;
-    if (r < jb.out && c < jb.in) {                            // (in is even-padded by ldp_r; an odd last column writes its zero neighbour)
-      uint32_t a, b; split2_pair(tl[rr][x2], tl[rr][x2 + 1], sc, a, b);
-      __half* o = jb.r + (long)r * 2 * jb.ldp_r + pl_off(c);
-      *reinterpret_cast<uint32_t*>(o) = a; *reinterpret_cast<uint32_t*>(o + PL_LO) = b;
+  float mxv = __int_as_float(mx[j]); if (!(mxv <= 3.0e38f)) mxv = 3.4e38f;
+  float inv; const float sc = row_scale(mxv, &inv);
+  const int x4 = (threadIdx.x & 15) * 4, y = threadIdx.x >> 4, c = c0 + x4;
+  const bool vec = (((uintptr_t)jb.src | (uintptr_t)(jb.in * 4) | (uintptr_t)(jb.stride * 4)) & 15) == 0;
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int r = r0 + y + 16 * k;
+    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < jb.out) {
+      const float* q = wplane_row(jb, r) + c;
+      if (vec) { if (c < jb.in) v[k] = *reinterpret_cast<const float4*>(q); }
+      else { if (c < jb.in) v[k].x = q[0]; if (c + 1 < jb.in) v[k].y = q[1]; if (c + 2 < jb.in) v[k].z = q[2]; if (c + 3 < jb.in) v[k].w = q[3]; }
     }
-    if (c0 == 0 && x2 == 0 && r < jb.out) jb.inv_r[r] = inv;
   }
-  for (int cc = y; cc < 64; cc += 8) {                        // transposed: plane row = in index, two neighbouring out indices per thread
-    const int c = c0 + cc, r = r0 + x2;
-    if (c < jb.in && r < jb.out) {
-      uint32_t a, b; split2_pair(tl[x2][cc], tl[x2 + 1][cc], sc, a, b);
-      __half* o = jb.c + (long)c * 2 * jb.ldp_c + pl_off(r);
-      *reinterpret_cast<uint32_t*>(o) = a; *reinterpret_cast<uint32_t*>(o + PL_LO) = b;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {                              // as stored: plane row = out index (a last group beyond `in` writes zeros: plane rows are whole blocks of 32)
+    const int rr = y + 16 * k, r = r0 + rr;
+    tl[rr][x4] = v[k].x; tl[rr][x4 + 1] = v[k].y; tl[rr][x4 + 2] = v[k].z; tl[rr][x4 + 3] = v[k].w;
+    if (r < jb.out && c < jb.in) {
+      uint2 a, b; split2_pair(v[k].x, v[k].y, sc, a.x, b.x); split2_pair(v[k].z, v[k].w, sc, a.y, b.y);
+      __half* o = jb.r + (long)r * 2 * jb.ldp_r + pl_off(c);
+      *reinterpret_cast<uint2*>(o) = a; *reinterpret_cast<uint2*>(o + PL_LO) = b;
+      if (c == 0) jb.inv_r[r] = inv;
     }
-    if (r0 == 0 && x2 == 0 && c < jb.in) jb.inv_c[c] = inv;
+  }
+  __syncthreads();
+  const int r = r0 + x4;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {                              // transposed: plane row = in index
+    const int cc = y + 16 * k, ci = c0 + cc;
+    if (ci < jb.in && r < jb.out) {
+      uint2 a, b; split2_pair(tl[x4][cc], tl[x4 + 1][cc], sc, a.x, b.x); split2_pair(tl[x4 + 2][cc], tl[x4 + 3][cc], sc, a.y, b.y);
+      __half* o = jb.c + (long)ci * 2 * jb.ldp_c + pl_off(r);
+      *reinterpret_cast<uint2*>(o) = a; *reinterpret_cast<uint2*>(o + PL_LO) = b;
+      if (r == 0) jb.inv_c[ci] = inv;
+    }
   }
 }
 // Host side of the table: one entry per registered matrix, looked up by the matrix's device address.
 struct WeightPlaneEntry { const float* src; int out, in; BfPlanes rows, cols; int part = 0; long stride = 0;      // (part = out: a single matrix)
   const float* bias = nullptr; const int* maxabs = nullptr; int layer = -1; int tile0 = 0, tiles = 0; };
 struct WeightPlaneTable {
-  std::vector<WeightPlaneEntry> e; DevBuf planes, scales, mx, jobs; int total_tiles = 0; bool dirty = true, used = false;      // used: some product has looked a matrix up
+  std::vector<WeightPlaneEntry> e; DevBuf planes, scales, mx, jobs, ranges; int total_tiles = 0;
+  bool dirty = true, used = false, max_ok = false;          // used: some product has looked a matrix up; max_ok: `mx` holds the maxima of the current parameters
   // entries [j0, j1) that belong to model layer `layer` (they are registered layer by layer, so the range is contiguous)
   void layer_range(int layer, int* j0, int* j1) const {
     *j0 = *j1 = 0; bool in = false;
@@ -924,6 +1029,8 @@ struct WeightPlaneTable {
     return nullptr;
   }
 };
+// The parameters a table entry covers (ascending; the biases count towards an entry's maximum).
+struct PlaneRange { const float *b, *e; };
 // Lays the table out for the matrices (src, out, in) and allocates its buffers (planes zeroed once: the padding columns
 // of a plane row are never written afterwards and must read as zero).
 inline int wplanes_build(Ctx* ctx, WeightPlaneTable& t, const std::vector<WeightPlaneEntry>& mats) {
@@ -949,24 +1056,43 @@ inline int wplanes_build(Ctx* ctx, WeightPlaneTable& t, const std::vector<Weight
   t.total_tiles = tiles;
   GN_TRY(t.jobs.alloc((jobs.size() * sizeof(WPlaneJob) + 3) / 4));
   GN_CUDA(copy_h2d(ctx, t.jobs.p, jobs.data(), jobs.size() * sizeof(WPlaneJob)));
-  t.dirty = true; return GN_OK;
+  std::vector<PlaneRange> rg;
+  for (auto& x : t.e) rg.push_back(PlaneRange{x.src, x.src + (x.out / x.part - 1) * x.stride + (size_t)x.part * x.in + (x.bias ? x.part : 0)});
+  GN_TRY(t.ranges.alloc(rg.size() * sizeof(PlaneRange) / 4)); GN_CUDA(copy_h2d(ctx, t.ranges.p, rg.data(), rg.size() * sizeof(PlaneRange)));
+  t.dirty = true; t.max_ok = false; return GN_OK;
 }
 // Re-splits every registered matrix if the parameters changed since the last call.
 // Entries [j0, j1) only, on `stream`: used right behind a layer's parameter update when the update runs layer by layer.
+inline int wplanes_max(Ctx* ctx, WeightPlaneTable& t, int j0, int j1, cudaStream_t stream) {
+  const int tile_off = t.e[j0].tile0, ntiles = t.e[j1 - 1].tile0 + t.e[j1 - 1].tiles - tile_off;
+  GN_CUDA(cudaMemsetAsync(reinterpret_cast<int*>(t.mx.p) + j0, 0, (size_t)(j1 - j0) * sizeof(int), stream));
+  wplanes_max_kernel<<<ntiles, 256, 0, stream>>>(reinterpret_cast<const WPlaneJob*>(t.jobs.p), (int)t.e.size(), reinterpret_cast<int*>(t.mx.p), tile_off);
+  ctx->launches++;
+  return check_launch("wplanes_max");
+}
+inline int wplanes_split(Ctx* ctx, WeightPlaneTable& t, int j0, int j1, cudaStream_t stream) {
+  const int tile_off = t.e[j0].tile0, ntiles = t.e[j1 - 1].tile0 + t.e[j1 - 1].tiles - tile_off;
+  wplanes_split_kernel<<<ntiles, 256, 0, stream>>>(reinterpret_cast<const WPlaneJob*>(t.jobs.p), (int)t.e.size(), reinterpret_cast<const int*>(t.mx.p), tile_off);
+  ctx->launches++;
+  double elems = 0; for (int j = j0; j < j1; j++) elems += (double)t.e[j].out * t.e[j].in;
+  ctx->split_bytes += 12.0 * elems;
+  return check_launch("wplanes_split");
+}
 inline int wplanes_refresh_range(Ctx* ctx, WeightPlaneTable& t, int j0, int j1, cudaStream_t stream) {
   if (j1 <= j0) return GN_OK;
-  const int nj = (int)t.e.size(), tile_off = t.e[j0].tile0, ntiles = t.e[j1 - 1].tile0 + t.e[j1 - 1].tiles - tile_off;
-  GN_CUDA(cudaMemsetAsync(reinterpret_cast<int*>(t.mx.p) + j0, 0, (size_t)(j1 - j0) * sizeof(int), stream));
-  wplanes_max_kernel<<<ntiles, 256, 0, stream>>>(reinterpret_cast<const WPlaneJob*>(t.jobs.p), nj, reinterpret_cast<int*>(t.mx.p), tile_off);
-  wplanes_split_kernel<<<ntiles, 256, 0, stream>>>(reinterpret_cast<const WPlaneJob*>(t.jobs.p), nj, reinterpret_cast<const int*>(t.mx.p), tile_off);
-  ctx->launches += 2;
-  double elems = 0; for (int j = j0; j < j1; j++) elems += (double)t.e[j].out * t.e[j].in;
-  ctx->split_bytes += 16.0 * elems;                          // 4 B read twice, 8 B written
-  return check_launch("wplanes_refresh");
+  GN_TRY(wplanes_max(ctx, t, j0, j1, stream));
+  return wplanes_split(ctx, t, j0, j1, stream);
+}
+// The maxima, where the last change of the parameters was not a training step's update.
+inline int wplanes_need_max(Ctx* ctx, WeightPlaneTable& t) {
+  if (t.e.empty() || !t.used || t.max_ok) return GN_OK;
+  GN_TRY(wplanes_max(ctx, t, 0, (int)t.e.size(), ctx->stream));
+  t.max_ok = true; return GN_OK;
 }
 inline int wplanes_refresh(Ctx* ctx, WeightPlaneTable& t) {
   if (t.e.empty() || !t.dirty) return GN_OK;
-  GN_TRY(wplanes_refresh_range(ctx, t, 0, (int)t.e.size(), ctx->stream));
+  if (!t.max_ok) { GN_TRY(wplanes_max(ctx, t, 0, (int)t.e.size(), ctx->stream)); t.max_ok = true; }
+  GN_TRY(wplanes_split(ctx, t, 0, (int)t.e.size(), ctx->stream));
   t.dirty = false; return GN_OK;
 }
 // Prepared planes for B of this contraction, if B is a registered matrix used in one of its two orientations.
@@ -1037,6 +1163,7 @@ inline int gemm_tc(Ctx* ctx, const GemmDesc& g) {
   if (g.n_seg) {
     if (g.n_seg % 32 || nb != 1 || g.R || g.plane_out) return fail(GN_ERR_INVALID_ARG, "gemm_tc: this contraction cannot write its columns in segments");
     ep.n_seg = g.n_seg; ep.c_seg = g.c_seg; ep.bias_seg = g.bias_seg;
+    ep.zmax = g.zmax; ep.zmax_T = g.zmax_T; ep.zmax_H = g.n_seg / 64; ep.zmax_seg = 3L * (g.M / std::max(1, g.zmax_T)) * ep.zmax_H;
   }
   if (g.plane_out) {
     const TcPlaneOut& po = *static_cast<const TcPlaneOut*>(g.plane_out);

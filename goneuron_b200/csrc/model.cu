@@ -72,10 +72,15 @@ static int gemm_tn(Ctx* ctx, int R, int N, int K, const float* dZ, long ldz, con
 // their planes as a stack, else one by one.  At 3600 rows of 384 the three projections are 87 tiles each: 1.8 rounds of the SMs
 // together, three alone.
 // Y_j[M, n] = X W_j^T + b_j; Y_j and b_j are cs and ws floats apart
-static int gemm_nt_stack(Ctx* ctx, int parts, int M, int n, int d, const float* X, long ldx, const float* W, long ws, const float* bias, float* Y, long cs, const BfPlanes* x_planes = nullptr) {
+static int gemm_nt_stack(Ctx* ctx, int parts, int M, int n, int d, const float* X, long ldx, const float* W, long ws, const float* bias, float* Y, long cs, const BfPlanes* x_planes = nullptr,
+                         int* zmax = nullptr, int zmax_T = 0, bool* zmax_done = nullptr) {
   GemmDesc g; g.M = M; g.N = parts * n; g.K = d; g.A = X; g.sa_m = ldx; g.sa_k = 1; g.B = W; g.sb_k = 1; g.sb_n = d; g.C = Y; g.ldc = n; g.bias = bias;
   g.n_seg = n; g.c_seg = cs; g.bias_seg = ws; g.a_planes = x_planes; BfPlanes w;
-  if (parts > 1 && n % 32 == 0 && gemm_on_tc(ctx, g) && wplanes_lookup(ctx, g, &w)) { g.b_planes = &w; return gemm(ctx, g); }
+  if (parts > 1 && n % 32 == 0 && gemm_on_tc(ctx, g) && wplanes_lookup(ctx, g, &w)) {
+    g.b_planes = &w;
+    if (zmax && d <= 2048 && ((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(Y) | (uintptr_t)((ws | cs) * 4)) & 15) == 0) { g.zmax = zmax; g.zmax_T = zmax_T; *zmax_done = true; }
+    return gemm(ctx, g);
+  }
   g.N = n; g.n_seg = 0;
   for (int j = 0; j < parts; j++) { g.B = W + j * ws; g.C = Y + j * cs; g.bias = bias ? bias + j * ws : nullptr; GN_TRY(gemm(ctx, g)); g.reuse_a_planes = true; }
   return GN_OK;
@@ -103,6 +108,14 @@ static int weight_bias_grads(gn_model* m, Ctx* ctx, int R, int N, int K, const f
   GemmDesc g; g.M = N; g.N = K; g.K = R; g.A = dZ; g.sa_m = 1; g.sa_k = ldz; g.B = X; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = K;
   if (gemm_on_tc(ctx, g)) GN_TRY(colsum(m, dZ, ldz, R, N, gb, false)); else g.a_sum = gb;
   return gemm(ctx, g);
+}
+
+// Does this weight gradient run on the side stream?  Only the CUDA-core engine's products can (no scratch), and only from some
+// 3 M multiply-adds on is it worth a fork and a join (a 1.3 M one in a step of small kernels cost 4 us more than it gave).
+static bool grads_on_side(Ctx* ctx, int stack, int R, int N, int K, long ldx) {
+  if ((double)stack * R * N * K < 3.0e6) return false;
+  GemmDesc g; g.M = N; g.N = K; g.K = R; g.sa_m = 1; g.sa_k = N; g.sb_k = ldx; g.sb_n = 1;
+  return !gemm_on_tc(ctx, g);
 }
 
 struct LayerRT;
@@ -180,12 +193,12 @@ namespace gn {
 // (beyond that the driver's own pageable copy, which overlaps its two stages, is the quicker way)
 constexpr size_t IO_ARGS = 64, STAGE_FLOATS = 1 << 18, STAGE_IN = 1 << 17;
 
-enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_COUNT };
+enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_SIDE, S_COUNT };
 
 static int ensure(gn_model* m, int slot, size_t n, float** out) {
   if ((int)m->scratch.size() < S_COUNT) m->scratch.resize(S_COUNT);
   DevBuf& b = m->scratch[slot];
-  if (b.n < n) { GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream)); m->epoch++; GN_TRY(b.alloc(n)); }
+  if (b.n < n) { GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream)); if (m->ctx->c.side_pending) GN_CUDA(cudaStreamSynchronize(m->ctx->c.side_stream)); m->epoch++; GN_TRY(b.alloc(n)); }
   *out = b.p; return GN_OK;
 }
 
@@ -394,9 +407,15 @@ template <bool RMS, int NV> struct NormRun {
     if ((n + 127) / 128 == NV) { GN_LAUNCH(ctx, (norm_fwd_vec_kernel<NV, RMS>), cdiv(rows, 8), 256, 0, x, ga, be, y, sa, sb, rows, n, eps, po); }
     else if constexpr (NV > 1) NormRun<RMS, NV - 1>::fwd(ctx, x, ga, be, y, sa, sb, rows, n, eps, po);
   }
-  static void bwd(Ctx* ctx, int blocks, const float* g, const float* x, const float* ga, const float* sa, const float* sb, float* dx, float* part, long rows, int n, const RowPlaneOut& po) {
-    if ((n + 127) / 128 == NV) { GN_LAUNCH(ctx, (norm_bwd_vec_kernel<NV, RMS>), blocks, 256, 0, g, x, ga, sa, sb, dx, part, rows, n, po); }
-    else if constexpr (NV > 1) NormRun<RMS, NV - 1>::bwd(ctx, blocks, g, x, ga, sa, sb, dx, part, rows, n, po);
+  static void bwd(Ctx* ctx, int blocks, const float* g, const float* x, const float* ga, const float* sa, const float* sb, float* dx, float* part, long rows, int n, long ldx, long lds, const RowPlaneOut& po) {
+    if ((n + 127) / 128 == NV) { GN_LAUNCH(ctx, (norm_bwd_vec_kernel<NV, RMS>), blocks, 256, 0, g, x, ga, sa, sb, dx, part, rows, n, ldx, lds, po); }
+    else if constexpr (NV > 1) NormRun<RMS, NV - 1>::bwd(ctx, blocks, g, x, ga, sa, sb, dx, part, rows, n, ldx, lds, po);
+  }
+};
+template <int NV> struct EmbedRun {
+  static void fwd(Ctx* ctx, const float* ids, const float* E, const float* P, float* out, long tokens, int T, int d, int V, int* idx, int row0_only, const RowPlaneOut& po) {
+    if ((d + 127) / 128 == NV) { GN_LAUNCH(ctx, embedding_fwd_vec_kernel<NV>, cdiv(tokens, 8), 256, 0, ids, E, P, out, tokens, T, d, V, idx, ctx->d_status, row0_only, po); }
+    else if constexpr (NV > 1) EmbedRun<NV - 1>::fwd(ctx, ids, E, P, out, tokens, T, d, V, idx, row0_only, po);
   }
 };
 static int norm_forward(Ctx* ctx, bool rms, const float* x, const float* gamma, const float* beta, float* y, float* stat, long rows, int n, float eps,
@@ -413,6 +432,19 @@ static int norm_forward(Ctx* ctx, bool rms, const float* x, const float* gamma, 
   }
   return check_launch("norm_forward");
 }
+// Register-row kernel: dx and the parameter sums from one reading of g and x; the blocks' partial sums are added by a second launch
+// unless there is only one.
+static int norm_backward_vec(gn_model* m, bool rms, const float* g, const float* x, long ldx, const float* gamma, const float* sa, const float* sb, long lds, float* dx,
+                             float* gGamma, float* gBeta, long rows, int n, const RowPlaneOut& out) {
+  Ctx* ctx = &m->ctx->c; float* part;
+  const int blocks = (int)std::max<long>(1, std::min<long>((rows + 7) / 8, (n <= 512 ? 2L : 1L) * ctx->sm_count));      // as many as are resident
+  const bool direct = blocks == 1 && (rms || gBeta == gGamma + n) && (reinterpret_cast<uintptr_t>(gGamma) & 15) == 0;
+  if (direct) part = gGamma; else GN_TRY(ensure(m, S_PART2, (size_t)blocks * 2 * n, &part));
+  if (rms) NormRun<true, 8>::bwd(ctx, blocks, g, x, gamma, sa, sb, dx, part, rows, n, ldx, lds, out);
+  else NormRun<false, 8>::bwd(ctx, blocks, g, x, gamma, sa, sb, dx, part, rows, n, ldx, lds, out);
+  if (!direct) GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, blocks, n, gGamma, rms ? nullptr : gBeta);
+  return check_launch("norm_backward");
+}
 // dx (may alias g), gGamma and gBeta (null for RMSNorm) are written.
 static int norm_backward(gn_model* m, bool rms, const float* g, const float* x, const float* gamma, const float* stat, float* dx, float* gGamma, float* gBeta, long rows, int n,
                          const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
@@ -420,12 +452,7 @@ static int norm_backward(gn_model* m, bool rms, const float* g, const float* x, 
   if (norm_vec_ok(n, {g, x, dx, gamma})) {
     const RowPlaneOut out = po ? *po : RowPlaneOut{};
     if (emitted) *emitted = out.p != nullptr;
-    const int blocks = (int)std::max<long>(1, std::min<long>((rows + 7) / 8, (n <= 512 ? 2L : 1L) * ctx->sm_count));      // as many as are resident
-    GN_TRY(ensure(m, S_PART2, (size_t)blocks * 2 * n, &part));
-    if (rms) NormRun<true, 8>::bwd(ctx, blocks, g, x, gamma, stat, stat, dx, part, rows, n, out);
-    else NormRun<false, 8>::bwd(ctx, blocks, g, x, gamma, stat, stat + rows, dx, part, rows, n, out);
-    GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, blocks, n, gGamma, rms ? nullptr : gBeta);
-    return check_launch("norm_backward");
+    return norm_backward_vec(m, rms, g, x, n, gamma, stat, rms ? stat : stat + rows, 1, dx, gGamma, gBeta, rows, n, out);
   }
   if (emitted) *emitted = false;
   const int chunks = (int)std::max<long>(1, std::min<long>(rows / 64, 128));
@@ -645,7 +672,10 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
     // the operand planes of the projections' input come from the norm that produced it (the previous block's) if it made any
     const BfPlanes* xp = m->fwd_planes_src == cur && m->fwd_planes.rows == N && m->fwd_planes.K == D ? &m->fwd_planes : nullptr;
     const long dd = (long)D * D + D;
-    if (!rows_only) GN_TRY(gemm_nt_stack(ctx, 3, N, D, D, cur, D, bp.wq, dd, bp.bq, l.q.p, l.k.p - l.q.p, xp));
+    const bool tc_att = !rows_only && use_fused_attention(d) && attn_tc_supported(ctx, hd, T, B, d.heads, D); bool zmax_done = false; int* zmax = nullptr;
+    AttnSaved* saved = training && !l.row0_grad ? &l.attn_saved : nullptr;      // planes of Q, K and V are kept for a backward pass that walks all queries
+    if (tc_att && !l.use_rope) GN_TRY(attn_tc_max_words(ctx, saved, B * d.heads, T, &zmax));
+    if (!rows_only) GN_TRY(gemm_nt_stack(ctx, 3, N, D, D, cur, D, bp.wq, dd, bp.bq, l.q.p, l.k.p - l.q.p, xp, zmax, T, &zmax_done));
     else {
       GN_TRY(gemm_nt_stack(ctx, 2, N, D, D, cur, D, bp.wk, dd, bp.bk, l.k.p, l.k.p - l.q.p, xp));
       GN_TRY(gemm_nt(ctx, NE, D, D, xe, ldx, bp.wq, bp.bq, l.q.p, D));
@@ -657,8 +687,7 @@ static int block_forward(gn_model* m, size_t li, int B, const float* cur, bool t
     }
     if (rows_only) GN_TRY(attn_rows_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, B, T, TE, D, d.heads, d.causal));
     else if (use_fused_attention(d)) {
-      // planes of Q, K and V are kept for a backward pass that walks all queries
-      if (attn_tc_supported(ctx, hd, T, B, d.heads, D)) GN_TRY(attn_tc_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal, training && !l.row0_grad ? &l.attn_saved : nullptr));
+      if (tc_att) GN_TRY(attn_tc_fwd(ctx, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal, saved, zmax_done));
       else GN_TRY(attn_fwd(ctx, hd, l.q.p, l.k.p, l.v.p, l.att.p, l.att_m.p, l.att_l.p, B, T, D, d.heads, d.causal));
     } else {
       float* P; GN_TRY(ensure(m, S_ATT0, (size_t)B * d.heads * T * T, &P));
@@ -802,7 +831,15 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
         if (fuse) P = m->params.p + m->L[li + 1].p_off;
         float* dst = fuse ? m->L[li + 1].out.p : l.out.p;
         l.out_rows = next_rows(m, fuse ? li + 1 : li, d.seq_len, d.out_size);
-        GN_LAUNCH(ctx, embedding_fwd_kernel, (unsigned)tokens, 128, 0, cur, p, P, dst, tokens, d.seq_len, d.out_size, d.in_size, (int*)l.idx.p, ctx->d_status, l.out_rows);
+        if (norm_vec_ok(d.out_size, {p, P, dst})) {
+          // a block that follows gets its projections' operand planes from here
+          RowPlaneOut po{}; const size_t nx = fuse ? li + 2 : li + 1;
+          if (!l.out_rows && nx < m->L.size() && m->L[nx].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[nx].d.dim == d.out_size && m->L[nx].d.seq_len == d.seq_len && norm_planes_wanted(ctx, (int)tokens, d.out_size, d.out_size)) {
+            GN_TRY(norm_planes_alloc(m, S_LNP1, S_LNI1, (int)tokens, d.out_size, &po, &m->fwd_planes, nullptr)); m->fwd_planes_src = dst;
+          }
+          EmbedRun<8>::fwd(ctx, cur, p, P, dst, tokens, d.seq_len, d.out_size, d.in_size, (int*)l.idx.p, l.out_rows, po);
+        } else
+          GN_LAUNCH(ctx, embedding_fwd_kernel, (unsigned)tokens, 128, 0, cur, p, P, dst, tokens, d.seq_len, d.out_size, d.in_size, (int*)l.idx.p, ctx->d_status, l.out_rows);
         cur = dst; if (fuse) { m->L[li + 1].out_rows = l.out_rows; li++; } break; }
       case GN_LAYER_POSENC: {
         long n = (long)B * l.out_size; l.out_rows = 0;
@@ -866,12 +903,21 @@ static int weight_bias_grads_stack(gn_model* m, int stack, int B, int out, int i
 }
 static int inner_dense_param_grads(gn_model* m, const float* dz, int B, int T, int out, const float* x, int in, float* gW, float* gb,
                                    const float* x_last = nullptr, const BfPlanes* dz_planes = nullptr, const float* dz_rowsum32 = nullptr, int stack = 1, long ws = 0) {
-  Ctx* ctx = &m->ctx->c; float* delta; GN_TRY(ensure(m, S_DELTA, (size_t)stack * B * out, &delta));
-  if (dz_rowsum32) GN_LAUNCH(ctx, token_sum_part32_kernel, dim3(cdiv(out, 512), B), 128, 0, dz_rowsum32, T / 32, out, delta);
-  else if (dz_planes) GN_LAUNCH(ctx, token_sum_planes_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, (const __half*)dz_planes->base, (const float*)dz_planes->inv_scale, (long)dz_planes->ldp, T, out, delta);
-  else GN_TRY(token_sums(ctx, dz, stack * B, T, out, delta));
-  return x_last ? weight_bias_grads_stack(m, stack, B, out, in, delta, x_last, (long)in, gW, gb, ws)
-                : weight_bias_grads_stack(m, stack, B, out, in, delta, x + (long)(T - 1) * in, (long)T * in, gW, gb, ws);
+  Ctx* ctx = &m->ctx->c; const bool side = grads_on_side(ctx, stack, B, out, in, in); float* delta;
+  GN_TRY(ensure(m, side ? S_SIDE : S_DELTA, (size_t)stack * B * out, &delta));
+  auto issue = [&]() -> int {
+    if (dz_rowsum32) GN_LAUNCH(ctx, token_sum_part32_kernel, dim3(cdiv(out, 512), B), 128, 0, dz_rowsum32, T / 32, out, delta);
+    else if (dz_planes) GN_LAUNCH(ctx, token_sum_planes_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, (const __half*)dz_planes->base, (const float*)dz_planes->inv_scale, (long)dz_planes->ldp, T, out, delta);
+    else GN_TRY(token_sums(ctx, dz, stack * B, T, out, delta));
+    return x_last ? weight_bias_grads_stack(m, stack, B, out, in, delta, x_last, (long)in, gW, gb, ws)
+                  : weight_bias_grads_stack(m, stack, B, out, in, delta, x + (long)(T - 1) * in, (long)T * in, gW, gb, ws);
+  };
+  return side ? side_run(ctx, issue) : issue();
+}
+// The gradients of a layer from dense rows of dz, beside the main stream where that is possible.
+static int side_weight_bias_grads(gn_model* m, int stack, int B, int out, int in, const float* dz, const float* x, long ldx, float* gW, float* gb, long ws = 0) {
+  Ctx* ctx = &m->ctx->c; auto issue = [&]() -> int { return weight_bias_grads_stack(m, stack, B, out, in, dz, x, ldx, gW, gb, ws); };
+  return grads_on_side(ctx, stack, B, out, in, ldx) ? side_run(ctx, issue) : issue();
 }
 // Can the FFN's hidden activation (and its gradient) of this block live as operand planes only?  The two contractions on
 // either side must both run on the tensor-core engine with prepared weight planes, and the plane-writing epilogue's shape
@@ -1015,14 +1061,15 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
   const float* gate_last = last(l.gate, kr.gate, F); const float* up_last = last(l.up, kr.up, F);
   const float* mid_last = l.mid_is_planes ? l.mid_last.p : last(l.mid, kr.mid, F); const long ld_mid = l.mid_is_planes ? F : ldF;
   float *dR2, *dR1, *comb, *dA, *dM;
-  GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, BD, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
+  GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, BD, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, 2 * BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
   auto norm = [&](const float* g, const float* x, const float* gamma, const float* stat, float* out, float* gG, float* gB) -> int {
+    if (norm_vec_ok(D, {g, x, gamma, out})) return norm_backward_vec(m, l.rms, g, x, ldD, gamma, stat, l.rms ? stat : stat + NE, TR, out, gG, gB, B, D, RowPlaneOut{});
     GN_LAUNCH(ctx, norm_bwd_rows_kernel, cdiv(B, 4), 128, 0, g, x, ldD, gamma, stat, l.rms ? nullptr : stat + NE, (long)TR, out, B, D);
     GN_LAUNCH(ctx, norm_pgrad_rows_kernel, cdiv(D, 32), 256, 0, g, x, ldD, stat, l.rms ? nullptr : stat + NE, (long)TR, B, D, gG, gB);
     return check_launch("norm_rows");
   };
   GN_TRY(norm(gout, r2_0, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2));
-  GN_TRY(weight_bias_grads(m, ctx, B, D, F, dR2, D, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
+  GN_TRY(side_weight_bias_grads(m, 1, B, D, F, dR2, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
   GemmDesc g; g.M = B; g.N = F; g.K = D; g.A = dR2; g.sa_m = D; g.sa_k = 1; g.B = bp.w2; g.sb_k = F; g.sb_n = 1; g.C = dM; g.ldc = F;
   if (l.ff_act == GN_ACT_RELU) { g.mask = mid_last; g.mask_ld = ld_mid; }
   GN_TRY(gemm(ctx, g));
@@ -1035,16 +1082,16 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
     GN_TRY(gemm_nn(ctx, B, F, D, dU, F, bp.v1, comb, D, comb, D));
   } else {
     if (l.ff_act == GN_ACT_GELU) GN_LAUNCH(ctx, scale_by_last_deriv_kernel, ew_grid(ctx, BF), 256, 0, dM, (const float*)l.zlast.p, 1, F, BF, (int)GN_ACT_GELU);
-    GN_TRY(weight_bias_grads(m, ctx, B, F, D, dM, F, n1_last, ldD, (float*)gp.w1, (float*)gp.b1));
+    GN_TRY(side_weight_bias_grads(m, 1, B, F, D, dM, n1_last, ldD, (float*)gp.w1, (float*)gp.b1));
     GN_TRY(gemm_nn(ctx, B, F, D, dM, F, bp.w1, comb, D, dR2, D));
   }
   GN_TRY(norm(comb, r1_0, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1));
-  GN_TRY(weight_bias_grads(m, ctx, B, D, D, dR1, D, att_last, ldD, (float*)gp.wo, (float*)gp.bo));
+  GN_TRY(side_weight_bias_grads(m, 1, B, D, D, dR1, att_last, ldD, (float*)gp.wo, (float*)gp.bo));
   GN_TRY(gemm_nn(ctx, B, D, D, dR1, D, bp.wo, dA, D));
   if (d.causal) {
     // the one probability of token 0 is 1: dV = dA at token 0, dQ = dK = 0
-    GN_CUDA(cudaMemsetAsync((void*)gp.wq, 0, (size_t)(gp.wv - gp.wq) * sizeof(float), ctx->stream));
-    GN_TRY(weight_bias_grads(m, ctx, B, D, D, dA, D, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
+    GN_TRY(side_run(ctx, [&]() -> int { GN_CUDA(cudaMemsetAsync((void*)gp.wq, 0, (size_t)(gp.wv - gp.wq) * sizeof(float), ctx->stream)); return GN_OK; }));
+    GN_TRY(side_weight_bias_grads(m, 1, B, D, D, dA, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
     GN_TRY(gemm_nn(ctx, B, D, D, dA, D, bp.wv, dx, D, dR1, D));
     *dx_row0 = true; return check_launch("block_backward_row0");
   }
@@ -1055,10 +1102,11 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
     rope(ctx, l, dK, nullptr, B * T, T, -1.f, 1);
     GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(D, 128), B), dim3(128, 4), 0, (const float*)dK, T, D, ks);
   }
-  GN_TRY(weight_bias_grads_stack(m, 3, B, D, D, dQ, x_last, ldX, (float*)gp.wq, (float*)gp.bq, (long)D * D + D));      // dQ | sum of dK | sum of dV
-  GN_TRY(gemm_nn(ctx, B, D, D, dQ, D, bp.wq, dR1, D, dR1, D));
+  GN_TRY(side_weight_bias_grads(m, 3, B, D, D, dQ, x_last, ldX, (float*)gp.wq, (float*)gp.bq, (long)D * D + D));      // dQ | sum of dK | sum of dV
+  float* dxq; GN_TRY(ensure(m, S_ND3, 2 * BD, &dxq)); dxq += BD;                           // (behind dA; dR1 may still be read on the side stream)
+  GN_TRY(gemm_nn(ctx, B, D, D, dQ, D, bp.wq, dxq, D, dR1, D));
   GN_TRY(gemm_nn_stack(ctx, 2, B * T, D, D, dK, ND, bp.wk, (long)D * D + D, dx, nullptr));
-  GN_LAUNCH(ctx, add_row0_kernel, B, 128, 0, (const float*)dR1, dx, T, D);
+  GN_LAUNCH(ctx, add_row0_kernel, B, 128, 0, (const float*)dxq, dx, T, D);
   *dx_row0 = false; return check_launch("block_backward_row0");
 }
 
@@ -1137,7 +1185,7 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
 
 static AdamArgs adam_args(float lr, float b1, float b2, float eps, int t, float grad_scale);
 static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, int64_t n, const AdamArgs& a, const AdamArgs* dargs, const int* status, cudaStream_t stream,
-                       const float* loss_sum, float* ret);
+                       const float* loss_sum, float* ret, const WeightPlaneTable* t = nullptr);
 
 static int backward(gn_model* m, int B, const float* gloss, int global_batch, int first_sample) {
   Ctx* ctx = &m->ctx->c;
@@ -1192,7 +1240,8 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
           else GN_LAUNCH(ctx, act_backward_kernel, ew_grid(ctx, n), 256, 0, g, d.activation == GN_ACT_RELU ? l.out.p : l.z.p, dzb, n, d.activation, act_alpha_of(d.activation, d.reserved));
           dz = dzb;
         }
-        GN_TRY(weight_bias_grads(m, ctx, B, d.out_size, d.in_size, dz, d.out_size, xin, d.in_size, gr, gr + wn));
+        if (need_dx) GN_TRY(side_weight_bias_grads(m, 1, B, d.out_size, d.in_size, dz, xin, d.in_size, gr, gr + wn));
+        else GN_TRY(weight_bias_grads(m, ctx, B, d.out_size, d.in_size, dz, d.out_size, xin, d.in_size, gr, gr + wn));
         gated = false;
         if (need_dx) {
           // a Dense(ReLU) below: its derivative, [activation > 0], gates this product's epilogue
@@ -1319,6 +1368,7 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         GN_TRY(norm_backward(m, true, g, xin, p, l.stat.p, dx, gr, nullptr, rows, d.dim)); g = dx; flip ^= 1;
         break; }
     }
+    GN_TRY(side_join(ctx));
     GN_TRY(check_launch("backward"));
     if (ctx->world > 1 && l.p_cnt > 0) {
       if (comm_at_end) deferred.push_back(li); else GN_TRY(layer_comm(li));
@@ -1340,8 +1390,12 @@ static AdamArgs adam_args(float lr, float b1, float b2, float eps, int t, float 
   return AdamArgs{effLR, b1, b2, 1.f - b1, 1.f - b2, eps, grad_scale};
 }
 static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, int64_t n, const AdamArgs& a, const AdamArgs* dargs, const int* status,
-                       cudaStream_t stream, const float* loss_sum, float* ret) {
-  adam_kernel<<<ew_grid(ctx, (n + 3) / 4), 256, 0, stream ? stream : ctx->stream>>>(p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret);
+                       cudaStream_t stream, const float* loss_sum, float* ret, const WeightPlaneTable* t) {
+  const unsigned grid = (unsigned)std::max<long>(1, std::min<long>(cdiv((n + 3) / 4, 256), 8L * ctx->sm_count)); stream = stream ? stream : ctx->stream;      // one resident round
+  if (t) {
+    GN_CUDA(cudaMemsetAsync(t->mx.p, 0, t->e.size() * sizeof(int), stream));
+    adam_kernel<true><<<grid, 256, 0, stream>>>(p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret, reinterpret_cast<const PlaneRange*>(t->ranges.p), (int)t->e.size(), reinterpret_cast<int*>(t->mx.p));
+  } else adam_kernel<false><<<grid, 256, 0, stream>>>(p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret, nullptr, 0, nullptr);
   ctx->launches++;
   return check_launch("adam");
 }
@@ -1394,7 +1448,8 @@ static int issue_backward(gn_model* m, const float* yp, const float* y_dev, int 
   }
   // Network.Step (net.go:260-284): NewStep() then StepInPlace with t = timestep + 1.  The pass reads the status word
   // first: after a bounded wait gave up it changes nothing.
-  return adam_launch(ctx, m->params.p, m->grads.p, m->m1.p, m->v2.p, m->P, a, reinterpret_cast<const AdamArgs*>(m->io.p), ctx->d_status, nullptr, m->loss_sum.p, ctx->d_ret);
+  return adam_launch(ctx, m->params.p, m->grads.p, m->m1.p, m->v2.p, m->P, a, reinterpret_cast<const AdamArgs*>(m->io.p), ctx->d_status, nullptr, m->loss_sum.p, ctx->d_ret,
+                     m->wplanes.used && !m->wplanes.e.empty() ? &m->wplanes : nullptr);
 }
 
 // Captured launches of a step (or of an inference pass).  A call whose sizes and buffers have been seen before is replayed as one or
@@ -1453,15 +1508,17 @@ static int train_step_issue(gn_model* m, const float* x, const float* y, bool ho
   const float inv = (float)(1.0 / (double)global_batch);                                        // net.go:703
   m->last_inv_batch = inv;
   const AdamArgs a = adam_args(m->lr, m->b1, m->b2, m->eps, m->timestep + 2, inv);
-  // small host batches go through one pinned block together with the coefficients: one copy instead of three
-  const bool staged = host && y_at + ny <= STAGE_IN;
+  GN_TRY(wplanes_need_max(ctx, m->wplanes));                   // (a captured step relies on them)
+  // small host batches (or a small x: token ids) go through one pinned block together with the coefficients: one copy instead of three
+  const bool staged = host && y_at + ny <= STAGE_IN, staged_x = staged || (host && nx * 4 < (128u << 10));
   memcpy(ctx->h_stage, &a, sizeof a);
   const float* xd = host ? m->io.p + IO_ARGS : x; const float* yd = host ? m->io.p + y_at : y;
-  if (staged) { memcpy(ctx->h_stage + IO_ARGS, x, nx * 4); memcpy(ctx->h_stage + y_at, y, ny * 4); }
+  if (staged_x) memcpy(ctx->h_stage + IO_ARGS, x, nx * 4);
+  if (staged) memcpy(ctx->h_stage + y_at, y, ny * 4);
   StepGraph key{B, global_batch, first_sample, xd, yd, staged, true};
   StepGraph* g = find_graph(m, key);
   const float* yp = nullptr;
-  auto copy_in = [&]() -> int { GN_CUDA(cudaMemcpyAsync(m->io.p, ctx->h_stage, (staged ? y_at + ny : IO_ARGS) * 4, cudaMemcpyHostToDevice, ctx->stream)); return GN_OK; };
+  auto copy_in = [&]() -> int { GN_CUDA(cudaMemcpyAsync(m->io.p, ctx->h_stage, (staged ? y_at + ny : staged_x ? IO_ARGS + nx : IO_ARGS) * 4, cudaMemcpyHostToDevice, ctx->stream)); return GN_OK; };
   auto first = [&]() -> int { return issue_forward(m, xd, B, global_batch, first_sample, &yp); };
   auto second = [&]() -> int { return issue_backward(m, yp, yd, B, global_batch, first_sample, a); };
   const bool split = host && !staged;                          // y is copied between the halves
@@ -1477,7 +1534,7 @@ static int train_step_issue(gn_model* m, const float* x, const float* y, bool ho
     if (g->refused) { g->drop(); m->wplanes.dirty = true; }
   }
   reset_counters(ctx);
-  if (split) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, x, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
+  if (split && !staged_x) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, x, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
   GN_CUDA(cudaEventRecord(m->ev0, ctx->stream));
   const bool replay = g && g->captured;
   if (replay) { GN_CUDA(cudaGraphLaunch(g->exec[0], ctx->stream)); }
@@ -1510,12 +1567,13 @@ static int train_step(gn_model* m, const float* x, const float* y, bool host, in
     // drain what was queued before the failure (both streams) so that nothing of this step runs after the call returned
     const std::string msg = last_error();
     if (ctx->comm_stream) cudaStreamSynchronize(ctx->comm_stream);
-    cudaStreamSynchronize(ctx->copy_stream); cudaStreamSynchronize(ctx->stream); cudaGetLastError();
-    last_error() = msg; return rc;
+    cudaStreamSynchronize(ctx->copy_stream); cudaStreamSynchronize(ctx->side_stream); cudaStreamSynchronize(ctx->stream); cudaGetLastError(); ctx->side_pending = false;
+    m->wplanes.dirty = true; m->wplanes.max_ok = false; last_error() = msg; return rc;
   }
   int st; memcpy(&st, &ctx->h_ret[1], sizeof(int));
-  if (st != 0) return clear_status(ctx, st);         // the Adam pass saw the same word and left parameters, moments and the step counter alone
+  if (st != 0) { m->wplanes.dirty = true; m->wplanes.max_ok = false; return clear_status(ctx, st); }         // the Adam pass saw the same word and left parameters, moments and the step counter alone
   m->timestep += 1;
+  m->wplanes.max_ok = m->wplanes.used;               // left behind by the update
   m->wplanes.dirty = !m->wplanes_layerwise;          // the parameters moved: their operand planes are stale, unless they were renewed layer by layer behind the update
   m->wplanes_layerwise = false;
   if (mean_loss) *mean_loss = ctx->h_ret[0] / (float)global_batch;
@@ -1578,6 +1636,9 @@ static int make_ctx(int device, int rank, int world, const unsigned char* id, gn
       if (c->c.tc_queue_pool) cudaFree(c->c.tc_queue_pool);
       if (c->c.copy_ev) cudaEventDestroy(c->c.copy_ev);
       if (c->c.copy_stream) cudaStreamDestroy(c->c.copy_stream);
+      if (c->c.fork_ev) cudaEventDestroy(c->c.fork_ev);
+      if (c->c.join_ev) cudaEventDestroy(c->c.join_ev);
+      if (c->c.side_stream) cudaStreamDestroy(c->c.side_stream);
       if (c->c.stream) cudaStreamDestroy(c->c.stream);
       delete c; } } guard{new gn_ctx()};
   gn_ctx* c = guard.c;
@@ -1585,6 +1646,8 @@ static int make_ctx(int device, int rank, int world, const unsigned char* id, gn
   if (const char* e = getenv("GONEURON_CUDA_SM_RESERVE")) c->c.sm_reserve = std::max(0, std::min(atoi(e), prop.multiProcessorCount / 2));
   GN_CUDA(cudaStreamCreateWithFlags(&c->c.stream, cudaStreamNonBlocking));
   GN_CUDA(cudaStreamCreateWithFlags(&c->c.copy_stream, cudaStreamNonBlocking)); GN_CUDA(cudaEventCreateWithFlags(&c->c.copy_ev, cudaEventDisableTiming));
+  GN_CUDA(cudaStreamCreateWithFlags(&c->c.side_stream, cudaStreamNonBlocking));
+  GN_CUDA(cudaEventCreateWithFlags(&c->c.fork_ev, cudaEventDisableTiming)); GN_CUDA(cudaEventCreateWithFlags(&c->c.join_ev, cudaEventDisableTiming));
   GN_CUDA(cudaMalloc(&c->c.d_status, 4 * sizeof(int)));      // status word | ticket of the loss kernels | a scratch word
   GN_CUDA(cudaMemsetAsync(c->c.d_status, 0, 4 * sizeof(int), c->c.stream)); GN_CUDA(cudaStreamSynchronize(c->c.stream));
   GN_CUDA(cudaHostAlloc((void**)&c->c.h_block, (2 * STAGE_FLOATS + 64) * sizeof(float), cudaHostAllocMapped));
@@ -1648,6 +1711,9 @@ int gn_shutdown(gn_ctx* ctx) {
   if (ctx->c.t0) { cudaEventDestroy(ctx->c.t0); cudaEventDestroy(ctx->c.t1); ctx->c.t0 = ctx->c.t1 = nullptr; }
   if (ctx->c.copy_ev) { cudaEventDestroy(ctx->c.copy_ev); ctx->c.copy_ev = nullptr; }
   if (ctx->c.copy_stream) { cudaStreamDestroy(ctx->c.copy_stream); ctx->c.copy_stream = nullptr; }
+  if (ctx->c.fork_ev) { cudaEventDestroy(ctx->c.fork_ev); ctx->c.fork_ev = nullptr; }
+  if (ctx->c.join_ev) { cudaEventDestroy(ctx->c.join_ev); ctx->c.join_ev = nullptr; }
+  if (ctx->c.side_stream) { cudaStreamDestroy(ctx->c.side_stream); ctx->c.side_stream = nullptr; }
   if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
   if (ctx->c.comm_stream) cudaStreamDestroy(ctx->c.comm_stream);
   ctx->c.comm_stream = nullptr;
@@ -1766,7 +1832,7 @@ int gn_model_set_params(gn_model* m, const float* host, int64_t n) {
   CHECK_MODEL(m); if (!host || n != m->P) return fail(GN_ERR_INVALID_ARG, "set_params: expected %lld floats, got %lld", (long long)m->P, (long long)n);
   std::lock_guard<std::mutex> lk(m->mu); USE_DEVICE(m);
   GN_CUDA(cudaMemcpyAsync(m->params.p, host, (size_t)n * 4, cudaMemcpyHostToDevice, m->ctx->c.stream));
-  m->wplanes.dirty = true;
+  m->wplanes.dirty = true; m->wplanes.max_ok = false;
   GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream)); return GN_OK;
 }
 int gn_model_get_params(gn_model* m, float* host, int64_t n) {

@@ -106,7 +106,7 @@ __global__ void loss_rows_kernel(const float* __restrict__ p, const float* __res
 // the gradient that reaches z (the loss gradient through the head's Jacobian, see head_jacobian_kernel).  A cluster of `cs`
 // blocks holds one row in registers, E values per thread; the four reductions (maximum, exponential sum, and loss and Jacobian
 // sum together) meet in distributed shared memory.  Three kernels of one block per row (softmax, loss, Jacobian) read
-// the row nine times: 180 us for 64 rows of 32000, against 21 now.
+// the row nine times: 172 us for 64 rows of 32000, against 31 now.
 constexpr int HEAD_THREADS = 256, HEAD_MAX_CS = 8, HEAD_MAX_E = 16;
 template <int E>
 __global__ void __launch_bounds__(HEAD_THREADS) head_loss_kernel(const float* __restrict__ z, const float* __restrict__ y, float* __restrict__ dz, float* __restrict__ loss,
@@ -403,12 +403,13 @@ __global__ void __launch_bounds__(256) norm_fwd_vec_kernel(const float* __restri
   row_store(v, y + row * n, n, lane);
   if (po.p) row_planes_emit(v, row, n, lane, po);
 }
+// Rows of g and dx are dense, row r of x lies at x + r ldx and its statistics at stat[r lds].
 // dx (may alias g), and this block's part of the parameter gradients: part[block][0] = sum g (x - mean) / sd (RMS: sum g x / rms),
 // part[block][1] = sum g.  The warps stride over the rows with the sums of their columns in registers, so g and x are read
 // once for both outputs (two passes before, the second at 1 TB/s: 18 of 25 us at 3600 rows of 384).
 template <int NV, bool RMS>
 __global__ void __launch_bounds__(256) norm_bwd_vec_kernel(const float* g, const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ stat_a,
-                                                           const float* __restrict__ stat_b, float* dx, float* __restrict__ part, long rows, int n, const RowPlaneOut po) {
+                                                           const float* __restrict__ stat_b, float* dx, float* __restrict__ part, long rows, int n, long ldx, long lds, const RowPlaneOut po) {
   __shared__ float4 red[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5; const float fn = (float)n;
   float4 ga[NV], sg_[NV], sb_[NV];
@@ -416,8 +417,8 @@ __global__ void __launch_bounds__(256) norm_bwd_vec_kernel(const float* g, const
   for (int k = 0; k < NV; k++) sg_[k] = sb_[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   row_load(ga, gamma, n, lane);
   for (long row = (long)blockIdx.x * 8 + w; row < rows; row += (long)gridDim.x * 8) {
-    float4 q[NV], d[NV]; row_load(q, g + row * n, n, lane); row_load(d, x + row * n, n, lane);
-    const float a = stat_a[row];
+    float4 q[NV], d[NV]; row_load(q, g + row * n, n, lane); row_load(d, x + row * ldx, n, lane);
+    const float a = stat_a[row * lds];
     float s = 0.f, sx = 0.f;
     if (RMS) {
       const float inv = 1.f / a;
@@ -431,7 +432,7 @@ __global__ void __launch_bounds__(256) norm_bwd_vec_kernel(const float* g, const
       for (int k = 0; k < NV; k++)
         q[k] = make_float4((ga[k].x * inv) * (q[k].x - d[k].x * f), (ga[k].y * inv) * (q[k].y - d[k].y * f), (ga[k].z * inv) * (q[k].z - d[k].z * f), (ga[k].w * inv) * (q[k].w - d[k].w * f));
     } else {
-      const float sd = stat_b[row], isd = 1.f / sd;
+      const float sd = stat_b[row * lds], isd = 1.f / sd;
 #pragma unroll
       for (int k = 0; k < NV; k++) {
         if (4 * lane + 128 * k < n) { d[k].x -= a; d[k].y -= a; d[k].z -= a; d[k].w -= a; }
@@ -600,6 +601,26 @@ __global__ void embedding_fwd_kernel(const float* __restrict__ ids, const float*
   const float* e = E + (long)id * d; float* o = out + (row0_only ? tok / T : tok) * d;
   if (P) { const float* p = P + (long)(tok % T) * d; for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = e[i] + p[i]; }
   else for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = e[i];
+}
+// The same with rows in registers (d <= 1024, a multiple of four, 16-byte rows), one warp per token; optionally the row as operand planes
+// for the projections of the block above.  Memory-bound; a block of 128 threads per token moved 268 MB in 85 us.
+template <int NV>
+__global__ void __launch_bounds__(256) embedding_fwd_vec_kernel(const float* __restrict__ ids, const float* __restrict__ E, const float* __restrict__ P, float* __restrict__ out, long tokens, int T, int d,
+                                                                int V, int* __restrict__ idx_out, int* __restrict__ status, int row0_only, const RowPlaneOut po) {
+  const long tok = (long)blockIdx.x * 8 + (threadIdx.x >> 5); if (tok >= tokens) return;
+  const int lane = threadIdx.x & 31; const float fid = ids[tok]; int id = (int)floorf(fid);
+  if (id < 0 || id >= V || !(fid == fid)) { if (lane == 0) atomicCAS(status, 0, GN_STATUS_BAD_TOKEN); id = id < 0 ? 0 : V - 1; }
+  if (lane == 0 && idx_out) idx_out[tok] = id;
+  if (row0_only && tok % T) return;
+  float4 v[NV]; row_load(v, E + (long)id * d, d, lane);
+  if (P) {
+    float4 p[NV]; row_load(p, P + (long)(tok % T) * d, d, lane);
+#pragma unroll
+    for (int k = 0; k < NV; k++) { v[k].x += p[k].x; v[k].y += p[k].y; v[k].z += p[k].z; v[k].w += p[k].w; }
+  }
+  const long row = row0_only ? tok / T : tok;
+  row_store(v, out + row * d, d, lane);
+  if (po.p) row_planes_emit(v, row, d, lane, po);
 }
 __global__ void posenc_fwd_kernel(const float* __restrict__ x, const float* __restrict__ P, float* __restrict__ out, long total, long per_sample) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) out[i] = x[i] + P[i % per_sample];
@@ -889,8 +910,12 @@ __global__ void scale_kernel(float* __restrict__ x, long n, float s) {
 // `dargs` (may be null): the coefficients are read from there instead of `a`, so that a captured launch follows the schedule.
 // `ret` (may be null; host memory): receives the step's loss sum and the status word, the caller's one read-back.
 struct AdamArgs { float effLR, b1, b2, omb1, omb2, eps, grad_scale; };
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, long n, const AdamArgs a, const AdamArgs* __restrict__ dargs,
-                            const int* __restrict__ status, const float* __restrict__ loss_sum, float* __restrict__ ret) {
+// `ranges` (MX): parameter ranges whose largest magnitude after the update is wanted, ascending; mx[j] (zero on entry) receives that of
+// range j -- the operand planes of the weight matrices are scaled by it, and finding it here saves a pass over all of them.  A
+// warp keeps the maximum of the range it is in in registers and hands it over when it leaves the range.  Memory-bound either way (28 bytes per parameter).
+template <bool MX>
+__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, long n, const AdamArgs a, const AdamArgs* __restrict__ dargs,
+                                                   const int* __restrict__ status, const float* __restrict__ loss_sum, float* __restrict__ ret, const PlaneRange* __restrict__ ranges, int nr, int* __restrict__ mx) {
   if (ret && blockIdx.x == 0 && threadIdx.x == 0) { ret[0] = *loss_sum; ret[1] = __int_as_float(*status); }
   if (status && *status != 0) return;
   const AdamArgs c = dargs ? *dargs : a;
@@ -907,14 +932,44 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
     vv = __fadd_rn(__fmul_rn(b2, vv), __fmul_rn(__fmul_rn(omb2, gs), gs));
     pp = __fsub_rn(pp, __fdiv_rn(__fmul_rn(effLR, mm), __fadd_rn(__fsqrt_rn(vv), eps)));
   };
-  const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x, nthreads = (long)gridDim.x * blockDim.x;
-  for (long i = tid; i < n4; i += nthreads) {
-    float4 P = p4[i], G = g4[i], M = m4[i], V = v4[i];
-    upd(P.x, G.x, M.x, V.x); upd(P.y, G.y, M.y, V.y); upd(P.z, G.z, M.z, V.z); upd(P.w, G.w, M.w, V.w);
-    p4[i] = P; m4[i] = M; v4[i] = V;
+  int j = 0; const float *js = nullptr, *je = nullptr; float mxv = 0.f; const int lane = threadIdx.x & 31;
+  auto one = [&](const float* q, float x, int from) {        // a parameter near a range's edge
+    for (int k = from; k < nr && ranges[k].b <= q; k++) if (q < ranges[k].e) atomicMax(mx + k, __float_as_int(fabsf(x)));
+  };
+  auto flush = [&]() {                                       // (the whole warp)
+    const float t = warp_max(mxv); mxv = 0.f;
+    if (lane == 0 && t > 0.f && t > __int_as_float(*(volatile int*)(mx + j))) atomicMax(mx + j, __float_as_int(t));
+  };
+  // (chunks of at most 32 KB per array, block by block: one contiguous run per block was 12 % slower at 134 M parameters)
+  const long chunk = max(256L, min(2048L, ((n4 + gridDim.x - 1) / gridDim.x + 255) & ~255L));
+  for (long i0 = blockIdx.x * chunk; i0 < n4; i0 += gridDim.x * chunk) {
+    const long i1 = min(n4, i0 + chunk);
+    for (long base = i0 + (threadIdx.x & ~31); base < i1; base += 256) {
+      const long i = base + lane; const bool act = i < i1; float4 P = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (act) {
+        const float4 G = g4[i]; float4 M = m4[i], V = v4[i]; P = p4[i];
+        upd(P.x, G.x, M.x, V.x); upd(P.y, G.y, M.y, V.y); upd(P.z, G.z, M.z, V.z); upd(P.w, G.w, M.w, V.w);
+        p4[i] = P; m4[i] = M; v4[i] = V;
+      }
+      if (MX) {
+        const float* w0 = p + head + 4 * base; const float* q = w0 + 4 * lane;
+        if (j < nr && w0 >= je) {                            // on to the first range that ends behind the warp's first parameter
+          if (je) flush();
+          int lo = j, hi = nr;
+          while (lo < hi) { const int mid = (lo + hi) >> 1; if (ranges[mid].e > w0) hi = mid; else lo = mid + 1; }
+          j = lo; if (j < nr) { js = ranges[j].b; je = ranges[j].e; }
+        }
+        if (j < nr && act) {
+          if (q >= js && q + 4 <= je) mxv = fmaxf(mxv, fmaxf(fmaxf(fabsf(P.x), fabsf(P.y)), fmaxf(fabsf(P.z), fabsf(P.w))));
+          else if (q + 4 > js) { one(q, P.x, j); one(q + 1, P.y, j); one(q + 2, P.z, j); one(q + 3, P.w, j); }
+        }
+      }
+    }
   }
-  if (tid < head) upd(p[tid], g[tid], m[tid], v[tid]);
-  for (long i = head + (n4 << 2) + tid; i < n; i += nthreads) upd(p[i], g[i], m[i], v[i]);
+  if (MX && j < nr) flush();
+  const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x, nthreads = (long)gridDim.x * blockDim.x;
+  if (tid < head) { upd(p[tid], g[tid], m[tid], v[tid]); if (MX) one(p + tid, p[tid], 0); }
+  for (long i = head + (n4 << 2) + tid; i < n; i += nthreads) { upd(p[i], g[i], m[i], v[i]); if (MX) one(p + i, p[i], 0); }
 }
 
 
