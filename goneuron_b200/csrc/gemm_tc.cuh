@@ -685,6 +685,58 @@ __global__ void __launch_bounds__(256) split2_cols_kernel(TcSrc s, int rows, int
   }
 }
 
+// Both passes in one launch, the source read once: a cluster of up to eight blocks owns 32 plane rows, each block a run of
+// contraction indices, kept in shared memory (rows of 33 floats: free of bank conflicts both ways) between the row maxima --
+// combined through the cluster -- and the planes.  Memory-bound.  For contractions of up to SPLIT_T_MAX indices (the run has to fit);
+// [1000, 1100] and [4096, 2816] transposed took 16 and 33 us in two passes and a memset.
+constexpr int SPLIT_T_CLUSTER = 8, SPLIT_T_RUN = 1536, SPLIT_T_MAX = SPLIT_T_CLUSTER * SPLIT_T_RUN;
+__global__ void __launch_bounds__(256) split2_cols_cluster_kernel(TcSrc s, int rows, int cols, __half* __restrict__ pl, float* __restrict__ inv_scale, int ldp, int per, int cs) {
+  extern __shared__ float slab[];                           // [per][33]
+  __shared__ float red[8][32], mxs[32];
+  const int z = blockIdx.y, rank = blockIdx.x % cs, r0 = blockIdx.x / cs * 32, k0 = rank * per, k1 = min(ldp, k0 + per), t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const float* src = s.p + (z / s.batch2) * s.b1 + (z % s.batch2) * s.b2;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(s.s_c * 4)) & 15) == 0 && r0 + 32 <= rows;
+  const int c4 = (t & 7) * 4, ko = t >> 3;                  // this thread: columns c4 .. c4 + 3 of stored rows k0 + ko + 32 i
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int k = k0 + ko; k < k1; k += 32) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k < cols) {
+      const float* q = src + (long)k * s.s_c + r0 + c4;
+      if (vec) v = *reinterpret_cast<const float4*>(q);
+      else { if (r0 + c4 < rows) v.x = q[0]; if (r0 + c4 + 1 < rows) v.y = q[1]; if (r0 + c4 + 2 < rows) v.z = q[2]; if (r0 + c4 + 3 < rows) v.w = q[3]; }
+    }
+    float* d = slab + (k - k0) * 33 + c4; d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+    m[0] = fmaxf(m[0], fabsf(v.x)); m[1] = fmaxf(m[1], fabsf(v.y)); m[2] = fmaxf(m[2], fabsf(v.z)); m[3] = fmaxf(m[3], fabsf(v.w));
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    m[j] = fmaxf(m[j], __shfl_xor_sync(0xffffffffu, m[j], 8)); m[j] = fmaxf(m[j], __shfl_xor_sync(0xffffffffu, m[j], 16));
+    if (lane < 8) red[w][c4 + j] = m[j];
+  }
+  __syncthreads();
+  if (t < 32) { float v = red[0][t]; for (int q = 1; q < 8; q++) v = fmaxf(v, red[q][t]); mxs[t] = v; }
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  if (t < 32) {
+    float v = 0.f;
+    for (int q = 0; q < cs; q++) v = fmaxf(v, cluster.map_shared_rank(mxs, q)[t]);
+    if (!(v <= 3.0e38f)) v = 3.4e38f;                       // an infinity in the column: row_scale() then uses s = 1
+    float inv; red[0][t] = row_scale(v, &inv);
+    if (rank == 0 && r0 + t < rows) inv_scale[(long)z * rows + r0 + t] = inv;
+  }
+  cluster.sync();                                           // (also: nobody leaves while its maxima are being read)
+  for (int kb = k0 + 32 * w; kb < k1; kb += 256)            // a warp per block of 32 contraction indices, four plane rows at a time
+#pragma unroll 2
+    for (int i = 0; i < 32; i += 4) {
+      const int r = i + (lane >> 3), k = (lane & 7) * 4; const float sc = red[0][r]; const float* q = slab + (kb - k0 + k) * 33 + r;
+      if (r0 + r >= rows) continue;
+      uint2 a, b; split2_pair(q[0], q[33], sc, a.x, b.x); split2_pair(q[66], q[99], sc, a.y, b.y);
+      __half* o = pl + ((long)z * rows + r0 + r) * 2 * ldp + pl_off(kb + k);
+      *reinterpret_cast<uint2*>(o) = a; *reinterpret_cast<uint2*>(o + PL_LO) = b;
+    }
+}
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                     CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -767,6 +819,14 @@ inline int tc_split(Ctx* ctx, const TcSrc& src, const BfPlanes& p, int* mx, floa
     GN_LAUNCH(ctx, split2_rows_kernel, dim3(cdiv(p.rows, 8), p.nbatch), 256, 0, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, rownorm);
   } else if (src.s_r == 1) {
     if (p.nbatch > 65535 || cdiv(p.rows, 64) > 65535 || cdiv(p.K, 256) > 65535) return fail(GN_ERR_UNSUPPORTED, "tc_split: operand too large for the transposing split");
+    if (p.ldp <= SPLIT_T_MAX) {
+      int cs = 1; while (cs < SPLIT_T_CLUSTER && p.ldp > 64 * cs) cs *= 2;
+      const int per = cdiv(cdiv(p.ldp, cs), 32) * 32, smem = per * 33 * (int)sizeof(float);
+      if (smem > 40 * 1024) GN_CUDA(cudaFuncSetAttribute(split2_cols_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      GN_CUDA(launch_kernel(ctx->stream, split2_cols_cluster_kernel, dim3(cdiv(p.rows, 32) * cs, p.nbatch), dim3(256), (size_t)smem, cs, false, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, per, cs));
+      ctx->launches++; ctx->split_bytes += 8.0 * (double)p.nbatch * p.rows * p.K;
+      return check_launch("tc_split");
+    }
     if (!mx) return fail(GN_ERR_INVALID_ARG, "tc_split: the transposing split needs a row-maximum buffer");
     GN_CUDA(cudaMemsetAsync(mx, 0, (size_t)p.nbatch * p.rows * sizeof(int), ctx->stream));
     GN_LAUNCH(ctx, colmax_kernel, dim3(cdiv(p.rows, 64), cdiv(p.K, 256), p.nbatch), 256, 0, src, p.rows, p.K, mx);

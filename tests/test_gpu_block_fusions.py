@@ -133,3 +133,29 @@ def test_gradients_beside_the_main_stream(device, pool, masks):
         got.append(([model.TrainBatch(x, y) for _ in range(6)], model.Params().copy()))
         model.Close()
     assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("R,N,K", [(40, 4200, 1040), (1000, 333, 1100), (4099, 256, 608), (12290, 96, 160)])
+def test_weight_gradients_from_transposed_splits(device, oracle, R, N, K):
+    """Dense weight gradients dZ^T X on the tensor cores: both operands are transposed on their way into planes.  One block per 32
+    columns up to a full cluster, ragged rows and columns, rows without 16-byte alignment, and (the last) a contraction that does not
+    fit the cluster's shared memory."""
+    layers = [D.Dense(K, N, D.TANH), D.Dense(N, 3, D.LINEAR)]
+    from goneuron_b200.sequential import Adam, Sequential
+    rng = np.random.Generator(np.random.PCG64(R))
+    params = configs.init_params(layers, rng)
+    x, y = rng.standard_normal((R, K)).astype(np.float32), rng.standard_normal((R, 3)).astype(np.float32)
+    model = Sequential(layers, device).Compile(Adam(1e-4), D.MSE)
+    model.SetParams(params)
+    model.TrainBatch(x, y)
+    g = model.Gradients()
+    model.Close()
+    W1, b1 = params[:K * N].reshape(N, K).astype(np.float64), params[K * N:K * N + N].astype(np.float64)
+    o = K * N + N
+    W2, b2 = params[o:o + 3 * N].reshape(3, N).astype(np.float64), params[o + 3 * N:o + 3 * N + 3].astype(np.float64)
+    X = x.astype(np.float64)
+    a = np.tanh(X @ W1.T + b1)
+    u = 2.0 * (a @ W2.T + b2 - y) / 3.0
+    dz = (u @ W2) * (1.0 - a * a)
+    for got, ref in ((g[:K * N].reshape(N, K), dz.T @ X), (g[K * N:o], dz.sum(0)), (g[o:o + 3 * N].reshape(3, N), u.T @ a)):
+        assert norm_err(got, ref / R) <= TOL
