@@ -328,11 +328,11 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 3 : 4) attn_bwd_kernel(
 // top block below a CLSPooling needs (plan_token_rows in model.cu).  Q and O are [B * TE, D], K and V [B * T, D].  One block per
 // (head, sequence); a thread forms the scores of its keys (16-byte loads along a key's row where they are aligned: `vec`), then
 // the threads split into groups of hd columns for the weighted sum.  Bound by reading K and V once.
-constexpr int AR_THREADS = 256;
+constexpr int AR_THREADS = 512;                             // (64 heads of 64 and 384 keys: 9.6 us, 15 with 256 threads and four loads in flight)
 __device__ __forceinline__ float ar_dot(const float* __restrict__ q, const float* __restrict__ k, int hd, bool vec) {
   float s = 0.f;
   if (vec) {
-#pragma unroll 4
+#pragma unroll 8
     for (int d = 0; d < hd; d += 4) {
       const float4 x = *reinterpret_cast<const float4*>(k + d);
       s = fmaf(q[d], x.x, s); s = fmaf(q[d + 1], x.y, s); s = fmaf(q[d + 2], x.z, s); s = fmaf(q[d + 3], x.w, s);

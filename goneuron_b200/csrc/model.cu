@@ -389,7 +389,8 @@ static inline unsigned ew_grid(Ctx* ctx, long n, int block = 256) { long g = (n 
 // out[c] (=|+=) sum over R rows of in[r*ld + c]
 static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate) {
   Ctx* ctx = &m->ctx->c;
-  int chunks = std::max(1, std::min(R / 64, 128));
+  // slabs of 16 rows and up for a batch (bound by the latency of a slab's loads), of 64 and up for many rows
+  const int chunks = std::max(1, R <= 1024 ? std::min(R / 16, 16) : std::min(R / 64, 128));
   float* part; GN_TRY(ensure(m, S_PART, (size_t)chunks * C * 2, &part));
   GN_LAUNCH(ctx, colsum_partial_kernel, dim3(cdiv(C, 128), chunks), 128, 0, in, ld, R, C, part);
   GN_LAUNCH(ctx, colsum_final_kernel, cdiv(C, 128), 128, 0, part, chunks, C, out, accumulate ? 1 : 0);
@@ -771,7 +772,7 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
           GN_TRY(gemm_nt(ctx, B, d.out_size, d.in_size, cur, d.in_size, W, bias, l.z.p, d.out_size));
           if (m->head_fused && li + 1 == m->L.size()) {}     // head_loss_kernel takes z
           else if (d.activation == GN_ACT_SOFTMAX || d.activation == GN_ACT_LOGSOFTMAX)
-            GN_LAUNCH(ctx, softmax_rows_kernel, B, 256, 0, l.z.p, l.out.p, d.out_size, d.activation == GN_ACT_LOGSOFTMAX ? 1 : 0);
+            GN_LAUNCH(ctx, softmax_rows_kernel, B, d.out_size >= 2048 ? 1024 : 256, 0, l.z.p, l.out.p, d.out_size, d.activation == GN_ACT_LOGSOFTMAX ? 1 : 0);
           else { long n = (long)B * d.out_size; GN_LAUNCH(ctx, act_forward_kernel, ew_grid(ctx, n), 256, 0, l.z.p, l.out.p, n, d.activation, act_alpha_of(d.activation, d.reserved)); }
         }
         cur = l.out.p; break; }
