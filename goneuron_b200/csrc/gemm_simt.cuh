@@ -53,7 +53,7 @@ struct GemmDesc {
 // these products need: they come from small batches and narrow layers (a [64, 784] x [784, 128] forward product, a
 // [96, 96] weight gradient over 5000 rows), where a single 128 x 128 tile per block left all but a few SMs idle and one block
 // walking the whole contraction -- 72 us for the former and 430 us for the latter, against 7 and 13 us now.
-// Global loads of a k-step go to registers while the previous one is multiplied, then to the other shared-memory buffer.
+// Global loads of a k-step go to registers while the two before it are multiplied, then to the other shared-memory buffer.
 // 16-byte loads along the operand's fast index where base, stride and range allow it.
 constexpr int SG_PAD = 4, SG_MAX_SPLITS = 8, SG_RUN = 32;      // runs start at multiples of SG_RUN, whatever the tile
 template <int BM, int BN, int BK, int TM, int TN> struct SgCfg {
@@ -145,39 +145,46 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
   const bool want_asum = g.a_sum != nullptr && nt == 0;
   float asum = 0.f;
 
-  SgSlab<BM, BK, THREADS, A_KFAST> fa; SgSlab<BN, BK, THREADS, !B_NFAST> fb;
-  auto fetch = [&](int k0) {
+  // two register sets: the loads of a k-step are issued two steps ahead (the products are short chains of steps, each of which
+  // would otherwise wait for most of a memory latency)
+  struct Step { SgSlab<BM, BK, THREADS, A_KFAST> a; SgSlab<BN, BK, THREADS, !B_NFAST> b; };
+  Step s0, s1; int buf = 0;
+  auto fetch = [&](Step& s, int k0) {
     const int nk = kend - k0;
-    fa.fetch(A + (long)m0 * g.sa_m + (long)k0 * g.sa_k, g.sa_m, g.sa_k, g.M - m0, nk, vec_a);
-    fb.fetch(B + (long)n0 * g.sb_n + (long)k0 * g.sb_k, g.sb_n, g.sb_k, g.N - n0, nk, vec_b);
+    s.a.fetch(A + (long)m0 * g.sa_m + (long)k0 * g.sa_k, g.sa_m, g.sa_k, g.M - m0, nk, vec_a);
+    s.b.fetch(B + (long)n0 * g.sb_n + (long)k0 * g.sb_k, g.sb_n, g.sb_k, g.N - n0, nk, vec_b);
+  };
+  auto step = [&](Step& next, Step& after, int k0) {          // `next` holds k-step k0 + BK
+    if (k0 + 2 * BK < kend) fetch(after, k0 + 2 * BK);
+    const float* As = sm + buf * Cfg::STAGE; const float* Bs = As + BK * LDA;
+#pragma unroll
+    for (int k = 0; k < BK; k++) {
+      float av[TM], bv[TN];
+#pragma unroll
+      for (int i = 0; i < TM; i++) av[i] = As[k * LDA + ty * TM + i];
+#pragma unroll
+      for (int j = 0; j < TN; j++) bv[j] = Bs[k * LDB + tx * TN + j];
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    if (want_asum && t < BM) {
+#pragma unroll
+      for (int k = 0; k < BK; k++) asum += As[k * LDA + t];
+    }
+    buf ^= 1;
+    if (k0 + BK < kend) { float* nx = sm + buf * Cfg::STAGE; next.a.put(nx, LDA); next.b.put(nx + BK * LDA, LDB); }
+    __syncthreads();
   };
   if (kbeg < kend) {
-    fetch(kbeg);
-    fa.put(sm, LDA); fb.put(sm + BK * LDA, LDB);
+    fetch(s0, kbeg);
+    if (kbeg + BK < kend) fetch(s1, kbeg + BK);
+    s0.a.put(sm, LDA); s0.b.put(sm + BK * LDA, LDB);
     __syncthreads();
-    int buf = 0;
-    for (int k0 = kbeg; k0 < kend; k0 += BK, buf ^= 1) {
-      const bool more = k0 + BK < kend;
-      if (more) fetch(k0 + BK);
-      const float* As = sm + buf * Cfg::STAGE; const float* Bs = As + BK * LDA;
-#pragma unroll
-      for (int k = 0; k < BK; k++) {
-        float av[TM], bv[TN];
-#pragma unroll
-        for (int i = 0; i < TM; i++) av[i] = As[k * LDA + ty * TM + i];
-#pragma unroll
-        for (int j = 0; j < TN; j++) bv[j] = Bs[k * LDB + tx * TN + j];
-#pragma unroll
-        for (int i = 0; i < TM; i++)
-#pragma unroll
-          for (int j = 0; j < TN; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-      }
-      if (want_asum && t < BM) {
-#pragma unroll
-        for (int k = 0; k < BK; k++) asum += As[k * LDA + t];
-      }
-      if (more) { float* nx = sm + (buf ^ 1) * Cfg::STAGE; fa.put(nx, LDA); fb.put(nx + BK * LDA, LDB); }
-      __syncthreads();
+    for (int k0 = kbeg; k0 < kend; k0 += 2 * BK) {
+      step(s1, s0, k0);
+      if (k0 + BK < kend) step(s0, s1, k0 + BK);
     }
   }
   if (splits == 1) {
@@ -347,9 +354,10 @@ inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
   }
   const long nb = (long)g.batch1 * g.batch2, t64 = (long)cdiv(g.M, 64) * cdiv(g.N, 64) * nb;
   const int s = gemm_simt_splits(g, ctx->sm_count, t64, (long)cdiv(g.N, 64));
-  // 16-row tiles for a handful of rows; 32 x 32 tiles (a quarter of the work per block) when 64 x 64 would not give every SM one
+  // 16-row tiles for a handful of rows; 32 x 32 tiles (a quarter of the work per block) when 64 x 64 would not give every SM one or
+  // be half empty
   if (g.M <= 16) return gemm_simt_tile<16, 64, 32, 2, 4>(ctx, g, s);
-  if (t64 * s < ctx->sm_count) return gemm_simt_tile<32, 32, 32, 4, 2>(ctx, g, s);
+  if (g.M <= 32 || t64 * s < ctx->sm_count) return gemm_simt_tile<32, 32, 32, 4, 2>(ctx, g, s);
   return gemm_simt_tile<64, 64, 16, 4, 4>(ctx, g, s);
 }
 

@@ -193,7 +193,7 @@ namespace gn {
 // (beyond that the driver's own pageable copy, which overlaps its two stages, is the quicker way)
 constexpr size_t IO_ARGS = 64, STAGE_FLOATS = 1 << 18, STAGE_IN = 1 << 17;
 
-enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_SIDE, S_COUNT };
+enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_SIDE, S_PART3, S_COUNT };
 
 static int ensure(gn_model* m, int slot, size_t n, float** out) {
   if ((int)m->scratch.size() < S_COUNT) m->scratch.resize(S_COUNT);
@@ -434,26 +434,29 @@ static int norm_forward(Ctx* ctx, bool rms, const float* x, const float* gamma, 
   return check_launch("norm_forward");
 }
 // Register-row kernel: dx and the parameter sums from one reading of g and x; the blocks' partial sums are added by a second launch
-// unless there is only one.
+// unless there is only one: beside the main stream if `side_slot` names a scratch slot that is this call's own until the layer's end.
 static int norm_backward_vec(gn_model* m, bool rms, const float* g, const float* x, long ldx, const float* gamma, const float* sa, const float* sb, long lds, float* dx,
-                             float* gGamma, float* gBeta, long rows, int n, const RowPlaneOut& out) {
+                             float* gGamma, float* gBeta, long rows, int n, const RowPlaneOut& out, int side_slot = 0) {
   Ctx* ctx = &m->ctx->c; float* part;
   const int blocks = (int)std::max<long>(1, std::min<long>((rows + 7) / 8, (n <= 512 ? 2L : 1L) * ctx->sm_count));      // as many as are resident
   const bool direct = blocks == 1 && (rms || gBeta == gGamma + n) && (reinterpret_cast<uintptr_t>(gGamma) & 15) == 0;
-  if (direct) part = gGamma; else GN_TRY(ensure(m, S_PART2, (size_t)blocks * 2 * n, &part));
+  if (direct) part = gGamma; else GN_TRY(ensure(m, side_slot ? side_slot : S_PART2, (size_t)blocks * 2 * n, &part));
   if (rms) NormRun<true, 8>::bwd(ctx, blocks, g, x, gamma, sa, sb, dx, part, rows, n, ldx, lds, out);
   else NormRun<false, 8>::bwd(ctx, blocks, g, x, gamma, sa, sb, dx, part, rows, n, ldx, lds, out);
-  if (!direct) GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, blocks, n, gGamma, rms ? nullptr : gBeta);
+  if (!direct) {
+    auto final = [&]() -> int { GN_LAUNCH(ctx, layernorm_pgrad_final_kernel, cdiv(n, 32), 1024, 0, part, blocks, n, gGamma, rms ? nullptr : gBeta); return GN_OK; };
+    GN_TRY(side_slot ? side_run(ctx, final) : final());
+  }
   return check_launch("norm_backward");
 }
 // dx (may alias g), gGamma and gBeta (null for RMSNorm) are written.
 static int norm_backward(gn_model* m, bool rms, const float* g, const float* x, const float* gamma, const float* stat, float* dx, float* gGamma, float* gBeta, long rows, int n,
-                         const RowPlaneOut* po = nullptr, bool* emitted = nullptr) {
+                         const RowPlaneOut* po = nullptr, bool* emitted = nullptr, int side_slot = 0) {
   Ctx* ctx = &m->ctx->c; float* part;
   if (norm_vec_ok(n, {g, x, dx, gamma})) {
     const RowPlaneOut out = po ? *po : RowPlaneOut{};
     if (emitted) *emitted = out.p != nullptr;
-    return norm_backward_vec(m, rms, g, x, n, gamma, stat, rms ? stat : stat + rows, 1, dx, gGamma, gBeta, rows, n, out);
+    return norm_backward_vec(m, rms, g, x, n, gamma, stat, rms ? stat : stat + rows, 1, dx, gGamma, gBeta, rows, n, out, side_slot);
   }
   if (emitted) *emitted = false;
   const int chunks = (int)std::max<long>(1, std::min<long>(rows / 64, 128));
@@ -943,12 +946,13 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   const bool fused = use_fused_attention(d);
   GN_TRY(ensure(m, S_ND0, ND, &dR2)); GN_TRY(ensure(m, S_NFF, (size_t)N * F, &dM)); GN_TRY(ensure(m, S_ND1, ND, &comb));
   GN_TRY(ensure(m, S_ND2, ND, &dR1)); GN_TRY(ensure(m, S_ND3, ND, &dA));
+  const bool side = grads_on_side(ctx, 1, B, F, D, D);      // (the block forks its stream anyway)
   if (!fused) { GN_TRY(ensure(m, S_ATT0, (size_t)B * Hh * T * T, &P)); GN_TRY(ensure(m, S_ATT1, (size_t)B * Hh * T * T, &dP)); }
   // norm 2
   // its result goes to the contraction with W2 as operand planes, with the row norms that contraction's plane-writing epilogue needs
   RowPlaneOut pob{}; BfPlanes dR2p{}; bool dR2_planes = false; float* rnb = nullptr;
   if (norm_planes_wanted(ctx, N, D, F)) { GN_TRY(ensure(m, S_RN, (size_t)N, &rnb)); GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &pob, &dR2p, rnb)); }
-  GN_TRY(norm_backward(m, l.rms, gout, l.r2.p, bp.g2, st + 2 * N, dR2, (float*)gp.g2, (float*)gp.be2, (long)N, D, pob.p ? &pob : nullptr, &dR2_planes));
+  GN_TRY(norm_backward(m, l.rms, gout, l.r2.p, bp.g2, st + 2 * N, dR2, (float*)gp.g2, (float*)gp.be2, (long)N, D, pob.p ? &pob : nullptr, &dR2_planes, side ? S_PART2 : 0));
   // ff2 then ff1, token by token in the reference (transformer.go:1238-1250)
   GN_TRY(inner_dense_param_grads(m, dR2, B, T, D, l.mid.p, F, (float*)gp.w2, (float*)gp.b2, l.mid_is_planes ? l.mid_last.p : nullptr));
   {
@@ -1009,7 +1013,7 @@ static int block_backward(gn_model* m, LayerRT& l, int B, const float* xin, cons
   // norm 1
   RowPlaneOut poa{}; BfPlanes dR1p{}; bool dR1_planes = false;
   if (norm_planes_wanted(ctx, N, D, D)) GN_TRY(norm_planes_alloc(m, S_LNP0, S_LNI0, N, D, &poa, &dR1p, nullptr));      // the planes of dR2 are dead by now
-  GN_TRY(norm_backward(m, l.rms, comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, (long)N, D, poa.p ? &poa : nullptr, &dR1_planes));
+  GN_TRY(norm_backward(m, l.rms, comb, l.r1.p, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, (long)N, D, poa.p ? &poa : nullptr, &dR1_planes, side ? S_PART3 : 0));
   // output projection
   GN_TRY(inner_dense_param_grads(m, dR1, B, T, D, l.att.p, D, (float*)gp.wo, (float*)gp.bo));
   {

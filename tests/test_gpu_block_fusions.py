@@ -159,3 +159,18 @@ def test_weight_gradients_from_transposed_splits(device, oracle, R, N, K):
     dz = (u @ W2) * (1.0 - a * a)
     for got, ref in ((g[:K * N].reshape(N, K), dz.T @ X), (g[K * N:o], dz.sum(0)), (g[o:o + 3 * N].reshape(3, N), u.T @ a)):
         assert norm_err(got, ref / R) <= TOL
+
+
+@pytest.mark.parametrize("M,N", [(5, 130), (24, 5001), (32, 96), (70, 130)])
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 64, 65, 97, 500])
+def test_cuda_core_contraction_steps(device, M, N, K):
+    """One, two, three and more k-steps (two are in flight ahead of the one multiplied), ragged last ones, every tile shape.
+    Bound: an fp32 sum of K products is within (K + 2) 2^-24 of sum |a b| + |bias|."""
+    from goneuron_b200 import _lib
+    rng = np.random.default_rng(M * 1000 + K)
+    a, b, bias = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    c = np.empty((M, N), np.float32)
+    _lib.check(_lib.load().gn_op_gemm_nt(device.handle, 0, M, N, K, _f(a), _f(b), _f(bias), _f(c)))
+    ref = a.astype(np.float64) @ b.astype(np.float64).T + bias
+    size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64).T + np.abs(bias)
+    assert np.max(np.abs(c - ref) / size) <= (K + 2) * 2.0 ** -24
