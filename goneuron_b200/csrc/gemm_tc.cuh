@@ -53,6 +53,7 @@ constexpr unsigned TC_SPIN_LIMIT = 1u << 24;    // default number of polls of on
 constexpr unsigned TC_DRAIN_LIMIT = 1u << 20;   // polls spent waiting for own work in flight after a wait gave up
 constexpr int TC_QUEUE_POOL = 2048;   // tile-queue counters per context before the pool is cleared again
 constexpr int TC_FLAG_SCALE = 8192; // plane output: `mask` holds factors (a GELU layer's derivatives, all below 1.25), not a gate
+constexpr int TC_FLAG_WIDE = 16384; // ... 32-byte accesses to C and R
 constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by the host when every pointer and stride allows it)
 // One stage = 32 contraction indices of both operands.  The two fp16 planes of an operand are interleaved in blocks of 32:
 // element (r, k) of a plane row has its high part at pl_off(k) and its low part PL_LO halves further, so a block of a row is 128
@@ -256,6 +257,9 @@ __device__ __forceinline__ void tc_acc_chunk(uint32_t taddr, uint32_t acc_main, 
 __device__ __forceinline__ void st_global_32(void* p, const uint32_t (&r)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
+__device__ __forceinline__ void ld_global_32(const float* p, float* r) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]) : "l"(p) : "memory");
+}
 template <int RS>
 __device__ __forceinline__ void tc_stage_rows(float* stg, const float (&v)[32], int lane, int hh) {
   __syncwarp();                                               // the previous half has been read back
@@ -337,6 +341,53 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
   } else {
   float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
   const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
+  if (ep.flags & TC_FLAG_WIDE) {
+    // A thread keeps the row that TMEM gave it and reads and writes whole 32-byte sectors of it: no exchange through shared memory
+    // and none of its warp barriers (the launches of a 64 x 512 step: 289 -> 274 us on average).  For 32-byte aligned rows; the
+    // exchange below serves the rest.
+    const bool row_ok = row < ep.M;
+    const float* Mrow = ep.mask && row_ok ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
+#pragma unroll 1
+    for (int cc = 0; cc < nch; cc++) {
+      const int c = cg * nch + cc, col = n0 + c * 32;
+      if (col >= ep.N) break;
+      const long so = ep.n_seg ? (col / ep.n_seg) * (ep.c_seg - ep.n_seg) : 0;      // (32 columns lie in one segment; with segments R is C)
+      float* Cr = C + so + (long)row * ep.ldc + col; const float* Rr = R && row_ok ? R + so + (long)row * ep.ldr + col : nullptr;
+      float rv[32];
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) rv[j + q] = 0.f;
+        if (Rr && col + j < ep.N) ld_global_32(Rr + j, rv + j);
+      }
+      float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
+      const float* sv = colv + cc * 32; const float* bv = sv + Cfg::CW; float zm = 0.f;
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+        uint32_t o[8];
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+          const float4 s4 = *reinterpret_cast<const float4*>(sv + j + q), b4 = *reinterpret_cast<const float4*>(bv + j + q);
+          float4 x = make_float4(v[j + q] * s4.x + b4.x + rv[j + q], v[j + q + 1] * s4.y + b4.y + rv[j + q + 1], v[j + q + 2] * s4.z + b4.z + rv[j + q + 2], v[j + q + 3] * s4.w + b4.w + rv[j + q + 3]);
+          if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
+          if (Mrow && col + j < ep.N) {
+            const float4 m4 = *reinterpret_cast<const float4*>(Mrow + col + j + q);
+            if (!(m4.x > 0.f)) x.x = 0.f; if (!(m4.y > 0.f)) x.y = 0.f; if (!(m4.z > 0.f)) x.z = 0.f; if (!(m4.w > 0.f)) x.w = 0.f;
+          }
+          o[q] = __float_as_uint(x.x); o[q + 1] = __float_as_uint(x.y); o[q + 2] = __float_as_uint(x.z); o[q + 3] = __float_as_uint(x.w);
+          if (ep.zmax && row_ok) zm = fmaxf(zm, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+        }
+        if (row_ok && col + j < ep.N) st_global_32(Cr + j, o);
+      }
+      if (ep.zmax) {                                                         // (32 rows of one sequence, 32 columns of one head)
+        zm = warp_max(zm); if (!(zm <= 3.0e38f)) zm = 3.4e38f;
+        const int sg = col / ep.n_seg;
+        if (lane == 0 && rbase < ep.M) atomicMax(ep.zmax + sg * ep.zmax_seg + (long)(rbase / ep.zmax_T) * ep.zmax_H + (col - sg * ep.n_seg) / 64, __float_as_int(zm));
+      }
+    }
+    __syncwarp();
+    return;
+  }
   if (ep.flags & TC_FLAG_VEC) {
 #pragma unroll 1
     for (int cc = 0; cc < nch; cc++) {
@@ -907,6 +958,8 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
   }
   if (ep.zmax && !vec) return fail(GN_ERR_INVALID_ARG, "tc_launch: maxima need 16-byte aligned operands");
   if (vec) ep.flags |= TC_FLAG_VEC;
+  auto a32 = [](const void* p, long ld, long o1, long o2) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)((ld | o1 | o2) * 4)) & 31) == 0; };
+  if (vec && ep.N % 8 == 0 && a32(ep.C, ep.ldc, ep.c_b1, ep.c_b2) && ep.c_seg % 8 == 0 && (!ep.R || a32(ep.R, ep.ldr, ep.r_b1, ep.r_b2))) ep.flags |= TC_FLAG_WIDE;
   {
     double by = 4.0 * ((double)ep.M + ep.N) * ep.K + 4.0 * (double)ep.M * ep.N * (ep.R ? 2 : 1);
     if (ep.flags & (GEMM_SKIP_UPPER | GEMM_KBEG_AT_M0 | GEMM_KEND_AT_M0)) by *= 0.5;
