@@ -1229,7 +1229,10 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
   for (int li = (int)m->L.size() - 1; li >= 0; li--) {
     LayerRT& l = m->L[li]; const gn_layer_desc& d = l.d;
     const float* xin = l.fin;
-    if (row0 && d.kind != GN_LAYER_TRANSFORMER_BLOCK && d.kind != GN_LAYER_POSENC && d.kind != GN_LAYER_EMBEDDING) {
+    // (a layer below may read the same floats as sequences of another length and width: token 0 is then a different part of them)
+    const bool takes_row0 = (d.kind == GN_LAYER_TRANSFORMER_BLOCK || d.kind == GN_LAYER_POSENC) ? d.seq_len == row0_T && d.dim == row0_D
+                                                                                               : d.kind == GN_LAYER_EMBEDDING && d.seq_len == row0_T && d.out_size == row0_D;
+    if (row0 && !takes_row0) {
       const long n = (long)B * row0_T * row0_D;             // a layer that wants the gradient of every token: zeros except token 0
       GN_LAUNCH(ctx, cls_bwd_kernel, ew_grid(ctx, n), 256, 0, g, pp[flip], row0_T, row0_D, n); g = pp[flip]; flip ^= 1; row0 = false;
     }

@@ -42,8 +42,19 @@ CASES = [
 
 @pytest.mark.parametrize("T,dim,heads,ff,masks,pool,kw", CASES)
 def test_token_rows_parity(device, oracle, T, dim, heads, ff, masks, pool, kw):
+    _parity(device, oracle, _model(T, dim, heads, ff, masks, pool, **kw))
+
+
+@pytest.mark.parametrize("below", [[], [D.PositionalEncoding(6, 32)], [D.TransformerBlock(32, 2, 6, 48, True)], [D.TransformerBlock(32, 2, 6, 48, False)],
+                                   [D.PositionalEncoding(6, 32), D.TransformerBlock(48, 3, 4, 40, True)]])
+def test_sequences_of_another_shape_below(device, oracle, below):
+    """The layers below a causal block under CLSPooling read the same 192 floats as tokens of another width: token 0 of the one is not
+    token 0 of the other."""
+    _parity(device, oracle, [D.Embedding(60, 32, 6)] + below + [D.TransformerBlock(24, 2, 8, 40, True), D.CLSPooling(8, 24), D.Dense(24, 11, D.LOGSOFTMAX)])
+
+
+def _parity(device, oracle, layers):
     from goneuron_b200.sequential import Adam, Sequential
-    layers = _model(T, dim, heads, ff, masks, pool, **kw)
     rng = np.random.Generator(np.random.PCG64(99))
     params = configs.init_params(layers, rng)
     x, y = configs.make_inputs("transformer", layers, 3, rng)
