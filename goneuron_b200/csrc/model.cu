@@ -327,6 +327,7 @@ static int alloc_activations(gn_model* m, int cap, bool training) {
   size_t c = (size_t)cap;
   plan_token_rows(m, training);
   m->epoch++;
+  m->cap = 0; m->cap_training = false;        // until every buffer is there: after a failure the next call, of whatever size, starts over
   size_t most[NBLK] = {}; int n_shared = 0;
   for (auto& l : m->L) if (l.d.kind == GN_LAYER_TRANSFORMER_BLOCK) {
     for (int k = 0; k < NBLK; k++) block_buf(l, k).release();
