@@ -25,6 +25,7 @@
 #pragma once
 #include "common.cuh"
 #include "gemm_tc.cuh"
+#include "static_pieces.cuh"
 
 namespace gn {
 
@@ -61,23 +62,20 @@ extern "C" int gn_op_gemm_nt_static(gn_ctx* ctx, int M, int N, int K, const floa
   std::lock_guard<std::mutex> lk(c->run_mu);
   GN_CUDA(cudaSetDevice(c->device));
   float* base = nullptr; GN_TRY(static_scratch_ptr(c->device, &base));
-  // Plane rows are padded to whole blocks of 32, so a product near the limit may not fit at once: then the larger of its two
-  // sides is walked in pieces (every output element is formed in the same way).
-  const long ldp = tc_ldp(K); long mc = M, nc = N;
-  auto floats = [&](long m, long n) { return (m + n) * ldp + ((m + 3) & ~3L) + n; };
-  while (floats(mc, nc) > GN_STATIC_SCRATCH_FLOATS) { long& x = mc >= nc ? mc : nc; x = ((x + 1) / 2 + 3) & ~3L; }
-  for (long n0 = 0; n0 < N; n0 += nc) for (long m0 = 0; m0 < M; m0 += mc) {
-    const int m = (int)std::min(mc, M - m0), n = (int)std::min(nc, N - n0);
+  const StaticPieces pc = static_pieces(M, N, K, GN_STATIC_SCRATCH_FLOATS);
+  for (long n0 = 0; n0 < N; n0 += pc.n) for (long m0 = 0; m0 < M; m0 += pc.m) for (long k0 = 0; k0 < K; k0 += pc.k) {
+    const int m = (int)std::min(pc.m, M - m0), n = (int)std::min(pc.n, N - n0), k = (int)std::min(pc.k, K - k0); const long ldp = tc_ldp(k);
     float* sa = base + ((long)m + n) * ldp; float* sb = sa + ((m + 3) & ~3);        // row scales: A's, then B's on a 16-byte boundary
-    BfPlanes PA{reinterpret_cast<__half*>(base), sa, m, K, (int)ldp, 1}, PB{reinterpret_cast<__half*>(base + (long)m * ldp), sb, n, K, (int)ldp, 1};
-    GN_TRY(tc_split(c, TcSrc{A_dev + m0 * K, (long)K, 1, 0, 0, 1}, PA, nullptr));
-    GN_TRY(tc_split(c, TcSrc{B_dev + n0 * K, (long)K, 1, 0, 0, 1}, PB, nullptr));
-    TcParams ep{C_dev + m0 * N + n0, (long)N, 0, 0, bias_dev ? bias_dev + n0 : nullptr, nullptr, 0, 0, 0, GN_ACT_LINEAR, m, n, K, 1, 0, c->d_status, nullptr, 0, 1};
+    BfPlanes PA{reinterpret_cast<__half*>(base), sa, m, k, (int)ldp, 1}, PB{reinterpret_cast<__half*>(base + (long)m * ldp), sb, n, k, (int)ldp, 1};
+    GN_TRY(tc_split(c, TcSrc{A_dev + m0 * K + k0, (long)K, 1, 0, 0, 1}, PA, nullptr));
+    GN_TRY(tc_split(c, TcSrc{B_dev + n0 * K + k0, (long)K, 1, 0, 0, 1}, PB, nullptr));
+    float* C = C_dev + m0 * N + n0; const bool first = k0 == 0;
+    TcParams ep{C, (long)N, 0, 0, first && bias_dev ? bias_dev + n0 : nullptr, first ? nullptr : C, first ? 0L : (long)N, 0, 0, GN_ACT_LINEAR, m, n, k, 1, 0, c->d_status, nullptr, 0, 1};
     // the regular entry point's slices of a long contraction: side by side where the array has room for their partial results, else one by one
     int bn = tc_pick_bn(c, m, n, 1, 0); const int splits = tc_split_count(c, ep, 1, &bn);
     float* part = sb + ((n + 3) & ~3);
     if (splits > 1 && (part - base) + (long)splits * m * n <= GN_STATIC_SCRATCH_FLOATS) GN_TRY(tc_run_slices(c, PA, PB, ep, splits, bn, part));
-    else GN_TRY(tc_run_rows(c, PA, PB, ep, bn, splits > 1 ? tc_slice_length(K, splits) : 0));
+    else GN_TRY(tc_run_rows(c, PA, PB, ep, bn, splits > 1 ? tc_slice_length(k, splits) : 0));
   }
   GN_CUDA(cudaStreamSynchronize(c->stream));
   return check_status_word(c);

@@ -81,3 +81,27 @@ def test_static_scratch_takes_every_size_of_the_documented_limit():
                 dev.free(p)
     finally:
         dev.close()
+
+
+@pytest.mark.parametrize("M,N,K", [(4, 4, 524_280), (1, 1, 2_097_144), (1, 2, 1_398_096), (3, 4, 599_176)])
+def test_static_scratch_takes_long_contractions(M, N, K):
+    """Few rows and a contraction at the documented limit: halved sides, and single rows walked along the contraction.  Bound: 2^-19 of
+    sum |a b| (22-bit operands, an accumulator that truncates once per 16 indices, partial sums in fp32)."""
+    from goneuron_b200 import _lib
+    from goneuron_b200.sequential import Device
+    L = _lib.load()
+    dev = Device(0)
+    try:
+        rng = np.random.default_rng(K)
+        A, B = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+        bias = rng.standard_normal(N).astype(np.float32)
+        dA, dB, db, dC = dev.alloc(A), dev.alloc(B), dev.alloc(bias), dev.alloc(np.zeros((M, N), np.float32))
+        _lib.check(L.gn_op_gemm_nt_static(dev.handle, M, N, K, dA, dB, db, dC))
+        out = np.empty((M, N), np.float32)
+        _lib.check(L.gn_device_download(dev.handle, _f(out), dC, out.size))
+        size = np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T
+        assert np.max(np.abs(out - (A.astype(np.float64) @ B.astype(np.float64).T + bias)) / size) <= 2.0 ** -19
+        for p in (dA, dB, db, dC):
+            dev.free(p)
+    finally:
+        dev.close()
