@@ -691,7 +691,7 @@ inline int attn_tc_prepare(Ctx* ctx, int n, const float* const* X, const bool* w
   float *words, *norms;
   if (store) { words = store + (size_t)2 * n * ne; norms = words + (size_t)Z * 16; }
   else { GN_TRY(attn_tc_buf(ctx, 8, (size_t)Z * 16, &words)); GN_TRY(attn_tc_buf(ctx, 9, (size_t)Z * T * 2, &norms)); }   // per tensor: amax, inv, nmax; one extra row for the caller
-  if (!have_max) GN_CUDA(cudaMemsetAsync(words, 0, (size_t)Z * 16 * sizeof(float), ctx->stream));
+  if (!have_max) GN_CUDA(stream_zero(ctx, words, (size_t)Z * 16 * sizeof(float)));
   AttnPrepJobs jobs{}; int nn = 0;
   for (int i = 0; i < n; i++) {
     AttnPrepJob& j = jobs.j[i]; j.X = X[i];
@@ -737,7 +737,7 @@ inline int attn_tc_store(Ctx* ctx, AttnSaved* save, int Z, int T, float** store)
 inline int attn_tc_max_words(Ctx* ctx, AttnSaved* save, int Z, int T, int** words) {
   float *store, *w; GN_TRY(attn_tc_store(ctx, save, Z, T, &store));
   if (store) w = store + (size_t)6 * Z * T * ATC_HD; else GN_TRY(attn_tc_buf(ctx, 8, (size_t)Z * 16, &w));
-  GN_CUDA(cudaMemsetAsync(w, 0, (size_t)Z * 16 * sizeof(float), ctx->stream));
+  GN_CUDA(stream_zero(ctx, w, (size_t)Z * 16 * sizeof(float)));
   *words = reinterpret_cast<int*>(w); return GN_OK;
 }
 inline int attn_tc_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal,

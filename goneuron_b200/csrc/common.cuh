@@ -26,6 +26,31 @@ inline int fail(int code, const char* fmt, ...) {
 
 struct NcclApi;   // resolved at run time from libnccl.so.2 (nccl_dl.cuh)
 
+// A run of launches and copies put together as a CUDA graph, node by node, while Ctx::rec points here: the helpers below then add a
+// node behind what their stream holds so far instead of issuing the work.  (Capturing the stream gives the same graph but forbids
+// other threads to synchronise the device, or to use the stream, for as long as it lasts -- theirs then fail, and the capture with
+// them -- and a copy that another call queues meanwhile becomes part of it.)
+struct GraphRec {
+  cudaGraph_t graph = nullptr;
+  struct Tail { cudaStream_t stream; std::vector<cudaGraphNode_t> nodes; bool kernel = false; };      // kernel: `nodes` is one kernel node
+  std::vector<Tail> tails;
+  GraphRec() {}
+  GraphRec(const GraphRec&) = delete; GraphRec& operator=(const GraphRec&) = delete;
+  ~GraphRec() { if (graph) cudaGraphDestroy(graph); }
+  Tail& tail(cudaStream_t s) { for (auto& t : tails) if (t.stream == s) return t; tails.push_back(Tail{s, {}}); return tails.back(); }
+  // what `from` holds so far comes before everything that `to` gets from now on
+  void join(cudaStream_t to, cudaStream_t from) {
+    const std::vector<cudaGraphNode_t> add = tail(from).nodes; Tail& t = tail(to);
+    for (auto n : add) { bool have = false; for (auto q : t.nodes) have |= q == n; if (!have) { t.nodes.push_back(n); t.kernel = t.kernel && t.nodes.size() == 1; } }
+  }
+  template <class F> cudaError_t add(cudaStream_t s, bool kernel, F&& make) {      // make(node, dependencies, their number)
+    Tail& t = tail(s); cudaGraphNode_t node;
+    const cudaError_t e = make(&node, t.nodes.data(), t.nodes.size());
+    if (e == cudaSuccess) { t.nodes.assign(1, node); t.kernel = kernel; }
+    return e;
+  }
+};
+
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -48,6 +73,7 @@ struct Ctx {
   // inputs, one for small outputs; d_ret / d_out: the device's addresses
   float *h_block = nullptr, *h_ret = nullptr, *h_stage = nullptr, *h_out = nullptr, *d_ret = nullptr, *d_out = nullptr;
   uint64_t epoch = 0;              // counts replacements of the context's scratch buffers
+  GraphRec* rec = nullptr;         // set while a step is put together as a graph instead of being issued
   bool tc_ok = false;              // tcgen05 engine usable (driver entry point for tensor maps found)
   void* encode_tiled = nullptr;    // cuTensorMapEncodeTiled
   unsigned spin_limit = 1u << 24;  // polls per bounded device-side wait (gn_ctx_set_spin_limit)
@@ -75,7 +101,8 @@ inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 // engine's scratch or any buffer that the main stream writes before side_join(), which the backward pass calls after every layer.
 template <class F> inline int side_run(Ctx* ctx, F&& f) {
   if (!ctx->side_stream || ctx->profile) return f();         // (profiling times the contractions one by one)
-  if (cudaEventRecord(ctx->fork_ev, ctx->stream) != cudaSuccess || cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0) != cudaSuccess)
+  if (ctx->rec) ctx->rec->join(ctx->side_stream, ctx->stream);
+  else if (cudaEventRecord(ctx->fork_ev, ctx->stream) != cudaSuccess || cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0) != cudaSuccess)
     return fail(GN_ERR_CUDA, "side stream: %s", cudaGetErrorString(cudaGetLastError()));
   cudaStream_t main = ctx->stream; ctx->stream = ctx->side_stream; ctx->side_pending = true;
   const int rc = f();
@@ -84,19 +111,42 @@ template <class F> inline int side_run(Ctx* ctx, F&& f) {
 inline int side_join(Ctx* ctx) {
   if (!ctx->side_pending) return GN_OK;
   ctx->side_pending = false;
+  if (ctx->rec) { ctx->rec->join(ctx->stream, ctx->side_stream); return GN_OK; }
   if (cudaEventRecord(ctx->join_ev, ctx->side_stream) != cudaSuccess || cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0) != cudaSuccess)
     return fail(GN_ERR_CUDA, "side stream: %s", cudaGetErrorString(cudaGetLastError()));
   return GN_OK;
 }
 
-// Every kernel launch of the library goes through these macros, so that the launch count is exact.
+// Every kernel launch of the library goes through these macros, so that the launch count is exact and a step can be recorded.
 // launch_kernel(): `cluster` > 0: that many neighbouring blocks of the grid's x dimension form a thread-block cluster; `early`: the
 // blocks may be placed while the preceding kernel still runs (programmatic stream serialisation), which wants a kernel that calls
 // pdl_wait() in every block before it touches anything its predecessors write, and pdl_launch() to let its own successor in.
 // (Launching every kernel of a step that way, waiting at its first instruction, was measured: within a replayed graph it is
 // slower than the ordinary edge, 78 -> 85 us for a step of 15 launches.  It pays where a kernel has something to fetch first.)
 template <class... P, class... A>
-inline cudaError_t launch_kernel(cudaStream_t stream, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster, bool early, A&&... args) {
+inline cudaError_t launch_kernel(Ctx* ctx, cudaStream_t stream, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster, bool early, A&&... args) {
+  ctx->launches++;
+  if (ctx->rec) {
+    GraphRec& rec = *ctx->rec;
+    return rec.add(stream, true, [&](cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t n) -> cudaError_t {
+      const bool edge = early && rec.tail(stream).kernel;
+      auto make = [&](P... values) {
+        void* pointers[] = {(void*)&values..., nullptr};
+        cudaKernelNodeParams p{}; p.func = (void*)kernel; p.gridDim = grid; p.blockDim = block; p.sharedMemBytes = (unsigned)smem; p.kernelParams = pointers;
+        return cudaGraphAddKernelNode(node, rec.graph, edge ? nullptr : deps, edge ? 0 : n, &p);
+      };
+      cudaError_t e = make(static_cast<P>(args)...);
+      if (e == cudaSuccess && cluster > 0) {
+        cudaLaunchAttributeValue v{}; v.clusterDim.x = cluster; v.clusterDim.y = v.clusterDim.z = 1;
+        e = cudaGraphKernelNodeSetAttribute(*node, cudaLaunchAttributeClusterDimension, &v);
+      }
+      if (e == cudaSuccess && edge) {
+        cudaGraphEdgeData d{}; d.from_port = cudaGraphKernelNodePortProgrammatic; d.type = cudaGraphDependencyTypeProgrammatic;
+        e = cudaGraphAddDependencies_v2(rec.graph, deps, node, &d, 1);
+      }
+      return e;
+    });
+  }
   cudaLaunchConfig_t cfg{}; cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute at[2]; int n = 0;
   if (early) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n++].val.programmaticStreamSerializationAllowed = 1; }
@@ -104,12 +154,26 @@ inline cudaError_t launch_kernel(cudaStream_t stream, void (*kernel)(P...), dim3
   cfg.attrs = at; cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
-#define GN_LAUNCH(ctx, kernel, grid, block, smem, ...)                         \
-  do { kernel<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__); (ctx)->launches++; } while (0)
-#define GN_CLUSTER_LAUNCH(ctx, kernel, grid, block, cx, ...)                   \
-  do { GN_CUDA(gn::launch_kernel((ctx)->stream, kernel, dim3(grid), dim3(block), (size_t)0, cx, false, __VA_ARGS__)); (ctx)->launches++; } while (0)
+// (an error of the first two is seen by the check_launch() behind them)
+#define GN_LAUNCH(ctx, kernel, grid, block, smem, ...) GN_LAUNCH_ON(ctx, (ctx)->stream, kernel, grid, block, smem, __VA_ARGS__)
+#define GN_LAUNCH_ON(ctx, stream, kernel, grid, block, smem, ...)              \
+  do { (void)gn::launch_kernel(ctx, stream, kernel, dim3(grid), dim3(block), (size_t)(smem), 0, false, __VA_ARGS__); } while (0)
+#define GN_CLUSTER_LAUNCH(ctx, kernel, grid, block, smem, cx, ...)             \
+  do { GN_CUDA(gn::launch_kernel(ctx, (ctx)->stream, kernel, dim3(grid), dim3(block), (size_t)(smem), cx, false, __VA_ARGS__)); } while (0)
 #define GN_EARLY_LAUNCH(ctx, kernel, grid, block, smem, ...)                   \
-  do { GN_CUDA(gn::launch_kernel((ctx)->stream, kernel, dim3(grid), dim3(block), (size_t)(smem), 0, true, __VA_ARGS__)); (ctx)->launches++; } while (0)
+  do { GN_CUDA(gn::launch_kernel(ctx, (ctx)->stream, kernel, dim3(grid), dim3(block), (size_t)(smem), 0, true, __VA_ARGS__)); } while (0)
+// `bytes` zeros at p / a copy, in stream order
+inline cudaError_t stream_zero(Ctx* ctx, cudaStream_t stream, void* p, size_t bytes) {
+  if (!ctx->rec) return cudaMemsetAsync(p, 0, bytes, stream);
+  const unsigned es = ((uintptr_t)p | bytes) % 4 == 0 ? 4 : 1;
+  cudaMemsetParams mp{}; mp.dst = p; mp.elementSize = es; mp.width = bytes / es; mp.height = 1;
+  return ctx->rec->add(stream, false, [&](cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t n) { return cudaGraphAddMemsetNode(node, ctx->rec->graph, deps, n, &mp); });
+}
+inline cudaError_t stream_zero(Ctx* ctx, void* p, size_t bytes) { return stream_zero(ctx, ctx->stream, p, bytes); }
+inline cudaError_t stream_copy(Ctx* ctx, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+  if (!ctx->rec) return cudaMemcpyAsync(dst, src, bytes, kind, ctx->stream);
+  return ctx->rec->add(ctx->stream, false, [&](cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t n) { return cudaGraphAddMemcpyNode1D(node, ctx->rec->graph, deps, n, dst, src, bytes, kind); });
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -322,10 +322,10 @@ inline int gemm_simt_tile(Ctx* ctx, const GemmDesc& g, int splits) {
   const bool ak = g.sa_k == 1, bn = g.sb_n == 1;
   const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
   const dim3 grid(cdiv(g.N, BN) * splits, cdiv(g.M, BM), g.batch1 * g.batch2); constexpr int THREADS = SgCfg<BM, BN, BK, TM, TN>::THREADS;
-  if (ak && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, splits, g, splits, va, vb);
-  else if (ak && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, splits, g, splits, va, vb);
-  else if (g.sa_m == 1 && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, splits, g, splits, va, vb);
-  else if (g.sa_m == 1 && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, splits, g, splits, va, vb);
+  if (ak && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, 0, splits, g, splits, va, vb);
+  else if (ak && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, 0, splits, g, splits, va, vb);
+  else if (g.sa_m == 1 && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, 0, splits, g, splits, va, vb);
+  else if (g.sa_m == 1 && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, 0, splits, g, splits, va, vb);
   else return fail(GN_ERR_UNSUPPORTED, "gemm_simt: neither stride of an operand is 1");
   return check_launch("gemm_simt");
 }
@@ -350,7 +350,7 @@ inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
   }
   if (gemm_skinny_ok(g)) {
     int s = 1; while (s < SG_MAX_SPLITS && g.K >= 512 * s) s *= 2;
-    GN_CLUSTER_LAUNCH(ctx, gemm_skinny_kernel, dim3(g.M * s), 256, s, g, s); return check_launch("gemm_skinny");
+    GN_CLUSTER_LAUNCH(ctx, gemm_skinny_kernel, dim3(g.M * s), 256, 0, s, g, s); return check_launch("gemm_skinny");
   }
   const long nb = (long)g.batch1 * g.batch2, t64 = (long)cdiv(g.M, 64) * cdiv(g.N, 64) * nb;
   const int s = gemm_simt_splits(g, ctx->sm_count, t64, (long)cdiv(g.N, 64));

@@ -879,12 +879,12 @@ inline int tc_split(Ctx* ctx, const TcSrc& src, const BfPlanes& p, int* mx, floa
       int cs = 1; while (cs < SPLIT_T_CLUSTER && p.ldp > 64 * cs) cs *= 2;
       const int per = cdiv(cdiv(p.ldp, cs), 32) * 32, smem = per * 33 * (int)sizeof(float);
       if (smem > 40 * 1024) GN_CUDA(cudaFuncSetAttribute(split2_cols_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      GN_CUDA(launch_kernel(ctx->stream, split2_cols_cluster_kernel, dim3(cdiv(p.rows, 32) * cs, p.nbatch), dim3(256), (size_t)smem, cs, false, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, per, cs));
-      ctx->launches++; ctx->split_bytes += 8.0 * (double)p.nbatch * p.rows * p.K;
+      GN_CLUSTER_LAUNCH(ctx, split2_cols_cluster_kernel, dim3(cdiv(p.rows, 32) * cs, p.nbatch), 256, smem, cs, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, per, cs);
+      ctx->split_bytes += 8.0 * (double)p.nbatch * p.rows * p.K;
       return check_launch("tc_split");
     }
     if (!mx) return fail(GN_ERR_INVALID_ARG, "tc_split: the transposing split needs a row-maximum buffer");
-    GN_CUDA(cudaMemsetAsync(mx, 0, (size_t)p.nbatch * p.rows * sizeof(int), ctx->stream));
+    GN_CUDA(stream_zero(ctx, mx, (size_t)p.nbatch * p.rows * sizeof(int)));
     GN_LAUNCH(ctx, colmax_kernel, dim3(cdiv(p.rows, 64), cdiv(p.K, 256), p.nbatch), 256, 0, src, p.rows, p.K, mx);
     GN_LAUNCH(ctx, split2_cols_kernel, dim3(cdiv(p.ldp, 64), cdiv(p.rows, 64), p.nbatch), 256, 0, src, p.rows, p.K, p.base, (const int*)mx, p.inv_scale, p.ldp);
   } else return fail(GN_ERR_UNSUPPORTED, "tc_split: neither stride of the operand is 1");
@@ -1183,15 +1183,13 @@ inline int wplanes_build(Ctx* ctx, WeightPlaneTable& t, const std::vector<Weight
 // Entries [j0, j1) only, on `stream`: used right behind a layer's parameter update when the update runs layer by layer.
 inline int wplanes_max(Ctx* ctx, WeightPlaneTable& t, int j0, int j1, cudaStream_t stream) {
   const int tile_off = t.e[j0].tile0, ntiles = t.e[j1 - 1].tile0 + t.e[j1 - 1].tiles - tile_off;
-  GN_CUDA(cudaMemsetAsync(reinterpret_cast<int*>(t.mx.p) + j0, 0, (size_t)(j1 - j0) * sizeof(int), stream));
-  wplanes_max_kernel<<<ntiles, 256, 0, stream>>>(reinterpret_cast<const WPlaneJob*>(t.jobs.p), (int)t.e.size(), reinterpret_cast<int*>(t.mx.p), tile_off);
-  ctx->launches++;
+  GN_CUDA(stream_zero(ctx, stream, reinterpret_cast<int*>(t.mx.p) + j0, (size_t)(j1 - j0) * sizeof(int)));
+  GN_LAUNCH_ON(ctx, stream, wplanes_max_kernel, ntiles, 256, 0, reinterpret_cast<const WPlaneJob*>(t.jobs.p), (int)t.e.size(), reinterpret_cast<int*>(t.mx.p), tile_off);
   return check_launch("wplanes_max");
 }
 inline int wplanes_split(Ctx* ctx, WeightPlaneTable& t, int j0, int j1, cudaStream_t stream) {
   const int tile_off = t.e[j0].tile0, ntiles = t.e[j1 - 1].tile0 + t.e[j1 - 1].tiles - tile_off;
-  wplanes_split_kernel<<<ntiles, 256, 0, stream>>>(reinterpret_cast<const WPlaneJob*>(t.jobs.p), (int)t.e.size(), reinterpret_cast<const int*>(t.mx.p), tile_off);
-  ctx->launches++;
+  GN_LAUNCH_ON(ctx, stream, wplanes_split_kernel, ntiles, 256, 0, reinterpret_cast<const WPlaneJob*>(t.jobs.p), (int)t.e.size(), reinterpret_cast<const int*>(t.mx.p), tile_off);
   double elems = 0; for (int j = j0; j < j1; j++) elems += (double)t.e[j].out * t.e[j].in;
   ctx->split_bytes += 12.0 * elems;
   return check_launch("wplanes_split");

@@ -1096,7 +1096,7 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
   GN_TRY(gemm_nn(ctx, B, D, D, dR1, D, bp.wo, dA, D));
   if (d.causal) {
     // the one probability of token 0 is 1: dV = dA at token 0, dQ = dK = 0
-    GN_TRY(side_run(ctx, [&]() -> int { GN_CUDA(cudaMemsetAsync((void*)gp.wq, 0, (size_t)(gp.wv - gp.wq) * sizeof(float), ctx->stream)); return GN_OK; }));
+    GN_TRY(side_run(ctx, [&]() -> int { GN_CUDA(stream_zero(ctx, (void*)gp.wq, (size_t)(gp.wv - gp.wq) * sizeof(float))); return GN_OK; }));
     GN_TRY(side_weight_bias_grads(m, 1, B, D, D, dA, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
     GN_TRY(gemm_nn(ctx, B, D, D, dA, D, bp.wv, dx, D, dR1, D));
     *dx_row0 = true; return check_launch("block_backward_row0");
@@ -1144,11 +1144,11 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
       GN_TRY(ensure(m, S_DM, (size_t)rows * R4g, &Dm)); GN_TRY(ensure(m, S_ZM, (size_t)rows * zs, &Zm));
       GN_TRY(ensure(m, S_TV, 2 * (n_om + n_p + (size_t)ng * 2), &dbl)); GN_TRY(ensure(m, S_SCAN, (size_t)nchunks * 2 * R4g * ZWg, &gmat));
       // rows of zeros: the group before every chunk's first, and what its last group lacks
-      if (nchunks > 8) { GN_CUDA(cudaMemsetAsync(Dm, 0, (size_t)rows * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm, 0, (size_t)rows * zs * 4, ctx->stream)); }
+      if (nchunks > 8) { GN_CUDA(stream_zero(ctx, Dm, (size_t)rows * R4g * 4)); GN_CUDA(stream_zero(ctx, Zm, (size_t)rows * zs * 4)); }
       else for (int c = 0; c < nchunks; c++) {
         const long n = std::min(Kc, n_updates - c * Kc), r0 = c * stride, r1 = r0 + CG_PAD + n, left = stride - CG_PAD - n;
-        GN_CUDA(cudaMemsetAsync(Dm + r0 * R4g, 0, (size_t)CG_PAD * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm + r0 * zs, 0, (size_t)CG_PAD * zs * 4, ctx->stream));
-        if (left > 0) { GN_CUDA(cudaMemsetAsync(Dm + r1 * R4g, 0, (size_t)left * R4g * 4, ctx->stream)); GN_CUDA(cudaMemsetAsync(Zm + r1 * zs, 0, (size_t)left * zs * 4, ctx->stream)); }
+        GN_CUDA(stream_zero(ctx, Dm + r0 * R4g, (size_t)CG_PAD * R4g * 4)); GN_CUDA(stream_zero(ctx, Zm + r0 * zs, (size_t)CG_PAD * zs * 4));
+        if (left > 0) { GN_CUDA(stream_zero(ctx, Dm + r1 * R4g, (size_t)left * R4g * 4)); GN_CUDA(stream_zero(ctx, Zm + r1 * zs, (size_t)left * zs * 4)); }
       }
       if (world > 1) {
         float* all; GN_TRY(ensure(m, S_W, (size_t)n_updates * (R4g + zs), &all));
@@ -1278,7 +1278,7 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
           else GN_LAUNCH(ctx, maxpool_bwd_gather_kernel, dim3(B * c.C, cdiv((long)c.H * c.W, 256)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
           g = dx; flip ^= 1; break;
         }
-        GN_CUDA(cudaMemsetAsync(dx, 0, (size_t)B * l.in_size * sizeof(float), ctx->stream));
+        GN_CUDA(stream_zero(ctx, dx, (size_t)B * l.in_size * sizeof(float)));
         long n = (long)B * l.out_size;
         GN_LAUNCH(ctx, maxpool_bwd_kernel, ew_grid(ctx, n), 256, 0, g, (const int*)l.idx.p, dx, c);
         g = dx; flip ^= 1; break; }
@@ -1319,7 +1319,7 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         const int chunk = (global_batch + m->W - 1) / m->W, T = row0 ? 1 : d.seq_len, Tid = d.seq_len, dim = d.out_size;     // T: tokens of a sample with a gradient
         const int nq = (global_batch + chunk - 1) / chunk;                       // qualifying samples of the global batch
         auto q_sample = [&](int q) { return std::min(global_batch - 1, q * chunk + chunk - 1); };
-        GN_CUDA(cudaMemsetAsync(gr, 0, (size_t)l.p_cnt * sizeof(float), ctx->stream));     // most rows of the table have no gradient
+        GN_CUDA(stream_zero(ctx, gr, (size_t)l.p_cnt * sizeof(float)));     // most rows of the table have no gradient
         const size_t smem = (size_t)T * sizeof(int);
         if (smem > 48 * 1024) GN_CUDA(cudaFuncSetAttribute(embedding_bwd_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const bool sparse = ctx->world > 1 && (double)nq * T * (dim + 1) < 0.5 * (double)l.p_cnt;
@@ -1328,7 +1328,7 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
           // every rank then builds the complete table gradient itself
           float* buf; GN_TRY(ensure(m, S_EMB, (size_t)nq * T * (dim + 1) + (size_t)nq * T, &buf));
           float* rows = buf; float* idsf = buf + (size_t)nq * T * dim; int* idsi = reinterpret_cast<int*>(idsf + (size_t)nq * T);
-          GN_CUDA(cudaMemsetAsync(buf, 0, (size_t)nq * T * (dim + 1) * sizeof(float), ctx->stream));
+          GN_CUDA(stream_zero(ctx, buf, (size_t)nq * T * (dim + 1) * sizeof(float)));
           for (int q = 0; q < nq; q++) {
             const int sl = q_sample(q) - first_sample; if (sl < 0 || sl >= B) continue;
             GN_LAUNCH(ctx, embedding_pack_kernel, T, 128, 0, g + (size_t)sl * T * dim, (const int*)l.idx.p + (size_t)sl * Tid, rows + (size_t)q * T * dim, idsf + (size_t)q * T, T, dim);
@@ -1352,7 +1352,7 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         }
         break; }
       case GN_LAYER_POSENC:
-        if (row0) GN_CUDA(cudaMemsetAsync(gr, 0, (size_t)l.p_cnt * sizeof(float), ctx->stream));
+        if (row0) GN_CUDA(stream_zero(ctx, gr, (size_t)l.p_cnt * sizeof(float)));
         { const int n = row0 ? d.dim : l.out_size; GN_TRY(colsum(m, g, n, B, n, gr, false)); } break;     // gP = sum over samples; dx = g
       case GN_LAYER_TRANSFORMER_BLOCK:
         if (row0) GN_TRY(block_backward_row0(m, l, B, xin, g, dx, &row0)); else GN_TRY(block_backward(m, l, B, xin, g, dx));
@@ -1402,10 +1402,9 @@ static int adam_launch(Ctx* ctx, float* p, const float* g, float* m1, float* v, 
                        cudaStream_t stream, const float* loss_sum, float* ret, const WeightPlaneTable* t) {
   const unsigned grid = (unsigned)std::max<long>(1, std::min<long>(cdiv((n + 3) / 4, 256), 8L * ctx->sm_count)); stream = stream ? stream : ctx->stream;      // one resident round
   if (t) {
-    GN_CUDA(cudaMemsetAsync(t->mx.p, 0, t->e.size() * sizeof(int), stream));
-    adam_kernel<true><<<grid, 256, 0, stream>>>(p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret, reinterpret_cast<const PlaneRange*>(t->ranges.p), (int)t->e.size(), reinterpret_cast<int*>(t->mx.p));
-  } else adam_kernel<false><<<grid, 256, 0, stream>>>(p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret, nullptr, 0, nullptr);
-  ctx->launches++;
+    GN_CUDA(stream_zero(ctx, stream, t->mx.p, t->e.size() * sizeof(int)));
+    GN_LAUNCH_ON(ctx, stream, adam_kernel<true>, grid, 256, 0, p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret, reinterpret_cast<const PlaneRange*>(t->ranges.p), (int)t->e.size(), reinterpret_cast<int*>(t->mx.p));
+  } else GN_LAUNCH_ON(ctx, stream, adam_kernel<false>, grid, 256, 0, p, g, m1, v, (long)n, a, dargs, status, loss_sum, ret, nullptr, 0, nullptr);
   return check_launch("adam");
 }
 // Meaning of a non-zero status word.
@@ -1437,7 +1436,7 @@ static int issue_backward(gn_model* m, const float* yp, const float* y_dev, int 
     int cs = 1; while (cs < HEAD_MAX_CS && n > cs * HEAD_THREADS * 4) cs *= 2;
     const int per = cdiv(n, cs * HEAD_THREADS); const dim3 grid(B * cs);
     auto* K = per <= 1 ? head_loss_kernel<1> : per <= 4 ? head_loss_kernel<4> : head_loss_kernel<HEAD_MAX_E>;
-    GN_CLUSTER_LAUNCH(ctx, K, grid, HEAD_THREADS, cs, (const float*)h.z.p, y_dev, m->lossg.p, m->loss_s.p, n, B, cs, lg, m->loss_kind, ticket, m->loss_sum.p);
+    GN_CLUSTER_LAUNCH(ctx, K, grid, HEAD_THREADS, 0, cs, (const float*)h.z.p, y_dev, m->lossg.p, m->loss_s.p, n, B, cs, lg, m->loss_kind, ticket, m->loss_sum.p);
   } else GN_LAUNCH(ctx, loss_rows_kernel, B, m->out_size <= 64 ? 32 : 256, 0, yp, y_dev, m->lossg.p, m->loss_s.p, m->out_size, m->loss_kind, ticket, m->loss_sum.p);
   GN_TRY(backward(m, B, m->lossg.p, global_batch, first_sample));
   if (ctx->world > 1) {
@@ -1461,9 +1460,9 @@ static int issue_backward(gn_model* m, const float* yp, const float* y_dev, int 
                      m->wplanes.used && !m->wplanes.e.empty() ? &m->wplanes : nullptr);
 }
 
-// Captured launches of a step (or of an inference pass).  A call whose sizes and buffers have been seen before is replayed as one or
+// Recorded launches of a step (or of an inference pass).  A call whose sizes and buffers have been seen before is replayed as one or
 // two CUDA graphs: a step is 10 to 300 launches of a few microseconds each, which the host would otherwise issue one by one.  The
-// first call with a set of sizes runs launch by launch (it may allocate), the second is captured.  A graph refers to
+// first call with a set of sizes runs launch by launch (it may allocate), the second is recorded (GraphRec).  A graph refers to
 // buffers by address, so it is dropped when the model or the context has replaced one (epoch).  What differs from call to
 // call lies in memory: inputs, the Adam coefficients (head of the model's `io` buffer), the results.
 struct StepGraph {
@@ -1472,9 +1471,11 @@ struct StepGraph {
     return B == o.B && global_batch == o.global_batch && first_sample == o.first_sample && x == o.x && y == o.y && staged == o.staged && training == o.training && spin == o.spin &&
            epoch_m == o.epoch_m && epoch_c == o.epoch_c;
   }
-  cudaGraphExec_t exec[2] = {nullptr, nullptr}; bool captured = false, refused = false; uint64_t last_use = 0;
+  cudaGraphExec_t exec[2] = {nullptr, nullptr}; bool recorded = false; uint64_t uses = 0, next_try = 1, last_use = 0;
   int64_t launches = 0, gemm_launches = 0; double gemm_flops = 0, gemm_bytes = 0, split_bytes = 0; const float* out = nullptr;
-  void drop() { for (auto& e : exec) if (e) { cudaGraphExecDestroy(e); e = nullptr; } captured = false; }
+  void drop() { for (auto& e : exec) if (e) { cudaGraphExecDestroy(e); e = nullptr; } recorded = false; }
+  bool due() { return !recorded && ++uses >= next_try; }      // (a graph that could not be made is tried again after 4, 16, 64 ... uses)
+  void done(bool ok) { recorded = ok; if (!ok) { drop(); next_try *= 4; } }
 };
 constexpr size_t MAX_GRAPHS = 8;                             // per model: batch sizes and device-resident batches in turn
 static StepGraph* find_graph(gn_model* m, StepGraph key) {
@@ -1499,15 +1500,14 @@ static void note_graph(gn_model* m, StepGraph key) {
   }
   m->graphs.emplace_back(new StepGraph(key));
 }
-// Runs `issue` under stream capture; *out stays null when the work cannot be captured (the caller then runs it directly).
-template <class F> static int capture(Ctx* ctx, F&& issue, cudaGraphExec_t* out) {
-  *out = nullptr; cudaGraph_t g = nullptr;
-  GN_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  const int rc = issue();
-  const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-  if (rc == GN_OK && e == cudaSuccess && g && cudaGraphInstantiate(out, g, 0) != cudaSuccess) *out = nullptr;
-  if (g) cudaGraphDestroy(g);
-  cudaGetLastError(); return GN_OK;
+// What `issue` would launch as a graph; *out stays null when that cannot be made (the caller then runs it directly).
+template <class F> static void record(gn_model* m, F&& issue, cudaGraphExec_t* out) {
+  Ctx* ctx = &m->ctx->c; const uint64_t em = m->epoch, ec = ctx->epoch; GraphRec rec; *out = nullptr;
+  struct Guard { Ctx* c; ~Guard() { c->rec = nullptr; c->side_pending = false; cudaGetLastError(); } } guard{ctx};
+  if (cudaGraphCreate(&rec.graph, 0) != cudaSuccess) { rec.graph = nullptr; return; }
+  ctx->rec = &rec;
+  if (issue() != GN_OK || em != m->epoch || ec != ctx->epoch) return;      // (a buffer that was replaced may be in earlier nodes)
+  if (cudaGraphInstantiate(out, rec.graph, 0) != cudaSuccess) *out = nullptr;
 }
 static void reset_counters(Ctx* ctx) { ctx->gemm_flops = 0; ctx->gemm_launches = 0; ctx->gemm_ms = 0; ctx->ev_used = 0; ctx->gemm_bytes = 0; ctx->split_bytes = 0; }
 
@@ -1517,7 +1517,7 @@ static int train_step_issue(gn_model* m, const float* x, const float* y, bool ho
   const float inv = (float)(1.0 / (double)global_batch);                                        // net.go:703
   m->last_inv_batch = inv;
   const AdamArgs a = adam_args(m->lr, m->b1, m->b2, m->eps, m->timestep + 2, inv);
-  GN_TRY(wplanes_need_max(ctx, m->wplanes));                   // (a captured step relies on them)
+  GN_TRY(wplanes_need_max(ctx, m->wplanes));                   // (a recorded step relies on them)
   // small host batches (or a small x: token ids) go through one pinned block together with the coefficients: one copy instead of three
   const bool staged = host && y_at + ny <= STAGE_IN, staged_x = staged || (host && nx * 4 < (128u << 10));
   memcpy(ctx->h_stage, &a, sizeof a);
@@ -1527,25 +1527,25 @@ static int train_step_issue(gn_model* m, const float* x, const float* y, bool ho
   StepGraph key{B, global_batch, first_sample, xd, yd, staged, true};
   StepGraph* g = find_graph(m, key);
   const float* yp = nullptr;
-  auto copy_in = [&]() -> int { GN_CUDA(cudaMemcpyAsync(m->io.p, ctx->h_stage, (staged ? y_at + ny : staged_x ? IO_ARGS + nx : IO_ARGS) * 4, cudaMemcpyHostToDevice, ctx->stream)); return GN_OK; };
+  auto copy_in = [&]() -> int { GN_CUDA(stream_copy(ctx, m->io.p, ctx->h_stage, (staged ? y_at + ny : staged_x ? IO_ARGS + nx : IO_ARGS) * 4, cudaMemcpyHostToDevice)); return GN_OK; };
   auto first = [&]() -> int { return issue_forward(m, xd, B, global_batch, first_sample, &yp); };
   auto second = [&]() -> int { return issue_backward(m, yp, yd, B, global_batch, first_sample, a); };
   const bool split = host && !staged;                          // y is copied between the halves
-  if (g && !g->captured && !g->refused) {
+  if (g && g->due()) {
     const int64_t l0 = ctx->launches; reset_counters(ctx);
     m->wplanes.dirty = true;                                   // as in every step: the parameters have moved since the planes were written
     if (split) {
-      GN_TRY(capture(ctx, [&]() -> int { GN_TRY(copy_in()); return first(); }, &g->exec[0]));
-      if (g->exec[0]) GN_TRY(capture(ctx, second, &g->exec[1]));
-    } else GN_TRY(capture(ctx, [&]() -> int { GN_TRY(copy_in()); GN_TRY(first()); return second(); }, &g->exec[0]));
-    g->captured = g->exec[0] && (!split || g->exec[1]); g->refused = !g->captured;
+      record(m, [&]() -> int { GN_TRY(copy_in()); return first(); }, &g->exec[0]);
+      if (g->exec[0]) record(m, second, &g->exec[1]);
+    } else record(m, [&]() -> int { GN_TRY(copy_in()); GN_TRY(first()); return second(); }, &g->exec[0]);
     g->launches = ctx->launches - l0; ctx->launches = l0; g->gemm_launches = ctx->gemm_launches; g->gemm_flops = ctx->gemm_flops; g->gemm_bytes = ctx->gemm_bytes; g->split_bytes = ctx->split_bytes;
-    if (g->refused) { g->drop(); m->wplanes.dirty = true; }
+    g->done(g->exec[0] && (!split || g->exec[1]));
+    if (!g->recorded) { m->wplanes.dirty = true; forget_planes(ctx); }
   }
   reset_counters(ctx);
   if (split && !staged_x) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, x, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
   GN_CUDA(cudaEventRecord(m->ev0, ctx->stream));
-  const bool replay = g && g->captured;
+  const bool replay = g && g->recorded;
   if (replay) { GN_CUDA(cudaGraphLaunch(g->exec[0], ctx->stream)); }
   else { GN_TRY(copy_in()); GN_TRY(first()); }
   if (split) {                                               // on a stream of its own: it must not wait for the first half
@@ -1602,23 +1602,24 @@ static int forward_batch(gn_model* m, const float* x, int B, float* out) {
   if (staged) memcpy(ctx->h_stage, x, nx * 4);
   if (m->wplanes.used) GN_TRY(wplanes_refresh(ctx, m->wplanes));           // no-op unless the parameters changed since the last pass
   auto body = [&]() -> int {
-    if (staged) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, ctx->h_stage, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
+    if (staged) GN_CUDA(stream_copy(ctx, m->io.p + IO_ARGS, ctx->h_stage, nx * 4, cudaMemcpyHostToDevice));
     GN_TRY(forward(m, xd, B, &yp, false));
     // a few KB are written to host memory by a kernel, more by the copy engine
     const bool by_kernel = ny <= 4096;
-    if (small && !by_kernel) GN_CUDA(cudaMemcpyAsync(ctx->h_out, yp, ny * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    if (small && !by_kernel) GN_CUDA(stream_copy(ctx, ctx->h_out, yp, ny * 4, cudaMemcpyDeviceToHost));
     GN_LAUNCH(ctx, finish_kernel, by_kernel ? cdiv(ny, 256) : 1, by_kernel ? 256 : 32, 0, yp, ctx->d_out, by_kernel ? (int)ny : 0, (const int*)ctx->d_status, ctx->d_ret);
     return check_launch("finish");
   };
   StepGraph key{B, 0, 0, xd, nullptr, staged, false};
   StepGraph* g = find_graph(m, key);
-  if (g && !g->captured && !g->refused) {
+  if (g && g->due()) {
     const int64_t l0 = ctx->launches;
-    GN_TRY(capture(ctx, body, &g->exec[0]));
-    ctx->launches = l0; g->captured = g->exec[0] != nullptr; g->refused = !g->captured; g->out = yp;
+    record(m, body, &g->exec[0]);
+    ctx->launches = l0; g->done(g->exec[0] != nullptr); g->out = yp;
+    if (!g->recorded) { m->wplanes.dirty = true; forget_planes(ctx); }
   }
   if (!staged) GN_CUDA(cudaMemcpyAsync(m->io.p + IO_ARGS, x, nx * 4, cudaMemcpyHostToDevice, ctx->stream));
-  if (g && g->captured) { GN_CUDA(cudaGraphLaunch(g->exec[0], ctx->stream)); yp = g->out; forget_planes(ctx); }
+  if (g && g->recorded) { GN_CUDA(cudaGraphLaunch(g->exec[0], ctx->stream)); yp = g->out; forget_planes(ctx); }
   else GN_TRY(body());
   if (!small) GN_CUDA(cudaMemcpyAsync(out, yp, ny * 4, cudaMemcpyDeviceToHost, ctx->stream));
   GN_CUDA(cudaStreamSynchronize(ctx->stream));

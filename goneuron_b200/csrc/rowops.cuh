@@ -910,7 +910,7 @@ __global__ void scale_kernel(float* __restrict__ x, long n, float s) {
 //   m = b1*m + (1-b1)*g' ; v = b2*v + (1-b2)*g'*g' ; p -= effLR * m / (sqrt(v) + eps)
 // `status` (may be null): the context's status word; when a bounded wait of an earlier kernel of this step gave up, the
 // gradients are not trustworthy and the pass leaves the parameters and moments untouched.
-// `dargs` (may be null): the coefficients are read from there instead of `a`, so that a captured launch follows the schedule.
+// `dargs` (may be null): the coefficients are read from there instead of `a`, so that a recorded launch follows the schedule.
 // `ret` (may be null; host memory): receives the step's loss sum and the status word, the caller's one read-back.
 struct AdamArgs { float effLR, b1, b2, omb1, omb2, eps, grad_scale; };
 // `ranges` (MX): parameter ranges whose largest magnitude after the update is wanted, ascending; mx[j] (zero on entry) receives that of
