@@ -147,7 +147,9 @@ const char* gn_last_error(void);
  * clipping, lstm.go:694,725-751); 1 = trainBatchSequential (net.go:721-784). */
 int gn_model_create(gn_ctx* ctx, const gn_layer_desc* layers, int n_layers,
                     int loss_kind, int virtual_workers, gn_model** out);
-int gn_model_destroy(gn_model* m);            /* idempotent; mirrors Layer.Close (layer.go:805-845) */
+/* Idempotent; mirrors Layer.Close (layer.go:805-845).  While other models live on the GPU, up to 8 GiB of what a model
+ * releases is kept for the next one (GONEURON_CUDA_KEEP_BYTES sets the bound); closing the last one returns all of it. */
+int gn_model_destroy(gn_model* m);
 int gn_model_param_count(gn_model* m, int64_t* n);
 int gn_model_in_size(gn_model* m, int64_t* n);   /* floats per input sample  */
 int gn_model_out_size(gn_model* m, int64_t* n);  /* floats per output sample */
