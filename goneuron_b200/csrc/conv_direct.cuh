@@ -12,9 +12,10 @@ namespace gn {
 
 // dst[ch * plane + r * ld + x] = src[ch][ylo + r][xlo + x], x < ld (a multiple of four), of `nch` channels with `rows` rows each; zero
 // outside the image and from channel `have` on.  All copies of a thread are in flight at once (one after the other, a load and
-// a store at a time, they were 60 us of the weight gradient); whole 16-byte pieces where the rows allow it.
+// a store at a time, they were 60 us of the weight gradient); whole 16-byte pieces where the rows
+// and the pointer (a first layer reads the caller's batch) allow it.
 __device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const float* __restrict__ src, int nch, int have, int rows, int ylo, int H, int W, int xlo) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5; const bool v4 = xlo == 0 && ld == W;      // W a multiple of four
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5; const bool v4 = xlo == 0 && ld == W && (reinterpret_cast<uintptr_t>(src) & 15) == 0;      // W a multiple of four
   const int n = v4 ? ld >> 2 : ld, lw = n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32, step = nw * (32 / lw), lx = lane & (lw - 1);
   int q = warp * (32 / lw) + lane / lw, ch = q / rows, r = q - ch * rows;
   for (; ch < nch;) {

@@ -85,3 +85,43 @@ def test_batchnorm_running_statistics_of_a_long_batch(device, oracle):
     model.TrainBatch(x, y)
     assert norm_err(model.State(), ref.state) <= TOL
     model.Close()
+
+
+ANY_POINTER = {
+    "conv 5x5": [D.Conv2D(3, 6, 5, 1, 0, D.RELU, 12, 16), D.Flatten(), D.Dense(6 * 8 * 12, 4, D.SOFTMAX)],
+    "conv 1x1": [D.Conv2D(4, 9, 1, 1, 0, D.TANH, 8, 8), D.Flatten(), D.Dense(9 * 64, 4, D.SOFTMAX)],
+    "conv 3x3": [D.Conv2D(2, 5, 3, 1, 1, D.RELU, 8, 8), D.Flatten(), D.Dense(5 * 64, 4, D.SOFTMAX)],
+    "pool": [D.MaxPool2D(3, 2, 2, 0, 8, 8), D.Flatten(), D.Dense(48, 4, D.SOFTMAX)],
+    "batch norm": [D.BatchNorm2D(3, 8, 8), D.Flatten(), D.Dense(192, 4, D.SOFTMAX)],
+    "dense": [D.Dense(64, 32, D.RELU), D.Dense(32, 4, D.SOFTMAX)],
+    "wide dense": [D.Dense(512, 640, D.RELU), D.Dense(640, 4, D.SOFTMAX)],
+    "lstm": [D.SequenceUnrollerLSTM(8, 16, 6, False), D.Dense(16, 4, D.SOFTMAX)],
+    "gru": [D.SequenceUnrollerGRU(8, 16, 6, False), D.Dense(16, 4, D.SOFTMAX)],
+    "block": [D.TransformerBlock(64, 2, 32, 128, False), D.Flatten(), D.Dense(2048, 4, D.SOFTMAX)],
+    "embedding": [D.Embedding(30, 32, 8), D.TransformerBlock(32, 2, 8, 64, True), D.CLSPooling(8, 32), D.Dense(32, 4, D.LOGSOFTMAX)],
+}
+
+
+@pytest.mark.parametrize("kind", sorted(ANY_POINTER))
+@pytest.mark.parametrize("batch", [5, 600])
+def test_batches_at_any_float_address(device, kind, batch):
+    """A batch in device memory may start at any float: the kernels that read it take their narrow loads there.  Against the same
+    batch at the allocation's start, whose sums are the same."""
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = ANY_POINTER[kind]
+    rng = np.random.Generator(np.random.PCG64(4))
+    params = configs.init_params(layers, rng)
+    in_size = {"conv 5x5": 576, "conv 1x1": 256, "conv 3x3": 128, "pool": 192, "batch norm": 192, "dense": 64, "wide dense": 512, "lstm": 48, "gru": 48, "block": 2048, "embedding": 8}[kind]
+    x = (rng.integers(0, 30, (batch, in_size)) if kind == "embedding" else rng.standard_normal((batch, in_size))).astype(np.float32)
+    y = np.eye(4, dtype=np.float32)[rng.integers(0, 4, batch)]
+    got = []
+    for at in (0, 1):
+        xd, yd = (device.alloc(np.concatenate([np.zeros(at, np.float32), a.ravel()])) for a in (x, y))
+        model = Sequential(layers, device).Compile(Adam(1e-3), D.CROSS_ENTROPY)
+        model.SetParams(params)
+        loss = model.TrainBatchDevice(C.c_void_p(xd.value + 4 * at), C.c_void_p(yd.value + 4 * at), batch)
+        got.append((loss, model.Gradients()))
+        model.Close()
+        device.free(xd); device.free(yd)
+    assert abs(got[0][0] - got[1][0]) <= 1e-6 * max(1.0, abs(got[0][0]))
+    assert norm_err(got[1][1], got[0][1]) <= 1e-6
