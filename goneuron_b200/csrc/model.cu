@@ -1565,21 +1565,23 @@ static int train_step_issue(gn_model* m, const float* x, const float* y, bool ho
   return GN_OK;
 }
 
+// A call that fails after work has been queued must not leave that work running behind the caller's back (the pinned blocks are the next
+// call's): waits for all of the context's streams.
+static int drained(gn_model* m, int rc) {
+  Ctx* ctx = &m->ctx->c; const std::string msg = last_error();
+  for (auto s : {ctx->comm_stream, ctx->copy_stream, ctx->side_stream, ctx->stream}) if (s) cudaStreamSynchronize(s);
+  cudaGetLastError(); ctx->side_pending = false;
+  m->wplanes.dirty = true; m->wplanes.max_ok = false; forget_planes(ctx); last_error() = msg; return rc;
+}
+
 static int train_step(gn_model* m, const float* x, const float* y, bool host, int B, int global_batch, int first_sample, float* mean_loss) {
   Ctx* ctx = &m->ctx->c;
   if (global_batch <= 0) { global_batch = B; first_sample = 0; }
   GN_TRY(ensure_capacity(m, B, true));
   int64_t launches0 = ctx->launches;
   m->wplanes_layerwise = false;
-  // Anything that fails after work has been queued must not leave that work running behind the caller's back.
   int rc = train_step_issue(m, x, y, host, B, global_batch, first_sample);
-  if (rc != GN_OK) {
-    // drain what was queued before the failure (both streams) so that nothing of this step runs after the call returned
-    const std::string msg = last_error();
-    if (ctx->comm_stream) cudaStreamSynchronize(ctx->comm_stream);
-    cudaStreamSynchronize(ctx->copy_stream); cudaStreamSynchronize(ctx->side_stream); cudaStreamSynchronize(ctx->stream); cudaGetLastError(); ctx->side_pending = false;
-    m->wplanes.dirty = true; m->wplanes.max_ok = false; last_error() = msg; return rc;
-  }
+  if (rc != GN_OK) return drained(m, rc);
   int st; memcpy(&st, &ctx->h_ret[1], sizeof(int));
   if (st != 0) { m->wplanes.dirty = true; m->wplanes.max_ok = false; return clear_status(ctx, st); }         // the Adam pass saw the same word and left parameters, moments and the step counter alone
   m->timestep += 1;
@@ -1595,9 +1597,8 @@ static int train_step(gn_model* m, const float* x, const float* y, bool host, in
 }
 
 // Batched inference, host to host.
-static int forward_batch(gn_model* m, const float* x, int B, float* out) {
+static int forward_issue(gn_model* m, const float* x, int B, float* out) {
   Ctx* ctx = &m->ctx->c; const size_t nx = (size_t)B * m->in_size, ny = (size_t)B * m->out_size;
-  GN_TRY(ensure_capacity(m, B, false));
   const bool staged = nx <= STAGE_IN, small = ny <= STAGE_FLOATS;      // through the pinned blocks, in and out
   const float* xd = m->io.p + IO_ARGS; const float* yp = nullptr;
   if (staged) memcpy(ctx->h_stage, x, nx * 4);
@@ -1626,7 +1627,13 @@ static int forward_batch(gn_model* m, const float* x, int B, float* out) {
   GN_CUDA(cudaStreamSynchronize(ctx->stream));
   if (!g) note_graph(m, key);
   if (small) memcpy(out, ctx->h_out, ny * 4);
-  int st; memcpy(&st, &ctx->h_ret[1], sizeof(int));
+  return GN_OK;
+}
+static int forward_batch(gn_model* m, const float* x, int B, float* out) {
+  GN_TRY(ensure_capacity(m, B, false));
+  const int rc = forward_issue(m, x, B, out);
+  if (rc != GN_OK) return drained(m, rc);
+  Ctx* ctx = &m->ctx->c; int st; memcpy(&st, &ctx->h_ret[1], sizeof(int));
   return st != 0 ? clear_status(ctx, st) : GN_OK;
 }
 

@@ -91,3 +91,33 @@ def test_head_parity(device, oracle, n, act, loss):
     assert abs(got - loss_ref) <= TOL * max(1.0, abs(loss_ref))
     assert_grads_close(layers, model.Gradients(), ref.grads, floor=lit.grads)
     model.Close()
+
+
+def test_a_failed_prediction_leaves_nothing_running(device):
+    """Convolutions of some tens of milliseconds, then a layer that the library refuses: when the call returns its error, the stream is
+    empty (the call's pinned block is the next call's), and the context goes on working."""
+    import time
+    from goneuron_b200 import _lib
+    from goneuron_b200.sequential import Adam, Sequential
+    hw = 1024
+    layers = [D.Conv2D(1, 16, 7, 1, 3, D.RELU, hw, hw), D.Conv2D(16, 16, 7, 1, 3, D.RELU, hw, hw), D.MaxPool2D(16, 64, 64, 0, hw, hw),
+              D.SequenceUnrollerLSTM(64, 512, 64, False), D.Dense(512, 2, D.LINEAR)]
+    model = Sequential(layers, device).Compile(Adam(1e-3), D.MSE)
+    x = np.random.default_rng(0).standard_normal((6, hw * hw)).astype(np.float32)
+    times = []
+    for _ in range(3):
+        t0 = time.perf_counter()
+        with pytest.raises(_lib.GoNeuronCudaError) as e:
+            model.PredictBatch(x)
+        t1 = time.perf_counter()
+        device.synchronize()
+        times.append((t1 - t0, time.perf_counter() - t1))
+        assert e.value.code == -5 and "shared memory" in str(e.value)
+    model.Close()
+    call, wait = min(times)
+    assert call + wait > 0.02 and wait < 0.1 * (call + wait), times
+    l2, k2, p2, x2, y2, lr = configs.make_case("mlp", batch=8)
+    other = Sequential(l2, device).Compile(Adam(lr), k2)
+    other.SetParams(p2)
+    assert np.isfinite(other.PredictBatch(x2)).all()
+    other.Close()
