@@ -26,7 +26,7 @@ __device__ __forceinline__ float act_fwd(int act, float x, float alpha = 0.f) {
     case GN_ACT_TANH: return tanh_rn(x);
     case GN_ACT_LEAKY_RELU: return x > 0.f ? x : alpha * x;
     case GN_ACT_ELU: return x > 0.f ? x : alpha * (exp_rn(x) - 1.f);
-    case GN_ACT_GELU: { float x3 = x * x * x; float arg = 0.7978845608028654f * (x + 0.044715f * x3); return 0.5f * x * (1.f + tanh_rn(arg)); }
+    case GN_ACT_GELU: return gelu_f(x);
     case GN_ACT_SILU: { if (x >= 0.f) return x * (1.f / (1.f + exp_rn(-x))); float e = exp_rn(x); return x * e / (1.f + e); }
     default: return x;
   }

@@ -70,6 +70,17 @@ def test_elementwise_functions_are_rounded_once(device):
         ulp = np.spacing(np.abs(want).astype(np.float32)).astype(np.float64)
         assert np.max(np.abs(got - want)[ok] / ulp[ok]) <= ulps, (act, np.max(np.abs(got - want)[ok] / ulp[ok]))
         assert np.max(np.abs(got - want)[~ok]) <= 1e-37
+    # GELU (the function of the plane-writing epilogues too): 2^-23 |x|, what the reference's float32 order leaves, and below it on average
+    gelu = lambda v: v / (1 + np.exp(-2 * np.sqrt(2 / np.pi) * (v + 0.044715 * v ** 3)))      # noqa: E731
+    xg = np.concatenate([rng.uniform(-6, 6, 400000), rng.uniform(-1, 1, 200000), 10.0 ** rng.uniform(-30, -1, 5000), [9.0, -9.0, 12.0, -12.0, 40.0]]).astype(np.float32).reshape(-1, 1)
+    model = Sequential([D.Dense(1, 1, D.GELU)], device).Compile(Adam(1e-3), D.MSE)
+    model.SetParams(np.array([1.0, 0.0], np.float32))
+    with np.errstate(over="ignore"):
+        err = np.abs(model.PredictBatch(xg) - gelu(xg.astype(np.float64))) / np.abs(xg.astype(np.float64))
+    assert np.max(err) <= 2.0 ** -23 and np.sqrt(np.mean(err[:400000] ** 2)) <= 2.0 ** -25, (np.max(err), np.sqrt(np.mean(err[:400000] ** 2)))
+    ends = model.PredictBatch(np.array([[np.inf], [-np.inf], [np.nan], [50], [-50], [0.0], [-3e38]], np.float32)).ravel()
+    assert ends[0] == np.inf and np.isnan(ends[1:3]).all() and np.array_equal(ends[3:], [50, 0, 0, 0])
+    model.Close()
     model = Sequential([D.Dense(1, 1, D.TANH)], device).Compile(Adam(1e-3), D.MSE)
     model.SetParams(np.array([1.0, 0.0], np.float32))
     assert np.array_equal(model.PredictBatch(np.array([[np.inf], [-np.inf], [50], [-50]], np.float32)).ravel(), [1, -1, 1, -1])
