@@ -893,10 +893,13 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
 // `x_last` != null: the last-token inputs as a dense [B, in] array instead of a strided view of x; `dz_planes` != null: dz
 // exists only as operand planes.
 // `stack` > 1: several layers with the same input, whose dz (and, `ws` apart, whose weight gradients) follow one another.
-static int token_sums(Ctx* ctx, const float* dz, int B, int T, int out, float* delta) {
-  if (out % 4 == 0 && ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(delta)) & 15) == 0)
-    GN_LAUNCH(ctx, token_sum_vec_kernel, dim3(cdiv(out, 128), B), dim3(32, 8), 0, dz, T, out, delta);
-  else GN_LAUNCH(ctx, token_sum_kernel, dim3(cdiv(out, 128), B), dim3(128, 4), 0, dz, T, out, delta);
+static int token_sums(Ctx* ctx, const float* dz, int n, int T, int out, float* delta) {      // n: sequences (of all layers of a stack)
+  const bool vec = out % 4 == 0 && ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(delta)) & 15) == 0;
+  for (int s0 = 0; s0 < n; s0 += 65535) {                   // (a grid's second dimension)
+    const dim3 grid(cdiv(out, 128), std::min(n - s0, 65535)); const float* z = dz + (long)s0 * T * out; float* d = delta + (long)s0 * out;
+    if (vec) GN_LAUNCH(ctx, token_sum_vec_kernel, grid, dim3(32, 8), 0, z, T, out, d);
+    else GN_LAUNCH(ctx, token_sum_kernel, grid, dim3(128, 4), 0, z, T, out, d);
+  }
   return check_launch("token_sums");
 }
 static int weight_bias_grads_stack(gn_model* m, int stack, int B, int out, int in, const float* delta, const float* x_last, long ldx, float* gW, float* gb, long ws) {

@@ -53,11 +53,16 @@ def test_sequences_of_another_shape_below(device, oracle, below):
     _parity(device, oracle, [D.Embedding(60, 32, 6)] + below + [D.TransformerBlock(24, 2, 8, 40, True), D.CLSPooling(8, 24), D.Dense(24, 11, D.LOGSOFTMAX)])
 
 
-def _parity(device, oracle, layers):
+def test_more_sequences_than_a_grid_dimension_has_for_three_projections(device, oracle):
+    """22 000 short sequences: the token sums of dQ, dK and dV are 66 000 rows of one launch's second dimension."""
+    _parity(device, oracle, _model(2, 16, 1, 16, [False], False, classes=3), batch=22000)
+
+
+def _parity(device, oracle, layers, batch=3):
     from goneuron_b200.sequential import Adam, Sequential
     rng = np.random.Generator(np.random.PCG64(99))
     params = configs.init_params(layers, rng)
-    x, y = configs.make_inputs("transformer", layers, 3, rng)
+    x, y = configs.make_inputs("transformer", layers, batch, rng)
     ref = oracle.OracleState(layers, D.CROSS_ENTROPY, params, lr=1e-4)
     out = oracle.OracleState(layers, D.CROSS_ENTROPY, params).forward_batch(x, threads=3, precision=64)
     lit = oracle.OracleState(layers, D.CROSS_ENTROPY, params, lr=1e-4)
