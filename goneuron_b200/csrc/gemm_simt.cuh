@@ -117,7 +117,7 @@ __device__ __forceinline__ float sg_finish(const GemmDesc& g, const float* R, in
 }
 
 template <int BM, int BN, int BK, int TM, int TN, bool A_KFAST, bool B_NFAST>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmDesc g, int splits, int vec_a, int vec_b) {
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmDesc g, int splits, int vec_a, int vec_b, int y0) {
   using Cfg = SgCfg<BM, BN, BK, TM, TN>;
   constexpr int THREADS = Cfg::THREADS, LDA = Cfg::LDA, LDB = Cfg::LDB, CX = BN / TN;
   __shared__ __align__(16) float sm[Cfg::SMEM_FLOATS];
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
   const float* B = g.B + b1 * g.b_b1 + b2 * g.b_b2;
   float* C = g.C + b1 * g.c_b1 + b2 * g.c_b2;
   const float* R = g.R ? g.R + b1 * g.r_b1 + b2 * g.r_b2 : nullptr;
-  const int m0 = blockIdx.y * BM, n0 = nt * BN;
+  const int m0 = (y0 + blockIdx.y) * BM, n0 = nt * BN;
   if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + BM - 1) return;             // (the whole cluster returns)
   int kbeg = 0, kend = g.K;
   if (g.flags & GEMM_KBEG_AT_M0) kbeg = (m0 / BK) * BK;
@@ -321,12 +321,15 @@ inline int gemm_simt_tile(Ctx* ctx, const GemmDesc& g, int splits) {
   auto vec = [](const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; };
   const bool ak = g.sa_k == 1, bn = g.sb_n == 1;
   const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
-  const dim3 grid(cdiv(g.N, BN) * splits, cdiv(g.M, BM), g.batch1 * g.batch2); constexpr int THREADS = SgCfg<BM, BN, BK, TM, TN>::THREADS;
-  if (ak && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, 0, splits, g, splits, va, vb);
-  else if (ak && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, 0, splits, g, splits, va, vb);
-  else if (g.sa_m == 1 && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, 0, splits, g, splits, va, vb);
-  else if (g.sa_m == 1 && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, 0, splits, g, splits, va, vb);
-  else return fail(GN_ERR_UNSUPPORTED, "gemm_simt: neither stride of an operand is 1");
+  const int tiles_m = cdiv(g.M, BM); constexpr int THREADS = SgCfg<BM, BN, BK, TM, TN>::THREADS;
+  for (int y0 = 0; y0 < tiles_m; y0 += 65535) {             // (a grid's second dimension)
+    const dim3 grid(cdiv(g.N, BN) * splits, std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
+    if (ak && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
+    else if (ak && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
+    else if (g.sa_m == 1 && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
+    else if (g.sa_m == 1 && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
+    else return fail(GN_ERR_UNSUPPORTED, "gemm_simt: neither stride of an operand is 1");
+  }
   return check_launch("gemm_simt");
 }
 // Blocks per output tile.  A run shorter than 64 is not worth a block.  Where the rows of A are samples (or tokens), the

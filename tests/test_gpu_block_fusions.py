@@ -174,3 +174,15 @@ def test_cuda_core_contraction_steps(device, M, N, K):
     ref = a.astype(np.float64) @ b.astype(np.float64).T + bias
     size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64).T + np.abs(bias)
     assert np.max(np.abs(c - ref) / size) <= (K + 2) * 2.0 ** -24
+
+
+def test_cuda_core_contraction_of_millions_of_rows(device):
+    """More tiles of 64 rows than a grid's second dimension has.  Bound as above."""
+    from goneuron_b200 import _lib
+    M, N, K = 65535 * 64 + 70, 8, 4
+    rng = np.random.default_rng(1)
+    a, b, bias = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    c = np.empty((M, N), np.float32)
+    _lib.check(_lib.load().gn_op_gemm_nt(device.handle, 0, M, N, K, _f(a), _f(b), _f(bias), _f(c)))
+    size = np.abs(a) @ np.abs(b).T + np.abs(bias)
+    assert np.max(np.abs(c - (a.astype(np.float64) @ b.astype(np.float64).T + bias)) / size) <= (K + 2) * 2.0 ** -24
