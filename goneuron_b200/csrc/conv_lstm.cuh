@@ -172,38 +172,43 @@ __global__ void conv1d_wgrad_kernel(const float* __restrict__ g, const float* __
 }
 
 struct PoolShape { int B, C, k, s, p, H, W, oH, oW; };
-// reference: maxpool2d.go:192-221 (init -inf, strict '>', first maximum wins, argmax = flat CHW index).  A block takes a piece of one
+// reference: maxpool2d.go:192-221 (init -inf, strict '>', first maximum wins, argmax = flat CHW index).  A block takes pieces of one
 // (sample, channel) plane: the index arithmetic is 32-bit and per pixel of the plane.
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int* __restrict__ arg, PoolShape c) {
-  const long pl = blockIdx.x; const int ch = (int)(pl % c.C), i = blockIdx.y * 256 + threadIdx.x; if (i >= c.oH * c.oW) return;
-  const int oh = i / c.oW, ow = i - oh * c.oW, h0 = oh * c.s - c.p, w0 = ow * c.s - c.p;
-  const float* xp = x + pl * c.H * c.W;
-  float mv = -INFINITY; int mi = -1;
-  if (c.k == 2 && c.p == 0) {                              // whole windows: both rows in flight
-    const float* q = xp + h0 * c.W + w0; const float a = q[0], b = q[1], d = q[c.W], e = q[c.W + 1]; const int at = (ch * c.H + h0) * c.W + w0;
-    if (a > mv) { mv = a; mi = at; } if (b > mv) { mv = b; mi = at + 1; } if (d > mv) { mv = d; mi = at + c.W; } if (e > mv) { mv = e; mi = at + c.W + 1; }
-  } else for (int kh = 0; kh < c.k; kh++) for (int kw = 0; kw < c.k; kw++) {
-    const int ih = h0 + kh, iw = w0 + kw;
-    if (ih >= 0 && ih < c.H && iw >= 0 && iw < c.W) { const float v = xp[ih * c.W + iw]; if (v > mv) { mv = v; mi = (ch * c.H + ih) * c.W + iw; } }
+  const long pl = blockIdx.x; const int ch = (int)(pl % c.C); const float* xp = x + pl * c.H * c.W;
+  for (unsigned at = blockIdx.y * 256 + threadIdx.x; at < (unsigned)(c.oH * c.oW); at += gridDim.y * 256) {
+    const int i = (int)at, oh = i / c.oW, ow = i - oh * c.oW, h0 = oh * c.s - c.p, w0 = ow * c.s - c.p;
+    float mv = -INFINITY; int mi = -1;
+    if (c.k == 2 && c.p == 0) {                              // whole windows: both rows in flight
+      const float* q = xp + h0 * c.W + w0; const float a = q[0], b = q[1], d = q[c.W], e = q[c.W + 1]; const int first = (ch * c.H + h0) * c.W + w0;
+      if (a > mv) { mv = a; mi = first; } if (b > mv) { mv = b; mi = first + 1; } if (d > mv) { mv = d; mi = first + c.W; } if (e > mv) { mv = e; mi = first + c.W + 1; }
+    } else for (int kh = 0; kh < c.k; kh++) for (int kw = 0; kw < c.k; kw++) {
+      const int ih = h0 + kh, iw = w0 + kw;
+      if (ih >= 0 && ih < c.H && iw >= 0 && iw < c.W) { const float v = xp[ih * c.W + iw]; if (v > mv) { mv = v; mi = (ch * c.H + ih) * c.W + iw; } }
+    }
+    y[pl * c.oH * c.oW + i] = mv; arg[pl * c.oH * c.oW + i] = mi;
   }
-  y[pl * c.oH * c.oW + i] = mv; arg[pl * c.oH * c.oW + i] = mi;
 }
 // Windows that do not overlap: every input element looks its one window up (no zero fill, no atomics).  `relu`: the derivative of a
 // ReLU right below is applied as well -- the element that won its window passes the gradient on only if it is positive (y > 0).
 __global__ void __launch_bounds__(256) maxpool_bwd_gather_kernel(const float* __restrict__ g, const int* __restrict__ arg, const float* __restrict__ y, float* __restrict__ dx, PoolShape c, int relu) {
-  const long pl = blockIdx.x; const int ch = (int)(pl % c.C), i = blockIdx.y * 256 + threadIdx.x; if (i >= c.H * c.W) return;
-  const int ih = i / c.W, iw = i - ih * c.W, oh = (ih + c.p) / c.s, ow = (iw + c.p) / c.s; float v = 0.f;
-  if (oh < c.oH && ow < c.oW) { const long o = pl * c.oH * c.oW + oh * c.oW + ow; if (arg[o] == ch * c.H * c.W + i && (!relu || y[o] > 0.f)) v = g[o]; }
-  dx[pl * c.H * c.W + i] = v;
+  const long pl = blockIdx.x; const int ch = (int)(pl % c.C);
+  for (unsigned at = blockIdx.y * 256 + threadIdx.x; at < (unsigned)(c.H * c.W); at += gridDim.y * 256) {
+    const int i = (int)at, ih = i / c.W, iw = i - ih * c.W, oh = (ih + c.p) / c.s, ow = (iw + c.p) / c.s; float v = 0.f;
+    if (oh < c.oH && ow < c.oW) { const long o = pl * c.oH * c.oW + oh * c.oW + ow; if (arg[o] == ch * c.H * c.W + i && (!relu || y[o] > 0.f)) v = g[o]; }
+    dx[pl * c.H * c.W + i] = v;
+  }
 }
 // 2 x 2 windows that tile the plane (W even, 8-byte aligned rows): a thread per window
 __global__ void __launch_bounds__(256) maxpool_bwd_2x2_kernel(const float* __restrict__ g, const int* __restrict__ arg, const float* __restrict__ y, float* __restrict__ dx, PoolShape c, int relu) {
-  const long pl = blockIdx.x; const int i = blockIdx.y * 256 + threadIdx.x; if (i >= c.oH * c.oW) return;
-  const int oh = i / c.oW, ow = i - oh * c.oW; const long o = pl * c.oH * c.oW + i;
-  const float v = relu && !(y[o] > 0.f) ? 0.f : g[o]; const int at = ((int)(pl % c.C) * c.H + 2 * oh) * c.W + 2 * ow, d = arg[o] - at;
-  float* q = dx + (pl * c.H + 2 * oh) * c.W + 2 * ow;
-  *reinterpret_cast<float2*>(q) = make_float2(d == 0 ? v : 0.f, d == 1 ? v : 0.f);
-  *reinterpret_cast<float2*>(q + c.W) = make_float2(d == c.W ? v : 0.f, d == c.W + 1 ? v : 0.f);
+  const long pl = blockIdx.x;
+  for (unsigned at = blockIdx.y * 256 + threadIdx.x; at < (unsigned)(c.oH * c.oW); at += gridDim.y * 256) {
+    const int i = (int)at, oh = i / c.oW, ow = i - oh * c.oW; const long o = pl * c.oH * c.oW + i;
+    const float v = relu && !(y[o] > 0.f) ? 0.f : g[o]; const int d = arg[o] - (((int)(pl % c.C) * c.H + 2 * oh) * c.W + 2 * ow);
+    float* q = dx + (pl * c.H + 2 * oh) * c.W + 2 * ow;
+    *reinterpret_cast<float2*>(q) = make_float2(d == 0 ? v : 0.f, d == 1 ? v : 0.f);
+    *reinterpret_cast<float2*>(q + c.W) = make_float2(d == c.W ? v : 0.f, d == c.W + 1 ? v : 0.f);
+  }
 }
 // dx zero-filled beforehand; windows may overlap when stride < kernel, hence the atomic add (maxpool2d.go:395-406)
 __global__ void maxpool_bwd_kernel(const float* __restrict__ g, const int* __restrict__ arg, float* __restrict__ dx, PoolShape c) {

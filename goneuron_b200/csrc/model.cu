@@ -789,7 +789,7 @@ static int forward(gn_model* m, const float* x, int B, const float** y_out, bool
       case GN_LAYER_MAXPOOL2D: {
         PoolShape c{B, d.in_size, d.kernel, d.stride, d.padding, d.in_h, d.in_w,
                     (d.in_h + 2 * d.padding - d.kernel) / d.stride + 1, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
-        GN_LAUNCH(ctx, maxpool_fwd_kernel, dim3(B * c.C, cdiv((long)c.oH * c.oW, 256)), 256, 0, cur, l.out.p, (int*)l.idx.p, c);
+        GN_LAUNCH(ctx, maxpool_fwd_kernel, dim3(B * c.C, std::min(cdiv((long)c.oH * c.oW, 256), 65535u)), 256, 0, cur, l.out.p, (int*)l.idx.p, c);
         cur = l.out.p; break; }
       case GN_LAYER_CONV1D: {
         Conv1Shape c{B, d.in_size, d.out_size, d.kernel, d.stride, d.padding, d.in_w, (d.in_w + 2 * d.padding - d.kernel) / d.stride + 1};
@@ -1278,8 +1278,8 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
         if (c.k <= c.s) {
           gated = relu_conv_below(li);
           if (c.k == 2 && c.s == 2 && c.p == 0 && c.H == 2 * c.oH && c.W == 2 * c.oW)
-            GN_LAUNCH(ctx, maxpool_bwd_2x2_kernel, dim3(B * c.C, cdiv((long)c.oH * c.oW, 256)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
-          else GN_LAUNCH(ctx, maxpool_bwd_gather_kernel, dim3(B * c.C, cdiv((long)c.H * c.W, 256)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
+            GN_LAUNCH(ctx, maxpool_bwd_2x2_kernel, dim3(B * c.C, std::min(cdiv((long)c.oH * c.oW, 256), 65535u)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
+          else GN_LAUNCH(ctx, maxpool_bwd_gather_kernel, dim3(B * c.C, std::min(cdiv((long)c.H * c.W, 256), 65535u)), 256, 0, g, (const int*)l.idx.p, (const float*)l.out.p, dx, c, gated ? 1 : 0);
           g = dx; flip ^= 1; break;
         }
         GN_CUDA(stream_zero(ctx, dx, (size_t)B * l.in_size * sizeof(float)));

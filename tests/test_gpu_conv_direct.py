@@ -71,6 +71,25 @@ def test_maxpool_gradient(device, oracle, k, s, p, hw):
     model.Close()
 
 
+def test_maxpool_of_a_large_plane(device):
+    """More than 65 535 x 256 pixels: a block takes several pieces of the plane, in all three kernels."""
+    from goneuron_b200.sequential import Adam, Sequential
+    hw = 8194                                                 # halves to 4097 x 4097 = 16.8 M pixels, then to 17 x 17
+    layers = [D.MaxPool2D(1, 2, 2, 0, hw, hw), D.MaxPool2D(1, 241, 241, 0, hw // 2, hw // 2), D.Flatten(), D.Dense(289, 2, D.LINEAR)]
+    rng = np.random.default_rng(2)
+    params = rng.standard_normal(289 * 2 + 2).astype(np.float32)
+    x, y = rng.standard_normal((1, hw * hw), dtype=np.float32), np.array([[1.0, -2.0]], np.float32)
+    model = Sequential(layers, device).Compile(Adam(1e-3), D.MSE)
+    model.SetParams(params)
+    p = x.reshape(17, 482, 17, 482).max((1, 3)).reshape(1, 289).astype(np.float64)
+    out = p @ params[:578].reshape(2, 289).T.astype(np.float64) + params[578:]
+    assert norm_err(model.PredictBatch(x), out) <= 1e-5
+    model.TrainBatch(x, y)                                    # (runs the gradients of both layers)
+    g = model.Gradients()
+    assert norm_err(g[:578].reshape(2, 289), (out - y).T @ p) <= 1e-5
+    model.Close()
+
+
 def test_batchnorm_running_statistics_of_a_long_batch(device, oracle):
     """More samples than a block stages at a time, more channels than a block has lanes."""
     from goneuron_b200.sequential import Adam, Sequential
