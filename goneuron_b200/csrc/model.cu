@@ -569,6 +569,8 @@ static int conv_backward(gn_model* m, const ConvShape& c, int act, float alpha, 
   if (dx) {
     const long ni = (long)c.B * c.inC * c.H * c.W;
     if (eng == CONV_TC && c.s == 1) { float* wtmp; GN_TRY(ensure(m, S_DELTA, (size_t)nW, &wtmp)); GN_TRY(conv_tc_dgrad(ctx, c, dz, p, wtmp, dx)); }
+    else if (c.s == 1 && c.k == 3) GN_LAUNCH(ctx, conv2d_dgrad_s1_kernel<3>, ew_grid(ctx, ni), 256, 0, dz, p, dx, c);
+    else if (c.s == 1 && c.k == 5) GN_LAUNCH(ctx, conv2d_dgrad_s1_kernel<5>, ew_grid(ctx, ni), 256, 0, dz, p, dx, c);
     else GN_LAUNCH(ctx, conv2d_dgrad_kernel, ew_grid(ctx, ni), 256, 0, dz, p, dx, c);
   }
   return check_launch("conv_backward");
