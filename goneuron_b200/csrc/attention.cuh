@@ -414,7 +414,9 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_bwd_kernel(const float* 
   }
   ar_weighted(ds, K + base, T, D, hd, part, dQ + row);
 }
-constexpr int AR_MAX_T = 16384;                             // scores of a row (twice, in the backward kernel) live in shared memory
+// The scores of a row (twice, in the backward kernel) and two rows of the head live in shared memory; beyond that all tokens are computed.
+constexpr int AR_MAX_T = 16384, AR_SMEM = 200 * 1024;
+inline bool attn_rows_fit(int T, int hd) { return T <= AR_MAX_T && ((size_t)2 * hd + 2 * T) * sizeof(float) <= AR_SMEM; }
 inline bool ar_vec(const float* a, const float* b, int D, int hd) { return D % 4 == 0 && hd % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0; }
 inline int attn_rows_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, int B, int T, int TE, int D, int H, int causal) {
   const int hd = D / H; const size_t smem = ((size_t)hd + T) * sizeof(float);

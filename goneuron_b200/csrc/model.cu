@@ -621,10 +621,10 @@ static void plan_token_rows(gn_model* m, bool training) {
   for (auto& l : m->L) { l.out_rows = 0; l.in_row0 = l.row0_grad = false; }
   for (int li = (int)m->L.size() - 1; li > 0; li--) {
     if (m->L[li].d.kind != GN_LAYER_CLS_POOLING) continue;
-    const int T = m->L[li].d.seq_len, D = m->L[li].d.dim; bool top = T <= AR_MAX_T;
-    if (!top) continue;
+    const int T = m->L[li].d.seq_len, D = m->L[li].d.dim; bool top = true;
     for (int k = li - 1; k >= 0 && m->L[k].d.kind == GN_LAYER_TRANSFORMER_BLOCK && m->L[k].d.dim == D && m->L[k].d.seq_len == T; k--) {
       LayerRT& b = m->L[k];
+      if (!attn_rows_fit(T, D / b.d.heads)) break;
       b.row0_grad = training;
       if (top || !training) b.out_rows = training && T > 1 ? 2 : 1;
       top = false;
@@ -1237,8 +1237,8 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
     LayerRT& l = m->L[li]; const gn_layer_desc& d = l.d;
     const float* xin = l.fin;
     // (a layer below may read the same floats as sequences of another length and width: token 0 is then a different part of them)
-    const bool takes_row0 = (d.kind == GN_LAYER_TRANSFORMER_BLOCK || d.kind == GN_LAYER_POSENC) ? d.seq_len == row0_T && d.dim == row0_D
-                                                                                               : d.kind == GN_LAYER_EMBEDDING && d.seq_len == row0_T && d.out_size == row0_D;
+    const bool takes_row0 = d.kind == GN_LAYER_TRANSFORMER_BLOCK ? l.row0_grad : d.kind == GN_LAYER_POSENC ? d.seq_len == row0_T && d.dim == row0_D
+                                                                                : d.kind == GN_LAYER_EMBEDDING && d.seq_len == row0_T && d.out_size == row0_D;
     if (row0 && !takes_row0) {
       const long n = (long)B * row0_T * row0_D;             // a layer that wants the gradient of every token: zeros except token 0
       GN_LAUNCH(ctx, cls_bwd_kernel, ew_grid(ctx, n), 256, 0, g, pp[flip], row0_T, row0_D, n); g = pp[flip]; flip ^= 1; row0 = false;
