@@ -1138,12 +1138,12 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
   {
     // The walk over scalars (recurrent.cuh) is the default; GONEURON_CUDA_LSTM_SCAN=cluster asks for the kernel below, which
     // applies the updates one by one to the matrix and otherwise runs only for chunks that are too long.
-    static const int mode = [] { const char* e = getenv("GONEURON_CUDA_LSTM_SCAN"); return !e ? 0 : (strcmp(e, "cluster") == 0 ? 1 : (strcmp(e, "gram") == 0 ? 2 : 0)); }();
+    static const bool on_matrix = [] { const char* e = getenv("GONEURON_CUDA_LSTM_SCAN"); return e && strcmp(e, "cluster") == 0; }();
     const int R4g = 4 * H, ZWg = in + H + 1, zs = clip_zs(ZWg), slabs = cdiv(R4g, 8);
     const long Kc = (long)chunk * T, n_updates = (long)GB * T, n_local = (long)B * T, groups = (Kc + CG - 1) / CG, stride = CG_PAD + groups * CG, ng = (long)nchunks * groups, rows = nchunks * stride;
     const bool fits = Kc <= CG_MAX_K && ng <= 65535;
-    if (world > 1 && !(mode != 1 && fits)) return fail(GN_ERR_UNSUPPORTED, "LSTM on more than one GPU needs the scalar form of the clipping recurrence (worker chunk of %ld updates)", Kc);
-    if (mode != 1 && fits) {
+    if (world > 1 && (on_matrix || !fits)) return fail(GN_ERR_UNSUPPORTED, "LSTM on more than one GPU needs the scalar form of the clipping recurrence (worker chunk of %ld updates)", Kc);
+    if (!on_matrix && fits) {
       float *G0, *G1, *Dm, *Zm, *dbl, *gmat;
       const size_t n_om = (size_t)ng * CG, n_p = (size_t)nchunks * 2 * CG * slabs;
       GN_TRY(ensure(m, S_GRAM0, (size_t)ng * CG * 2 * CG, &G0)); GN_TRY(ensure(m, S_GRAM1, (size_t)ng * CG * 2 * CG, &G1));

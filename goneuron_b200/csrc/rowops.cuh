@@ -721,17 +721,7 @@ __global__ void attn_ds_kernel(const float* __restrict__ P, float* __restrict__ 
   s = warp_sum(s);
   for (int j = lane; j < T; j += 32) d[j] = j < lim ? p[j] * (d[j] - s) * inv_scale : 0.f;
 }
-// dZ1[s,t,c] = dM[s,t,c] * 1[M[s,T-1,c] > 0]: inside a TransformerBlock every token's ff1.Backward uses
-// the pre-activation of the LAST token (layer.go:563-567 via transformer.go:1238-1250).
-__global__ void relu_mask_last_token_kernel(float* __restrict__ dM, const float* __restrict__ M, int T, int C, long total) {
-  long per = (long)T * C;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    long s = i / per; int c = (int)(i % C);
-    if (!(M[s * per + (long)(T - 1) * C + c] > 0.f)) dM[i] = 0.f;
-  }
-}
 
-// ---------------------------------------------------------------- misc elementwise
 // ---------------------------------------------------------------- TransformerBlock variants
 // Rotary embeddings on a [tokens, D] tensor in place (transformer.go:212-236): within every head, element i of the first
 // half and element i + hd/2 are rotated by the angle of (position, i); `tab` holds cos | sin per (position, i), computed on
@@ -894,13 +884,6 @@ __global__ void add_token_reversed_kernel(const float* __restrict__ a, const flo
     const long row = e / C; const int c = (int)(e - row * C); const long s = row / T; const int t = (int)(row - s * T);
     out[e] = a[e] + b[(s * T + (T - 1 - t)) * C + c];
   }
-}
-
-__global__ void add3_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c, float* __restrict__ out, long n) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) out[i] = a[i] + b[i] + (c ? c[i] : 0.f);
-}
-__global__ void scale_kernel(float* __restrict__ x, long n, float s) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) x[i] *= s;
 }
 
 // ---------------------------------------------------------------- Adam

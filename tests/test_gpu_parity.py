@@ -296,11 +296,12 @@ def test_direct_convolution_path_in_subprocess():
     assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
 
 
-@pytest.mark.parametrize("mode", ["gram", "cluster"])
+@pytest.mark.parametrize("mode", ["scalars", "cluster"])
 def test_lstm_scan_variants_in_subprocess(mode):
-    """The LSTM gradient-clipping recurrence has two implementations: a thread-block-cluster kernel that applies
-    the updates one by one, and the Gram-matrix form used when a worker chunk has many updates.  The switch
-    GONEURON_CUDA_LSTM_SCAN forces one of them for every size; both must give the same parity."""
+    """The LSTM gradient-clipping recurrence has two implementations: the walk over scalars, which is the default, and a
+    thread-block-cluster kernel that applies the updates to the matrix one by one, for worker chunks of more than 2^20 updates.
+    GONEURON_CUDA_LSTM_SCAN=cluster asks for the second at every size (any other value changes nothing); both must give the
+    same parity."""
     import os
     import subprocess
     import sys
