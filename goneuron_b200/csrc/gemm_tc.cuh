@@ -201,11 +201,11 @@ struct TcParams {
 };
 
 // Epilogue of one output tile.  8 or 16 warps share it: a warp may only read the TMEM lanes of its quadrant (warp % 4), so
-// two or four warps serve each quadrant and take a part of the tile's columns each (`cg`); one output row per thread (TMEM lane
-// = row), 32 consecutive columns per tcgen05.ld, written as 8 float4.  The per-column factors (inverse scale of B's
-// rows, bias) of the warp's columns are staged in shared memory by tc_epilogue_stage BEFORE the warp waits for the
-// accumulator, so that their latency is hidden behind the MMAs; residual and gate values of a chunk are fetched before
-// the TMEM wait for the same reason.  (With four warps and the factors fetched per chunk the epilogue of a tile took as
+// two or four warps serve each quadrant and take a part of the tile's columns each (`cg`); tcgen05.ld gives a thread 32 consecutive
+// columns of one output row (TMEM lane = row).  What becomes of them depends on the rows' alignment, see tc_epilogue_tile.  The
+// per-column factors (inverse scale of B's rows, bias) of the warp's columns are staged in shared memory by tc_epilogue_stage
+// BEFORE the warp waits for the accumulator, so that their latency is hidden behind the MMAs; residual values of a chunk are fetched
+// before the TMEM load for the same reason.  (With four warps and the factors fetched per chunk the epilogue of a tile took as
 // long as its MMAs at K = 1024 and held the tensor pipe back.)  `acc_main` / `acc_cross` are the TMEM column offsets of
 // the two accumulators of this tile (MERGED: there is only acc_main); `bw` is the tile's width (BN, or BN / 2 for a half tile).
 template <int BN, bool PL>
@@ -224,12 +224,16 @@ __device__ __forceinline__ void tc_epilogue_stage(const TcParams& ep, int n0, in
     }
     __syncwarp();
 }
-// `stg`: this warp's staging buffer of 16 rows x TC_STG_LD floats.  The TMEM load gives every thread ITS row (lane = row), and a
-// store of that shape touches 32 different 128-byte lines per instruction.  So the accumulators of 32 columns go through
-// shared memory, 16 rows at a time, and come back with eight neighbouring lanes on one row: every store, residual and gate
-// access is four whole 128-byte lines.  The loops over chunks and row halves are not unrolled: a launch with one tile per CTA runs
-// this code once, from a cold instruction cache, and there the previous, fully unrolled version (with all variants in one body)
-// took 12 000 cycles for a 128 x 128 tile against 6 000 for the tiles after it -- as much as the MMAs of a contraction over 512.
+// Four ways to write a chunk of 32 columns:
+//   planes (PL)          a thread keeps its row: 32 columns are one block of the planes, stored a 32-byte sector at a time
+//   fp32, 32-byte rows   a thread keeps its row and reads and writes whole sectors of it (TC_FLAG_WIDE)
+//   fp32, 16-byte rows   through `stg`, the warp's staging buffer of TcCfg::RS rows x TC_STG_LD floats, RS rows at a time, and back with
+//                        eight neighbouring lanes on one row: every store, residual and gate access is four whole 128-byte lines, where
+//                        16-byte accesses with a row per thread would touch 32 lines per instruction (TC_FLAG_VEC)
+//   anything else        element by element (NCHW output, unaligned rows)
+// The loops over chunks and rows are not unrolled: a launch with one tile per CTA runs this code once, from a cold instruction
+// cache, and there the previous, fully unrolled version (with all variants in one body) took 12 000 cycles for a 128 x 128 tile
+// against 6 000 for the tiles after it -- as much as the MMAs of a contraction over 512.
 constexpr int TC_STG_LD = 36;
 // acc[j] of column c * 32 + j for this lane's row, times the row's inverse scale
 template <bool MERGED>

@@ -71,7 +71,8 @@ def test_blocks_on_the_tensor_cores(device, oracle, T, dim, heads, ff, kw):
 @pytest.mark.parametrize("M,N,K", [(64, 352, 6000), (16, 100, 65600), (130, 65, 12000), (100, 1030, 1056)])
 def test_contraction_in_slices(device, M, N, K):
     """Few output tiles and a long contraction: slices of 256 indices and up, a ragged last one, outputs with and without
-    16-byte rows.  Bound: 2^-21 of sum |a b| for the operands' 22 bits and the accumulator's truncation per 16 indices, against the sum's own size."""
+    16-byte rows.  Bound: 2^-19 of sum |a b|: 2^-21 for the operands' 22 bits (three dropped terms of 2^-22 each), and as much again three times for the
+    accumulator, which truncates once per 16 indices and term, and the partial sums in fp32."""
     from goneuron_b200 import _lib
     rng = np.random.default_rng(K)
     a, b, bias = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32), rng.standard_normal(N).astype(np.float32)
