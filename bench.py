@@ -195,11 +195,11 @@ def measure_tf32_peak(seconds=1.5):
 
 
 # DRAM traffic of the contraction kernel from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum of one
-# gemm_tc_persist_kernel<256> launch, M = 16384 tokens, N = K = 1024, on the 32-sequence case; see the summary of that
+# gemm_tc_persist_kernel<256> launch, M = 16384 tokens, N = K = 1024, through gn_op_gemm_nt; see the summary of that
 # capture under profiles/): measured bytes over the launch's algorithmic bytes.  Traffic grows in proportion with the
 # operand and output sizes, so a full step's figure is this ratio times the step's algorithmic bytes.
 # (Below 1: most of the 67 MB output is still in the 126 MB L2 when the launch ends and is written back later.)
-NCU_TRAFFIC_RATIO = {"captured_bytes": 71.455744e6 + 24.339968e6, "algorithmic_bytes": 4.0 * (16384 + 1024) * 1024 + 4.0 * 16384 * 1024}
+NCU_TRAFFIC_RATIO = {"captured_bytes": 71.4624e6 + 23.107328e6, "algorithmic_bytes": 4.0 * (16384 + 1024) * 1024 + 4.0 * 16384 * 1024}
 
 
 def run_workload(torch, dist, dev, workload, rank, world, local, steps, warmup, e2e=True, sampler=None):
@@ -347,7 +347,7 @@ def main():
     roofline = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops_sustained"], "unit": "TFLOP/s",
                 "frac": achieved / pk["bf16_tflops_sustained"],
                 "traffic": ratio * pf["gemm_bytes"] if ratio else None,
-                "traffic_note": "DRAM bytes of the step's contraction launches: ncu-measured bytes / algorithmic bytes of one captured launch (32-sequence case) times the step's algorithmic bytes",
+                "traffic_note": "DRAM bytes of the step's contraction launches: ncu-measured bytes / algorithmic bytes of one captured launch (16 384 x 1024 over 1024) times the step's algorithmic bytes",
                 "algorithmic_bytes_per_step": pf["gemm_bytes"],
                 "kernel": "contraction kernel launches of the step (gemm_tc_persist_kernel: three fp16 tcgen05 MMAs per fp32 product on row-scaled split planes; small shapes on the fp32 SIMT kernel), CUDA events around each launch",
                 "flops_per_step": pf["gemm_flops"], "launches_per_step": pf["gemm_launches"], "ms_per_step": pf["gemm_ms"], "allreduce_ms_per_step": pf["allreduce_ms"],
