@@ -12,10 +12,10 @@ namespace gn {
 
 // dst[ch * plane + r * ld + x] = src[ch][ylo + r][xlo + x], x < ld (a multiple of four), of `nch` channels with `rows` rows each; zero
 // outside the image and from channel `have` on.  All copies of a thread are in flight at once (one after the other, a load and
-// a store at a time, they were 60 us of the weight gradient); whole 16-byte pieces where the rows
-// and the pointer (a first layer reads the caller's batch) allow it.
-__device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const float* __restrict__ src, int nch, int have, int rows, int ylo, int H, int W, int xlo) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5; const bool v4 = xlo == 0 && ld == W && (reinterpret_cast<uintptr_t>(src) & 15) == 0;      // W a multiple of four
+// a store at a time, they were 60 us of the weight gradient); whole 16-byte pieces where the rows allow it and the
+// pointer does (`aligned`: decided by the host; a first layer reads the caller's batch).
+__device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const float* __restrict__ src, int nch, int have, int rows, int ylo, int H, int W, int xlo, bool aligned) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5; const bool v4 = aligned && xlo == 0 && ld == W;      // W a multiple of four
   const int n = v4 ? ld >> 2 : ld, lw = n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32, step = nw * (32 / lw), lx = lane & (lw - 1);
   int q = warp * (32 / lw) + lane / lw, ch = q / rows, r = q - ch * rows;
   for (; ch < nch;) {
@@ -32,7 +32,7 @@ __device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const 
 // A thread owns 4 neighbouring pixels x OC = 8 (or 4) channels; a block a band of `rb` rows of one image and `og` groups of OC
 // channels, with the source rows and the weights of `icc` source channels at a time in shared memory: 2 + 2 K 16-byte shared
 // loads per 32 K multiply-adds.
-struct ConvTile { int Cs, Cd, sH, sW, dH, dW, p, rb, og, icc, qw, swp; };
+struct ConvTile { int Cs, Cd, sH, sW, dH, dW, p, rb, og, icc, qw, swp, aligned; };
 template <int K, int OC, bool BWD>
 __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict__ src, const float* __restrict__ W, const float* __restrict__ bias,
                                                         float* __restrict__ z, float* __restrict__ out, const ConvTile c, int act, float alpha) {
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict_
   for (int s0 = 0; s0 < c.Cs; s0 += c.icc) {
     const int ns = min(c.icc, c.Cs - s0);
     if (s0 > 0) __syncthreads();
-    conv_stage(xs, rows * c.swp, c.swp, sb + (long)s0 * c.sH * c.sW, ns, ns, rows, y0 - c.p, c.sH, c.sW, -c.p);
+    conv_stage(xs, rows * c.swp, c.swp, sb + (long)s0 * c.sH * c.sW, ns, ns, rows, y0 - c.p, c.sH, c.sW, -c.p, c.aligned);
     for (int e = tid; e < ocb * ns * K * K; e += blockDim.x) {
       const int o = e % ocb, r = e / ocb, t = r % (K * K), s = r / (K * K);      // neighbouring threads, neighbouring words of shared memory
       const bool in = d0 + o < c.Cd;
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict_
 // multiply-adds.  A block takes the bands of several images in turn (unit = image, band) and leaves one set of partial sums;
 // conv_wgrad_final_kernel adds the blocks' sets in order.  Channel planes in shared memory lie 4 (mod 8) floats apart, so that
 // the lanes of a warp (neighbouring channels) hit different banks.
-struct ConvWg { int Cs, Cd, H, W, oH, oW, p, rb, bands, ocb, icb, pg, swp, gwp, xplane, gplane, units; };
+struct ConvWg { int Cs, Cd, H, W, oH, oW, p, rb, bands, ocb, icb, pg, swp, gwp, xplane, gplane, units, aligned; };
 template <int K> struct ConvWgOT { static constexpr int v = K == 1 ? 8 : K == 3 ? 4 : 2; };
 template <int K>
 __global__ void __launch_bounds__(256) conv_wgrad_tile_kernel(const float* __restrict__ g, const float* __restrict__ src, float* __restrict__ part, const ConvWg c) {
@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(256) conv_wgrad_tile_kernel(const float* __res
   for (int u = blockIdx.x; u < c.units; u += gridDim.x) {
     const int b = u / c.bands, y0 = (u - b * c.bands) * c.rb, nr = min(c.rb, c.oH - y0);
     __syncthreads();
-    conv_stage(xs, c.xplane, c.swp, src + ((long)b * c.Cs + i0) * c.H * c.W, c.icb, c.Cs - i0, rows, y0 - c.p, c.H, c.W, -c.p);
-    conv_stage(gs, c.gplane, c.gwp, g + ((long)b * c.Cd + o0) * c.oH * c.oW, c.ocb, c.Cd - o0, c.rb, y0, c.oH, c.oW, 0);
+    conv_stage(xs, c.xplane, c.swp, src + ((long)b * c.Cs + i0) * c.H * c.W, c.icb, c.Cs - i0, rows, y0 - c.p, c.H, c.W, -c.p, c.aligned);
+    conv_stage(gs, c.gplane, c.gwp, g + ((long)b * c.Cd + o0) * c.oH * c.oW, c.ocb, c.Cd - o0, c.rb, y0, c.oH, c.oW, 0, true);
     cp_async_wait();
     __syncthreads();
     if (live) for (int r = pg; r < nr; r += c.pg) {
@@ -203,6 +203,7 @@ inline bool conv_direct_preferred(const ConvShape& c) { return conv_direct_suppo
 
 template <int K, int OC, bool BWD>
 inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
+  c.aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
   c.qw = cdiv(c.dW, 4); c.swp = 4 * c.qw + (K > 1 ? 4 : 0);
   const int groups = cdiv(c.Cd, OC);
   c.og = std::min(groups, std::max(1, std::min(32 / OC, 256 / c.qw)));
@@ -266,7 +267,7 @@ inline size_t conv_wgrad_part_floats(Ctx* ctx, const ConvShape& s) {
 template <int K>
 inline int conv_wgrad_launch(Ctx* ctx, const ConvShape& s, const float* g, const float* x, float* part, float* gW) {
   constexpr int OT = ConvWgOT<K>::v; int sets; size_t smem;
-  const ConvWg c = conv_wgrad_plan(ctx, s, OT, &sets, &smem);
+  ConvWg c = conv_wgrad_plan(ctx, s, OT, &sets, &smem); c.aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   const int items = c.ocb / OT * c.icb, threads = (items * c.pg + 31) & ~31, n = s.outC * s.inC * K * K + s.outC;
   GN_CUDA(cudaFuncSetAttribute(conv_wgrad_tile_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GN_LAUNCH(ctx, conv_wgrad_tile_kernel<K>, dim3(sets, cdiv(s.inC, c.icb) * cdiv(s.outC, c.ocb)), threads, smem, g, x, part, c);
