@@ -7,7 +7,6 @@
 #include <cstdarg>
 #include <cstdlib>
 #include <initializer_list>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -209,52 +208,54 @@ struct ProfScope {
   ~ProfScope() { if (e1) cudaEventRecord(e1, c->stream); }
 };
 
-// Device memory of the library's buffers.  The driver takes 0.1 to 1 ms per cudaMalloc and cudaFree, and more for large blocks; a
-// Transformer model has some hundred buffers.  So blocks that are released while a model lives on their GPU are kept for the next buffer of
-// their size, up to keep_limit() bytes; everything beyond goes back to the driver at once, all of it does when the GPU's last model
-// or context is closed, and whenever the driver has no memory left.  (A cudaMemPool_t in this place maps
-// fresh memory in other portions: creating a six-block encoder of width 512 in a process that has one already took 4.4 to 14 ms instead
-// of 2.3, its first pass 2.6 instead of 6.  With kept blocks both take 0.2 and 1.2 ms; with cudaMalloc and cudaFree alone 2.5 and 24,
-// and 20 to close.)
-// A block is handed on only after every stream of the library on its GPU has finished what it held at the release: cudaFree
-// waits for the device in the same way.  Not cudaDeviceSynchronize: that fails while any other thread has a stream in capture.
-struct DeviceBlocks {
+// Device memory of the library's buffers comes from one CUDA memory pool per GPU.  While a model lives there the pool keeps up to
+// keep_limit() bytes of what models and scratch buffers have released (a model of the same size created later gets it back without
+// going to the driver: Compile and first pass of a causal Transformer of width 256 take 0.2 and 1.4 ms instead of 1.9 and 9 with
+// cudaMalloc); the rest, and everything once the GPU's last model or context is closed, goes back to the driver.
+// (A list of cudaMalloc blocks by size, and parts of 128 MiB blocks, were as quick to prepare, but steps ran 0.4 to 1.4 % slower in them.)
+// An allocation is usable on every stream when take() returns.  put() hands memory on only after every stream of the library on the GPU
+// has finished what it held, as cudaFree waits for the device.  Not cudaDeviceSynchronize: that fails while any other thread has
+// a stream in capture.  The pool's own stream orders its allocations and releases; nothing else runs there.
+struct DeviceMemory {
   static constexpr int MAX = 64;
-  struct Gpu { std::mutex mu; std::multimap<size_t, void*> kept; size_t kept_bytes = 0; int models = 0, contexts = 0; std::vector<cudaStream_t> streams; };
+  struct Gpu { std::mutex mu; cudaMemPool_t pool = nullptr; cudaStream_t stream = nullptr; int models = 0, contexts = 0; std::vector<cudaStream_t> streams; };
   Gpu gpu[MAX];
-  static DeviceBlocks& get() { static DeviceBlocks* p = new DeviceBlocks(); return *p; }      // (lives until the process ends)
-  static size_t keep_limit() {
-    static const size_t n = [] { const char* e = getenv("GONEURON_CUDA_KEEP_BYTES"); return e ? (size_t)strtoull(e, nullptr, 10) : (size_t)8 << 30; }();
+  static DeviceMemory& get() { static DeviceMemory* p = new DeviceMemory(); return *p; }      // (lives until the process ends)
+  static unsigned long long keep_limit() {
+    static const unsigned long long n = [] { const char* e = getenv("GONEURON_CUDA_KEEP_BYTES"); return e ? strtoull(e, nullptr, 10) : 8ull << 30; }();
     return n;
   }
-  // the driver's granularity: 512 bytes, 2 MiB for blocks of their own
-  static size_t rounded(size_t bytes) { const size_t g = bytes > ((size_t)1 << 20) ? (size_t)2 << 20 : 512; return (bytes + g - 1) / g * g; }
   // The functions below want `dev` to be the current device.
-  static void give_back(Gpu& g) { for (auto& b : g.kept) cudaFree(b.second); g.kept.clear(); g.kept_bytes = 0; }
-  cudaError_t take(int dev, size_t* bytes, void** p) {      // *bytes: wanted on entry, the block's on return
-    *bytes = rounded(*bytes);
-    if (dev < 0 || dev >= MAX) return cudaMalloc(p, *bytes);
-    Gpu& g = gpu[dev]; std::lock_guard<std::mutex> lk(g.mu);
-    auto it = g.kept.lower_bound(*bytes);
-    if (it != g.kept.end() && it->first <= *bytes + *bytes / 8) { *bytes = it->first; *p = it->second; g.kept_bytes -= it->first; g.kept.erase(it); return cudaSuccess; }
-    cudaError_t e = cudaMalloc(p, *bytes);
-    if (e == cudaErrorMemoryAllocation && !g.kept.empty()) { cudaGetLastError(); give_back(g); e = cudaMalloc(p, *bytes); }
-    return e;
+  static void set_keep(Gpu& g) { unsigned long long n = g.models > 0 && g.contexts > 0 ? keep_limit() : 0; cudaMemPoolSetAttribute(g.pool, cudaMemPoolAttrReleaseThreshold, &n); }
+  static void trim(Gpu& g) { if (g.pool) { cudaStreamSynchronize(g.stream); cudaMemPoolTrimTo(g.pool, 0); } }
+  static cudaError_t open(Gpu& g, int dev) {
+    if (g.pool) return cudaSuccess;
+    cudaMemPoolProps pr{}; pr.allocType = cudaMemAllocationTypePinned; pr.location.type = cudaMemLocationTypeDevice; pr.location.id = dev;
+    cudaError_t e = g.stream ? cudaSuccess : cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemPoolCreate(&g.pool, &pr);
+    if (e != cudaSuccess) { g.pool = nullptr; return e; }
+    set_keep(g); return cudaSuccess;
   }
-  void put(int dev, size_t bytes, void* p, bool idle) {      // idle: the caller has waited for everything that uses the block
-    if (dev >= 0 && dev < MAX) {
-      Gpu& g = gpu[dev]; std::lock_guard<std::mutex> lk(g.mu);
-      bool keep = g.models > 0 && g.kept_bytes + bytes <= keep_limit();
-      if (keep && !idle) for (auto s : g.streams) keep = keep && cudaStreamSynchronize(s) == cudaSuccess;
-      if (keep) { g.kept.emplace(bytes, p); g.kept_bytes += bytes; return; }
-    }
-    cudaFree(p);
+  cudaError_t take(int dev, size_t bytes, void** p) {
+    if (dev < 0 || dev >= MAX) return cudaErrorInvalidDevice;
+    Gpu& g = gpu[dev]; std::lock_guard<std::mutex> lk(g.mu);
+    cudaError_t e = open(g, dev);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes, g.pool, g.stream);
+    if (e == cudaErrorMemoryAllocation && g.pool) { cudaGetLastError(); trim(g); e = cudaMallocFromPoolAsync(p, bytes, g.pool, g.stream); }
+    return e != cudaSuccess ? e : cudaStreamSynchronize(g.stream);
+  }
+  void put(int dev, void* p, bool idle) {                    // idle: the caller has waited for everything that uses the memory
+    Gpu& g = gpu[dev]; std::lock_guard<std::mutex> lk(g.mu);
+    if (!idle) for (auto s : g.streams) if (cudaStreamSynchronize(s) != cudaSuccess) return;      // (a broken context: nobody gets this memory any more)
+    cudaFreeAsync(p, g.stream);
+    if (g.models <= 0) cudaStreamSynchronize(g.stream);      // (where the pool gives back what it need not keep)
   }
   void count(int dev, int d_models, int d_contexts) {
     if (dev < 0 || dev >= MAX) return;
     Gpu& g = gpu[dev]; std::lock_guard<std::mutex> lk(g.mu);
     g.models += d_models; g.contexts += d_contexts;
-    if (g.models <= 0 || g.contexts <= 0) give_back(g);
+    if (g.pool) set_keep(g);
+    if (g.models <= 0 || g.contexts <= 0) trim(g);
   }
   void streams(int dev, std::initializer_list<cudaStream_t> list, bool there) {
     if (dev < 0 || dev >= MAX) return;
@@ -267,17 +268,17 @@ struct DeviceBlocks {
 
 // Owning device buffer, or a view of part of another one.
 struct DevBuf {
-  float* p = nullptr; size_t n = 0, bytes = 0; bool owner = true; int dev = 0;
+  float* p = nullptr; size_t n = 0; bool owner = true; int dev = 0;
   DevBuf() {}
   DevBuf(const DevBuf&) = delete; DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), bytes(o.bytes), owner(o.owner), dev(o.dev) { o.p = nullptr; o.n = 0; }
-  DevBuf& operator=(DevBuf&& o) noexcept { release(); p = o.p; n = o.n; bytes = o.bytes; owner = o.owner; dev = o.dev; o.p = nullptr; o.n = 0; return *this; }
+  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), owner(o.owner), dev(o.dev) { o.p = nullptr; o.n = 0; }
+  DevBuf& operator=(DevBuf&& o) noexcept { release(); p = o.p; n = o.n; owner = o.owner; dev = o.dev; o.p = nullptr; o.n = 0; return *this; }
   ~DevBuf() { release(); }
   void release() {
     if (p && owner) {
       int cur = dev; cudaGetDevice(&cur);
       if (cur != dev) cudaSetDevice(dev);
-      DeviceBlocks::get().put(dev, bytes, p, DeviceBlocks::Idle::depth() > 0);
+      DeviceMemory::get().put(dev, p, DeviceMemory::Idle::depth() > 0);
       if (cur != dev) cudaSetDevice(cur);
     }
     p = nullptr; n = 0; owner = true;
@@ -285,8 +286,8 @@ struct DevBuf {
   void view(float* q, size_t count) { release(); p = q; n = count; owner = false; }
   int alloc(size_t count) {
     release(); if (count == 0) return GN_OK;
-    cudaGetDevice(&dev); bytes = count * sizeof(float);
-    const cudaError_t e = DeviceBlocks::get().take(dev, &bytes, (void**)&p);
+    cudaGetDevice(&dev);
+    const cudaError_t e = DeviceMemory::get().take(dev, count * sizeof(float), (void**)&p);
     if (e != cudaSuccess) { cudaGetLastError(); p = nullptr; return fail(GN_ERR_OOM, "device allocation of %zu bytes failed: %s", count * sizeof(float), cudaGetErrorString(e)); }
     n = count; return GN_OK;
   }

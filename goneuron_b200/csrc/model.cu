@@ -324,7 +324,7 @@ static bool block_shares(const gn_model* m, const LayerRT& l, bool training) {
 // (Re)allocates every per-layer activation buffer for `cap` samples.
 static int alloc_activations(gn_model* m, int cap, bool training) {
   GN_CUDA(cudaStreamSynchronize(m->ctx->c.stream));
-  DeviceBlocks::Idle waited;                  // (between steps the context's other streams have been joined to this one)
+  DeviceMemory::Idle waited;                  // (between steps the context's other streams have been joined to this one)
   size_t c = (size_t)cap;
   plan_token_rows(m, training);
   m->epoch++;
@@ -1686,8 +1686,8 @@ static int make_ctx(int device, int rank, int world, const unsigned char* id, gn
     GN_CUDA(cudaStreamCreateWithFlags(&c->c.comm_stream, cudaStreamNonBlocking));
   }
   guard.c = nullptr;
-  DeviceBlocks::get().count(device, 0, 1);
-  DeviceBlocks::get().streams(device, {c->c.stream, c->c.side_stream, c->c.copy_stream, c->c.comm_stream}, true);
+  DeviceMemory::get().count(device, 0, 1);
+  DeviceMemory::get().streams(device, {c->c.stream, c->c.side_stream, c->c.copy_stream, c->c.comm_stream}, true);
   *out = c; return GN_OK;
 }
 
@@ -1729,7 +1729,7 @@ int gn_shutdown(gn_ctx* ctx) {
   for (auto& e : ctx->c.ev_pool) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
   ctx->c.ev_pool.clear();
   ctx->c.release_owned();                               // operand-plane scratch of the contraction and attention engines
-  DeviceBlocks::get().streams(ctx->c.device, {ctx->c.stream, ctx->c.side_stream, ctx->c.copy_stream, ctx->c.comm_stream}, false);
+  DeviceMemory::get().streams(ctx->c.device, {ctx->c.stream, ctx->c.side_stream, ctx->c.copy_stream, ctx->c.comm_stream}, false);
   if (ctx->c.d_status) cudaFree(ctx->c.d_status);
   if (ctx->c.h_block) { cudaFreeHost(ctx->c.h_block); ctx->c.h_block = nullptr; }
   if (ctx->c.tc_queue_pool) { cudaFree(ctx->c.tc_queue_pool); ctx->c.tc_queue_pool = nullptr; }
@@ -1743,7 +1743,7 @@ int gn_shutdown(gn_ctx* ctx) {
   if (ctx->c.comm_stream) cudaStreamDestroy(ctx->c.comm_stream);
   ctx->c.comm_stream = nullptr;
   ctx->c.comm = nullptr; ctx->c.d_status = nullptr; ctx->c.stream = nullptr; ctx->alive = false;
-  DeviceBlocks::get().count(ctx->c.device, 0, -1);
+  DeviceMemory::get().count(ctx->c.device, 0, -1);
   return GN_OK;   // the handle itself stays allocated so that a second call is harmless
 }
 
@@ -1831,7 +1831,7 @@ int gn_model_create(gn_ctx* ctx, const gn_layer_desc* layers, int n_layers, int 
   m->layer_ev.resize(m->L.size() + 1);
   for (auto& e : m->layer_ev) GN_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   m->scratch.resize(S_COUNT);
-  DeviceBlocks::get().count(ctx->c.device, 1, 0);
+  DeviceMemory::get().count(ctx->c.device, 1, 0);
   *out = m.release(); return GN_OK;
 }
 
@@ -1842,14 +1842,14 @@ int gn_model_destroy(gn_model* m) {
   bool idle = true;
   if (m->ctx->alive) for (auto s : {m->ctx->c.stream, m->ctx->c.side_stream, m->ctx->c.copy_stream, m->ctx->c.comm_stream}) if (s) idle = cudaStreamSynchronize(s) == cudaSuccess && idle;
   if (m->ctx->c.weight_planes == &m->wplanes) m->ctx->c.weight_planes = nullptr;
-  DeviceBlocks::get().count(m->ctx->c.device, -1, 0);
-  std::unique_ptr<DeviceBlocks::Idle> waited(idle ? new DeviceBlocks::Idle() : nullptr);
+  std::unique_ptr<DeviceMemory::Idle> waited(idle ? new DeviceMemory::Idle() : nullptr);
   m->wplanes = gn::WeightPlaneTable();
   m->drop_graphs();
   m->L.clear(); m->scratch.clear(); for (auto& b : m->shared) b.release(); m->state.release(); m->params.release(); m->grads.release(); m->m1.release(); m->v2.release();
   m->io.release(); m->lossg.release(); m->loss_s.release(); m->loss_sum.release();
   if (m->ev0) cudaEventDestroy(m->ev0); if (m->ev1) cudaEventDestroy(m->ev1); if (m->ar0) cudaEventDestroy(m->ar0); if (m->ar1) cudaEventDestroy(m->ar1);
   if (m->comm_done) cudaEventDestroy(m->comm_done); if (m->gather_ev) cudaEventDestroy(m->gather_ev); m->gather_ev = nullptr; for (auto e : m->layer_ev) cudaEventDestroy(e); m->layer_ev.clear();
+  DeviceMemory::get().count(m->ctx->c.device, -1, 0);
   m->ev0 = m->ev1 = m->ar0 = m->ar1 = m->comm_done = nullptr; m->alive = false; return GN_OK;
 }
 
