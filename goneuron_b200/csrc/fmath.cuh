@@ -81,8 +81,8 @@ __host__ __device__ __forceinline__ float tanh_rn(float x) {
 //   y > 1: x - x / (m + 2),   |y| <= 1: x / 2 + x (m / 2) / (m + 2),   y < -1: x (m + 1) / (m + 2)
 // so that what the quotient's two ulp apply to is at most a quarter of x.  Against float64 over all x the error is below 9.5e-8 |x|,
 // root mean square 2.4e-8 |x|; the reference's own order, float32 around a rounded tanh, has 1.20e-7 and 3.3e-8 (it adds 1 to the tanh).
-// With the hardware's exponential and quotient it was 1.8e-7 and 4.7e-8, at the same speed (a training step of 24 sequences of 150 tokens,
-// width 384: 1296 us; 1387 with the tanh above).
+// With the hardware's exponential and quotient it was 1.8e-7 and 4.7e-8 for some twenty instructions less (a training step of 24
+// sequences of 150 tokens, width 384: 1297 us, now 1312; 1387 with the tanh above).
 __device__ __forceinline__ float gelu_f(float x) {
   const float y = fminf(fmaxf(x * fmaf(0.07135481627f * x, x, 1.5957691216057308f), -80.f), 80.f);      // (a NaN becomes -80)
   const float t = fmaf(y, 1.44269504088896341f, 12582912.f), n = t - 12582912.f;       // 1.5 2^23: rounds to a whole number, low bits of t
