@@ -1148,7 +1148,7 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
       const size_t n_om = (size_t)ng * CG, n_p = (size_t)nchunks * 2 * CG * slabs;
       GN_TRY(ensure(m, S_GRAM0, (size_t)ng * CG * 2 * CG, &G0)); GN_TRY(ensure(m, S_GRAM1, (size_t)ng * CG * 2 * CG, &G1));
       GN_TRY(ensure(m, S_DM, (size_t)rows * R4g, &Dm)); GN_TRY(ensure(m, S_ZM, (size_t)rows * zs, &Zm));
-      GN_TRY(ensure(m, S_TV, 2 * (n_om + n_p + (size_t)ng * 2), &dbl)); GN_TRY(ensure(m, S_SCAN, (size_t)nchunks * 2 * R4g * ZWg, &gmat));
+      GN_TRY(ensure(m, S_TV, 2 * (n_om + n_p + (size_t)ng * 2) + nchunks, &dbl)); GN_TRY(ensure(m, S_SCAN, (size_t)nchunks * 2 * R4g * ZWg, &gmat));
       // rows of zeros: the group before every chunk's first, and what its last group lacks
       if (nchunks > 8) { GN_CUDA(stream_zero(ctx, Dm, (size_t)rows * R4g * 4)); GN_CUDA(stream_zero(ctx, Zm, (size_t)rows * zs * 4)); }
       else for (int c = 0; c < nchunks; c++) {
@@ -1172,7 +1172,9 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
       const long q4 = ng * CG * 2 * CG / 4;
       GN_LAUNCH(ctx, lstm_gram_mul_kernel, ew_grid(ctx, q4), 256, 0, G0, (const float*)G1, q4);
       double* db = reinterpret_cast<double*>(dbl);
-      const ClipArgs a{Dm, Zm, G0, db, db + n_om, db + n_om + n_p, gmat, R4g, ZWg, (int)groups, slabs, stride};
+      int* start = reinterpret_cast<int*>(db + n_om + n_p + (size_t)ng * 2);
+      GN_LAUNCH(ctx, lstm_clip_start_kernel, nchunks, 1024, 0, (const float*)G0, (int)groups, start);
+      const ClipArgs a{Dm, Zm, G0, db, db + n_om, db + n_om + n_p, gmat, start, R4g, ZWg, (int)groups, slabs, stride};
       const size_t smem = clip_smem(ZWg);
       GN_CUDA(cudaFuncSetAttribute(lstm_clip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       for (int j = 0; j <= groups; j++) GN_EARLY_LAUNCH(ctx, lstm_clip_kernel, dim3(1 + slabs, nchunks), CG_THREADS, smem, a, j);

@@ -48,6 +48,51 @@ def test_recurrent_parity(device, oracle, net, I, H, T, batch, W, seq):
     model.Close()
 
 
+@pytest.mark.parametrize("scale,W", [(1e-6, 1), (1e-2, 1), (1.0, 1), (1e4, 1), (1e4, 4), ("early", 1), ("early", 2), ("late", 1)])
+def test_clipping_walk_starts_where_the_result_can_still_see(device, oracle, scale, W):
+    """800 updates in seven groups (four chunks of 200, two of 400): nothing is clipped, some of it is, the last dozens of updates decide the
+    result, or one sample's do -- an early one, whose group has to be walked although later groups only add small
+    updates, or one in the last group."""
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = [D.SequenceUnrollerLSTM(7, 20, 40, False), D.Dense(20, 2, D.LINEAR)]
+    rng = np.random.Generator(np.random.PCG64(5))
+    params = configs.init_params(layers, rng)
+    x, y = configs.make_inputs("lstm", layers, 20, rng)
+    if isinstance(scale, str):
+        y *= 1e-4
+        y[2 if scale == "early" else 19] *= 1e9
+    else:
+        y *= scale
+    ref = oracle.OracleState(layers, D.MSE, params, lr=1e-3)
+    lit = oracle.OracleState(layers, D.MSE, params, lr=1e-3)
+    ref.train_batch(x, y, W=W, threads=4, precision=64)
+    lit.train_batch(x, y, W=W, threads=W, precision=32)
+    model = Sequential(layers, device, virtual_workers=W).Compile(Adam(1e-3), D.MSE)
+    model.SetParams(params)
+    model.TrainBatch(x, y)
+    assert_grads_close(layers, model.Gradients(), ref.grads, floor=lit.grads)
+    model.Close()
+
+
+def test_clipping_keeps_what_is_not_finite(device, oracle):
+    """An infinite target in the first sample: its updates are lost in no way, however large the later ones are."""
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = [D.SequenceUnrollerLSTM(7, 20, 40, False), D.Dense(20, 2, D.LINEAR)]
+    rng = np.random.Generator(np.random.PCG64(6))
+    params = configs.init_params(layers, rng)
+    x, y = configs.make_inputs("lstm", layers, 20, rng)
+    y *= 1e4
+    y[0] = np.inf
+    ref = oracle.OracleState(layers, D.MSE, params, lr=1e-3)
+    ref.train_batch(x, y, threads=4, precision=64)
+    model = Sequential(layers, device).Compile(Adam(1e-3), D.MSE)
+    model.SetParams(params)
+    model.TrainBatch(x, y)
+    n = params.size - 42                                  # the LSTM's parameters
+    assert np.isnan(ref.grads[:n]).all() and np.isnan(model.Gradients()[:n]).all()
+    model.Close()
+
+
 def test_elementwise_functions_are_rounded_once(device):
     """exp and tanh come out within 0.54 ulp of the float64 value (one rounding gives 0.5).  Sigmoid and SiLU add two and three float32
     operations; a relative error of 2^-24 each and 1.08 * 2^-24 from the exponential is at most 3.1 and 4.1 ulp of the result."""
