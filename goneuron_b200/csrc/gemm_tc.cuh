@@ -53,7 +53,6 @@ constexpr unsigned TC_SPIN_LIMIT = 1u << 24;    // default number of polls of on
 constexpr unsigned TC_DRAIN_LIMIT = 1u << 20;   // polls spent waiting for own work in flight after a wait gave up
 constexpr int TC_QUEUE_POOL = 2048;   // tile-queue counters per context before the pool is cleared again
 constexpr int TC_FLAG_SCALE = 8192; // plane output: `mask` holds factors (a GELU layer's derivatives, all below 1.25), not a gate
-constexpr int TC_FLAG_WIDE = 16384; // ... 32-byte accesses to C and R
 constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by the host when every pointer and stride allows it)
 // One stage = 32 contraction indices of both operands.  The two fp16 planes of an operand are interleaved in blocks of 32:
 // element (r, k) of a plane row has its high part at pl_off(k) and its low part PL_LO halves further, so a block of a row is 128
@@ -63,19 +62,15 @@ constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by
 // [8192, 1024] x [1024, 256] from 26.8 to 18.6, [32768, 1024] x [1024, 1024] from 136 to 119 (zeros as data: no power limit).
 constexpr int TC_BK = 32, PL_LO = 32;
 __host__ __device__ __forceinline__ int pl_off(int k) { return ((k >> 5) << 6) | (k & 31); }
-// PL: the variant that writes its result as operand planes.  Its epilogue has twice the work per element (activation or factors, scale,
-// two conversions) and takes 16 warps, four per TMEM lane quadrant; the fp32 epilogue is bound by its stores and runs best with
-// eight.  [18944, 256] over 128 with GELU planes: 28.8 us with eight, 22.7 with 16; as fp32 13.5 and 14.5.
+// PL: the variant that writes its result as operand planes.
 template <int BN, bool PL> struct TcCfg {
-  static constexpr int EW = PL ? 16 : 8, CG = EW / 4, RS = 128 / EW;              // epilogue warps, column groups, rows per pass through a warp's staging buffer
+  static constexpr int EW = PL ? 16 : 8, CG = EW / 4, CC = PL ? 16 : 32;          // epilogue warps, column groups, columns of a chunk
   static constexpr int THREADS = 64 + 32 * EW;                                    // TMA warp, MMA warp, epilogue warps
   static constexpr int A_BYTES = TC_BM * 128, B_BYTES = BN * 128;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (192 * 1024) / STAGE_BYTES > 8 ? 8 : (192 * 1024) / STAGE_BYTES;
-  static constexpr int CW = BN / CG < 32 ? 32 : BN / CG;                    // columns of an epilogue warp
-  static constexpr int COLV_FLOATS = EW * 2 * CW;                       // per epilogue warp: scale and bias of its columns
-  static constexpr int STG_FLOATS = PL ? 0 : EW * RS * 36;                                // per epilogue warp: RS rows x 32 (+4) accumulators in transit
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/ + (COLV_FLOATS + STG_FLOATS) * 4;
+  static constexpr int STG_FLOATS = EW * 32 * CC;                                 // per epilogue warp: 32 rows x CC columns in transit
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/ + STG_FLOATS * 4;
   static constexpr bool MERGED = BN > 128;                                        // one accumulator per slot
   static constexpr int SLOT_COLS = MERGED ? BN : 2 * BN;
   static constexpr int TMEM_COLS = 2 * SLOT_COLS;
@@ -161,6 +156,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 }
 
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+        "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+
 // ------------------------------------------------------------------ splitting a value into operand planes
 // Power of two s that brings a row whose largest magnitude is mx into [2^14, 2^15) (fp16 overflows at 65504), and its
 // inverse.  s = 1 for a row of zeros (and for a row that holds an infinity or a NaN, which the products then carry on).
@@ -201,228 +204,190 @@ struct TcParams {
 };
 
 // Epilogue of one output tile.  8 or 16 warps share it: a warp may only read the TMEM lanes of its quadrant (warp % 4), so
-// two or four warps serve each quadrant and take a part of the tile's columns each (`cg`); tcgen05.ld gives a thread 32 consecutive
-// columns of one output row (TMEM lane = row).  What becomes of them depends on the rows' alignment, see tc_epilogue_tile.  The
-// per-column factors (inverse scale of B's rows, bias) of the warp's columns are staged in shared memory by tc_epilogue_stage
-// BEFORE the warp waits for the accumulator, so that their latency is hidden behind the MMAs; residual values of a chunk are fetched
-// before the TMEM load for the same reason.  (With four warps and the factors fetched per chunk the epilogue of a tile took as
-// long as its MMAs at K = 1024 and held the tensor pipe back.)  `acc_main` / `acc_cross` are the TMEM column offsets of
-// the two accumulators of this tile (MERGED: there is only acc_main); `bw` is the tile's width (BN, or BN / 2 for a half tile).
-template <int BN, bool PL>
-__device__ __forceinline__ void tc_epilogue_stage(const TcParams& ep, int n0, int z, int cg, int lane, int bw, float* colv) {
-    if (!(ep.flags & TC_FLAG_VEC)) return;
-    using Cfg = TcCfg<BN, PL>;
-    const int ncw = max(bw / Cfg::CG, 32), cbase = n0 + cg * ncw;
-    if (cg * ncw >= bw) return;
-    const float* isb = ep.isb + (long)z * ep.N;
-    __syncwarp();
-    for (int i = lane * 4; i < ncw; i += 128) {
-      const int col = cbase + i; const bool in = col < ep.N;
-      const long bo = ep.n_seg ? col + (col / ep.n_seg) * (ep.bias_seg - ep.n_seg) : col;
-      *reinterpret_cast<float4*>(colv + i) = in ? __ldg(reinterpret_cast<const float4*>(isb + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(colv + Cfg::CW + i) = (in && ep.bias) ? __ldg(reinterpret_cast<const float4*>(ep.bias + bo)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncwarp();
-}
-// Four ways to write a chunk of 32 columns:
-//   planes (PL)          a thread keeps its row: 32 columns are one block of the planes, stored a 32-byte sector at a time
-//   fp32, 32-byte rows   a thread keeps its row and reads and writes whole sectors of it (TC_FLAG_WIDE)
-//   fp32, 16-byte rows   through `stg`, the warp's staging buffer of TcCfg::RS rows x TC_STG_LD floats, RS rows at a time, and back with
-//                        eight neighbouring lanes on one row: every store, residual and gate access is four whole 128-byte lines, where
-//                        16-byte accesses with a row per thread would touch 32 lines per instruction (TC_FLAG_VEC)
-//   anything else        element by element (NCHW output, unaligned rows)
-// The loops over chunks and rows are not unrolled: a launch with one tile per CTA runs this code once, from a cold instruction
-// cache, and there the previous, fully unrolled version (with all variants in one body) took 12 000 cycles for a 128 x 128 tile
-// against 6 000 for the tiles after it -- as much as the MMAs of a contraction over 512.
-constexpr int TC_STG_LD = 36;
-// acc[j] of column c * 32 + j for this lane's row, times the row's inverse scale
-template <bool MERGED>
-__device__ __forceinline__ void tc_acc_chunk(uint32_t taddr, uint32_t acc_main, uint32_t acc_cross, bool any, float isa, float (&v)[32]) {
+// two or four warps serve each quadrant and take a part of the tile's columns each (`cg`), in chunks of TcCfg::CC.  tcgen05.ld gives a
+// thread consecutive columns of one output row (TMEM lane = row); the chunk goes through `stg`, the warp's staging buffer of 32 rows
+// (16-byte units swizzled by the row: no bank conflicts either way), and comes back with eight (planes: four) neighbouring lanes on
+// a row and four columns of eight (four) rows per lane.  From there on an access to global memory touches four lines of 128 bytes (eight half
+// lines).  What a chunk reads -- column factors, residual, gate -- is fetched while the one before it is stored, the first chunk's
+// before the accumulator is waited for.
+// (A thread that kept the row TMEM gave it and moved whole 32-byte sectors of it touched 32 lines per instruction: 1700 cycles to
+// store a chunk, 13 bytes per clock and SM; 9000 cycles for a 128 x 128 tile with a residual, as much as its MMAs over 384.  Now
+// about 4500.  [3072, 512] over 512 with a residual 13.7 -> 11.4 us, [3072, 1536] over 512 16.9 -> 15.5; as planes [3072, 2048] over
+// 512 23.6 -> 21.5, [3600, 1536] over 384 gated by factors 23.3 -> 20.1, with GELU 29.1 -> 28.4.)
+// fp32 results go best with eight warps and unrolled rows; planes take twice the arithmetic per element and 16 warps (with eight,
+// GELU: 35 us).  The loops over chunks are not unrolled: a launch with one tile per CTA runs this code once, from a cold instruction cache.
+// acc[j] of column j of a chunk for this lane's row, times the row's inverse scale
+template <bool MERGED, int CC>
+__device__ __forceinline__ void tc_acc_chunk(uint32_t taddr, uint32_t acc_main, uint32_t acc_cross, bool any, float isa, float (&v)[CC]) {
   if (any) {
-    uint32_t r[32];
-    tmem_ld32(taddr + acc_main, r);
-    if constexpr (!MERGED) {
-      uint32_t q[32];
-      tmem_ld32(taddr + acc_cross, q);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    uint32_t r[CC], q[MERGED ? 1 : CC];
+    if constexpr (CC == 32) { tmem_ld32(taddr + acc_main, r); if constexpr (!MERGED) tmem_ld32(taddr + acc_cross, q); }
+    else { tmem_ld16(taddr + acc_main, r); if constexpr (!MERGED) tmem_ld16(taddr + acc_cross, q); }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 32; j++) v[j] = (__uint_as_float(r[j]) + __uint_as_float(q[j])) * isa;
-    } else {
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]) * isa;
+    for (int j = 0; j < CC; j++) {
+      if constexpr (MERGED) v[j] = __uint_as_float(r[j]) * isa; else v[j] = (__uint_as_float(r[j]) + __uint_as_float(q[j])) * isa;
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = 0.f;
+    for (int j = 0; j < CC; j++) v[j] = 0.f;
   }
 }
-// 32 bytes from one thread, 32-byte aligned
-__device__ __forceinline__ void st_global_32(void* p, const uint32_t (&r)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-__device__ __forceinline__ void ld_global_32(const float* p, float* r) {
-  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]) : "l"(p) : "memory");
-}
-template <int RS>
-__device__ __forceinline__ void tc_stage_rows(float* stg, const float (&v)[32], int lane, int hh) {
-  __syncwarp();                                               // the previous half has been read back
-  if (lane / RS == hh) {
-    float* s = stg + lane % RS * TC_STG_LD;
-#pragma unroll
-    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(s + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-  }
-  __syncwarp();
-}
-template <int BN, bool PL, bool MERGED>
-__device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tmem_base, uint32_t acc_main, uint32_t acc_cross,
-                                                 int m0, int n0, int z, int quad, int cg, int lane, int nkb, int bw, const float* colv, float* stg) {
+// `acc_main` / `acc_cross` are the TMEM column offsets of the two accumulators of this tile (MERGED: there is only acc_main); `bw` is the
+// tile's width (BN, or BN / 2 for a half tile).  `wait` blocks until the accumulator is complete; false: it gave up.
+template <int BN, bool PL, bool MERGED, class W>
+__device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tmem_base, uint32_t acc_main, uint32_t acc_cross,
+                                                 int m0, int n0, int z, int quad, int cg, int lane, int nkb, int bw, float* stg, W&& wait) {
   using Cfg = TcCfg<BN, PL>;
-  const int z1 = z / ep.batch2, z2 = z - z1 * ep.batch2, nch = max(bw / (32 * Cfg::CG), 1);      // chunks of 32 columns per warp
-  if (cg * nch * 32 >= bw) return;                                           // a narrow tile has fewer chunks than column groups
-  const int rbase = m0 + quad * 32, row = rbase + lane;
+  const int z1 = z / ep.batch2, z2 = z - z1 * ep.batch2, nch = max(bw / (Cfg::CC * Cfg::CG), 1);      // chunks per warp
+  if (cg * nch * Cfg::CC >= bw) return wait();                               // a narrow tile has fewer chunks than column groups
+  const int rbase = m0 + quad * 32, row = rbase + lane, c_end = min(cg * nch + nch, (ep.N - n0 + Cfg::CC - 1) / Cfg::CC);
+  const bool row_ok = row < ep.M;
   const uint32_t tquad = tmem_base + ((uint32_t)(quad * 32) << 16);
-  const float isa = row < ep.M ? ep.isa[(ep.k_slice ? 0L : (long)z * ep.M) + row] : 1.f;         // 1 / (scale of this row's A vector), a power of two
-  const int rl = lane >> 3, c4 = (lane & 7) * 4;                             // after the exchange: rows 4 t + rl, columns c4 .. c4 + 3
+  const float isa = row_ok ? ep.isa[(ep.k_slice ? 0L : (long)z * ep.M) + row] : 1.f;             // 1 / (scale of this row's A vector), a power of two
+  const float* isb = ep.isb + (ep.k_slice ? 0L : (long)z * ep.N);
   if constexpr (PL) {
-    // plane output: the result becomes the next contraction's A operand
-    float osc = 1.f;                                                         // this lane's row's scale
-    if (row < ep.M) {
+    // Plane output: the result becomes the next contraction's A operand.  Twice the work per element (activation or factors, scale,
+    // two conversions): 16 warps, chunks of 16 columns, after the exchange four lanes on a row.
+    const int rl = lane >> 2, c4 = lane & 3, r0 = rbase + rl;                // this lane's rows r0 + 8 t and columns 4 c4 .. 4 c4 + 3 of a chunk
+    const bool few = ep.mask_group >= 32;                                    // 32 rows belong to two sequences at most: their gates are fetched ahead
+    const int g0 = ep.mask ? rbase / ep.mask_group : 0, g_next = ep.mask ? (g0 + 1) * ep.mask_group : 0;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f); float4 sv = zero, bv = zero, k0 = zero, k1 = zero;
+    auto fetch = [&](int c) {
+      const int col = n0 + c * 16 + 4 * c4; if (c >= c_end) return;          // (N is a multiple of 32)
+      sv = __ldg(reinterpret_cast<const float4*>(isb + col)); if (ep.bias) bv = __ldg(reinterpret_cast<const float4*>(ep.bias + col));
+      if (ep.mask && few) {
+        const float* q = ep.mask + (long)g0 * ep.mask_ld + col;
+        if (rbase < ep.M) k0 = __ldg(reinterpret_cast<const float4*>(q));
+        if (g_next < min(rbase + 32, ep.M)) k1 = __ldg(reinterpret_cast<const float4*>(q + ep.mask_ld));
+      }
+    };
+    fetch(cg * nch);
+    float osc = 1.f;                                                         // the scale of row `row`
+    if (row_ok) {
       const float an = ep.a_rownorm[row], bound = sqrtf(fmaf(an, an, 1.f)) * sqrtf((float)ep.K + 1.f) * __int_as_float(*ep.b_maxabs);
       float oinv; osc = row_scale(ep.flags & TC_FLAG_SCALE ? 1.25f * bound : bound, &oinv);
       if (n0 == 0 && cg == 0) ep.out_inv[row] = oinv;
     }
-    // A thread keeps the row that TMEM gave it: 32 columns of a row are one block of the planes, 64 bytes of each, stored 32 bytes (a
-    // whole sector) at a time.  Through shared memory, eight lanes on a row and 8-byte
-    // stores, the warps mostly waited for one another: [3600, 1536] over 384 with GELU 30.9 us, now 24.8.
-    const bool row_ok = row < ep.M; const int seq = ep.last_T > 0 ? row / ep.last_T : 0; const bool is_last = ep.c_last && row_ok && row - seq * ep.last_T == ep.last_T - 1;
+    const unsigned last = ep.c_last ? __ballot_sync(0xffffffffu, row_ok && row % ep.last_T == ep.last_T - 1) >> rl : 0u;      // bit 8 t: row r0 + 8 t is a sequence's last
+    if (!wait()) return false;
 #pragma unroll 1
-    for (int cc = 0; cc < nch; cc++) {
-      const int c = cg * nch + cc, col = n0 + c * 32;
-      if (col >= ep.N) break;                                                // (N is a multiple of 32)
-      float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
-      const float* sv = colv + cc * 32; const float* bv = sv + Cfg::CW;
-      const float* mrow = ep.mask && row_ok ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld + col : nullptr;
-      __half* o = ep.out_p + (long)row * 2 * ep.out_ldp + pl_off(col);
+    for (int c = cg * nch; c < c_end; c++) {
+      const int col = n0 + c * 16 + 4 * c4;
+      {
+        float v[16]; tc_acc_chunk<MERGED, 16>(tquad + c * 16, acc_main, acc_cross, nkb > 0, isa, v);
+        __syncwarp();                                                        // the previous chunk has been read back
 #pragma unroll
-      for (int j = 0; j < 32; j += 16) {
-        uint32_t hi[8], lo[8];
+        for (int j = 0; j < 4; j++) *reinterpret_cast<float4*>(stg + lane * 16 + ((j ^ (lane >> 1 & 3)) << 2)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+      }
+      float4 a[4];
 #pragma unroll
-        for (int q = 0; q < 16; q += 4) {
-          const float4 s4 = *reinterpret_cast<const float4*>(sv + j + q), b4 = *reinterpret_cast<const float4*>(bv + j + q);
-          float4 x = make_float4(v[j + q] * s4.x + b4.x, v[j + q + 1] * s4.y + b4.y, v[j + q + 2] * s4.z + b4.z, v[j + q + 3] * s4.w + b4.w);
-          if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
-          else if (ep.act == GN_ACT_GELU) {
-            if (is_last && ep.z_last) *reinterpret_cast<float4*>(ep.z_last + (long)seq * ep.N + col + j + q) = x;
-            x.x = gelu_f(x.x); x.y = gelu_f(x.y); x.z = gelu_f(x.z); x.w = gelu_f(x.w);
-          }
-          if (mrow) {
-            const float4 m4 = *reinterpret_cast<const float4*>(mrow + j + q);
-            if (ep.flags & TC_FLAG_SCALE) { x.x *= m4.x; x.y *= m4.y; x.z *= m4.z; x.w *= m4.w; }
-            else { if (!(m4.x > 0.f)) x.x = 0.f; if (!(m4.y > 0.f)) x.y = 0.f; if (!(m4.z > 0.f)) x.z = 0.f; if (!(m4.w > 0.f)) x.w = 0.f; }
-          }
-          if (is_last) *reinterpret_cast<float4*>(ep.c_last + (long)seq * ep.N + col + j + q) = x;
-          split2_pair(x.x, x.y, osc, hi[q / 2], lo[q / 2]); split2_pair(x.z, x.w, osc, hi[q / 2 + 1], lo[q / 2 + 1]);
-          v[j + q] = x.x; v[j + q + 1] = x.y; v[j + q + 2] = x.z; v[j + q + 3] = x.w;
+      for (int t = 0; t < 4; t++) { const int r = 8 * t + rl; a[t] = *reinterpret_cast<const float4*>(stg + r * 16 + ((c4 ^ (r >> 1 & 3)) << 2)); }
+#pragma unroll
+      for (int t = 0; t < 4; t++) a[t] = make_float4(a[t].x * sv.x + bv.x, a[t].y * sv.y + bv.y, a[t].z * sv.z + bv.z, a[t].w * sv.w + bv.w);
+      if (ep.act == GN_ACT_RELU) {
+#pragma unroll
+        for (int t = 0; t < 4; t++) a[t] = make_float4(fmaxf(a[t].x, 0.f), fmaxf(a[t].y, 0.f), fmaxf(a[t].z, 0.f), fmaxf(a[t].w, 0.f));
+      } else if (ep.act == GN_ACT_GELU) {
+        if (last && ep.z_last) {
+#pragma unroll
+          for (int t = 0; t < 4; t++) if (last >> (8 * t) & 1) *reinterpret_cast<float4*>(ep.z_last + (long)((r0 + 8 * t) / ep.last_T) * ep.N + col) = a[t];
         }
-        if (row_ok) { st_global_32(o + j, hi); st_global_32(o + j + PL_LO, lo); }
+#pragma unroll
+        for (int t = 0; t < 4; t++) a[t] = make_float4(gelu_f(a[t].x), gelu_f(a[t].y), gelu_f(a[t].z), gelu_f(a[t].w));
+      }
+      if (ep.mask) {
+        float4 m[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const int r = r0 + 8 * t;
+          m[t] = few ? (r < g_next ? k0 : k1) : r < ep.M ? *reinterpret_cast<const float4*>(ep.mask + (long)(r / ep.mask_group) * ep.mask_ld + col) : zero;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          if (ep.flags & TC_FLAG_SCALE) { a[t].x *= m[t].x; a[t].y *= m[t].y; a[t].z *= m[t].z; a[t].w *= m[t].w; }
+          else { if (!(m[t].x > 0.f)) a[t].x = 0.f; if (!(m[t].y > 0.f)) a[t].y = 0.f; if (!(m[t].z > 0.f)) a[t].z = 0.f; if (!(m[t].w > 0.f)) a[t].w = 0.f; }
+        }
+      }
+      fetch(c + 1);                                                          // under this chunk's conversions and stores
+      if (last) {
+#pragma unroll
+        for (int t = 0; t < 4; t++) if (last >> (8 * t) & 1) *reinterpret_cast<float4*>(ep.c_last + (long)((r0 + 8 * t) / ep.last_T) * ep.N + col) = a[t];
+      }
+      __half* o = ep.out_p + (long)r0 * 2 * ep.out_ldp + pl_off(col); float4 u = zero;
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const float sc = __shfl_sync(0xffffffffu, osc, 8 * t + rl);
+        uint2 hi, lo; split2_pair(a[t].x, a[t].y, sc, hi.x, lo.x); split2_pair(a[t].z, a[t].w, sc, hi.y, lo.y);
+        if (r0 + 8 * t < ep.M) {
+          __half* q = o + (long)(16 * t) * ep.out_ldp; *reinterpret_cast<uint2*>(q) = hi; *reinterpret_cast<uint2*>(q + PL_LO) = lo;
+          u.x += a[t].x; u.y += a[t].y; u.z += a[t].z; u.w += a[t].w;
+        }
       }
       if (ep.rowsum32) {
         // the consumer of a plane output's token sums (the weight gradient of the layer below) gets them from here instead of
-        // re-reading the planes: lane c ends up with the sum of column c over the warp's rows, in a fixed order
+        // re-reading the planes: the sum of every column over the warp's rows, in a fixed order
 #pragma unroll
-        for (int h = 16; h > 0; h >>= 1)
-#pragma unroll
-          for (int k = 0; k < h; k++) {
-            const float lo_ = row_ok ? v[k] : 0.f, hi_ = row_ok ? v[k + h] : 0.f; const bool up = lane & h;
-            const float got = __shfl_xor_sync(0xffffffffu, up ? (h == 16 ? lo_ : v[k]) : (h == 16 ? hi_ : v[k + h]), h);
-            v[k] = (up ? (h == 16 ? hi_ : v[k + h]) : (h == 16 ? lo_ : v[k])) + got;
-          }
-        if (rbase < ep.M) ep.rowsum32[(long)(rbase >> 5) * ep.N + col + lane] = v[0];
+        for (int h = 4; h < 32; h <<= 1) {
+          u.x += __shfl_xor_sync(0xffffffffu, u.x, h); u.y += __shfl_xor_sync(0xffffffffu, u.y, h);
+          u.z += __shfl_xor_sync(0xffffffffu, u.z, h); u.w += __shfl_xor_sync(0xffffffffu, u.w, h);
+        }
+        if (rl == 0 && rbase < ep.M) *reinterpret_cast<float4*>(ep.rowsum32 + (long)(rbase >> 5) * ep.N + col) = u;
       }
     }
     __syncwarp();
-  } else {
+    return true;
+  }
   float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
   const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
-  if (ep.flags & TC_FLAG_WIDE) {
-    // A thread keeps the row that TMEM gave it and reads and writes whole 32-byte sectors of it: no exchange through shared memory
-    // and none of its warp barriers (the launches of a 64 x 512 step: 289 -> 274 us on average).  For 32-byte aligned rows; the
-    // exchange below serves the rest.
-    const bool row_ok = row < ep.M;
-    const float* Mrow = ep.mask && row_ok ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
-#pragma unroll 1
-    for (int cc = 0; cc < nch; cc++) {
-      const int c = cg * nch + cc, col = n0 + c * 32;
-      if (col >= ep.N) break;
-      const long so = ep.n_seg ? (col / ep.n_seg) * (ep.c_seg - ep.n_seg) : 0;      // (32 columns lie in one segment; with segments R is C)
-      float* Cr = C + so + (long)row * ep.ldc + col; const float* Rr = R && row_ok ? R + so + (long)row * ep.ldr + col : nullptr;
-      float rv[32];
-#pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-#pragma unroll
-        for (int q = 0; q < 8; q++) rv[j + q] = 0.f;
-        if (Rr && col + j < ep.N) ld_global_32(Rr + j, rv + j);
-      }
-      float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
-      const float* sv = colv + cc * 32; const float* bv = sv + Cfg::CW; float zm = 0.f;
-#pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-        uint32_t o[8];
-#pragma unroll
-        for (int q = 0; q < 8; q += 4) {
-          const float4 s4 = *reinterpret_cast<const float4*>(sv + j + q), b4 = *reinterpret_cast<const float4*>(bv + j + q);
-          float4 x = make_float4(v[j + q] * s4.x + b4.x + rv[j + q], v[j + q + 1] * s4.y + b4.y + rv[j + q + 1], v[j + q + 2] * s4.z + b4.z + rv[j + q + 2], v[j + q + 3] * s4.w + b4.w + rv[j + q + 3]);
-          if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
-          if (Mrow && col + j < ep.N) {
-            const float4 m4 = *reinterpret_cast<const float4*>(Mrow + col + j + q);
-            if (!(m4.x > 0.f)) x.x = 0.f; if (!(m4.y > 0.f)) x.y = 0.f; if (!(m4.z > 0.f)) x.z = 0.f; if (!(m4.w > 0.f)) x.w = 0.f;
-          }
-          o[q] = __float_as_uint(x.x); o[q + 1] = __float_as_uint(x.y); o[q + 2] = __float_as_uint(x.z); o[q + 3] = __float_as_uint(x.w);
-          if (ep.zmax && row_ok) zm = fmaxf(zm, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-        }
-        if (row_ok && col + j < ep.N) st_global_32(Cr + j, o);
-      }
-      if (ep.zmax) {                                                         // (32 rows of one sequence, 32 columns of one head)
-        zm = warp_max(zm); if (!(zm <= 3.0e38f)) zm = 3.4e38f;
-        const int sg = col / ep.n_seg;
-        if (lane == 0 && rbase < ep.M) atomicMax(ep.zmax + sg * ep.zmax_seg + (long)(rbase / ep.zmax_T) * ep.zmax_H + (col - sg * ep.n_seg) / 64, __float_as_int(zm));
-      }
-    }
-    __syncwarp();
-    return;
-  }
   if (ep.flags & TC_FLAG_VEC) {
+    const int rl = lane >> 3, c8 = lane & 7, r0 = rbase + rl;                // after the exchange: this lane's rows r0 + 4 t and columns 4 c8 .. 4 c8 + 3 of a chunk
+    float4 sv, bv, rv[8];                                                    // what the next chunk needs for them
+    auto fetch = [&](int c) {
+      const int col = n0 + c * 32 + 4 * c8; const bool ok = c < c_end && col < ep.N; const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      const int seg = ep.n_seg && ok ? col / ep.n_seg : 0;                   // (32 columns lie in one segment)
+      sv = ok ? __ldg(reinterpret_cast<const float4*>(isb + col)) : zero;
+      bv = ok && ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + col + (long)seg * (ep.bias_seg - ep.n_seg))) : zero;
+      const float* q = R ? R + (long)seg * (ep.c_seg - ep.n_seg) + (long)r0 * ep.ldr + col : nullptr;      // (with segments R is C)
+#pragma unroll
+      for (int t = 0; t < 8; t++) rv[t] = R && ok && r0 + 4 * t < ep.M ? *reinterpret_cast<const float4*>(q + (long)(4 * t) * ep.ldr) : zero;
+    };
+    fetch(cg * nch);
+    if (!wait()) return false;
 #pragma unroll 1
-    for (int cc = 0; cc < nch; cc++) {
-      const int c = cg * nch + cc, col = n0 + c * 32 + c4; const bool col_ok = col < ep.N;
-      if (n0 + c * 32 >= ep.N) break;
-      float v[32]; tc_acc_chunk<MERGED>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
-      const float4 sv = *reinterpret_cast<const float4*>(colv + cc * 32 + c4), bv = *reinterpret_cast<const float4*>(colv + Cfg::CW + cc * 32 + c4);
+    for (int c = cg * nch; c < c_end; c++) {
+      const int col = n0 + c * 32 + 4 * c8; const bool col_ok = col < ep.N;
+      {
+        float v[32]; tc_acc_chunk<MERGED, 32>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
+        __syncwarp();                                                        // the previous chunk has been read back
+#pragma unroll
+        for (int j = 0; j < 8; j++) *reinterpret_cast<float4*>(stg + lane * 32 + ((j ^ (lane & 7)) << 2)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+      }
+      float4 a[8];
+#pragma unroll
+      for (int t = 0; t < 8; t++) { const int r = 4 * t + rl; a[t] = *reinterpret_cast<const float4*>(stg + r * 32 + ((c8 ^ (r & 7)) << 2)); }
+#pragma unroll
+      for (int t = 0; t < 8; t++) a[t] = make_float4(a[t].x * sv.x + bv.x + rv[t].x, a[t].y * sv.y + bv.y + rv[t].y, a[t].z * sv.z + bv.z + rv[t].z, a[t].w * sv.w + bv.w + rv[t].w);
+      fetch(c + 1);                                                          // under this chunk's stores
+      if (ep.act == GN_ACT_RELU) {
+#pragma unroll
+        for (int t = 0; t < 8; t++) a[t] = make_float4(fmaxf(a[t].x, 0.f), fmaxf(a[t].y, 0.f), fmaxf(a[t].z, 0.f), fmaxf(a[t].w, 0.f));
+      }
+      if (ep.mask && col_ok) {
+        float4 m[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) m[t] = r0 + 4 * t < ep.M ? *reinterpret_cast<const float4*>(ep.mask + (long)((r0 + 4 * t) / ep.mask_group) * ep.mask_ld + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int t = 0; t < 8; t++) { if (!(m[t].x > 0.f)) a[t].x = 0.f; if (!(m[t].y > 0.f)) a[t].y = 0.f; if (!(m[t].z > 0.f)) a[t].z = 0.f; if (!(m[t].w > 0.f)) a[t].w = 0.f; }
+      }
+      const int seg = ep.n_seg ? col / ep.n_seg : 0; float* o = C + (long)seg * (ep.c_seg - ep.n_seg) + (long)r0 * ep.ldc + col;
       float zm = 0.f;
-      const long so = ep.n_seg ? ((n0 + c * 32) / ep.n_seg) * (ep.c_seg - ep.n_seg) : 0;      // (32 columns lie in one segment; with segments R is C)
-      float* Cs = C + so; const float* Rs = R + so;
-#pragma unroll 1
-      for (int hh = 0; hh < 32 / Cfg::RS; hh++) {
-        const int r0 = rbase + Cfg::RS * hh + rl;
-        float4 rv[Cfg::RS / 4];                                                        // residual, fetched before the exchange so that its latency overlaps it
 #pragma unroll
-        for (int t = 0; t < Cfg::RS / 4; t++) rv[t] = (R && col_ok && r0 + 4 * t < ep.M) ? *reinterpret_cast<const float4*>(Rs + (long)(r0 + 4 * t) * ep.ldr + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-        tc_stage_rows<Cfg::RS>(stg, v, lane, hh);
-#pragma unroll
-        for (int t = 0; t < Cfg::RS / 4; t++) {
-          const int r = r0 + 4 * t;
-          const float4 a = *reinterpret_cast<const float4*>(stg + (4 * t + rl) * TC_STG_LD + c4);
-          float4 x = make_float4(a.x * sv.x + bv.x + rv[t].x, a.y * sv.y + bv.y + rv[t].y, a.z * sv.z + bv.z + rv[t].z, a.w * sv.w + bv.w + rv[t].w);
-          if (ep.act == GN_ACT_RELU) { x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f); }
-          if (!col_ok || r >= ep.M) continue;
-          if (ep.mask) {
-            const float4 mv = *reinterpret_cast<const float4*>(ep.mask + (long)(r / ep.mask_group) * ep.mask_ld + col);
-            if (!(mv.x > 0.f)) x.x = 0.f; if (!(mv.y > 0.f)) x.y = 0.f; if (!(mv.z > 0.f)) x.z = 0.f; if (!(mv.w > 0.f)) x.w = 0.f;
-          }
-          *reinterpret_cast<float4*>(Cs + (long)r * ep.ldc + col) = x;
-          if (ep.zmax) zm = fmaxf(zm, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-        }
+      for (int t = 0; t < 8; t++) if (col_ok && r0 + 4 * t < ep.M) {
+        *reinterpret_cast<float4*>(o + (long)(4 * t) * ep.ldc) = a[t];
+        zm = fmaxf(zm, fmaxf(fmaxf(fabsf(a[t].x), fabsf(a[t].y)), fmaxf(fabsf(a[t].z), fabsf(a[t].w))));
       }
       if (ep.zmax) {                                                         // (32 rows of one sequence, 32 columns of one head)
         zm = warp_max(zm); if (!(zm <= 3.0e38f)) zm = 3.4e38f;
@@ -431,11 +396,10 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
       }
     }
     __syncwarp();
-    return;
+    return true;
   }
+  if (!wait()) return false;
   // scalar path (unaligned operands, NCHW store): one output row per thread
-  const bool row_ok = row < ep.M;
-  const float* isb = ep.isb + (ep.k_slice ? 0L : (long)z * ep.N);
   const float* Rrow = (R && row_ok) ? R + (long)row * ep.ldr : nullptr;
   const float* Mrow = (ep.mask && row_ok) ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
   float* Crow = ep.nchw_P > 0 ? C + (long)(row / ep.nchw_P) * ep.N * ep.nchw_P + row % ep.nchw_P : C + (long)row * ep.ldc;
@@ -445,7 +409,7 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
     const int col0 = n0 + (cg * nch + cc) * 32;
     if (col0 >= ep.N) break;
     const int seg = ep.n_seg ? col0 / ep.n_seg : 0; const long c_off = ep.n_seg ? seg * (ep.c_seg - ep.n_seg) : 0, b_off = ep.n_seg ? seg * (ep.bias_seg - ep.n_seg) : 0;
-    float v[32]; tc_acc_chunk<MERGED>(tquad + (cg * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
+    float v[32]; tc_acc_chunk<MERGED, 32>(tquad + (cg * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
 #pragma unroll
     for (int j = 0; j < 32; j++) {
       const int col = col0 + j;
@@ -458,7 +422,7 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& ep, uint32_t tm
       Crow[c_off + col * cstep] = x;
     }
   }
-  }
+  return true;
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -478,7 +442,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
   uint64_t* qbars = bars + 2 * STAGES + 6;                         // tile queue: qfull[4], qempty[4], then the four queued items
   volatile int* qitem = (volatile int*)(qbars + 8);
   const uint32_t qfull0 = smem_u32(qbars), qempty0 = smem_u32(qbars + 4);
-  float* colv_all = (float*)(smem + STAGES * STAGE_BYTES + 256);   // epilogue warps' column factors
+  float* stg_all = (float*)(smem + STAGES * STAGE_BYTES + 256);    // epilogue warps' staging buffers
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
   const uint32_t drain = smem_u32(bars + 2 * STAGES + 4);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp-uniform for the compiler, too)
@@ -622,20 +586,19 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
     __syncwarp();
   } else {
     const int quad = warp & 3, cg = (warp - 2) >> 2; uint32_t lt = 0;
-    float* colv = colv_all + (warp - 2) * 2 * Cfg::CW;
-    float* stg = colv_all + Cfg::COLV_FLOATS + (warp - 2) * Cfg::RS * TC_STG_LD;
+    float* stg = stg_all + (warp - 2) * 32 * Cfg::CC;
     int tile, half;
     for (int w = 0; work(w, tile, half); w++) {
       int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
       const uint32_t slot = lt & 1, u = lt >> 1; lt++;
       const int bw = half < 0 ? BN : BN / 2;
-      tc_epilogue_stage<BN, PL>(ep, n0, ep.k_slice ? 0 : z, cg, lane, bw, colv);
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(tfull0 + 8 * slot, u & 1, limit, abort_flag) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      const bool ok = tc_epilogue_tile<BN, PL, MERGED>(ep, tmem_base, slot * SLOT_COLS, slot * SLOT_COLS + BN, m0, n0, z, quad, cg, lane, nkb, bw, stg, [&]() -> bool {
+        int got = 1;
+        if (lane == 0) got = mbar_wait(tfull0 + 8 * slot, u & 1, limit, abort_flag) ? 1 : 0;
+        got = __shfl_sync(0xffffffffu, got, 0);
+        tc_fence_after(); return got != 0;
+      });
       if (!ok) { if (lane == 0 && !*abort_flag) give_up(3); break; }
-      tc_fence_after();
-      tc_epilogue_tile<BN, PL, MERGED>(ep, tmem_base, slot * SLOT_COLS, slot * SLOT_COLS + BN, m0, n0, z, quad, cg, lane, nkb, bw, colv, stg);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty0 + 8 * slot);
@@ -962,8 +925,6 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
   }
   if (ep.zmax && !vec) return fail(GN_ERR_INVALID_ARG, "tc_launch: maxima need 16-byte aligned operands");
   if (vec) ep.flags |= TC_FLAG_VEC;
-  auto a32 = [](const void* p, long ld, long o1, long o2) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)((ld | o1 | o2) * 4)) & 31) == 0; };
-  if (vec && ep.N % 8 == 0 && a32(ep.C, ep.ldc, ep.c_b1, ep.c_b2) && ep.c_seg % 8 == 0 && (!ep.R || a32(ep.R, ep.ldr, ep.r_b1, ep.r_b2))) ep.flags |= TC_FLAG_WIDE;
   {
     double by = 4.0 * ((double)ep.M + ep.N) * ep.K + 4.0 * (double)ep.M * ep.N * (ep.R ? 2 : 1);
     if (ep.flags & (GEMM_SKIP_UPPER | GEMM_KBEG_AT_M0 | GEMM_KEND_AT_M0)) by *= 0.5;
