@@ -38,6 +38,7 @@ struct GemmDesc {
   int* zmax = nullptr; int zmax_T = 0;                  // with n_seg: largest magnitudes per sequence and head of the result (TcParams::zmax)
   int n_seg = 0, k_seg = 0, m_seg = 0; long c_seg = 0, bias_seg = 0, a_seg = 0;
   int batch1 = 1, batch2 = 1;                           // batch index b -> (b / batch2, b % batch2)
+  const int* z_first = nullptr;                         // tensor-core engine may leave out problem (i, j) where j < z_first[i] (device memory): nothing reads its result
   long a_b1 = 0, a_b2 = 0, b_b1 = 0, b_b2 = 0, c_b1 = 0, c_b2 = 0, r_b1 = 0, r_b2 = 0;
   // Causal structure of attention: tiles that are entirely masked are never touched.
   //   GEMM_SKIP_UPPER : do not compute output tiles with n0 > m0 + BM - 1 (S = Q K^T)

@@ -200,6 +200,7 @@ struct TcParams {
   int n_seg = 0; long c_seg = 0, bias_seg = 0;                         // > 0 (a multiple of 32): columns j n_seg .. lie c_seg (biases: bias_seg) floats after those of segment j - 1, see GemmDesc::n_seg
   int* zmax = nullptr; int zmax_T = 0, zmax_H = 0; long zmax_seg = 0;  // receives the largest magnitude per (segment, sequence of zmax_T rows, head of 64 columns), see attn_tc_max_words
   int k_slice = 0, splits = 1;                                         // k_slice > 0 (a multiple of 32): z is not a problem but a slice of the contraction, C + z c_b1 its partial result
+  const int* z_first = nullptr;                                        // problems (i, j) with j < z_first[i] are left out
   float* rowsum32 = nullptr;                                           // plane output: sums of the result over every 32 consecutive rows, [ceil(M / 32)][N]
 };
 
@@ -508,6 +509,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
     const int nt = tile % tiles_n, q = tile / tiles_n, mt = q % tiles_m; z = q / tiles_m;
     m0 = mt * TC_BM; n0 = nt * BN + (half > 0 ? BN / 2 : 0);
     if ((ep.flags & GEMM_SKIP_UPPER) && n0 > m0 + TC_BM - 1) return false;
+    if (ep.z_first && z % ep.batch2 < ep.z_first[z / ep.batch2]) return false;
     int kbeg = 0, kend = ep.K;
     if (ep.k_slice) { kbeg = z * ep.k_slice; kend = min(ep.K, kbeg + ep.k_slice); }
     if (ep.flags & GEMM_KBEG_AT_M0) kbeg = (m0 / BK) * BK;
@@ -623,7 +625,8 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
 // Two fp16 planes per operand, fp16(x s) and fp16(x s - fp16(x s)), interleaved (pl_off), and the inverse 1/s of every plane row's scale.
 // Rows may consist of segments of `seg` elements (> 0, a multiple of 32), each `seg_stride` floats after the one before: column c at
 // p + r * s_r + c % seg + (c / seg) * seg_stride.
-struct TcSrc { const float* p; long s_r, s_c, b1, b2; int batch2; int seg = 0; long seg_stride = 0; };
+// Problem z is left out if z % batch2 < first[z / batch2] (rows split as they lie only).
+struct TcSrc { const float* p; long s_r, s_c, b1, b2; int batch2; int seg = 0; long seg_stride = 0; const int* first = nullptr; };
 // One warp per plane row: first the row's largest magnitude (the row is read a second time from L1 / L2 afterwards),
 // then eight elements per lane and step (two 16-byte loads, one 16-byte store per plane).  blockIdx.y = problem index.
 // `rownorm` (may be null): receives the L2 norm of every row (a factor of the bound of a plane-output contraction).
@@ -631,7 +634,7 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int
                                                           float* __restrict__ rownorm) {
   const int z = blockIdx.y, lane = threadIdx.x & 31;
   const long r = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (r >= rows) return;
+  if (r >= rows || (s.first && z % s.batch2 < s.first[z / s.batch2])) return;
   const float* src = s.p + (z / s.batch2) * s.b1 + (z % s.batch2) * s.b2 + r * s.s_r;
   const int seg = s.seg ? s.seg : cols; const long over = s.seg ? s.seg_stride - s.seg : 0;
   const bool vec = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(over * 4)) & 15) == 0;
@@ -1233,14 +1236,14 @@ inline int gemm_tc(Ctx* ctx, const GemmDesc& g) {
   } else if (!g.a_rownorm && g.reuse_a_planes && nb == 1 && sc.last_a == g.A && sc.last_m == g.M && sc.last_k == g.K && sc.last_ld == g.sa_m && g.sa_k == 1) {
     // same tensor as the previous call (the Q, K and V projections share their input): planes still valid
   } else {
-    GN_TRY(tc_split(ctx, TcSrc{g.A, g.sa_m, g.sa_k, g.a_b1, g.a_b2, g.batch2}, A, mx, g.a_rownorm));
+    GN_TRY(tc_split(ctx, TcSrc{g.A, g.sa_m, g.sa_k, g.a_b1, g.a_b2, g.batch2, 0, 0, g.z_first}, A, mx, g.a_rownorm));
     sc.last_a = (nb == 1 && g.sa_k == 1) ? g.A : nullptr; sc.last_m = g.M; sc.last_k = g.K; sc.last_ld = g.sa_m;
   }
   if (g.b_planes) {
     B = *static_cast<const BfPlanes*>(g.b_planes);
     if (B.rows != g.N || B.K != g.K || B.nbatch != nb) return fail(GN_ERR_INVALID_ARG, "gemm_tc: prepared planes of B do not match the contraction");
-  } else GN_TRY(tc_split(ctx, TcSrc{g.B, g.sb_n, g.sb_k, g.b_b1, g.b_b2, g.batch2}, B, mx));
-  TcParams ep{g.C, g.ldc, g.c_b1, g.c_b2, g.bias, g.R, g.ldr, g.r_b1, g.r_b2, g.act, g.M, g.N, g.K, g.batch2, g.flags, ctx->d_status, g.mask, g.mask_ld, g.mask_group};
+  } else GN_TRY(tc_split(ctx, TcSrc{g.B, g.sb_n, g.sb_k, g.b_b1, g.b_b2, g.batch2, 0, 0, g.z_first}, B, mx));
+  TcParams ep{g.C, g.ldc, g.c_b1, g.c_b2, g.bias, g.R, g.ldr, g.r_b1, g.r_b2, g.act, g.M, g.N, g.K, g.batch2, g.flags, ctx->d_status, g.mask, g.mask_ld, g.mask_group}; ep.z_first = g.z_first;
   if (g.n_seg) {
     if (g.n_seg % 32 || nb != 1 || g.R || g.plane_out) return fail(GN_ERR_INVALID_ARG, "gemm_tc: this contraction cannot write its columns in segments");
     ep.n_seg = g.n_seg; ep.c_seg = g.c_seg; ep.bias_seg = g.bias_seg;

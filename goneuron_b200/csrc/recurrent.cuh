@@ -316,8 +316,9 @@ inline int gru_bwd_reg(Ctx* ctx, const float* gout, const float* Wh, const float
 // later updates with |u_i| > 2.  Groups for which that is below 2^-CLIP_FORGET, far under the last bit of a double, are not walked: the
 // walk starts from zero at the first group that can be seen in the result (lstm_clip_start_kernel), at group 0 if there is none,
 // or if any update is not finite.  Gradients that are carried back through many steps grow by orders of magnitude per sequence
-// (median |u| 2e5 for 64 steps of 128 units), and a few dozen updates decide the result: that step of 256 samples went from 1777 to
-// 667 us.  Where nothing can be left out the extra launch costs about 5 us.
+// (median |u| 2e5 for 64 steps of 128 units), and a few dozen updates decide the result.  What is not walked is not gathered and
+// has no Gram blocks either: that step of 256 samples went from 1777 us to 667 without the walk and to 578 without the rest.
+// Where nothing can be left out the two launches that look for the start cost about 12 us.
 constexpr int CG = 128, CG_THREADS = 512, CG_PAD = CG, CG_TILE = 160;        // CG_PAD: rows of zeros before a chunk: group -1
 constexpr int CG_GD = CG + 1;
 constexpr long CG_MAX_K = 1L << 20;                         // updates per worker chunk
@@ -329,9 +330,10 @@ inline size_t clip_smem(int ZW) {
 }
 // Rows of Dm [., 4H] and Zm [., zs]: chunk c's updates from row c * stride + lead on.  k: update in global order.
 __global__ void lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
-                                           int T, int in, int H, int zs, long n_updates, long Kc, long stride, long lead) {
+                                           int T, int in, int H, int zs, long n_updates, long Kc, long stride, long lead, const int* __restrict__ start) {
   const int R4 = 4 * H, ZW = in + H + 1;
   const long k = blockIdx.x; if (k >= n_updates) return;
+  if (start && k % Kc < (long)(start[k / Kc] - 1) * CG) return;               // before the first walked group and the one it is multiplied with
   const int s = (int)(k / T), t = T - 1 - (int)(k % T); const long row = (k / Kc) * stride + lead + k % Kc;
   for (int e = threadIdx.x; e < R4 + zs; e += blockDim.x) {
     if (e < R4) Dm[row * R4 + e] = D[((long)s * T + t) * R4 + e];
@@ -349,28 +351,52 @@ __global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __r
   const long k = blockIdx.x, row = (k / Kc) * stride + lead + k % Kc;
   for (int e = threadIdx.x; e < w; e += blockDim.x) dst[row * w + e] = src[k * w + e];
 }
-__global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restrict__ G2, long total4) {
+__global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restrict__ G2, long total4, int groups, const int* __restrict__ start) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total4; i += (long)gridDim.x * blockDim.x) {
+    const int j = (int)(i / (CG * CG / 2)); if (j % groups < start[j / groups]) continue;
     float4 a = reinterpret_cast<float4*>(G)[i]; const float4 b = reinterpret_cast<const float4*>(G2)[i];
     a.x *= b.x; a.y *= b.y; a.z *= b.z; a.w *= b.w; reinterpret_cast<float4*>(G)[i] = a;
   }
 }
 constexpr int CLIP_FORGET = 128;
 constexpr float CLIP_FINITE = 1e36f;                        // squared norms above this count as not finite
-// start[chunk]: the first group to walk.  G holds the squared norms on the diagonals of the groups' own Gram blocks.
-__global__ void __launch_bounds__(1024) lstm_clip_start_kernel(const float* __restrict__ G, int groups, int* __restrict__ start) {
-  __shared__ float part[32]; __shared__ int first;
-  const int chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5; const float* g = G + (long)chunk * groups * CG * 2 * CG;
-  auto norm2 = [&](int j, int r) { return g[((long)j * CG + r) * 2 * CG + CG + r]; };
-  int fine = 1;
+// |u_k|^2 = |d_k|^2 |z_k|^2 of every update, in update order; a warp each.  From the layer's own arrays (d, x, h as in
+// lstm_gather_updates_kernel below), so that updates that are not walked need not be gathered.
+__global__ void __launch_bounds__(256) lstm_update_norms_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ un, int T, int in, int H, long n_updates) {
+  const long k = blockIdx.x * 8L + (threadIdx.x >> 5); const int lane = threadIdx.x & 31; if (k >= n_updates) return;
+  const long s = k / T; const int t = T - 1 - (int)(k % T); float d2 = 0.f, z2 = 0.f;
+  const float* d = D + (s * T + t) * 4 * H; const float* xl = x + s * T * in + (long)(T - 1) * in; const float* h = h_all + (s * T + max(t - 1, 0)) * H;
 #pragma unroll 4
-  for (long k = tid; k < (long)groups * CG; k += 1024) fine &= norm2((int)(k / CG), (int)(k % CG)) <= CLIP_FINITE;
+  for (int e = lane; e < 4 * H; e += 32) d2 = fmaf(d[e], d[e], d2);
+  for (int e = lane; e < in; e += 32) z2 = fmaf(xl[e], xl[e], z2);
+  if (t > 0) for (int e = lane; e < H; e += 32) z2 = fmaf(h[e], h[e], z2);
+  d2 = warp_sum(d2); z2 = warp_sum(z2) + 1.f;
+  if (lane == 0) un[k] = d2 * z2;
+}
+// ... from gathered rows
+__global__ void __launch_bounds__(256) lstm_row_norms_kernel(const float* __restrict__ Dm, const float* __restrict__ Zm, float* __restrict__ un, int R4, int zs, long n_updates, long Kc, long stride, long lead) {
+  const long k = blockIdx.x * 8L + (threadIdx.x >> 5); const int lane = threadIdx.x & 31; if (k >= n_updates) return;
+  const long row = (k / Kc) * stride + lead + k % Kc; float d2 = 0.f, z2 = 0.f;
+#pragma unroll 4
+  for (int e = lane; e < R4; e += 32) d2 = fmaf(Dm[row * R4 + e], Dm[row * R4 + e], d2);
+  for (int e = lane; e < zs; e += 32) z2 = fmaf(Zm[row * zs + e], Zm[row * zs + e], z2);
+  d2 = warp_sum(d2); z2 = warp_sum(z2);
+  if (lane == 0) un[k] = d2 * z2;
+}
+// start[chunk]: the first group to walk
+__global__ void __launch_bounds__(1024) lstm_clip_start_kernel(const float* __restrict__ un, long n_updates, long Kc, int* __restrict__ start) {
+  __shared__ float part[32]; __shared__ int first;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5; const long k0 = blockIdx.x * Kc, n = min(Kc, n_updates - k0); const float* u = un + k0;
+  const int groups = (int)((Kc + CG - 1) / CG);
+  int fine = 1;
+#pragma unroll 8
+  for (long k = tid; k < n; k += 1024) fine &= u[k] <= CLIP_FINITE;
   fine = __syncthreads_and(fine);
   // a warp per group, 32 groups at a time from the end: log2 of the factor by which a group's updates shrink what was before it
   float sum = 0.f; int j0 = 0;
   for (int hi = groups; fine && hi > 0; hi -= 32) {
     const int j = hi - 1 - warp; float l = 0.f;
-    if (j >= 0) for (int r = lane; r < CG; r += 32) { const float n = sqrtf(norm2(j, r)); if (n > 2.01f) l += log2f(n - 1.f); }      // (0.01: the norms are rounded)
+    if (j >= 0) for (int r = lane; r < CG; r += 32) { const long k = (long)j * CG + r; const float q = k < n ? sqrtf(u[k]) : 0.f; if (q > 2.01f) l += log2f(q - 1.f); }      // (0.01: the norms are rounded)
     l = warp_sum(l);
     if (lane == 0) part[warp] = l;
     __syncthreads();
@@ -382,7 +408,7 @@ __global__ void __launch_bounds__(1024) lstm_clip_start_kernel(const float* __re
     if (first >= 0) { j0 = first; break; }
     __syncthreads();
   }
-  if (tid == 0) start[chunk] = j0;
+  if (tid == 0) start[blockIdx.x] = j0;
 }
 struct ClipArgs {
   const float *D, *Z, *G;        // rows of a chunk start at chunk * stride (CG_PAD rows of zeros first); G [chunk][group][CG][2 CG]: against groups j-1, j
