@@ -68,6 +68,15 @@ def test_blocks_on_the_tensor_cores(device, oracle, T, dim, heads, ff, kw):
     _parity(device, oracle, layers, 10)
 
 
+@pytest.mark.parametrize("T,batch", [(5, 160), (31, 26), (32, 26), (33, 24)])
+def test_plane_epilogue_gates_of_short_sequences(device, oracle, T, batch):
+    """The plane-writing epilogue fetches the factors of two sequences per 32 rows ahead; sequences of fewer than 32 tokens have more, and a
+    sequence's last row can lie anywhere in a warp's rows.  (GELU: its factors differ everywhere.)"""
+    layers = [D.Embedding(50, 192, T), D.PositionalEncoding(T, 192)] + [D.TransformerBlock(192, 6, T, 416, False, D.GELU, False, False) for _ in range(2)]
+    layers += [D.Flatten(), D.Dense(T * 192, 7, D.LOGSOFTMAX)]
+    _parity(device, oracle, layers, batch)
+
+
 @pytest.mark.parametrize("M,N,K", [(64, 352, 6000), (16, 100, 65600), (130, 65, 12000), (100, 1030, 1056)])
 def test_contraction_in_slices(device, M, N, K):
     """Few output tiles and a long contraction: slices of 256 indices and up, a ragged last one, outputs with and without
