@@ -670,6 +670,58 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int
     *reinterpret_cast<uint4*>(o + pl_off(c) + PL_LO) = b;
   }
 }
+// The same for few, long rows (the gradient of a head's output: 64 x 8192), where a warp per row leaves most SMs idle: a cluster of up to eight
+// blocks per row, every thread holding up to 32 of the row's elements in registers between the maximum and the planes.  Bound by
+// the latency of its loads and of one exchange through the cluster.  64 x 8192 took a warp per row 21 us with cold caches; a training step of the small causal
+// Transformer, which splits one such gradient, went from 742 to 730 us.  From 2048 columns on, where a warp walks its row eight times.
+constexpr int SPLIT_W_CLUSTER = 8, SPLIT_W_MAX = SPLIT_W_CLUSTER * 256 * 32;
+__global__ void __launch_bounds__(256) split2_wide_rows_kernel(TcSrc s, int rows, int cols, __half* __restrict__ pl, float* __restrict__ inv_scale, int ldp, float* __restrict__ rownorm, int cs) {
+  __shared__ float red[2][8], part[2];
+  const int z = blockIdx.y, rank = blockIdx.x % cs, lane = threadIdx.x & 31, warp = threadIdx.x >> 5; const long r = blockIdx.x / cs;
+  if (s.first && z % s.batch2 < s.first[z / s.batch2]) return;
+  const float* src = s.p + (z / s.batch2) * s.b1 + (z % s.batch2) * s.b2 + r * s.s_r;
+  const int seg = s.seg ? s.seg : cols; const long over = s.seg ? s.seg_stride - s.seg : 0;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(over * 4)) & 15) == 0;
+  float t[4][8], mx = 0.f, sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = 8 * ((i * cs + rank) * 256 + (int)threadIdx.x); const float* q = src + c + (over ? c / seg * over : 0);
+    if (vec && c + 7 < cols) {
+      const float4 a = *reinterpret_cast<const float4*>(q), b = *reinterpret_cast<const float4*>(q + 4);
+      t[i][0] = a.x; t[i][1] = a.y; t[i][2] = a.z; t[i][3] = a.w; t[i][4] = b.x; t[i][5] = b.y; t[i][6] = b.z; t[i][7] = b.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; j++) t[i][j] = c + j < cols ? q[j] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) { mx = fmaxf(mx, fabsf(t[i][j])); sq = fmaf(t[i][j], t[i][j], sq); }
+  }
+  mx = warp_max(mx); sq = warp_sum(sq);
+  if (lane == 0) { red[0][warp] = mx; red[1][warp] = sq; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) { mx = fmaxf(mx, red[0][w]); sq += red[1][w]; }
+    part[0] = mx; part[1] = sq;
+  }
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  mx = sq = 0.f;
+  for (int k = 0; k < cs; k++) { const float* q = cluster.map_shared_rank(part, k); mx = fmaxf(mx, q[0]); sq += q[1]; }
+  cluster.sync();                                           // (nobody leaves while its part is being read)
+  float inv; const float sc = row_scale(mx, &inv);
+  if (rank == 0 && threadIdx.x == 0) { inv_scale[(long)z * rows + r] = inv; if (rownorm) rownorm[(long)z * rows + r] = sqrtf(sq) * 1.0001f; }
+  __half* o = pl + ((long)z * rows + r) * 2 * ldp;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = 8 * ((i * cs + rank) * 256 + (int)threadIdx.x);
+    if (c < ldp) {
+      uint4 a, b;
+      split2_pair(t[i][0], t[i][1], sc, a.x, b.x); split2_pair(t[i][2], t[i][3], sc, a.y, b.y); split2_pair(t[i][4], t[i][5], sc, a.z, b.z); split2_pair(t[i][6], t[i][7], sc, a.w, b.w);
+      *reinterpret_cast<uint4*>(o + pl_off(c)) = a;
+      *reinterpret_cast<uint4*>(o + pl_off(c) + PL_LO) = b;
+    }
+  }
+}
 // Largest magnitude of every plane row of a transposed operand (= of every column of the stored matrix): a block covers
 // 64 plane rows x 256 contraction indices, reads run along the stored matrix's fast index, one atomicMax per row and block
 // on the bit pattern (non-negative floats order like integers).  `mx` must be zero on entry.
@@ -842,7 +894,10 @@ inline int tc_split(Ctx* ctx, const TcSrc& src, const BfPlanes& p, int* mx, floa
   if (rownorm && src.s_c != 1) return fail(GN_ERR_UNSUPPORTED, "tc_split: row norms are only formed by the row-wise split");
   if (src.s_c == 1) {
     if (p.nbatch > 65535) return fail(GN_ERR_UNSUPPORTED, "tc_split: more than 65535 problems in a batch");
-    GN_LAUNCH(ctx, split2_rows_kernel, dim3(cdiv(p.rows, 8), p.nbatch), 256, 0, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, rownorm);
+    if ((long)p.rows * p.nbatch <= ctx->sm_count && p.ldp >= 2048 && p.ldp <= SPLIT_W_MAX) {
+      int cs = 1; while (cs < SPLIT_W_CLUSTER && p.ldp > cs * 256 * 8) cs *= 2;      // eight elements a thread where that takes no more than eight blocks
+      GN_CLUSTER_LAUNCH(ctx, split2_wide_rows_kernel, dim3(p.rows * cs, p.nbatch), 256, 0, cs, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, rownorm, cs);
+    } else GN_LAUNCH(ctx, split2_rows_kernel, dim3(cdiv(p.rows, 8), p.nbatch), 256, 0, src, p.rows, p.K, p.base, p.inv_scale, p.ldp, rownorm);
   } else if (src.s_r == 1) {
     if (p.nbatch > 65535 || cdiv(p.rows, 64) > 65535 || cdiv(p.K, 256) > 65535) return fail(GN_ERR_UNSUPPORTED, "tc_split: operand too large for the transposing split");
     if (p.ldp <= SPLIT_T_MAX) {

@@ -47,6 +47,26 @@ def test_tc_gemm_matches_fp64(device, M, N, K):
     assert e_tc < 3e-5
 
 
+@pytest.mark.parametrize("M,K", [(1, 2017), (3, 2016), (148, 2048), (149, 2048), (64, 2049), (64, 2080), (5, 16384), (7, 16387), (2, 65536), (2, 65537)])
+def test_tc_gemm_few_long_rows(device, M, K):
+    """Few, long rows of A are split by a cluster of blocks per row: the edges of one to eight blocks, of eight elements per thread and of the
+    longest row it takes (shorter ones, the next length and one row more than there are SMs go the general way); rows of very different
+    magnitudes, one of zeros.  The bound is that of the shapes above, row by row."""
+    rng = np.random.default_rng(M + K)
+    A = (rng.standard_normal((M, K)) * 10.0 ** rng.integers(-6, 7, size=(M, 1))).astype(np.float32)
+    A[:, -1] *= 50
+    if M > 2:
+        A[1] = 0
+    B = rng.standard_normal((96, K)).astype(np.float32)
+    ref = A.astype(np.float64) @ B.astype(np.float64).T
+    tc, simt = _gemm(device, 1, A, B, None), _gemm(device, 0, A, B, None)
+    for m in range(M):
+        if m == 1 and M > 2:
+            assert not tc[m].any()
+        else:
+            assert norm_err(tc[m], ref[m]) <= 2e-6 + 4 * norm_err(simt[m], ref[m]) + 5e-9 * K, m
+
+
 def test_tc_gemm_exact_small_integers(device):
     # small integer-valued operands are exact in BF16: the result must be exact
     rng = np.random.default_rng(3)
