@@ -1064,6 +1064,7 @@ inline int tc_run_slices(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const T
   TcParams es = ep;
   es.k_slice = tc_slice_length(ep.K, splits); es.splits = cdiv(ep.K, es.k_slice);
   es.C = part; es.ldc = ep.N; es.c_b1 = (long)ep.M * ep.N; es.c_b2 = 0; es.batch2 = 1; es.bias = nullptr; es.R = nullptr; es.mask = nullptr; es.act = GN_ACT_LINEAR;
+  es.z_first = nullptr;                                     // goes by problems, and z counts the slices of the only one
   GN_TRY(tc_launch(ctx, A, B, es, ep.N <= 64 ? 64 : bn));
   GN_LAUNCH(ctx, tc_sum_slices_kernel, (unsigned)std::min<long>(cdiv((long)ep.M * ep.N, 1024), 4L * ctx->sm_count), 256, 0, (const float*)part, es.splits, ep.M, ep.N, ep);
   return check_launch("tc_sum_slices");

@@ -21,6 +21,7 @@ def device():
     ("lstm", 3, 1, 5, 3, 1, False), ("lstm", 4, 31, 9, 5, 1, True), ("lstm", 5, 33, 4, 149, 1, False), ("lstm", 6, 127, 3, 300, 1, False),
     ("lstm", 6, 128, 2, 151, 3, False), ("lstm", 2, 129, 3, 4, 1, False), ("lstm", 2, 160, 2, 150, 1, False), ("lstm", 1, 224, 2, 3, 1, False),
     ("lstm", 300, 9, 3, 100, 1, False),                  # a gradient wider than one column tile of the clipping kernel
+    ("lstm", 4096, 8, 8, 8, 1, False),                   # a single group whose Gram product over the inputs is cut into slices
     ("lstm", 7, 20, 64, 2, 1, False),                    # one whole group
     ("lstm", 7, 20, 43, 3, 1, False),                    # 129 updates: a group of one
     ("lstm", 7, 20, 40, 10, 1, False), ("lstm", 7, 20, 40, 10, 4, False), ("lstm", 7, 20, 13, 21, 10, False),      # several groups; short last chunks; more than eight chunks
