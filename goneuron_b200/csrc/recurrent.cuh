@@ -317,8 +317,8 @@ inline int gru_bwd_reg(Ctx* ctx, const float* gout, const float* Wh, const float
 // walk starts from zero at the first group that can be seen in the result (lstm_clip_start_kernel), at group 0 if there is none,
 // or if any update is not finite.  Gradients that are carried back through many steps grow by orders of magnitude per sequence
 // (median |u| 2e5 for 64 steps of 128 units), and a few dozen updates decide the result.  What is not walked is not gathered and
-// has no Gram blocks either: that step of 256 samples went from 1777 us to 667 without the walk and to 578 without the rest.
-// Where nothing can be left out the two launches that look for the start cost about 12 us.
+// has no Gram blocks either: that step of 256 samples, on a batch in device memory, went from 1682 us to 496.  Where nothing can be left
+// out it takes 1685: the norms and the search take 8 us, and the rows of zeros come without launches of their own.
 constexpr int CG = 128, CG_THREADS = 512, CG_PAD = CG, CG_TILE = 160;        // CG_PAD: rows of zeros before a chunk: group -1
 constexpr int CG_GD = CG + 1;
 constexpr long CG_MAX_K = 1L << 20;                         // updates per worker chunk
@@ -328,23 +328,35 @@ inline size_t clip_smem(int ZW) {
   const int wp = clip_tile(ZW) | 1; const size_t slab = ((size_t)2 * CG * wp + CG * 8 + (size_t)wp * 8 + 8) * sizeof(float), walk = (size_t)CG * CG_GD * sizeof(double);
   return slab > walk ? slab : walk;
 }
-// Rows of Dm [., 4H] and Zm [., zs]: chunk c's updates from row c * stride + lead on.  k: update in global order.
-__global__ void lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
-                                           int T, int in, int H, int zs, long n_updates, long Kc, long stride, long lead, const int* __restrict__ start) {
+// Rows of Dm [., 4H] and Zm [., zs], a block each: chunk c's updates from row c * stride + lead on, zeros in the rows before and behind them.
+// (Zeroing those rows separately took two to four more launches per chunk.)  `un` (may be null): receives |u_k|^2 = |d_k|^2 |z_k|^2.
+__global__ void __launch_bounds__(128) lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
+                                           int T, int in, int H, int zs, long n_updates, long Kc, long stride, long lead, const int* __restrict__ start, float* __restrict__ un) {
+  __shared__ float part[2][4];
   const int R4 = 4 * H, ZW = in + H + 1;
-  const long k = blockIdx.x; if (k >= n_updates) return;
-  if (start && k % Kc < (long)(start[k / Kc] - 1) * CG) return;               // before the first walked group and the one it is multiplied with
-  const int s = (int)(k / T), t = T - 1 - (int)(k % T); const long row = (k / Kc) * stride + lead + k % Kc;
+  const long row = blockIdx.x, chunk = row / stride, r = row - chunk * stride - lead, k = chunk * Kc + r;
+  if (start && r < (long)(start[chunk] - 1) * CG) return;                     // before the first walked group and the one it is multiplied with
+  if (r < 0 || r >= Kc || k >= n_updates) {
+    for (int e = threadIdx.x; e < R4 + zs; e += blockDim.x) { if (e < R4) Dm[row * R4 + e] = 0.f; else Zm[row * zs + e - R4] = 0.f; }
+    return;
+  }
+  const int s = (int)(k / T), t = T - 1 - (int)(k % T); float d2 = 0.f, z2 = 0.f;
   for (int e = threadIdx.x; e < R4 + zs; e += blockDim.x) {
-    if (e < R4) Dm[row * R4 + e] = D[((long)s * T + t) * R4 + e];
+    float v;
+    if (e < R4) { v = D[((long)s * T + t) * R4 + e]; Dm[row * R4 + e] = v; d2 = fmaf(v, v, d2); }
     else {
-      const int c = e - R4; float v;
+      const int c = e - R4;
       if (c < in) v = x[(long)s * T * in + (long)(T - 1) * in + c];                 // input of the LAST forward call (lstm.go:592-621)
       else if (c < in + H) v = t > 0 ? h_all[((long)s * T + (t - 1)) * H + (c - in)] : 0.f;
       else v = c < ZW ? 1.f : 0.f;
-      Zm[row * zs + c] = v;
+      Zm[row * zs + c] = v; z2 = fmaf(v, v, z2);
     }
   }
+  if (!un) return;
+  d2 = warp_sum(d2); z2 = warp_sum(z2);
+  if ((threadIdx.x & 31) == 0) { part[0][threadIdx.x >> 5] = d2; part[1][threadIdx.x >> 5] = z2; }
+  __syncthreads();
+  if (threadIdx.x == 0) un[k] = ((part[0][0] + part[0][1]) + (part[0][2] + part[0][3])) * ((part[1][0] + part[1][1]) + (part[1][2] + part[1][3]));
 }
 // rows of `w` floats from contiguous order into the chunks' layout (after a gather over the ranks)
 __global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int w, long Kc, long stride, long lead) {
@@ -353,15 +365,15 @@ __global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __r
 }
 __global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restrict__ G2, long total4, int groups, const int* __restrict__ start) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total4; i += (long)gridDim.x * blockDim.x) {
-    const int j = (int)(i / (CG * CG / 2)); if (j % groups < start[j / groups]) continue;
+    const int j = (int)(i / (CG * CG / 2)); if (start && j % groups < start[j / groups]) continue;
     float4 a = reinterpret_cast<float4*>(G)[i]; const float4 b = reinterpret_cast<const float4*>(G2)[i];
     a.x *= b.x; a.y *= b.y; a.z *= b.z; a.w *= b.w; reinterpret_cast<float4*>(G)[i] = a;
   }
 }
-constexpr int CLIP_FORGET = 128;
+constexpr int CLIP_FORGET = 128, CLIP_FEW = 32;
 constexpr float CLIP_FINITE = 1e36f;                        // squared norms above this count as not finite
-// |u_k|^2 = |d_k|^2 |z_k|^2 of every update, in update order; a warp each.  From the layer's own arrays (d, x, h as in
-// lstm_gather_updates_kernel below), so that updates that are not walked need not be gathered.
+// |u_k|^2 of every update, in update order; a warp each.  From the layer's own arrays (d, x, h as in lstm_gather_updates_kernel), so that
+// updates that are not walked need not be gathered.
 __global__ void __launch_bounds__(256) lstm_update_norms_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ un, int T, int in, int H, long n_updates) {
   const long k = blockIdx.x * 8L + (threadIdx.x >> 5); const int lane = threadIdx.x & 31; if (k >= n_updates) return;
   const long s = k / T; const int t = T - 1 - (int)(k % T); float d2 = 0.f, z2 = 0.f;
@@ -414,7 +426,7 @@ struct ClipArgs {
   const float *D, *Z, *G;        // rows of a chunk start at chunk * stride (CG_PAD rows of zeros first); G [chunk][group][CG][2 CG]: against groups j-1, j
   double *om, *p, *st;           // [chunk][groups][CG] weights of a group's updates; [chunk][2][CG][slabs] parts of p by parity of the group; [chunk][groups][2]: s_j, |g|^2
   float* g;                      // [chunk][2][4H][ZW]
-  const int* start;              // [chunk] first group to walk
+  const int* start;              // [chunk] first group to walk; null: group 0
   int R4, ZW, groups, slabs; long stride;
 };
 __global__ void __launch_bounds__(CG_THREADS) lstm_clip_kernel(const ClipArgs a, int j) {
@@ -426,7 +438,7 @@ __global__ void __launch_bounds__(CG_THREADS) lstm_clip_kernel(const ClipArgs a,
   // The same goes for the first group to walk.  A launch before it has nothing to do and nothing to wait for: the next one is let
   // in when its blocks are gone.
   if (j == 0) pdl_wait();
-  const int j0 = a.start[chunk];
+  const int j0 = a.start ? a.start[chunk] : 0;
   if (j < j0) return;
   if (blockIdx.x == 0) {
     if (j >= a.groups) { pdl_wait(); return; }

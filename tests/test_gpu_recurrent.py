@@ -49,25 +49,26 @@ def test_recurrent_parity(device, oracle, net, I, H, T, batch, W, seq):
     model.Close()
 
 
-@pytest.mark.parametrize("scale,W", [(1e-6, 1), (1e-2, 1), (1.0, 1), (1e4, 1), (1e4, 4), ("early", 1), ("early", 2), ("late", 1)])
-def test_clipping_walk_starts_where_the_result_can_still_see(device, oracle, scale, W):
-    """800 updates in seven groups (four chunks of 200, two of 400): nothing is clipped, some of it is, the last dozens of updates decide the
-    result, or one sample's do -- an early one, whose group has to be walked although later groups only add small
-    updates, or one in the last group."""
+@pytest.mark.parametrize("scale,W,batch", [(1e-6, 1, 20), (1e-2, 1, 20), (1.0, 1, 20), (1e4, 1, 20), (1e4, 4, 20), ("early", 1, 20), ("early", 2, 20), ("late", 1, 20),
+                                           (1e-6, 1, 160), (1e4, 1, 160), ("early", 1, 160), ("late", 1, 160), (1e-6, 40, 160), (1e4, 40, 160), ("early", 40, 160)])
+def test_clipping_walk_starts_where_the_result_can_still_see(device, oracle, scale, W, batch):
+    """800 updates in seven groups (four chunks of 200, two of 400), 6400 in fifty, forty chunks of 160: nothing is clipped, some of it is,
+    the last dozens of updates decide the result, or one sample's do -- an early one, whose group has to be walked although later
+    groups only add small updates, or one in the last group."""
     from goneuron_b200.sequential import Adam, Sequential
     layers = [D.SequenceUnrollerLSTM(7, 20, 40, False), D.Dense(20, 2, D.LINEAR)]
     rng = np.random.Generator(np.random.PCG64(5))
     params = configs.init_params(layers, rng)
-    x, y = configs.make_inputs("lstm", layers, 20, rng)
+    x, y = configs.make_inputs("lstm", layers, batch, rng)
     if isinstance(scale, str):
         y *= 1e-4
-        y[2 if scale == "early" else 19] *= 1e9
+        y[2 if scale == "early" else batch - 1] *= 1e9
     else:
         y *= scale
     ref = oracle.OracleState(layers, D.MSE, params, lr=1e-3)
     lit = oracle.OracleState(layers, D.MSE, params, lr=1e-3)
     ref.train_batch(x, y, W=W, threads=4, precision=64)
-    lit.train_batch(x, y, W=W, threads=W, precision=32)
+    lit.train_batch(x, y, W=W, threads=min(W, 8), precision=32)
     model = Sequential(layers, device, virtual_workers=W).Compile(Adam(1e-3), D.MSE)
     model.SetParams(params)
     model.TrainBatch(x, y)
