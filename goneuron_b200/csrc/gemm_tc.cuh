@@ -977,7 +977,7 @@ inline int tc_launch(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcPar
   if (ep.mask) vec = vec && ep.mask_ld % 4 == 0 && a16(ep.mask);
   if (ep.nchw_P > 0) { if (ep.R || A.nbatch != 1) return fail(GN_ERR_UNSUPPORTED, "tc_launch: NCHW store with a residual or a batch"); vec = false; }
   if (ep.out_p) {
-    if (!(ep.N % 32 == 0 && ep.out_ldp % 32 == 0 && (reinterpret_cast<uintptr_t>(ep.out_p) & 31) == 0 && (!ep.bias || a16(ep.bias)) && a16(ep.isb) && (!ep.mask || (ep.mask_ld % 4 == 0 && a16(ep.mask))) && (!ep.c_last || a16(ep.c_last)) && (!ep.z_last || a16(ep.z_last))))
+    if (!(ep.N % 32 == 0 && ep.out_ldp % 32 == 0 && (reinterpret_cast<uintptr_t>(ep.out_p) & 31) == 0 && (!ep.bias || a16(ep.bias)) && a16(ep.isb) && (!ep.mask || (ep.mask_ld % 4 == 0 && a16(ep.mask))) && (!ep.c_last || a16(ep.c_last)) && (!ep.z_last || a16(ep.z_last)) && (!ep.rowsum32 || a16(ep.rowsum32))))
       return fail(GN_ERR_INVALID_ARG, "tc_launch: plane output needs whole blocks of 32 columns and aligned operands");
     vec = true;
   }
