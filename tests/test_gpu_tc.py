@@ -51,7 +51,8 @@ def test_tc_gemm_matches_fp64(device, M, N, K):
 def test_tc_gemm_few_long_rows(device, M, K):
     """Few, long rows of A are split by a cluster of blocks per row: the edges of one to eight blocks, of eight elements per thread and of the
     longest row it takes (shorter ones, the next length and one row more than there are SMs go the general way); rows of very different
-    magnitudes, one of zeros.  The bound is that of the shapes above, row by row."""
+    magnitudes, one of zeros.  The bounds are those of the shapes above, row by row; with the low plane lost a row is off by about 2e-4
+    (each product by up to 2^-11, either way)."""
     rng = np.random.default_rng(M + K)
     A = (rng.standard_normal((M, K)) * 10.0 ** rng.integers(-6, 7, size=(M, 1))).astype(np.float32)
     A[:, -1] *= 50
@@ -64,7 +65,9 @@ def test_tc_gemm_few_long_rows(device, M, K):
         if m == 1 and M > 2:
             assert not tc[m].any()
         else:
-            assert norm_err(tc[m], ref[m]) <= 2e-6 + 4 * norm_err(simt[m], ref[m]) + 5e-9 * K, m
+            e_tc = norm_err(tc[m], ref[m])
+            assert e_tc <= 2e-6 + 4 * norm_err(simt[m], ref[m]) + 5e-9 * K, m
+            assert e_tc < 3e-5, m
 
 
 def test_tc_gemm_exact_small_integers(device):

@@ -16,19 +16,26 @@ CASES = [("mlp", {}, 64, 1), ("transformer_small", dict(vocab=512, dim=64, seq_l
          ("cnn", dict(hw=12, c0=2, c1=5, c2=7, classes=3), 10, 1),
          ("lstm", dict(in_size=5, hidden=24, seq_len=7), 12, 1),       # one worker chunk spans both ranks: update factors gathered, scan replicated
          ("lstm", dict(in_size=5, hidden=24, seq_len=7), 12, 4),       # worker chunks inside the ranks' shards
+         ("lstm", dict(in_size=5, hidden=24, seq_len=40), 40, 1),      # 13 groups of updates; with targets this large (_case) only the last ones are walked
          ("cnn_bn", dict(hw=10, c0=2, c1=5, classes=3), 8, 1),         # BatchNorm2D running statistics across ranks
          ("gru", dict(in_size=5, hidden=24, seq_len=7), 10, 1)]
+
+
+def _case(ci):
+    from goneuron_b200 import configs
+    name, kw, gb, W = CASES[ci]
+    layers, loss_kind, params, x, y, lr = configs.make_case(name, batch=gb, **kw)
+    return layers, loss_kind, params, x, y * 1e4 if kw.get("seq_len") == 40 else y, lr
 
 
 def _rank(rank, world, uid, out_dir):
     sys.path.insert(0, ROOT)
     os.environ["NCCL_NVLS_ENABLE"] = "0"
-    from goneuron_b200 import configs
     from goneuron_b200.sequential import Adam, Device, Sequential
     from goneuron_b200.sharding import shard_bounds
     dev = Device(rank, rank, world, uid)
     for ci, (name, kw, gb, W) in enumerate(CASES):
-        layers, loss_kind, params, x, y, lr = configs.make_case(name, batch=gb, **kw)
+        layers, loss_kind, params, x, y, lr = _case(ci)
         s, e = shard_bounds(gb, rank, world)
         model = Sequential(layers, dev, virtual_workers=W).Compile(Adam(lr), loss_kind)
         model.SetParams(params)
@@ -46,13 +53,12 @@ def test_two_gpu_data_parallel_step(tmp_path, oracle):
     if torch.cuda.device_count() < 2:
         pytest.skip("needs two GPUs")
     import torch.multiprocessing as mp
-    from goneuron_b200 import configs
     from goneuron_b200.sequential import Device
     from tests.parity import TOL, assert_grads_close, assert_weights_close, norm_err
     uid = Device.unique_id()
     mp.spawn(_rank, args=(2, uid, str(tmp_path)), nprocs=2, join=True)
     for ci, (name, kw, gb, W) in enumerate(CASES):
-        layers, loss_kind, params, x, y, lr = configs.make_case(name, batch=gb, **kw)
+        layers, loss_kind, params, x, y, lr = _case(ci)
         ref = oracle.OracleState(layers, loss_kind, params, lr=lr)
         l1 = ref.train_batch(x, y, W=W, threads=8, precision=64)
         g1, p1 = ref.grads.copy(), ref.params.copy()
