@@ -209,12 +209,13 @@ struct TcParams {
 // thread consecutive columns of one output row (TMEM lane = row); the chunk goes through `stg`, the warp's staging buffer of 32 rows
 // (16-byte units swizzled by the row: no bank conflicts either way), and comes back with eight (planes: four) neighbouring lanes on
 // a row and four columns of eight (four) rows per lane.  From there on an access to global memory touches four lines of 128 bytes (eight half
-// lines).  What a chunk reads -- column factors, residual, gate -- is fetched while the one before it is stored, the first chunk's
-// before the accumulator is waited for.
+// lines).  A chunk's column factors and residual, and for planes the gate where 32 rows have two gate rows at most (mask_group >= 32), are
+// fetched while the chunk before it is stored, the first chunk's before the accumulator is waited for; any other gate is read where it is applied.
 // (A thread that kept the row TMEM gave it and moved whole 32-byte sectors of it touched 32 lines per instruction: 1700 cycles to
 // store a chunk, 13 bytes per clock and SM; 9000 cycles for a 128 x 128 tile with a residual, as much as its MMAs over 384.  Now
 // about 4500.  [3072, 512] over 512 with a residual 13.7 -> 11.4 us, [3072, 1536] over 512 16.9 -> 15.5; as planes [3072, 2048] over
-// 512 23.6 -> 21.5, [3600, 1536] over 384 gated by factors 23.3 -> 20.1, with GELU 29.1 -> 28.4.)
+// 512 23.6 -> 21.5, [3600, 1536] over 384 gated by factors 23.3 -> 20.1, with GELU 29.1 -> 28.4.  Where the main loop hides the epilogue the
+// exchange takes shared-memory bandwidth from it: [16384, 1024] over 1024 77.6 -> 78.5, [32768, 3072] over 1024 431 -> 432.)
 // fp32 results go best with eight warps and unrolled rows; planes take twice the arithmetic per element and 16 warps (with eight,
 // GELU: 35 us).  The loops over chunks are not unrolled: a launch with one tile per CTA runs this code once, from a cold instruction cache.
 // acc[j] of column j of a chunk for this lane's row, times the row's inverse scale
@@ -672,8 +673,10 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(TcSrc s, int rows, int
 }
 // The same for few, long rows (the gradient of a head's output: 64 x 8192), where a warp per row leaves most SMs idle: a cluster of up to eight
 // blocks per row, every thread holding up to 32 of the row's elements in registers between the maximum and the planes.  Bound by
-// the latency of its loads and of one exchange through the cluster.  64 x 8192 took a warp per row 21 us with cold caches; a training step of the small causal
-// Transformer, which splits one such gradient, went from 742 to 730 us.  From 2048 columns on, where a warp walks its row eight times.
+// the latency of its loads and of one exchange through the cluster.  A training step of the small causal Transformer, which splits one such
+// gradient (64 x 8192), went from 742 to 730 us.  From 2048 columns on, where a warp walks its row eight times, and up to as many rows as
+// SMs.  us with cold caches, a warp per row -> this: 1 x 2048 6.2 -> 4.7, 148 x 2048 6.9 -> 4.8, 64 x 4096 10.8 -> 5.1, 64 x 8192 21 -> 5.4,
+// 148 x 8192 21 -> 8.6, 148 x 16384 40 -> 14, 1 x 65536 133 -> 6, 148 x 65536 152 -> 21.
 constexpr int SPLIT_W_CLUSTER = 8, SPLIT_W_MAX = SPLIT_W_CLUSTER * 256 * 32;
 __global__ void __launch_bounds__(256) split2_wide_rows_kernel(TcSrc s, int rows, int cols, __half* __restrict__ pl, float* __restrict__ inv_scale, int ldp, float* __restrict__ rownorm, int cs) {
   __shared__ float red[2][8], part[2];
@@ -1040,7 +1043,7 @@ __global__ void __launch_bounds__(256) tc_sum_slices_kernel(const float* __restr
   }
 }
 // Slices and tile width by estimated time, from measured rates (us): 0.335 / 0.43 per 32 contraction indices of a 128 / 256 wide
-// tile, 3 / 5 for the last tile's epilogue, 3 for the second launch and 4 TB/s for its partial results.  Slices keep at least 256
+// tile, 3 / 5 for the last tile's epilogue (2.4 / 3.9 since it stores whole lines; not tuned again), 3 for the second launch and 4 TB/s for its partial results.  Slices keep at least 256
 // indices, and have to win by a tenth.
 inline int tc_split_count(Ctx* ctx, const TcParams& ep, long nbatch, int* bn) {
   if (nbatch != 1 || ep.out_p || ep.n_seg || ep.nchw_P || ep.flags || ep.K < 1024 || ctx->tc_kslice > 0 || ctx->tc_force_bn) return 1;
