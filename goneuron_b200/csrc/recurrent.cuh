@@ -1,6 +1,7 @@
 // recurrent.cuh -- LSTM and GRU recurrences, forward and back-propagation through time, and the LSTM gradient-clipping recurrence.
 #pragma once
 #include <cooperative_groups.h>
+#include <type_traits>
 #include "common.cuh"
 #include "rowops.cuh"
 
@@ -8,49 +9,138 @@ namespace gn {
 
 // ------------------------------------------------------------------ recurrence kernels
 // A recurrence is a chain of T small matrix-vector products, bound by the latency of one step.  A block owns NS samples (two when
-// there are more samples than SMs) and has four threads per hidden unit, each with a quarter of the unit's dot product: a step
-// is a quarter of the multiply-adds in a row, one exchange through shared memory, and the activations.  For up to 128
-// hidden units a thread keeps its weights in registers for the whole sequence (RU_Q per matrix).  One thread per unit with the
-// weights in shared memory (forward) or L2 (backward) took 147 / 888 us for the LSTM of 128 units, 64 steps, 256 samples.
-constexpr int RU_Q = 32;
+// there are more samples than SMs).  For up to 128 hidden units (HB blocks of 32) a thread has C columns of the matrix and a 2 C-th
+// of the contraction, and keeps their weights for the whole sequence.  The 2 C threads of a column group are
+// neighbours in a warp: every 16 bytes of the vector that a lane fetches are used for C columns, and rounds of shuffles that halve what a lane
+// still holds leave every lane with the sum of ONE unit of ONE sample, the unit whose element-wise part it does.  A step is
+// that, and one barrier behind the new vector.
+// Four threads per unit, a column each, fetched four times as much of the vector (shared memory delivers 128 bytes per clock to
+// registers, broadcast or not: 4096 of the 5000 cycles of a backward step of the LSTM), and passed partial sums through shared memory behind a second
+// barrier.  us before -> now, 64 steps of 128 units, 256 samples: LSTM 65.6 -> 49 forward, 166 -> 80 backward, GRU 210 -> 94 and 122 -> 53; 100
+// samples: 49 -> 44, 123 -> 57, 143 -> 80 and 74 -> 49.  What is left of a step is its chain: 0.46 us for 32 units.
+// (fma.rn.f32x2, two rows at a time, is no faster here: LSTM backward, 96 units, 71.8 us against 63.5.)
 struct RecShape { int T, in, H, return_seq, B; };
 __host__ __device__ __forceinline__ int rec_hp(int H) { return (H + 31) & ~31; }
 __host__ __device__ __forceinline__ int rec_jq(int H) { return (((H + 3) / 4) + 3) & ~3; }        // length of a quarter, a multiple of 4
+constexpr int REC_REG_H = 128;                               // units up to which the register kernels go
+// Floats between the pieces (of ks values, a multiple of four) of a vector: an odd number of 16-byte units, so that they lie in different banks
+__host__ __device__ constexpr int rec_vs(int ks) { return ks | 4; }
 
-// dot product of a quarter: w . v over jq values; w in registers (REGS) or at ws[jj * ld]
-template <bool REGS>
-__device__ __forceinline__ float rec_dot(const float (&w)[RU_Q], const float* __restrict__ ws, int ld, const float* __restrict__ v, int jq) {
-  float a = 0.f, b = 0.f;
-  if (REGS) {
+// acc[s][c] += w[.][c] . v_s over R values; the samples' vectors are `vs` floats apart
+template <int NS, int R, int C>
+__device__ __forceinline__ void rec_fma(float (&acc)[NS][C], const float (&w)[R][C], const float* __restrict__ v, int vs) {
 #pragma unroll
-    for (int j = 0; j < RU_Q; j += 8) {
-      if (j < jq) { const float4 x = *reinterpret_cast<const float4*>(v + j); a = fmaf(w[j], x.x, a); b = fmaf(w[j + 1], x.y, b); a = fmaf(w[j + 2], x.z, a); b = fmaf(w[j + 3], x.w, b); }
-      if (j + 4 < jq) { const float4 x = *reinterpret_cast<const float4*>(v + j + 4); a = fmaf(w[j + 4], x.x, a); b = fmaf(w[j + 5], x.y, b); a = fmaf(w[j + 6], x.z, a); b = fmaf(w[j + 7], x.w, b); }
+  for (int r = 0; r < R; r += 4) {
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+      const float4 x = *reinterpret_cast<const float4*>(v + s * vs + r);
+#pragma unroll
+      for (int c = 0; c < C; c++) acc[s][c] = fmaf(w[r + 3][c], x.w, fmaf(w[r + 2][c], x.z, fmaf(w[r + 1][c], x.y, fmaf(w[r][c], x.x, acc[s][c]))));
     }
-  } else {
-#pragma unroll 4
-    for (int j = 0; j < jq; j += 2) { a = fmaf(ws[j * ld], v[j], a); b = fmaf(ws[(j + 1) * ld], v[j + 1], b); }
   }
-  return a + b;
 }
+// The sums over the 2 C threads of a column group; lane C s + c of the group receives column c of sample s (NS = 1: so do lanes C + c)
+template <int NS, int C>
+__device__ __forceinline__ float rec_reduce(const float (&acc)[NS][C], int lane) {
+  float v[NS * C];
+#pragma unroll
+  for (int s = 0; s < NS; s++)
+#pragma unroll
+    for (int c = 0; c < C; c++) v[C * s + c] = acc[s][c];
+  if (NS == 1) {                               // (the order of a sample's sums does not depend on NS)
+#pragma unroll
+    for (int c = 0; c < C; c++) v[c] += __shfl_xor_sync(0xffffffffu, v[c], C);
+  }
+#pragma unroll
+  for (int h = NS * C / 2; h >= 1; h >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int k = 0; k < h; k++) { const float give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k]; v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h); }
+  }
+  return v[0];
+}
+template <int NS, int C> __device__ __forceinline__ void rec_clear(float (&acc)[NS][C]) {
+#pragma unroll
+  for (int s = 0; s < NS; s++)
+#pragma unroll
+    for (int c = 0; c < C; c++) acc[s][c] = 0.f;
+}
+// Rows k .. k + 3 (k a multiple of four) of columns col0 .. col0 + C - 1 of a matrix [H, H], zero outside.  KFAST: element (row k, column c)
+// lies at m[c * H + k], else at m[k * H + c].  `vec`: H is a multiple of four and m 16-byte aligned.
+template <bool KFAST, int C>
+__device__ __forceinline__ void rec_weights(float (*w)[C], const float* __restrict__ m, int H, int k, int col0, bool vec) {
+#pragma unroll
+  for (int c4 = 0; c4 < C; c4 += 4)
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      const int slow = KFAST ? col0 + c4 + a : k + a, fast = KFAST ? k : col0 + c4; const float* q = m + (long)slow * H + fast; float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (slow < H && fast < H) {
+        if (vec) { const float4 y = *reinterpret_cast<const float4*>(q); x[0] = y.x; x[1] = y.y; x[2] = y.z; x[3] = y.w; }
+        else { x[0] = q[0]; if (fast + 1 < H) x[1] = q[1]; if (fast + 2 < H) x[2] = q[2]; if (fast + 3 < H) x[3] = q[3]; }
+      }
+#pragma unroll
+      for (int b = 0; b < 4; b++) w[KFAST ? b : a][c4 + (KFAST ? a : b)] = x[b];
+    }
+}
+__device__ __forceinline__ bool rec_vec(const float* m, int H) { return ((reinterpret_cast<uintptr_t>(m) | (uintptr_t)(H * 4)) & 15) == 0; }
+// This thread's part of the recurrence: column group, piece of the contraction, and the (sample, unit) whose element-wise part it does
+template <int NS, int C> struct RecLane {
+  int lane, sp, col0, unit, es; long s; bool el;
+  __device__ __forceinline__ RecLane(int H, int B) {
+    lane = threadIdx.x & 31; sp = lane & (2 * C - 1); col0 = (threadIdx.x >> 5) * 16 + lane / (2 * C) * C; unit = col0 + (sp & (C - 1)); es = sp / C;
+    s = (long)blockIdx.x * NS + es; el = es < NS && unit < H && s < B;
+  }
+};
 
 // LSTM forward.  reference: lstm.go:276-407.  The reference's gate helpers (lstm.go:1065-1101) run over the first H of the 4H
 // pre-activation rows, so only the input gate receives Wx x + Wh h; forget, cell and output gates see their biases alone and
 // are constant over time.  `ig` holds the input projections Wx[0:H] x_t of every (sample, step) on entry (one contraction, issued
 // before) and the input gate on exit; cell, tanh(cell) and hidden states are kept too.
-template <int NS, bool REGS>
-__global__ void __launch_bounds__(REGS ? 512 : 1024) lstm_fwd_kernel(const float* __restrict__ Wh, const float* __restrict__ bias, float* __restrict__ ig_all, float* __restrict__ c_all,
-                                                                     float* __restrict__ tc_all, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
+template <int NS, int HB>
+__global__ void __launch_bounds__(64 * HB) lstm_fwd_reg_kernel(const float* __restrict__ Wh, const float* __restrict__ bias, float* __restrict__ ig_all, float* __restrict__ c_all,
+                                                               float* __restrict__ tc_all, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
+  constexpr int KS = 4 * HB, VS = rec_vs(KS);
+  __shared__ __align__(16) float hb[2][NS][8 * VS];
+  const int H = q_.H, T = q_.T; const RecLane<NS, 4> L(H, q_.B); const int i = L.unit;
+  float w[KS][4]; const bool vec = rec_vec(Wh, H);
+#pragma unroll
+  for (int k = 0; k < KS; k += 4) rec_weights<true, 4>(w + k, Wh, H, L.sp * KS + k, L.col0, vec);
+  for (int e = threadIdx.x; e < 2 * NS * 8 * VS; e += blockDim.x) hb[0][0][e] = 0.f;
+  float bi = 0.f, fg = 0.f, cg = 0.f, og = 0.f, c = 0.f, x = 0.f, x1 = 0.f;
+  const long base = L.s * T * H + i; const int at = i / KS * VS + i % KS;
+  if (L.el) {
+    bi = bias[i]; fg = act_fwd(GN_ACT_SIGMOID, bias[H + i]); cg = act_fwd(GN_ACT_TANH, bias[2 * H + i]); og = act_fwd(GN_ACT_SIGMOID, bias[3 * H + i]);
+    x = ig_all[base]; if (T > 1) x1 = ig_all[base + H];
+  }
+  __syncthreads();
+  for (int t = 0; t < T; t++) {
+    float acc[NS][4]; rec_clear(acc);
+    rec_fma(acc, w, &hb[t & 1][0][L.sp * VS], 8 * VS);
+    const float sum = rec_reduce(acc, L.lane);
+    if (L.el) {
+      const long o = base + (long)t * H;
+      const float pre = bi + x + sum;
+      x = x1; if (t + 2 < T) x1 = ig_all[o + 2 * H];               // two steps ahead: a step is about as long as a load
+      const float ig = act_fwd(GN_ACT_SIGMOID, pre);
+      c = fg * c + ig * cg;
+      const float tc = act_fwd(GN_ACT_TANH, c), h = og * tc;
+      hb[(t + 1) & 1][L.es][at] = h;
+      ig_all[o] = ig; c_all[o] = c; tc_all[o] = tc; h_all[o] = h;
+      if (q_.return_seq) out[o] = h; else if (t == T - 1) out[L.s * H + i] = h;
+    }
+    __syncthreads();
+  }
+}
+// ... of wider layers: four threads per unit, each with a quarter of its dot product, weights in shared memory
+template <int NS>
+__global__ void __launch_bounds__(1024) lstm_fwd_kernel(const float* __restrict__ Wh, const float* __restrict__ bias, float* __restrict__ ig_all, float* __restrict__ c_all,
+                                                        float* __restrict__ tc_all, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
   extern __shared__ __align__(16) float sm[];
   const int H = q_.H, T = q_.T, Hp = rec_hp(H), jq = rec_jq(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
   float* hb = sm;                              // [2][NS][4 jq]
   float* part = hb + 2 * NS * 4 * jq;          // [4][NS][Hp]
-  float* ws = part + 4 * NS * Hp;              // !REGS: [4 jq][Hp]
-  float w[RU_Q];
-  if (REGS) {
-#pragma unroll
-    for (int j = 0; j < RU_Q; j++) { const int k = q * jq + j; w[j] = (i < H && j < jq && k < H) ? Wh[(long)i * H + k] : 0.f; }
-  } else for (int e = threadIdx.x; e < 4 * jq * Hp; e += blockDim.x) { const int k = e / Hp, r = e - k * Hp; ws[e] = (r < H && k < H) ? Wh[(long)r * H + k] : 0.f; }
+  float* ws = part + 4 * NS * Hp;              // [4 jq][Hp]
+  for (int e = threadIdx.x; e < 4 * jq * Hp; e += blockDim.x) { const int k = e / Hp, r = e - k * Hp; ws[e] = (r < H && k < H) ? Wh[(long)r * H + k] : 0.f; }
   for (int e = threadIdx.x; e < 2 * NS * 4 * jq; e += blockDim.x) hb[e] = 0.f;
   // the elementwise part of (sample, unit): the first NS * Hp threads
   const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
@@ -63,8 +153,14 @@ __global__ void __launch_bounds__(REGS ? 512 : 1024) lstm_fwd_kernel(const float
   __syncthreads();
   for (int t = 0; t < T; t++) {
     const float* hp = hb + (t & 1) * NS * 4 * jq; float* hn = hb + ((t + 1) & 1) * NS * 4 * jq;
+    const float* wq = ws + (q * jq) * Hp + i;
 #pragma unroll
-    for (int k = 0; k < NS; k++) part[(q * NS + k) * Hp + i] = rec_dot<REGS>(w, ws + (q * jq) * Hp + i, Hp, hp + k * 4 * jq + q * jq, jq);
+    for (int k = 0; k < NS; k++) {
+      const float* v = hp + k * 4 * jq + q * jq; float a = 0.f, b = 0.f;
+#pragma unroll 4
+      for (int j = 0; j < jq; j += 2) { a = fmaf(wq[j * Hp], v[j], a); b = fmaf(wq[(j + 1) * Hp], v[j + 1], b); }
+      part[(q * NS + k) * Hp + i] = a + b;
+    }
     __syncthreads();
     if (el) {
       const long o = base + (long)t * H;
@@ -85,10 +181,123 @@ __global__ void __launch_bounds__(REGS ? 512 : 1024) lstm_fwd_kernel(const float
 
 // LSTM back-propagation through time; writes the gate deltas D[s, t, 4H].  reference: lstm.go:476-698 + unroller.go:190-209: the
 // hidden-state gradient handed to step t-1 is the gradient of step t PLUS Wh^T d (a running sum), because LSTM.Backward adds
-// dhPrev into its argument.  Thread (gate q, unit i) sums over gate q's H rows of column i: the first `rs` rows (a multiple of
-// four) from shared memory, the next RR from registers, the rest (none up to 128 units) from global memory.
-template <int NS, int RR, int MAXT>
-__global__ void __launch_bounds__(MAXT) lstm_bwd_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ bias, const float* __restrict__ ig_all,
+// dhPrev into its argument.
+// Element-wise part, for one (sample, unit)
+struct LstmBwdUnit {
+  float cur = 0.f, dcn = 0.f, fg = 0.f, cg = 0.f, og = 0.f, kf = 0.f, kg = 0.f, ko = 0.f, ig = 0.f, tc = 0.f, cp = 0.f;
+  __device__ __forceinline__ void init(const float* bias, const float* gout, const float* ig_all, const float* c_all, const float* tc_all, const RecShape& q, long s, int i, long base) {
+    const int H = q.H, T = q.T; const float bf = bias[H + i], bg = bias[2 * H + i], bo = bias[3 * H + i];
+    fg = act_fwd(GN_ACT_SIGMOID, bf); cg = act_fwd(GN_ACT_TANH, bg); og = act_fwd(GN_ACT_SIGMOID, bo);
+    kf = act_der(GN_ACT_SIGMOID, bf); kg = act_der(GN_ACT_TANH, bg); ko = act_der(GN_ACT_SIGMOID, bo);
+    const long o = base + (long)(T - 1) * H;
+    ig = ig_all[o]; tc = tc_all[o]; cp = T > 1 ? c_all[o - H] : 0.f;
+    if (!q.return_seq) cur = gout[s * H + i];
+  }
+  __device__ __forceinline__ void step(float& di, float& df, float& dg, float& dq) {
+    const float dc = cur * og * (1.f - tc * tc) + dcn;
+    di = dc * cg * (ig * (1.f - ig)); df = dc * cp * kf; dg = dc * ig * kg; dq = cur * tc * ko;
+    dcn = dc * fg;
+  }
+};
+// Up to 128 units, the matrix [4 Hp, H]: two columns out of 16 per piece of 8 HB rows.  Beyond 96 units a thread's 256 weights do not fit its
+// registers: the last 12 of its 32 rows lie in tensor memory, from where they come four rows at a time while rows from registers
+// are multiplied (from shared memory, which the vectors keep busy already: 96 us instead of 80, 100 samples 80 instead of 57).
+constexpr int LB_TM_ROWS = 12, LB_TM_COLS = 256;             // columns: 2 x 12 x 8 (two warps share a quarter of the lanes), a power of two
+__device__ __forceinline__ void rec_tm_load(float (&w)[4][8], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=f"(w[0][0]), "=f"(w[0][1]), "=f"(w[0][2]), "=f"(w[0][3]), "=f"(w[0][4]), "=f"(w[0][5]), "=f"(w[0][6]), "=f"(w[0][7]),
+        "=f"(w[1][0]), "=f"(w[1][1]), "=f"(w[1][2]), "=f"(w[1][3]), "=f"(w[1][4]), "=f"(w[1][5]), "=f"(w[1][6]), "=f"(w[1][7]),
+        "=f"(w[2][0]), "=f"(w[2][1]), "=f"(w[2][2]), "=f"(w[2][3]), "=f"(w[2][4]), "=f"(w[2][5]), "=f"(w[2][6]), "=f"(w[2][7]),
+        "=f"(w[3][0]), "=f"(w[3][1]), "=f"(w[3][2]), "=f"(w[3][3]), "=f"(w[3][4]), "=f"(w[3][5]), "=f"(w[3][6]), "=f"(w[3][7])
+      : "r"(addr) : "memory");
+}
+// (the registers are operands: nothing that uses them moves ahead of the wait)
+__device__ __forceinline__ void rec_tm_wait(float (&w)[4][8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+      : "+f"(w[0][0]), "+f"(w[0][1]), "+f"(w[0][2]), "+f"(w[0][3]), "+f"(w[0][4]), "+f"(w[0][5]), "+f"(w[0][6]), "+f"(w[0][7]),
+        "+f"(w[1][0]), "+f"(w[1][1]), "+f"(w[1][2]), "+f"(w[1][3]), "+f"(w[1][4]), "+f"(w[1][5]), "+f"(w[1][6]), "+f"(w[1][7]),
+        "+f"(w[2][0]), "+f"(w[2][1]), "+f"(w[2][2]), "+f"(w[2][3]), "+f"(w[2][4]), "+f"(w[2][5]), "+f"(w[2][6]), "+f"(w[2][7]),
+        "+f"(w[3][0]), "+f"(w[3][1]), "+f"(w[3][2]), "+f"(w[3][3]), "+f"(w[3][4]), "+f"(w[3][5]), "+f"(w[3][6]), "+f"(w[3][7])
+      :: "memory");
+}
+__device__ __forceinline__ void rec_tm_store(const float (&w)[4][8], uint32_t addr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};"
+      :: "f"(w[0][0]), "f"(w[0][1]), "f"(w[0][2]), "f"(w[0][3]), "f"(w[0][4]), "f"(w[0][5]), "f"(w[0][6]), "f"(w[0][7]),
+         "f"(w[1][0]), "f"(w[1][1]), "f"(w[1][2]), "f"(w[1][3]), "f"(w[1][4]), "f"(w[1][5]), "f"(w[1][6]), "f"(w[1][7]),
+         "f"(w[2][0]), "f"(w[2][1]), "f"(w[2][2]), "f"(w[2][3]), "f"(w[2][4]), "f"(w[2][5]), "f"(w[2][6]), "f"(w[2][7]),
+         "f"(w[3][0]), "f"(w[3][1]), "f"(w[3][2]), "f"(w[3][3]), "f"(w[3][4]), "f"(w[3][5]), "f"(w[3][6]), "f"(w[3][7]), "r"(addr) : "memory");
+}
+template <int NS, int HB>
+__global__ void __launch_bounds__(64 * HB) lstm_bwd_reg_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ bias, const float* __restrict__ ig_all,
+                                                               const float* __restrict__ c_all, const float* __restrict__ tc_all, float* __restrict__ D, const RecShape q_) {
+  constexpr int C = 8, KS = 8 * HB, VS = rec_vs(KS), TR = HB == 4 ? LB_TM_ROWS : 0, RR = KS - TR, HALF = RR / 8 * 4;
+  __shared__ __align__(16) float db[2][NS][2 * C * VS];
+  __shared__ uint32_t tm_slot;
+  const int H = q_.H, T = q_.T, warp = threadIdx.x >> 5; const RecLane<NS, C> L(H, q_.B); const int i = L.unit;
+  if (TR > 0 && warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&tm_slot)), "r"(LB_TM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  const float* wg = Wh + (long)(L.sp >> 2) * H * H; const int k0 = (L.sp & 3) * KS; const bool vec = rec_vec(wg, H);      // (four pieces per gate)
+  float w1[HALF][C], w2[RR - HALF][C], wt[4][C];
+#pragma unroll
+  for (int k = 0; k < HALF; k += 4) rec_weights<false, C>(w1 + k, wg, H, k0 + k, L.col0, vec);
+#pragma unroll
+  for (int k = HALF; k < RR; k += 4) rec_weights<false, C>(w2 + (k - HALF), wg, H, k0 + k, L.col0, vec);
+  for (int e = threadIdx.x; e < 2 * NS * 2 * C * VS; e += 64 * HB) db[0][0][e] = 0.f;
+  LstmBwdUnit u; const long base = L.s * T * H + i;
+  if (L.el) u.init(bias, gout, ig_all, c_all, tc_all, q_, L.s, i, base);
+  float n_ig = 0.f, n_tc = 0.f, n_cp = 0.f;                  // the next step's: loaded two steps ahead, a load takes about as long as a short step
+  auto ahead = [&](int t) { const long o = base + (long)t * H; n_ig = ig_all[o]; n_tc = tc_all[o]; n_cp = t > 0 ? c_all[o - H] : 0.f; };
+  if (L.el && T > 1) ahead(T - 2);
+  if (TR > 0) tc_fence_before();
+  __syncthreads();
+  if (TR > 0) tc_fence_after();
+  const uint32_t tm = TR > 0 ? tm_slot + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * TR * C : 0;
+  if constexpr (TR > 0) {
+#pragma unroll
+    for (int k = 0; k < TR; k += 4) { rec_weights<false, C>(wt, wg, H, k0 + RR + k, L.col0, vec); rec_tm_store(wt, tm + k * C); }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
+  auto unit_step = [&](int t) {
+    if (!L.el) return;
+    if (q_.return_seq) u.cur += gout[base + (long)t * H];
+    float di, df, dg, dq; u.step(di, df, dg, dq);
+    float* e = db[t & 1][L.es] + i / KS * VS + i % KS; e[0] = di; e[4 * VS] = df; e[8 * VS] = dg; e[12 * VS] = dq;
+    float* Dr = D + (L.s * T + t) * 4 * H + i; Dr[0] = di; Dr[H] = df; Dr[2 * H] = dg; Dr[3 * H] = dq;
+    u.ig = n_ig; u.tc = n_tc; u.cp = n_cp;
+    if (t > 1) ahead(t - 2);
+  };
+  for (int t = T - 1; t > 0; t--) {
+    if constexpr (TR > 0) rec_tm_load(wt, tm);               // (loads never reach across iterations: their registers are not to be moved before the wait)
+    unit_step(t);
+    __syncthreads();
+    float acc[NS][C]; rec_clear(acc);
+    const float* v = db[t & 1][0] + L.sp * VS; constexpr int vs = 2 * C * VS;
+    if constexpr (TR > 0) {
+      rec_tm_wait(wt); rec_fma(acc, wt, v + RR, vs); rec_tm_load(wt, tm + 4 * C);
+      rec_fma(acc, w1, v, vs);
+      rec_tm_wait(wt); rec_fma(acc, wt, v + RR + 4, vs); rec_tm_load(wt, tm + 8 * C);
+      rec_fma(acc, w2, v + HALF, vs);
+      rec_tm_wait(wt); rec_fma(acc, wt, v + RR + 8, vs);
+    } else { rec_fma(acc, w1, v, vs); rec_fma(acc, w2, v + HALF, vs); }
+    const float sum = rec_reduce(acc, L.lane);
+    if (L.el) u.cur += sum;
+  }
+  unit_step(0);
+  if constexpr (TR > 0) {
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_slot), "r"(LB_TM_COLS) : "memory");
+  }
+}
+// ... of wider layers.  Thread (gate q, unit i) sums over gate q's H rows of column i: the first `rs` rows (a multiple of four) from
+// shared memory, the next RR from registers, the rest from global memory.
+template <int NS, int RR>
+__global__ void __launch_bounds__(1024) lstm_bwd_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ bias, const float* __restrict__ ig_all,
                                                         const float* __restrict__ c_all, const float* __restrict__ tc_all, float* __restrict__ D, const RecShape q_, int rs) {
   extern __shared__ __align__(16) float sm[];
   const int H = q_.H, T = q_.T, Hp = rec_hp(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
@@ -101,27 +310,17 @@ __global__ void __launch_bounds__(MAXT) lstm_bwd_kernel(const float* __restrict_
   for (int j = 0; j < RR; j++) w[j] = (i < H && rs + j < H) ? Wh[((long)q * H + rs + j) * H + i] : 0.f;
   for (int e = threadIdx.x; e < NS * 4 * Hp; e += blockDim.x) db[e] = 0.f;
   const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
-  float cur = 0.f, dcn = 0.f, fg = 0.f, cg = 0.f, og = 0.f, kf = 0.f, kg = 0.f, ko = 0.f, ig = 0.f, tc = 0.f, cp = 0.f;
-  const long base = ((long)s * T) * H + i;
-  if (el) {
-    const float bf = bias[H + i], bg = bias[2 * H + i], bo = bias[3 * H + i];
-    fg = act_fwd(GN_ACT_SIGMOID, bf); cg = act_fwd(GN_ACT_TANH, bg); og = act_fwd(GN_ACT_SIGMOID, bo);
-    kf = act_der(GN_ACT_SIGMOID, bf); kg = act_der(GN_ACT_TANH, bg); ko = act_der(GN_ACT_SIGMOID, bo);
-    const long o = base + (long)(T - 1) * H;
-    ig = ig_all[o]; tc = tc_all[o]; cp = T > 1 ? c_all[o - H] : 0.f;
-    if (!q_.return_seq) cur = gout[(long)s * H + i];
-  }
+  LstmBwdUnit u; const long base = ((long)s * T) * H + i;
+  if (el) u.init(bias, gout, ig_all, c_all, tc_all, q_, s, i, base);
   __syncthreads();
   for (int t = T - 1; t >= 0; t--) {
     if (el) {
       const long o = base + (long)t * H;
-      if (q_.return_seq) cur += gout[o];
-      const float dc = cur * og * (1.f - tc * tc) + dcn;
-      const float di = dc * cg * (ig * (1.f - ig)), df = dc * cp * kf, dg = dc * ig * kg, dq = cur * tc * ko;
-      dcn = dc * fg;
+      if (q_.return_seq) u.cur += gout[o];
+      float di, df, dg, dq; u.step(di, df, dg, dq);
       float* d = db + es * 4 * Hp + i; d[0] = di; d[Hp] = df; d[2 * Hp] = dg; d[3 * Hp] = dq;
       float* Dr = D + ((long)s * T + t) * 4 * H + i; Dr[0] = di; Dr[H] = df; Dr[2 * H] = dg; Dr[3 * H] = dq;
-      if (t > 0) { ig = ig_all[o - H]; tc = tc_all[o - H]; cp = t > 1 ? c_all[o - 2 * H] : 0.f; }
+      if (t > 0) { u.ig = ig_all[o - H]; u.tc = tc_all[o - H]; u.cp = t > 1 ? c_all[o - 2 * H] : 0.f; }
     }
     if (t == 0) break;
     __syncthreads();
@@ -153,62 +352,50 @@ __global__ void __launch_bounds__(MAXT) lstm_bwd_kernel(const float* __restrict_
 #pragma unroll
     for (int k = 0; k < NS; k++) part[(q * NS + k) * Hp + i] = acc[k];
     __syncthreads();
-    if (el) cur += (part[es * Hp + i] + part[(NS + es) * Hp + i]) + (part[(2 * NS + es) * Hp + i] + part[(3 * NS + es) * Hp + i]);
+    if (el) u.cur += (part[es * Hp + i] + part[(NS + es) * Hp + i]) + (part[(2 * NS + es) * Hp + i] + part[(3 * NS + es) * Hp + i]);
   }
 }
 
 // GRU forward for up to 128 units.  reference: gru.go:192-288.  `gates` [B, T, 3H] holds b + Wx x_t of every step on entry (one
 // contraction over all rows, issued before) and the gate values z | r | candidate on exit.  The layer has 2H recurrent rows: the
 // candidate's recurrent product uses the reset gate's rows on r (.) h_prev (gru.go:247-258).
-template <int NS>
-__global__ void __launch_bounds__(512) gru_fwd_reg_kernel(const float* __restrict__ Wh, float* __restrict__ gates, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
-  extern __shared__ __align__(16) float sm[];
-  const int H = q_.H, T = q_.T, Hp = rec_hp(H), jq = rec_jq(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
-  float* hb = sm;                              // [NS][4 jq]  h_prev
-  float* rb = hb + NS * 4 * jq;                // [NS][4 jq]  r (.) h_prev
-  float* part = rb + NS * 4 * jq;              // [2][4][NS][Hp]
-  float wz[RU_Q], wr[RU_Q];
+template <int NS, int HB>
+__global__ void __launch_bounds__(64 * HB) gru_fwd_reg_kernel(const float* __restrict__ Wh, float* __restrict__ gates, float* __restrict__ h_all, float* __restrict__ out, const RecShape q_) {
+  constexpr int KS = 4 * HB, VS = rec_vs(KS);
+  __shared__ __align__(16) float hb[NS][8 * VS], rb[NS][8 * VS];      // h_prev, r (.) h_prev
+  const int H = q_.H, T = q_.T; const RecLane<NS, 4> L(H, q_.B); const int i = L.unit;
+  float wz[KS][4], wr[KS][4]; const bool vec = rec_vec(Wh, H);
 #pragma unroll
-  for (int j = 0; j < RU_Q; j++) {
-    const int k = q * jq + j; const bool in = i < H && j < jq && k < H;
-    wz[j] = in ? Wh[(long)i * H + k] : 0.f; wr[j] = in ? Wh[(long)(H + i) * H + k] : 0.f;
+  for (int k = 0; k < KS; k += 4) {
+    rec_weights<true, 4>(wz + k, Wh, H, L.sp * KS + k, L.col0, vec);
+    rec_weights<true, 4>(wr + k, Wh + (long)H * H, H, L.sp * KS + k, L.col0, vec);
   }
-  for (int e = threadIdx.x; e < 2 * NS * 4 * jq; e += blockDim.x) hb[e] = 0.f;
-  const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
-  float* gp = gates + (long)s * T * 3 * H + i; float h = 0.f, az = 0.f, ar = 0.f, ac = 0.f;
-  if (el) { az = gp[0]; ar = gp[H]; ac = gp[2 * H]; }
+  for (int e = threadIdx.x; e < NS * 8 * VS; e += blockDim.x) { hb[0][e] = 0.f; rb[0][e] = 0.f; }
+  float* gp = gates + L.s * T * 3 * H + i; const int at = i / KS * VS + i % KS;
+  float h = 0.f, az = 0.f, ar = 0.f, ac = 0.f, nz = 0.f, nr = 0.f, nc = 0.f;      // this step's and the next one's
+  if (L.el) { az = gp[0]; ar = gp[H]; ac = gp[2 * H]; if (T > 1) { const float* g = gp + 3 * H; nz = g[0]; nr = g[H]; nc = g[2 * H]; } }
   __syncthreads();
   for (int t = 0; t < T; t++) {
-#pragma unroll
-    for (int k = 0; k < NS; k++) {
-      const float* v = hb + k * 4 * jq + q * jq;
-      part[(q * NS + k) * Hp + i] = rec_dot<true>(wz, nullptr, 0, v, jq);
-      part[((4 + q) * NS + k) * Hp + i] = rec_dot<true>(wr, nullptr, 0, v, jq);
-    }
+    float a[NS][4], b[NS][4]; rec_clear(a); rec_clear(b);
+    rec_fma(a, wr, &hb[0][L.sp * VS], 8 * VS);
+    const float sr = rec_reduce(a, L.lane); float r = 0.f;
+    if (L.el) { r = act_fwd(GN_ACT_SIGMOID, ar + sr); rb[L.es][at] = r * h; }
+    rec_fma(b, wz, &hb[0][L.sp * VS], 8 * VS);
+    const float sz = rec_reduce(b, L.lane);
     __syncthreads();
-    float z = 0.f, r = 0.f;
-    if (el) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) { az += part[(k * NS + es) * Hp + i]; ar += part[((4 + k) * NS + es) * Hp + i]; }
-      r = act_fwd(GN_ACT_SIGMOID, ar);
-      rb[es * 4 * jq + i] = r * h;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NS; k++) part[(q * NS + k) * Hp + i] = rec_dot<true>(wr, nullptr, 0, rb + k * 4 * jq + q * jq, jq);
-    if (el) z = act_fwd(GN_ACT_SIGMOID, az);
-    __syncthreads();
-    if (el) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) ac += part[(k * NS + es) * Hp + i];
-      const float c = act_fwd(GN_ACT_TANH, ac);
+    rec_clear(a);
+    rec_fma(a, wr, &rb[0][L.sp * VS], 8 * VS);
+    const float sc = rec_reduce(a, L.lane);
+    if (L.el) {
+      const float z = act_fwd(GN_ACT_SIGMOID, az + sz), c = act_fwd(GN_ACT_TANH, ac + sc);
       h = h + z * (c - h);
-      hb[es * 4 * jq + i] = h;
+      hb[L.es][at] = h;
       float* g = gp + (long)t * 3 * H; g[0] = z; g[H] = r; g[2 * H] = c;
-      const long o = ((long)s * T + t) * H + i;
+      const long o = (L.s * T + t) * H + i;
       h_all[o] = h;
-      if (q_.return_seq) out[o] = h; else if (t == T - 1) out[(long)s * H + i] = h;
-      if (t + 1 < T) { g += 3 * H; az = g[0]; ar = g[H]; ac = g[2 * H]; }
+      if (q_.return_seq) out[o] = h; else if (t == T - 1) out[L.s * H + i] = h;
+      az = nz; ar = nr; ac = nc;
+      if (t + 2 < T) { g += 6 * H; nz = g[0]; nr = g[H]; nc = g[2 * H]; }
     }
     __syncthreads();
   }
@@ -218,80 +405,100 @@ __global__ void __launch_bounds__(512) gru_fwd_reg_kernel(const float* __restric
 // z, the candidate's contribution to dh_prev is indexed by the output unit's reset gate, and dh_prev is ADDED to the incoming
 // gradient before it is handed to the previous step.  Writes the gate deltas D [B,T,3H] (update | zero | candidate), h_{t-1} [B,T,H]
 // and r (.) h_{t-1} [B,T,H] for the weight-gradient contractions.
-template <int NS>
-__global__ void __launch_bounds__(512) gru_bwd_reg_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ gates, const float* __restrict__ h_all,
-                                                          float* __restrict__ D, float* __restrict__ hprev_all, float* __restrict__ rh_all, const RecShape q_) {
-  extern __shared__ __align__(16) float sm[];
-  const int H = q_.H, T = q_.T, Hp = rec_hp(H), jq = rec_jq(H), q = threadIdx.x / Hp, i = threadIdx.x - q * Hp;
-  float* ub = sm;                              // [NS][4 jq]  update deltas
-  float* cb = ub + NS * 4 * jq;                // [NS][4 jq]  candidate deltas times r
-  float* part = cb + NS * 4 * jq;              // [4][NS][Hp]
-  float wz[RU_Q], wr[RU_Q];
+template <int NS, int HB>
+__global__ void __launch_bounds__(64 * HB) gru_bwd_reg_kernel(const float* __restrict__ gout, const float* __restrict__ Wh, const float* __restrict__ gates, const float* __restrict__ h_all,
+                                                              float* __restrict__ D, float* __restrict__ hprev_all, float* __restrict__ rh_all, const RecShape q_) {
+  constexpr int KS = 4 * HB, VS = rec_vs(KS);
+  __shared__ __align__(16) float vb[2][2][NS][8 * VS];      // by parity of the step: update deltas | candidate deltas times r
+  const int H = q_.H, T = q_.T; const RecLane<NS, 4> L(H, q_.B); const int i = L.unit;
+  float wz[KS][4], wr[KS][4]; const bool vec = rec_vec(Wh, H);
 #pragma unroll
-  for (int j = 0; j < RU_Q; j++) {
-    const int k = q * jq + j; const bool in = i < H && j < jq && k < H;
-    wz[j] = in ? Wh[(long)k * H + i] : 0.f; wr[j] = in ? Wh[((long)H + k) * H + i] : 0.f;
+  for (int k = 0; k < KS; k += 4) {
+    rec_weights<false, 4>(wz + k, Wh, H, L.sp * KS + k, L.col0, vec);
+    rec_weights<false, 4>(wr + k, Wh + (long)H * H, H, L.sp * KS + k, L.col0, vec);
   }
-  for (int e = threadIdx.x; e < 2 * NS * 4 * jq; e += blockDim.x) ub[e] = 0.f;
-  const int es = threadIdx.x / Hp, s = blockIdx.x * NS + es; const bool el = es < NS && i < H && s < q_.B;
-  const float* gp = gates + (long)s * T * 3 * H + i; const long base = ((long)s * T) * H + i;
+  for (int e = threadIdx.x; e < 4 * NS * 8 * VS; e += blockDim.x) vb[0][0][0][e] = 0.f;
+  const float* gp = gates + L.s * T * 3 * H + i; const long base = L.s * T * H + i; const int at = i / KS * VS + i % KS;
   float cur = 0.f, z = 0.f, r = 0.f, c = 0.f, hp = 0.f;
-  if (el) {
+  if (L.el) {
     const float* g = gp + (long)(T - 1) * 3 * H; z = g[0]; r = g[H]; c = g[2 * H]; hp = T > 1 ? h_all[base + (long)(T - 2) * H] : 0.f;
-    if (!q_.return_seq) cur = gout[(long)s * H + i];
+    if (!q_.return_seq) cur = gout[L.s * H + i];
   }
   __syncthreads();
   for (int t = T - 1; t >= 0; t--) {
     const float zt = z;
-    if (el) {
+    if (L.el) {
       const long o = base + (long)t * H;
       if (q_.return_seq) cur += gout[o];
       const float du = cur * (c - hp) * z * (1.f - z), dc = cur * (1.f - z) * (1.f - c * c);
-      float* Dr = D + ((long)s * T + t) * 3 * H + i; Dr[0] = du; Dr[H] = 0.f; Dr[2 * H] = dc;
+      float* Dr = D + (L.s * T + t) * 3 * H + i; Dr[0] = du; Dr[H] = 0.f; Dr[2 * H] = dc;
       hprev_all[o] = hp; rh_all[o] = r * hp;
-      ub[es * 4 * jq + i] = du; cb[es * 4 * jq + i] = dc * r;
+      vb[t & 1][0][L.es][at] = du; vb[t & 1][1][L.es][at] = dc * r;
       if (t > 0) { const float* g = gp + (long)(t - 1) * 3 * H; z = g[0]; r = g[H]; c = g[2 * H]; hp = t > 1 ? h_all[o - 2 * H] : 0.f; }
     }
     if (t == 0) break;
     __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NS; k++)
-      part[(q * NS + k) * Hp + i] = rec_dot<true>(wz, nullptr, 0, ub + k * 4 * jq + q * jq, jq) + rec_dot<true>(wr, nullptr, 0, cb + k * 4 * jq + q * jq, jq);
-    __syncthreads();
-    if (el) { const float sum = (part[es * Hp + i] + part[(NS + es) * Hp + i]) + (part[(2 * NS + es) * Hp + i] + part[(3 * NS + es) * Hp + i]); cur = cur + (sum + cur * zt); }
+    float acc[NS][4]; rec_clear(acc);
+    rec_fma(acc, wz, &vb[t & 1][0][0][L.sp * VS], 8 * VS);
+    rec_fma(acc, wr, &vb[t & 1][1][0][L.sp * VS], 8 * VS);
+    const float sum = rec_reduce(acc, L.lane);
+    if (L.el) cur = cur + (sum + cur * zt);
   }
 }
 
 // ------------------------------------------------------------------ launchers
+// f<NS, HB>() for the number of samples per block and of blocks of 32 units
+template <class F> inline int rec_dispatch(const Ctx* ctx, const RecShape& q, F&& f) {
+  const bool two = q.B > ctx->sm_count;
+  auto by_hb = [&](auto ns) -> int {
+    switch ((q.H + 31) / 32) {
+      case 1: return f(ns, std::integral_constant<int, 1>{});
+      case 2: return f(ns, std::integral_constant<int, 2>{});
+      case 3: return f(ns, std::integral_constant<int, 3>{});
+      default: return f(ns, std::integral_constant<int, 4>{});
+    }
+  };
+  return two ? by_hb(std::integral_constant<int, 2>{}) : by_hb(std::integral_constant<int, 1>{});
+}
 inline int lstm_fwd(Ctx* ctx, const float* Wh, const float* bias, float* ig, float* c, float* tc, float* h, float* out, const RecShape& q) {
-  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const bool regs = q.H <= 4 * RU_Q;
-  const size_t smem = ((size_t)2 * ns * 4 * jq + 4 * ns * Hp + (regs ? 0 : (size_t)4 * jq * Hp)) * sizeof(float);
-  auto* K = regs ? (ns == 2 ? lstm_fwd_kernel<2, true> : lstm_fwd_kernel<1, true>) : (ns == 2 ? lstm_fwd_kernel<2, false> : lstm_fwd_kernel<1, false>);
+  if (q.H <= REC_REG_H) return rec_dispatch(ctx, q, [&](auto ns, auto hb) -> int {
+    GN_LAUNCH(ctx, (lstm_fwd_reg_kernel<ns(), hb()>), cdiv(q.B, ns()), 64 * hb(), 0, Wh, bias, ig, c, tc, h, out, q);
+    return check_launch("lstm_fwd");
+  });
+  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1;
+  const size_t smem = ((size_t)2 * ns * 4 * jq + 4 * ns * Hp + (size_t)4 * jq * Hp) * sizeof(float);
+  auto* K = ns == 2 ? lstm_fwd_kernel<2> : lstm_fwd_kernel<1>;
   if (4 * Hp > 1024 || smem > 220 * 1024) return fail(GN_ERR_UNSUPPORTED, "LSTM of hidden size %d needs %zu bytes of shared memory", q.H, smem);
   GN_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GN_LAUNCH(ctx, K, cdiv(q.B, ns), 4 * Hp, smem, Wh, bias, ig, c, tc, h, out, q);
   return check_launch("lstm_fwd");
 }
 inline int lstm_bwd(Ctx* ctx, const float* gout, const float* Wh, const float* bias, const float* ig, const float* c, const float* tc, float* D, const RecShape& q) {
-  const int Hp = rec_hp(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const bool small = Hp <= 128;
+  if (q.H <= REC_REG_H) return rec_dispatch(ctx, q, [&](auto ns, auto hb) -> int {
+    GN_LAUNCH(ctx, (lstm_bwd_reg_kernel<ns(), hb()>), cdiv(q.B, ns()), 64 * hb(), 0, gout, Wh, bias, ig, c, tc, D, q);
+    return check_launch("lstm_bwd");
+  });
+  const int Hp = rec_hp(q.H), ns = q.B > ctx->sm_count ? 2 : 1;
   const size_t fixed = (size_t)8 * ns * Hp * sizeof(float), row = (size_t)4 * Hp * sizeof(float);
-  // registers hold 64 (24) rows of each gate's column, shared memory as many of the others as fit, in fours
-  const int rs = (int)std::min<size_t>((std::max(0, q.H - (small ? 64 : 24)) + 3) & ~3, ((200 * 1024 - fixed) / row) & ~(size_t)3); const size_t smem = fixed + rs * row;
-  auto* K = small ? (ns == 2 ? lstm_bwd_kernel<2, 64, 512> : lstm_bwd_kernel<1, 64, 512>) : (ns == 2 ? lstm_bwd_kernel<2, 24, 1024> : lstm_bwd_kernel<1, 24, 1024>);
+  // registers hold 24 rows of each gate's column, shared memory as many of the others as fit, in fours
+  const int rs = (int)std::min<size_t>((q.H - 24 + 3) & ~3, ((200 * 1024 - fixed) / row) & ~(size_t)3); const size_t smem = fixed + rs * row;
+  auto* K = ns == 2 ? lstm_bwd_kernel<2, 24> : lstm_bwd_kernel<1, 24>;
   GN_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GN_LAUNCH(ctx, K, cdiv(q.B, ns), 4 * Hp, smem, gout, Wh, bias, ig, c, tc, D, q, rs);
   return check_launch("lstm_bwd");
 }
-inline bool gru_reg_ok(int H) { return H <= 4 * RU_Q; }
+inline bool gru_reg_ok(int H) { return H <= REC_REG_H; }
 inline int gru_fwd_reg(Ctx* ctx, const float* Wh, float* gates, float* h, float* out, const RecShape& q) {
-  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const size_t smem = ((size_t)8 * ns * jq + 8 * ns * Hp) * sizeof(float);
-  GN_LAUNCH(ctx, (ns == 2 ? gru_fwd_reg_kernel<2> : gru_fwd_reg_kernel<1>), cdiv(q.B, ns), 4 * Hp, smem, Wh, gates, h, out, q);
-  return check_launch("gru_fwd");
+  return rec_dispatch(ctx, q, [&](auto ns, auto hb) -> int {
+    GN_LAUNCH(ctx, (gru_fwd_reg_kernel<ns(), hb()>), cdiv(q.B, ns()), 64 * hb(), 0, Wh, gates, h, out, q);
+    return check_launch("gru_fwd");
+  });
 }
 inline int gru_bwd_reg(Ctx* ctx, const float* gout, const float* Wh, const float* gates, const float* h, float* D, float* hprev, float* rh, const RecShape& q) {
-  const int Hp = rec_hp(q.H), jq = rec_jq(q.H), ns = q.B > ctx->sm_count ? 2 : 1; const size_t smem = ((size_t)8 * ns * jq + 4 * ns * Hp) * sizeof(float);
-  GN_LAUNCH(ctx, (ns == 2 ? gru_bwd_reg_kernel<2> : gru_bwd_reg_kernel<1>), cdiv(q.B, ns), 4 * Hp, smem, gout, Wh, gates, h, D, hprev, rh, q);
-  return check_launch("gru_bwd");
+  return rec_dispatch(ctx, q, [&](auto ns, auto hb) -> int {
+    GN_LAUNCH(ctx, (gru_bwd_reg_kernel<ns(), hb()>), cdiv(q.B, ns()), 64 * hb(), 0, gout, Wh, gates, h, D, hprev, rh, q);
+    return check_launch("gru_bwd");
+  });
 }
 
 // ------------------------------------------------------------------ LSTM gradient clipping

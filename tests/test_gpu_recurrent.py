@@ -26,6 +26,9 @@ def device():
     ("lstm", 7, 20, 43, 3, 1, False),                    # 129 updates: a group of one
     ("lstm", 7, 20, 40, 10, 1, False), ("lstm", 7, 20, 40, 10, 4, False), ("lstm", 7, 20, 13, 21, 10, False),      # several groups; short last chunks; more than eight chunks
     ("gru", 3, 1, 5, 3, 1, False), ("gru", 4, 33, 6, 149, 1, True), ("gru", 5, 97, 4, 7, 1, False), ("gru", 5, 128, 3, 150, 1, False), ("gru", 5, 129, 3, 6, 1, False),
+    # blocks of 32 units, one or two samples a block, weights beyond the registers (97 units and more), widths that no 16-byte load divides, one step
+    ("lstm", 3, 97, 1, 3, 1, False), ("lstm", 5, 96, 5, 150, 1, True), ("lstm", 5, 101, 4, 149, 1, True), ("lstm", 5, 64, 6, 149, 1, False), ("lstm", 5, 100, 2, 148, 1, False), ("lstm", 3, 2, 3, 150, 1, True),
+    ("gru", 5, 64, 1, 2, 1, False), ("gru", 5, 96, 5, 150, 1, True), ("gru", 5, 63, 4, 149, 1, False), ("gru", 3, 2, 3, 150, 1, False),
 ])
 def test_recurrent_parity(device, oracle, net, I, H, T, batch, W, seq):
     from goneuron_b200.sequential import Adam, Sequential
