@@ -52,6 +52,17 @@ struct GraphRec {
     if (e == cudaSuccess) { t.nodes.assign(1, node); t.kernel = kernel; }
     return e;
   }
+  // Work on stream `s` that a replay leaves out unless a kernel before it has set `handle` (condition()) to a non-zero value.
+  cudaError_t condition(cudaGraphConditionalHandle* handle) { return cudaGraphConditionalHandleCreate(handle, graph, 0, cudaGraphCondAssignDefault); }
+  template <class F> cudaError_t only_if(cudaStream_t s, cudaGraphConditionalHandle handle, F&& body) {
+    cudaGraphNodeParams p{}; p.type = cudaGraphNodeTypeConditional; p.conditional.handle = handle; p.conditional.type = cudaGraphCondTypeIf; p.conditional.size = 1;
+    const cudaError_t e = add(s, false, [&](cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t n) { return cudaGraphAddNode(node, graph, deps, n, &p); });
+    if (e != cudaSuccess) return e;
+    cudaGraph_t outer = graph; std::vector<Tail> outer_tails; outer_tails.swap(tails);
+    graph = p.conditional.phGraph_out[0];                     // (belongs to the node)
+    body();
+    graph = outer; tails.swap(outer_tails); return cudaSuccess;
+  }
 };
 
 struct Ctx {

@@ -1177,7 +1177,10 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
       };
       if (world == 1 && (!late || few)) gather(nullptr, late ? un : nullptr);
       else if (world == 1) GN_LAUNCH(ctx, lstm_update_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, un, T, in, H, n_updates);
-      if (late) GN_LAUNCH(ctx, lstm_clip_start_kernel, nchunks, 1024, 0, (const float*)un, n_updates, Kc, start); else start = nullptr;
+      // in a recorded step the launches for all but the last groups are one conditional node
+      cudaGraphConditionalHandle skip = 0; const int tail = groups >= CLIP_SKIP_MIN && ctx->rec ? (int)groups - CLIP_TAIL : 0;
+      if (tail) GN_CUDA(ctx->rec->condition(&skip));
+      if (late) GN_LAUNCH(ctx, lstm_clip_start_kernel, nchunks, 1024, 0, (const float*)un, n_updates, Kc, start, skip, tail); else start = nullptr;
       if (world == 1 && late && !few) gather(start, nullptr);
       // Gram blocks of every group against the group before it and itself
       GemmDesc g; g.M = CG; g.N = 2 * CG; g.batch1 = nchunks; g.batch2 = (int)groups; g.ldc = 2 * CG; g.z_first = start; g.c_b1 = groups * CG * 2 * CG; g.c_b2 = CG * 2 * CG; g.sa_k = g.sb_k = 1;
@@ -1188,7 +1191,9 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
       const ClipArgs a{Dm, Zm, G0, db, db + n_om, db + n_om + n_p, gmat, start, R4g, ZWg, (int)groups, slabs, stride};
       const size_t smem = clip_smem(ZWg);
       GN_CUDA(cudaFuncSetAttribute(lstm_clip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      for (int j = 0; j <= groups; j++) GN_EARLY_LAUNCH(ctx, lstm_clip_kernel, dim3(1 + slabs, nchunks), CG_THREADS, smem, a, j);
+      auto walk = [&](int from, int to) -> int { for (int j = from; j < to; j++) GN_EARLY_LAUNCH(ctx, lstm_clip_kernel, dim3(1 + slabs, nchunks), CG_THREADS, smem, a, j); return GN_OK; };
+      if (tail) { int rc = GN_OK; GN_CUDA(ctx->rec->only_if(ctx->stream, skip, [&] { rc = walk(0, tail); })); GN_TRY(rc); }
+      GN_TRY(walk(tail, (int)groups + 1));
       GN_LAUNCH(ctx, lstm_scatter_grad_kernel, cdiv((long)R4g * ZWg, 256), 256, 0, (const float*)gmat, (int)(groups & 1), nchunks, in, H, m->grads.p + l.p_off);
       return check_launch("lstm_backward");
     }

@@ -577,7 +577,7 @@ __global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restr
     a.x *= b.x; a.y *= b.y; a.z *= b.z; a.w *= b.w; reinterpret_cast<float4*>(G)[i] = a;
   }
 }
-constexpr int CLIP_FORGET = 128, CLIP_FEW = 32;
+constexpr int CLIP_FORGET = 128, CLIP_FEW = 32, CLIP_TAIL = 16, CLIP_SKIP_MIN = 64;      // (last groups whose launches are never left out; groups from which on the others may be)
 constexpr float CLIP_FINITE = 1e36f;                        // squared norms above this count as not finite
 // |u_k|^2 of every update, in update order; a warp each.  From the layer's own arrays (d, x, h as in lstm_gather_updates_kernel), so that
 // updates that are not walked need not be gathered.
@@ -602,8 +602,11 @@ __global__ void __launch_bounds__(256) lstm_row_norms_kernel(const float* __rest
   d2 = warp_sum(d2); z2 = warp_sum(z2);
   if (lane == 0) un[k] = d2 * z2;
 }
-// start[chunk]: the first group to walk
-__global__ void __launch_bounds__(1024) lstm_clip_start_kernel(const float* __restrict__ un, long n_updates, long Kc, int* __restrict__ start) {
+// start[chunk]: the first group to walk.  `skip` (0: none): condition of the launches for groups before `tail` in a recorded step, which
+// are left out as a whole if no chunk starts there.  A launch of the walk that has nothing to do still costs 0.9 us, a condition about 10, and 20
+// if its body runs: 128 groups of which the last few are walked 414 -> 289 us (a step of 64 steps, 256 samples), all walked 1604 -> 1618; 32 groups 227
+// either way, all walked 520 -> 542: from 64 groups on.
+__global__ void __launch_bounds__(1024) lstm_clip_start_kernel(const float* __restrict__ un, long n_updates, long Kc, int* __restrict__ start, cudaGraphConditionalHandle skip, int tail) {
   __shared__ float part[32]; __shared__ int first;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5; const long k0 = blockIdx.x * Kc, n = min(Kc, n_updates - k0); const float* u = un + k0;
   const int groups = (int)((Kc + CG - 1) / CG);
@@ -627,7 +630,7 @@ __global__ void __launch_bounds__(1024) lstm_clip_start_kernel(const float* __re
     if (first >= 0) { j0 = first; break; }
     __syncthreads();
   }
-  if (tid == 0) start[blockIdx.x] = j0;
+  if (tid == 0) { start[blockIdx.x] = j0; if (skip && j0 < tail) cudaGraphSetConditional(skip, 1); }
 }
 struct ClipArgs {
   const float *D, *Z, *G;        // rows of a chunk start at chunk * stride (CG_PAD rows of zeros first); G [chunk][group][CG][2 CG]: against groups j-1, j

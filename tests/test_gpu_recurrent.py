@@ -136,3 +136,29 @@ def test_elementwise_functions_are_rounded_once(device):
     assert np.array_equal(model.PredictBatch(np.array([[np.inf], [-np.inf], [50], [-50]], np.float32)).ravel(), [1, -1, 1, -1])
     assert np.isnan(model.PredictBatch(np.array([[np.nan]], np.float32))).all()
     model.Close()
+
+
+@pytest.mark.parametrize("W,batch", [(1, 224), (2, 448)])
+def test_replayed_step_walks_what_its_updates_ask_for(device, W, batch):
+    """Seventy groups per chunk.  One recorded step is replayed with targets after which everything is walked, the last groups are, and (two
+    chunks) one chunk is walked as a whole; every gradient is that of a model whose first step, issued launch by launch, it is."""
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = [D.SequenceUnrollerLSTM(7, 20, 40, False), D.Dense(20, 2, D.LINEAR)]
+    rng = np.random.Generator(np.random.PCG64(6))
+    params = configs.init_params(layers, rng)
+    x, y = configs.make_inputs("lstm", layers, batch, rng)
+    half = np.ones_like(y)
+    half[: batch // 2] = 1e-6
+
+    def make(p):
+        m = Sequential(layers, device, virtual_workers=W).Compile(Adam(1e-3), D.MSE)
+        m.SetParams(p)
+        return m
+    model = make(params)
+    for scale in (1e4, 1e4, 1e-6, 1e4, 1e4 * half, 1e-6, 1e4):
+        other = make(model.Params())
+        t = (y * scale).astype(np.float32)
+        assert model.TrainBatch(x, t) == other.TrainBatch(x, t)
+        assert np.array_equal(model.Gradients(), other.Gradients())
+        other.Close()
+    model.Close()
