@@ -309,6 +309,9 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool ok 
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async16_part(float* dst, const float* src, int n) {      // n floats from src, zeros behind them
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(4 * n) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -48,20 +48,13 @@ struct GemmDesc {
 };
 
 // ------------------------------------------------------------------ tiled kernel
-// One BM x BN output tile per cluster of `splits` blocks (1, 2, 4 or 8).  The contraction is cut into `splits` equal runs, one
-// per block of the cluster; the blocks leave their sums in shared memory, and after a cluster barrier each of them adds up and
-// stores its share of the tile's elements, always in rank order, so a result does not depend on scheduling.  This is what
-// these products need: they come from small batches and narrow layers (a [64, 784] x [784, 128] forward product, a
-// [96, 96] weight gradient over 5000 rows), where a single 128 x 128 tile per block left all but a few SMs idle and one block
-// walking the whole contraction -- 72 us for the former and 430 us for the latter, against 7 and 13 us now.
-// Global loads of a k-step go to registers while the two before it are multiplied, then to the other shared-memory buffer.
-// 16-byte loads along the operand's fast index where base, stride and range allow it.
-constexpr int SG_PAD = 4, SG_MAX_SPLITS = 8, SG_RUN = 32;      // runs start at multiples of SG_RUN, whatever the tile
+// One BM x BN output tile per block.  Global loads of a k-step go to registers while the two before it are multiplied, then to the
+// other shared-memory buffer.  16-byte loads along the operand's fast index where base, stride and range allow it.
+constexpr int SG_PAD = 4;
 template <int BM, int BN, int BK, int TM, int TN> struct SgCfg {
   static constexpr int THREADS = (BM / TM) * (BN / TN);
   static constexpr int LDA = BM + SG_PAD, LDB = BN + SG_PAD;
   static constexpr int STAGE = BK * (LDA + LDB);
-  static constexpr int SMEM_FLOATS = 2 * STAGE > BM * BN ? 2 * STAGE : BM * BN;
 };
 
 // A rows x BK slab of an operand: element (r, k) at p[r * s_r + k * s_k], r < nr, k < nk (both relative), zero outside.
@@ -118,25 +111,20 @@ __device__ __forceinline__ float sg_finish(const GemmDesc& g, const float* R, in
 }
 
 template <int BM, int BN, int BK, int TM, int TN, bool A_KFAST, bool B_NFAST>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmDesc g, int splits, int vec_a, int vec_b, int y0) {
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmDesc g, int vec_a, int vec_b, int y0) {
   using Cfg = SgCfg<BM, BN, BK, TM, TN>;
   constexpr int THREADS = Cfg::THREADS, LDA = Cfg::LDA, LDB = Cfg::LDB, CX = BN / TN;
-  __shared__ __align__(16) float sm[Cfg::SMEM_FLOATS];
-  __shared__ float asum_sh[BM];
-  const int b = blockIdx.z, b1 = b / g.batch2, b2 = b % g.batch2, rank = blockIdx.x % splits, nt = blockIdx.x / splits;
+  __shared__ __align__(16) float sm[2 * Cfg::STAGE];
+  const int b = blockIdx.z, b1 = b / g.batch2, b2 = b % g.batch2, nt = blockIdx.x;
   const float* A = g.A + b1 * g.a_b1 + b2 * g.a_b2;
   const float* B = g.B + b1 * g.b_b1 + b2 * g.b_b2;
   float* C = g.C + b1 * g.c_b1 + b2 * g.c_b2;
   const float* R = g.R ? g.R + b1 * g.r_b1 + b2 * g.r_b2 : nullptr;
   const int m0 = (y0 + blockIdx.y) * BM, n0 = nt * BN;
-  if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + BM - 1) return;             // (the whole cluster returns)
+  if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + BM - 1) return;
   int kbeg = 0, kend = g.K;
   if (g.flags & GEMM_KBEG_AT_M0) kbeg = (m0 / BK) * BK;
   if (g.flags & GEMM_KEND_AT_M0) kend = min(g.K, m0 + BM);
-  if (splits > 1) {
-    const int per = (((kend - kbeg + splits - 1) / splits + SG_RUN - 1) / SG_RUN) * SG_RUN;
-    kbeg = min(kend, kbeg + rank * per); kend = min(kend, kbeg + per);
-  }
   const int t = threadIdx.x, ty = t / CX, tx = t % CX;
   float acc[TM][TN];
 #pragma unroll
@@ -188,73 +176,63 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
       if (k0 + BK < kend) step(s0, s1, k0 + BK);
     }
   }
-  if (splits == 1) {
 #pragma unroll
-    for (int i = 0; i < TM; i++) {
-      const int m = m0 + ty * TM + i;
-      if (m >= g.M) continue;
+  for (int i = 0; i < TM; i++) {
+    const int m = m0 + ty * TM + i;
+    if (m >= g.M) continue;
 #pragma unroll
-      for (int j = 0; j < TN; j++) { const int n = n0 + tx * TN + j; if (n < g.N) C[m * g.ldc + n] = sg_finish(g, R, m, n, acc[i][j]); }
-    }
-    if (want_asum && t < BM && m0 + t < g.M) g.a_sum[m0 + t] = asum;
-    return;
+    for (int j = 0; j < TN; j++) { const int n = n0 + tx * TN + j; if (n < g.N) C[m * g.ldc + n] = sg_finish(g, R, m, n, acc[i][j]); }
   }
-  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++) sm[(ty * TM + i) * BN + tx * TN + j] = acc[i][j];
-  if (want_asum && t < BM) asum_sh[t] = asum;
-  cluster.sync();
-  const int share = BM * BN / splits;
-  for (int e = rank * share + t; e < (rank + 1) * share; e += THREADS) {
-    const int m = m0 + e / BN, n = n0 + e % BN;
-    if (m >= g.M || n >= g.N) continue;
-    float v = 0.f;
-    for (int q = 0; q < splits; q++) v += cluster.map_shared_rank(sm, q)[e];
-    C[m * g.ldc + n] = sg_finish(g, R, m, n, v);
-  }
-  if (want_asum && rank == 0 && t < BM && m0 + t < g.M) {
-    float v = 0.f;
-    for (int q = 0; q < splits; q++) v += cluster.map_shared_rank(asum_sh, q)[t];
-    g.a_sum[m0 + t] = v;
-  }
-  cluster.sync();                                             // nobody leaves while its sums are being read
+  if (want_asum && t < BM && m0 + t < g.M) g.a_sum[m0 + t] = asum;
 }
 
 // Skinny outputs (N <= 16, both operands K-major, one problem): a tile would be mostly padding.  A cluster of `splits`
-// blocks owns one output row: their threads stride over K with all N sums in registers, combine through shared memory, and
+// blocks owns RPB output rows: their threads stride over K with all N sums of each row in registers, combine through shared memory, and
 // rank 0 adds the blocks' sums in rank order.  C(m,n) = act(sum_k A(m,k) B(n,k) + bias[n] + R(m,n)).  One block per row (K = 4704,
-// N = 10: 18 loads deep) took 18 us for 50 rows; eight take 7.
+// N = 10: 18 loads deep) took 18 us for 50 rows; eight take 6.  Bound by what is fetched of B, once per block: four rows share it where there are
+// enough (128 rows, K = 2048, N = 10: 8.5 -> 5.4 us; 300 rows, K = 128: 3.1 either way; 1000: 5.5 -> 4.0).
 constexpr int SKINNY_N = 16;
+template <int RPB>
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmDesc g, int splits) {
-  __shared__ float red[8][SKINNY_N];
-  __shared__ float tot[SKINNY_N];
-  const int m = blockIdx.x / splits, rank = blockIdx.x % splits, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const float* a = g.A + (long)m * g.sa_m;
-  float acc[SKINNY_N];
+  __shared__ float red[8][RPB][SKINNY_N];
+  __shared__ float tot[RPB][SKINNY_N];
+  const int m0 = blockIdx.x / splits * RPB, rank = blockIdx.x % splits, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float* a[RPB]; float acc[RPB][SKINNY_N];
 #pragma unroll
-  for (int n = 0; n < SKINNY_N; n++) acc[n] = 0.f;
+  for (int r = 0; r < RPB; r++) {
+    a[r] = g.A + (long)(RPB == 1 ? m0 : min(m0 + r, g.M - 1)) * g.sa_m;        // (a row beyond the last is the last one again, and not stored)
+#pragma unroll
+    for (int n = 0; n < SKINNY_N; n++) acc[r][n] = 0.f;
+  }
   for (int k = rank * 256 + threadIdx.x; k < g.K; k += 256 * splits) {
-    const float av = a[k];
+    float av[RPB];
 #pragma unroll
-    for (int n = 0; n < SKINNY_N; n++) if (n < g.N) acc[n] = fmaf(av, g.B[(long)n * g.sb_n + k], acc[n]);
+    for (int r = 0; r < RPB; r++) av[r] = a[r][k];
+#pragma unroll
+    for (int n = 0; n < SKINNY_N; n++) if (n < g.N) {
+      const float bv = g.B[(long)n * g.sb_n + k];
+#pragma unroll
+      for (int r = 0; r < RPB; r++) acc[r][n] = fmaf(av[r], bv, acc[r][n]);
+    }
   }
 #pragma unroll
-  for (int n = 0; n < SKINNY_N; n++) { if (n < g.N) { const float v = warp_sum(acc[n]); if (lane == 0) red[w][n] = v; } }
+  for (int n = 0; n < SKINNY_N; n++) if (n < g.N) {
+#pragma unroll
+    for (int r = 0; r < RPB; r++) { const float v = warp_sum(acc[r][n]); if (lane == 0) red[w][r][n] = v; }
+  }
   __syncthreads();
-  if (threadIdx.x < g.N) {
+  const int r = threadIdx.x / SKINNY_N, n = threadIdx.x % SKINNY_N; const bool mine = r < RPB && n < g.N;
+  if (mine) {
     float v = 0.f;
-    for (int q = 0; q < 8; q++) v += red[q][threadIdx.x];
-    tot[threadIdx.x] = v;
+    for (int q = 0; q < 8; q++) v += red[q][r][n];
+    tot[r][n] = v;
   }
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   if (splits > 1) cluster.sync(); else __syncthreads();
-  if (rank == 0 && threadIdx.x < g.N) {
-    const int n = threadIdx.x;
+  if (rank == 0 && mine && m0 + r < g.M) {
     float v = 0.f;
-    for (int q = 0; q < splits; q++) v += splits > 1 ? cluster.map_shared_rank(tot, q)[n] : tot[n];
-    g.C[(long)m * g.ldc + n] = sg_finish(g, g.R, m, n, v);
+    for (int q = 0; q < splits; q++) v += splits > 1 ? cluster.map_shared_rank(&tot[0][0], q)[r * SKINNY_N + n] : tot[r][n];
+    g.C[(long)(m0 + r) * g.ldc + n] = sg_finish(g, g.R, m0 + r, n, v);
   }
   if (splits > 1) cluster.sync();
 }
@@ -317,29 +295,244 @@ inline bool gemm_outer_small_ok(const GemmDesc& g) {
          !g.a_planes && !g.b_planes && !g.plane_out && !g.a_rownorm && !g.m_seg && (long)g.M * g.N >= 64 * 64;
 }
 
+// ------------------------------------------------------------------ small products
+// Products whose 64 x 64 tiles leave most SMs idle: the few rows of a head, of a block's token rows or of a small batch, weight gradients of narrow
+// layers.  They are bound by latency (64 rows by a [256, 256] matrix are 0.2 us of multiply-adds), so a block has as much in flight and as
+// few dependent steps as possible.  A cluster of up to eight blocks owns a tile of 4 TM rows by 32 columns, each with a run of the
+// contraction; a block asks for up to three stages of 64 indices ahead (asynchronous copies of 16 bytes in the operands' own order); each of its
+// eight warps multiplies eight indices of every stage for the whole tile, TM x 4 outputs per lane; the warps' sums meet in shared
+// memory; and a block's sums are written straight to the blocks of the cluster that own them: one exchange, after which nobody reads
+// from anybody else.
+// Order of an output's sum: the contraction is cut into chunks; within one, a warp's indices ascending, then the warps; the chunks pairwise.
+// A block of the cluster takes a power of two of neighbouring chunks, so their number per block (it falls with the number of tiles) does not
+// matter, and where the rows of A are samples a sample's result is the same in every batch.
+// us per launch in a recorded chain, a 32 x 32 tile in two register-staged steps per run, results read from the other blocks -> this:
+//   64 x 256 over 256 4.9 -> 3.8, over 1024 6.8 -> 6.0; 128 x 1024 over 256 7.6 -> 5.9; 1 x 128 over 784 5.6 -> 3.4; 8 x 8192 over 512 13.3 -> 7.1;
+//   16 x 512 over 8192 25.6 -> 15.2; a 96 x 96 weight gradient over 5000 rows 14.3 -> 10.4.  The same chain of empty launches: 2.2.
+constexpr int SP_KB = 64, SP_BN = 32, SP_STAGES = 4, SP_THREADS = 256, SP_MAX_SPLITS = 8;
+constexpr int sp_smem(int tm) { return (SP_STAGES * SP_KB * (4 * tm + SP_BN) + 8 * 4 * tm * SP_BN) * (int)sizeof(float); }
+// Brings ROWS operand rows x 64 indices into shared memory, stage by stage.  KFAST: [row][64], 16-byte units swizzled by the row's position among
+// fours (eight lanes that read one unit of rows four apart find it in different banks); else [64][ROWS].
+template <int ROWS, bool KFAST>
+struct SpLoad {
+  static constexpr int NV = ROWS * SP_KB / 4, NQ = (NV + SP_THREADS - 1) / SP_THREADS;
+  const float *base, *src[NQ]; long s_r, s_k; int nr; bool vec;
+  __device__ __forceinline__ static void place(int q, int& r, int& k) {
+    const int e = q * SP_THREADS + threadIdx.x;
+    if (KFAST) { r = e >> 4; k = (e & 15) * 4; } else { r = e % (ROWS / 4) * 4; k = e / (ROWS / 4); }
+  }
+  __device__ __forceinline__ SpLoad(const float* p, long s_r_, long s_k_, int nr_, bool v) : base(p), s_r(s_r_), s_k(s_k_), nr(nr_), vec(v) {
+#pragma unroll
+    for (int q = 0; q < NQ; q++) { int r, k; place(q, r, k); src[q] = p + (KFAST ? r * s_r + k : r + k * s_k); }
+  }
+  __device__ __forceinline__ void fetch(float* __restrict__ dst, int nk) {      // nk: indices that are left, this stage included
+    if (vec) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        int r, k; place(q, r, k);
+        if (NV % SP_THREADS != 0 && q * SP_THREADS + (int)threadIdx.x >= NV) break;
+        const int n = KFAST ? (r < nr ? min(max(nk - k, 0), 4) : 0) : (k < nk ? min(max(nr - r, 0), 4) : 0);
+        cp_async16_part(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) : k * ROWS + r), n ? src[q] : base, n);
+        src[q] += KFAST ? (long)SP_KB : SP_KB * s_k;
+      }
+    } else {
+      const int r0 = KFAST ? threadIdx.x >> 6 : threadIdx.x % ROWS, k0 = KFAST ? threadIdx.x & 63 : threadIdx.x / ROWS; const float* p = base + r0 * s_r + k0 * s_k;
+#pragma unroll
+      for (int q = 0; q < ROWS / 4; q++) {
+        const int r = KFAST ? r0 + 4 * q : r0, k = KFAST ? k0 : k0 + SP_THREADS / ROWS * q; const bool ok = r < nr && k < nk;
+        cp_async4(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) + (k & 3) : k * ROWS + r), ok ? p : base, ok);
+        p += KFAST ? 4 * s_r : SP_THREADS / ROWS * s_k;
+      }
+      if (nk > SP_KB) base += SP_KB * s_k;
+    }
+  }
+};
+// `splits` blocks per cluster, `chunks` chunks per block, each of `per` indices (a multiple of 64)
+template <int TM, bool A_KFAST, bool B_NFAST>
+__global__ void __launch_bounds__(SP_THREADS, 2) gemm_small_kernel(const GemmDesc g, int splits, int chunks, int per, int vec_a, int vec_b, int y0) {
+  constexpr int BM = 4 * TM, STAGE = SP_KB * (BM + SP_BN), NV = BM * SP_BN / 4;
+  extern __shared__ __align__(16) float sm[];                 // ring of stages, A | B; the warps' sums [8][BM][32]
+  __shared__ __align__(16) float4 xch[NV];                    // what the cluster's blocks send: [block][share]
+  __shared__ float as_sm[8][BM], as_x[SP_MAX_SPLITS][BM];
+  const int b = blockIdx.z, b1 = b / g.batch2, b2 = b % g.batch2, rank = blockIdx.x % splits, nt = blockIdx.x / splits;
+  const float* A = g.A + b1 * g.a_b1 + b2 * g.a_b2;
+  const float* B = g.B + b1 * g.b_b1 + b2 * g.b_b2;
+  float* C = g.C + b1 * g.c_b1 + b2 * g.c_b2;
+  const float* R = g.R ? g.R + b1 * g.r_b1 + b2 * g.r_b2 : nullptr;
+  const int m0 = (y0 + blockIdx.y) * BM, n0 = nt * SP_BN;
+  if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + BM - 1) return;             // (the whole cluster returns)
+  if (splits > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // "running": nobody is written to before
+  int kbeg = rank * chunks * per, kend = min(g.K, kbeg + chunks * per);
+  if (g.flags & GEMM_KBEG_AT_M0) kbeg = max(kbeg, m0 / SP_KB * SP_KB);
+  if (g.flags & GEMM_KEND_AT_M0) kend = min(kend, m0 + BM);
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31, mg = lane >> 3, ng = lane & 7, stages = kend > kbeg ? (kend - kbeg + SP_KB - 1) / SP_KB : 0;
+  const int k_at = stages ? kbeg : 0;                         // (a block without indices fetches nothing)
+  SpLoad<BM, A_KFAST> la(A + (long)m0 * g.sa_m + (long)k_at * g.sa_k, g.sa_m, g.sa_k, g.M - m0, vec_a);
+  SpLoad<SP_BN, !B_NFAST> lb(B + (long)n0 * g.sb_n + (long)k_at * g.sb_k, g.sb_n, g.sb_k, g.N - n0, vec_b);
+  auto fetch = [&](int s) {
+    if (s < stages) { float* d = sm + s % SP_STAGES * STAGE; la.fetch(d, kend - kbeg - s * SP_KB); lb.fetch(d + SP_KB * BM, kend - kbeg - s * SP_KB); }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < SP_STAGES - 1; s++) fetch(s);
+  float asum[TM];
+#pragma unroll
+  for (int i = 0; i < TM; i++) asum[i] = 0.f;
+  const bool want_asum = !A_KFAST && g.a_sum != nullptr && nt == 0;
+  auto add = [](const float4& a, const float4& x) { return make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w); };
+  float4* red = reinterpret_cast<float4*>(sm + SP_STAGES * STAGE);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f); float4 v = zero, s1 = zero, s2 = zero, s4 = zero;      // of this thread's four outputs: the sum, and sums of 1, 2, 4 chunks that wait for their neighbours
+  int s = 0;
+  for (int c = 0; c < chunks; c++) {
+    const int s_end = min(stages, ((rank * chunks + c + 1) * per - kbeg) / SP_KB);
+    float acc[TM][4];
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    for (; s < s_end; s++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(SP_STAGES - 2) : "memory");
+      __syncthreads();
+      const float* As = sm + s % SP_STAGES * STAGE; const float* Bs = As + SP_KB * BM;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {                           // four indices at a time
+        const int k = 8 * w + 4 * h; float a[4][TM], bv[4][4];
+        if (TM == 8 && h == 0) fetch(s + SP_STAGES - 1);      // into the stage that everybody has left behind
+#pragma unroll
+        for (int i = 0; i < TM; i += A_KFAST ? 1 : TM < 4 ? TM : 4) {
+          if (A_KFAST) {
+            const int r = mg * TM + i; const float4 x = *reinterpret_cast<const float4*>(As + r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2));
+            a[0][i] = x.x; a[1][i] = x.y; a[2][i] = x.z; a[3][i] = x.w;
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              const float* p = As + (k + q) * BM + mg * TM + i;
+              if (TM < 4) { const float2 x = *reinterpret_cast<const float2*>(p); a[q][i] = x.x; a[q][i + 1] = x.y; }
+              else { const float4 x = *reinterpret_cast<const float4*>(p); a[q][i] = x.x; a[q][(i + 1) % TM] = x.y; a[q][(i + 2) % TM] = x.z; a[q][(i + 3) % TM] = x.w; }
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (B_NFAST) {
+            const float4 x = *reinterpret_cast<const float4*>(Bs + (k + j) * SP_BN + 4 * ng); bv[j][0] = x.x; bv[j][1] = x.y; bv[j][2] = x.z; bv[j][3] = x.w;
+          } else {
+            const int r = 4 * ng + j; const float4 x = *reinterpret_cast<const float4*>(Bs + r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2));
+            bv[0][j] = x.x; bv[1][j] = x.y; bv[2][j] = x.z; bv[3][j] = x.w;
+          }
+        }
+        if (TM < 8 && h == 0) fetch(s + SP_STAGES - 1);       // (under the first loads, where the registers allow it)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+          for (int i = 0; i < TM; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[q][i], bv[q][j], acc[i][j]);
+        if (want_asum) {
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int i = 0; i < TM; i++) asum[i] += a[q][i];
+        }
+      }
+    }
+    if (c > 0) __syncthreads();                               // (the sums of the chunk before have been read)
+#pragma unroll
+    for (int i = 0; i < TM; i++) red[w * NV + (mg * TM + i) * 8 + ng] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    if (c + 1 == chunks && want_asum && ng == 0) {
+#pragma unroll
+      for (int i = 0; i < TM; i++) as_sm[w][mg * TM + i] = asum[i];
+    }
+    __syncthreads();
+    if (t < NV) {
+      v = red[t];
+#pragma unroll
+      for (int q = 1; q < 8; q++) v = add(v, red[q * NV + t]);
+      if (c & 1) {
+        v = add(s1, v);
+        if (c & 2) { v = add(s2, v); if (c & 4) v = add(s4, v); else s4 = v; } else s2 = v;
+      } else s1 = v;
+    }
+  }
+  float as = 0.f;
+  if (want_asum && t < BM) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) as += as_sm[q][t];
+  }
+  int at = t; bool mine = t < NV;                             // the four outputs this thread finishes
+  if (splits > 1) {
+    const int share = NV / splits;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (t < NV) cluster.map_shared_rank(xch, t / share)[rank * share + t % share] = v;
+    if (want_asum && t < BM) cluster.map_shared_rank(&as_x[0][0], 0)[rank * BM + t] = as;
+    cluster.sync();
+    mine = t < share; at = rank * share + t;
+    if (mine) {
+      v = add(xch[t], xch[share + t]);
+      if (splits > 2) v = add(v, add(xch[2 * share + t], xch[3 * share + t]));
+      if (splits > 4) v = add(v, add(add(xch[4 * share + t], xch[5 * share + t]), add(xch[6 * share + t], xch[7 * share + t])));
+    }
+    if (want_asum && rank == 0 && t < BM) { as = 0.f; for (int q = 0; q < splits; q++) as += as_x[q][t]; }
+  }
+  if (want_asum && rank == 0 && t < BM && m0 + t < g.M) g.a_sum[m0 + t] = as;
+  const int m = m0 + (at >> 3), n = n0 + (at & 7) * 4;
+  if (!mine || m >= g.M || n >= g.N) return;
+  float* c = C + (long)m * g.ldc + n; const float x[4] = {v.x, v.y, v.z, v.w}; float o[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) o[j] = n + j < g.N ? sg_finish(g, R, m, n + j, x[j]) : 0.f;
+  if (n + 3 < g.N && (reinterpret_cast<uintptr_t>(c) & 15) == 0) *reinterpret_cast<float4*>(c) = make_float4(o[0], o[1], o[2], o[3]);
+  else for (int j = 0; j < 4; j++) if (n + j < g.N) c[j] = o[j];
+}
+template <int TM>
+inline int gemm_small_tile(Ctx* ctx, const GemmDesc& g, int splits, int chunks, int per) {
+  auto vec = [](const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; };
+  const bool ak = g.sa_k == 1 && !g.a_sum, bn = g.sb_n == 1;      // (the sums of A's rows come with the other layout; one row has both)
+  const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
+  const int tiles_m = cdiv(g.M, 4 * TM), smem = sp_smem(TM);
+  for (int y0 = 0; y0 < tiles_m; y0 += 65535) {             // (a grid's second dimension)
+    const dim3 grid(cdiv(g.N, SP_BN) * splits, std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
+    auto run = [&](auto* K) -> int {
+      GN_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      GN_CLUSTER_LAUNCH(ctx, K, grid, SP_THREADS, smem, splits, g, splits, chunks, per, va, vb, y0); return GN_OK;
+    };
+    if (ak && bn) GN_TRY(run(gemm_small_kernel<TM, true, true>));
+    else if (ak && g.sb_k == 1) GN_TRY(run(gemm_small_kernel<TM, true, false>));
+    else if (g.sa_m == 1 && bn) GN_TRY(run(gemm_small_kernel<TM, false, true>));
+    else if (g.sa_m == 1 && g.sb_k == 1) GN_TRY(run(gemm_small_kernel<TM, false, false>));
+    else return fail(GN_ERR_UNSUPPORTED, "gemm_small: neither stride of an operand is 1");
+  }
+  return check_launch("gemm_small");
+}
+// How many chunks, and over how many blocks they go.  A chunk shorter than 64 indices (96 where a sample has more than 256 outputs) is not worth
+// its own sum; the number of chunks goes by the matrix alone where the rows of A are samples (or tokens), see above.  Blocks until
+// five eighths of the SMs have one, and, as two fit an SM, up to twice as many while a run is 384 indices or longer.
+inline int gemm_small(Ctx* ctx, const GemmDesc& g) {
+  const int tm = g.M <= 8 ? 2 : g.M <= 16 ? 4 : 8; const bool rows = g.sa_k == 1;
+  const long tn = cdiv(g.N, SP_BN), tiles = tn * cdiv(g.M, 4 * tm) * g.batch1 * g.batch2; const int run = rows && tn > 8 ? 96 : 64;
+  auto more = [&](long blocks, int n) { return blocks * n < 5L * ctx->sm_count / 8 || (blocks * n <= ctx->sm_count && g.K >= 384 * n); };
+  int all = 1, splits = 1;
+  while (all < SP_MAX_SPLITS && g.K >= 2 * run * all && more(rows ? tn : tiles, all)) all *= 2;
+  while (splits < all && more(tiles, splits)) splits *= 2;
+  const int per = cdiv(cdiv(g.K, all), SP_KB) * SP_KB, chunks = all / splits;
+  return tm == 2 ? gemm_small_tile<2>(ctx, g, splits, chunks, per) : tm == 4 ? gemm_small_tile<4>(ctx, g, splits, chunks, per) : gemm_small_tile<8>(ctx, g, splits, chunks, per);
+}
+
 template <int BM, int BN, int BK, int TM, int TN>
-inline int gemm_simt_tile(Ctx* ctx, const GemmDesc& g, int splits) {
+inline int gemm_simt_tile(Ctx* ctx, const GemmDesc& g) {
   auto vec = [](const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; };
   const bool ak = g.sa_k == 1, bn = g.sb_n == 1;
   const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
   const int tiles_m = cdiv(g.M, BM); constexpr int THREADS = SgCfg<BM, BN, BK, TM, TN>::THREADS;
   for (int y0 = 0; y0 < tiles_m; y0 += 65535) {             // (a grid's second dimension)
-    const dim3 grid(cdiv(g.N, BN) * splits, std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
-    if (ak && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
-    else if (ak && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
-    else if (g.sa_m == 1 && bn) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
-    else if (g.sa_m == 1 && g.sb_k == 1) GN_CLUSTER_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, 0, splits, g, splits, va, vb, y0);
+    const dim3 grid(cdiv(g.N, BN), std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
+    if (ak && bn) GN_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>), grid, THREADS, 0, g, va, vb, y0);
+    else if (ak && g.sb_k == 1) GN_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>), grid, THREADS, 0, g, va, vb, y0);
+    else if (g.sa_m == 1 && bn) GN_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>), grid, THREADS, 0, g, va, vb, y0);
+    else if (g.sa_m == 1 && g.sb_k == 1) GN_LAUNCH(ctx, (gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>), grid, THREADS, 0, g, va, vb, y0);
     else return fail(GN_ERR_UNSUPPORTED, "gemm_simt: neither stride of an operand is 1");
   }
   return check_launch("gemm_simt");
-}
-// Blocks per output tile.  A run shorter than 64 is not worth a block.  Where the rows of A are samples (or tokens), the
-// number does not depend on how many there are: a sample's result is the same in every batch.
-inline int gemm_simt_splits(const GemmDesc& g, int sm_count, long tiles_all, long tiles_n) {
-  const long have = g.sa_k == 1 ? tiles_n : tiles_all;
-  int s = 1;
-  while (s < SG_MAX_SPLITS && g.K >= 128 * s && have * s < sm_count) s *= 2;
-  return s;
 }
 inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
   if (g.M <= 0 || g.N <= 0) return GN_OK;
@@ -353,16 +546,19 @@ inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
     return check_launch("outer_sum");
   }
   if (gemm_skinny_ok(g)) {
-    int s = 1; while (s < SG_MAX_SPLITS && g.K >= 512 * s) s *= 2;
-    GN_CLUSTER_LAUNCH(ctx, gemm_skinny_kernel, dim3(g.M * s), 256, 0, s, g, s); return check_launch("gemm_skinny");
+    int s = 1; while (s < SP_MAX_SPLITS && g.K >= 512 * s) s *= 2;
+    if ((long)g.M * s > 4L * ctx->sm_count) GN_CLUSTER_LAUNCH(ctx, gemm_skinny_kernel<4>, dim3(cdiv(g.M, 4) * s), 256, 0, s, g, s);
+    else GN_CLUSTER_LAUNCH(ctx, gemm_skinny_kernel<1>, dim3(g.M * s), 256, 0, s, g, s);
+    return check_launch("gemm_skinny");
   }
-  const long nb = (long)g.batch1 * g.batch2, t64 = (long)cdiv(g.M, 64) * cdiv(g.N, 64) * nb;
-  const int s = gemm_simt_splits(g, ctx->sm_count, t64, (long)cdiv(g.N, 64));
+  // (which kernel adds up a sample's sums must not depend on the number of samples either)
+  const long t64 = (long)cdiv(g.M, 64) * cdiv(g.N, 64) * g.batch1 * g.batch2;
+  if (g.K >= SP_KB && (g.sa_k == 1 || t64 < ctx->sm_count) && (!g.a_sum || g.sa_m == 1)) return gemm_small(ctx, g);
   // 16-row tiles for a handful of rows; 32 x 32 tiles (a quarter of the work per block) when 64 x 64 would not give every SM one or
   // be half empty
-  if (g.M <= 16) return gemm_simt_tile<16, 64, 32, 2, 4>(ctx, g, s);
-  if (g.M <= 32 || t64 * s < ctx->sm_count) return gemm_simt_tile<32, 32, 32, 4, 2>(ctx, g, s);
-  return gemm_simt_tile<64, 64, 16, 4, 4>(ctx, g, s);
+  if (g.M <= 16) return gemm_simt_tile<16, 64, 32, 2, 4>(ctx, g);
+  if (g.M <= 32 || t64 < ctx->sm_count) return gemm_simt_tile<32, 32, 32, 4, 2>(ctx, g);
+  return gemm_simt_tile<64, 64, 16, 4, 4>(ctx, g);
 }
 
 }  // namespace gn

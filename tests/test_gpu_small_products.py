@@ -1,0 +1,61 @@
+"""The small-product kernel at the edges of its tiles (8, 16 and 32 rows by 32 columns), stages of 64 indices, chunks and clusters, with and
+without 16-byte copies, against float64."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from goneuron_b200 import _lib, configs, descriptors as D
+from tests.parity import TOL, assert_grads_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def device():
+    from goneuron_b200.sequential import Device
+    d = Device(0)
+    yield d
+    d.close()
+
+
+def product(device, A, B, bias):
+    f = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))
+    out = np.empty((A.shape[0], B.shape[0]), np.float32)
+    _lib.check(_lib.load().gn_op_gemm_nt(device.handle, 0, A.shape[0], B.shape[0], A.shape[1], f(A), f(B), f(bias), f(out)))
+    return out
+
+
+@pytest.mark.parametrize("N,K", [(17, 64), (32, 65), (33, 128), (100, 257), (256, 1024), (260, 191), (384, 1536), (1100, 333), (2047, 512), (37, 4099), (20, 8192)])
+def test_rows_against_float64_and_the_same_in_every_batch(device, N, K):
+    """A warp adds up K / 8 products at most, then come seven warps, at most three levels of chunks and the bias: every output is within
+    (K / 8 + 16) 2^-24 of the sum of magnitudes.  Rows do not depend on how many there are, whatever tile and cluster that gives."""
+    rng = np.random.Generator(np.random.PCG64(N + K))
+    A = rng.standard_normal((140, K)).astype(np.float32)
+    B = rng.standard_normal((N, K)).astype(np.float32)
+    bias = rng.standard_normal(N).astype(np.float32)
+    exact = A.astype(np.float64) @ B.astype(np.float64).T + bias
+    bound = (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T + np.abs(bias)) * (K / 8 + 16) * 2.0 ** -24
+    whole = product(device, A, B, bias)
+    assert np.all(np.abs(whole - exact) <= bound)
+    for m in (1, 7, 8, 9, 16, 17, 32, 33, 65):
+        assert np.array_equal(product(device, A[:m], B, bias), whole[:m]), m
+
+
+@pytest.mark.parametrize("I,H,O,batch", [(64, 64, 64, 64), (65, 33, 17, 65), (100, 200, 40, 70), (31, 129, 18, 300), (784, 128, 20, 127), (36, 300, 24, 1000), (9, 70, 1, 256)])
+def test_dense_gradients(device, oracle, I, H, O, batch):
+    """Input and weight gradients of Dense layers: the operands' other orders, and the bias gradients that come with them."""
+    from goneuron_b200.sequential import Adam, Sequential
+    layers = [D.Dense(I, H, D.TANH), D.Dense(H, O, D.LINEAR)]
+    rng = np.random.Generator(np.random.PCG64(I + batch))
+    params = configs.init_params(layers, rng)
+    x = rng.standard_normal((batch, I)).astype(np.float32)
+    y = rng.standard_normal((batch, O)).astype(np.float32)
+    ref = oracle.OracleState(layers, D.MSE, params, lr=1e-3)
+    loss_ref = ref.train_batch(x, y, threads=4, precision=64)
+    model = Sequential(layers, device).Compile(Adam(1e-3), D.MSE)
+    model.SetParams(params)
+    loss = model.TrainBatch(x, y)
+    assert abs(loss - loss_ref) <= TOL * max(1.0, abs(loss_ref))
+    assert_grads_close(layers, model.Gradients(), ref.grads)
+    model.Close()
