@@ -11,12 +11,12 @@
 namespace gn {
 
 // dst[ch * plane + r * ld + x] = src[ch][ylo + r][xlo + x], x < ld (a multiple of four), of `nch` channels with `rows` rows each; zero
-// outside the image and from channel `have` on.  All copies of a thread are in flight at once (one after the other, a load and
+// outside the image and from channel `have` on (bare: columns from W on are left alone).  All copies of a thread are in flight at once (one after the other, a load and
 // a store at a time, they were 60 us of the weight gradient); whole 16-byte pieces where the rows allow it and the
 // pointer does (`aligned`: decided by the host; a first layer reads the caller's batch).
-__device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const float* __restrict__ src, int nch, int have, int rows, int ylo, int H, int W, int xlo, bool aligned) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5; const bool v4 = aligned && xlo == 0 && ld == W;      // W a multiple of four
-  const int n = v4 ? ld >> 2 : ld, lw = n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32, step = nw * (32 / lw), lx = lane & (lw - 1);
+__device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const float* __restrict__ src, int nch, int have, int rows, int ylo, int H, int W, int xlo, bool aligned, bool bare = false) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5; const bool v4 = aligned && xlo == 0 && (W & 3) == 0 && (W == ld || bare);
+  const int n = v4 ? W >> 2 : ld, lw = n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32, step = nw * (32 / lw), lx = lane & (lw - 1);
   int q = warp * (32 / lw) + lane / lw, ch = q / rows, r = q - ch * rows;
   for (; ch < nch;) {
     const int y = ylo + r; const bool in = ch < have && y >= 0 && y < H; const float* s = src + ((long)ch * H + y) * W + xlo; float* d = dst + ch * plane + r * ld;
@@ -26,78 +26,132 @@ __device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const 
   }
 }
 
+// (Not inlined: 16 to 32 copies of all activations in an epilogue that runs once per thread came from a cold instruction cache, 14 us instead of 9 for
+// ReLU.  Four values at a time, so that they overlap.)
+__device__ __noinline__ float4 conv_act(int act, float4 v, float alpha) {
+  return make_float4(act_fwd(act, v.x, alpha), act_fwd(act, v.y, alpha), act_fwd(act, v.z, alpha), act_fwd(act, v.w, alpha));
+}
+
 // ------------------------------------------------------------------ forward and input gradient
 // dst[b, d, y, x] = act( bias[d] + sum_{s, kh, kw} w(d, s, kh, kw) src[b, s, y + kh - p, x + kw - p] ), zeros outside.  Forward: w = W[d][s].
 // Input gradient (BWD): src = gradient of the pre-activation, w = W[s][d] mirrored, p = K - 1 - pad.
-// A thread owns 4 neighbouring pixels x OC = 8 (or 4) channels; a block a band of `rb` rows of one image and `og` groups of OC
-// channels, with the source rows and the weights of `icc` source channels at a time in shared memory: 2 + 2 K 16-byte shared
-// loads per 32 K multiply-adds.
-struct ConvTile { int Cs, Cd, sH, sW, dH, dW, p, rb, og, icc, qw, swp, aligned; };
-template <int K, int OC, bool BWD>
+// A thread owns 4 neighbouring pixels of two rows x 4 channels and every `ks`-th source channel; a block a band of `rb` rows of one image and
+// `og` groups of 4 channels, with the source rows and the weights of `icc` source channels at a time in shared memory.  What bounds it is less
+// the arithmetic than everything around it: index arithmetic and uncoalesced copies on the way into shared memory, by few threads, took most
+// of its time.  So the weights are copied in their own order, image rows in 16-byte pieces where the window keeps the image's size (SAME; the border is
+// then left out where the pixels are read, not stored), and the input gradient's source channels are dealt out to `ks` groups of threads (by the
+// shapes alone: a sample's sums are the same in every batch), whose sums meet in shared memory.  A 3 x 3 window's weights stay in registers for both rows.
+// One row and up to 8 channels per thread, everything copied element by element in the order of shared memory -> this, us in a recorded chain: 3 -> 16 channels, 128
+// images of 32 x 32 14.3 -> 7.0; 16 -> 32, 16 x 16 forward 23.4 -> 13.4, input gradient 36.5 -> 13.2; 1 -> 24, 50 of 28 x 28 5.9 -> 4.5.
+struct ConvTile { int Cs, Cd, sH, sW, dH, dW, p, rb, og, icc, qw, swp, aligned, ks; };
+template <int K, bool BWD, bool SAME>
 __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict__ src, const float* __restrict__ W, const float* __restrict__ bias,
                                                         float* __restrict__ z, float* __restrict__ out, const ConvTile c, int act, float alpha) {
+  constexpr int KK = K * K, RP = 2, OC = 4, HALO = (K - 1) / 2;
   extern __shared__ __align__(16) float sm[];
-  const int rows = c.rb + K - 1, ocb = c.og * OC, tid = threadIdx.x;
-  float* xs = sm; float* ws = xs + c.icc * rows * c.swp;            // [icc][rows][swp], [icc][K K][ocb]
-  const int y0 = blockIdx.x * c.rb, b = blockIdx.y, d0 = blockIdx.z * ocb;
-  const int px = tid % (c.rb * c.qw), g = tid / (c.rb * c.qw), ry = px / c.qw, qx = px - ry * c.qw; const bool live = g < c.og;
+  const int rows = c.rb + K - 1, ocb = c.og * OC, wn = BWD ? ocb * KK : c.icc * KK | 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  float* xs = sm; float* ws = xs + c.icc * rows * c.swp;            // [icc][rows][swp]; weights [ocb][wn] (forward: icc K K of them, odd: channel groups in different banks) or [icc][wn]
+  const int y0 = blockIdx.x * c.rb, b = blockIdx.y, d0 = blockIdx.z * ocb, npx = c.rb / RP * c.qw;
+  const int px = tid % npx, gk = tid / npx, g = gk % c.og, kq = gk / c.og, ry = px / c.qw * RP, qx = px % c.qw; const bool live = kq < c.ks;
   const float* sb = src + (long)b * c.Cs * c.sH * c.sW;
-  float acc[OC][4];
+  float acc[RP][OC][4];
 #pragma unroll
-  for (int o = 0; o < OC; o++) { acc[o][0] = acc[o][1] = acc[o][2] = acc[o][3] = 0.f; }
+  for (int r = 0; r < RP; r++)
+#pragma unroll
+    for (int o = 0; o < OC; o++) { acc[r][o][0] = acc[r][o][1] = acc[r][o][2] = acc[r][o][3] = 0.f; }
   for (int s0 = 0; s0 < c.Cs; s0 += c.icc) {
     const int ns = min(c.icc, c.Cs - s0);
     if (s0 > 0) __syncthreads();
-    conv_stage(xs, rows * c.swp, c.swp, sb + (long)s0 * c.sH * c.sW, ns, ns, rows, y0 - c.p, c.sH, c.sW, -c.p, c.aligned);
-    for (int e = tid; e < ocb * ns * K * K; e += blockDim.x) {
-      const int o = e % ocb, r = e / ocb, t = r % (K * K), s = r / (K * K);      // neighbouring threads, neighbouring words of shared memory
-      const bool in = d0 + o < c.Cd;
-      const float* wp = BWD ? W + ((long)(s0 + s) * c.Cd + d0 + o) * (K * K) + (K * K - 1 - t) : W + ((long)(d0 + o) * c.Cs + s0 + s) * (K * K) + t;
-      cp_async4(ws + (s * K * K + t) * ocb + o, in ? wp : W, in);
+    conv_stage(xs, rows * c.swp, c.swp, sb + (long)s0 * c.sH * c.sW, ns, ns, rows, y0 - c.p, c.sH, c.sW, SAME ? 0 : -c.p, c.aligned, SAME);
+    for (int k = warp; k < (BWD ? ns : ocb); k += nw) {              // a warp per run of the weights
+      const float* q = BWD ? W + ((long)(s0 + k) * c.Cd + d0) * KK : W + ((long)(d0 + k) * c.Cs + s0) * KK;
+      const int n = BWD ? wn : ns * KK, have = BWD ? min(ocb, c.Cd - d0) * KK : d0 + k < c.Cd ? n : 0;
+#pragma unroll 4
+      for (int e = lane; e < n; e += 32) cp_async4(ws + k * wn + e, e < have ? q + e : W, e < have);
     }
     cp_async_wait();
     __syncthreads();
-    if (live) for (int s = 0; s < ns; s++) {
+    if (live) for (int s = kq; s < ns; s += c.ks) {
+      const float* xr = xs + (s * rows + ry) * c.swp + 4 * qx; const float* wr = BWD ? ws + s * wn + OC * KK * g : ws + OC * wn * g + s * KK;
+      auto weight = [&](int t, int o) -> float { return BWD ? wr[o * KK + KK - 1 - t] : wr[o * wn + t]; };
+      auto row = [&](int r, float (&v)[8]) {                        // v[kw + i]: source column 4 qx + i + kw - p
+        const float* q = xr + r * c.swp; const float4 m = *reinterpret_cast<const float4*>(q);
+        if (SAME) {
+          v[HALO] = m.x; v[HALO + 1] = m.y; v[HALO + 2] = m.z; v[HALO + 3] = m.w;
+          if constexpr (K == 3) { v[0] = qx > 0 ? q[-1] : 0.f; v[5] = qx + 1 < c.qw ? q[4] : 0.f; }
+          if constexpr (K == 5) {
+            const float2 zero = make_float2(0.f, 0.f), l = qx > 0 ? *reinterpret_cast<const float2*>(q - 2) : zero, h = qx + 1 < c.qw ? *reinterpret_cast<const float2*>(q + 4) : zero;
+            v[0] = l.x; v[1] = l.y; v[6] = h.x; v[7] = h.y;
+          }
+        } else {
+          v[0] = m.x; v[1] = m.y; v[2] = m.z; v[3] = m.w;
+          if (K > 1) *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(q + 4);
+        }
+      };
+      float w[K == 5 ? K : KK][OC];
+      if constexpr (K < 5) {
 #pragma unroll
-      for (int kh = 0; kh < K; kh++) {
-        const float* xr = xs + (s * rows + ry + kh) * c.swp + 4 * qx;
-        float v[8];
-        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(xr);
-        if (K > 1) *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(xr + 4);
+        for (int t = 0; t < KK; t++)
 #pragma unroll
-        for (int kw = 0; kw < K; kw++) {
-          const float* wr = ws + (s * K * K + kh * K + kw) * ocb + OC * g;
-          float wv[OC];
+          for (int o = 0; o < OC; o++) w[t][o] = weight(t, o);
+      }
 #pragma unroll
-          for (int o = 0; o < OC; o += 4) *reinterpret_cast<float4*>(wv + o) = *reinterpret_cast<const float4*>(wr + o);
+      for (int r = 0; r < K + RP - 1; r++) {
+        float v[8]; row(r, v);
 #pragma unroll
-          for (int o = 0; o < OC; o++)
+        for (int k = 0; k < RP; k++) if (r - k >= 0 && r - k < K) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) acc[o][i] = fmaf(wv[o], v[kw + i], acc[o][i]);
+          for (int kw = 0; kw < K; kw++) {
+            const int t = (r - k) * K + kw;
+#pragma unroll
+            for (int o = 0; o < OC; o++) {
+              const float wv = K < 5 ? w[K < 5 ? t : 0][o] : weight(t, o);
+#pragma unroll
+              for (int i = 0; i < 4; i++) acc[k][o][i] = fmaf(wv, v[kw + i], acc[k][o][i]);
+            }
+          }
         }
       }
     }
   }
-  const int y = y0 + ry;
-  if (!live || y >= c.dH) return;
-#pragma unroll
-  for (int o = 0; o < OC; o++) {
-    const int d = d0 + OC * g + o; if (d >= c.Cd) break;
+  auto finish = [&](int r, int o, float (&v)[4]) {
+    const int y = y0 + ry + r, d = d0 + OC * g + o; if (y >= c.dH || d >= c.Cd) return;
     const float bv = bias ? bias[d] : 0.f; const long at = (((long)b * c.Cd + d) * c.dH + y) * c.dW + 4 * qx;
-    float v[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = acc[o][i] + bv;
+    for (int i = 0; i < 4; i++) v[i] += bv;
     if (z) {
 #pragma unroll
       for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) z[at + i] = v[i];
     }
+    if (act == GN_ACT_RELU) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = act_fwd(act, v[i], alpha);
+      for (int i = 0; i < 4; i++) v[i] = v[i] > 0.f ? v[i] : 0.f;
+    } else if (act != GN_ACT_LINEAR) { const float4 a = conv_act(act, make_float4(v[0], v[1], v[2], v[3]), alpha); v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; }
     if ((c.dW & 3) == 0) *reinterpret_cast<float4*>(out + at) = make_float4(v[0], v[1], v[2], v[3]);
     else {
 #pragma unroll
       for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) out[at + i] = v[i];
     }
+  };
+  if (c.ks > 1) {                                                    // the groups' sums, in order; every group finishes a share of the rows and channels
+    const int all = npx * c.og, at = tid - kq * all;
+    __syncthreads();
+    if (live) {
+#pragma unroll
+      for (int e = 0; e < RP * OC * 4; e++) sm[(kq * RP * OC * 4 + e) * all + at] = acc[e / (OC * 4)][e / 4 % OC][e % 4];
+    }
+    __syncthreads();
+    if (live) for (int q = kq; q < RP * OC; q += c.ks) {
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int k = 0; k < c.ks; k++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] += sm[(k * RP * OC * 4 + q * 4 + i) * all + at];
+      }
+      finish(q / OC, q % OC, v);
+    }
+  } else if (live) {
+#pragma unroll
+    for (int q = 0; q < RP * OC; q++) finish(q / OC, q % OC, acc[q / OC][q % OC]);
   }
 }
 
@@ -105,7 +159,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict_
 // dW[o, s, kh, kw] = sum_{b, y, x} g[b, o, y, x] src[b, s, y + kh - p, x + kw - p].  A thread owns OT output channels x one input channel x all
 // taps and walks the rows y = pg (mod PG) of a band, four pixels at a time: K 2 + OT 16-byte shared loads per 4 OT K^2
 // multiply-adds.  A block takes the bands of several images in turn (unit = image, band) and leaves one set of partial sums;
-// conv_wgrad_final_kernel adds the blocks' sets in order.  Channel planes in shared memory lie 4 (mod 8) floats apart, so that
+// conv_wgrad_tile_final_kernel adds the blocks' sets in order.  Channel planes in shared memory lie 4 (mod 8) floats apart, so that
 // the lanes of a warp (neighbouring channels) hit different banks.
 struct ConvWg { int Cs, Cd, H, W, oH, oW, p, rb, bands, ocb, icb, pg, swp, gwp, xplane, gplane, units, aligned; };
 template <int K> struct ConvWgOT { static constexpr int v = K == 1 ? 8 : K == 3 ? 4 : 2; };
@@ -153,7 +207,7 @@ __global__ void __launch_bounds__(256) conv_wgrad_tile_kernel(const float* __res
     }
   }
   // the pixel groups' sums, in order, through shared memory
-  constexpr int NV = OT * (KK + 1); const int nW = c.Cd * c.Cs * KK, all = items * c.pg; float* prow = part + (long)blockIdx.x * (nW + c.Cd);
+  constexpr int NV = OT * (KK + 1); const int all = items * c.pg; float* prow = part + ((long)blockIdx.x * gridDim.y + blockIdx.y) * items * NV;
   float* red = sm;                                                   // [NV][pg][items]
   __syncthreads();
   if (live) {
@@ -165,12 +219,10 @@ __global__ void __launch_bounds__(256) conv_wgrad_tile_kernel(const float* __res
     }
   }
   __syncthreads();
-  for (int e = tid; e < items * NV; e += blockDim.x) {
-    const int q = e % items, v = e / items, o = v / (KK + 1), t = v - o * (KK + 1), d = o0 + (q / c.icb) * OT + o, s = i0 + q % c.icb;
-    if (d >= c.Cd || s >= c.Cs || (t == KK && s > 0)) continue;
+  if (live) for (int v = pg; v < NV; v += c.pg) {                    // (in the order of the threads; the kernel below finds the places)
     float a = 0.f;
-    for (int k = 0; k < c.pg; k++) a += red[v * all + k * items + q];
-    prow[t < KK ? ((long)d * c.Cs + s) * KK + t : (long)nW + d] = a;
+    for (int k = 0; k < c.pg; k++) a += red[v * all + k * items + it];
+    prow[v * items + it] = a;
   }
 }
 // dst[i] = sum over the blocks' sets, in order: 32 elements x 8 groups of sets per block (weights, then biases: the gradient slice is laid out W | b)
@@ -189,6 +241,26 @@ __global__ void __launch_bounds__(256) conv_wgrad_final_kernel(const float* __re
     dst[i] = s;
   }
 }
+// The same for the sets of conv_wgrad_tile_kernel; an element's place in a set: channel tile, OT x (taps, bias), item.
+template <int K>
+__global__ void __launch_bounds__(256) conv_wgrad_tile_final_kernel(const float* __restrict__ part, int sets, int n, float* __restrict__ dst, const ConvWg c) {
+  constexpr int OT = ConvWgOT<K>::v, KK = K * K, NV = OT * (KK + 1);
+  __shared__ float red[8][33];
+  const int tx = threadIdx.x & 31, grp = threadIdx.x >> 5, i = blockIdx.x * 32 + tx, items = c.ocb / OT * c.icb;
+  float s = 0.f;
+  if (i < n) {
+#pragma unroll 8
+    for (int k = grp; k < sets; k += 8) s += part[(long)k * n + i];
+  }
+  red[grp][tx] = s;
+  __syncthreads();
+  if (grp > 0 || i >= n) return;
+  const int tile = i / (items * NV), e = i - tile * items * NV, v = e / items, q = e - v * items, ict = (c.Cs + c.icb - 1) / c.icb;
+  const int o = v / (KK + 1), t = v - o * (KK + 1), d = tile / ict * c.ocb + q / c.icb * OT + o, s_ = tile % ict * c.icb + q % c.icb;
+  if (d >= c.Cd || s_ >= c.Cs || (t == KK && s_ > 0)) return;
+  for (int k = 1; k < 8; k++) s += red[k][tx];
+  dst[t < KK ? ((long)d * c.Cs + s_) * KK + t : (long)c.Cd * c.Cs * KK + d] = s;
+}
 
 // ------------------------------------------------------------------ host side
 constexpr size_t CD_SMEM = 96 * 1024;
@@ -201,38 +273,48 @@ inline bool conv_direct_supported(const ConvShape& c) {
 // 64 -> 128: 219 / 217 / 218 against 147 / 312 / 271; 128 -> 128: 427 / 379 / 422 against 270 / 571 / 274.
 inline bool conv_direct_preferred(const ConvShape& c) { return conv_direct_supported(c) && (long)c.inC * c.outC * c.k * c.k <= 64L * 96 * 9; }
 
-template <int K, int OC, bool BWD>
+template <int K, bool BWD, bool SAME>
 inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
-  c.aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  c.qw = cdiv(c.dW, 4); c.swp = 4 * c.qw + (K > 1 ? 4 : 0);
-  const int groups = cdiv(c.Cd, OC);
-  c.og = std::min(groups, std::max(1, std::min(32 / OC, 256 / c.qw)));
-  c.rb = std::max(1, std::min(c.dH, 256 / (c.qw * c.og)));
-  // at least three blocks per SM, so that one computes while another's copies are under way
-  while (c.rb > 1 && c.rb * c.qw * c.og > 64 && (long)B * cdiv(c.dH, c.rb) * cdiv(groups, c.og) < 3L * ctx->sm_count) c.rb = (c.rb + 1) / 2;
+  constexpr int RP = 2, OC = 4;
+  c.qw = cdiv(c.dW, 4); c.swp = SAME ? c.sW : 4 * c.qw + (K > 1 ? 4 : 0);
+  if (SAME && (c.qw == 2 || c.qw == 4)) while (RP * c.swp % 32 != 4 * c.qw) c.swp += 4;      // neighbouring rows of threads in neighbouring banks
+  const int groups = cdiv(c.Cd, OC), row_groups = cdiv(c.dH, RP);                 // groups of two rows
+  // Input gradients: source channels in up to four groups of threads while a block still has three groups of rows (or all).  us with 1 / 2 / 4: 16 -> 32
+  // channels, 128 images of 16 x 16 17.0 / 14.2 / 13.2; 32 -> 64, 64 of 20 x 20 43 / 41 / 48; 16 -> 64, 20 of 16 x 16 30 / 21 / 15.  Forward in one group: a block has
+  // enough threads there (13.4 / - / 15.3), and ReLU and pooling see sums in the order of the channels.
+  c.ks = !BWD ? 1 : c.Cs >= 16 ? 4 : c.Cs >= 8 ? 2 : 1;
+  while (c.ks > 1 && 256 / c.ks < c.qw * std::min(groups, 32 / OC) * std::min(row_groups, 3)) c.ks /= 2;
+  const int most = 256 / c.ks;
+  c.og = std::min(groups, std::max(1, std::min(32 / OC, most / c.qw)));
+  int rg = std::max(1, std::min(row_groups, most / (c.qw * c.og)));
+  // three blocks for two SMs at least (one each: 13 % slower for 50 images of 28 x 28, three each: 14 % for 16 -> 32 channels)
+  while (rg > 1 && rg * c.qw * c.og * c.ks > 64 && 2L * B * cdiv(row_groups, rg) * cdiv(groups, c.og) < 3L * ctx->sm_count) rg = (rg + 1) / 2;
+  rg = cdiv(row_groups, cdiv(row_groups, rg));                       // even bands
+  c.rb = rg * RP;
   const size_t per = ((size_t)(c.rb + K - 1) * c.swp + (size_t)K * K * c.og * OC) * sizeof(float);
   c.icc = std::max<int>(1, std::min<int>(c.Cs, 48 * 1024 / per));
-  const size_t smem = c.icc * per; const int threads = (c.qw * c.rb * c.og + 31) & ~31;
-  GN_CUDA(cudaFuncSetAttribute(conv_tile_kernel<K, OC, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GN_LAUNCH(ctx, (conv_tile_kernel<K, OC, BWD>), dim3(cdiv(c.dH, c.rb), B, cdiv(groups, c.og)), threads, smem, src, W, bias, z, out, c, act, alpha);
+  if (c.icc < c.Cs) c.icc = std::max(c.ks, c.icc / c.ks * c.ks);     // (a channel's group of threads does not depend on how many are staged at once)
+  const int all = c.qw * rg * c.og, threads = (all * c.ks + 31) & ~31;
+  const size_t smem = std::max(c.icc * per + (size_t)c.og * OC * sizeof(float), (size_t)(c.ks > 1 ? c.ks : 0) * RP * OC * 4 * all * sizeof(float));
+  GN_CUDA(cudaFuncSetAttribute(conv_tile_kernel<K, BWD, SAME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GN_LAUNCH(ctx, (conv_tile_kernel<K, BWD, SAME>), dim3(cdiv(c.dH, c.rb), B, cdiv(groups, c.og)), threads, smem, src, W, bias, z, out, c, act, alpha);
   return check_launch("conv_tile");
 }
 template <int K, bool BWD>
-inline int conv_tile_launch(Ctx* ctx, int B, const ConvTile& c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
-  // four channels per thread where eight would not give every SM sub-partition three warps (or where there are no more)
-  const long warps = (long)B * c.dH * cdiv(c.dW, 4) * cdiv(c.Cd, 8) / 32;
-  if (c.Cd <= 4 || warps < 12L * ctx->sm_count) return conv_tile_run<K, 4, BWD>(ctx, B, c, src, W, bias, z, out, act, alpha);
-  return conv_tile_run<K, 8, BWD>(ctx, B, c, src, W, bias, z, out, act, alpha);
+inline int conv_tile_launch(Ctx* ctx, int B, ConvTile c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
+  c.aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  if (c.aligned && c.sW % 4 == 0 && c.dW == c.sW && 2 * c.p == K - 1) return conv_tile_run<K, BWD, true>(ctx, B, c, src, W, bias, z, out, act, alpha);
+  return conv_tile_run<K, BWD, false>(ctx, B, c, src, W, bias, z, out, act, alpha);
 }
 // z may be null (LINEAR, RELU)
 inline int conv_direct_forward(Ctx* ctx, const ConvShape& s, const float* x, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
-  const ConvTile c{s.inC, s.outC, s.H, s.W, s.oH, s.oW, s.p};
+  ConvTile c{s.inC, s.outC, s.H, s.W, s.oH, s.oW, s.p};
   if (s.k == 1) return conv_tile_launch<1, false>(ctx, s.B, c, x, W, bias, z, out, act, alpha);
   if (s.k == 3) return conv_tile_launch<3, false>(ctx, s.B, c, x, W, bias, z, out, act, alpha);
   return conv_tile_launch<5, false>(ctx, s.B, c, x, W, bias, z, out, act, alpha);
 }
 inline int conv_direct_dgrad(Ctx* ctx, const ConvShape& s, const float* g, const float* W, float* dx) {
-  const ConvTile c{s.outC, s.inC, s.oH, s.oW, s.H, s.W, s.k - 1 - s.p};
+  ConvTile c{s.outC, s.inC, s.oH, s.oW, s.H, s.W, s.k - 1 - s.p};
   if (s.k == 1) return conv_tile_launch<1, true>(ctx, s.B, c, g, W, nullptr, nullptr, dx, GN_ACT_LINEAR, 0.f);
   if (s.k == 3) return conv_tile_launch<3, true>(ctx, s.B, c, g, W, nullptr, nullptr, dx, GN_ACT_LINEAR, 0.f);
   return conv_tile_launch<5, true>(ctx, s.B, c, g, W, nullptr, nullptr, dx, GN_ACT_LINEAR, 0.f);
@@ -261,17 +343,17 @@ inline ConvWg conv_wgrad_plan(Ctx* ctx, const ConvShape& s, int OT, int* sets, s
   return c;
 }
 inline size_t conv_wgrad_part_floats(Ctx* ctx, const ConvShape& s) {
-  int sets; size_t smem; conv_wgrad_plan(ctx, s, s.k == 1 ? 8 : s.k == 3 ? 4 : 2, &sets, &smem);
-  return (size_t)sets * ((size_t)s.outC * s.inC * s.k * s.k + s.outC);
+  const int OT = s.k == 1 ? 8 : s.k == 3 ? 4 : 2; int sets; size_t smem; const ConvWg c = conv_wgrad_plan(ctx, s, OT, &sets, &smem);
+  return (size_t)sets * cdiv(s.inC, c.icb) * cdiv(s.outC, c.ocb) * c.icb * c.ocb * (s.k * s.k + 1);
 }
 template <int K>
 inline int conv_wgrad_launch(Ctx* ctx, const ConvShape& s, const float* g, const float* x, float* part, float* gW) {
   constexpr int OT = ConvWgOT<K>::v; int sets; size_t smem;
   ConvWg c = conv_wgrad_plan(ctx, s, OT, &sets, &smem); c.aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  const int items = c.ocb / OT * c.icb, threads = (items * c.pg + 31) & ~31, n = s.outC * s.inC * K * K + s.outC;
+  const int items = c.ocb / OT * c.icb, threads = (items * c.pg + 31) & ~31, tiles = cdiv(s.inC, c.icb) * cdiv(s.outC, c.ocb), n = tiles * items * OT * (K * K + 1);
   GN_CUDA(cudaFuncSetAttribute(conv_wgrad_tile_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GN_LAUNCH(ctx, conv_wgrad_tile_kernel<K>, dim3(sets, cdiv(s.inC, c.icb) * cdiv(s.outC, c.ocb)), threads, smem, g, x, part, c);
-  GN_LAUNCH(ctx, conv_wgrad_final_kernel, cdiv(n, 32), 256, 0, (const float*)part, sets, n, gW);
+  GN_LAUNCH(ctx, conv_wgrad_tile_kernel<K>, dim3(sets, tiles), threads, smem, g, x, part, c);
+  GN_LAUNCH(ctx, conv_wgrad_tile_final_kernel<K>, cdiv(n, 32), 256, 0, (const float*)part, sets, n, gW, c);
   return check_launch("conv_wgrad");
 }
 // weight and bias gradients (gb follows gW); `part`: conv_wgrad_part_floats

@@ -28,6 +28,8 @@ def _f(a):
     (1, 1, 1, 1, 0, 1, 1, D.LINEAR), (2, 3, 8, 1, 0, 5, 7, D.RELU), (3, 9, 17, 3, 1, 7, 6, D.RELU), (2, 5, 7, 3, 0, 9, 10, D.TANH), (1, 33, 40, 3, 2, 12, 13, D.RELU),
     (200, 1, 24, 3, 1, 28, 28, D.RELU), (2, 70, 65, 3, 1, 8, 8, D.LINEAR), (3, 4, 6, 5, 2, 31, 33, D.SIGMOID), (2, 40, 9, 5, 4, 6, 5, D.RELU), (1, 2, 3, 3, 1, 300, 301, D.RELU),
     (2, 3, 100, 3, 1, 40, 40, D.RELU), (4, 16, 4, 3, 1, 2, 3, D.LINEAR),
+    # windows that keep an image of whole 16-byte pieces: widths of 4 to 508, odd heights, channels dealt out to one, two and four groups, more than are staged at once
+    (3, 5, 6, 3, 1, 3, 4, D.TANH), (2, 9, 18, 3, 1, 7, 8, D.RELU), (2, 17, 33, 5, 2, 9, 16, D.RELU), (1, 8, 20, 3, 1, 4, 508, D.LINEAR), (2, 130, 19, 3, 1, 11, 20, D.TANH), (5, 20, 12, 1, 0, 5, 12, D.RELU),
     (2, 3, 4, 3, 1, 5, 513, D.RELU), (1, 2, 5, 5, 2, 7, 520, D.TANH), (1, 2, 3, 3, 3, 6, 9, D.RELU), (1, 2, 3, 1, 0, 3, 600, D.RELU)])      # the plain kernels' side of the limits
 def test_conv_direct(device, B, inC, outC, k, p, H, W, act):
     from goneuron_b200 import _lib
