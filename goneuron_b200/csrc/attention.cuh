@@ -323,6 +323,166 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 3 : 4) attn_bwd_kernel(
   at_store<HD>(dK, ak, 1.f, 1.f, base, j0, j1, T, D, t); at_store<HD>(dV, av, 1.f, 1.f, base, j0, j1, T, D, t);
 }
 
+// ---------------------------------------------------------------- whole heads
+// The same arithmetic in the same order, a block per head: short sequences fit shared memory as a whole, so every tensor is read and split
+// once (the blocks of 64 rows above read and split each one again for every block of the other side, between two barriers, with nothing in flight meanwhile)
+// and then every warp walks its rows by itself.  Rows are padded to 32, and keys (queries) go 32 at a time where 64 are not there: what is
+// left out is masked or zero.  With a causal mask a warp's query rows and key rows cost the same together, whichever they are.  Bound by
+// the latency of its chains of dependent MMAs and element-wise work; figures at at_head_better.
+__host__ __device__ __forceinline__ int at_pad(int T) { return (T + 31) & ~31; }
+template <int HD> inline size_t at_head_smem(int T, bool bwd) { return (size_t)at_pad(T) * ((bwd ? 4 : 3) * AtCfg<HD>::LDH * sizeof(__half) + (bwd ? 7 : 3) * sizeof(float)); }
+// all rows of a head (zeros from T to the padded end); see at_load
+template <int HD, bool DOT>
+__device__ __forceinline__ void at_load_head(__half* s, float* inv, const float* __restrict__ src, long base, int T, int D, const float* __restrict__ other = nullptr, float* dot = nullptr) {
+  using C = AtCfg<HD>; constexpr int NP = DOT ? 2 : 4;
+  const int c4 = threadIdx.x % C::V4, step = blockDim.x / C::V4, Tp = at_pad(T);
+  for (int p0 = threadIdx.x / C::V4; p0 - (int)(threadIdx.x / C::V4) < Tp; p0 += NP * step) {      // (the same number of rounds in every thread)
+    float4 v[NP], w[DOT ? NP : 1];
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+      const int row = p0 + p * step; const long o = base + (long)row * D + c4 * 4;
+      v[p] = row < T ? *reinterpret_cast<const float4*>(src + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (DOT) w[p] = row < T ? *reinterpret_cast<const float4*>(other + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+      const int r = p0 + p * step;
+      float mx = fmaxf(fmaxf(fabsf(v[p].x), fabsf(v[p].y)), fmaxf(fabsf(v[p].z), fabsf(v[p].w))), d = 0.f;
+      if constexpr (DOT) d = (v[p].x * w[p].x + v[p].y * w[p].y) + (v[p].z * w[p].z + v[p].w * w[p].w);
+#pragma unroll
+      for (int o = C::V4 / 2; o > 0; o >>= 1) { mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); if constexpr (DOT) d += __shfl_xor_sync(0xffffffffu, d, o); }
+      float iv; const float sc = row_scale(mx, &iv);
+      uint2 hi, lo; split2_pair(v[p].x, v[p].y, sc, hi.x, lo.x); split2_pair(v[p].z, v[p].w, sc, hi.y, lo.y);
+      if (r < Tp) {
+        *reinterpret_cast<uint2*>(s + r * C::LDH + c4 * 4) = hi; *reinterpret_cast<uint2*>(s + r * C::LDH + HD + c4 * 4) = lo;
+        if (c4 == 0) { inv[r] = iv; if constexpr (DOT) dot[r] = d; }
+      }
+    }
+  }
+}
+template <int HD, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) attn_head_fwd_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
+                                                                      float* __restrict__ O, float* __restrict__ Mst, float* __restrict__ Lst, int T, int D, int H, int causal, float inv_scale) {
+  using C = AtCfg<HD>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  const int Tp = at_pad(T), h = blockIdx.x, b = blockIdx.y, nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  __half* Qs = reinterpret_cast<__half*>(at_sm); __half* Ks = Qs + Tp * C::LDH; __half* Vs = Ks + Tp * C::LDH;
+  float* iq = reinterpret_cast<float*>(Vs + Tp * C::LDH); float* ik = iq + Tp; float* iv = ik + Tp;
+  const long base = (long)b * T * D + (long)h * HD, sb = ((long)b * H + h) * T;
+  at_load_head<HD, false>(Qs, iq, Q, base, T, D); at_load_head<HD, false>(Ks, ik, K, base, T, D); at_load_head<HD, false>(Vs, iv, V, base, T, D);
+  __syncthreads();
+  for (int r0 = warp * 16; r0 < T; r0 += nw * 16) {
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[HD / 8][4];
+#pragma unroll
+    for (int i = 0; i < HD / 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    const int i0 = r0 + g, i1 = i0 + 8, kend = causal ? min(Tp, at_pad(r0 + 16)) : Tp;
+    const float f0 = iq[i0] * inv_scale, f1 = iq[i1] * inv_scale;
+    auto block = [&](int k0, auto nn) {
+      constexpr int NN = decltype(nn)::value;
+      float s[NN][4]; at_rows_product<HD, NN>(s, Qs, Ks + k0 * C::LDH, r0, lane);
+      const bool edge = k0 + 8 * NN > T || (causal && k0 + 8 * NN > r0);
+      float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+      for (int n = 0; n < NN; n++) {
+        const float2 kk = *reinterpret_cast<const float2*>(ik + k0 + n * 8 + 2 * t);
+        s[n][0] *= f0 * kk.x; s[n][1] *= f0 * kk.y; s[n][2] *= f1 * kk.x; s[n][3] *= f1 * kk.y;
+        if (edge) {
+#pragma unroll
+          for (int e = 0; e < 4; e++) { const int j = k0 + n * 8 + 2 * t + (e & 1); if (j >= T || (causal && j > (e < 2 ? i0 : i1))) s[n][e] = -INFINITY; }
+        }
+        mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1])); mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
+      }
+      const float mn0 = fmaxf(m[0], quad_max(mx0)), mn1 = fmaxf(m[1], quad_max(mx1));
+      const float c0 = __expf(m[0] - mn0), c1 = __expf(m[1] - mn1);
+      float rs0 = 0.f, rs1 = 0.f;
+#pragma unroll
+      for (int n = 0; n < NN; n++) {
+        s[n][0] = __expf(s[n][0] - mn0); s[n][1] = __expf(s[n][1] - mn0); s[n][2] = __expf(s[n][2] - mn1); s[n][3] = __expf(s[n][3] - mn1);
+        rs0 += s[n][0] + s[n][1]; rs1 += s[n][2] + s[n][3];
+      }
+      l[0] = l[0] * c0 + quad_sum(rs0); l[1] = l[1] * c1 + quad_sum(rs1); m[0] = mn0; m[1] = mn1;
+      at_sum_rows<HD, NN>(o, c0, c1, s, Vs + k0 * C::LDH, iv + k0, lane);
+    };
+    int k0 = 0;
+    for (; k0 + 64 <= kend; k0 += 64) block(k0, std::integral_constant<int, 8>{});
+    if (k0 < kend) block(k0, std::integral_constant<int, 4>{});
+    at_store<HD>(O, o, 1.f / l[0], 1.f / l[1], base, i0, i1, T, D, t);
+    if (t == 0) {
+      if (i0 < T) { Mst[sb + i0] = m[0]; Lst[sb + i0] = l[0]; }
+      if (i1 < T) { Mst[sb + i1] = m[1]; Lst[sb + i1] = l[1]; }
+    }
+  }
+}
+template <int HD, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) attn_head_bwd_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ O,
+                                                                      const float* __restrict__ dO, const float* __restrict__ Mst, const float* __restrict__ Lst,
+                                                                      float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV, int T, int D, int H, int causal, float inv_scale) {
+  using C = AtCfg<HD>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  const int Tp = at_pad(T), h = blockIdx.x, b = blockIdx.y, nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  __half* Qs = reinterpret_cast<__half*>(at_sm); __half* Gs = Qs + Tp * C::LDH; __half* Ks = Gs + Tp * C::LDH; __half* Vs = Ks + Tp * C::LDH;
+  float* iq = reinterpret_cast<float*>(Vs + Tp * C::LDH); float* ig = iq + Tp; float* ik = ig + Tp; float* iv = ik + Tp; float* st_m = iv + Tp; float* st_il = st_m + Tp; float* st_d = st_il + Tp;
+  const long base = (long)b * T * D + (long)h * HD, sb = ((long)b * H + h) * T;
+  for (int i = threadIdx.x; i < Tp; i += blockDim.x) { st_m[i] = i < T ? Mst[sb + i] : 0.f; st_il[i] = i < T ? 1.f / Lst[sb + i] : 0.f; }
+  at_load_head<HD, false>(Qs, iq, Q, base, T, D); at_load_head<HD, true>(Gs, ig, dO, base, T, D, O, st_d);
+  at_load_head<HD, false>(Ks, ik, K, base, T, D); at_load_head<HD, false>(Vs, iv, V, base, T, D);
+  __syncthreads();
+  for (int r0 = warp * 16; r0 < T; r0 += nw * 16) {
+    {   // dQ of 16 query rows
+      const int i0 = r0 + g, i1 = i0 + 8, kend = causal ? min(Tp, at_pad(r0 + 16)) : Tp;
+      const float m0 = st_m[i0], m1 = st_m[i1], il0 = st_il[i0], il1 = st_il[i1], d0 = st_d[i0], d1 = st_d[i1], f0 = iq[i0] * inv_scale, f1 = iq[i1] * inv_scale, g0 = ig[i0], g1 = ig[i1];
+      float acc[HD / 8][4];
+#pragma unroll
+      for (int i = 0; i < HD / 8; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll 1
+      for (int k0 = 0; k0 < kend; k0 += 32) {
+        const bool edge = k0 + 32 > T || (causal && k0 + 32 > r0);
+        float s[4][4], dp[4][4]; at_rows_product<HD, 4>(s, Qs, Ks + k0 * C::LDH, r0, lane); at_rows_product<HD, 4>(dp, Gs, Vs + k0 * C::LDH, r0, lane);
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+          const float2 kk = *reinterpret_cast<const float2*>(ik + k0 + n * 8 + 2 * t), vv = *reinterpret_cast<const float2*>(iv + k0 + n * 8 + 2 * t);
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const float fk = e & 1 ? kk.y : kk.x, fv = e & 1 ? vv.y : vv.x;
+            const int j = k0 + n * 8 + 2 * t + (e & 1), i = e < 2 ? i0 : i1;
+            const float p = edge && (j >= T || (causal && j > i)) ? 0.f : __expf(s[n][e] * ((e < 2 ? f0 : f1) * fk) - (e < 2 ? m0 : m1)) * (e < 2 ? il0 : il1);      // (rows beyond T: il = 0)
+            s[n][e] = p * (dp[n][e] * ((e < 2 ? g0 : g1) * fv) - (e < 2 ? d0 : d1)) * inv_scale;        // dS
+          }
+        }
+        at_sum_rows<HD, 4>(acc, 1.f, 1.f, s, Ks + k0 * C::LDH, ik + k0, lane);
+      }
+      at_store<HD>(dQ, acc, 1.f, 1.f, base, i0, i1, T, D, t);
+    }
+    {   // dK and dV of 16 key rows
+      const int j0 = r0 + g, j1 = j0 + 8;
+      const float f0 = ik[j0] * inv_scale, f1 = ik[j1] * inv_scale, v0 = iv[j0], v1 = iv[j1];
+      float ak[HD / 8][4], av[HD / 8][4];
+#pragma unroll
+      for (int i = 0; i < HD / 8; i++) { ak[i][0] = ak[i][1] = ak[i][2] = ak[i][3] = 0.f; av[i][0] = av[i][1] = av[i][2] = av[i][3] = 0.f; }
+#pragma unroll 1
+      for (int q0 = causal ? r0 & ~31 : 0; q0 < Tp; q0 += 32) {
+        const bool edge = r0 + 16 > T || (causal && q0 < r0 + 16);
+        float s[4][4], dp[4][4]; at_rows_product<HD, 4>(s, Ks, Qs + q0 * C::LDH, r0, lane); at_rows_product<HD, 4>(dp, Vs, Gs + q0 * C::LDH, r0, lane);
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+          const int c0 = q0 + n * 8 + 2 * t;
+          const float2 qq = *reinterpret_cast<const float2*>(iq + c0), gg = *reinterpret_cast<const float2*>(ig + c0), mm = *reinterpret_cast<const float2*>(st_m + c0),
+                       ll = *reinterpret_cast<const float2*>(st_il + c0), dd = *reinterpret_cast<const float2*>(st_d + c0);
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const int i = c0 + (e & 1), j = e < 2 ? j0 : j1;
+            const float p = edge && (j >= T || (causal && j > i)) ? 0.f : __expf(s[n][e] * ((e < 2 ? f0 : f1) * (e & 1 ? qq.y : qq.x)) - (e & 1 ? mm.y : mm.x)) * (e & 1 ? ll.y : ll.x);      // (columns beyond T: il = 0)
+            dp[n][e] = p * (dp[n][e] * ((e < 2 ? v0 : v1) * (e & 1 ? gg.y : gg.x)) - (e & 1 ? dd.y : dd.x)) * inv_scale;      // dS^T
+            s[n][e] = p;                                                                                                     // P^T
+          }
+        }
+        at_sum_rows<HD, 4>(av, 1.f, 1.f, s, Gs + q0 * C::LDH, ig + q0, lane); at_sum_rows<HD, 4>(ak, 1.f, 1.f, dp, Qs + q0 * C::LDH, iq + q0, lane);
+      }
+      at_store<HD>(dK, ak, 1.f, 1.f, base, j0, j1, T, D, t); at_store<HD>(dV, av, 1.f, 1.f, base, j0, j1, T, D, t);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- a few query rows
 // Attention of TE = 1 or 2 query rows per sequence (token 0, and the last token) against all T keys, any head size: what the
 // top block below a CLSPooling needs (plan_token_rows in model.cu).  Q and O are [B * TE, D], K and V [B * T, D].  One block per
@@ -435,8 +595,41 @@ inline int attn_rows_bwd(Ctx* ctx, const float* Q, long ldq, const float* K, con
 // ---------------------------------------------------------------- launchers
 inline bool attn_fused_supported(int hd, int D) { return (hd == 16 || hd == 32 || hd == 64) && D % 4 == 0; }
 
+// Warps of a block per head: one per 16 rows up to 16, then as few as take the same number of turns
+inline int at_head_warps(int T) { const int n = cdiv(T, 16); return n <= 16 ? n : cdiv(n, cdiv(n, 16)); }
+// Blocks of 64 rows or a block per head?  By estimated time (us, from measured rates).  A block per head takes `h0` and `h1` per 32 keys and turn; two that share an
+// SM take 1.4 times as long as one.  A round of the others, as many as are resident, takes `t0` and `t1` per 64 keys (rows of padding count half), the last
+// round's end a quarter of one, and a block by itself 0.62 of one.  Measured, 64 rows against a head, heads x tokens (size 32, no mask) forward / backward: 288 x 150 24 - 16 /
+// 69 - 45, 512 x 150 40 - 31 / 119 - 89, 512 x 128 19 - 23 / 65 - 64, 288 x 256 39 - 34 / 129 - 101, 160 x 150 16 - 16 / 43 - 45, 64 x 150 11 - 12 / 20 - 32;
+// size 64: 288 x 150 39 - 40 / 140 - 103, 288 x 200 71 - 57 / -; with a causal mask 288 x 150, 32: 19 - 13 / 54 - 31.
+template <int HD> inline bool at_head_better(const Ctx* ctx, long heads, int T, int causal, bool bwd) {
+  const size_t smem = at_head_smem<HD>(T, bwd); if (smem > 227 * 1024) return false;
+  constexpr bool wide = HD == 64;
+  const double h0 = bwd ? (wide ? 1 : 3) : (wide ? 4 : 2.5), h1 = bwd ? (wide ? 9.6 : 6.2) : (wide ? 3.6 : 1.9), t0 = bwd ? (wide ? 7 : 5) : (wide ? 5 : 4), t1 = bwd ? (wide ? 11 : 6.7) : (wide ? 6.3 : 4);
+  const int warps = at_head_warps(T), kc = at_pad(T) / 32, turns = cdiv(cdiv(T, 16), warps), nb = cdiv(T, AT_BLK);
+  const bool pairs = warps <= 10 && 2 * (smem + 1024) <= 228 * 1024 && !(wide && bwd); const long n = cdiv(heads, ctx->sm_count);
+  const double u = h0 + h1 * kc * turns * (causal ? 0.5 * (kc + 1) / kc : 1.0), head = u * (pairs ? n / 2 * 1.4 + n % 2 : n);
+  const double w = t0 + t1 * 0.5 * (nb + T / 64.0) * (causal ? 0.5 * (nb + 1) / nb : 1.0), rounds = (double)heads * nb * (bwd ? 2 : 1) / ((wide ? 3.0 : 4.0) * ctx->sm_count);
+  return head < 0.92 * w * std::max(0.62, rounds + 0.25);
+}
+template <int HD>
+inline int attn_head_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
+  const int smem = (int)at_head_smem<HD>(T, false), warps = at_head_warps(T); auto* kern = warps <= 10 ? attn_head_fwd_kernel<HD, 320, 2> : attn_head_fwd_kernel<HD, 512, 1>;
+  GN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  GN_LAUNCH(ctx, kern, dim3(H, B), 32 * warps, smem, Q, K, V, O, M, L, T, D, H, causal, 1.f / sqrtf((float)HD));
+  return check_launch("attn_head_fwd");
+}
+template <int HD>
+inline int attn_head_bwd(Ctx* ctx, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
+                         float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
+  const int smem = (int)at_head_smem<HD>(T, true), warps = at_head_warps(T); auto* kern = warps <= 10 ? attn_head_bwd_kernel<HD, 320, HD == 64 ? 1 : 2> : attn_head_bwd_kernel<HD, 512, 1>;
+  GN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  GN_LAUNCH(ctx, kern, dim3(H, B), 32 * warps, smem, Q, K, V, O, dO, M, L, dQ, dK, dV, T, D, H, causal, 1.f / sqrtf((float)HD));
+  return check_launch("attn_head_bwd");
+}
 template <int HD>
 inline int attn_fwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
+  if (at_head_better<HD>(ctx, (long)B * H, T, causal, false)) return attn_head_fwd<HD>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
   const int smem = 3 * AtCfg<HD>::TILE * (int)sizeof(__half) + 3 * AT_BLK * (int)sizeof(float);
   GN_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, attn_fwd_kernel<HD>, dim3(cdiv(T, AT_BLK), H, B), AT_THREADS, smem, Q, K, V, O, M, L, T, D, H, causal, 1.f / sqrtf((float)HD));
@@ -445,6 +638,7 @@ inline int attn_fwd_launch(Ctx* ctx, const float* Q, const float* K, const float
 template <int HD>
 inline int attn_bwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
                            float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
+  if (at_head_better<HD>(ctx, (long)B * H, T, causal, true)) return attn_head_bwd<HD>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
   const int smem = 4 * AtCfg<HD>::TILE * (int)sizeof(__half) + 7 * AT_BLK * (int)sizeof(float);
   GN_CUDA(cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, attn_bwd_kernel<HD>, dim3(2 * cdiv(T, AT_BLK), H, B), AT_THREADS, smem, Q, K, V, O, dO, M, L, dQ, dK, dV, T, D, H, causal, 1.f / sqrtf((float)HD));

@@ -51,6 +51,8 @@ def run(device, engine, Q, K, V, dO, B, T, D, H, causal):
 
 CASES = [  # engine, B, T, D, H, causal
     (0, 2, 80, 128, 2, 1), (0, 3, 150, 96, 3, 1), (0, 2, 64, 64, 4, 0),
+    # enough heads for a block each: padded tails, widths of 16, 32 and 64, more than 16 groups of rows (two turns per warp), more than 10
+    (0, 96, 150, 96, 3, 0), (0, 96, 130, 96, 3, 1), (0, 72, 200, 128, 4, 1), (0, 72, 150, 256, 4, 0), (0, 96, 272, 48, 3, 1),
     (1, 1, 128, 64, 1, 1), (1, 2, 128, 128, 2, 1), (1, 3, 256, 128, 2, 1), (1, 2, 512, 192, 3, 1), (1, 2, 256, 128, 2, 0),
 ]
 
@@ -68,6 +70,18 @@ def test_attention_matches_fp64(device, engine, B, T, D, H, causal):
     for name, a, b in zip(("O", "dQ", "dK", "dV"), (got[0], got[3], got[4], got[5]), (ref[0], ref[3], ref[4], ref[5])):
         e = norm_err(a, b)
         assert e < TOL, f"{name}: normalised error {e:.3e}"
+
+
+@pytest.mark.parametrize("B,T,D,H,causal", [(96, 150, 96, 3, 0), (72, 161, 128, 4, 1), (72, 150, 256, 4, 0), (96, 272, 48, 3, 1)])
+def test_sequences_do_not_depend_on_the_batch(device, B, T, D, H, causal):
+    """A block per head (many heads) and blocks of 64 rows (few): the same bits."""
+    rng = np.random.default_rng(T)
+    Q, K, V, dO = (rng.standard_normal((B * T, D)).astype(np.float32) for _ in range(4))
+    many = run(device, 0, Q, K, V, dO, B, T, D, H, causal)
+    few = run(device, 0, *(x[: 2 * T].copy() for x in (Q, K, V, dO)), 2, T, D, H, causal)
+    for a, b in zip(many, few):
+        n = b.shape[0]
+        assert np.array_equal(a[:n], b)
 
 
 def test_attention_bounded_waits_fail_fast_and_the_context_stays_usable(device):
