@@ -249,13 +249,12 @@ inline bool gemm_skinny_ok(const GemmDesc& g) {
 // size.  blockIdx.z: several products of one shape, their C (and a_sum) c_b apart (the Q, K and V projections' gradients).
 constexpr int OS_KMAX = 64;
 template <int TM>
-__global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict__ A, long sa_k, long a_b, const float* __restrict__ B, long sb_k, long b_b, float* __restrict__ C, long ldc, long c_b,
-                                                        int M, int N, int K, float alpha, float* __restrict__ a_sum, int va, int vb) {
+__device__ __forceinline__ void outer_tile(const float* __restrict__ A, long sa_k, const float* __restrict__ B, long sb_k, float* __restrict__ C, long ldc, int M, int N, int K, float alpha,
+                                           float* __restrict__ a_sum, int va, int vb, int m0, int n0) {
   constexpr int BM = 16 * TM;
   __shared__ __align__(16) float As[OS_KMAX][BM];
   __shared__ __align__(16) float Bs[OS_KMAX][64];
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  A += blockIdx.z * a_b; B += blockIdx.z * b_b; C += blockIdx.z * c_b;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   if (va && m0 + BM <= M) for (int i = tid; i < K * (BM / 4); i += 256) { const int k = i / (BM / 4), c = i % (BM / 4) * 4; cp_async16(&As[k][c], A + (long)k * sa_k + m0 + c); }
   else
 #pragma unroll 4
@@ -266,7 +265,7 @@ __global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict_
     for (int i = tid; i < K * 64; i += 256) { const int k = i >> 6, c = i & 63; Bs[k][c] = n0 + c < N ? B[(long)k * sb_k + n0 + c] : 0.f; }
   cp_async_wait();
   __syncthreads();
-  if (a_sum && blockIdx.x == 0 && tid < BM && m0 + tid < M) { float v = 0.f; for (int k = 0; k < K; k++) v += As[k][tid]; a_sum[blockIdx.z * c_b + m0 + tid] = v; }
+  if (a_sum && n0 == 0 && tid < BM && m0 + tid < M) { float v = 0.f; for (int k = 0; k < K; k++) v += As[k][tid]; a_sum[m0 + tid] = v; }
   float acc[TM][4] = {};
 #pragma unroll 4
   for (int k = 0; k < K; k++) {
@@ -289,6 +288,24 @@ __global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict_
     else
       for (int j = 0; j < 4; j++) if (n0 + tx * 4 + j < N) crow[j] = alpha * acc[i][j];
   }
+}
+template <int TM>
+__global__ void __launch_bounds__(256) outer_sum_kernel(const float* __restrict__ A, long sa_k, long a_b, const float* __restrict__ B, long sb_k, long b_b, float* __restrict__ C, long ldc, long c_b,
+                                                        int M, int N, int K, float alpha, float* __restrict__ a_sum, int va, int vb) {
+  outer_tile<TM>(A + blockIdx.z * a_b, sa_k, B + blockIdx.z * b_b, sb_k, C + blockIdx.z * c_b, ldc, M, N, K, alpha, a_sum ? a_sum + blockIdx.z * c_b : nullptr, va, vb, blockIdx.y * 16 * TM, blockIdx.x * 64);
+}
+// Several such sums over the same number of rows in one launch, a tile per block: a launch of a few dozen tiles takes as long as one of 160, and
+// a block's four gradients one after the other took as long as the rest of its backward pass beside them.
+struct OuterGroup {
+  struct P { const float *A, *B; float *C, *a_sum; long sa_k, sb_k, ldc; int M, N, va, vb, tile0; } p[4];
+  int n = 0, K = 0;
+};
+template <int TM>
+__global__ void __launch_bounds__(256) outer_group_kernel(const OuterGroup g) {
+  int j = 0;
+  while (j + 1 < g.n && (int)blockIdx.x >= g.p[j + 1].tile0) j++;
+  const OuterGroup::P& q = g.p[j]; const int t = blockIdx.x - q.tile0, tn = (q.N + 63) / 64;
+  outer_tile<TM>(q.A, q.sa_k, q.B, q.sb_k, q.C, q.ldc, q.M, q.N, g.K, 1.f, q.a_sum, q.va, q.vb, t / tn * 16 * TM, t % tn * 64);
 }
 inline bool gemm_outer_small_ok(const GemmDesc& g) {
   return g.sa_m == 1 && g.sb_n == 1 && g.K >= 1 && g.K <= OS_KMAX && g.batch2 == 1 && g.batch1 <= 65535 && !g.bias && !g.R && !g.mask && g.act == GN_ACT_LINEAR && g.flags == 0 &&
@@ -516,6 +533,19 @@ inline int gemm_small(Ctx* ctx, const GemmDesc& g) {
   while (splits < all && more(tiles, splits)) splits *= 2;
   const int per = cdiv(cdiv(g.K, all), SP_KB) * SP_KB, chunks = all / splits;
   return tm == 2 ? gemm_small_tile<2>(ctx, g, splits, chunks, per) : tm == 4 ? gemm_small_tile<4>(ctx, g, splits, chunks, per) : gemm_small_tile<8>(ctx, g, splits, chunks, per);
+}
+
+// One launch for the products `d` (each gemm_outer_small_ok with the same K, alpha 1 and no batch)
+inline int gemm_outer_group(Ctx* ctx, const GemmDesc* d, int n) {
+  OuterGroup g; g.n = n; g.K = d[0].K;
+  auto vec = [](const float* p, long ld) { return (int)((reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0); };
+  auto lay = [&](int bm) { int tiles = 0; for (int j = 0; j < n; j++) { g.p[j].tile0 = tiles; tiles += (int)(cdiv(d[j].M, bm) * cdiv(d[j].N, 64)); } return tiles; };
+  for (int j = 0; j < n; j++) g.p[j] = OuterGroup::P{d[j].A, d[j].B, d[j].C, d[j].a_sum, d[j].sa_k, d[j].sb_k, d[j].ldc, d[j].M, d[j].N, vec(d[j].A, d[j].sa_k), vec(d[j].B, d[j].sb_k), 0};
+  // 128-row tiles once they give every SM two blocks
+  int tiles = lay(128);
+  if (tiles >= 2 * ctx->sm_count) GN_LAUNCH(ctx, outer_group_kernel<8>, tiles, 256, 0, g);
+  else { tiles = lay(64); GN_LAUNCH(ctx, outer_group_kernel<4>, tiles, 256, 0, g); }
+  return check_launch("outer_group");
 }
 
 template <int BM, int BN, int BK, int TM, int TN>

@@ -930,6 +930,23 @@ static int side_weight_bias_grads(gn_model* m, int stack, int B, int out, int in
   Ctx* ctx = &m->ctx->c; auto issue = [&]() -> int { return weight_bias_grads_stack(m, stack, B, out, in, dz, x, ldx, gW, gb, ws); };
   return grads_on_side(ctx, stack, B, out, in, ldx) ? side_run(ctx, issue) : issue();
 }
+// The parameter gradients of up to four layers from dense rows of dz, in one launch beside the main stream where they are sums of few outer products;
+// others go one by one when they are added.
+struct GradGroup {
+  gn_model* m; GemmDesc d[4]; int n = 0;
+  int add(int B, int out, int in, const float* dz, const float* x, long ldx, float* gW, float* gb) {
+    GemmDesc g; g.M = out; g.N = in; g.K = B; g.A = dz; g.sa_m = 1; g.sa_k = out; g.B = x; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = in; g.a_sum = gb;
+    if (m->ctx->c.profile || !gemm_outer_small_ok(g) || n == 4) return side_weight_bias_grads(m, 1, B, out, in, dz, x, ldx, gW, gb);
+    d[n++] = g; return GN_OK;
+  }
+  int flush() {
+    if (!n) return GN_OK;
+    Ctx* ctx = &m->ctx->c; double macs = 0; for (int j = 0; j < n; j++) macs += (double)d[j].M * d[j].N * d[j].K;
+    ctx->gemm_flops += 2.0 * macs; ctx->gemm_launches++;
+    auto issue = [&]() -> int { return gemm_outer_group(ctx, d, n); };
+    const int rc = macs >= 3.0e6 ? side_run(ctx, issue) : issue(); n = 0; return rc;
+  }
+};
 // Can the FFN's hidden activation (and its gradient) of this block live as operand planes only?  The two contractions on
 // either side must both run on the tensor-core engine with prepared weight planes, and the plane-writing epilogue's shape
 // rules must hold.
@@ -1074,14 +1091,16 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
   const float* mid_last = l.mid_is_planes ? l.mid_last.p : last(l.mid, kr.mid, F); const long ld_mid = l.mid_is_planes ? F : ldF;
   float *dR2, *dR1, *comb, *dA, *dM;
   GN_TRY(ensure(m, S_ND0, BD, &dR2)); GN_TRY(ensure(m, S_ND1, BD, &comb)); GN_TRY(ensure(m, S_ND2, BD, &dR1)); GN_TRY(ensure(m, S_ND3, 2 * BD, &dA)); GN_TRY(ensure(m, S_NFF, BF, &dM));
-  auto norm = [&](const float* g, const float* x, const float* gamma, const float* stat, float* out, float* gG, float* gB) -> int {
-    if (norm_vec_ok(D, {g, x, gamma, out})) return norm_backward_vec(m, l.rms, g, x, ldD, gamma, stat, l.rms ? stat : stat + NE, TR, out, gG, gB, B, D, RowPlaneOut{});
+  const bool side = grads_on_side(ctx, 1, B, F, D, D);      // (the block forks its stream anyway)
+  auto norm = [&](const float* g, const float* x, const float* gamma, const float* stat, float* out, float* gG, float* gB, int slot) -> int {
+    if (norm_vec_ok(D, {g, x, gamma, out})) return norm_backward_vec(m, l.rms, g, x, ldD, gamma, stat, l.rms ? stat : stat + NE, TR, out, gG, gB, B, D, RowPlaneOut{}, side ? slot : 0);
     GN_LAUNCH(ctx, norm_bwd_rows_kernel, cdiv(B, 4), 128, 0, g, x, ldD, gamma, stat, l.rms ? nullptr : stat + NE, (long)TR, out, B, D);
     GN_LAUNCH(ctx, norm_pgrad_rows_kernel, cdiv(D, 32), 256, 0, g, x, ldD, stat, l.rms ? nullptr : stat + NE, (long)TR, B, D, gG, gB);
     return check_launch("norm_rows");
   };
-  GN_TRY(norm(gout, r2_0, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2));
-  GN_TRY(side_weight_bias_grads(m, 1, B, D, F, dR2, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
+  GN_TRY(norm(gout, r2_0, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2, S_PART2));
+  GradGroup grads{m};
+  GN_TRY(grads.add(B, D, F, dR2, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
   GemmDesc g; g.M = B; g.N = F; g.K = D; g.A = dR2; g.sa_m = D; g.sa_k = 1; g.B = bp.w2; g.sb_k = F; g.sb_n = 1; g.C = dM; g.ldc = F;
   if (l.ff_act == GN_ACT_RELU) { g.mask = mid_last; g.mask_ld = ld_mid; }
   GN_TRY(gemm(ctx, g));
@@ -1094,19 +1113,21 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
     GN_TRY(gemm_nn(ctx, B, F, D, dU, F, bp.v1, comb, D, comb, D));
   } else {
     if (l.ff_act == GN_ACT_GELU) GN_LAUNCH(ctx, scale_by_last_deriv_kernel, ew_grid(ctx, BF), 256, 0, dM, (const float*)l.zlast.p, 1, F, BF, (int)GN_ACT_GELU);
-    GN_TRY(side_weight_bias_grads(m, 1, B, F, D, dM, n1_last, ldD, (float*)gp.w1, (float*)gp.b1));
+    GN_TRY(grads.add(B, F, D, dM, n1_last, ldD, (float*)gp.w1, (float*)gp.b1));
     GN_TRY(gemm_nn(ctx, B, F, D, dM, F, bp.w1, comb, D, dR2, D));
   }
-  GN_TRY(norm(comb, r1_0, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1));
-  GN_TRY(side_weight_bias_grads(m, 1, B, D, D, dR1, att_last, ldD, (float*)gp.wo, (float*)gp.bo));
+  GN_TRY(norm(comb, r1_0, bp.g1, st, dR1, (float*)gp.g1, (float*)gp.be1, S_PART3));
+  GN_TRY(grads.add(B, D, D, dR1, att_last, ldD, (float*)gp.wo, (float*)gp.bo));
   GN_TRY(gemm_nn(ctx, B, D, D, dR1, D, bp.wo, dA, D));
   if (d.causal) {
     // the one probability of token 0 is 1: dV = dA at token 0, dQ = dK = 0
     GN_TRY(side_run(ctx, [&]() -> int { GN_CUDA(stream_zero(ctx, (void*)gp.wq, (size_t)(gp.wv - gp.wq) * sizeof(float))); return GN_OK; }));
-    GN_TRY(side_weight_bias_grads(m, 1, B, D, D, dA, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
+    GN_TRY(grads.add(B, D, D, dA, x_last, ldX, (float*)gp.wv, (float*)gp.bv));
+    GN_TRY(grads.flush());
     GN_TRY(gemm_nn(ctx, B, D, D, dA, D, bp.wv, dx, D, dR1, D));
     *dx_row0 = true; return check_launch("block_backward_row0");
   }
+  GN_TRY(grads.flush());
   float *dQ, *dK, *dV, *ks, *vs;
   GN_TRY(ensure(m, S_XROWS, 3 * BD, &dQ)); ks = dQ + BD; vs = ks + BD; GN_TRY(ensure(m, S_ND4, 2 * ND, &dK)); dV = dK + ND;
   GN_TRY(attn_rows_bwd(ctx, l.q.p, (long)TE * D, l.k.p, l.v.p, dA, dQ, dK, dV, ks, vs, B, T, D, d.heads));
