@@ -62,7 +62,9 @@ constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by
 // [8192, 1024] x [1024, 256] from 26.8 to 18.6, [32768, 1024] x [1024, 1024] from 136 to 119 (zeros as data: no power limit).
 constexpr int TC_BK = 32, PL_LO = 32;
 __host__ __device__ __forceinline__ int pl_off(int k) { return ((k >> 5) << 6) | (k & 31); }
-// PL: the variant that writes its result as operand planes.
+// What a variant of the kernel writes: fp32 in 16-byte pieces, operand planes, or fp32 where 16-byte pieces do not fit (an odd number of columns, NCHW).  (The
+// last one's code beside the first one's cost every product 2 %.)  PL: planes.
+enum TcOut { TC_OUT_VEC, TC_OUT_PLANES, TC_OUT_ANY };
 template <int BN, bool PL> struct TcCfg {
   static constexpr int EW = PL ? 16 : 8, CG = EW / 4, CC = PL ? 16 : 32;          // epilogue warps, column groups, columns of a chunk
   static constexpr int THREADS = 64 + 32 * EW;                                    // TMA warp, MMA warp, epilogue warps
@@ -237,10 +239,10 @@ __device__ __forceinline__ void tc_acc_chunk(uint32_t taddr, uint32_t acc_main, 
 }
 // `acc_main` / `acc_cross` are the TMEM column offsets of the two accumulators of this tile (MERGED: there is only acc_main); `bw` is the
 // tile's width (BN, or BN / 2 for a half tile).  `wait` blocks until the accumulator is complete; false: it gave up.
-template <int BN, bool PL, bool MERGED, class W>
+template <int BN, TcOut OUT, bool MERGED, class W>
 __device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tmem_base, uint32_t acc_main, uint32_t acc_cross,
                                                  int m0, int n0, int z, int quad, int cg, int lane, int nkb, int bw, float* stg, W&& wait) {
-  using Cfg = TcCfg<BN, PL>;
+  constexpr bool PL = OUT == TC_OUT_PLANES; using Cfg = TcCfg<BN, PL>;
   const int z1 = z / ep.batch2, z2 = z - z1 * ep.batch2, nch = max(bw / (Cfg::CC * Cfg::CG), 1);      // chunks per warp
   if (cg * nch * Cfg::CC >= bw) return wait();                               // a narrow tile has fewer chunks than column groups
   const int rbase = m0 + quad * 32, row = rbase + lane, c_end = min(cg * nch + nch, (ep.N - n0 + Cfg::CC - 1) / Cfg::CC);
@@ -343,7 +345,7 @@ __device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tm
   }
   float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
   const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
-  if (ep.flags & TC_FLAG_VEC) {
+  if constexpr (OUT == TC_OUT_VEC) {
     const int rl = lane >> 3, c8 = lane & 7, r0 = rbase + rl;                // after the exchange: this lane's rows r0 + 4 t and columns 4 c8 .. 4 c8 + 3 of a chunk
     float4 sv, bv, rv[8];                                                    // what the next chunk needs for them
     auto fetch = [&](int c) {
@@ -400,28 +402,55 @@ __device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tm
     __syncwarp();
     return true;
   }
+  if (ep.nchw_P == 0) {
+    // rows that 16-byte accesses do not fit (an odd number of columns): through the staging buffer all the same, then a row at a time, a column per lane.
+    // (A row per lane, a column at a time, touched 32 lines per instruction: [2048, 1001] over 256 29 -> 16 us.)
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = cg * nch; c < c_end; c++) {
+      const int col = n0 + c * 32 + lane; const bool col_ok = col < ep.N; const int seg = ep.n_seg ? (n0 + c * 32) / ep.n_seg : 0;      // (32 columns lie in one segment)
+      const float sv = col_ok ? __ldg(isb + col) : 0.f, bv = col_ok && ep.bias ? __ldg(ep.bias + col + (long)seg * (ep.bias_seg - ep.n_seg)) : 0.f;
+      {
+        float v[32]; tc_acc_chunk<MERGED, 32>(tquad + c * 32, acc_main, acc_cross, nkb > 0, isa, v);
+        __syncwarp();                                                        // the previous chunk has been read back
+#pragma unroll
+        for (int j = 0; j < 8; j++) *reinterpret_cast<float4*>(stg + lane * 32 + ((j ^ (lane & 7)) << 2)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+      }
+      const long off = (long)seg * (ep.c_seg - ep.n_seg) + col; float* o = C + off; const float* q = R ? R + off : nullptr;      // (with segments R is C)
+#pragma unroll 1
+      for (int r4 = 0; r4 < 32; r4 += 4) {
+        float a[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const int r = r4 + t; const bool ok = col_ok && rbase + r < ep.M;
+          a[t] = stg[r * 32 + ((((lane >> 2) ^ (r & 7)) << 2) | (lane & 3))] * sv + bv + (q && ok ? q[(long)(rbase + r) * ep.ldr] : 0.f);
+          if (ep.act == GN_ACT_RELU) a[t] = fmaxf(a[t], 0.f);
+          if (ep.mask && ok && !(ep.mask[(long)((rbase + r) / ep.mask_group) * ep.mask_ld + col] > 0.f)) a[t] = 0.f;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) if (col_ok && rbase + r4 + t < ep.M) o[(long)(rbase + r4 + t) * ep.ldc] = a[t];
+      }
+    }
+    __syncwarp();
+    return true;
+  }
   if (!wait()) return false;
-  // scalar path (unaligned operands, NCHW store): one output row per thread
-  const float* Rrow = (R && row_ok) ? R + (long)row * ep.ldr : nullptr;
-  const float* Mrow = (ep.mask && row_ok) ? ep.mask + (long)(row / ep.mask_group) * ep.mask_ld : nullptr;
-  float* Crow = ep.nchw_P > 0 ? C + (long)(row / ep.nchw_P) * ep.N * ep.nchw_P + row % ep.nchw_P : C + (long)row * ep.ldc;
-  const long cstep = ep.nchw_P > 0 ? ep.nchw_P : 1;
+  // NCHW store: one output row per thread
+  float* Crow = C + (long)(row / ep.nchw_P) * ep.N * ep.nchw_P + row % ep.nchw_P;
 #pragma unroll 1
   for (int cc = 0; cc < nch; cc++) {
     const int col0 = n0 + (cg * nch + cc) * 32;
     if (col0 >= ep.N) break;
-    const int seg = ep.n_seg ? col0 / ep.n_seg : 0; const long c_off = ep.n_seg ? seg * (ep.c_seg - ep.n_seg) : 0, b_off = ep.n_seg ? seg * (ep.bias_seg - ep.n_seg) : 0;
     float v[32]; tc_acc_chunk<MERGED, 32>(tquad + (cg * nch + cc) * 32, acc_main, acc_cross, nkb > 0, isa, v);
 #pragma unroll
     for (int j = 0; j < 32; j++) {
       const int col = col0 + j;
       if (!row_ok || col >= ep.N) continue;
       float x = v[j] * isb[col];
-      if (ep.bias) x += ep.bias[b_off + col];
-      if (Rrow) x += Rrow[c_off + col];
+      if (ep.bias) x += ep.bias[col];
       if (ep.act == GN_ACT_RELU) x = fmaxf(x, 0.f);
-      if (Mrow && !(Mrow[col] > 0.f)) x = 0.f;
-      Crow[c_off + col * cstep] = x;
+      Crow[(long)col * ep.nchw_P] = x;
     }
   }
   return true;
@@ -429,10 +458,10 @@ __device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tm
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
-template <int BN, bool PL>
-__global__ void __launch_bounds__(TcCfg<BN, PL>::THREADS, 1)
+template <int BN, TcOut OUT>
+__global__ void __launch_bounds__(TcCfg<BN, OUT == TC_OUT_PLANES>::THREADS, 1)
 gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ TcParams ep, int tiles_m, int tiles_n, int total_tiles, int full_end, int n_half, int* tile_queue) {
-  using Cfg = TcCfg<BN, PL>;
+  using Cfg = TcCfg<BN, OUT == TC_OUT_PLANES>;
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES, BK = TC_BK;
   constexpr bool MERGED = Cfg::MERGED;
   constexpr uint32_t TMEM_COLS = Cfg::TMEM_COLS, SLOT_COLS = Cfg::SLOT_COLS;
@@ -595,7 +624,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
       int m0, n0, z, kb0, nkb; if (!decode(tile, half, m0, n0, z, kb0, nkb)) continue;
       const uint32_t slot = lt & 1, u = lt >> 1; lt++;
       const int bw = half < 0 ? BN : BN / 2;
-      const bool ok = tc_epilogue_tile<BN, PL, MERGED>(ep, tmem_base, slot * SLOT_COLS, slot * SLOT_COLS + BN, m0, n0, z, quad, cg, lane, nkb, bw, stg, [&]() -> bool {
+      const bool ok = tc_epilogue_tile<BN, OUT, MERGED>(ep, tmem_base, slot * SLOT_COLS, slot * SLOT_COLS + BN, m0, n0, z, quad, cg, lane, nkb, bw, stg, [&]() -> bool {
         int got = 1;
         if (lane == 0) got = mbar_wait(tfull0 + 8 * slot, u & 1, limit, abort_flag) ? 1 : 0;
         got = __shfl_sync(0xffffffffu, got, 0);
@@ -856,12 +885,13 @@ inline int tc_planes(Ctx* ctx, int which, long nbatch, long rows, int K, BfPlane
 }
 inline int* tc_rowmax_buf(Ctx* ctx) { return reinterpret_cast<int*>(tc_scratch(ctx).mx.p); }
 
-template <int BN, bool PL> inline bool tc_set_smem() { return cudaFuncSetAttribute(gemm_tc_persist_kernel<BN, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<BN, PL>::SMEM_BYTES) == cudaSuccess; }
+template <int BN, TcOut OUT> inline bool tc_set_smem1() { return cudaFuncSetAttribute(gemm_tc_persist_kernel<BN, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<BN, OUT == TC_OUT_PLANES>::SMEM_BYTES) == cudaSuccess; }
+template <int BN> inline bool tc_set_smem() { return tc_set_smem1<BN, TC_OUT_VEC>() && tc_set_smem1<BN, TC_OUT_PLANES>() && tc_set_smem1<BN, TC_OUT_ANY>(); }
 inline void tc_init(Ctx* ctx) {
   ctx->tc_ok = false;
   void* fn = nullptr; cudaDriverEntryPointQueryResult q;
   if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn || q != cudaDriverEntryPointSuccess) { cudaGetLastError(); return; }
-  if (!(tc_set_smem<64, false>() && tc_set_smem<128, false>() && tc_set_smem<256, false>() && tc_set_smem<64, true>() && tc_set_smem<128, true>() && tc_set_smem<256, true>())) { cudaGetLastError(); return; }
+  if (!(tc_set_smem<64>() && tc_set_smem<128>() && tc_set_smem<256>())) { cudaGetLastError(); return; }
   ctx->encode_tiled = fn; ctx->tc_ok = true;
   if (const char* e = getenv("GONEURON_CUDA_TC_BN")) ctx->tc_force_bn = atoi(e);
   if (const char* e = getenv("GONEURON_CUDA_TC_KSLICE")) ctx->tc_kslice = atoi(e);
@@ -950,8 +980,9 @@ inline int tc_launch_persist(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, con
   int* queue = nullptr;
   if (ctx->tc_tile_queue && total > grid) GN_TRY(tc_next_queue(ctx, &queue));
   ProfScope prof(ctx);
-  if (ep.out_p) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, true>), grid, (TcCfg<BN, true>::THREADS), (TcCfg<BN, true>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
-  else GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, false>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  if (ep.out_p) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_PLANES>), grid, (TcCfg<BN, true>::THREADS), (TcCfg<BN, true>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  else if (ep.flags & TC_FLAG_VEC) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_VEC>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  else GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_ANY>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
   return check_launch("gemm_tc_persist");
 }
 // Output tile width for a problem: 64 for narrow outputs; 256 (three quarters of the shared-memory traffic per MMA
@@ -1020,33 +1051,46 @@ inline int tc_run_rows(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, const TcP
 // partial result; a second kernel adds the partial results in slice order (fp32) and applies the epilogue.
 __global__ void __launch_bounds__(256) tc_sum_slices_kernel(const float* __restrict__ part, int splits, int M, int N, const TcParams ep) {
   const long mn = (long)M * N, n4 = mn >> 2; const bool vec = (N & 3) == 0;
-  for (long e = blockIdx.x * 256L + threadIdx.x; e < (vec ? n4 : mn); e += gridDim.x * 256L) {
-    const long i = vec ? 4 * e : e; const int r = (int)(i / N), c = (int)(i - (long)r * N), w = vec ? 4 : 1;
-    float x[4] = {};
-    if (vec) {
-      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-      for (int z = 0; z < splits; z++) { const float4 u = *reinterpret_cast<const float4*>(part + z * mn + i); t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
-      x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
-    } else
-#pragma unroll 4
-      for (int z = 0; z < splits; z++) x[0] += part[z * mn + i];
-    for (int k = 0; k < w; k++) {
-      if (ep.bias) x[k] += ep.bias[c + k];
-      if (ep.R) x[k] += ep.R[(long)r * ep.ldr + c + k];
-      if (ep.act == GN_ACT_RELU) x[k] = fmaxf(x[k], 0.f);
-      if (ep.mask && !(ep.mask[(long)(r / ep.mask_group) * ep.mask_ld + c + k] > 0.f)) x[k] = 0.f;
+  auto finish = [&](float x, int r, int c) {
+    if (ep.bias) x += ep.bias[c];
+    if (ep.R) x += ep.R[(long)r * ep.ldr + c];
+    if (ep.act == GN_ACT_RELU) x = fmaxf(x, 0.f);
+    if (ep.mask && !(ep.mask[(long)(r / ep.mask_group) * ep.mask_ld + c] > 0.f)) x = 0.f;
+    return x;
+  };
+  if (!vec) {                                               // four elements of a thread in flight together, a block apart
+    for (long i0 = blockIdx.x * 1024L + threadIdx.x; i0 < mn; i0 += gridDim.x * 1024L) {
+      float x[4] = {};
+#pragma unroll 2
+      for (int z = 0; z < splits; z++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) if (i0 + 256 * k < mn) x[k] += part[z * mn + i0 + 256 * k];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const long i = i0 + 256 * k; if (i >= mn) break;
+        const int r = mn < (1L << 31) ? (int)i / N : (int)(i / N), c = (int)(i - (long)r * N);
+        ep.C[(long)r * ep.ldc + c] = finish(x[k], r, c);
+      }
     }
+    return;
+  }
+  for (long e = blockIdx.x * 256L + threadIdx.x; e < n4; e += gridDim.x * 256L) {
+    const long i = 4 * e; const int r = (int)(i / N), c = (int)(i - (long)r * N);
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int z = 0; z < splits; z++) { const float4 u = *reinterpret_cast<const float4*>(part + z * mn + i); t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+    const float x[4] = {finish(t.x, r, c), finish(t.y, r, c + 1), finish(t.z, r, c + 2), finish(t.w, r, c + 3)};
     float* o = ep.C + (long)r * ep.ldc + c;
-    if (vec && ((ep.ldc & 3) | (long)(reinterpret_cast<uintptr_t>(ep.C) & 15)) == 0) *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
-    else for (int k = 0; k < w; k++) o[k] = x[k];
+    if (((ep.ldc & 3) | (long)(reinterpret_cast<uintptr_t>(ep.C) & 15)) == 0) *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
+    else for (int k = 0; k < 4; k++) o[k] = x[k];
   }
 }
 // Slices and tile width by estimated time, from measured rates (us): 0.335 / 0.43 per 32 contraction indices of a 128 / 256 wide
 // tile, 3 / 5 for the last tile's epilogue (2.4 / 3.9 since it stores whole lines; not tuned again), 3 for the second launch and 4 TB/s for its partial results.  Slices keep at least 256
 // indices, and have to win by a tenth.
 inline int tc_split_count(Ctx* ctx, const TcParams& ep, long nbatch, int* bn) {
-  if (nbatch != 1 || ep.out_p || ep.n_seg || ep.nchw_P || ep.flags || ep.K < 1024 || ctx->tc_kslice > 0 || ctx->tc_force_bn) return 1;
+  if (nbatch != 1 || ep.out_p || ep.n_seg || ep.nchw_P || ep.flags || ep.K < 512 || ctx->tc_kslice > 0 || ctx->tc_force_bn) return 1;
   const long sms = persist_sms(ctx), tm = cdiv(ep.M, TC_BM); const double kb = cdiv(ep.K, TC_BK);
   auto cost = [&](int w, int sl) {
     const long tiles = tm * cdiv(ep.N, w); double rounds = std::ceil((double)tiles * sl / sms);

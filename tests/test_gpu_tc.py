@@ -30,7 +30,9 @@ def _gemm(device, engine, A, B, bias):
                                    (2048, 1024, 1024), (4096, 256, 4096),
                                    (256, 384, 70000),           # a weight-gradient shape: contraction over all tokens, cut into slices
                                    # more tiles than SMs with a short last round: its tiles run as half tiles (256- and 128-wide tilings)
-                                   (25600, 256, 96), (12800, 500, 64), (25600, 128, 96), (5760, 1024, 128)])
+                                   (25600, 256, 96), (12800, 500, 64), (25600, 128, 96), (5760, 1024, 128),
+                                   # rows that 16-byte accesses do not fit: 64-, 128- and 256-wide tiles, half tiles, slices
+                                   (300, 33, 96), (200, 129, 64), (12800, 501, 64), (5760, 1023, 128), (1100, 333, 1000), (70, 1001, 515)])
 def test_tc_gemm_matches_fp64(device, M, N, K):
     rng = np.random.default_rng(M * 7 + N * 3 + K)
     A = rng.standard_normal((M, K)).astype(np.float32)

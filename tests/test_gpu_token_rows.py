@@ -37,6 +37,8 @@ CASES = [
     (24, 64, 2, 96, [False, False], True, dict(ff_act=D.SILU, rms_norm=True, rope=True)),
     (24, 64, 2, 96, [True, True], True, dict(ff_act=D.GELU, rope=True)), (24, 64, 2, 96, [False], True, dict(ff_act=D.GELU)),
     (128, 128, 2, 256, [True, True], False, {}), (128, 128, 2, 256, [False], False, {}), (40, 64, 2, 96, [True, True], False, dict(rope=True)),
+    (250, 250, 2, 502, [False], False, {}),                                                          # residuals and gates of rows that 16-byte accesses do not fit
+    (24, 66, 2, 70, [True, True], True, {}), (24, 128, 2, 130, [True, True, True], True, {}),         # a block's weight gradients in one launch, odd tiles
 ]
 
 
