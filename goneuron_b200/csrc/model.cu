@@ -1186,7 +1186,7 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
         }
         float* all; GN_TRY(ensure(m, S_W, (size_t)n_updates * (R4g + zs), &all));
         float* Da = all; float* Za = all + (size_t)n_updates * R4g; float* Dl = Da + (size_t)row0 * T * R4g; float* Zl = Za + (size_t)row0 * T * zs;      // this rank's rows
-        GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)n_local, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, n_local, n_local, 0L, 0L, (const int*)nullptr, (float*)nullptr);
+        GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)n_local, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, n_local, n_local, n_local, 0L, (const int*)nullptr, (float*)nullptr);
         GN_TRY(all_gather_on_comm(m, Dl, Da, (size_t)n_local * R4g, "LSTM update factors D"));
         GN_TRY(all_gather_on_comm(m, Zl, Za, (size_t)n_local * zs, "LSTM update factors Z"));
         GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Da, Dm, R4g, Kc, stride, (long)CG_PAD);
