@@ -103,7 +103,7 @@ static int gemm_tn_stack(Ctx* ctx, int parts, int R, int n, int d, const float* 
   return GN_OK;
 }
 // gemm_tn with the bias gradient gb[N] = sum of dZ over its rows, inside the product where the CUDA-core engine runs it.
-static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate);
+static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate, int slot = 0);
 static int weight_bias_grads(gn_model* m, Ctx* ctx, int R, int N, int K, const float* dZ, long ldz, const float* X, long ldx, float* gW, float* gb) {
   GemmDesc g; g.M = N; g.N = K; g.K = R; g.A = dZ; g.sa_m = 1; g.sa_k = ldz; g.B = X; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = K;
   if (gemm_on_tc(ctx, g)) GN_TRY(colsum(m, dZ, ldz, R, N, gb, false)); else g.a_sum = gb;
@@ -193,7 +193,7 @@ namespace gn {
 // (beyond that the driver's own pageable copy, which overlaps its two stages, is the quicker way)
 constexpr size_t IO_ARGS = 64, STAGE_FLOATS = 1 << 18, STAGE_IN = 1 << 17;
 
-enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_SIDE, S_PART3, S_COUNT };
+enum Slot { S_BNG = 0, S_EMB, S_GRAM0, S_GRAM1, S_DM, S_ZM, S_W, S_TV, S_G0, S_G1, S_ND0, S_ND1, S_ND2, S_ND3, S_ND4, S_NFF, S_NFF2, S_NFF3, S_RN, S_NFFI, S_LNP0, S_LNI0, S_LNP1, S_LNI1, S_RS32, S_ATT0, S_ATT1, S_DELTA, S_PART, S_PART2, S_DZ, S_SCAN, S_XROWS, S_SIDE, S_PART3, S_PART4, S_COUNT };
 
 static int ensure(gn_model* m, int slot, size_t n, float** out) {
   if ((int)m->scratch.size() < S_COUNT) m->scratch.resize(S_COUNT);
@@ -389,11 +389,11 @@ static int ensure_capacity(gn_model* m, int B, bool training) {
 static inline unsigned ew_grid(Ctx* ctx, long n, int block = 256) { long g = (n + block - 1) / block; long mx = (long)ctx->sm_count * 16; return (unsigned)std::max<long>(1, std::min(g, mx)); }
 
 // out[c] (=|+=) sum over R rows of in[r*ld + c]
-static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate) {
+static int colsum(gn_model* m, const float* in, long ld, int R, int C, float* out, bool accumulate, int slot) {
   Ctx* ctx = &m->ctx->c;
   // slabs of 16 rows and up for a batch (bound by the latency of a slab's loads), of 64 and up for many rows
   const int chunks = std::max(1, R <= 1024 ? std::min(R / 16, 16) : std::min(R / 64, 128));
-  float* part; GN_TRY(ensure(m, S_PART, (size_t)chunks * C * 2, &part));
+  float* part; GN_TRY(ensure(m, slot ? slot : S_PART, (size_t)chunks * C * 2, &part));
   GN_LAUNCH(ctx, colsum_partial_kernel, dim3(cdiv(C, 128), chunks), 128, 0, in, ld, R, C, part);
   GN_LAUNCH(ctx, colsum_final_kernel, cdiv(C, 128), 128, 0, part, chunks, C, out, accumulate ? 1 : 0);
   return check_launch("colsum");
@@ -1186,7 +1186,7 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
         }
         float* all; GN_TRY(ensure(m, S_W, (size_t)n_updates * (R4g + zs), &all));
         float* Da = all; float* Za = all + (size_t)n_updates * R4g; float* Dl = Da + (size_t)row0 * T * R4g; float* Zl = Za + (size_t)row0 * T * zs;      // this rank's rows
-        GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)n_local, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, n_local, n_local, n_local, 0L, (const int*)nullptr, (float*)nullptr);
+        GN_LAUNCH(ctx, lstm_gather_updates_kernel, cdiv(n_local, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, n_local, n_local, n_local, n_local, 0L, (const int*)nullptr, (float*)nullptr);
         GN_TRY(all_gather_on_comm(m, Dl, Da, (size_t)n_local * R4g, "LSTM update factors D"));
         GN_TRY(all_gather_on_comm(m, Zl, Za, (size_t)n_local * zs, "LSTM update factors Z"));
         GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Da, Dm, R4g, Kc, stride, (long)CG_PAD);
@@ -1194,7 +1194,7 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
         if (late) GN_LAUNCH(ctx, lstm_row_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)Dm, (const float*)Zm, un, R4g, zs, n_updates, Kc, stride, (long)CG_PAD);
       }
       auto gather = [&](const int* from, float* norms) {
-        GN_LAUNCH(ctx, lstm_gather_updates_kernel, (unsigned)rows, 128, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dm, Zm, T, in, H, zs, n_local, Kc, stride, (long)CG_PAD, from, norms);
+        GN_LAUNCH(ctx, lstm_gather_updates_kernel, cdiv(rows, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dm, Zm, T, in, H, zs, n_local, rows, Kc, stride, (long)CG_PAD, from, norms);
       };
       if (world == 1 && (!late || few)) gather(nullptr, late ? un : nullptr);
       else if (world == 1) GN_LAUNCH(ctx, lstm_update_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, un, T, in, H, n_updates);
@@ -1294,7 +1294,11 @@ static int backward(gn_model* m, int B, const float* gloss, int global_batch, in
           else GN_LAUNCH(ctx, act_backward_kernel, ew_grid(ctx, n), 256, 0, g, d.activation == GN_ACT_RELU ? l.out.p : l.z.p, dzb, n, d.activation, act_alpha_of(d.activation, d.reserved));
           dz = dzb;
         }
-        if (need_dx) GN_TRY(side_weight_bias_grads(m, 1, B, d.out_size, d.in_size, dz, xin, d.in_size, gr, gr + wn));
+        GemmDesc gw; gw.M = d.out_size; gw.N = d.in_size; gw.K = B; gw.A = dz; gw.sa_m = 1; gw.sa_k = d.out_size; gw.B = xin; gw.sb_k = d.in_size; gw.sb_n = 1; gw.C = gr; gw.ldc = d.in_size;
+        if (gemm_on_tc(ctx, gw)) {      // the bias gradient beside the weight gradient's operand planes and product (batch 1000, 1100 outputs: 10 us)
+          GN_TRY(side_run(ctx, [&]() -> int { return colsum(m, dz, d.out_size, B, d.out_size, gr + wn, false, S_PART4); }));
+          GN_TRY(gemm(ctx, gw));
+        } else if (need_dx) GN_TRY(side_weight_bias_grads(m, 1, B, d.out_size, d.in_size, dz, xin, d.in_size, gr, gr + wn));
         else GN_TRY(weight_bias_grads(m, ctx, B, d.out_size, d.in_size, dz, d.out_size, xin, d.in_size, gr, gr + wn));
         gated = false;
         if (need_dx) {

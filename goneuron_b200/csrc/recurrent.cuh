@@ -535,35 +535,33 @@ inline size_t clip_smem(int ZW) {
   const int wp = clip_tile(ZW) | 1; const size_t slab = ((size_t)2 * CG * wp + CG * 8 + (size_t)wp * 8 + 8) * sizeof(float), walk = (size_t)CG * CG_GD * sizeof(double);
   return slab > walk ? slab : walk;
 }
-// Rows of Dm [., 4H] and Zm [., zs], a block each: chunk c's updates from row c * stride + lead on, zeros in the rows before and behind them.
-// (Zeroing those rows separately took two to four more launches per chunk.)  `un` (may be null): receives |u_k|^2 = |d_k|^2 |z_k|^2.
-__global__ void __launch_bounds__(128) lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
-                                           int T, int in, int H, int zs, long n_updates, long Kc, long stride, long lead, const int* __restrict__ start, float* __restrict__ un) {
-  __shared__ float part[2][4];
-  const int R4 = 4 * H, ZW = in + H + 1;
-  const long row = blockIdx.x, chunk = row / stride, r = row - chunk * stride - lead, k = chunk * Kc + r;
+// Rows of Dm [., 4H] and Zm [., zs], a warp each: chunk c's updates from row c * stride + lead on, zeros in the rows before and behind them.
+// (Zeroing those rows separately took two to four more launches per chunk.)  `un` (may be null): receives |u_k|^2 = |d_k|^2 |z_k|^2.  With a block per row
+// the rows that are left out, nearly all of 16 384, cost 12 us.
+__global__ void __launch_bounds__(256) lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
+                                           int T, int in, int H, int zs, long n_updates, long rows, long Kc, long stride, long lead, const int* __restrict__ start, float* __restrict__ un) {
+  const int R4 = 4 * H, ZW = in + H + 1, lane = threadIdx.x & 31;
+  const long row = blockIdx.x * 8L + (threadIdx.x >> 5); if (row >= rows) return;
+  const long chunk = row / stride, r = row - chunk * stride - lead, k = chunk * Kc + r;
   if (start && r < (long)(start[chunk] - 1) * CG) return;                     // before the first walked group and the one it is multiplied with
   if (r < 0 || r >= Kc || k >= n_updates) {
-    for (int e = threadIdx.x; e < R4 + zs; e += blockDim.x) { if (e < R4) Dm[row * R4 + e] = 0.f; else Zm[row * zs + e - R4] = 0.f; }
+    for (int e = lane; e < R4 + zs; e += 32) { if (e < R4) Dm[row * R4 + e] = 0.f; else Zm[row * zs + e - R4] = 0.f; }
     return;
   }
   const int s = (int)(k / T), t = T - 1 - (int)(k % T); float d2 = 0.f, z2 = 0.f;
-  for (int e = threadIdx.x; e < R4 + zs; e += blockDim.x) {
+#pragma unroll 4
+  for (int e = lane; e < R4; e += 32) { const float v = D[((long)s * T + t) * R4 + e]; Dm[row * R4 + e] = v; d2 = fmaf(v, v, d2); }
+#pragma unroll 4
+  for (int c = lane; c < zs; c += 32) {
     float v;
-    if (e < R4) { v = D[((long)s * T + t) * R4 + e]; Dm[row * R4 + e] = v; d2 = fmaf(v, v, d2); }
-    else {
-      const int c = e - R4;
-      if (c < in) v = x[(long)s * T * in + (long)(T - 1) * in + c];                 // input of the LAST forward call (lstm.go:592-621)
-      else if (c < in + H) v = t > 0 ? h_all[((long)s * T + (t - 1)) * H + (c - in)] : 0.f;
-      else v = c < ZW ? 1.f : 0.f;
-      Zm[row * zs + c] = v; z2 = fmaf(v, v, z2);
-    }
+    if (c < in) v = x[(long)s * T * in + (long)(T - 1) * in + c];                 // input of the LAST forward call (lstm.go:592-621)
+    else if (c < in + H) v = t > 0 ? h_all[((long)s * T + (t - 1)) * H + (c - in)] : 0.f;
+    else v = c < ZW ? 1.f : 0.f;
+    Zm[row * zs + c] = v; z2 = fmaf(v, v, z2);
   }
   if (!un) return;
   d2 = warp_sum(d2); z2 = warp_sum(z2);
-  if ((threadIdx.x & 31) == 0) { part[0][threadIdx.x >> 5] = d2; part[1][threadIdx.x >> 5] = z2; }
-  __syncthreads();
-  if (threadIdx.x == 0) un[k] = ((part[0][0] + part[0][1]) + (part[0][2] + part[0][3])) * ((part[1][0] + part[1][1]) + (part[1][2] + part[1][3]));
+  if (lane == 0) un[k] = d2 * z2;
 }
 // rows of `w` floats from contiguous order into the chunks' layout (after a gather over the ranks)
 __global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int w, long Kc, long stride, long lead) {
