@@ -5,6 +5,7 @@
 // and into tiles that are mostly padding.  For 128 images of 32 x 32 x 3 -> 16 channels and 16 x 16 x 16 -> 32 a training step spent
 // 390 us there; the multiply-adds themselves are 1.15 GFLOP, 16 us at the CUDA cores' fp32 rate.
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 #include "conv_lstm.cuh"
 
@@ -24,12 +25,6 @@ __device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const 
     else for (int x = lx; x < n; x += lw) { const bool ok = in && xlo + x >= 0 && xlo + x < W; cp_async4(d + x, ok ? s + x : src, ok); }
     for (r += step; r >= rows; r -= rows) ch++;
   }
-}
-
-// (Not inlined: 16 to 32 copies of all activations in an epilogue that runs once per thread came from a cold instruction cache, 14 us instead of 9 for
-// ReLU.  Four values at a time, so that they overlap.)
-__device__ __noinline__ float4 conv_act(int act, float4 v, float alpha) {
-  return make_float4(act_fwd(act, v.x, alpha), act_fwd(act, v.y, alpha), act_fwd(act, v.z, alpha), act_fwd(act, v.w, alpha));
 }
 
 // ------------------------------------------------------------------ forward and input gradient
@@ -114,44 +109,88 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict_
       }
     }
   }
-  auto finish = [&](int r, int o, float (&v)[4]) {
-    const int y = y0 + ry + r, d = d0 + OC * g + o; if (y >= c.dH || d >= c.Cd) return;
-    const float bv = bias ? bias[d] : 0.f; const long at = (((long)b * c.Cd + d) * c.dH + y) * c.dW + 4 * qx;
+  auto place = [&](int r, int o, long& at) -> bool {                 // where a thread's four pixels of row r, channel o go
+    const int y = y0 + ry + r, d = d0 + OC * g + o; at = (((long)b * c.Cd + d) * c.dH + y) * c.dW + 4 * qx; return y < c.dH && d < c.Cd;
+  };
+  auto put = [&](float* p, long at, const float (&v)[4]) {
+    if ((c.dW & 3) == 0) *reinterpret_cast<float4*>(p + at) = make_float4(v[0], v[1], v[2], v[3]);
+    else {
 #pragma unroll
-    for (int i = 0; i < 4; i++) v[i] += bv;
-    if (z) {
-#pragma unroll
-      for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) z[at + i] = v[i];
+      for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) p[at + i] = v[i];
     }
+  };
+  if constexpr (BWD) {
+    if (c.ks > 1) {                                                  // the groups' sums, in order; every group finishes a share of the rows and channels
+      const int all = npx * c.og, at = tid - kq * all;
+      __syncthreads();
+      if (live) {
+#pragma unroll
+        for (int e = 0; e < RP * OC * 4; e++) sm[(kq * RP * OC * 4 + e) * all + at] = acc[e / (OC * 4)][e / 4 % OC][e % 4];
+      }
+      __syncthreads();
+      if (live) for (int q = kq; q < RP * OC; q += c.ks) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f}; long o;
+        for (int k = 0; k < c.ks; k++) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) v[i] += sm[(k * RP * OC * 4 + q * 4 + i) * all + at];
+        }
+        if (place(q / OC, q % OC, o)) put(out, o, v);
+      }
+      return;
+    }
+  }
+  if (live) {
+#pragma unroll
+    for (int o = 0; o < OC; o++) {
+      const int d = d0 + OC * g + o; const float bv = bias && d < c.Cd ? bias[d] : 0.f;
+#pragma unroll
+      for (int r = 0; r < RP; r++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[r][o][i] += bv;
+        long at; if (z && place(r, o, at)) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) z[at + i] = acc[r][o][i];
+        }
+      }
+    }
+  }
+  if (act != GN_ACT_RELU && act != GN_ACT_LINEAR) {
+    // Through shared memory into a loop with one copy of each activation's code, eight values side by side.  (32 inlined copies of all of them, run once, came
+    // from a cold instruction cache: ReLU took 14 us instead of 9 for 128 images of 32 x 32, 3 -> 16 channels.)
+    __syncthreads();
+    if (!live) return;
+#pragma unroll
+    for (int e = 0; e < RP * OC * 4; e++) sm[e * blockDim.x + tid] = acc[e / (OC * 4)][e / 4 % OC][e % 4];
+    auto apply = [&](auto kind) {
+#pragma unroll 1
+      for (int o = 0; o < OC; o++) {
+        float v[RP][4]; long at;
+#pragma unroll
+        for (int e = 0; e < RP * 4; e++) v[e / 4][e % 4] = act_fwd(decltype(kind)::value, sm[((e / 4 * OC + o) * 4 + e % 4) * blockDim.x + tid], alpha);
+#pragma unroll
+        for (int r = 0; r < RP; r++) if (place(r, o, at)) put(out, at, v[r]);
+      }
+    };
+    switch (act) {
+      case GN_ACT_SIGMOID: apply(std::integral_constant<int, GN_ACT_SIGMOID>{}); break;
+      case GN_ACT_TANH: apply(std::integral_constant<int, GN_ACT_TANH>{}); break;
+      case GN_ACT_LEAKY_RELU: apply(std::integral_constant<int, GN_ACT_LEAKY_RELU>{}); break;
+      case GN_ACT_ELU: apply(std::integral_constant<int, GN_ACT_ELU>{}); break;
+      case GN_ACT_GELU: apply(std::integral_constant<int, GN_ACT_GELU>{}); break;
+      case GN_ACT_SILU: apply(std::integral_constant<int, GN_ACT_SILU>{}); break;
+      default: apply(std::integral_constant<int, GN_ACT_LINEAR>{});
+    }
+    return;
+  }
+  if (!live) return;
+#pragma unroll
+  for (int q = 0; q < RP * OC; q++) {
+    float (&v)[4] = acc[q / OC][q % OC]; long at;
     if (act == GN_ACT_RELU) {
 #pragma unroll
       for (int i = 0; i < 4; i++) v[i] = v[i] > 0.f ? v[i] : 0.f;
-    } else if (act != GN_ACT_LINEAR) { const float4 a = conv_act(act, make_float4(v[0], v[1], v[2], v[3]), alpha); v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; }
-    if ((c.dW & 3) == 0) *reinterpret_cast<float4*>(out + at) = make_float4(v[0], v[1], v[2], v[3]);
-    else {
-#pragma unroll
-      for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) out[at + i] = v[i];
     }
-  };
-  if (c.ks > 1) {                                                    // the groups' sums, in order; every group finishes a share of the rows and channels
-    const int all = npx * c.og, at = tid - kq * all;
-    __syncthreads();
-    if (live) {
-#pragma unroll
-      for (int e = 0; e < RP * OC * 4; e++) sm[(kq * RP * OC * 4 + e) * all + at] = acc[e / (OC * 4)][e / 4 % OC][e % 4];
-    }
-    __syncthreads();
-    if (live) for (int q = kq; q < RP * OC; q += c.ks) {
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int k = 0; k < c.ks; k++) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) v[i] += sm[(k * RP * OC * 4 + q * 4 + i) * all + at];
-      }
-      finish(q / OC, q % OC, v);
-    }
-  } else if (live) {
-#pragma unroll
-    for (int q = 0; q < RP * OC; q++) finish(q / OC, q % OC, acc[q / OC][q % OC]);
+    if (place(q / OC, q % OC, at)) put(out, at, v);
   }
 }
 
@@ -219,11 +258,9 @@ __global__ void __launch_bounds__(256) conv_wgrad_tile_kernel(const float* __res
     }
   }
   __syncthreads();
-  if (live) for (int v = pg; v < NV; v += c.pg) {                    // (in the order of the threads; the kernel below finds the places)
-    float a = 0.f;
-    for (int k = 0; k < c.pg; k++) a += red[v * all + k * items + it];
-    prow[v * items + it] = a;
-  }
+  auto sum = [&](int v, int q) { float a = 0.f; for (int k = 0; k < c.pg; k++) a += red[v * all + k * items + q]; prow[v * items + q] = a; };      // (in the order of the threads; the kernel below finds the places)
+  if (2 * all > (int)blockDim.x) { if (live) for (int v = pg; v < NV; v += c.pg) sum(v, it); }
+  else for (int e = tid; e < items * NV; e += blockDim.x) sum(e / items, e % items);      // (few items: all threads add up)
 }
 // dst[i] = sum over the blocks' sets, in order: 32 elements x 8 groups of sets per block (weights, then biases: the gradient slice is laid out W | b)
 __global__ void __launch_bounds__(256) conv_wgrad_final_kernel(const float* __restrict__ part, int sets, int n, float* __restrict__ dst) {
@@ -295,7 +332,7 @@ inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const fl
   c.icc = std::max<int>(1, std::min<int>(c.Cs, 48 * 1024 / per));
   if (c.icc < c.Cs) c.icc = std::max(c.ks, c.icc / c.ks * c.ks);     // (a channel's group of threads does not depend on how many are staged at once)
   const int all = c.qw * rg * c.og, threads = (all * c.ks + 31) & ~31;
-  const size_t smem = std::max(c.icc * per + (size_t)c.og * OC * sizeof(float), (size_t)(c.ks > 1 ? c.ks : 0) * RP * OC * 4 * all * sizeof(float));
+  const size_t smem = std::max(c.icc * per + (size_t)c.og * OC * sizeof(float), (size_t)(c.ks > 1 ? c.ks * all : act != GN_ACT_RELU && act != GN_ACT_LINEAR ? threads : 0) * RP * OC * 4 * sizeof(float));
   GN_CUDA(cudaFuncSetAttribute(conv_tile_kernel<K, BWD, SAME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GN_LAUNCH(ctx, (conv_tile_kernel<K, BWD, SAME>), dim3(cdiv(c.dH, c.rb), B, cdiv(groups, c.og)), threads, smem, src, W, bias, z, out, c, act, alpha);
   return check_launch("conv_tile");
@@ -335,6 +372,7 @@ inline ConvWg conv_wgrad_plan(Ctx* ctx, const ConvShape& s, int OT, int* sets, s
     const int want = std::max<int>(1, std::min<long>(s.oH, ctx->sm_count / std::max<long>(1, s.B * tiles)));
     c.rb = std::min(c.rb, (int)cdiv(s.oH, want)); c.bands = cdiv(s.oH, c.rb);
   }
+  c.rb = cdiv(s.oH, c.bands);                                        // even bands (a short last one takes a block as well: 3 -> 32 channels, 64 images of 40 x 40 24.2 -> 20.7 us, 32 -> 64, 20 x 20 63.9 -> 45.0)
   c.xplane = plane((c.rb + s.k - 1) * c.swp); c.gplane = plane(c.rb * c.gwp);
   const int items = c.ocb / OT * c.icb; c.pg = std::max(1, std::min(c.rb, 256 / items));
   c.units = s.B * c.bands;
