@@ -524,8 +524,8 @@ inline int gru_bwd_reg(Ctx* ctx, const float* gout, const float* Wh, const float
 // walk starts from zero at the first group that can be seen in the result (lstm_clip_start_kernel), at group 0 if there is none,
 // or if any update is not finite.  Gradients that are carried back through many steps grow by orders of magnitude per sequence
 // (median |u| 2e5 for 64 steps of 128 units), and a few dozen updates decide the result.  What is not walked is not gathered and
-// has no Gram blocks either: that step of 256 samples, on a batch in device memory, went from 1682 us to 496.  Where nothing can be left
-// out it takes 1685: the norms and the search take 8 us, and the rows of zeros come without launches of their own.
+// has no Gram blocks either: that step of 256 samples, on a batch in device memory, went from 1682 us to 496 (289 since, with the recurrences above and lstm_clip_start_kernel's
+// condition).  Where nothing can be left out it took 1685 (now 1618): the norms and the search take 8 us, and the rows of zeros come without launches of their own.
 constexpr int CG = 128, CG_THREADS = 512, CG_PAD = CG, CG_TILE = 160;        // CG_PAD: rows of zeros before a chunk: group -1
 constexpr int CG_GD = CG + 1;
 constexpr long CG_MAX_K = 1L << 20;                         // updates per worker chunk
