@@ -324,41 +324,62 @@ inline bool gemm_outer_small_ok(const GemmDesc& g) {
 // A block of the cluster takes a power of two of neighbouring chunks, so their number per block (it falls with the number of tiles) does not
 // matter, and where the rows of A are samples a sample's result is the same in every batch.
 // us per launch in a recorded chain, a 32 x 32 tile in two register-staged steps per run, results read from the other blocks -> this:
-//   64 x 256 over 256 4.9 -> 3.8, over 1024 6.8 -> 6.0; 128 x 1024 over 256 7.6 -> 5.9; 1 x 128 over 784 5.6 -> 3.4; 8 x 8192 over 512 13.3 -> 7.1;
-//   16 x 512 over 8192 25.6 -> 15.2; a 96 x 96 weight gradient over 5000 rows 14.3 -> 10.4.  The same chain of empty launches: 2.2.
+//   64 x 256 over 256 4.9 -> 3.7, over 1024 7.5 -> 5.9; 128 x 1024 over 256 7.6 -> 5.8; 1 x 128 over 784 5.6 -> 3.5; 8 x 8192 over 512 13.3 -> 7.4;
+//   16 x 512 over 8192 25.7 -> 15.4; a 96 x 96 weight gradient over 5000 rows 14.3 -> 10.1.  The same chain of empty launches: 2.2.
 constexpr int SP_KB = 64, SP_BN = 32, SP_STAGES = 4, SP_THREADS = 256, SP_MAX_SPLITS = 8;
 constexpr int sp_smem(int tm) { return (SP_STAGES * SP_KB * (4 * tm + SP_BN) + 8 * 4 * tm * SP_BN) * (int)sizeof(float); }
 // Brings ROWS operand rows x 64 indices into shared memory, stage by stage.  KFAST: [row][64], 16-byte units swizzled by the row's position among
 // fours (eight lanes that read one unit of rows four apart find it in different banks); else [64][ROWS].
-template <int ROWS, bool KFAST>
+template <int ROWS, bool KFAST, int THREADS = SP_THREADS>
 struct SpLoad {
-  static constexpr int NV = ROWS * SP_KB / 4, NQ = (NV + SP_THREADS - 1) / SP_THREADS;
+  static constexpr int NV = ROWS * SP_KB / 4, NQ = (NV + THREADS - 1) / THREADS;
   const float *base, *src[NQ]; long s_r, s_k; int nr; bool vec;
   __device__ __forceinline__ static void place(int q, int& r, int& k) {
-    const int e = q * SP_THREADS + threadIdx.x;
+    const int e = q * THREADS + threadIdx.x;
     if (KFAST) { r = e >> 4; k = (e & 15) * 4; } else { r = e % (ROWS / 4) * 4; k = e / (ROWS / 4); }
   }
   __device__ __forceinline__ SpLoad(const float* p, long s_r_, long s_k_, int nr_, bool v) : base(p), s_r(s_r_), s_k(s_k_), nr(nr_), vec(v) {
 #pragma unroll
     for (int q = 0; q < NQ; q++) { int r, k; place(q, r, k); src[q] = p + (KFAST ? r * s_r + k : r + k * s_k); }
   }
-  __device__ __forceinline__ void fetch(float* __restrict__ dst, int nk) {      // nk: indices that are left, this stage included
+  // nk: indices that are left, this stage included; upto: how many of the stage's are read later.  PLAIN: rows that 16-byte copies do not fit come by
+  // loads and stores, 16 of a thread's at a time, instead of 4-byte asynchronous copies (whole stages waited for at once: 2 to 10 % quicker).
+  template <bool PLAIN = false>
+  __device__ __forceinline__ void fetch(float* __restrict__ dst, int nk, int upto = SP_KB) {
     if (vec) {
 #pragma unroll
       for (int q = 0; q < NQ; q++) {
         int r, k; place(q, r, k);
-        if (NV % SP_THREADS != 0 && q * SP_THREADS + (int)threadIdx.x >= NV) break;
+        if (NV % THREADS != 0 && q * THREADS + (int)threadIdx.x >= NV) break;
+        if (k >= upto) continue;
         const int n = KFAST ? (r < nr ? min(max(nk - k, 0), 4) : 0) : (k < nk ? min(max(nr - r, 0), 4) : 0);
         cp_async16_part(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) : k * ROWS + r), n ? src[q] : base, n);
         src[q] += KFAST ? (long)SP_KB : SP_KB * s_k;
       }
     } else {
       const int r0 = KFAST ? threadIdx.x >> 6 : threadIdx.x % ROWS, k0 = KFAST ? threadIdx.x & 63 : threadIdx.x / ROWS; const float* p = base + r0 * s_r + k0 * s_k;
+      constexpr int RSTEP = THREADS / SP_KB, KSTEP = THREADS / ROWS;
+      if (PLAIN) {
+        constexpr int NF = 16;
+        for (int q0 = 0; q0 < ROWS * SP_KB / THREADS; q0 += NF) {
+          float x[NF];
 #pragma unroll
-      for (int q = 0; q < ROWS / 4; q++) {
-        const int r = KFAST ? r0 + 4 * q : r0, k = KFAST ? k0 : k0 + SP_THREADS / ROWS * q; const bool ok = r < nr && k < nk;
-        cp_async4(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) + (k & 3) : k * ROWS + r), ok ? p : base, ok);
-        p += KFAST ? 4 * s_r : SP_THREADS / ROWS * s_k;
+          for (int j = 0; j < NF; j++) {
+            const int r = KFAST ? r0 + RSTEP * (q0 + j) : r0, k = KFAST ? k0 : k0 + KSTEP * (q0 + j);
+            x[j] = r < nr && k < nk ? *p : 0.f; p += KFAST ? RSTEP * s_r : KSTEP * s_k;
+          }
+#pragma unroll
+          for (int j = 0; j < NF; j++) {
+            const int r = KFAST ? r0 + RSTEP * (q0 + j) : r0, k = KFAST ? k0 : k0 + KSTEP * (q0 + j);
+            if (k < upto) dst[KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) + (k & 3) : k * ROWS + r] = x[j];
+          }
+        }
+      } else
+#pragma unroll
+      for (int q = 0; q < ROWS * SP_KB / THREADS; q++) {
+        const int r = KFAST ? r0 + RSTEP * q : r0, k = KFAST ? k0 : k0 + KSTEP * q; const bool ok = r < nr && k < nk;
+        if (k < upto) cp_async4(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) + (k & 3) : k * ROWS + r), ok ? p : base, ok);
+        p += KFAST ? RSTEP * s_r : KSTEP * s_k;
       }
       if (nk > SP_KB) base += SP_KB * s_k;
     }
@@ -501,11 +522,139 @@ __global__ void __launch_bounds__(SP_THREADS, 2) gemm_small_kernel(const GemmDes
   if (n + 3 < g.N && (reinterpret_cast<uintptr_t>(c) & 15) == 0) *reinterpret_cast<float4*>(c) = make_float4(o[0], o[1], o[2], o[3]);
   else for (int j = 0; j < 4; j++) if (n + j < g.N) c[j] = o[j];
 }
+// The same sums, bit for bit, where there are many tiles: 64 x 32 outputs per block, 4 x 4 per thread, a chunk of the contraction (up to RS_MAX_PER indices) in
+// shared memory at a time.  The kernel above passes eight partial sums of every output through shared memory and starts anew for each 32 x 32 tile: two
+// blocks per SM hide that in one round of blocks, several rounds do not.  Here a thread adds up the eight parts by itself, one after the other (indices
+// 0 .. 7 of every stage, then 8 .. 15 of every stage, ...), and keeps the sums of one, two or four chunks (CHUNKS) in registers; further chunks are those of
+// the cluster's other blocks, which leave their sums in shared memory and finish a share of the tile each.  Figures at gemm_small.
+constexpr int RS_BM = 64, RS_BN = 32, RS_THREADS = RS_BM * RS_BN / 16, RS_STAGE = SP_KB * (RS_BM + RS_BN), RS_MAX_PER = 4 * SP_KB;
+template <int CHUNKS, bool B_NFAST>
+__global__ void __launch_bounds__(RS_THREADS, 4) gemm_rows_kernel(const GemmDesc g, int splits, int per, int vec_a, int vec_b, int y0) {
+  constexpr int TX = RS_BN / 4;
+  extern __shared__ __align__(16) float sm[];                 // the stages of a chunk, A | B, laid out as above
+  const int b = blockIdx.z, b1 = b / g.batch2, b2 = b % g.batch2, rank = blockIdx.x % splits;
+  const float* A = g.A + b1 * g.a_b1 + b2 * g.a_b2;
+  const float* B = g.B + b1 * g.b_b1 + b2 * g.b_b2;
+  float* C = g.C + b1 * g.c_b1 + b2 * g.c_b2;
+  const float* R = g.R ? g.R + b1 * g.r_b1 + b2 * g.r_b2 : nullptr;
+  const int m0 = (y0 + blockIdx.y) * RS_BM, n0 = blockIdx.x / splits * RS_BN, tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  if ((g.flags & GEMM_SKIP_UPPER) && n0 > m0 + RS_BM - 1) return;
+  const int kbeg = g.flags & GEMM_KBEG_AT_M0 ? m0 : 0, kend = g.flags & GEMM_KEND_AT_M0 ? min(g.K, m0 + RS_BM) : g.K;
+  float v[4][4], s1[4][4], s2[4][4];                          // the sum; sums of one and two chunks that wait for their neighbours
+#pragma unroll
+  for (int c = 0; c < CHUNKS; c++) {
+    const int at = (rank * CHUNKS + c) * per, k0 = max(at, kbeg), k1 = min(at + per, kend), stages = k1 > k0 ? (k1 - k0 + SP_KB - 1) / SP_KB : 0, k_at = stages ? k0 : 0;
+    if (c > 0) __syncthreads();                               // (the chunk before has been read)
+    SpLoad<RS_BM, true, RS_THREADS> la(A + (long)m0 * g.sa_m + k_at, g.sa_m, 1, g.M - m0, vec_a);
+    SpLoad<RS_BN, !B_NFAST, RS_THREADS> lb(B + (long)n0 * g.sb_n + (long)k_at * g.sb_k, g.sb_n, g.sb_k, g.N - n0, vec_b);
+    for (int s = 0; s < stages; s++) {
+      float* d = sm + s * RS_STAGE; const int nk = k1 - k0 - s * SP_KB, upto = min((nk + 7) & ~7, SP_KB);
+      la.template fetch<true>(d, nk, upto); lb.template fetch<true>(d + SP_KB * RS_BM, nk, upto);
+    }
+    cp_async_wait();
+    __syncthreads();
+#pragma unroll 1
+    for (int w = 0; w < 8; w++) {
+      float acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+      const int ws = max(0, k1 - k0 - 8 * w + SP_KB - 1) / SP_KB;      // stages that hold indices of this part
+      for (int s = 0; s < ws; s++) {
+        const float* As = sm + s * RS_STAGE; const float* Bs = As + SP_KB * RS_BM;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int k = 8 * w + 4 * h; float a[4][4], bv[4][4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const float4 x = *reinterpret_cast<const float4*>(As + (4 * ty + i) * SP_KB + (((k >> 2) ^ (ty & 7)) << 2));
+            a[0][i] = x.x; a[1][i] = x.y; a[2][i] = x.z; a[3][i] = x.w;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            if (B_NFAST) {
+              const float4 x = *reinterpret_cast<const float4*>(Bs + (k + j) * RS_BN + 4 * tx); bv[j][0] = x.x; bv[j][1] = x.y; bv[j][2] = x.z; bv[j][3] = x.w;
+            } else {
+              const float4 x = *reinterpret_cast<const float4*>(Bs + (4 * tx + j) * SP_KB + (((k >> 2) ^ tx) << 2));
+              bv[0][j] = x.x; bv[1][j] = x.y; bv[2][j] = x.z; bv[3][j] = x.w;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+              for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[q][i], bv[q][j], acc[i][j]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[i][j] = w == 0 ? acc[i][j] : v[i][j] + acc[i][j];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (c & 1) { v[i][j] = s1[i][j] + v[i][j]; if (c & 2) v[i][j] = s2[i][j] + v[i][j]; else s2[i][j] = v[i][j]; }
+        else s1[i][j] = v[i][j];
+      }
+  }
+  auto store = [&](int m, int n, float x0, float x1, float x2, float x3) {
+    if (m >= g.M || n >= g.N) return;
+    float* c = C + (long)m * g.ldc + n; const float x[4] = {x0, x1, x2, x3}; float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) o[j] = n + j < g.N ? sg_finish(g, R, m, n + j, x[j]) : 0.f;
+    if (n + 3 < g.N && (reinterpret_cast<uintptr_t>(c) & 15) == 0) *reinterpret_cast<float4*>(c) = make_float4(o[0], o[1], o[2], o[3]);
+    else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) if (n + j < g.N) c[j] = o[j];
+    }
+  };
+  if (splits > 1) {                                            // the blocks' sums, pairwise; every block finishes a share of the tile
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    float4* xch = reinterpret_cast<float4*>(sm);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++) xch[(4 * ty + i) * TX + tx] = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+    cluster.sync();
+    const int share = RS_BM * TX / splits;
+    for (int e = rank * share + threadIdx.x; e < (rank + 1) * share; e += RS_THREADS) {
+      auto add = [](const float4& a, const float4& x) { return make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w); };
+      auto pair = [&](int q) { return add(cluster.map_shared_rank(xch, q)[e], cluster.map_shared_rank(xch, q + 1)[e]); };
+      float4 x = pair(0);
+      if (splits > 2) x = add(x, pair(2));
+      if (splits > 4) { const float4 y = pair(4); x = add(x, add(y, pair(6))); }
+      store(m0 + e / TX, n0 + e % TX * 4, x.x, x.y, x.z, x.w);
+    }
+    cluster.sync();                                            // nobody leaves while its sums are being read
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) store(m0 + 4 * ty + i, n0 + 4 * tx, v[i][0], v[i][1], v[i][2], v[i][3]);
+}
+inline bool sg_vec(const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; }
+inline int gemm_rows(Ctx* ctx, const GemmDesc& g, int splits, int chunks, int per) {
+  const bool bn = g.sb_n == 1; if (!bn && g.sb_k != 1) return fail(GN_ERR_UNSUPPORTED, "gemm_rows: neither stride of an operand is 1");
+  const int va = sg_vec(g.A, g.sa_m, g.a_b1, g.a_b2), vb = sg_vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2), tiles_m = cdiv(g.M, RS_BM), smem = per / SP_KB * RS_STAGE * (int)sizeof(float);
+  for (int y0 = 0; y0 < tiles_m; y0 += 65535) {
+    const dim3 grid(cdiv(g.N, RS_BN) * splits, std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
+    auto run = [&](auto* K) -> int {
+      GN_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (splits > 1) GN_CLUSTER_LAUNCH(ctx, K, grid, RS_THREADS, smem, splits, g, splits, per, va, vb, y0);
+      else GN_LAUNCH(ctx, K, grid, RS_THREADS, smem, g, splits, per, va, vb, y0);
+      return GN_OK;
+    };
+    if (bn) GN_TRY(chunks == 1 ? run(gemm_rows_kernel<1, true>) : chunks == 2 ? run(gemm_rows_kernel<2, true>) : run(gemm_rows_kernel<4, true>));
+    else GN_TRY(chunks == 1 ? run(gemm_rows_kernel<1, false>) : chunks == 2 ? run(gemm_rows_kernel<2, false>) : run(gemm_rows_kernel<4, false>));
+  }
+  return check_launch("gemm_rows");
+}
 template <int TM>
 inline int gemm_small_tile(Ctx* ctx, const GemmDesc& g, int splits, int chunks, int per) {
-  auto vec = [](const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; };
   const bool ak = g.sa_k == 1 && !g.a_sum, bn = g.sb_n == 1;      // (the sums of A's rows come with the other layout; one row has both)
-  const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
+  const int va = (ak || g.sa_m == 1) && sg_vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && sg_vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
   const int tiles_m = cdiv(g.M, 4 * TM), smem = sp_smem(TM);
   for (int y0 = 0; y0 < tiles_m; y0 += 65535) {             // (a grid's second dimension)
     const dim3 grid(cdiv(g.N, SP_BN) * splits, std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
@@ -521,17 +670,43 @@ inline int gemm_small_tile(Ctx* ctx, const GemmDesc& g, int splits, int chunks, 
   }
   return check_launch("gemm_small");
 }
-// How many chunks, and over how many blocks they go.  A chunk shorter than 64 indices (96 where a sample has more than 256 outputs) is not worth
-// its own sum; the number of chunks goes by the matrix alone where the rows of A are samples (or tokens), see above.  Blocks until
-// five eighths of the SMs have one, and, as two fit an SM, up to twice as many while a run is 384 indices or longer.
+// How many chunks, over how many blocks they go, and which kernel.  A chunk shorter than 64 indices (96 where a sample has more than 256 outputs) is not worth
+// its own sum; the number of chunks goes by the matrix alone where the rows of A are samples (or tokens), see above: few enough for five eighths of the SMs, or
+// for all of them with runs of 384 indices, and seven tenths of them have to have indices (640 in eight chunks of whole stages would be five of 128).
+// The rest changes no bit.  Weight gradients and 16 rows or fewer: blocks by the same measure.  Else by estimated time, from measurements of 1900 shapes between
+// 17 and 16 384 rows (us; 5 and 10 % off).  gemm_small_kernel: 1.4, and for every round of two blocks per SM 1.65 times what a block alone takes, 0.57 + 0.73 per stage
+// of 64 indices + 0.45 per chunk + 0.45 for an exchange.  gemm_rows_kernel: 2.6, and 1.38 per 64 indices + 1.25 per chunk, 0.55 more of that for each further block
+// on the SM; 1.15 times as much where 16-byte copies do not fit.  us, 32 x 32 tiles -> 64 x 32: 4096 x 200 over 72 15.3 -> 9.7, 16 384 x 40 over 64 11.8 -> 8.7, 3000 x 300
+// over 64 11.5 -> 8.6, 500 x 1500 over 130 20.7 -> 14.5, 1024 x 200 over 256 10.4 -> 9.3, 511 x 300 over 500 15.5 -> 11.3; the other way 256 x 600 over 80 5.1 -> 6.0, 1024 x 100 over
+// 192 5.1 -> 6.1.  Chunks, geometric mean of the time of 1900 smaller shapes against these lines: half, three quarters, all of the
+// SMs 1.000, 1.002, 1.003; runs of 256, 768 instead of 384 1.001, 1.000; chunks of 64, 128 instead of 96 1.002, 0.999, of 96, 128 instead of 64 1.015, 1.027.
+// Still slower than one pass over 64 x 64 tiles (whose order of sums is another one): more than 1000 tiles over 64 to 96 indices, 16 384 x 40 over 64 8.7 against 7.4, and rows
+// that 16-byte copies do not fit, 777 x 1500 over 65 17.0 against 12.5.
 inline int gemm_small(Ctx* ctx, const GemmDesc& g) {
   const int tm = g.M <= 8 ? 2 : g.M <= 16 ? 4 : 8; const bool rows = g.sa_k == 1;
-  const long tn = cdiv(g.N, SP_BN), tiles = tn * cdiv(g.M, 4 * tm) * g.batch1 * g.batch2; const int run = rows && tn > 8 ? 96 : 64;
-  auto more = [&](long blocks, int n) { return blocks * n < 5L * ctx->sm_count / 8 || (blocks * n <= ctx->sm_count && g.K >= 384 * n); };
-  int all = 1, splits = 1;
-  while (all < SP_MAX_SPLITS && g.K >= 2 * run * all && more(rows ? tn : tiles, all)) all *= 2;
-  while (splits < all && more(tiles, splits)) splits *= 2;
-  const int per = cdiv(cdiv(g.K, all), SP_KB) * SP_KB, chunks = all / splits;
+  const long nb = (long)g.batch1 * g.batch2, tn = cdiv(g.N, SP_BN), tiles = tn * cdiv(g.M, 4 * tm) * nb; const int run = rows && tn > 8 ? 96 : 64, sms = ctx->sm_count;
+  auto more = [&](long blocks, int n) { return blocks * n < 5L * sms / 8 || (blocks * n <= sms && g.K >= 384 * n); };
+  auto length = [&](int n) { return (int)cdiv(cdiv(g.K, n), SP_KB) * SP_KB; };
+  int all = 1, splits = 1; bool big = false;
+  while (all < SP_MAX_SPLITS && g.K >= 2 * run * all && more(rows ? tn : tiles, all) && 10 * cdiv(g.K, length(2 * all)) >= 14u * all) all *= 2;
+  const int per = length(all);
+  if (tm < 8 || !rows) { while (splits < all && more(tiles, splits)) splits *= 2; }
+  else {
+    const bool bn = g.sb_n == 1, can = !g.a_sum && per <= RS_MAX_PER;
+    const double odd = sg_vec(g.A, g.sa_m, g.a_b1, g.a_b2) && sg_vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2) ? 1.0 : 1.15; double best = 1e30;
+    for (int s = 1; s <= all; s *= 2) {
+      const int chunks = all / s, len = std::min(g.K, chunks * per);
+      const long rest = (tiles * s - 1) % (2L * sms) + 1, full = (tiles * s - rest) / (2L * sms);
+      const double one = 0.57 + 0.73 * cdiv(len, SP_KB) + 0.45 * chunks + (s > 1 ? 0.45 : 0.0), t = 1.4 + one * (1.65 * full + (rest > sms ? 1.65 : 1.0));
+      if (t < best) { best = t; splits = s; big = false; }
+      if (!can || chunks > 4) continue;
+      const double fit = std::min(4L, 227L * 1024 / (per / SP_KB * RS_STAGE * 4 + 1024)), q = (double)(tn * cdiv(g.M, RS_BM) * nb * s) / sms, work = 1.38 * len / SP_KB + 1.25 * chunks;
+      const double u = odd * (2.6 + work * (q <= fit ? 1.0 + 0.55 * (std::ceil(q) - 1.0) : (1.0 + 0.55 * (fit - 1.0)) * q / fit));
+      if (u < best) { best = u; splits = s; big = true; }
+    }
+  }
+  const int chunks = all / splits;
+  if (big) return gemm_rows(ctx, g, splits, chunks, per);
   return tm == 2 ? gemm_small_tile<2>(ctx, g, splits, chunks, per) : tm == 4 ? gemm_small_tile<4>(ctx, g, splits, chunks, per) : gemm_small_tile<8>(ctx, g, splits, chunks, per);
 }
 
@@ -550,9 +725,8 @@ inline int gemm_outer_group(Ctx* ctx, const GemmDesc* d, int n) {
 
 template <int BM, int BN, int BK, int TM, int TN>
 inline int gemm_simt_tile(Ctx* ctx, const GemmDesc& g) {
-  auto vec = [](const float* p, long ld, long b1, long b2) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0 && b1 % 4 == 0 && b2 % 4 == 0; };
   const bool ak = g.sa_k == 1, bn = g.sb_n == 1;
-  const int va = (ak || g.sa_m == 1) && vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
+  const int va = (ak || g.sa_m == 1) && sg_vec(g.A, ak ? g.sa_m : g.sa_k, g.a_b1, g.a_b2), vb = (bn || g.sb_k == 1) && sg_vec(g.B, bn ? g.sb_k : g.sb_n, g.b_b1, g.b_b2);
   const int tiles_m = cdiv(g.M, BM); constexpr int THREADS = SgCfg<BM, BN, BK, TM, TN>::THREADS;
   for (int y0 = 0; y0 < tiles_m; y0 += 65535) {             // (a grid's second dimension)
     const dim3 grid(cdiv(g.N, BN), std::min(tiles_m - y0, 65535), g.batch1 * g.batch2);
@@ -583,7 +757,9 @@ inline int gemm_simt(Ctx* ctx, const GemmDesc& g) {
   }
   // (which kernel adds up a sample's sums must not depend on the number of samples either)
   const long t64 = (long)cdiv(g.M, 64) * cdiv(g.N, 64) * g.batch1 * g.batch2;
-  if (g.K >= SP_KB && (g.sa_k == 1 || t64 < ctx->sm_count) && (!g.a_sum || g.sa_m == 1)) return gemm_small(ctx, g);
+  // (weight gradients of short contractions: more tiles than two per SM are quicker without the sums of eight warps, 1100 x 333 over 100 7.9 -> 7.0)
+  const bool quick = g.sa_k != 1 && g.K < 128 && (long)cdiv(g.M, 32) * cdiv(g.N, 32) * g.batch1 * g.batch2 > 2L * ctx->sm_count;
+  if (g.K >= SP_KB && (g.sa_k == 1 || (t64 < ctx->sm_count && !quick)) && (!g.a_sum || g.sa_m == 1)) return gemm_small(ctx, g);
   // 16-row tiles for a handful of rows; 32 x 32 tiles (a quarter of the work per block) when 64 x 64 would not give every SM one or
   // be half empty
   if (g.M <= 16) return gemm_simt_tile<16, 64, 32, 2, 4>(ctx, g);

@@ -42,7 +42,24 @@ def test_rows_against_float64_and_the_same_in_every_batch(device, N, K):
         assert np.array_equal(product(device, A[:m], B, bias), whole[:m]), m
 
 
-@pytest.mark.parametrize("I,H,O,batch", [(64, 64, 64, 64), (65, 33, 17, 65), (100, 200, 40, 70), (31, 129, 18, 300), (784, 128, 20, 127), (36, 300, 24, 1000), (9, 70, 1, 256)])
+@pytest.mark.parametrize("M,N,K", [(3001, 33, 72), (5000, 33, 65), (2050, 130, 65), (9001, 33, 130), (5000, 70, 130), (9001, 33, 260),      # one, two and four chunks per block
+                                   (5000, 33, 128), (5000, 100, 191), (777, 70, 256), (300, 100, 512),                              # ... a chunk per block of two, four and eight
+                                   (5000, 100, 256), (5000, 100, 512), (5000, 33, 512)])                                            # ... several per block of several
+def test_many_rows_have_the_sums_of_few(device, N, K, M):
+    """Many tiles go to a kernel of larger tiles, which adds up in the same order: the same bits, whatever clusters both take."""
+    rng = np.random.Generator(np.random.PCG64(M + N + K))
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K)).astype(np.float32)
+    bias = rng.standard_normal(N).astype(np.float32)
+    whole = product(device, A, B, bias)
+    for rows in (slice(0, 70), slice(M // 2, M // 2 + 33), slice(M - 65, M)):
+        assert np.array_equal(product(device, A[rows], B, bias), whole[rows])
+    bound = (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T + np.abs(bias)) * (K / 8 + 16) * 2.0 ** -24
+    assert np.all(np.abs(whole - (A.astype(np.float64) @ B.astype(np.float64).T + bias)) <= bound)
+
+
+@pytest.mark.parametrize("I,H,O,batch", [(64, 64, 64, 64), (65, 33, 17, 65), (100, 200, 40, 70), (31, 129, 18, 300), (784, 128, 20, 127), (36, 300, 24, 1000), (9, 70, 1, 256),
+                                          (9, 200, 72, 2050), (9, 99, 256, 2050), (333, 1100, 20, 100)])      # many tiles
 def test_dense_gradients(device, oracle, I, H, O, batch):
     """Input and weight gradients of Dense layers: the operands' other orders, and the bias gradients that come with them."""
     from goneuron_b200.sequential import Adam, Sequential
