@@ -30,19 +30,20 @@ __device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const 
 // ------------------------------------------------------------------ forward and input gradient
 // dst[b, d, y, x] = act( bias[d] + sum_{s, kh, kw} w(d, s, kh, kw) src[b, s, y + kh - p, x + kw - p] ), zeros outside.  Forward: w = W[d][s].
 // Input gradient (BWD): src = gradient of the pre-activation, w = W[s][d] mirrored, p = K - 1 - pad.
-// A thread owns 4 neighbouring pixels of two rows x 4 channels and every `ks`-th source channel; a block a band of `rb` rows of one image and
+// A thread owns 4 neighbouring pixels of RP = two rows (one, where the activation is the longer part) x 4 channels and every `ks`-th source channel; a block a band of `rb` rows of one image and
 // `og` groups of 4 channels, with the source rows and the weights of `icc` source channels at a time in shared memory.  What bounds it is less
 // the arithmetic than everything around it: index arithmetic and uncoalesced copies on the way into shared memory, by few threads, took most
 // of its time.  So the weights are copied in their own order, image rows in 16-byte pieces where the window keeps the image's size (SAME; the border is
 // then left out where the pixels are read, not stored), and the input gradient's source channels are dealt out to `ks` groups of threads (by the
 // shapes alone: a sample's sums are the same in every batch), whose sums meet in shared memory.  A 3 x 3 window's weights stay in registers for both rows.
+// SMOOTH: an activation other than ReLU and linear (in a kernel of its own: beside it ReLU's took 2 to 3 % longer).
 // One row and up to 8 channels per thread, everything copied element by element in the order of shared memory -> this, us in a recorded chain: 3 -> 16 channels, 128
 // images of 32 x 32 14.3 -> 7.0; 16 -> 32, 16 x 16 forward 23.4 -> 13.4, input gradient 36.5 -> 13.2; 1 -> 24, 50 of 28 x 28 5.9 -> 4.5.
 struct ConvTile { int Cs, Cd, sH, sW, dH, dW, p, rb, og, icc, qw, swp, aligned, ks; };
-template <int K, bool BWD, bool SAME>
+template <int K, bool BWD, bool SAME, int RP, bool SMOOTH>
 __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict__ src, const float* __restrict__ W, const float* __restrict__ bias,
                                                         float* __restrict__ z, float* __restrict__ out, const ConvTile c, int act, float alpha) {
-  constexpr int KK = K * K, RP = 2, OC = 4, HALO = (K - 1) / 2;
+  constexpr int KK = K * K, OC = 4, HALO = (K - 1) / 2;
   extern __shared__ __align__(16) float sm[];
   const int rows = c.rb + K - 1, ocb = c.og * OC, wn = BWD ? ocb * KK : c.icc * KK | 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   float* xs = sm; float* ws = xs + c.icc * rows * c.swp;            // [icc][rows][swp]; weights [ocb][wn] (forward: icc K K of them, odd: channel groups in different banks) or [icc][wn]
@@ -147,15 +148,12 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(const float* __restrict_
       for (int r = 0; r < RP; r++) {
 #pragma unroll
         for (int i = 0; i < 4; i++) acc[r][o][i] += bv;
-        long at; if (z && place(r, o, at)) {
-#pragma unroll
-          for (int i = 0; i < 4; i++) if (4 * qx + i < c.dW) z[at + i] = acc[r][o][i];
-        }
+        if constexpr (SMOOTH) { long at; if (z && place(r, o, at)) put(z, at, acc[r][o]); }
       }
     }
   }
-  if (act != GN_ACT_RELU && act != GN_ACT_LINEAR) {
-    // Through shared memory into a loop with one copy of each activation's code, eight values side by side.  (32 inlined copies of all of them, run once, came
+  if constexpr (SMOOTH) {
+    // Through shared memory into a loop with one copy of each activation's code, four or eight values side by side.  (32 inlined copies of all of them, run once, came
     // from a cold instruction cache: ReLU took 14 us instead of 9 for 128 images of 32 x 32, 3 -> 16 channels.)
     __syncthreads();
     if (!live) return;
@@ -310,9 +308,9 @@ inline bool conv_direct_supported(const ConvShape& c) {
 // 64 -> 128: 219 / 217 / 218 against 147 / 312 / 271; 128 -> 128: 427 / 379 / 422 against 270 / 571 / 274.
 inline bool conv_direct_preferred(const ConvShape& c) { return conv_direct_supported(c) && (long)c.inC * c.outC * c.k * c.k <= 64L * 96 * 9; }
 
-template <int K, bool BWD, bool SAME>
+template <int K, bool BWD, bool SAME, int RP, bool SMOOTH>
 inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
-  constexpr int RP = 2, OC = 4;
+  constexpr int OC = 4;
   c.qw = cdiv(c.dW, 4); c.swp = SAME ? c.sW : 4 * c.qw + (K > 1 ? 4 : 0);
   if (SAME && (c.qw == 2 || c.qw == 4)) while (RP * c.swp % 32 != 4 * c.qw) c.swp += 4;      // neighbouring rows of threads in neighbouring banks
   const int groups = cdiv(c.Cd, OC), row_groups = cdiv(c.dH, RP);                 // groups of two rows
@@ -324,6 +322,12 @@ inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const fl
   const int most = 256 / c.ks;
   c.og = std::min(groups, std::max(1, std::min(32 / OC, most / c.qw)));
   int rg = std::max(1, std::min(row_groups, most / (c.qw * c.og)));
+  if (SMOOTH && RP == 1) {
+    // the busiest SM's rows, with one and a half per block for what a block costs by itself (100 images of 28 x 28, 1 -> 12 channels, tanh: 300 blocks of 10 rows
+    // 11.2 us, 400 of 7 8.8)
+    auto cost = [&](int r) { return cdiv((long)B * cdiv(row_groups, r) * cdiv(groups, c.og), ctx->sm_count) * (r + 1.5); };
+    for (int r = rg - 1; r >= 1 && r * c.qw * c.og >= 64; r--) if (cost(r) < cost(rg)) rg = r;
+  } else
   // three blocks for two SMs at least (one each: 13 % slower for 50 images of 28 x 28, three each: 14 % for 16 -> 32 channels)
   while (rg > 1 && rg * c.qw * c.og * c.ks > 64 && 2L * B * cdiv(row_groups, rg) * cdiv(groups, c.og) < 3L * ctx->sm_count) rg = (rg + 1) / 2;
   rg = cdiv(row_groups, cdiv(row_groups, rg));                       // even bands
@@ -332,16 +336,25 @@ inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const fl
   c.icc = std::max<int>(1, std::min<int>(c.Cs, 48 * 1024 / per));
   if (c.icc < c.Cs) c.icc = std::max(c.ks, c.icc / c.ks * c.ks);     // (a channel's group of threads does not depend on how many are staged at once)
   const int all = c.qw * rg * c.og, threads = (all * c.ks + 31) & ~31;
-  const size_t smem = std::max(c.icc * per + (size_t)c.og * OC * sizeof(float), (size_t)(c.ks > 1 ? c.ks * all : act != GN_ACT_RELU && act != GN_ACT_LINEAR ? threads : 0) * RP * OC * 4 * sizeof(float));
-  GN_CUDA(cudaFuncSetAttribute(conv_tile_kernel<K, BWD, SAME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GN_LAUNCH(ctx, (conv_tile_kernel<K, BWD, SAME>), dim3(cdiv(c.dH, c.rb), B, cdiv(groups, c.og)), threads, smem, src, W, bias, z, out, c, act, alpha);
+  const size_t smem = std::max(c.icc * per + (size_t)c.og * OC * sizeof(float), (size_t)(c.ks > 1 ? c.ks * all : SMOOTH ? threads : 0) * RP * OC * 4 * sizeof(float));
+  GN_CUDA(cudaFuncSetAttribute(conv_tile_kernel<K, BWD, SAME, RP, SMOOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GN_LAUNCH(ctx, (conv_tile_kernel<K, BWD, SAME, RP, SMOOTH>), dim3(cdiv(c.dH, c.rb), B, cdiv(groups, c.og)), threads, smem, src, W, bias, z, out, c, act, alpha);
   return check_launch("conv_tile");
 }
 template <int K, bool BWD>
 inline int conv_tile_launch(Ctx* ctx, int B, ConvTile c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
   c.aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  if (c.aligned && c.sW % 4 == 0 && c.dW == c.sW && 2 * c.p == K - 1) return conv_tile_run<K, BWD, true>(ctx, B, c, src, W, bias, z, out, act, alpha);
-  return conv_tile_run<K, BWD, false>(ctx, B, c, src, W, bias, z, out, act, alpha);
+  const bool same = c.aligned && c.sW % 4 == 0 && c.dW == c.sW && 2 * c.p == K - 1;
+  if constexpr (!BWD) {
+    if (act != GN_ACT_RELU && act != GN_ACT_LINEAR) {
+      // One row per thread, unless there are enough threads for two and the sums are the longer part.  us with two / one rows, tanh: 1 -> 24 channels, 50 images of 28 x 28
+      // 11.3 / 8.6; 32 -> 64, 128 of 8 x 8 28.1 / 19.4; 3 -> 32, 64 of 40 x 40 30.2 / 27.9; 16 -> 32, 128 of 16 x 16 20.2 / 18.9, 256 29.4 / 33.5; 24 -> 24, 64 of 32 x 32 32.1 / 43.2.
+      const bool two = c.Cs >= 8 && (long)B * cdiv(c.dH, 2) * cdiv(c.dW, 4) * cdiv(c.Cd, 4) > 260L * ctx->sm_count;
+      if (two) return same ? conv_tile_run<K, BWD, true, 2, true>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 2, true>(ctx, B, c, src, W, bias, z, out, act, alpha);
+      return same ? conv_tile_run<K, BWD, true, 1, true>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 1, true>(ctx, B, c, src, W, bias, z, out, act, alpha);
+    }
+  }
+  return same ? conv_tile_run<K, BWD, true, 2, false>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 2, false>(ctx, B, c, src, W, bias, z, out, act, alpha);
 }
 // z may be null (LINEAR, RELU)
 inline int conv_direct_forward(Ctx* ctx, const ConvShape& s, const float* x, const float* W, const float* bias, float* z, float* out, int act, float alpha) {

@@ -30,6 +30,9 @@ def _f(a):
     (2, 3, 100, 3, 1, 40, 40, D.RELU), (4, 16, 4, 3, 1, 2, 3, D.LINEAR),
     # windows that keep an image of whole 16-byte pieces: widths of 4 to 508, odd heights, channels dealt out to one, two and four groups, more than are staged at once
     (3, 5, 6, 3, 1, 3, 4, D.TANH), (2, 9, 18, 3, 1, 7, 8, D.RELU), (2, 17, 33, 5, 2, 9, 16, D.RELU), (1, 8, 20, 3, 1, 4, 508, D.LINEAR), (2, 130, 19, 3, 1, 11, 20, D.TANH), (5, 20, 12, 1, 0, 5, 12, D.RELU),
+    # other activations: a row per thread (windows of every size, both ways of staging, narrow images, bands of few rows), and two rows (many threads)
+    (4, 3, 9, 5, 2, 7, 8, D.TANH), (3, 4, 6, 3, 1, 9, 16, D.SIGMOID), (100, 1, 12, 3, 1, 28, 28, D.TANH), (3, 6, 7, 1, 0, 5, 12, D.SIGMOID), (2, 3, 5, 1, 0, 4, 6, D.TANH), (2, 3, 9, 5, 0, 14, 15, D.TANH),
+    (70, 9, 33, 3, 1, 17, 32, D.TANH), (90, 8, 30, 3, 0, 19, 33, D.SIGMOID),
     (2, 3, 4, 3, 1, 5, 513, D.RELU), (1, 2, 5, 5, 2, 7, 520, D.TANH), (1, 2, 3, 3, 3, 6, 9, D.RELU), (1, 2, 3, 1, 0, 3, 600, D.RELU)])      # the plain kernels' side of the limits
 def test_conv_direct(device, B, inC, outC, k, p, H, W, act):
     from goneuron_b200 import _lib
