@@ -627,9 +627,15 @@ inline int attn_head_bwd(Ctx* ctx, const float* Q, const float* K, const float* 
   GN_LAUNCH(ctx, kern, dim3(H, B), 32 * warps, smem, Q, K, V, O, dO, M, L, dQ, dK, dV, T, D, H, causal, 1.f / sqrtf((float)HD));
   return check_launch("attn_head_bwd");
 }
+enum AtKernel { AT_AUTO, AT_ROWS, AT_HEAD };                   // the kernel of the shape, blocks of 64 rows, or a block per head (the tests ask for one)
+template <int HD> inline int at_choose(const Ctx* ctx, AtKernel pick, long heads, int T, int causal, bool bwd, bool* head) {
+  *head = pick == AT_HEAD || (pick == AT_AUTO && at_head_better<HD>(ctx, heads, T, causal, bwd));
+  return *head && at_head_smem<HD>(T, bwd) > 227 * 1024 ? fail(GN_ERR_UNSUPPORTED, "attention: a head of %d tokens, size %d, does not fit shared memory", T, HD) : GN_OK;
+}
 template <int HD>
-inline int attn_fwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
-  if (at_head_better<HD>(ctx, (long)B * H, T, causal, false)) return attn_head_fwd<HD>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
+inline int attn_fwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal, AtKernel pick) {
+  bool head; GN_TRY(at_choose<HD>(ctx, pick, (long)B * H, T, causal, false, &head));
+  if (head) return attn_head_fwd<HD>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
   const int smem = 3 * AtCfg<HD>::TILE * (int)sizeof(__half) + 3 * AT_BLK * (int)sizeof(float);
   GN_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, attn_fwd_kernel<HD>, dim3(cdiv(T, AT_BLK), H, B), AT_THREADS, smem, Q, K, V, O, M, L, T, D, H, causal, 1.f / sqrtf((float)HD));
@@ -637,23 +643,24 @@ inline int attn_fwd_launch(Ctx* ctx, const float* Q, const float* K, const float
 }
 template <int HD>
 inline int attn_bwd_launch(Ctx* ctx, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
-                           float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
-  if (at_head_better<HD>(ctx, (long)B * H, T, causal, true)) return attn_head_bwd<HD>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
+                           float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal, AtKernel pick) {
+  bool head; GN_TRY(at_choose<HD>(ctx, pick, (long)B * H, T, causal, true, &head));
+  if (head) return attn_head_bwd<HD>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
   const int smem = 4 * AtCfg<HD>::TILE * (int)sizeof(__half) + 7 * AT_BLK * (int)sizeof(float);
   GN_CUDA(cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, attn_bwd_kernel<HD>, dim3(2 * cdiv(T, AT_BLK), H, B), AT_THREADS, smem, Q, K, V, O, dO, M, L, dQ, dK, dV, T, D, H, causal, 1.f / sqrtf((float)HD));
   return check_launch("attn_bwd");
 }
-inline int attn_fwd(Ctx* ctx, int hd, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
-  if (hd == 64) return attn_fwd_launch<64>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
-  if (hd == 32) return attn_fwd_launch<32>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
-  return attn_fwd_launch<16>(ctx, Q, K, V, O, M, L, B, T, D, H, causal);
+inline int attn_fwd(Ctx* ctx, int hd, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal, AtKernel pick = AT_AUTO) {
+  if (hd == 64) return attn_fwd_launch<64>(ctx, Q, K, V, O, M, L, B, T, D, H, causal, pick);
+  if (hd == 32) return attn_fwd_launch<32>(ctx, Q, K, V, O, M, L, B, T, D, H, causal, pick);
+  return attn_fwd_launch<16>(ctx, Q, K, V, O, M, L, B, T, D, H, causal, pick);
 }
 inline int attn_bwd(Ctx* ctx, int hd, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
-                    float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
-  if (hd == 64) return attn_bwd_launch<64>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
-  if (hd == 32) return attn_bwd_launch<32>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
-  return attn_bwd_launch<16>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal);
+                    float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal, AtKernel pick = AT_AUTO) {
+  if (hd == 64) return attn_bwd_launch<64>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal, pick);
+  if (hd == 32) return attn_bwd_launch<32>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal, pick);
+  return attn_bwd_launch<16>(ctx, Q, K, V, O, dO, M, L, dQ, dK, dV, B, T, D, H, causal, pick);
 }
 
 }  // namespace gn

@@ -2035,16 +2035,17 @@ int gn_op_attention(gn_ctx* ctx, int engine, int B, int T, int D, int H, int cau
   const int hd = D / H; const size_t n = (size_t)B * T * D, ns = (size_t)B * H * T;
   if (!attn_fused_supported(hd, D)) return fail(GN_ERR_UNSUPPORTED, "op_attention: head size %d", hd);
   if (engine == 1 && !attn_tc_supported(c, hd, T, B, H, D)) return fail(GN_ERR_UNSUPPORTED, "tcgen05 attention cannot run this shape (head size %d, T=%d)", hd, T);
+  const AtKernel pick = engine == 2 ? AT_ROWS : engine == 3 ? AT_HEAD : AT_AUTO;
   DevBuf q, k, v, o, m, l, g, dv_, dq, dk, dvv;
   GN_TRY(q.alloc(n)); GN_TRY(k.alloc(n)); GN_TRY(v.alloc(n)); GN_TRY(o.alloc(n)); GN_TRY(m.alloc(ns)); GN_TRY(l.alloc(ns));
   GN_CUDA(copy_h2d(c, q.p, Q, n * 4)); GN_CUDA(copy_h2d(c, k.p, K, n * 4)); GN_CUDA(copy_h2d(c, v.p, V, n * 4));
   if (engine == 1) GN_TRY(attn_tc_fwd(c, q.p, k.p, v.p, o.p, m.p, l.p, B, T, D, H, causal));
-  else GN_TRY(attn_fwd(c, hd, q.p, k.p, v.p, o.p, m.p, l.p, B, T, D, H, causal));
+  else GN_TRY(attn_fwd(c, hd, q.p, k.p, v.p, o.p, m.p, l.p, B, T, D, H, causal, pick));
   if (dO) {
     GN_TRY(g.alloc(n)); GN_TRY(dv_.alloc(ns)); GN_TRY(dq.alloc(n)); GN_TRY(dk.alloc(n)); GN_TRY(dvv.alloc(n));
     GN_CUDA(copy_h2d(c, g.p, dO, n * 4));
     if (engine == 1) GN_TRY(attn_tc_bwd(c, q.p, k.p, v.p, o.p, g.p, m.p, l.p, dv_.p, dq.p, dk.p, dvv.p, B, T, D, H, causal));
-    else GN_TRY(attn_bwd(c, hd, q.p, k.p, v.p, o.p, g.p, m.p, l.p, dq.p, dk.p, dvv.p, B, T, D, H, causal));
+    else GN_TRY(attn_bwd(c, hd, q.p, k.p, v.p, o.p, g.p, m.p, l.p, dq.p, dk.p, dvv.p, B, T, D, H, causal, pick));
     GN_CUDA(copy_d2h(c, dQ, dq.p, n * 4)); GN_CUDA(copy_d2h(c, dK, dk.p, n * 4)); GN_CUDA(copy_d2h(c, dV, dvv.p, n * 4));
   }
   GN_CUDA(copy_d2h(c, O, o.p, n * 4));

@@ -233,7 +233,9 @@ int gn_op_adam(gn_ctx* ctx, float* params, const float* grads, float* m1, float*
  * row-major with head h in columns [h*D/H, (h+1)*D/H); M and L (may be NULL) receive the row maximum and the
  * row sum of the softmax, [B*H*T].  Forward: scores q.k/sqrt(hd), causal mask, softmax, weighted sum of v
  * (transformer.go:470-503); with dO != NULL also the backward pass (transformer.go:589-657).
- * engine: 0 = warp-level tensor-core kernels, 1 = tcgen05 kernels (head size 64, T a multiple of 128). */
+ * engine: 0 = warp-level tensor-core kernels, 1 = tcgen05 kernels (head size 64, T a multiple of 128); of the former
+ * 2 = those with a block per 64 rows, 3 = those with a block per head (GN_ERR_UNSUPPORTED where a head does not fit
+ * shared memory), 0 = whichever is quicker for the shape. */
 int gn_op_attention(gn_ctx* ctx, int engine, int B, int T, int D, int H, int causal,
                     const float* Q, const float* K, const float* V, const float* dO,
                     float* O, float* M, float* L, float* dQ, float* dK, float* dV);

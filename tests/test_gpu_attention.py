@@ -84,6 +84,54 @@ def test_sequences_do_not_depend_on_the_batch(device, B, T, D, H, causal):
         assert np.array_equal(a[:n], b)
 
 
+HEADS = [  # T, head size: one to sixteen warps and two turns, lengths around multiples of 16, 32 and 64, passes of loads that end with the rows and that do not
+    (1, 32), (17, 16), (33, 32), (80, 32), (100, 16), (127, 64), (150, 32), (161, 64), (176, 64), (192, 64), (200, 32), (208, 16), (255, 32), (256, 16), (257, 32), (300, 16), (352, 32)]
+
+
+@pytest.mark.parametrize("causal", [0, 1])
+@pytest.mark.parametrize("T,hd", HEADS)
+def test_block_per_head_against_fp64_and_blocks_of_64_rows(device, T, hd, causal):
+    """Each kernel is asked for by name: float64 for the block per head, and the same bits from the blocks of 64 rows."""
+    B, H = 2, 3
+    D = H * hd
+    rng = np.random.default_rng(T + hd)
+    Q, K, V, dO = (rng.standard_normal((B * T, D)).astype(np.float32) * sc for sc in (1.5, 1.5, 1.0, 1.0))
+    got = run(device, 3, Q, K, V, dO, B, T, D, H, causal)
+    ref = reference(Q, K, V, dO, B, T, D, H, causal)
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), (got[0], got[3], got[4], got[5]), (ref[0], ref[3], ref[4], ref[5])):
+        # one token: the score's gradient is p (dp - dp), zero up to rounding
+        assert norm_err(a, b) < TOL if np.any(b) else np.max(np.abs(a)) < 1e-5, name
+    for a, b in zip(got, run(device, 2, Q, K, V, dO, B, T, D, H, causal)):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("causal", [0, 1])
+@pytest.mark.parametrize("T", [193, 200, 255, 256])
+def test_forward_of_heads_whose_backward_pass_does_not_fit(device, T, causal):
+    """Size 64: up to 256 tokens fit forward, 192 backward.  By itself the backward pass takes blocks of 64 rows; asked for a block per head it refuses."""
+    from goneuron_b200 import _lib
+    B, H, D = 52, 3, 192                                      # (more heads than SMs: forward takes a block per head of its own accord)
+    rng = np.random.default_rng(T)
+    Q, K, V, dO = (rng.standard_normal((B * T, D)).astype(np.float32) for _ in range(4))
+    f = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))
+    L = _lib.load()
+    out = []
+    for engine in (3, 2):
+        O, M, S = np.empty_like(Q), np.empty(B * H * T, np.float32), np.empty(B * H * T, np.float32)
+        _lib.check(L.gn_op_attention(device.handle, engine, B, T, D, H, causal, f(Q), f(K), f(V), None, f(O), f(M), f(S), None, None, None))
+        out.append((O, M, S))
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    auto, rows = (run(device, e, Q, K, V, dO, B, T, D, H, causal) for e in (0, 2))
+    assert all(np.array_equal(a, b) for a, b in zip(auto, rows)) and np.array_equal(auto[0], out[0][0])
+    one = slice(0, 2 * T)
+    ref = reference(Q[one], K[one], V[one], dO[one], 2, T, D, H, causal)
+    for a, b in zip((auto[0], auto[3], auto[4], auto[5]), (ref[0], ref[3], ref[4], ref[5])):
+        assert norm_err(a[one], b) < TOL
+    with pytest.raises(_lib.GoNeuronCudaError) as e:
+        run(device, 3, Q, K, V, dO, B, T, D, H, causal)
+    assert e.value.code == -5 and "shared memory" in str(e.value)
+
+
 def test_attention_bounded_waits_fail_fast_and_the_context_stays_usable(device):
     """Failure detection without a GPU fault: with a poll limit of 1 the first wait of the tcgen05 attention kernels runs
     out; the status word is set at once, every other wait of the launch then gives up within a few polls, the kernels run
