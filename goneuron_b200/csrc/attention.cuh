@@ -595,26 +595,32 @@ inline int attn_rows_bwd(Ctx* ctx, const float* Q, long ldq, const float* K, con
 // ---------------------------------------------------------------- launchers
 inline bool attn_fused_supported(int hd, int D) { return (hd == 16 || hd == 32 || hd == 64) && D % 4 == 0; }
 
-// Warps of a block per head: one per 16 rows up to 16, then as few as take the same number of turns
-inline int at_head_warps(int T) { const int n = cdiv(T, 16); return n <= 16 ? n : cdiv(n, cdiv(n, 16)); }
+// Warps of a block per head: one per 16 rows up to 16, then as few as take the same number of turns.  Heads of 32 and 64 count the rows of padding: where the number
+// would be odd, the padding took a second pass of loads (288 heads of 200 tokens, size 32, causal 28.1 -> 24.3 us, of 80 tokens 9.6 -> 8.0).
+template <int HD> inline int at_head_warps(int T) { const int n = HD == 16 ? cdiv(T, 16) : at_pad(T) / 16; return n <= 16 ? n : cdiv(n, cdiv(n, 16)); }
 // Blocks of 64 rows or a block per head?  By estimated time (us, from measured rates).  A block per head takes `h0` and `h1` per 32 keys and turn; two that share an
 // SM take 1.4 times as long as one.  A round of the others, as many as are resident, takes `t0` and `t1` per 64 keys (rows of padding count half), the last
-// round's end a quarter of one, and a block by itself 0.62 of one.  Measured, 64 rows against a head, heads x tokens (size 32, no mask) forward / backward: 288 x 150 24 - 16 /
-// 69 - 45, 512 x 150 40 - 31 / 119 - 89, 512 x 128 19 - 23 / 65 - 64, 288 x 256 39 - 34 / 129 - 101, 160 x 150 16 - 16 / 43 - 45, 64 x 150 11 - 12 / 20 - 32;
-// size 64: 288 x 150 39 - 40 / 140 - 103, 288 x 200 71 - 57 / -; with a causal mask 288 x 150, 32: 19 - 13 / 54 - 31.
+// round's end a quarter of one, and a block by itself 0.62 of one.  Not by estimate: forward with a causal mask more than two heads per SM (three for narrow heads of
+// which two share one), whose blocks last as long as their last rows while the others fill the gaps; backward, size 64, heads of one pass.
+// Measured, 64 rows against a head, heads x tokens, forward / backward (- where a head does not fit): size 32, no mask: 288 x 150 24 - 17 / 68 - 45, 512 x 128 19 - 23 / 65 - 64,
+// 288 x 200 39 - 31 / 115 - 88, 160 x 150 16 - 16 / 43 - 45; causal: 288 x 150 18.6 - 12.9 / 54 - 31, 512 x 200 44 - 46 / 143 - 125.  Size 64: 288 x 150 39 - 40 / 139 - 103,
+// 288 x 200 71 - 53 / -.  Size 16 (rates of 32): 288 x 150 18.0 - 12.9 / 46 - 31; causal 13.9 - 10.9 / 37 - 21, 512 x 200 31.6 - 38.2 / 95 - 84.  Over 2900 shapes of 8 to 1000 heads and
+// 17 to 512 tokens, both directions, the choice is slower than blocks of 64 rows in 0.5 %, by 17 % at most (7 us instead of 6); it takes the head's kernel in 13 %, where that is
+// 1.24 times as fast on average.
 template <int HD> inline bool at_head_better(const Ctx* ctx, long heads, int T, int causal, bool bwd) {
   const size_t smem = at_head_smem<HD>(T, bwd); if (smem > 227 * 1024) return false;
   constexpr bool wide = HD == 64;
   const double h0 = bwd ? (wide ? 1 : 3) : (wide ? 4 : 2.5), h1 = bwd ? (wide ? 9.6 : 6.2) : (wide ? 3.6 : 1.9), t0 = bwd ? (wide ? 7 : 5) : (wide ? 5 : 4), t1 = bwd ? (wide ? 11 : 6.7) : (wide ? 6.3 : 4);
-  const int warps = at_head_warps(T), kc = at_pad(T) / 32, turns = cdiv(cdiv(T, 16), warps), nb = cdiv(T, AT_BLK);
+  const int warps = at_head_warps<HD>(T), kc = at_pad(T) / 32, turns = cdiv(cdiv(T, 16), warps), nb = cdiv(T, AT_BLK);
   const bool pairs = warps <= 10 && 2 * (smem + 1024) <= 228 * 1024 && !(wide && bwd); const long n = cdiv(heads, ctx->sm_count);
+  if (bwd ? wide && kc == 1 : causal && n > 2 && (wide || !pairs)) return false;
   const double u = h0 + h1 * kc * turns * (causal ? 0.5 * (kc + 1) / kc : 1.0), head = u * (pairs ? n / 2 * 1.4 + n % 2 : n);
   const double w = t0 + t1 * 0.5 * (nb + T / 64.0) * (causal ? 0.5 * (nb + 1) / nb : 1.0), rounds = (double)heads * nb * (bwd ? 2 : 1) / ((wide ? 3.0 : 4.0) * ctx->sm_count);
   return head < 0.92 * w * std::max(0.62, rounds + 0.25);
 }
 template <int HD>
 inline int attn_head_fwd(Ctx* ctx, const float* Q, const float* K, const float* V, float* O, float* M, float* L, int B, int T, int D, int H, int causal) {
-  const int smem = (int)at_head_smem<HD>(T, false), warps = at_head_warps(T); auto* kern = warps <= 10 ? attn_head_fwd_kernel<HD, 320, 2> : attn_head_fwd_kernel<HD, 512, 1>;
+  const int smem = (int)at_head_smem<HD>(T, false), warps = at_head_warps<HD>(T); auto* kern = warps <= 10 ? attn_head_fwd_kernel<HD, 320, 2> : attn_head_fwd_kernel<HD, 512, 1>;
   GN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, kern, dim3(H, B), 32 * warps, smem, Q, K, V, O, M, L, T, D, H, causal, 1.f / sqrtf((float)HD));
   return check_launch("attn_head_fwd");
@@ -622,7 +628,7 @@ inline int attn_head_fwd(Ctx* ctx, const float* Q, const float* K, const float* 
 template <int HD>
 inline int attn_head_bwd(Ctx* ctx, const float* Q, const float* K, const float* V, const float* O, const float* dO, const float* M, const float* L,
                          float* dQ, float* dK, float* dV, int B, int T, int D, int H, int causal) {
-  const int smem = (int)at_head_smem<HD>(T, true), warps = at_head_warps(T); auto* kern = warps <= 10 ? attn_head_bwd_kernel<HD, 320, HD == 64 ? 1 : 2> : attn_head_bwd_kernel<HD, 512, 1>;
+  const int smem = (int)at_head_smem<HD>(T, true), warps = at_head_warps<HD>(T); auto* kern = warps <= 10 ? attn_head_bwd_kernel<HD, 320, HD == 64 ? 1 : 2> : attn_head_bwd_kernel<HD, 512, 1>;
   GN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GN_LAUNCH(ctx, kern, dim3(H, B), 32 * warps, smem, Q, K, V, O, dO, M, L, dQ, dK, dV, T, D, H, causal, 1.f / sqrtf((float)HD));
   return check_launch("attn_head_bwd");
