@@ -71,11 +71,12 @@ extern "C" int gn_op_gemm_nt_static(gn_ctx* ctx, int M, int N, int K, const floa
     GN_TRY(tc_split(c, TcSrc{B_dev + n0 * K + k0, (long)K, 1, 0, 0, 1}, PB, nullptr));
     float* C = C_dev + m0 * N + n0; const bool first = k0 == 0;
     TcParams ep{C, (long)N, 0, 0, first && bias_dev ? bias_dev + n0 : nullptr, first ? nullptr : C, first ? 0L : (long)N, 0, 0, GN_ACT_LINEAR, m, n, k, 1, 0, c->d_status, nullptr, 0, 1};
-    // the regular entry point's slices of a long contraction: side by side where the array has room for their partial results, else one by one
-    int bn = tc_pick_bn(c, m, n, 1, 0); const int splits = tc_split_count(c, ep, 1, &bn);
-    float* part = sb + ((n + 3) & ~3);
-    if (splits > 1 && (part - base) + (long)splits * m * n <= GN_STATIC_SCRATCH_FLOATS) GN_TRY(tc_run_slices(c, PA, PB, ep, splits, bn, part));
-    else GN_TRY(tc_run_rows(c, PA, PB, ep, bn, splits > 1 ? tc_slice_length(k, splits) : 0));
+    const int whole = tc_pick_bn(c, m, n, 1, 0); int bn = whole; const int splits = tc_split_count(c, ep, 1, &bn);
+    switch (static_slices(splits, m, n, k, GN_STATIC_SCRATCH_FLOATS)) {
+      case StaticSlices::SIDE_BY_SIDE: GN_TRY(tc_run_slices(c, PA, PB, ep, splits, bn, sb + ((n + 3) & ~3))); break;
+      case StaticSlices::ONE_BY_ONE: GN_TRY(tc_run_rows(c, PA, PB, ep, bn, tc_slice_length(k, splits))); break;
+      default: GN_TRY(tc_run_rows(c, PA, PB, ep, whole));
+    }
   }
   GN_CUDA(cudaStreamSynchronize(c->stream));
   return check_status_word(c);

@@ -21,4 +21,15 @@ inline StaticPieces static_pieces(long M, long N, long K, long limit) {
   return p;
 }
 
+// How a pass whose contraction the regular entry point would cut into `splits` slices runs: side by side where the array has room for their partial
+// results behind what the pass keeps, else one after the other (contractions of 1024 and more: long accumulator runs truncate more often), else whole:
+// slices of a shorter contraction are cut for speed alone, and one after the other they are slower (128 x 3900 over 1000 69 us, whole 51).
+enum class StaticSlices { WHOLE, SIDE_BY_SIDE, ONE_BY_ONE };
+inline StaticSlices static_slices(int splits, long m, long n, long k, long limit) {
+  if (splits <= 1) return StaticSlices::WHOLE;
+  const long part = ((m + n) * ((k + 31) / 32 * 32) + ((m + 3) & ~3L) + ((n + 3) & ~3L));
+  if (part + splits * m * n <= limit) return StaticSlices::SIDE_BY_SIDE;
+  return k >= 1024 ? StaticSlices::ONE_BY_ONE : StaticSlices::WHOLE;
+}
+
 }  // namespace gn

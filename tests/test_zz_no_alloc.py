@@ -83,7 +83,8 @@ def test_static_scratch_takes_every_size_of_the_documented_limit():
         dev.close()
 
 
-@pytest.mark.parametrize("M,N,K", [(4, 4, 524_280), (1, 1, 2_097_144), (1, 2, 1_398_096), (3, 4, 599_176)])
+@pytest.mark.parametrize("M,N,K", [(256, 2300, 1000), (128, 3900, 1023), (128, 3900, 1024),      # no room for the slices' partial results: whole, and one after the other
+                                   (4, 4, 524_280), (1, 1, 2_097_144), (1, 2, 1_398_096), (3, 4, 599_176)])
 def test_static_scratch_takes_long_contractions(M, N, K):
     """Few rows and a contraction at the documented limit: halved sides, and single rows walked along the contraction.  Bound: 2^-19 of
     sum |a b| (22-bit operands, an accumulator that truncates once per 16 indices, partial sums in fp32)."""
