@@ -32,7 +32,9 @@ def _gemm(device, engine, A, B, bias):
                                    # more tiles than SMs with a short last round: its tiles run as half tiles (256- and 128-wide tilings)
                                    (25600, 256, 96), (12800, 500, 64), (25600, 128, 96), (5760, 1024, 128),
                                    # rows that 16-byte accesses do not fit: 64-, 128- and 256-wide tiles, half tiles, slices
-                                   (300, 33, 96), (200, 129, 64), (12800, 501, 64), (5760, 1023, 128), (1100, 333, 1000), (70, 1001, 515)])
+                                   (300, 33, 96), (200, 129, 64), (12800, 501, 64), (5760, 1023, 128), (1100, 333, 1000), (70, 1001, 515),
+                                   # slices: two, three, five, six and seven of them, added up four columns at a time
+                                   (1000, 1000, 2048), (128, 1024, 768), (600, 600, 2048), (1024, 384, 2048), (512, 1100, 8192)])
 def test_tc_gemm_matches_fp64(device, M, N, K):
     rng = np.random.default_rng(M * 7 + N * 3 + K)
     A = rng.standard_normal((M, K)).astype(np.float32)
