@@ -1096,15 +1096,17 @@ __global__ void __launch_bounds__(256) tc_sum_slices_kernel(const float* __restr
   }
 }
 // Slices and tile width by estimated time, from measured rates (us): 0.335 / 0.43 per 32 contraction indices of a 128 / 256 wide
-// tile, 3 / 5 for the last tile's epilogue (2.4 / 3.9 since it stores whole lines; not tuned again), 3 for the second launch and 4 TB/s for its partial results.  Slices keep at least 256
-// indices, and have to win by a tenth.
+// tile, 2.4 / 3.9 for the last tile's epilogue, 3 for the second launch and 4 TB/s for its partial results.  Slices keep at least 256
+// indices, and have to win by a tenth.  Over 249 products with contractions of 512 to 32 000 (us, whole or in other slices -> as chosen): every choice below 1024 that differs from one
+// launch wins, [5000, 33] over 768 14.6 -> 12.6 the least, [150, 768] over 1000 16.0 -> 11.3; [1000, 1000] over 1500 21.6 -> 17.4, [1024, 1024] over 2048 20.2 -> 18.7 (256 wide in four, by today's
+// epilogues; with 3 / 5 for them 128 wide in two).  Rows that 16-byte pieces do not fit go by the same figures: their epilogue is longer, and slices win by more ([1100, 333] over 1000 30.8 -> 18.2).
 inline int tc_split_count(Ctx* ctx, const TcParams& ep, long nbatch, int* bn) {
   if (nbatch != 1 || ep.out_p || ep.n_seg || ep.nchw_P || ep.flags || ep.K < 512 || ctx->tc_kslice > 0 || ctx->tc_force_bn) return 1;
   const long sms = persist_sms(ctx), tm = cdiv(ep.M, TC_BM); const double kb = cdiv(ep.K, TC_BK);
   auto cost = [&](int w, int sl) {
     const long tiles = tm * cdiv(ep.N, w); double rounds = std::ceil((double)tiles * sl / sms);
     if (sl == 1 && tc_tail_halves(ctx, tiles, w, 0) > 0) rounds -= 0.38;
-    return rounds * (kb / sl) * (w == 256 ? 0.43 : 0.335) + (w == 256 ? 5.0 : 3.0) + (sl > 1 ? 3.0 + 1e-6 * ep.M * ep.N * (sl + 1) : 0.0);
+    return rounds * (kb / sl) * (w == 256 ? 0.43 : 0.335) + (w == 256 ? 3.9 : 2.4) + (sl > 1 ? 3.0 + 1e-6 * ep.M * ep.N * (sl + 1) : 0.0);
   };
   double best = 0.9 * cost(tc_pick_bn(ctx, ep.M, ep.N, 1, 0) == 256 ? 256 : 128, 1); int splits = 1;
   for (int w : {128, 256}) if (w == 128 || ep.N > 128)
