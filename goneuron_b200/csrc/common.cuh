@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/goneuron_cuda.h"
+#include "graph_rec.cuh"
 
 namespace gn {
 
@@ -28,42 +29,6 @@ inline int fail(int code, const char* fmt, ...) {
 #define GN_TRY(call) do { int rc_ = (call); if (rc_ != GN_OK) return rc_; } while (0)
 
 struct NcclApi;   // resolved at run time from libnccl.so.2 (nccl_dl.cuh)
-
-// A run of launches and copies put together as a CUDA graph, node by node, while Ctx::rec points here: the helpers below then add a
-// node behind what their stream holds so far instead of issuing the work.  (Capturing the stream gives the same graph but forbids
-// other threads to synchronise the device, or to use the stream, for as long as it lasts -- theirs then fail, and the capture with
-// them -- and a copy that another call queues meanwhile becomes part of it.)
-struct GraphRec {
-  cudaGraph_t graph = nullptr;
-  struct Tail { cudaStream_t stream; std::vector<cudaGraphNode_t> nodes; bool kernel = false; };      // kernel: `nodes` is one kernel node
-  std::vector<Tail> tails;
-  GraphRec() {}
-  GraphRec(const GraphRec&) = delete; GraphRec& operator=(const GraphRec&) = delete;
-  ~GraphRec() { if (graph) cudaGraphDestroy(graph); }
-  Tail& tail(cudaStream_t s) { for (auto& t : tails) if (t.stream == s) return t; tails.push_back(Tail{s, {}}); return tails.back(); }
-  // what `from` holds so far comes before everything that `to` gets from now on
-  void join(cudaStream_t to, cudaStream_t from) {
-    const std::vector<cudaGraphNode_t> add = tail(from).nodes; Tail& t = tail(to);
-    for (auto n : add) { bool have = false; for (auto q : t.nodes) have |= q == n; if (!have) { t.nodes.push_back(n); t.kernel = t.kernel && t.nodes.size() == 1; } }
-  }
-  template <class F> cudaError_t add(cudaStream_t s, bool kernel, F&& make) {      // make(node, dependencies, their number)
-    Tail& t = tail(s); cudaGraphNode_t node;
-    const cudaError_t e = make(&node, t.nodes.data(), t.nodes.size());
-    if (e == cudaSuccess) { t.nodes.assign(1, node); t.kernel = kernel; }
-    return e;
-  }
-  // Work on stream `s` that a replay leaves out unless a kernel before it has set `handle` (condition()) to a non-zero value.
-  cudaError_t condition(cudaGraphConditionalHandle* handle) { return cudaGraphConditionalHandleCreate(handle, graph, 0, cudaGraphCondAssignDefault); }
-  template <class F> cudaError_t only_if(cudaStream_t s, cudaGraphConditionalHandle handle, F&& body) {
-    cudaGraphNodeParams p{}; p.type = cudaGraphNodeTypeConditional; p.conditional.handle = handle; p.conditional.type = cudaGraphCondTypeIf; p.conditional.size = 1;
-    const cudaError_t e = add(s, false, [&](cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t n) { return cudaGraphAddNode(node, graph, deps, n, &p); });
-    if (e != cudaSuccess) return e;
-    cudaGraph_t outer = graph; std::vector<Tail> outer_tails; outer_tails.swap(tails);
-    graph = p.conditional.phGraph_out[0];                     // (belongs to the node)
-    body();
-    graph = outer; tails.swap(outer_tails); return cudaSuccess;
-  }
-};
 
 struct Ctx {
   int device = 0;
@@ -88,6 +53,7 @@ struct Ctx {
   float *h_block = nullptr, *h_ret = nullptr, *h_stage = nullptr, *h_out = nullptr, *d_ret = nullptr, *d_out = nullptr;
   uint64_t epoch = 0;              // counts replacements of the context's scratch buffers
   GraphRec* rec = nullptr;         // set while a step is put together as a graph instead of being issued
+  bool graph_conditions = true;    // conditional graph nodes can be made (until one is refused)
   bool tc_ok = false;              // tcgen05 engine usable (driver entry point for tensor maps found)
   void* encode_tiled = nullptr;    // cuTensorMapEncodeTiled
   unsigned spin_limit = 1u << 24;  // polls per bounded device-side wait (gn_ctx_set_spin_limit)

@@ -1199,8 +1199,7 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
       if (world == 1 && (!late || few)) gather(nullptr, late ? un : nullptr);
       else if (world == 1) GN_LAUNCH(ctx, lstm_update_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, un, T, in, H, n_updates);
       // in a recorded step the launches for all but the last groups are one conditional node
-      cudaGraphConditionalHandle skip = 0; const int tail = groups >= CLIP_SKIP_MIN && ctx->rec ? (int)groups - CLIP_TAIL : 0;
-      if (tail) GN_CUDA(ctx->rec->condition(&skip));
+      cudaGraphConditionalHandle skip = 0; const int tail = groups >= CLIP_SKIP_MIN && ctx->rec && ctx->rec->condition(&skip) ? (int)groups - CLIP_TAIL : 0;
       if (late) GN_LAUNCH(ctx, lstm_clip_start_kernel, nchunks, 1024, 0, (const float*)un, n_updates, Kc, start, skip, tail); else start = nullptr;
       if (world == 1 && late && !few) gather(start, nullptr);
       // Gram blocks of every group against the group before it and itself
@@ -1551,12 +1550,9 @@ static void note_graph(gn_model* m, StepGraph key) {
 }
 // What `issue` would launch as a graph; *out stays null when that cannot be made (the caller then runs it directly).
 template <class F> static void record(gn_model* m, F&& issue, cudaGraphExec_t* out) {
-  Ctx* ctx = &m->ctx->c; const uint64_t em = m->epoch, ec = ctx->epoch; GraphRec rec; *out = nullptr;
-  struct Guard { Ctx* c; ~Guard() { c->rec = nullptr; c->side_pending = false; cudaGetLastError(); } } guard{ctx};
-  if (cudaGraphCreate(&rec.graph, 0) != cudaSuccess) { rec.graph = nullptr; return; }
-  ctx->rec = &rec;
-  if (issue() != GN_OK || em != m->epoch || ec != ctx->epoch) return;      // (a buffer that was replaced may be in earlier nodes)
-  if (cudaGraphInstantiate(out, rec.graph, 0) != cudaSuccess) *out = nullptr;
+  Ctx* ctx = &m->ctx->c; const uint64_t em = m->epoch, ec = ctx->epoch; *out = nullptr;
+  struct Guard { Ctx* c; ~Guard() { c->side_pending = false; cudaGetLastError(); } } guard{ctx};
+  *out = record_graph(ctx->rec, ctx->graph_conditions, [&] { return issue() == GN_OK && em == m->epoch && ec == ctx->epoch; });      // (a buffer that was replaced may be in earlier nodes)
 }
 static void reset_counters(Ctx* ctx) { ctx->gemm_flops = 0; ctx->gemm_launches = 0; ctx->gemm_ms = 0; ctx->ev_used = 0; ctx->gemm_bytes = 0; ctx->split_bytes = 0; }
 
