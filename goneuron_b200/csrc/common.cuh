@@ -97,7 +97,8 @@ inline int side_join(Ctx* ctx) {
   return GN_OK;
 }
 
-// Every kernel launch of the library goes through these macros, so that the launch count is exact and a step can be recorded.
+// Every kernel launch of the library goes through these macros, so that all are counted and a step can be recorded.  (A replayed step counts what was
+// recorded, launches behind a condition among them whether they ran or not.)
 // launch_kernel(): `cluster` > 0: that many neighbouring blocks of the grid's x dimension form a thread-block cluster; `early`: the
 // blocks may be placed while the preceding kernel still runs (programmatic stream serialisation), which wants a kernel that calls
 // pdl_wait() in every block before it touches anything its predecessors write, and pdl_launch() to let its own successor in.

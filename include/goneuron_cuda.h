@@ -198,7 +198,9 @@ int gn_model_state_count(gn_model* m, int64_t* n);
 int gn_model_get_state(gn_model* m, float* host, int64_t n);
 int gn_model_set_state(gn_model* m, const float* host, int64_t n);
 
-/* Counters of the last gn_train_batch: kernels launched by this library, and
+/* Counters of the last gn_train_batch: kernels launched by this library (a step that is replayed as a
+ * CUDA graph counts the launches it holds: those of an LSTM's clipping walk that its search for the first
+ * update leaves out as a whole are among them, so that the count is an upper bound there), and
  * device time in ms of the whole step / of the part of the gradient all-reduce that
  * the compute stream had to wait for (the per-layer all-reduces run on a second
  * stream under the rest of the backward pass); CUDA events on the context's stream. */
