@@ -1161,7 +1161,8 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
     // applies the updates one by one to the matrix and otherwise runs only for chunks that are too long.
     static const bool on_matrix = [] { const char* e = getenv("GONEURON_CUDA_LSTM_SCAN"); return e && strcmp(e, "cluster") == 0; }();
     const int R4g = 4 * H, ZWg = in + H + 1, zs = clip_zs(ZWg), slabs = cdiv(R4g, 8);
-    const long Kc = (long)chunk * T, n_updates = (long)GB * T, n_local = (long)B * T, groups = (Kc + CG - 1) / CG, stride = CG_PAD + groups * CG, ng = (long)nchunks * groups, rows = nchunks * stride;
+    const long Kc = (long)chunk * T, n_updates = (long)GB * T, n_local = (long)B * T, groups = (Kc + CG - 1) / CG, ng = (long)nchunks * groups;
+    const UpdateRows u = update_rows_of_chunks(n_updates, Kc, nchunks, CG, CG_PAD); const long stride = u.stride, rows = u.rows;
     const bool fits = Kc <= CG_MAX_K && ng <= 65535;
     if (world > 1 && (on_matrix || !fits)) return fail(GN_ERR_UNSUPPORTED, "LSTM on more than one GPU needs the scalar form of the clipping recurrence (worker chunk of %ld updates)", Kc);
     if (!on_matrix && fits) {
@@ -1186,15 +1187,15 @@ static int lstm_backward(gn_model* m, LayerRT& l, size_t li, int B, const float*
         }
         float* all; GN_TRY(ensure(m, S_W, (size_t)n_updates * (R4g + zs), &all));
         float* Da = all; float* Za = all + (size_t)n_updates * R4g; float* Dl = Da + (size_t)row0 * T * R4g; float* Zl = Za + (size_t)row0 * T * zs;      // this rank's rows
-        GN_LAUNCH(ctx, lstm_gather_updates_kernel, cdiv(n_local, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, n_local, n_local, n_local, n_local, 0L, (const int*)nullptr, (float*)nullptr);
+        GN_LAUNCH(ctx, lstm_gather_updates_kernel, cdiv(n_local, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dl, Zl, T, in, H, zs, update_rows_of_rank(n_local), (const int*)nullptr, (float*)nullptr);
         GN_TRY(all_gather_on_comm(m, Dl, Da, (size_t)n_local * R4g, "LSTM update factors D"));
         GN_TRY(all_gather_on_comm(m, Zl, Za, (size_t)n_local * zs, "LSTM update factors Z"));
-        GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Da, Dm, R4g, Kc, stride, (long)CG_PAD);
-        GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Za, Zm, zs, Kc, stride, (long)CG_PAD);
-        if (late) GN_LAUNCH(ctx, lstm_row_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)Dm, (const float*)Zm, un, R4g, zs, n_updates, Kc, stride, (long)CG_PAD);
+        GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Da, Dm, R4g, u);
+        GN_LAUNCH(ctx, lstm_place_rows_kernel, (unsigned)n_updates, 128, 0, (const float*)Za, Zm, zs, u);
+        if (late) GN_LAUNCH(ctx, lstm_row_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)Dm, (const float*)Zm, un, R4g, zs, u);
       }
       auto gather = [&](const int* from, float* norms) {
-        GN_LAUNCH(ctx, lstm_gather_updates_kernel, cdiv(rows, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dm, Zm, T, in, H, zs, n_local, rows, Kc, stride, (long)CG_PAD, from, norms);
+        GN_LAUNCH(ctx, lstm_gather_updates_kernel, cdiv(rows, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, Dm, Zm, T, in, H, zs, u, from, norms);
       };
       if (world == 1 && (!late || few)) gather(nullptr, late ? un : nullptr);
       else if (world == 1) GN_LAUNCH(ctx, lstm_update_norms_kernel, cdiv(n_updates, 8), 256, 0, (const float*)l.dgate.p, xin, (const float*)l.h_all.p, un, T, in, H, n_updates);

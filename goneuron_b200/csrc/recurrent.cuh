@@ -4,6 +4,7 @@
 #include <type_traits>
 #include "common.cuh"
 #include "rowops.cuh"
+#include "update_rows.cuh"
 
 namespace gn {
 
@@ -535,16 +536,16 @@ inline size_t clip_smem(int ZW) {
   const int wp = clip_tile(ZW) | 1; const size_t slab = ((size_t)2 * CG * wp + CG * 8 + (size_t)wp * 8 + 8) * sizeof(float), walk = (size_t)CG * CG_GD * sizeof(double);
   return slab > walk ? slab : walk;
 }
-// Rows of Dm [., 4H] and Zm [., zs], a warp each: chunk c's updates from row c * stride + lead on, zeros in the rows before and behind them.
+// Rows of Dm [., 4H] and Zm [., zs] as `u` lays them out, a warp each; this rank's updates are the first ones.
 // (Zeroing those rows separately took two to four more launches per chunk.)  `un` (may be null): receives |u_k|^2 = |d_k|^2 |z_k|^2.  With a block per row
 // the rows that are left out, nearly all of 16 384, cost 12 us.
 __global__ void __launch_bounds__(256) lstm_gather_updates_kernel(const float* __restrict__ D, const float* __restrict__ x, const float* __restrict__ h_all, float* __restrict__ Dm, float* __restrict__ Zm,
-                                           int T, int in, int H, int zs, long n_updates, long rows, long Kc, long stride, long lead, const int* __restrict__ start, float* __restrict__ un) {
+                                           int T, int in, int H, int zs, const UpdateRows u, const int* __restrict__ start, float* __restrict__ un) {
   const int R4 = 4 * H, ZW = in + H + 1, lane = threadIdx.x & 31;
-  const long row = blockIdx.x * 8L + (threadIdx.x >> 5); if (row >= rows) return;
-  const long chunk = row / stride, r = row - chunk * stride - lead, k = chunk * Kc + r;
-  if (start && r < (long)(start[chunk] - 1) * CG) return;                     // before the first walked group and the one it is multiplied with
-  if (r < 0 || r >= Kc || k >= n_updates) {
+  const long row = blockIdx.x * 8L + (threadIdx.x >> 5); if (row >= u.rows) return;
+  const UpdateRows::At at = u.at(row); const long k = at.k;
+  if (start && at.r < (long)(start[at.chunk] - 1) * CG) return;               // before the first walked group and the one it is multiplied with
+  if (!at.update) {
     for (int e = lane; e < R4 + zs; e += 32) { if (e < R4) Dm[row * R4 + e] = 0.f; else Zm[row * zs + e - R4] = 0.f; }
     return;
   }
@@ -564,8 +565,8 @@ __global__ void __launch_bounds__(256) lstm_gather_updates_kernel(const float* _
   if (lane == 0) un[k] = d2 * z2;
 }
 // rows of `w` floats from contiguous order into the chunks' layout (after a gather over the ranks)
-__global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int w, long Kc, long stride, long lead) {
-  const long k = blockIdx.x, row = (k / Kc) * stride + lead + k % Kc;
+__global__ void lstm_place_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int w, const UpdateRows u) {
+  const long k = blockIdx.x, row = u.row_of(k);
   for (int e = threadIdx.x; e < w; e += blockDim.x) dst[row * w + e] = src[k * w + e];
 }
 __global__ void lstm_gram_mul_kernel(float* __restrict__ G, const float* __restrict__ G2, long total4, int groups, const int* __restrict__ start) {
@@ -591,9 +592,9 @@ __global__ void __launch_bounds__(256) lstm_update_norms_kernel(const float* __r
   if (lane == 0) un[k] = d2 * z2;
 }
 // ... from gathered rows
-__global__ void __launch_bounds__(256) lstm_row_norms_kernel(const float* __restrict__ Dm, const float* __restrict__ Zm, float* __restrict__ un, int R4, int zs, long n_updates, long Kc, long stride, long lead) {
-  const long k = blockIdx.x * 8L + (threadIdx.x >> 5); const int lane = threadIdx.x & 31; if (k >= n_updates) return;
-  const long row = (k / Kc) * stride + lead + k % Kc; float d2 = 0.f, z2 = 0.f;
+__global__ void __launch_bounds__(256) lstm_row_norms_kernel(const float* __restrict__ Dm, const float* __restrict__ Zm, float* __restrict__ un, int R4, int zs, const UpdateRows u) {
+  const long k = blockIdx.x * 8L + (threadIdx.x >> 5); const int lane = threadIdx.x & 31; if (k >= u.n) return;
+  const long row = u.row_of(k); float d2 = 0.f, z2 = 0.f;
 #pragma unroll 4
   for (int e = lane; e < R4; e += 32) d2 = fmaf(Dm[row * R4 + e], Dm[row * R4 + e], d2);
   for (int e = lane; e < zs; e += 32) z2 = fmaf(Zm[row * zs + e], Zm[row * zs + e], z2);
