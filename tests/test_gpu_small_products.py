@@ -42,6 +42,23 @@ def test_rows_against_float64_and_the_same_in_every_batch(device, N, K):
         assert np.array_equal(product(device, A[:m], B, bias), whole[:m]), m
 
 
+@pytest.mark.parametrize("N", [1, 10, 16])
+@pytest.mark.parametrize("K", [128, 513, 1100, 2048, 4704])
+def test_few_columns_against_float64_and_the_same_in_every_batch(device, N, K):
+    """Sixteen columns or fewer: one row per cluster of blocks, or four where there are many (from 593, 297, 149 and 75 rows on for clusters of one, two, four and eight), with one to three rows
+    left over.  A thread adds up K / 256 products at most, then come five exchanges, eight warps, eight blocks and the bias."""
+    rng = np.random.Generator(np.random.PCG64(N + K))
+    A = rng.standard_normal((603, K)).astype(np.float32)
+    B = rng.standard_normal((N, K)).astype(np.float32)
+    bias = rng.standard_normal(N).astype(np.float32)
+    exact = A.astype(np.float64) @ B.astype(np.float64).T + bias
+    bound = (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T + np.abs(bias)) * (K / 256 + 24) * 2.0 ** -24
+    whole = product(device, A, B, bias)
+    assert np.all(np.abs(whole - exact) <= bound)
+    for m in (1, 2, 70, 74, 75, 148, 150, 296, 299, 592, 601, 602):
+        assert np.array_equal(product(device, A[:m], B, bias), whole[:m]), m
+
+
 @pytest.mark.parametrize("M,N,K", [(3001, 33, 72), (5000, 33, 65), (2050, 130, 65), (9001, 33, 130), (5000, 70, 130), (9001, 33, 260),      # one, two and four chunks per block
                                    (5000, 33, 128), (5000, 100, 191), (777, 70, 256), (300, 100, 512),                              # ... a chunk per block of two, four and eight
                                    (5000, 100, 256), (5000, 100, 512), (5000, 33, 512)])                                            # ... several per block of several
