@@ -325,7 +325,7 @@ inline bool gemm_outer_small_ok(const GemmDesc& g) {
 // matter, and where the rows of A are samples a sample's result is the same in every batch.
 // us per launch in a recorded chain, a 32 x 32 tile in two register-staged steps per run, results read from the other blocks -> this:
 //   64 x 256 over 256 4.9 -> 3.7, over 1024 7.5 -> 5.9; 128 x 1024 over 256 7.6 -> 5.8; 1 x 128 over 784 5.6 -> 3.5; 8 x 8192 over 512 13.3 -> 7.4;
-//   16 x 512 over 8192 25.7 -> 15.4; a 96 x 96 weight gradient over 5000 rows 14.3 -> 10.1.  The same chain of empty launches: 2.2.
+//   16 x 512 over 8192 25.7 -> 14.7; a 96 x 96 weight gradient over 5000 rows 14.3 -> 9.7.  The same chain of empty launches: 2.2.
 constexpr int SP_KB = 64, SP_BN = 32, SP_STAGES = 4, SP_THREADS = 256, SP_MAX_SPLITS = 8;
 constexpr int sp_smem(int tm) { return (SP_STAGES * SP_KB * (4 * tm + SP_BN) + 8 * 4 * tm * SP_BN) * (int)sizeof(float); }
 // Brings ROWS operand rows x 64 indices into shared memory, stage by stage.  KFAST: [row][64], 16-byte units swizzled by the row's position among
@@ -342,16 +342,16 @@ struct SpLoad {
 #pragma unroll
     for (int q = 0; q < NQ; q++) { int r, k; place(q, r, k); src[q] = p + (KFAST ? r * s_r + k : r + k * s_k); }
   }
-  // nk: indices that are left, this stage included; upto: how many of the stage's are read later.  PLAIN: rows that 16-byte copies do not fit come by
+  // nk: indices that are left, this stage included.  PART (a check per copy of it cost the kernel below 2 %): only the first `upto` of the stage are wanted, and rows that 16-byte copies do not fit come by
   // loads and stores, 16 of a thread's at a time, instead of 4-byte asynchronous copies (whole stages waited for at once: 2 to 10 % quicker).
-  template <bool PLAIN = false>
+  template <bool PART = false>
   __device__ __forceinline__ void fetch(float* __restrict__ dst, int nk, int upto = SP_KB) {
     if (vec) {
 #pragma unroll
       for (int q = 0; q < NQ; q++) {
         int r, k; place(q, r, k);
         if (NV % THREADS != 0 && q * THREADS + (int)threadIdx.x >= NV) break;
-        if (k >= upto) continue;
+        if (PART && k >= upto) continue;
         const int n = KFAST ? (r < nr ? min(max(nk - k, 0), 4) : 0) : (k < nk ? min(max(nr - r, 0), 4) : 0);
         cp_async16_part(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) : k * ROWS + r), n ? src[q] : base, n);
         src[q] += KFAST ? (long)SP_KB : SP_KB * s_k;
@@ -359,7 +359,7 @@ struct SpLoad {
     } else {
       const int r0 = KFAST ? threadIdx.x >> 6 : threadIdx.x % ROWS, k0 = KFAST ? threadIdx.x & 63 : threadIdx.x / ROWS; const float* p = base + r0 * s_r + k0 * s_k;
       constexpr int RSTEP = THREADS / SP_KB, KSTEP = THREADS / ROWS;
-      if (PLAIN) {
+      if (PART) {
         constexpr int NF = 16;
         for (int q0 = 0; q0 < ROWS * SP_KB / THREADS; q0 += NF) {
           float x[NF];
@@ -378,7 +378,7 @@ struct SpLoad {
 #pragma unroll
       for (int q = 0; q < ROWS * SP_KB / THREADS; q++) {
         const int r = KFAST ? r0 + RSTEP * q : r0, k = KFAST ? k0 : k0 + KSTEP * q; const bool ok = r < nr && k < nk;
-        if (k < upto) cp_async4(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) + (k & 3) : k * ROWS + r), ok ? p : base, ok);
+        cp_async4(dst + (KFAST ? r * SP_KB + (((k >> 2) ^ (r >> 2 & 7)) << 2) + (k & 3) : k * ROWS + r), ok ? p : base, ok);
         p += KFAST ? RSTEP * s_r : KSTEP * s_k;
       }
       if (nk > SP_KB) base += SP_KB * s_k;
