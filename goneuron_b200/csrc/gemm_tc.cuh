@@ -62,9 +62,9 @@ constexpr int TC_FLAG_VEC = 4096;   // epilogue may use 16-byte accesses (set by
 // [8192, 1024] x [1024, 256] from 26.8 to 18.6, [32768, 1024] x [1024, 1024] from 136 to 119 (zeros as data: no power limit).
 constexpr int TC_BK = 32, PL_LO = 32;
 __host__ __device__ __forceinline__ int pl_off(int k) { return ((k >> 5) << 6) | (k & 31); }
-// What a variant of the kernel writes: fp32 in 16-byte pieces, operand planes, or fp32 where 16-byte pieces do not fit (an odd number of columns, NCHW).  (The
-// last one's code beside the first one's cost every product 2 %.)  PL: planes.
-enum TcOut { TC_OUT_VEC, TC_OUT_PLANES, TC_OUT_ANY };
+// What a variant of the kernel writes: fp32 in 16-byte pieces or in NCHW order, operand planes, or rows of fp32 that 16-byte pieces do not fit (an odd number of columns).  (The
+// last one's code beside the first one's cost every product 2 %; without the NCHW order's beside it 256-wide tiles were 0.3 us slower, [4096, 1000] over 256 11.5 -> 11.8.)  PL: planes.
+enum TcOut { TC_OUT_VEC, TC_OUT_PLANES, TC_OUT_ROWS };
 template <int BN, bool PL> struct TcCfg {
   static constexpr int EW = PL ? 16 : 8, CG = EW / 4, CC = PL ? 16 : 32;          // epilogue warps, column groups, columns of a chunk
   static constexpr int THREADS = 64 + 32 * EW;                                    // TMA warp, MMA warp, epilogue warps
@@ -345,7 +345,7 @@ __device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tm
   }
   float* C = ep.C + z1 * ep.c_b1 + z2 * ep.c_b2;
   const float* R = ep.R ? ep.R + z1 * ep.r_b1 + z2 * ep.r_b2 : nullptr;
-  if constexpr (OUT == TC_OUT_VEC) {
+  if (OUT == TC_OUT_VEC && (ep.flags & TC_FLAG_VEC)) {
     const int rl = lane >> 3, c8 = lane & 7, r0 = rbase + rl;                // after the exchange: this lane's rows r0 + 4 t and columns 4 c8 .. 4 c8 + 3 of a chunk
     float4 sv, bv, rv[8];                                                    // what the next chunk needs for them
     auto fetch = [&](int c) {
@@ -402,7 +402,7 @@ __device__ __forceinline__ bool tc_epilogue_tile(const TcParams& ep, uint32_t tm
     __syncwarp();
     return true;
   }
-  if (ep.nchw_P == 0) {
+  if constexpr (OUT == TC_OUT_ROWS) {
     // rows that 16-byte accesses do not fit (an odd number of columns): through the staging buffer all the same, then a row at a time, a column per lane.
     // (A row per lane, a column at a time, touched 32 lines per instruction: [2048, 1001] over 256 29 -> 16 us.)
     if (!wait()) return false;
@@ -886,7 +886,7 @@ inline int tc_planes(Ctx* ctx, int which, long nbatch, long rows, int K, BfPlane
 inline int* tc_rowmax_buf(Ctx* ctx) { return reinterpret_cast<int*>(tc_scratch(ctx).mx.p); }
 
 template <int BN, TcOut OUT> inline bool tc_set_smem1() { return cudaFuncSetAttribute(gemm_tc_persist_kernel<BN, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<BN, OUT == TC_OUT_PLANES>::SMEM_BYTES) == cudaSuccess; }
-template <int BN> inline bool tc_set_smem() { return tc_set_smem1<BN, TC_OUT_VEC>() && tc_set_smem1<BN, TC_OUT_PLANES>() && tc_set_smem1<BN, TC_OUT_ANY>(); }
+template <int BN> inline bool tc_set_smem() { return tc_set_smem1<BN, TC_OUT_VEC>() && tc_set_smem1<BN, TC_OUT_PLANES>() && tc_set_smem1<BN, TC_OUT_ROWS>(); }
 inline void tc_init(Ctx* ctx) {
   ctx->tc_ok = false;
   void* fn = nullptr; cudaDriverEntryPointQueryResult q;
@@ -981,8 +981,8 @@ inline int tc_launch_persist(Ctx* ctx, const BfPlanes& A, const BfPlanes& B, con
   if (ctx->tc_tile_queue && total > grid) GN_TRY(tc_next_queue(ctx, &queue));
   ProfScope prof(ctx);
   if (ep.out_p) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_PLANES>), grid, (TcCfg<BN, true>::THREADS), (TcCfg<BN, true>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
-  else if (ep.flags & TC_FLAG_VEC) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_VEC>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
-  else GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_ANY>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  else if ((ep.flags & TC_FLAG_VEC) || ep.nchw_P > 0) GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_VEC>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
+  else GN_LAUNCH(ctx, (gemm_tc_persist_kernel<BN, TC_OUT_ROWS>), grid, (TcCfg<BN, false>::THREADS), (TcCfg<BN, false>::SMEM_BYTES), mA, mB, ep, tiles_m, tiles_n, (int)total, full_end, n_half, queue);
   return check_launch("gemm_tc_persist");
 }
 // Output tile width for a problem: 64 for narrow outputs; 256 (three quarters of the shared-memory traffic per MMA
