@@ -930,13 +930,15 @@ static int side_weight_bias_grads(gn_model* m, int stack, int B, int out, int in
   Ctx* ctx = &m->ctx->c; auto issue = [&]() -> int { return weight_bias_grads_stack(m, stack, B, out, in, dz, x, ldx, gW, gb, ws); };
   return grads_on_side(ctx, stack, B, out, in, ldx) ? side_run(ctx, issue) : issue();
 }
-// The parameter gradients of up to four layers from dense rows of dz, in one launch beside the main stream where they are sums of few outer products;
-// others go one by one when they are added.
+// The parameter gradients of up to four layers from dense rows of dz, in one launch where they are sums of few outer products; others go one by one when they are
+// added.  `chain`: what follows on the main stream are more links of small products (a causal block's token rows), and the launch runs beside them.  Else products over
+// all tokens follow, whose blocks want whole SMs: large gradients go beside the main stream at once, one by one, and the launch for the small ones is a link of it.
+// (Training steps, us, one launch beside the main stream -> this: 33 x 432 tokens, 512 wide, one block 499 -> 478, 36 x 71, 768 wide, seven 5584 -> 5553.)
 struct GradGroup {
-  gn_model* m; GemmDesc d[4]; int n = 0;
+  gn_model* m; bool chain; GemmDesc d[4]; int n = 0;
   int add(int B, int out, int in, const float* dz, const float* x, long ldx, float* gW, float* gb) {
     GemmDesc g; g.M = out; g.N = in; g.K = B; g.A = dz; g.sa_m = 1; g.sa_k = out; g.B = x; g.sb_k = ldx; g.sb_n = 1; g.C = gW; g.ldc = in; g.a_sum = gb;
-    if (m->ctx->c.profile || !gemm_outer_small_ok(g) || n == 4) return side_weight_bias_grads(m, 1, B, out, in, dz, x, ldx, gW, gb);
+    if (m->ctx->c.profile || !gemm_outer_small_ok(g) || n == 4 || (!chain && grads_on_side(&m->ctx->c, 1, B, out, in, ldx))) return side_weight_bias_grads(m, 1, B, out, in, dz, x, ldx, gW, gb);
     d[n++] = g; return GN_OK;
   }
   int flush() {
@@ -944,7 +946,7 @@ struct GradGroup {
     Ctx* ctx = &m->ctx->c; double macs = 0; for (int j = 0; j < n; j++) macs += (double)d[j].M * d[j].N * d[j].K;
     ctx->gemm_flops += 2.0 * macs; ctx->gemm_launches++;
     auto issue = [&]() -> int { return gemm_outer_group(ctx, d, n); };
-    const int rc = macs >= 3.0e6 ? side_run(ctx, issue) : issue(); n = 0; return rc;
+    const int rc = chain && macs >= 3.0e6 ? side_run(ctx, issue) : issue(); n = 0; return rc;
   }
 };
 // Can the FFN's hidden activation (and its gradient) of this block live as operand planes only?  The two contractions on
@@ -1099,7 +1101,7 @@ static int block_backward_row0(gn_model* m, LayerRT& l, int B, const float* xin,
     return check_launch("norm_rows");
   };
   GN_TRY(norm(gout, r2_0, bp.g2, st + 2 * NE, dR2, (float*)gp.g2, (float*)gp.be2, S_PART2));
-  GradGroup grads{m};
+  GradGroup grads{m, d.causal != 0};
   GN_TRY(grads.add(B, D, F, dR2, mid_last, ld_mid, (float*)gp.w2, (float*)gp.b2));
   GemmDesc g; g.M = B; g.N = F; g.K = D; g.A = dR2; g.sa_m = D; g.sa_k = 1; g.B = bp.w2; g.sb_k = F; g.sb_n = 1; g.C = dM; g.ldc = F;
   if (l.ff_act == GN_ACT_RELU) { g.mask = mid_last; g.mask_ld = ld_mid; }
