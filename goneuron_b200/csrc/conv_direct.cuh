@@ -30,7 +30,7 @@ __device__ __forceinline__ void conv_stage(float* dst, int plane, int ld, const 
 // ------------------------------------------------------------------ forward and input gradient
 // dst[b, d, y, x] = act( bias[d] + sum_{s, kh, kw} w(d, s, kh, kw) src[b, s, y + kh - p, x + kw - p] ), zeros outside.  Forward: w = W[d][s].
 // Input gradient (BWD): src = gradient of the pre-activation, w = W[s][d] mirrored, p = K - 1 - pad.
-// A thread owns 4 neighbouring pixels of RP = two rows (one, where the activation is the longer part) x 4 channels and every `ks`-th source channel; a block a band of `rb` rows of one image and
+// A thread owns 4 neighbouring pixels of RP = two rows (one, where there are few threads, or the activation is the longer part) x 4 channels and every `ks`-th source channel; a block a band of `rb` rows of one image and
 // `og` groups of 4 channels, with the source rows and the weights of `icc` source channels at a time in shared memory.  What bounds it is less
 // the arithmetic than everything around it: index arithmetic and uncoalesced copies on the way into shared memory, by few threads, took most
 // of its time.  So the weights are copied in their own order, image rows in 16-byte pieces where the window keeps the image's size (SAME; the border is
@@ -308,25 +308,29 @@ inline bool conv_direct_supported(const ConvShape& c) {
 // 64 -> 128: 219 / 217 / 218 against 147 / 312 / 271; 128 -> 128: 427 / 379 / 422 against 270 / 571 / 274.
 inline bool conv_direct_preferred(const ConvShape& c) { return conv_direct_supported(c) && (long)c.inC * c.outC * c.k * c.k <= 64L * 96 * 9; }
 
+// Input gradients: source channels in up to four groups of threads while a block still has three groups of two rows (or all): by the shapes alone.  us with 1 / 2 / 4: 16 -> 32
+// channels, 128 images of 16 x 16 17.0 / 14.2 / 13.2; 32 -> 64, 64 of 20 x 20 43 / 41 / 48; 16 -> 64, 20 of 16 x 16 30 / 21 / 15.  Forward in one group: a block has
+// enough threads there (13.4 / - / 15.3), and ReLU and pooling see sums in the order of the channels.
+inline int conv_dgrad_groups(const ConvTile& c) {
+  int ks = c.Cs >= 16 ? 4 : c.Cs >= 8 ? 2 : 1; const int qw = cdiv(c.dW, 4), groups = cdiv(c.Cd, 4);
+  while (ks > 1 && 256 / ks < qw * std::min(groups, 8) * std::min((int)cdiv(c.dH, 2), 3)) ks /= 2;
+  return ks;
+}
 template <int K, bool BWD, bool SAME, int RP, bool SMOOTH>
 inline int conv_tile_run(Ctx* ctx, int B, ConvTile c, const float* src, const float* W, const float* bias, float* z, float* out, int act, float alpha) {
   constexpr int OC = 4;
   c.qw = cdiv(c.dW, 4); c.swp = SAME ? c.sW : 4 * c.qw + (K > 1 ? 4 : 0);
   if (SAME && (c.qw == 2 || c.qw == 4)) while (RP * c.swp % 32 != 4 * c.qw) c.swp += 4;      // neighbouring rows of threads in neighbouring banks
   const int groups = cdiv(c.Cd, OC), row_groups = cdiv(c.dH, RP);                 // groups of two rows
-  // Input gradients: source channels in up to four groups of threads while a block still has three groups of rows (or all).  us with 1 / 2 / 4: 16 -> 32
-  // channels, 128 images of 16 x 16 17.0 / 14.2 / 13.2; 32 -> 64, 64 of 20 x 20 43 / 41 / 48; 16 -> 64, 20 of 16 x 16 30 / 21 / 15.  Forward in one group: a block has
-  // enough threads there (13.4 / - / 15.3), and ReLU and pooling see sums in the order of the channels.
-  c.ks = !BWD ? 1 : c.Cs >= 16 ? 4 : c.Cs >= 8 ? 2 : 1;
-  while (c.ks > 1 && 256 / c.ks < c.qw * std::min(groups, 32 / OC) * std::min(row_groups, 3)) c.ks /= 2;
+  c.ks = BWD ? conv_dgrad_groups(c) : 1;
   const int most = 256 / c.ks;
   c.og = std::min(groups, std::max(1, std::min(32 / OC, most / c.qw)));
   int rg = std::max(1, std::min(row_groups, most / (c.qw * c.og)));
-  if (SMOOTH && RP == 1) {
+  if (RP == 1) {
     // the busiest SM's rows, with one and a half per block for what a block costs by itself (100 images of 28 x 28, 1 -> 12 channels, tanh: 300 blocks of 10 rows
     // 11.2 us, 400 of 7 8.8)
     auto cost = [&](int r) { return cdiv((long)B * cdiv(row_groups, r) * cdiv(groups, c.og), ctx->sm_count) * (r + 1.5); };
-    for (int r = rg - 1; r >= 1 && r * c.qw * c.og >= 64; r--) if (cost(r) < cost(rg)) rg = r;
+    for (int r = rg - 1; r >= 1 && r * c.qw * c.og * c.ks >= 64; r--) if (cost(r) < cost(rg)) rg = r;
   } else
   // three blocks for two SMs at least (one each: 13 % slower for 50 images of 28 x 28, three each: 14 % for 16 -> 32 channels)
   while (rg > 1 && rg * c.qw * c.og * c.ks > 64 && 2L * B * cdiv(row_groups, rg) * cdiv(groups, c.og) < 3L * ctx->sm_count) rg = (rg + 1) / 2;
@@ -348,11 +352,18 @@ inline int conv_tile_launch(Ctx* ctx, int B, ConvTile c, const float* src, const
   if constexpr (!BWD) {
     if (act != GN_ACT_RELU && act != GN_ACT_LINEAR) {
       // One row per thread, unless there are enough threads for two and the sums are the longer part.  us with two / one rows, tanh: 1 -> 24 channels, 50 images of 28 x 28
-      // 11.3 / 8.6; 32 -> 64, 128 of 8 x 8 28.1 / 19.4; 3 -> 32, 64 of 40 x 40 30.2 / 27.9; 16 -> 32, 128 of 16 x 16 20.2 / 18.9, 256 29.4 / 33.5; 24 -> 24, 64 of 32 x 32 32.1 / 43.2.
-      const bool two = c.Cs >= 8 && (long)B * cdiv(c.dH, 2) * cdiv(c.dW, 4) * cdiv(c.Cd, 4) > 260L * ctx->sm_count;
+      // 11.3 / 8.6; 24 -> 24, 64 of 30 x 30, 1 x 1 26.5 / 18.3; 32 -> 64, 128 of 8 x 8 28.1 / 19.4; 3 -> 32, 64 of 40 x 40 30.2 / 27.9; 16 -> 32, 128 of 16 x 16 20.2 / 18.9, 256 29.4 / 33.5; 24 -> 24, 64 of 32 x 32 32.1 / 43.2.
+      const bool two = c.Cs * K * K >= 72 && (long)B * cdiv(c.dH, 2) * cdiv(c.dW, 4) * cdiv(c.Cd, 4) > 260L * ctx->sm_count;
       if (two) return same ? conv_tile_run<K, BWD, true, 2, true>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 2, true>(ctx, B, c, src, W, bias, z, out, act, alpha);
       return same ? conv_tile_run<K, BWD, true, 1, true>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 1, true>(ctx, B, c, src, W, bias, z, out, act, alpha);
     }
+  }
+  if constexpr (BWD) {
+    // One row per thread where there are few threads (fewer where rows come in 16-byte pieces: 3 -> 26, 120 of 28 x 28 14.9 with one row, 13.1 with two), or nothing that
+    // two rows share (1 x 1 windows, unless rows come in 16-byte pieces).  us with two / one: 16 -> 64 channels, 20
+    // images of 16 x 16, 3 x 3 15.1 / 11.7, 1 x 1 9.8 / 5.6; 24 -> 24, 64 of 30 x 30 39.9 / 31.0, 1 x 1 14.1 / 10.5; 16 -> 32, 128 of 16 x 16 12.9 / 15.9; 32 -> 64, 64 of 20 x 20 40.6 / 48.8.
+    const bool two = (K > 1 || same) && (long)B * cdiv(c.dH, 2) * cdiv(c.dW, 4) * cdiv(c.Cd, 4) * conv_dgrad_groups(c) > (same ? 300L : 320L) * ctx->sm_count;
+    if (!two) return same ? conv_tile_run<K, BWD, true, 1, false>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 1, false>(ctx, B, c, src, W, bias, z, out, act, alpha);
   }
   return same ? conv_tile_run<K, BWD, true, 2, false>(ctx, B, c, src, W, bias, z, out, act, alpha) : conv_tile_run<K, BWD, false, 2, false>(ctx, B, c, src, W, bias, z, out, act, alpha);
 }

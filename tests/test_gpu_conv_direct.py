@@ -33,6 +33,7 @@ def _f(a):
     # other activations: a row per thread (windows of every size, both ways of staging, narrow images, bands of few rows), and two rows (many threads)
     (4, 3, 9, 5, 2, 7, 8, D.TANH), (3, 4, 6, 3, 1, 9, 16, D.SIGMOID), (100, 1, 12, 3, 1, 28, 28, D.TANH), (3, 6, 7, 1, 0, 5, 12, D.SIGMOID), (2, 3, 5, 1, 0, 4, 6, D.TANH), (2, 3, 9, 5, 0, 14, 15, D.TANH),
     (70, 9, 33, 3, 1, 17, 32, D.TANH), (90, 8, 30, 3, 0, 19, 33, D.SIGMOID),
+    (200, 16, 32, 1, 0, 16, 16, D.RELU), (200, 16, 16, 5, 2, 12, 12, D.RELU), (60, 24, 24, 1, 0, 30, 30, D.TANH),      # input gradients of many threads: two rows, and 1 x 1 windows in one
     (2, 3, 4, 3, 1, 5, 513, D.RELU), (1, 2, 5, 5, 2, 7, 520, D.TANH), (1, 2, 3, 3, 3, 6, 9, D.RELU), (1, 2, 3, 1, 0, 3, 600, D.RELU)])      # the plain kernels' side of the limits
 def test_conv_direct(device, B, inC, outC, k, p, H, W, act):
     from goneuron_b200 import _lib
